@@ -11,28 +11,25 @@ size_t mm_tiles_bytes(int64_t rows, int64_t n_expert, int64_t n_out);
 size_t mm_tiled_bytes(int64_t rows, int64_t n_expert, int64_t k);
 cudaError_t launch_gather_tiles(const void *x, int x_f16, int x_per_row, int top_k, int k, const uint32_t *tpe,
                                 const int32_t *ids_map, int map_stride, int n_expert, void *xt, int32_t *pos,
-                                int32_t *spos, int32_t *sfid, cudaStream_t s);
+                                int32_t *spos, int32_t *sfid, int nt, cudaStream_t s);
+int mm_tile_rows(int64_t rows, int64_t n_expert);
 lmoe_status launch_mm_gateup(const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const void *xt,
                              const uint32_t *tpe, const int32_t *ids_map, int64_t map_stride, int64_t list_rows,
                              float *act, int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream);
-bool mm_down_available(const lmoe_expert_stack *down);
-lmoe_status launch_mm_down(const lmoe_expert_stack *down, const void *xt, const uint32_t *tpe, const int32_t *ids_map,
-                           int64_t map_stride, int64_t list_rows, const float *row_scale, float *out, int sorted,
-                           void *tiles_ws, uint32_t *flag, cudaStream_t stream);
 lmoe_status launch_mm_id(const lmoe_expert_stack *st, const void *xt, const uint32_t *tpe, const int32_t *ids_map,
-                         int64_t map_stride, int64_t list_rows, const float *row_scale, float *out, void *tiles_ws,
-                         uint32_t *flag, cudaStream_t stream);
+                         int64_t map_stride, int64_t list_rows, const float *row_scale, float *out, int sorted,
+                         void *tiles_ws, uint32_t *flag, cudaStream_t stream);
 
 namespace {
 
 // One warp per row: act = silu(g) * u; l2 = clamp(||act||, 1e-8, 1e30); the f16 operand of the
 // down projection is act * 32768 / l2 (src/moe.rs:292-302), written in the grouped GEMM's tile
-// order (row tile pos / LMOE_MM_N, row pos % LMOE_MM_N, 128-byte swizzle, groups of 8 as [0 2 1 3 4 6 5 7]);
+// order (row tile pos / nt, row pos % nt, 128-byte swizzle, groups of 8 as [0 2 1 3 4 6 5 7]);
 // scale[row] = l2 * 2^-15 * weight[row] undoes it in the down epilogue together with the
 // routing weight (src/ops/combine.metal:102-133).
 __global__ void __launch_bounds__(256) swiglu_rows_kernel(const float *__restrict__ g, const float *__restrict__ u,
                                                           const float *__restrict__ w, const int32_t *__restrict__ pos,
-                                                          int64_t rows, int ff, uint8_t *__restrict__ act,
+                                                          int64_t rows, int ff, int nt, uint8_t *__restrict__ act,
                                                           float *__restrict__ scale) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -66,7 +63,7 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const float *__restric
         __align__(16) __half2 h[4] = {__floats2half2_rn(a[0], a[2]), __floats2half2_rn(a[1], a[3]),
                                       __floats2half2_rn(a[4], a[6]), __floats2half2_rn(a[5], a[7])};
         const int ci = i >> 3;
-        const size_t off = (((size_t)(p / LMOE_MM_N) * (ff / 64) + (ci >> 3)) * LMOE_MM_N + (p % LMOE_MM_N)) * 128 +
+        const size_t off = (((size_t)(p / nt) * (ff / 64) + (ci >> 3)) * nt + (p % nt)) * 128 +
                            ((size_t)((ci & 7) ^ (p & 7)) << 4);
         *reinterpret_cast<uint4 *>(act + off) = *reinterpret_cast<const uint4 *>(h);
     }
@@ -77,7 +74,7 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const float *__restric
 // With `sfid` the rows of `a` (and of `scale`) are in expert-sorted order and sfid[row] is the flat id.
 __global__ void __launch_bounds__(256) rescale_rows_kernel(const float *__restrict__ a, const float *__restrict__ w,
                                                            const int32_t *__restrict__ pos, const int32_t *__restrict__ sfid,
-                                                           int64_t rows, int ff, uint8_t *__restrict__ act,
+                                                           int64_t rows, int ff, int nt, uint8_t *__restrict__ act,
                                                            float *__restrict__ scale) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -100,7 +97,7 @@ __global__ void __launch_bounds__(256) rescale_rows_kernel(const float *__restri
         __align__(16) __half2 h[4] = {__floats2half2_rn(a0.x * k, a0.z * k), __floats2half2_rn(a0.y * k, a0.w * k),
                                       __floats2half2_rn(a1.x * k, a1.z * k), __floats2half2_rn(a1.y * k, a1.w * k)};
         const int ci = i >> 3;
-        const size_t off = (((size_t)(p / LMOE_MM_N) * (ff / 64) + (ci >> 3)) * LMOE_MM_N + (p % LMOE_MM_N)) * 128 +
+        const size_t off = (((size_t)(p / nt) * (ff / 64) + (ci >> 3)) * nt + (p % nt)) * 128 +
                            ((size_t)((ci & 7) ^ (p & 7)) << 4);
         *reinterpret_cast<uint4 *>(act + off) = *reinterpret_cast<const uint4 *>(h);
     }
@@ -257,36 +254,32 @@ lmoe_status ffn_grouped(const lmoe_expert_stack *gate, const lmoe_expert_stack *
     float *rs = c.take<float>((size_t)rows);
     int32_t *sfid = c.take<int32_t>((size_t)rows);
     void *tiles = ws + c.off;
+    const int nt = mm_tile_rows(rows, ne);
     lmoe_status st;
     const bool fused_gu = gate->dtype == LMOE_Q4_K && up->dtype == LMOE_Q4_K;
-    const bool fused_dn = mm_down_available(down);
-    const bool sorted = spos && scale_out && fused_gu && fused_dn;
+    const bool sorted = spos && scale_out && fused_gu;
     if (sorted_used) *sorted_used = sorted;
     if (masked) {
         // some (token, slot) pairs name no expert: the lists skip them, and the per-row arrays mark them
-        if (!sorted) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "masked slots need the fused Q4_K / Q6_K kernels");
+        if (!sorted) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "masked slots need the fused Q4_K gate/up kernel");
         LMOE_CUDA(cudaMemsetAsync(spos, 0xFF, (size_t)rows * 4, s));
         LMOE_CUDA(cudaMemsetAsync(sfid, 0xFF, (size_t)rows * 4, s));
     }
     LMOE_CUDA(launch_gather_tiles(x, x_f16, 1, top_k, (int)hidden, tpe, ids_map, (int)map_stride, (int)ne, xt, pos,
-                                  sorted ? spos : nullptr, sorted ? sfid : nullptr, s));
+                                  sorted ? spos : nullptr, sorted ? sfid : nullptr, nt, s));
     if (fused_gu) {
         // both projections in one pass over the activations, SwiGLU in the epilogue
         if ((st = launch_mm_gateup(gate, up, xt, tpe, ids_map, map_stride, rows, g, sorted, tiles, flag, s))) return st;
-        rescale_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(g, row_w, pos, sorted ? sfid : nullptr, rows, (int)ff,
+        rescale_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(g, row_w, pos, sorted ? sfid : nullptr, rows, (int)ff, nt,
                                                                        act, sorted ? scale_out : rs);
         LMOE_LAUNCH_CHECK("rescale_rows_kernel");
     } else {
-        if ((st = launch_mm_id(gate, xt, tpe, ids_map, map_stride, rows, nullptr, g, tiles, flag, s))) return st;
-        if ((st = launch_mm_id(up, xt, tpe, ids_map, map_stride, rows, nullptr, u, tiles, flag, s))) return st;
-        swiglu_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(g, u, row_w, pos, rows, (int)ff, act, rs);
+        if ((st = launch_mm_id(gate, xt, tpe, ids_map, map_stride, rows, nullptr, g, 0, tiles, flag, s))) return st;
+        if ((st = launch_mm_id(up, xt, tpe, ids_map, map_stride, rows, nullptr, u, 0, tiles, flag, s))) return st;
+        swiglu_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(g, u, row_w, pos, rows, (int)ff, nt, act, rs);
         LMOE_LAUNCH_CHECK("swiglu_rows_kernel");
     }
-    if (fused_dn)
-        st = launch_mm_down(down, act, tpe, ids_map, map_stride, rows, sorted ? nullptr : rs, y, sorted, tiles, flag, s);
-    else
-        st = launch_mm_id(down, act, tpe, ids_map, map_stride, rows, rs, y, tiles, flag, s);
-    return st;
+    return launch_mm_id(down, act, tpe, ids_map, map_stride, rows, sorted ? nullptr : rs, y, sorted, tiles, flag, s);
 }
 
 bool layer_mm_ok(const lmoe_layer *L) {
@@ -439,8 +432,8 @@ static lmoe_status mm_id_run(const lmoe_expert_stack *stack, const float *x, int
     const uint32_t *tpe = static_cast<const uint32_t *>(map0);
     const int32_t *ids_map = reinterpret_cast<const int32_t *>(static_cast<const uint8_t *>(map0) + stack->n_expert * 4);
     LMOE_CUDA(launch_gather_tiles(x, 0, (int)x_per_row, (int)top_k, (int)k, tpe, ids_map, (int)t, (int)stack->n_expert, xt,
-                                  nullptr, nullptr, nullptr, s));
-    return launch_mm_id(stack, xt, tpe, ids_map, t, t * top_k, nullptr, out, tiles, flag, s);
+                                  nullptr, nullptr, nullptr, mm_tile_rows(t * top_k, stack->n_expert), s));
+    return launch_mm_id(stack, xt, tpe, ids_map, t, t * top_k, nullptr, out, 0, tiles, flag, s);
 }
 
 extern "C" lmoe_status lmoe_mul_mm_id_shared(const lmoe_expert_stack *stack, const float *x, int64_t t, int64_t x_per_row,
