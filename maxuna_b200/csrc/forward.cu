@@ -11,7 +11,7 @@ lmoe_status launch_moe_decode(const lmoe_layer *Ly, const float *x, int t, float
                               void *workspace, size_t workspace_bytes, int first_launch, cudaStream_t stream);
 // prefill.cu
 size_t prefill_workspace_bytes(const lmoe_layer *Ly, int64_t t);
-lmoe_status launch_moe_prefill(const lmoe_layer *Ly, const float *x, int64_t t, float *out, uint32_t *ids_out,
+lmoe_status launch_moe_prefill(const lmoe_layer *Ly, const float *x, const float *residual, int64_t t, float *out, uint32_t *ids_out,
                                float *w_out, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 
 size_t experts_prefill_workspace_bytes(const lmoe_layer *L, int64_t t);
@@ -167,7 +167,7 @@ extern "C" lmoe_status lmoe_moe_forward_prefill(const lmoe_layer *layer, const f
     lmoe_status st = forward_check(layer, x, t, out);
     if (st) return st;
     if (t == 0) return LMOE_OK;
-    return launch_moe_prefill(layer, x, t, out, ids_out, weights_out, workspace, workspace_bytes, (cudaStream_t)stream);
+    return launch_moe_prefill(layer, x, nullptr, t, out, ids_out, weights_out, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 // The device-side address of a page-locked, device-mapped host buffer; NULL for pageable or unknown memory
@@ -339,10 +339,9 @@ extern "C" lmoe_status lmoe_moe_layer_forward(const lmoe_layer *layer, const flo
     float *normed = reinterpret_cast<float *>(static_cast<uint8_t *>(workspace) + block_ws);
     if ((st = lmoe_rms_norm(ffn_inp, norm_weight, eps, t, layer->hidden, normed, stream))) return st;
     // mat-vec kernel up to 64 tokens, grouped GEMM beyond (measured crossover; the reference's own is 32)
-    if (t >= lmoe_mm_id_min_seq())
-        st = lmoe_moe_forward_prefill(layer, normed, t, out, ids_out, weights_out, workspace, block_ws, stream);
-    else
-        st = lmoe_moe_forward_decode(layer, normed, t, out, ids_out, weights_out, workspace, block_ws, stream);
+    if (t >= lmoe_mm_id_min_seq()) // x = ffn_inp + ffn_out in the slot sum
+        return launch_moe_prefill(layer, normed, ffn_inp, t, out, ids_out, weights_out, workspace, block_ws, (cudaStream_t)stream);
+    st = lmoe_moe_forward_decode(layer, normed, t, out, ids_out, weights_out, workspace, block_ws, stream);
     if (st) return st;
     // x = ffn_inp + ffn_out
     LMOE_CUDA(launch_add_inplace(out, ffn_inp, t * layer->hidden, (cudaStream_t)stream));

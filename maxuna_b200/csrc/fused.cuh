@@ -13,3 +13,10 @@ enum {
 // seam checks shared by the mat-vec and grouped-GEMM entry points (api.cu)
 lmoe_status lmoe_id_shape_check(const lmoe_expert_stack *stack, const void *x, int64_t t, int64_t x_per_row,
                                 int64_t k, const void *ids, int64_t t_ids, int64_t top_k, const void *out);
+
+// Rows of one grouped product (mm_id.cu): `rows` routed rows over n_expert lists, `extra` rows of the shared expert behind
+// them, row tiles of nt rows.
+struct MmRows {
+    int64_t rows, extra, max_tiles;
+    int n_expert, nt;
+};

@@ -52,7 +52,9 @@ __global__ void combine_kernel(const float *__restrict__ down, const float *__re
 }
 
 // One block per expert: scan the tokens in chunks of 1024 (four consecutive tokens per thread), keep the
-// token order, write flat ids `token*top_k + slot`.
+// token order, write flat ids `token*top_k + slot`.  VEC: the four tokens' ids as top_k 16-byte words (t a multiple of
+// four, `ids` aligned): a quarter of the load instructions, which are what the scan spends its time on.
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 map0_kernel(const uint32_t *__restrict__ ids, int t, int top_k, int n_expert, uint32_t *__restrict__ tpe,
             int32_t *__restrict__ ids_map) {
@@ -64,17 +66,38 @@ map0_kernel(const uint32_t *__restrict__ ids, int t, int top_k, int n_expert, ui
     __syncthreads();
     int32_t *dst = ids_map + (size_t)e * t;
     for (int t0 = 0; t0 < t; t0 += 1024) {
-        int slot[4], mine = 0;
+        int slot[4] = {-1, -1, -1, -1}, mine = 0;
+        const int tok0 = t0 + 4 * (int)threadIdx.x;
+        if (VEC) {
+            if (tok0 < t) {
+                const uint4 *p = reinterpret_cast<const uint4 *>(ids + (size_t)tok0 * top_k);
+                int j = 0, s = 0; // token and slot of the next id
+                for (int i = 0; i < top_k; i++) {
+                    const uint4 v = __ldg(p + i);
+                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int token = t0 + 4 * (int)threadIdx.x + j;
-            slot[j] = -1;
-            if (token < t) {
-                for (int s = 0; s < top_k; s++)
-                    if (ids[(size_t)token * top_k + s] == (uint32_t)e) { slot[j] = s; break; }
+                    for (int q = 0; q < 4; q++) {
+                        if (w[q] == (uint32_t)e) {
+#pragma unroll
+                            for (int jj = 0; jj < 4; jj++)
+                                if (jj == j && slot[jj] < 0) slot[jj] = s;
+                        }
+                        if (++s == top_k) { s = 0; j++; }
+                    }
+                }
             }
-            mine += slot[j] >= 0;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int token = tok0 + j;
+                if (token < t) {
+                    for (int s = 0; s < top_k; s++)
+                        if (ids[(size_t)token * top_k + s] == (uint32_t)e) { slot[j] = s; break; }
+                }
+            }
         }
+#pragma unroll
+        for (int j = 0; j < 4; j++) mine += slot[j] >= 0;
         // exclusive prefix of the per-thread counts inside the warp, then over the warps
         int pre = mine;
 #pragma unroll
@@ -174,7 +197,10 @@ cudaError_t launch_combine(const float *down, const float *col_l2, const float *
 cudaError_t launch_map0(const uint32_t *ids, int t, int top_k, int n_expert, uint32_t *tpe, int32_t *ids_map,
                         cudaStream_t s) {
     if (n_expert == 0) return cudaSuccess;
-    map0_kernel<<<n_expert, 256, 0, s>>>(ids, t, top_k, n_expert, tpe, ids_map);
+    if (t % 4 == 0 && (reinterpret_cast<uintptr_t>(ids) & 15u) == 0)
+        map0_kernel<true><<<n_expert, 256, 0, s>>>(ids, t, top_k, n_expert, tpe, ids_map);
+    else
+        map0_kernel<false><<<n_expert, 256, 0, s>>>(ids, t, top_k, n_expert, tpe, ids_map);
     return cudaGetLastError();
 }
 

@@ -139,45 +139,39 @@ __device__ __forceinline__ uint32_t h2_sub_mul(uint32_t v, uint32_t base, uint32
     return r;
 }
 
-// ---- tile list -----------------------------------------------------------------------
-// tiles[i] = {expert, first list index, valid rows, first weight row, row-tile slot, first sorted row};
-// m tiles vary fastest so
-// CTAs running side by side share the same activation rows in L2.
-__global__ void __launch_bounds__(512) build_tiles_kernel(const uint32_t *__restrict__ tpe, int n_expert, int n_out,
-                                                          int32_t *__restrict__ tiles, int32_t *__restrict__ n_tiles,
-                                                          int max_tiles, int m_step, int nt_rows) {
-    __shared__ int pre[513], rpre[513];
-    const int m_tiles = (n_out + m_step - 1) / m_step;
-    const int e = threadIdx.x;
-    const int cnt = e < n_expert ? (int)((tpe[e] + nt_rows - 1) / nt_rows) * m_tiles : 0;
-    pre[e + 1] = cnt;
-    rpre[e + 1] = e < n_expert ? (int)tpe[e] : 0;
-    if (e == 0) pre[0] = rpre[0] = 0;
-    __syncthreads();
-    if (e == 0)
-        for (int i = 1; i <= 512; i++) pre[i] += pre[i - 1];
-    if (e == 32)
-        for (int i = 1; i <= 512; i++) rpre[i] += rpre[i - 1];
-    __syncthreads();
-    // every thread takes tiles idx, idx + 512, ...; the expert of a tile is found in the prefix table
-    const int total = min(pre[512], max_tiles);
-    for (int o = threadIdx.x; o < total; o += 512) {
-        int lo = 0, hi = n_expert - 1;
-        while (lo < hi) { // last expert whose first tile is <= o
-            const int mid = (lo + hi + 1) >> 1;
-            if (pre[mid] <= o) lo = mid; else hi = mid - 1;
-        }
-        const int ex = lo, rel = o - pre[ex];
-        const int nt = rel / m_tiles, m = rel - nt * m_tiles, n0 = nt * nt_rows;
-        const int rows = (int)tpe[ex];
-        tiles[8 * o + 0] = ex;
-        tiles[8 * o + 1] = n0;
-        tiles[8 * o + 2] = min(nt_rows, rows - n0);
-        tiles[8 * o + 3] = m * m_step;
-        tiles[8 * o + 4] = pre[ex] / m_tiles + nt;
-        tiles[8 * o + 5] = rpre[ex] + n0; // first row of the tile in expert-sorted row order
+// ---- row tiles -----------------------------------------------------------------------
+// The routed rows of an expert are cut into tiles of nt.  tiles[i] = {expert, first list index, valid rows, first row in
+// expert-sorted order}; i is also the slot of the tile in the tile-ordered operands.  A GEMM tile is (row tile, block of
+// 128 weight rows), the latter varying fastest, so CTAs running side by side share the same activation rows in L2.
+// With `extra` > 0 one more list follows the experts' ("expert" n_expert): the rows 0 .. extra-1 of the shared expert.
+__global__ void __launch_bounds__(1024) row_tiles_kernel(const uint32_t *__restrict__ tpe, int n_expert, int extra, int nt,
+                                                         int4 *__restrict__ tiles, int32_t *__restrict__ n_tiles, int max_tiles) {
+    __shared__ int2 warp_sum[32];
+    const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+    const int rows = e < n_expert ? (int)tpe[e] : (e == n_expert ? extra : 0);
+    const int cnt = (rows + nt - 1) / nt;
+    int ct = cnt, cr = rows; // inclusive prefix sums
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, ct, o), b = __shfl_up_sync(0xffffffffu, cr, o);
+        if (lane >= o) { ct += a; cr += b; }
     }
-    if (e == 0) *n_tiles = min(pre[512], max_tiles);
+    if (lane == 31) warp_sum[warp] = make_int2(ct, cr);
+    __syncthreads();
+    if (warp == 0) {
+        int2 v = warp_sum[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, v.x, o), b = __shfl_up_sync(0xffffffffu, v.y, o);
+            if (lane >= o) { v.x += a; v.y += b; }
+        }
+        warp_sum[lane] = v;
+        if (lane == 31) *n_tiles = min(v.x, max_tiles);
+    }
+    __syncthreads();
+    const int t0 = ct - cnt + (warp ? warp_sum[warp - 1].x : 0), r0 = cr - rows + (warp ? warp_sum[warp - 1].y : 0);
+    for (int i = 0; i < cnt; i++)
+        if (t0 + i < max_tiles) tiles[t0 + i] = make_int4(e, i * nt, min(nt, rows - i * nt), r0 + i * nt);
 }
 
 // Routed rows -> the f16 B operand in TILE ORDER.  Row tile `slot` (nt routed rows of one expert)
@@ -185,51 +179,35 @@ __global__ void __launch_bounds__(512) build_tiles_kernel(const uint32_t *__rest
 // of a B stage: row rr at rr*128 B, its 16-byte chunk c at position c ^ (rr & 7) (the 128-byte
 // swizzle of the tensor core's K-major layout), 8 values per chunk in the order [0 2 1 3 4 6 5 7]
 // (the order in which the dequantiser emits a chunk of weights).  A B stage is then ONE bulk copy.
+// (Tile::gather4 loads straight from token order take 62 cycles for four rows, 2960 for the 192 rows of a stage that is
+// multiplied in 770.)
 // pos[flat id] = slot*nt + rr lets later kernels (SwiGLU) write rows in the same order.
 __device__ __forceinline__ size_t tiled_off(int slot, int k_stages, int ks, int rr, int c, int nt) {
     return (((size_t)slot * k_stages + ks) * nt + rr) * 128 + ((size_t)(c ^ (rr & 7)) << 4);
 }
 
+// A block takes GT_ROWS rows of one row tile, one warp per row: the work is even however the rows fall to the experts.
+constexpr int GT_ROWS = 32;
 template <bool XF16>
 __global__ void __launch_bounds__(256) gather_tiles_kernel(const void *__restrict__ xv, int x_per_row, int top_k, int k,
-                                                           const uint32_t *__restrict__ tpe, const int32_t *__restrict__ ids_map,
-                                                           int map_stride, int n_expert, int nt, uint8_t *__restrict__ xt,
+                                                           const int4 *__restrict__ tiles, const int32_t *__restrict__ n_tiles,
+                                                           const int32_t *__restrict__ ids_map, int map_stride, int n_expert,
+                                                           int routed_rows, int nt, uint8_t *__restrict__ xt,
                                                            int32_t *__restrict__ pos, int32_t *__restrict__ spos,
                                                            int32_t *__restrict__ sfid) {
-    __shared__ int warp_sum[8], warp_rows[8];
-    __shared__ int slot0_s, row0_s;
-    const int e = blockIdx.x;
-    // slot of this expert's first row tile = number of row tiles of all earlier experts; likewise its
-    // first row in expert-sorted order = number of rows of all earlier experts
-    int part = 0, rpart = 0;
-    for (int i = threadIdx.x; i < e; i += 256) {
-        part += (int)((tpe[i] + nt - 1) / nt);
-        rpart += (int)tpe[i];
-    }
-    for (int o = 16; o; o >>= 1) {
-        part += __shfl_xor_sync(0xffffffffu, part, o);
-        rpart += __shfl_xor_sync(0xffffffffu, rpart, o);
-    }
-    if ((threadIdx.x & 31) == 0) { warp_sum[threadIdx.x >> 5] = part; warp_rows[threadIdx.x >> 5] = rpart; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0, r = 0;
-        for (int i = 0; i < 8; i++) { t += warp_sum[i]; r += warp_rows[i]; }
-        slot0_s = t;
-        row0_s = r;
-    }
-    __syncthreads();
-    const int slot0 = slot0_s, srow0 = row0_s, rows = (int)tpe[e], k_stages = k / MM_K, chunks = k / 8;
-    // one warp per routed row, eight rows of the expert in flight per block
-    const int lane = threadIdx.x & 31;
-    for (int i = blockIdx.y * 8 + (threadIdx.x >> 5); i < rows; i += gridDim.y * 8) {
-        const int fid = ids_map[(size_t)e * map_stride + i];
-        const size_t srow = (size_t)(x_per_row == 1 ? fid / top_k : fid) * k;
-        const int slot = slot0 + i / nt, rr = i % nt;
+    const int slot = blockIdx.x;
+    if (slot >= *n_tiles) return;
+    const int4 T = tiles[slot];
+    const int lane = threadIdx.x & 31, k_stages = k / MM_K, chunks = k / 8;
+    const int end = min(T.z, (int)(blockIdx.y + 1) * GT_ROWS);
+    for (int rr = blockIdx.y * GT_ROWS + (threadIdx.x >> 5); rr < end; rr += 8) {
+        const bool shared = T.x == n_expert; // the shared expert's rows are the tokens in order, their ids follow the routed ones
+        const int fid = shared ? routed_rows + T.y + rr : ids_map[(size_t)T.x * map_stride + T.y + rr];
+        const size_t srow = (size_t)(shared ? T.y + rr : (x_per_row == 1 ? fid / top_k : fid)) * k;
         if (lane == 0) {
             if (pos) pos[fid] = slot * nt + rr;
-            if (spos) spos[fid] = srow0 + i;
-            if (sfid) sfid[srow0 + i] = fid;
+            if (spos) spos[fid] = T.w + rr;
+            if (sfid) sfid[T.w + rr] = fid;
         }
 #pragma unroll 4
         for (int ci = lane; ci < chunks; ci += 32) {
@@ -298,16 +276,18 @@ struct GmCfg {
 struct GmParams {
     // Q4_K: 2-D byte views [n_expert * n_out rows][row_bytes], box = 144 bytes x 128 rows.
     // Q6_K (n_out a multiple of 8): eight rows as one line, [rows / 8][8 * row_bytes], box = 240 bytes x 16 lines
-    CUtensorMap map[2];
+    // [0, 1]: the experts' stacks (gate / up, or one projection), [2, 3]: the shared expert's
+    CUtensorMap map[4];
     CUtensorMap map_out;     // NPROJ = 1, sorted rows: `out` as [rows][n_out] f32, box = 32 values x 16 rows
     int rows8;
-    const uint8_t *w[2];     // stack blocks (gate / up, or one projection)
+    const uint8_t *w[2];     // Q6_K, n_out not a multiple of 8: stack blocks, shared expert's blocks
+    int n_expert, m_tiles;   // list number of the shared expert; blocks of 128 weight rows
     int64_t expert_bytes;
     int n_out, k;
     const uint8_t *xt;       // f16 activations in tile order (see gather_tiles_kernel)
     const int32_t *ids_map;  // [n_expert, map_stride] flat ids
     int map_stride;
-    const int32_t *tiles;    // [n_tiles][8], see build_tiles_kernel
+    const int4 *tiles;       // row tiles, see row_tiles_kernel
     const int32_t *n_tiles;
     const float *row_scale;  // per flat id, or NULL (NPROJ = 1, rows by flat id)
     float *out;              // rows of n_out values
@@ -394,14 +374,16 @@ __device__ __forceinline__ void dequant_q6k_regs(const Q6Fields &F, int lh, uint
 // One entry of the tile table.  Every role reads the entry of its next tile while it works on the current one: a table
 // read costs most of a microsecond, a fifth of a thin tile's whole time.
 struct GmTile {
-    int e, l0, nv, m0, slot, srow;
+    int e, sh; // expert; 1 for the shared expert (then e is 0)
+    int l0, nv, m0, slot, srow;
 };
 __device__ __forceinline__ GmTile gm_tile(const GmParams &P, int tile, int n_tiles) {
-    GmTile T = {0, 0, 0, 0, 0, 0};
+    GmTile T = {0, 0, 0, 0, 0, 0, 0};
     if (tile < n_tiles) {
-        const int4 a = __ldg(reinterpret_cast<const int4 *>(P.tiles) + 2 * tile);
-        const int2 b = __ldg(reinterpret_cast<const int2 *>(P.tiles) + 4 * tile + 2);
-        T = {a.x, a.y, a.z, a.w, b.x, b.y};
+        const int slot = tile / P.m_tiles;
+        const int4 a = __ldg(P.tiles + slot);
+        const int sh = a.x == P.n_expert;
+        T = {sh ? 0 : a.x, sh, a.y, a.z, (tile - slot * P.m_tiles) * MM_M, slot, a.w};
     }
     return T;
 }
@@ -508,7 +490,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
     static_assert(C::NB <= 8 && C::RAW_SLOTS <= 4 && C::NA <= 4, "barrier table");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n_tiles = *P.n_tiles;
+    const int n_tiles = *P.n_tiles * P.m_tiles;
     const int n_blk = P.k / QK_K, k_blocks = P.k / MM_K;
     const int row_bytes = n_blk * (DT == LMOE_Q4_K ? Q4K_BYTES : Q6K_BYTES);
 
@@ -647,7 +629,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                         mb_expect_tx(&raw_full[slot], (uint32_t)C::RAW_SLOT);
 #pragma unroll
                         for (int p = 0; p < NPROJ; p++)
-                            tma_load_2d(dst + p * MM_M * Q4K_BYTES, &P.map[p], b * Q4K_BYTES, T.e * P.n_out + T.m0, &raw_full[slot]);
+                            tma_load_2d(dst + p * MM_M * Q4K_BYTES, &P.map[2 * T.sh + p], b * Q4K_BYTES, T.e * P.n_out + T.m0, &raw_full[slot]);
                     }
                 } else if (P.rows8) {
                     // 210-byte blocks start at any even address, and a row is not a multiple of 16 bytes long, but eight rows
@@ -658,7 +640,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                         mb_expect_tx(&raw_full[slot], (uint32_t)C::RAW_SLOT);
 #pragma unroll
                         for (int r8 = 0; r8 < 8; r8++)
-                            tma_load_2d(dst + r8 * 16 * GM_Q6_PITCH, &P.map[0], (r8 * row_bytes + b * Q6K_BYTES) & ~15,
+                            tma_load_2d(dst + r8 * 16 * GM_Q6_PITCH, &P.map[2 * T.sh], (r8 * row_bytes + b * Q6K_BYTES) & ~15,
                                         (T.e * P.n_out + T.m0) >> 3, &raw_full[slot]);
                     }
                 } else {
@@ -668,7 +650,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                     __syncwarp();
                     const int64_t o0 = (int64_t)T.e * P.expert_bytes + (int64_t)T.m0 * row_bytes + b * Q6K_BYTES;
                     for (int r = lane; r < vrows; r += 32)
-                        bulk_g2s(dst + ((r & 7) * 16 + (r >> 3)) * GM_Q6_PITCH, P.w[0] + ((o0 + (int64_t)r * row_bytes) & ~(int64_t)15),
+                        bulk_g2s(dst + ((r & 7) * 16 + (r >> 3)) * GM_Q6_PITCH, P.w[T.sh] + ((o0 + (int64_t)r * row_bytes) & ~(int64_t)15),
                                  GM_Q6_COPY, &raw_full[slot]);
                 }
                 __syncwarp();
@@ -777,37 +759,52 @@ static int mm_m_tiles(int64_t n_out) { return (int)((n_out + MM_M - 1) / MM_M); 
 // against 739; 640: 3192 against 2790).
 int mm_tile_rows(int64_t rows, int64_t n_expert) { return rows <= 40 * n_expert ? 128 : 192; }
 
-int64_t mm_max_tiles(int64_t rows, int64_t n_expert, int64_t n_out) {
-    const int nt = mm_tile_rows(rows, n_expert);
-    return ((rows + nt - 1) / nt + n_expert) * mm_m_tiles(n_out);
-}
+// Row tiles that `rows` routed rows over n_lists lists can make.
+static int64_t mm_max_row_tiles(int64_t rows, int64_t n_lists, int nt) { return (rows + nt - 1) / nt + n_lists; }
 
 bool mm_id_kernel_available(int dtype, int64_t n_out, int64_t k) {
     return (dtype == LMOE_Q4_K || dtype == LMOE_Q6_K) && n_out > 0 && k > 0 && k % QK_K == 0;
 }
 
-size_t mm_tiles_bytes(int64_t rows, int64_t n_expert, int64_t n_out) {
-    return lmoe_align_up((size_t)mm_max_tiles(rows, n_expert, n_out) * 32 + 256, 256);
+// Sizes and scratch of one grouped product: `rows` routed rows over n_expert lists, and `extra` rows of the shared expert.
+MmRows mm_rows(int64_t rows, int64_t extra, int64_t n_expert) {
+    MmRows R;
+    R.rows = rows;
+    R.extra = extra;
+    R.n_expert = (int)n_expert;
+    R.nt = mm_tile_rows(rows, n_expert);
+    R.max_tiles = mm_max_row_tiles(rows, n_expert, R.nt) + (extra ? mm_max_row_tiles(extra, 1, R.nt) : 0);
+    return R;
+}
+// Row tile table; its last 256 bytes hold the tile count.
+size_t mm_tiles_bytes(const MmRows &R) { return lmoe_align_up((size_t)R.max_tiles * sizeof(int4), 256) + 256; }
+// The tile-ordered f16 operand of width k.
+size_t mm_tiled_bytes(const MmRows &R, int64_t k) { return lmoe_align_up((size_t)R.max_tiles * (size_t)(k / MM_K) * R.nt * 128, 256); }
+
+static int32_t *mm_tile_count(const MmRows &R, void *tiles_ws) {
+    return reinterpret_cast<int32_t *>(static_cast<uint8_t *>(tiles_ws) + mm_tiles_bytes(R) - 256);
 }
 
-// Bytes of the tile-ordered f16 operand for `rows` routed rows of width k.
-size_t mm_tiled_bytes(int64_t rows, int64_t n_expert, int64_t k) {
-    const int nt = mm_tile_rows(rows, n_expert);
-    return lmoe_align_up((size_t)((rows + nt - 1) / nt + n_expert) * (size_t)(k / MM_K) * nt * 128, 256);
-}
-
-cudaError_t launch_gather_tiles(const void *x, int x_f16, int x_per_row, int top_k, int k, const uint32_t *tpe,
-                                const int32_t *ids_map, int map_stride, int n_expert, void *xt, int32_t *pos,
-                                int32_t *spos, int32_t *sfid, int nt, cudaStream_t s) {
-    // enough blocks per expert to cover the device even when one expert holds all the rows
-    const int gy = n_expert >= 64 ? 16 : (n_expert >= 8 ? 128 : 1024);
+// Row tiles from the per-expert counts, then the operand in tile order.  pos / spos / sfid (each may be NULL): position in
+// tile order and in expert-sorted order of every flat id, flat id of every sorted row; the shared expert's rows have the
+// flat ids rows, rows + 1, ...
+lmoe_status launch_gather_tiles(const MmRows &R, const void *x, int x_f16, int x_per_row, int top_k, int k, const uint32_t *tpe,
+                                const int32_t *ids_map, int64_t map_stride, void *tiles_ws, void *xt, int32_t *pos, int32_t *spos,
+                                int32_t *sfid, cudaStream_t s) {
+    if (R.n_expert > 512) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "grouped GEMM supports at most 512 experts");
+    int4 *tiles = static_cast<int4 *>(tiles_ws);
+    int32_t *n_tiles = mm_tile_count(R, tiles_ws);
+    row_tiles_kernel<<<1, 1024, 0, s>>>(tpe, R.n_expert, (int)R.extra, R.nt, tiles, n_tiles, (int)R.max_tiles);
+    LMOE_LAUNCH_CHECK("row_tiles_kernel");
+    const dim3 grid((unsigned)R.max_tiles, (unsigned)((R.nt + GT_ROWS - 1) / GT_ROWS));
     if (x_f16)
-        gather_tiles_kernel<true><<<dim3(n_expert, gy), 256, 0, s>>>(x, x_per_row, top_k, k, tpe, ids_map, map_stride, n_expert, nt,
-                                                                     static_cast<uint8_t *>(xt), pos, spos, sfid);
+        gather_tiles_kernel<true><<<grid, 256, 0, s>>>(x, x_per_row, top_k, k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
+                                                       (int)R.rows, R.nt, static_cast<uint8_t *>(xt), pos, spos, sfid);
     else
-        gather_tiles_kernel<false><<<dim3(n_expert, gy), 256, 0, s>>>(x, x_per_row, top_k, k, tpe, ids_map, map_stride, n_expert, nt,
-                                                                      static_cast<uint8_t *>(xt), pos, spos, sfid);
-    return cudaGetLastError();
+        gather_tiles_kernel<false><<<grid, 256, 0, s>>>(x, x_per_row, top_k, k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
+                                                        (int)R.rows, R.nt, static_cast<uint8_t *>(xt), pos, spos, sfid);
+    LMOE_LAUNCH_CHECK("gather_tiles_kernel");
+    return LMOE_OK;
 }
 
 // A 2-D TMA view [rows][row_elems], boxes of box_elems x box_rows.  The encoder is a driver entry point, fetched through
@@ -843,40 +840,36 @@ static lmoe_status make_rows_map(CUtensorMap *map, const void *base, uint64_t ro
     return make_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, row_bytes, rows, box_bytes, box_rows);
 }
 
+// st / sh: the stacks of the one or two projections, of the experts and (NULL without extra rows) of the shared expert.
 template <int DT, int NPROJ, int NT>
-static lmoe_status launch_grouped(const lmoe_expert_stack *st0, const lmoe_expert_stack *st1, const void *xt, const uint32_t *tpe,
-                                  const int32_t *ids_map, int64_t map_stride, int64_t list_rows, const float *row_scale, float *out,
+static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *const (&st)[2], const lmoe_expert_stack *const (&sh)[2],
+                                  const void *xt, const int32_t *ids_map, int64_t map_stride, const float *row_scale, float *out,
                                   int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
     using C = GmCfg<DT, NPROJ, NT>;
-    if (st0->n_expert > 512) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "grouped GEMM supports at most 512 experts");
-    const int64_t max_tiles = mm_max_tiles(list_rows, st0->n_expert, st0->n_out);
-    int32_t *tiles = static_cast<int32_t *>(tiles_ws);
-    int32_t *n_tiles = reinterpret_cast<int32_t *>(static_cast<uint8_t *>(tiles_ws) + lmoe_align_up((size_t)max_tiles * 32, 256));
-    build_tiles_kernel<<<1, 512, 0, stream>>>(tpe, (int)st0->n_expert, (int)st0->n_out, tiles, n_tiles, (int)max_tiles, MM_M, NT);
-    LMOE_LAUNCH_CHECK("build_tiles_kernel");
     GmParams P;
-    const lmoe_expert_stack *st[2] = {st0, NPROJ == 2 ? st1 : st0};
-    for (int p = 0; p < 2; p++) {
-        P.w[p] = st[p]->blocks();
-        if (DT == LMOE_Q4_K) {
-            lmoe_status mst = make_rows_map(&P.map[p], st[p]->blocks(), (uint64_t)st[p]->row_bytes(),
-                                            (uint64_t)st[p]->n_expert * st[p]->n_out, Q4K_BYTES, MM_M);
-            if (mst) return mst;
-        }
-    }
-    P.rows8 = st0->n_out % 8 == 0;
-    P.vec = st0->n_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
-    if (DT == LMOE_Q6_K && P.rows8) {
-        lmoe_status mst = make_rows_map(&P.map[0], st0->blocks(), 8 * (uint64_t)st0->row_bytes(),
-                                        (uint64_t)st0->n_expert * st0->n_out / 8, GM_Q6_PITCH, MM_M / 8);
+    P.rows8 = st[0]->n_out % 8 == 0;
+    for (int p = 0; p < 2 * NPROJ; p++) {
+        const lmoe_expert_stack *s = p < NPROJ ? st[p] : sh[p - NPROJ];
+        if (!s) continue;
+        CUtensorMap *map = &P.map[2 * (p / NPROJ) + p % NPROJ];
+        lmoe_status mst = LMOE_OK;
+        if (DT == LMOE_Q4_K)
+            mst = make_rows_map(map, s->blocks(), (uint64_t)s->row_bytes(), (uint64_t)s->n_expert * s->n_out, Q4K_BYTES, MM_M);
+        else if (P.rows8)
+            mst = make_rows_map(map, s->blocks(), 8 * (uint64_t)s->row_bytes(), (uint64_t)s->n_expert * s->n_out / 8, GM_Q6_PITCH, MM_M / 8);
         if (mst) return mst;
     }
-    P.expert_bytes = st0->expert_bytes(); P.n_out = (int)st0->n_out; P.k = (int)st0->k;
+    P.w[0] = st[0]->blocks();
+    P.w[1] = sh[0] ? sh[0]->blocks() : nullptr;
+    P.expert_bytes = st[0]->expert_bytes(); P.n_out = (int)st[0]->n_out; P.k = (int)st[0]->k;
+    P.n_expert = R.n_expert; P.m_tiles = mm_m_tiles(st[0]->n_out);
     P.xt = static_cast<const uint8_t *>(xt); P.ids_map = ids_map; P.map_stride = (int)map_stride;
-    P.tiles = tiles; P.n_tiles = n_tiles; P.row_scale = row_scale; P.out = out; P.sorted = sorted; P.flag = flag;
+    P.tiles = static_cast<const int4 *>(tiles_ws); P.n_tiles = mm_tile_count(R, tiles_ws);
+    P.row_scale = row_scale; P.out = out; P.sorted = sorted; P.flag = flag;
+    P.vec = st[0]->n_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
     if (NPROJ == 1 && sorted && P.vec) {
-        lmoe_status mst = make_map_2d(&P.map_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, out, (uint64_t)st0->n_out, (uint64_t)list_rows, 32,
-                                      GM_BOX_ROWS);
+        lmoe_status mst = make_map_2d(&P.map_out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, out, (uint64_t)st[0]->n_out, (uint64_t)(R.rows + R.extra),
+                                      32, GM_BOX_ROWS);
         if (mst) return mst;
     }
     static thread_local int c_dev = -1, c_sms = 0;
@@ -892,24 +885,22 @@ static lmoe_status launch_grouped(const lmoe_expert_stack *st0, const lmoe_exper
     return LMOE_OK;
 }
 
-// One grouped projection. `xt`: the f16 operand in tile order; `tiles_ws`: mm_tiles_bytes() scratch whose last 256 bytes
-// hold the tile count; `flag`: 4 device words (zero = clean).  Rows of `out` by flat id, times row_scale when given, or
-// (`sorted`) unscaled in expert-sorted order.
-lmoe_status launch_mm_id(const lmoe_expert_stack *st, const void *xt, const uint32_t *tpe, const int32_t *ids_map, int64_t map_stride,
-                         int64_t list_rows, const float *row_scale, float *out, int sorted, void *tiles_ws, uint32_t *flag,
-                         cudaStream_t stream) {
-    auto fn = mm_tile_rows(list_rows, st->n_expert) == 128
-                  ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128> : launch_grouped<LMOE_Q6_K, 1, 128>)
-                  : (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 192> : launch_grouped<LMOE_Q6_K, 1, 192>);
-    return fn(st, nullptr, xt, tpe, ids_map, map_stride, list_rows, row_scale, out, sorted, tiles_ws, flag, stream);
+// One grouped projection on the row tiles that launch_gather_tiles made (`xt`: the f16 operand in tile order; `flag`: 4 device
+// words, zero = clean).  Rows of `out` by flat id, times row_scale when given, or (`sorted`) unscaled in expert-sorted order.
+lmoe_status launch_mm_id(const MmRows &R, const lmoe_expert_stack *st, const lmoe_expert_stack *shared, const void *xt,
+                         const int32_t *ids_map, int64_t map_stride, const float *row_scale, float *out, int sorted, void *tiles_ws,
+                         uint32_t *flag, cudaStream_t stream) {
+    auto fn = R.nt == 128 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128> : launch_grouped<LMOE_Q6_K, 1, 128>)
+                          : (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 192> : launch_grouped<LMOE_Q6_K, 1, 192>);
+    return fn(R, {st, nullptr}, {shared, nullptr}, xt, ids_map, map_stride, row_scale, out, sorted, tiles_ws, flag, stream);
 }
 
-// gate and up of one expert block in one kernel, SwiGLU applied: act[rows, ff] (f32).
-lmoe_status launch_mm_gateup(const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const void *xt,
-                             const uint32_t *tpe, const int32_t *ids_map, int64_t map_stride, int64_t list_rows,
-                             float *act, int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
+// gate and up in one kernel, SwiGLU applied: act[rows, ff] (f32), rows by flat id or in expert-sorted order.
+lmoe_status launch_mm_gateup(const MmRows &R, const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *sh_gate,
+                             const lmoe_expert_stack *sh_up, const void *xt, const int32_t *ids_map, int64_t map_stride, float *act,
+                             int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
     if (gate->dtype != LMOE_Q4_K || up->dtype != LMOE_Q4_K)
         return lmoe_fail(LMOE_ERR_UNSUPPORTED, "the fused gate/up kernel is built for Q4_K stacks");
-    auto fn = mm_tile_rows(list_rows, gate->n_expert) == 128 ? launch_grouped<LMOE_Q4_K, 2, 128> : launch_grouped<LMOE_Q4_K, 2, 192>;
-    return fn(gate, up, xt, tpe, ids_map, map_stride, list_rows, nullptr, act, sorted, tiles_ws, flag, stream);
+    auto fn = R.nt == 128 ? launch_grouped<LMOE_Q4_K, 2, 128> : launch_grouped<LMOE_Q4_K, 2, 192>;
+    return fn(R, {gate, up}, {sh_gate, sh_up}, xt, ids_map, map_stride, nullptr, act, sorted, tiles_ws, flag, stream);
 }

@@ -5,20 +5,19 @@
 #include "fused.cuh"
 
 // mm_id.cu
-int64_t mm_max_tiles(int64_t rows, int64_t n_expert, int64_t n_out);
 bool mm_id_kernel_available(int dtype, int64_t n_out, int64_t k);
-size_t mm_tiles_bytes(int64_t rows, int64_t n_expert, int64_t n_out);
-size_t mm_tiled_bytes(int64_t rows, int64_t n_expert, int64_t k);
-cudaError_t launch_gather_tiles(const void *x, int x_f16, int x_per_row, int top_k, int k, const uint32_t *tpe,
-                                const int32_t *ids_map, int map_stride, int n_expert, void *xt, int32_t *pos,
-                                int32_t *spos, int32_t *sfid, int nt, cudaStream_t s);
-int mm_tile_rows(int64_t rows, int64_t n_expert);
-lmoe_status launch_mm_gateup(const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const void *xt,
-                             const uint32_t *tpe, const int32_t *ids_map, int64_t map_stride, int64_t list_rows,
-                             float *act, int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream);
-lmoe_status launch_mm_id(const lmoe_expert_stack *st, const void *xt, const uint32_t *tpe, const int32_t *ids_map,
-                         int64_t map_stride, int64_t list_rows, const float *row_scale, float *out, int sorted,
-                         void *tiles_ws, uint32_t *flag, cudaStream_t stream);
+MmRows mm_rows(int64_t rows, int64_t extra, int64_t n_expert);
+size_t mm_tiles_bytes(const MmRows &R);
+size_t mm_tiled_bytes(const MmRows &R, int64_t k);
+lmoe_status launch_gather_tiles(const MmRows &R, const void *x, int x_f16, int x_per_row, int top_k, int k, const uint32_t *tpe,
+                                const int32_t *ids_map, int64_t map_stride, void *tiles_ws, void *xt, int32_t *pos, int32_t *spos,
+                                int32_t *sfid, cudaStream_t s);
+lmoe_status launch_mm_gateup(const MmRows &R, const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *sh_gate,
+                             const lmoe_expert_stack *sh_up, const void *xt, const int32_t *ids_map, int64_t map_stride, float *act,
+                             int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream);
+lmoe_status launch_mm_id(const MmRows &R, const lmoe_expert_stack *st, const lmoe_expert_stack *shared, const void *xt,
+                         const int32_t *ids_map, int64_t map_stride, const float *row_scale, float *out, int sorted, void *tiles_ws,
+                         uint32_t *flag, cudaStream_t stream);
 
 namespace {
 
@@ -71,10 +70,11 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const float *__restric
 }
 
 // Same range guard for an activation that is already silu(g)*u (f32): l2, rescale, f16, tile order.
-// With `sfid` the rows of `a` (and of `scale`) are in expert-sorted order and sfid[row] is the flat id.
+// With `sfid` the rows of `a` (and of `scale`) are in expert-sorted order and sfid[row] is the flat id; ids from `routed` on
+// are the shared expert's rows, which carry no routing weight.
 __global__ void __launch_bounds__(256) rescale_rows_kernel(const float *__restrict__ a, const float *__restrict__ w,
                                                            const int32_t *__restrict__ pos, const int32_t *__restrict__ sfid,
-                                                           int64_t rows, int ff, int nt, uint8_t *__restrict__ act,
+                                                           int64_t rows, int64_t routed, int ff, int nt, uint8_t *__restrict__ act,
                                                            float *__restrict__ scale) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -101,12 +101,12 @@ __global__ void __launch_bounds__(256) rescale_rows_kernel(const float *__restri
                            ((size_t)((ci & 7) ^ (p & 7)) << 4);
         *reinterpret_cast<uint4 *>(act + off) = *reinterpret_cast<const uint4 *>(h);
     }
-    if (lane == 0) scale[row] = l2 * 0x1p-15f * (w ? w[fid] : 1.0f);
+    if (lane == 0) scale[row] = l2 * 0x1p-15f * (w && fid < routed ? w[fid] : 1.0f);
 }
 
-// out[t, c] = sum over slots (in slot order) of y[t, s, c], then + shared[t, c].
-__global__ void sum_slots_kernel(const float *__restrict__ y, const float *__restrict__ shared, int64_t t, int top_k,
-                                 int n4, float *__restrict__ out) {
+// out[t, c] = sum over slots (in slot order) of y[t, s, c], then + shared[t, c], then + residual[t, c].
+__global__ void sum_slots_kernel(const float *__restrict__ y, const float *__restrict__ shared,
+                                 const float *__restrict__ residual, int64_t t, int top_k, int n4, float *__restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= t * n4) return;
     const int64_t tok = i / n4, c = i - tok * n4;
@@ -120,33 +120,51 @@ __global__ void sum_slots_kernel(const float *__restrict__ y, const float *__res
         const float4 v = reinterpret_cast<const float4 *>(shared)[i];
         s.x = __fadd_rn(s.x, v.x); s.y = __fadd_rn(s.y, v.y); s.z = __fadd_rn(s.z, v.z); s.w = __fadd_rn(s.w, v.w);
     }
+    if (residual) {
+        const float4 v = reinterpret_cast<const float4 *>(residual)[i];
+        s.x = __fadd_rn(s.x, v.x); s.y = __fadd_rn(s.y, v.y); s.z = __fadd_rn(s.z, v.z); s.w = __fadd_rn(s.w, v.w);
+    }
     reinterpret_cast<float4 *>(out)[i] = s;
 }
 
 // Same sum when the partial rows are unscaled and in expert-sorted order: row spos[flat id] of `y`
-// times scale[that row]; likewise for the shared expert's rows.  A negative position marks an empty slot.
-__global__ void sum_sorted_kernel(const float *__restrict__ y, const float *__restrict__ scale,
+// times scale[that row]; likewise for the shared expert's rows, then + residual.  A negative position marks an empty slot.
+// Twelve rows' loads are in flight per element: the sum is one pass over y at the memory's rate.
+__global__ void __launch_bounds__(256) sum_sorted_kernel(const float *__restrict__ y, const float *__restrict__ scale,
                                   const int32_t *__restrict__ spos, const float *__restrict__ shared,
-                                  const float *__restrict__ sh_scale, const int32_t *__restrict__ sh_spos, int64_t t,
-                                  int top_k, int n4, float *__restrict__ out) {
+                                  const float *__restrict__ sh_scale, const int32_t *__restrict__ sh_spos,
+                                  const float *__restrict__ residual, int64_t t, int top_k, int n4, float *__restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= t * n4) return;
     const int64_t tok = i / n4, c = i - tok * n4;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = 0; k < top_k; k++) {
-        const int64_t r = spos[tok * top_k + k];
-        if (r < 0) continue;                               // empty slot
-        const float sc = scale ? scale[r] : 1.0f;
-        const float4 v = reinterpret_cast<const float4 *>(y)[r * n4 + c];
-        s.x = __fadd_rn(s.x, __fmul_rn(v.x, sc)); s.y = __fadd_rn(s.y, __fmul_rn(v.y, sc));
-        s.z = __fadd_rn(s.z, __fmul_rn(v.z, sc)); s.w = __fadd_rn(s.w, __fmul_rn(v.w, sc));
+    const int32_t *sp = spos + tok * top_k;
+    const int n = top_k + (shared ? 1 : 0);
+    for (int k0 = 0; k0 < n; k0 += 12) {
+        float4 v[12];
+        float sc[12];
+        uint32_t present = 0u;
+#pragma unroll
+        for (int j = 0; j < 12; j++) {
+            const int k = k0 + j;
+            const bool sh = k == top_k;
+            const int64_t r = k >= n ? -1 : (sh ? (sh_spos ? sh_spos[tok] : tok) : sp[k]);
+            const float *base = sh ? shared : y, *sb = sh ? sh_scale : scale;
+            sc[j] = r >= 0 && sb ? sb[r] : 1.0f;
+            v[j] = r >= 0 ? __ldcs(reinterpret_cast<const float4 *>(base) + r * n4 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            present |= (uint32_t)(r >= 0) << j;
+        }
+#pragma unroll
+        for (int j = 0; j < 12; j++) {
+            if (present & (1u << j)) {
+                s.x = __fadd_rn(s.x, __fmul_rn(v[j].x, sc[j])); s.y = __fadd_rn(s.y, __fmul_rn(v[j].y, sc[j]));
+                s.z = __fadd_rn(s.z, __fmul_rn(v[j].z, sc[j])); s.w = __fadd_rn(s.w, __fmul_rn(v[j].w, sc[j]));
+            }
+        }
     }
-    if (shared) {
-        const int64_t r = sh_spos ? sh_spos[tok] : tok;
-        const float sc = sh_scale ? sh_scale[r] : 1.0f;
-        const float4 v = reinterpret_cast<const float4 *>(shared)[r * n4 + c];
-        s.x = __fadd_rn(s.x, __fmul_rn(v.x, sc)); s.y = __fadd_rn(s.y, __fmul_rn(v.y, sc));
-        s.z = __fadd_rn(s.z, __fmul_rn(v.z, sc)); s.w = __fadd_rn(s.w, __fmul_rn(v.w, sc));
+    if (residual) {
+        const float4 v = reinterpret_cast<const float4 *>(residual)[i];
+        s.x = __fadd_rn(s.x, v.x); s.y = __fadd_rn(s.y, v.y); s.z = __fadd_rn(s.z, v.z); s.w = __fadd_rn(s.w, v.w);
     }
     reinterpret_cast<float4 *>(out)[i] = s;
 }
@@ -221,65 +239,66 @@ struct Carver {
     }
 };
 
-// Scratch of one grouped SwiGLU FFN over `rows` routed rows.
-size_t ffn_bytes(int64_t rows, int64_t hidden, int64_t ff, int64_t n_expert) {
+// Scratch of one grouped SwiGLU FFN.
+size_t ffn_bytes(const MmRows &R, int64_t hidden, int64_t ff) {
+    const size_t all = (size_t)(R.rows + R.extra);
     size_t o = 0;
-    o += mm_tiled_bytes(rows, n_expert, hidden);             // x in tile order
-    o += lmoe_align_up((size_t)rows * 4, 256);               // position of every flat id
-    o += 2 * lmoe_align_up((size_t)rows * ff * 4, 256);      // gate, up
-    o += mm_tiled_bytes(rows, n_expert, ff);                 // f16 activation in tile order
-    o += lmoe_align_up((size_t)rows * 4, 256);               // row scale
-    o += lmoe_align_up((size_t)rows * 4, 256);               // flat id of every sorted row
-    const size_t t1 = mm_tiles_bytes(rows, n_expert, ff), t2 = mm_tiles_bytes(rows, n_expert, hidden);
-    o += t1 > t2 ? t1 : t2;
+    o += mm_tiled_bytes(R, hidden);                          // x in tile order
+    o += lmoe_align_up(all * 4, 256);                        // position of every flat id
+    o += 2 * lmoe_align_up(all * ff * 4, 256);               // gate, up
+    o += mm_tiled_bytes(R, ff);                              // f16 activation in tile order
+    o += lmoe_align_up(all * 4, 256);                        // row scale
+    o += lmoe_align_up(all * 4, 256);                        // flat id of every sorted row
+    o += mm_tiles_bytes(R);
     return o;
 }
 
 // y[rows, hidden] = row_weight * FFN_{expert of row}(x[row / top_k]); lists as produced by map0.
-// With `spos` / `scale_out` (both [rows], caller-owned) and the fused kernels available, y instead holds the
+// With `spos` / `scale_out` (both [rows + extra], caller-owned) and Q4_K gate/up stacks, y instead holds the
 // UNSCALED rows in expert-sorted order: row spos[flat id], to be multiplied by scale_out[that row]; the
-// tensor-core epilogues then store whole tile columns side by side instead of scattering by flat id.
-// *sorted_used tells which form was produced.  `masked`: ids >= n_expert were left out of the lists.
-lmoe_status ffn_grouped(const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *down,
-                        const void *x, int top_k, int64_t t, const uint32_t *tpe, const int32_t *ids_map,
-                        int64_t map_stride, const float *row_w, float *y, uint8_t *ws, uint32_t *flag,
-                        cudaStream_t s, int32_t *spos = nullptr, float *scale_out = nullptr, bool *sorted_used = nullptr,
-                        int x_f16 = 0, int masked = 0) {
-    const int64_t rows = t * top_k, ff = gate->n_out, hidden = gate->k, ne = gate->n_expert;
+// tensor-core epilogues then store whole tile columns side by side instead of scattering by flat id.  Only in that form
+// can R.extra rows of the shared expert (`sh`: its gate, up, down) ride along: one launch of each kernel serves both.
+// `masked`: ids >= n_expert were left out of the lists.
+bool ffn_sorts(const lmoe_expert_stack *gate, const lmoe_expert_stack *up) { return gate->dtype == LMOE_Q4_K && up->dtype == LMOE_Q4_K; }
+
+lmoe_status ffn_grouped(const MmRows &R, const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *down,
+                        const lmoe_expert_stack *const (&sh)[3], const void *x, int top_k, const uint32_t *tpe, const int32_t *ids_map,
+                        int64_t map_stride, const float *row_w, float *y, uint8_t *ws, uint32_t *flag, cudaStream_t s,
+                        int32_t *spos = nullptr, float *scale_out = nullptr, int x_f16 = 0, int masked = 0) {
+    const int64_t all = R.rows + R.extra, ff = gate->n_out, hidden = gate->k;
     Carver c{ws, 0};
-    uint8_t *xt = c.take<uint8_t>(mm_tiled_bytes(rows, ne, hidden));
-    int32_t *pos = c.take<int32_t>((size_t)rows);
-    float *g = c.take<float>((size_t)rows * ff), *u = c.take<float>((size_t)rows * ff);
-    uint8_t *act = c.take<uint8_t>(mm_tiled_bytes(rows, ne, ff));
-    float *rs = c.take<float>((size_t)rows);
-    int32_t *sfid = c.take<int32_t>((size_t)rows);
+    uint8_t *xt = c.take<uint8_t>(mm_tiled_bytes(R, hidden));
+    int32_t *pos = c.take<int32_t>((size_t)all);
+    float *g = c.take<float>((size_t)all * ff), *u = c.take<float>((size_t)all * ff);
+    uint8_t *act = c.take<uint8_t>(mm_tiled_bytes(R, ff));
+    float *rs = c.take<float>((size_t)all);
+    int32_t *sfid = c.take<int32_t>((size_t)all);
     void *tiles = ws + c.off;
-    const int nt = mm_tile_rows(rows, ne);
     lmoe_status st;
-    const bool fused_gu = gate->dtype == LMOE_Q4_K && up->dtype == LMOE_Q4_K;
-    const bool sorted = spos && scale_out && fused_gu;
-    if (sorted_used) *sorted_used = sorted;
+    const bool fused_gu = ffn_sorts(gate, up), sorted = spos && scale_out && fused_gu;
     if (masked) {
         // some (token, slot) pairs name no expert: the lists skip them, and the per-row arrays mark them
         if (!sorted) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "masked slots need the fused Q4_K gate/up kernel");
-        LMOE_CUDA(cudaMemsetAsync(spos, 0xFF, (size_t)rows * 4, s));
-        LMOE_CUDA(cudaMemsetAsync(sfid, 0xFF, (size_t)rows * 4, s));
+        LMOE_CUDA(cudaMemsetAsync(spos, 0xFF, (size_t)all * 4, s));
+        LMOE_CUDA(cudaMemsetAsync(sfid, 0xFF, (size_t)all * 4, s));
     }
-    LMOE_CUDA(launch_gather_tiles(x, x_f16, 1, top_k, (int)hidden, tpe, ids_map, (int)map_stride, (int)ne, xt, pos,
-                                  sorted ? spos : nullptr, sorted ? sfid : nullptr, nt, s));
+    if ((st = launch_gather_tiles(R, x, x_f16, 1, top_k, (int)hidden, tpe, ids_map, map_stride, tiles, xt, pos, sorted ? spos : nullptr,
+                                  sorted ? sfid : nullptr, s)))
+        return st;
+    const unsigned row_blocks = (unsigned)((all + 7) / 8);
     if (fused_gu) {
         // both projections in one pass over the activations, SwiGLU in the epilogue
-        if ((st = launch_mm_gateup(gate, up, xt, tpe, ids_map, map_stride, rows, g, sorted, tiles, flag, s))) return st;
-        rescale_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(g, row_w, pos, sorted ? sfid : nullptr, rows, (int)ff, nt,
-                                                                       act, sorted ? scale_out : rs);
+        if ((st = launch_mm_gateup(R, gate, up, sh[0], sh[1], xt, ids_map, map_stride, g, sorted, tiles, flag, s))) return st;
+        rescale_rows_kernel<<<row_blocks, 256, 0, s>>>(g, row_w, pos, sorted ? sfid : nullptr, all, R.rows, (int)ff, R.nt, act,
+                                                       sorted ? scale_out : rs);
         LMOE_LAUNCH_CHECK("rescale_rows_kernel");
     } else {
-        if ((st = launch_mm_id(gate, xt, tpe, ids_map, map_stride, rows, nullptr, g, 0, tiles, flag, s))) return st;
-        if ((st = launch_mm_id(up, xt, tpe, ids_map, map_stride, rows, nullptr, u, 0, tiles, flag, s))) return st;
-        swiglu_rows_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(g, u, row_w, pos, rows, (int)ff, nt, act, rs);
+        if ((st = launch_mm_id(R, gate, nullptr, xt, ids_map, map_stride, nullptr, g, 0, tiles, flag, s))) return st;
+        if ((st = launch_mm_id(R, up, nullptr, xt, ids_map, map_stride, nullptr, u, 0, tiles, flag, s))) return st;
+        swiglu_rows_kernel<<<row_blocks, 256, 0, s>>>(g, u, row_w, pos, all, (int)ff, R.nt, act, rs);
         LMOE_LAUNCH_CHECK("swiglu_rows_kernel");
     }
-    return launch_mm_id(down, act, tpe, ids_map, map_stride, rows, sorted ? nullptr : rs, y, sorted, tiles, flag, s);
+    return launch_mm_id(R, down, sh[2], act, ids_map, map_stride, sorted ? nullptr : rs, y, sorted, tiles, flag, s);
 }
 
 bool layer_mm_ok(const lmoe_layer *L) {
@@ -291,61 +310,59 @@ bool layer_mm_ok(const lmoe_layer *L) {
 } // namespace
 
 // Scratch of the routed (+ shared) experts of `t` tokens with `top_k` slots each, after the routing decision.
+static MmRows experts_rows(const lmoe_layer *L, int64_t t, int64_t top_k, int add_shared) {
+    return mm_rows(t * top_k, add_shared && L->sh_gate && ffn_sorts(L->gate, L->up) ? t : 0, L->n_expert);
+}
 static size_t experts_ws_bytes(const lmoe_layer *L, int64_t t, int64_t top_k) {
-    const int64_t rows = t * top_k;
+    const MmRows R = experts_rows(L, t, top_k, 1);
+    const size_t all = (size_t)(t * (top_k + 1));
     size_t o = 0;
     o += lmoe_map0_scratch_bytes(L->n_expert, t);
-    o += lmoe_align_up((size_t)rows * L->hidden * 4, 256);           // routed partial rows
-    o += lmoe_align_up((size_t)t * L->hidden * 4, 256);              // shared expert rows
+    o += lmoe_align_up(all * L->hidden * 4, 256);                    // partial rows
     o += lmoe_align_up((size_t)(t + 64) * 4, 256);                   // identity list
-    o += 2 * lmoe_align_up((size_t)rows * 4, 256);                   // sorted position and scale of every routed row
-    o += 2 * lmoe_align_up((size_t)t * 4, 256);                      // the same for the shared expert's rows
-    o += ffn_bytes(rows, L->hidden, L->expert_ff, L->n_expert);
+    o += 2 * lmoe_align_up(all * 4, 256);                            // sorted position and scale of every row
+    const size_t a = ffn_bytes(R, L->hidden, L->expert_ff), b = ffn_bytes(mm_rows(t, 0, 1), L->hidden, L->expert_ff);
+    o += a > b ? a : b;
     return o;
 }
 
 // The experts of a block on a routing decision that is already on the device: per-expert row lists, grouped
-// GEMMs, slot-order sum, optionally the shared expert.  x: [t, hidden] f32 or f16; ids / w: [t, top_k]
+// GEMMs, slot-order sum, optionally the shared expert and a residual.  x: [t, hidden] f32 or f16; ids / w: [t, top_k]
 // (`masked`: ids >= n_expert are empty slots).  `ws` holds experts_ws_bytes(); `flag` is the device flag.
 static lmoe_status experts_prefill(const lmoe_layer *L, const void *x, int x_f16, const uint32_t *ids, const float *w,
-                                   int64_t t, int64_t top_k, int masked, int add_shared, float *out, uint8_t *ws,
-                                   uint32_t *flag, cudaStream_t s) {
+                                   int64_t t, int64_t top_k, int masked, int add_shared, const float *residual, float *out,
+                                   uint8_t *ws, uint32_t *flag, cudaStream_t s) {
     const int64_t rows = t * top_k, H = L->hidden;
+    const MmRows R = experts_rows(L, t, top_k, add_shared);
     Carver c{ws, 0};
     uint8_t *map0 = c.take<uint8_t>(lmoe_map0_scratch_bytes(L->n_expert, t));
-    float *y = c.take<float>((size_t)rows * H);
-    float *ysh = c.take<float>((size_t)t * H);
+    float *y = c.take<float>((size_t)(rows + t) * H);
     uint32_t *sh_list = c.take<uint32_t>((size_t)t + 64);
-    int32_t *spos = c.take<int32_t>((size_t)rows);
-    float *rscale = c.take<float>((size_t)rows);
-    int32_t *sh_spos = c.take<int32_t>((size_t)t);
-    float *sh_scale = c.take<float>((size_t)t);
+    int32_t *spos = c.take<int32_t>((size_t)(rows + t));
+    float *rscale = c.take<float>((size_t)(rows + t));
     uint8_t *ffn_ws = ws + c.off;
     uint32_t *tpe = reinterpret_cast<uint32_t *>(map0);
     int32_t *ids_map = reinterpret_cast<int32_t *>(map0 + L->n_expert * 4);
     // ids >= n_expert match no expert's list: those slots stay empty
     LMOE_CUDA(launch_map0(ids, (int)t, (int)top_k, (int)L->n_expert, tpe, ids_map, s));
-    bool sorted = false, sh_sorted = false;
-    lmoe_status st = ffn_grouped(L->gate, L->up, L->down, x, (int)top_k, t, tpe, ids_map, t, w, y, ffn_ws, flag, s, spos,
-                                 rscale, &sorted, x_f16, masked);
+    const bool sorted = ffn_sorts(L->gate, L->up), shared = add_shared && L->sh_gate;
+    lmoe_status st = ffn_grouped(R, L->gate, L->up, L->down, {R.extra ? L->sh_gate : nullptr, R.extra ? L->sh_up : nullptr, R.extra ? L->sh_down : nullptr},
+                                 x, (int)top_k, tpe, ids_map, t, w, y, ffn_ws, flag, s, spos, rscale, x_f16, masked);
     if (st) return st;
-    const float *shared = nullptr;
-    if (add_shared && L->sh_gate) {
+    float *ysh = y + (size_t)rows * H;
+    if (shared && !R.extra) {
         iota_list_kernel<<<(unsigned)((t + 255) / 256), 256, 0, s>>>(t, sh_list, reinterpret_cast<int32_t *>(sh_list + 64));
         LMOE_LAUNCH_CHECK("iota_list_kernel");
-        // the shared expert's rows take the same form as the routed ones, so one kernel sums both
-        st = ffn_grouped(L->sh_gate, L->sh_up, L->sh_down, x, 1, t, sh_list, reinterpret_cast<int32_t *>(sh_list + 64), t,
-                         nullptr, ysh, ffn_ws, flag, s, sorted ? sh_spos : nullptr, sorted ? sh_scale : nullptr, &sh_sorted,
-                         x_f16);
+        st = ffn_grouped(mm_rows(t, 0, 1), L->sh_gate, L->sh_up, L->sh_down, {nullptr, nullptr, nullptr}, x, 1, sh_list,
+                         reinterpret_cast<int32_t *>(sh_list + 64), t, nullptr, ysh, ffn_ws, flag, s, nullptr, nullptr, x_f16);
         if (st) return st;
-        shared = ysh;
     }
     const int64_t n = t * (H / 4);
-    if (sorted && (!shared || sh_sorted))
-        sum_sorted_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(y, rscale, spos, shared, sh_scale, sh_spos, t,
+    if (sorted)
+        sum_sorted_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(y, rscale, spos, shared ? y : nullptr, rscale, spos + rows, residual, t,
                                                                       (int)top_k, (int)(H / 4), out);
     else
-        sum_slots_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(y, shared, t, (int)top_k, (int)(H / 4), out);
+        sum_slots_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(y, shared ? ysh : nullptr, residual, t, (int)top_k, (int)(H / 4), out);
     LMOE_LAUNCH_CHECK("sum_slots_kernel");
     return LMOE_OK;
 }
@@ -360,7 +377,7 @@ size_t prefill_workspace_bytes(const lmoe_layer *L, int64_t t) {
     return o;
 }
 
-lmoe_status launch_moe_prefill(const lmoe_layer *L, const float *x, int64_t t, float *out, uint32_t *ids_out,
+lmoe_status launch_moe_prefill(const lmoe_layer *L, const float *x, const float *residual, int64_t t, float *out, uint32_t *ids_out,
                                float *w_out, void *workspace, size_t workspace_bytes, cudaStream_t s) {
     if (!layer_mm_ok(L)) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "no grouped-GEMM kernel for this layer's shapes / dtypes");
     if (!workspace || workspace_bytes < prefill_workspace_bytes(L, t))
@@ -378,7 +395,7 @@ lmoe_status launch_moe_prefill(const lmoe_layer *L, const float *x, int64_t t, f
     LMOE_CUDA(cudaMemsetAsync(flag, 0, 16, s)); // a fresh device flag: the workspace needs no initialisation
     LMOE_CUDA(launch_route_logits(L->router, x, (int)t, (int)H, (int)L->n_expert, logits, s));
     LMOE_CUDA(launch_route_select(logits, L->bias, (int)t, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, ids, w, s));
-    lmoe_status st = experts_prefill(L, x, 0, ids, w, t, L->top_k, 0, 1, out, ex_ws, flag, s);
+    lmoe_status st = experts_prefill(L, x, 0, ids, w, t, L->top_k, 0, 1, residual, out, ex_ws, flag, s);
     if (st) return st;
     if (ids_out) LMOE_CUDA(cudaMemcpyAsync(ids_out, ids, (size_t)rows * 4, cudaMemcpyDeviceToDevice, s));
     if (w_out) LMOE_CUDA(cudaMemcpyAsync(w_out, w, (size_t)rows * 4, cudaMemcpyDeviceToDevice, s));
@@ -398,7 +415,7 @@ lmoe_status launch_experts_prefill(const lmoe_layer *L, const float *x, const ui
     if (t * L->top_k > INT32_MAX / 2) return lmoe_fail(LMOE_ERR_INVALID, "too many routed rows");
     uint32_t *flag = reinterpret_cast<uint32_t *>(workspace);
     LMOE_CUDA(cudaMemsetAsync(flag, 0, 16, s));
-    return experts_prefill(L, x, 0, ids, w, t, L->top_k, 1, add_shared, out, static_cast<uint8_t *>(workspace) + 65536, flag, s);
+    return experts_prefill(L, x, 0, ids, w, t, L->top_k, 1, add_shared, nullptr, out, static_cast<uint8_t *>(workspace) + 65536, flag, s);
 }
 
 // ---- op-level entry points ------------------------------------------------------------
@@ -408,8 +425,8 @@ extern "C" int32_t lmoe_mm_id_supported(int32_t dtype, int64_t top_k) {
 
 extern "C" size_t lmoe_mm_id_workspace_bytes(const lmoe_expert_stack *stack, int64_t t, int64_t top_k, int64_t x_per_row) {
     if (!stack || t < 0 || top_k < 1 || x_per_row < 1) return 0;
-    return 256 + mm_tiled_bytes(t * top_k, stack->n_expert, stack->k) +
-           mm_tiles_bytes(t * top_k, stack->n_expert, stack->n_out);
+    const MmRows R = mm_rows(t * top_k, 0, stack->n_expert);
+    return 256 + mm_tiled_bytes(R, stack->k) + mm_tiles_bytes(R);
 }
 
 static lmoe_status mm_id_run(const lmoe_expert_stack *stack, const float *x, int64_t t, int64_t x_per_row, int64_t k,
@@ -427,13 +444,14 @@ static lmoe_status mm_id_run(const lmoe_expert_stack *stack, const float *x, int
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     uint32_t *flag = reinterpret_cast<uint32_t *>(ws);
     uint8_t *xt = ws + 256;
-    void *tiles = ws + 256 + mm_tiled_bytes(t * top_k, stack->n_expert, k);
+    const MmRows R = mm_rows(t * top_k, 0, stack->n_expert);
+    void *tiles = ws + 256 + mm_tiled_bytes(R, k);
     LMOE_CUDA(cudaMemsetAsync(flag, 0, 16, s));
     const uint32_t *tpe = static_cast<const uint32_t *>(map0);
     const int32_t *ids_map = reinterpret_cast<const int32_t *>(static_cast<const uint8_t *>(map0) + stack->n_expert * 4);
-    LMOE_CUDA(launch_gather_tiles(x, 0, (int)x_per_row, (int)top_k, (int)k, tpe, ids_map, (int)t, (int)stack->n_expert, xt,
-                                  nullptr, nullptr, nullptr, mm_tile_rows(t * top_k, stack->n_expert), s));
-    return launch_mm_id(stack, xt, tpe, ids_map, t, t * top_k, nullptr, out, 0, tiles, flag, s);
+    if ((st = launch_gather_tiles(R, x, 0, (int)x_per_row, (int)top_k, (int)k, tpe, ids_map, t, tiles, xt, nullptr, nullptr, nullptr, s)))
+        return st;
+    return launch_mm_id(R, stack, nullptr, xt, ids_map, t, nullptr, out, 0, tiles, flag, s);
 }
 
 extern "C" lmoe_status lmoe_mul_mm_id_shared(const lmoe_expert_stack *stack, const float *x, int64_t t, int64_t x_per_row,
@@ -472,9 +490,14 @@ extern "C" lmoe_status lmoe_mul_mm_id(const lmoe_expert_stack *stack, const floa
 }
 
 // ---- expert-parallel pieces -------------------------------------------------------------
+// (the same entries serve the shared expert alone, whose single list may take another tile size)
+static size_t rows_ffn_bytes(const lmoe_layer *L, int64_t rows) {
+    const size_t a = ffn_bytes(mm_rows(rows, 0, L->n_expert), L->hidden, L->expert_ff), b = ffn_bytes(mm_rows(rows, 0, 1), L->hidden, L->expert_ff);
+    return a > b ? a : b;
+}
 static size_t rows_ws_bytes(const lmoe_layer *L, int64_t rows) {
     return 65536 + lmoe_map0_scratch_bytes(L->n_expert, rows) + lmoe_align_up((size_t)(rows + 64) * 4, 256) +
-           ffn_bytes(rows, L->hidden, L->expert_ff, L->n_expert);
+           rows_ffn_bytes(L, rows);
 }
 
 static lmoe_status experts_rows_run(const lmoe_layer *L, const void *x, int x_f16, const uint32_t *local_ids,
@@ -497,8 +520,8 @@ static lmoe_status experts_rows_run(const lmoe_layer *L, const void *x, int x_f1
     int32_t *ids_map = reinterpret_cast<int32_t *>(map0 + L->n_expert * 4);
     LMOE_CUDA(cudaMemsetAsync(flag, 0, 16, s));
     LMOE_CUDA(launch_map0(local_ids, (int)rows, 1, (int)L->n_expert, tpe, ids_map, s));
-    return ffn_grouped(L->gate, L->up, L->down, x, 1, rows, tpe, ids_map, rows, row_weights, out, ffn_ws, flag, s, nullptr,
-                       nullptr, nullptr, x_f16);
+    return ffn_grouped(mm_rows(rows, 0, L->n_expert), L->gate, L->up, L->down, {nullptr, nullptr, nullptr}, x, 1, tpe, ids_map, rows,
+                       row_weights, out, ffn_ws, flag, s, nullptr, nullptr, x_f16);
 }
 
 extern "C" lmoe_status lmoe_experts_forward_rows(const lmoe_layer *L, const float *x, const uint32_t *local_ids,
@@ -537,7 +560,7 @@ extern "C" lmoe_status lmoe_experts_forward_tokens_f16(const lmoe_layer *L, cons
     cudaStream_t s = (cudaStream_t)stream;
     uint32_t *flag = reinterpret_cast<uint32_t *>(workspace);
     LMOE_CUDA(cudaMemsetAsync(flag, 0, 16, s));
-    return experts_prefill(L, x_f16, 1, ids, weights, t, top_k, 1, 0, out, static_cast<uint8_t *>(workspace) + 65536, flag, s);
+    return experts_prefill(L, x_f16, 1, ids, weights, t, top_k, 1, 0, nullptr, out, static_cast<uint8_t *>(workspace) + 65536, flag, s);
 }
 
 extern "C" lmoe_status lmoe_shared_forward(const lmoe_layer *L, const float *x, int64_t t, float *out, void *workspace,
@@ -558,8 +581,8 @@ extern "C" lmoe_status lmoe_shared_forward(const lmoe_layer *L, const float *x, 
     LMOE_CUDA(cudaMemsetAsync(flag, 0, 16, s));
     iota_list_kernel<<<(unsigned)((t + 255) / 256), 256, 0, s>>>(t, list, reinterpret_cast<int32_t *>(list + 64));
     LMOE_LAUNCH_CHECK("iota_list_kernel");
-    return ffn_grouped(L->sh_gate, L->sh_up, L->sh_down, x, 1, t, list, reinterpret_cast<int32_t *>(list + 64), t, nullptr,
-                       out, ffn_ws, flag, s);
+    return ffn_grouped(mm_rows(t, 0, 1), L->sh_gate, L->sh_up, L->sh_down, {nullptr, nullptr, nullptr}, x, 1, list,
+                       reinterpret_cast<int32_t *>(list + 64), t, nullptr, out, ffn_ws, flag, s);
 }
 
 extern "C" size_t lmoe_rows_workspace_bytes(const lmoe_layer *L, int64_t rows) {
@@ -619,7 +642,7 @@ extern "C" lmoe_status lmoe_ep_combine(const float *rows, const int32_t *row_pos
         return lmoe_fail(LMOE_ERR_INVALID, "ep_combine: rows, shared and out must be 16-byte aligned");
     if (t == 0) return LMOE_OK;
     const int64_t n = t * (hidden / 4);
-    sum_sorted_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(rows, nullptr, row_pos, shared, nullptr, nullptr,
+    sum_sorted_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(rows, nullptr, row_pos, shared, nullptr, nullptr, nullptr,
                                                                                t, (int)top_k, (int)(hidden / 4), out);
     LMOE_LAUNCH_CHECK("sum_sorted_kernel");
     return LMOE_OK;
