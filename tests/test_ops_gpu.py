@@ -100,6 +100,30 @@ def test_mv_shape_mismatch_errors(orc, dev):
 
 
 @pytest.mark.parametrize("dt,name", DTYPES)
+@pytest.mark.parametrize("n_expert,n_out,k,t,top_k,xpr", [
+    (1, 64, 256, 3, 1, 1), (1, 65, 512, 4, 1, 1), (1, 63, 1280, 33, 1, 1), (1, 130, 3072, 5, 13, 13),  # one matrix: 3 / 4 / 33 / 65 pairs
+    (3, 127, 768, 2, 3, 3), (2, 16, 8192 + 256, 1, 2, 1)])                                            # odd block counts, two staged chunks
+def test_mv_tile_edges(orc, dev, dt, name, n_expert, n_out, k, t, top_k, xpr):
+    """Row, pair and K edges of the two mat-vec kernels, an empty slot and an outlier channel.  Bound: activations and sums
+    carry at least 22 bits per 256-wide block and the oracle's own f32 sums err by about sqrt(k) * 2^-24 (5e-6 at 8448)."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    raw = orc.quantize(dt, orc.pseudo_random(n_expert * n_out * k, 0x900 + k, -1.0, 1.0))
+    stack = ExpertStack.from_bytes(raw, dt, n_expert, n_out, k, device=dev)
+    x = orc.pseudo_random(t * xpr * k, 0x33, -1.0, 1.0).reshape(t, xpr, k)
+    x[0, 0, 7] = 50.0
+    ids = (np.arange(t * top_k, dtype=np.uint32) % n_expert).reshape(t, top_k)
+    got = ops.mul_mv_id(stack, torch.from_numpy(x).to(dev), torch.from_numpy(ids.astype(np.int32)).to(dev)).cpu().numpy()
+    assert orc.rel_l2(got, orc.mul_id(dt, raw, n_expert, n_out, k, x, ids)) < 1e-5
+    ids[t - 1, top_k - 1] = n_expert
+    hole = ops.mul_mv_id(stack, torch.from_numpy(x).to(dev), torch.from_numpy(ids.astype(np.int32)).to(dev)).cpu().numpy()
+    assert not hole[t - 1, top_k - 1].any()
+    hole[t - 1, top_k - 1] = got[t - 1, top_k - 1]
+    assert np.array_equal(hole, got)
+
+
+@pytest.mark.parametrize("dt,name", DTYPES)
 def test_plain_mv(orc, dev, dt, name):
     from maxuna_b200 import ops
 
