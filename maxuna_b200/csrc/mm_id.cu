@@ -230,6 +230,46 @@ __global__ void __launch_bounds__(256) gather_tiles_kernel(const void *__restric
     }
 }
 
+// The gate/up product takes its activation rows straight from token order: x once as f16 [tokens][k] (8-value chunks as
+// [0 2 1 3 4 6 5 7]), and src[slot * nt + rr] = row of it that tile row (slot, rr) multiplies.  The kernel's loaders fetch the
+// rows of every 64-k block with 16-byte asynchronous copies; a row of a token that ten experts share stays in L2 instead of
+// being written out and read back ten times.  Blocks [0, convert_blocks) convert x, the others take a row tile each.
+template <bool XF16>
+__global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict__ xv, int64_t x_chunks, int convert_blocks, int top_k,
+                                                         const int4 *__restrict__ tiles, const int32_t *__restrict__ n_tiles,
+                                                         const int32_t *__restrict__ ids_map, int map_stride, int n_expert,
+                                                         int routed_rows, int nt, uint8_t *__restrict__ xh, int32_t *__restrict__ src,
+                                                         int32_t *__restrict__ pos, int32_t *__restrict__ spos, int32_t *__restrict__ sfid) {
+    if ((int)blockIdx.x < convert_blocks) {
+        const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+        if (i >= x_chunks) return;
+        uint4 o;
+        if (XF16) {
+            // rows already in f16 (the expert-parallel wire format): only the order inside the chunk changes
+            const uint4 v = __ldg(static_cast<const uint4 *>(xv) + i);
+            o = make_uint4(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x5410),
+                           __byte_perm(v.z, v.w, 0x7632));
+        } else {
+            const float4 a = __ldg(static_cast<const float4 *>(xv) + 2 * i), b = __ldg(static_cast<const float4 *>(xv) + 2 * i + 1);
+            __align__(16) __half2 h[4] = {__floats2half2_rn(a.x, a.z), __floats2half2_rn(a.y, a.w), __floats2half2_rn(b.x, b.z),
+                                          __floats2half2_rn(b.y, b.w)};
+            o = *reinterpret_cast<const uint4 *>(h);
+        }
+        reinterpret_cast<uint4 *>(xh)[i] = o;
+        return;
+    }
+    const int slot = blockIdx.x - convert_blocks, rr = threadIdx.x;
+    if (slot >= *n_tiles) return;
+    const int4 T = tiles[slot];
+    if (rr >= T.z) return;
+    const bool shared = T.x == n_expert; // the shared expert's rows are the tokens in order, their ids follow the routed ones
+    const int fid = shared ? routed_rows + T.y + rr : ids_map[(size_t)T.x * map_stride + T.y + rr];
+    src[slot * nt + rr] = shared ? T.y + rr : fid / top_k;
+    pos[fid] = slot * nt + rr;
+    if (spos) spos[fid] = T.w + rr;
+    if (sfid) sfid[T.w + rr] = fid;
+}
+
 // ---- the grouped GEMM kernel -------------------------------------------------------------
 // One kernel, three uses: NPROJ = 2 multiplies a block of routed rows by 128 gate rows AND the matching 128 up
 // rows (every activation stage is loaded once for both, SwiGLU in the epilogue); NPROJ = 1 is a single
@@ -248,8 +288,9 @@ __global__ void __launch_bounds__(256) gather_tiles_kernel(const void *__restric
 // Tensor-memory columns: [0, NT) and [NT, 2 NT): the gate and up accumulators, or the two accumulator
 // buffers of a single projection (its epilogue runs beside the next tile's multiplies); the rest holds the operand
 // stages, 64 columns each: two beside 192-row tiles, four beside 128-row tiles.
-//   warp 0    MMA issuer    warp 1 B loader    warp 2 loader of the quantized columns    (warp 3 idle)
-//   warps 4-7 epilogue (NPROJ = 2: shared with the dequantising warps, which idle then)    warps 8-23 dequant
+//   warp 0    MMA issuer    warp 2 loader of the quantized columns    warps 8-23 dequant
+//   single projection: warp 1 B loader (bulk copies of the tile-ordered operand), warps 4-7 epilogue
+//   two projections: warps 4-7 B loaders (rows in token order), the epilogue falls to the dequantising warps
 constexpr int GM_DQ_WARPS = 16, GM_DQ0 = 8; // number of dequantising warps, the first of them
 constexpr int GM_THREADS = (GM_DQ_WARPS + 8) * 32;
 constexpr int GM_Q6_PITCH = 240; // a 210-byte block inside its 224-byte aligned window; 60 words: rows spread over the banks
@@ -266,7 +307,8 @@ struct GmCfg {
     static constexpr int B_BLK = NT * MM_K * 2;         // a 64-k block of the B operand
     static constexpr int NB = 96 * 1024 / B_BLK;        // ring of them
     static constexpr int NA = (512 - 2 * NT) / 64 >= 4 ? 4 : 2, A_COL0 = 2 * NT;
-    static constexpr int EPI_WARPS = NPROJ == 2 ? GM_DQ_WARPS + 4 : 4;
+    static constexpr int EPI_WARPS = NPROJ == 2 ? GM_DQ_WARPS : 4;
+    static constexpr int B_ARRIVALS = NPROJ == 2 ? 4 : 1; // per ring slot
     static constexpr int O_RAW = NB * B_BLK, O_EPI = O_RAW + RAW_SLOTS * RAW_SLOT, O_BAR = O_EPI + EPI_WARPS * EPI_BYTES;
     static constexpr int SMEM = O_BAR + 512 + 1024; // barriers, slack to align the base to 1024 bytes
     static_assert(A_COL0 + 64 * NA <= 512, "tensor memory");
@@ -284,7 +326,8 @@ struct GmParams {
     int n_expert, m_tiles;   // list number of the shared expert; blocks of 128 weight rows
     int64_t expert_bytes;
     int n_out, k;
-    const uint8_t *xt;       // f16 activations in tile order (see gather_tiles_kernel)
+    const uint8_t *xt;       // NPROJ = 1: f16 activations in tile order (see gather_tiles_kernel); 2: in token order
+    const int32_t *src;      // NPROJ = 2: row of xt of every tile row (see stage_rows_kernel)
     const int32_t *ids_map;  // [n_expert, map_stride] flat ids
     int map_stride;
     const int4 *tiles;       // row tiles, see row_tiles_kernel
@@ -504,7 +547,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             mb_init(&acc_empty[s], C::EPI_WARPS);
         }
         for (int i = 0; i < C::NB; i++) {
-            mb_init(&b_full[i], 1);
+            mb_init(&b_full[i], C::B_ARRIVALS);
             mb_init(&b_empty[i], 1);
         }
         for (int i = 0; i < C::RAW_SLOTS; i++) {
@@ -528,7 +571,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         // part: the projection (NPROJ = 2), the 64-wide k half of a stage (Q4_K) or the 16-wide l range (Q6_K)
         const int grp = (warp - GM_DQ0) >> 3, part = (warp >> 2) & 1, q = warp & 3, r = 32 * q + lane;
         const uint32_t ta = tmem_base + ((uint32_t)(32 * q) << 16) + C::A_COL0;
-        float *stage = reinterpret_cast<float *>(smem + C::O_EPI + (NPROJ == 2 ? (warp - 4) * C::EPI_BYTES : 0));
+        float *stage = reinterpret_cast<float *>(smem + C::O_EPI + (NPROJ == 2 ? (warp - GM_DQ0) * C::EPI_BYTES : 0));
         uint32_t use = 0, slot = 0, rph = 0, it = 0; // stages of this group, ring slot and its phase, tiles
         // the group's stage number `use` goes to operand slot (2 use + grp) mod NA; with two stages per column, i = use mod 2
         auto store = [&](const uint32_t (&o)[32], uint32_t i) {
@@ -604,7 +647,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                 if ((16 * c0 < T.nv || k_blocks <= 4) && ok) {
                     ok &= mb_wait(&acc_full[0], it & 1);
                     tc_fence_after();
-                    gm_epilogue<NPROJ, NT>(P, T, tmem_base, stage, q, lane, c0, 5);
+                    gm_epilogue<NPROJ, NT>(P, T, tmem_base, stage, q, lane, c0, 4);
                     tc_fence_before();
                 }
                 __syncwarp();
@@ -657,7 +700,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                 if (++slot == C::RAW_SLOTS) { slot = 0; rph ^= 1; }
             }
         }
-    } else if (warp == 1) {
+    } else if (NPROJ == 1 && warp == 1) {
         // ---------------- B loader: one bulk copy per 64-k block (the operand is stored in tile order) ----------------
         const bool el = elect_one();
         uint32_t slot = 0, ph = 0;
@@ -723,7 +766,57 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             if (el) tc_commit(&acc_full[buf]);
             __syncwarp();
         }
-    } else if (warp >= 4) {
+    } else if (NPROJ == 2 && warp >= 4) {
+        // ---------------- B loaders: thread = (16-byte chunk of the 128-byte row piece, every 16th row) ----------------
+        const int lt = tid - 128, ch = lt & 7, r0 = lt >> 3;
+        const uint32_t dst0 = s32(b_st) + (uint32_t)(r0 * 128 + ((ch ^ (r0 & 7)) << 4));
+        const uint32_t row16 = (uint32_t)(P.k >> 3); // 16-byte words of a row
+        uint32_t slot = 0, ph = 0, done = 0, behind = 0; // ring slot and phase; oldest slot not yet announced, how many there are
+        // A slot is announced two slots late: by then its copies have landed and the wait costs nothing.
+        auto announce = [&]() {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mb_arrive(&b_full[done]);
+            if (++done == C::NB) done = 0;
+            behind--;
+        };
+        GmTile T, next = gm_tile(P, blockIdx.x, n_tiles);
+        int nsrc[NT / 16];
+        auto rows = [&](const GmTile &N) {
+#pragma unroll
+            for (int i = 0; i < NT / 16; i++) nsrc[i] = r0 + 16 * i < N.nv ? __ldg(P.src + N.slot * NT + r0 + 16 * i) : 0;
+        };
+        rows(next);
+        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+            T = next;
+            next = gm_tile(P, tile + gridDim.x, n_tiles);
+            uint32_t off[NT / 16];
+#pragma unroll
+            for (int i = 0; i < NT / 16; i++) off[i] = (uint32_t)nsrc[i] * row16 + ch;
+            rows(next);
+            const int grp = gm_b_group<NT>(T.nv);
+            const uint32_t sub = C::B_BLK / grp;
+            for (int kb = 0; kb < k_blocks && ok; kb += grp) {
+                ok &= mb_wait(&b_empty[slot], ph ^ 1);
+                for (int g = 0; g < grp; g++) {
+                    const uint32_t dst = dst0 + slot * C::B_BLK + g * sub;
+                    const uint4 *base = reinterpret_cast<const uint4 *>(P.xt) + (size_t)(kb + g) * 8;
+#pragma unroll
+                    for (int i = 0; i < NT / 16; i++)
+                        if (r0 + 16 * i < T.nv)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 2048), "l"(base + off[i]) : "memory");
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                if (++slot == C::NB) { slot = 0; ph ^= 1; }
+                if (++behind == 3) {
+                    asm volatile("cp.async.wait_group 2;" ::: "memory");
+                    announce();
+                }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        while (behind > 0) announce();
+    } else if (NPROJ == 1 && warp >= 4) {
         // ---------------- epilogue ----------------
         float *stage = reinterpret_cast<float *>(smem + C::O_EPI + (warp - 4) * C::EPI_BYTES);
         uint32_t it = 0;
@@ -731,10 +824,10 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, it++) {
             T = next;
             next = gm_tile(P, tile + gridDim.x, n_tiles);
-            const uint32_t buf = NPROJ == 2 ? 0u : it & 1;
-            ok &= mb_wait(&acc_full[buf], NPROJ == 2 ? it & 1 : (it >> 1) & 1);
+            const uint32_t buf = it & 1;
+            ok &= mb_wait(&acc_full[buf], (it >> 1) & 1);
             tc_fence_after();
-            gm_epilogue<NPROJ, NT>(P, T, tmem_base + buf * NT, stage, warp & 3, lane, NPROJ == 2 ? 4 : 0, NPROJ == 2 ? 5 : 1);
+            gm_epilogue<NPROJ, NT>(P, T, tmem_base + buf * NT, stage, warp & 3, lane, 0, 1);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mb_arrive(&acc_empty[buf]);
@@ -781,6 +874,9 @@ size_t mm_tiles_bytes(const MmRows &R) { return lmoe_align_up((size_t)R.max_tile
 // The tile-ordered f16 operand of width k.
 size_t mm_tiled_bytes(const MmRows &R, int64_t k) { return lmoe_align_up((size_t)R.max_tiles * (size_t)(k / MM_K) * R.nt * 128, 256); }
 
+// Source rows of the tile rows (stage_rows_kernel).
+size_t mm_src_bytes(const MmRows &R) { return lmoe_align_up((size_t)R.max_tiles * R.nt * 4, 256); }
+
 static int32_t *mm_tile_count(const MmRows &R, void *tiles_ws) {
     return reinterpret_cast<int32_t *>(static_cast<uint8_t *>(tiles_ws) + mm_tiles_bytes(R) - 256);
 }
@@ -804,6 +900,29 @@ lmoe_status launch_gather_tiles(const MmRows &R, const void *x, int x_f16, int x
         gather_tiles_kernel<false><<<grid, 256, 0, s>>>(x, x_per_row, top_k, k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
                                                         (int)R.rows, R.nt, static_cast<uint8_t *>(xt), pos, spos, sfid);
     LMOE_LAUNCH_CHECK("gather_tiles_kernel");
+    return LMOE_OK;
+}
+
+// The same tables for the gate/up kernel: x as f16 in token order (`xh`, x_rows rows of k values) and the source row of every
+// tile row (`src`, mm_src_bytes).
+lmoe_status launch_stage_rows(const MmRows &R, const void *x, int x_f16, int64_t x_rows, int top_k, int k, const uint32_t *tpe,
+                              const int32_t *ids_map, int64_t map_stride, void *tiles_ws, void *xh, int32_t *src, int32_t *pos,
+                              int32_t *spos, int32_t *sfid, cudaStream_t s) {
+    if (R.n_expert > 512) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "grouped GEMM supports at most 512 experts");
+    int4 *tiles = static_cast<int4 *>(tiles_ws);
+    int32_t *n_tiles = mm_tile_count(R, tiles_ws);
+    row_tiles_kernel<<<1, 1024, 0, s>>>(tpe, R.n_expert, (int)R.extra, R.nt, tiles, n_tiles, (int)R.max_tiles);
+    LMOE_LAUNCH_CHECK("row_tiles_kernel");
+    const int64_t chunks = x_rows * (k / 8);
+    const int conv = (int)((chunks + 255) / 256);
+    const unsigned grid = (unsigned)(conv + R.max_tiles);
+    if (x_f16)
+        stage_rows_kernel<true><<<grid, 256, 0, s>>>(x, chunks, conv, top_k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
+                                                     (int)R.rows, R.nt, static_cast<uint8_t *>(xh), src, pos, spos, sfid);
+    else
+        stage_rows_kernel<false><<<grid, 256, 0, s>>>(x, chunks, conv, top_k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
+                                                      (int)R.rows, R.nt, static_cast<uint8_t *>(xh), src, pos, spos, sfid);
+    LMOE_LAUNCH_CHECK("stage_rows_kernel");
     return LMOE_OK;
 }
 
@@ -843,8 +962,8 @@ static lmoe_status make_rows_map(CUtensorMap *map, const void *base, uint64_t ro
 // st / sh: the stacks of the one or two projections, of the experts and (NULL without extra rows) of the shared expert.
 template <int DT, int NPROJ, int NT>
 static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *const (&st)[2], const lmoe_expert_stack *const (&sh)[2],
-                                  const void *xt, const int32_t *ids_map, int64_t map_stride, const float *row_scale, float *out,
-                                  int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
+                                  const void *xt, const int32_t *src, const int32_t *ids_map, int64_t map_stride, const float *row_scale,
+                                  float *out, int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
     using C = GmCfg<DT, NPROJ, NT>;
     GmParams P;
     P.rows8 = st[0]->n_out % 8 == 0;
@@ -863,7 +982,7 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
     P.w[1] = sh[0] ? sh[0]->blocks() : nullptr;
     P.expert_bytes = st[0]->expert_bytes(); P.n_out = (int)st[0]->n_out; P.k = (int)st[0]->k;
     P.n_expert = R.n_expert; P.m_tiles = mm_m_tiles(st[0]->n_out);
-    P.xt = static_cast<const uint8_t *>(xt); P.ids_map = ids_map; P.map_stride = (int)map_stride;
+    P.xt = static_cast<const uint8_t *>(xt); P.src = src; P.ids_map = ids_map; P.map_stride = (int)map_stride;
     P.tiles = static_cast<const int4 *>(tiles_ws); P.n_tiles = mm_tile_count(R, tiles_ws);
     P.row_scale = row_scale; P.out = out; P.sorted = sorted; P.flag = flag;
     P.vec = st[0]->n_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
@@ -892,15 +1011,15 @@ lmoe_status launch_mm_id(const MmRows &R, const lmoe_expert_stack *st, const lmo
                          uint32_t *flag, cudaStream_t stream) {
     auto fn = R.nt == 128 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128> : launch_grouped<LMOE_Q6_K, 1, 128>)
                           : (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 192> : launch_grouped<LMOE_Q6_K, 1, 192>);
-    return fn(R, {st, nullptr}, {shared, nullptr}, xt, ids_map, map_stride, row_scale, out, sorted, tiles_ws, flag, stream);
+    return fn(R, {st, nullptr}, {shared, nullptr}, xt, nullptr, ids_map, map_stride, row_scale, out, sorted, tiles_ws, flag, stream);
 }
 
 // gate and up in one kernel, SwiGLU applied: act[rows, ff] (f32), rows by flat id or in expert-sorted order.
 lmoe_status launch_mm_gateup(const MmRows &R, const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *sh_gate,
-                             const lmoe_expert_stack *sh_up, const void *xt, const int32_t *ids_map, int64_t map_stride, float *act,
+                             const lmoe_expert_stack *sh_up, const void *xh, const int32_t *src, const int32_t *ids_map, int64_t map_stride, float *act,
                              int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
     if (gate->dtype != LMOE_Q4_K || up->dtype != LMOE_Q4_K)
         return lmoe_fail(LMOE_ERR_UNSUPPORTED, "the fused gate/up kernel is built for Q4_K stacks");
     auto fn = R.nt == 128 ? launch_grouped<LMOE_Q4_K, 2, 128> : launch_grouped<LMOE_Q4_K, 2, 192>;
-    return fn(R, {gate, up}, {sh_gate, sh_up}, xt, ids_map, map_stride, nullptr, act, sorted, tiles_ws, flag, stream);
+    return fn(R, {gate, up}, {sh_gate, sh_up}, xh, src, ids_map, map_stride, nullptr, act, sorted, tiles_ws, flag, stream);
 }

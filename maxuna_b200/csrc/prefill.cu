@@ -12,8 +12,12 @@ size_t mm_tiled_bytes(const MmRows &R, int64_t k);
 lmoe_status launch_gather_tiles(const MmRows &R, const void *x, int x_f16, int x_per_row, int top_k, int k, const uint32_t *tpe,
                                 const int32_t *ids_map, int64_t map_stride, void *tiles_ws, void *xt, int32_t *pos, int32_t *spos,
                                 int32_t *sfid, cudaStream_t s);
+size_t mm_src_bytes(const MmRows &R);
+lmoe_status launch_stage_rows(const MmRows &R, const void *x, int x_f16, int64_t x_rows, int top_k, int k, const uint32_t *tpe,
+                              const int32_t *ids_map, int64_t map_stride, void *tiles_ws, void *xh, int32_t *src, int32_t *pos,
+                              int32_t *spos, int32_t *sfid, cudaStream_t s);
 lmoe_status launch_mm_gateup(const MmRows &R, const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *sh_gate,
-                             const lmoe_expert_stack *sh_up, const void *xt, const int32_t *ids_map, int64_t map_stride, float *act,
+                             const lmoe_expert_stack *sh_up, const void *xh, const int32_t *src, const int32_t *ids_map, int64_t map_stride, float *act,
                              int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream);
 lmoe_status launch_mm_id(const MmRows &R, const lmoe_expert_stack *st, const lmoe_expert_stack *shared, const void *xt,
                          const int32_t *ids_map, int64_t map_stride, const float *row_scale, float *out, int sorted, void *tiles_ws,
@@ -243,7 +247,8 @@ struct Carver {
 size_t ffn_bytes(const MmRows &R, int64_t hidden, int64_t ff) {
     const size_t all = (size_t)(R.rows + R.extra);
     size_t o = 0;
-    o += mm_tiled_bytes(R, hidden);                          // x in tile order
+    o += mm_tiled_bytes(R, hidden);                          // x in tile order, or in token order (never more)
+    o += mm_src_bytes(R);                                    // source row of every tile row
     o += lmoe_align_up(all * 4, 256);                        // position of every flat id
     o += 2 * lmoe_align_up(all * ff * 4, 256);               // gate, up
     o += mm_tiled_bytes(R, ff);                              // f16 activation in tile order
@@ -268,6 +273,7 @@ lmoe_status ffn_grouped(const MmRows &R, const lmoe_expert_stack *gate, const lm
     const int64_t all = R.rows + R.extra, ff = gate->n_out, hidden = gate->k;
     Carver c{ws, 0};
     uint8_t *xt = c.take<uint8_t>(mm_tiled_bytes(R, hidden));
+    int32_t *src = reinterpret_cast<int32_t *>(c.take<uint8_t>(mm_src_bytes(R)));
     int32_t *pos = c.take<int32_t>((size_t)all);
     float *g = c.take<float>((size_t)all * ff), *u = c.take<float>((size_t)all * ff);
     uint8_t *act = c.take<uint8_t>(mm_tiled_bytes(R, ff));
@@ -282,17 +288,19 @@ lmoe_status ffn_grouped(const MmRows &R, const lmoe_expert_stack *gate, const lm
         LMOE_CUDA(cudaMemsetAsync(spos, 0xFF, (size_t)all * 4, s));
         LMOE_CUDA(cudaMemsetAsync(sfid, 0xFF, (size_t)all * 4, s));
     }
-    if ((st = launch_gather_tiles(R, x, x_f16, 1, top_k, (int)hidden, tpe, ids_map, map_stride, tiles, xt, pos, sorted ? spos : nullptr,
-                                  sorted ? sfid : nullptr, s)))
-        return st;
     const unsigned row_blocks = (unsigned)((all + 7) / 8);
     if (fused_gu) {
         // both projections in one pass over the activations, SwiGLU in the epilogue
-        if ((st = launch_mm_gateup(R, gate, up, sh[0], sh[1], xt, ids_map, map_stride, g, sorted, tiles, flag, s))) return st;
+        if ((st = launch_stage_rows(R, x, x_f16, R.rows / top_k, top_k, (int)hidden, tpe, ids_map, map_stride, tiles, xt, src, pos,
+                                    sorted ? spos : nullptr, sorted ? sfid : nullptr, s)))
+            return st;
+        if ((st = launch_mm_gateup(R, gate, up, sh[0], sh[1], xt, src, ids_map, map_stride, g, sorted, tiles, flag, s))) return st;
         rescale_rows_kernel<<<row_blocks, 256, 0, s>>>(g, row_w, pos, sorted ? sfid : nullptr, all, R.rows, (int)ff, R.nt, act,
                                                        sorted ? scale_out : rs);
         LMOE_LAUNCH_CHECK("rescale_rows_kernel");
     } else {
+        if ((st = launch_gather_tiles(R, x, x_f16, 1, top_k, (int)hidden, tpe, ids_map, map_stride, tiles, xt, pos, nullptr, nullptr, s)))
+            return st;
         if ((st = launch_mm_id(R, gate, nullptr, xt, ids_map, map_stride, nullptr, g, 0, tiles, flag, s))) return st;
         if ((st = launch_mm_id(R, up, nullptr, xt, ids_map, map_stride, nullptr, u, 0, tiles, flag, s))) return st;
         swiglu_rows_kernel<<<row_blocks, 256, 0, s>>>(g, u, row_w, pos, all, (int)ff, R.nt, act, rs);
