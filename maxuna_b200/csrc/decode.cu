@@ -66,7 +66,7 @@ struct Cfg {
     static constexpr int NRED = NG == 1 ? 3 : 2 * NG;   // K-split partial buffers between the consumers and the epilogue warp
     static constexpr int MIN_CTAS = NG == 1 ? 2 : 1;
 };
-constexpr int SYNC_PASS0 = 32;   // layer sync words: [0] grid barrier, [1] exit count, [32 + pass] phase-1 units done
+constexpr int SYNC_PASS0 = 32;   // layer sync words: [0] grid barrier, [1] exit count, [2] tokens routed, [32 + pass] phase-1 units done
 constexpr int SYNC_WORDS = SYNC_PASS0 + 1024;
 constexpr int DEC_MAX_T = 64;
 constexpr int MAX_NTOK = 4;
@@ -117,20 +117,21 @@ struct DecLayout {
         o_ring = o; o += nstage * stage_bytes;
         o_xc = o;
         int xc_bytes = ncol * xs;
-        const int sel_bytes = 2 * n_expert * 4 + 2 * ncw * 32 * 4; // routing scratch aliases the activation cache
+        // scratch of the routing phase aliases the activation cache: keys, scores and the selected scores; later the expert counts
+        // and the id list of larger batches
+        const int sel_bytes = (2 * n_expert + 4 + 32) * 4, list_bytes = (n_expert + tk) * 4;
         if (sel_bytes > xc_bytes) xc_bytes = sel_bytes;
+        if (list_bytes > xc_bytes) xc_bytes = list_bytes;
         o += (xc_bytes + 15) / 16 * 16;
         o_s = o; o += ncol * ss * 2;
         o_sx = o; o += (kmax / QK_K) * 8 * 4; // [256-block][8 columns] digit scales
-        // the K-split partial buffers (phases 1-2) share their space with two routing tables that are
-        // only alive while the token lists are built: expert counts and the id list
-        int red_bytes = nred * CW * 16 * ncol * 4;
-        if (red_bytes < (n_expert + tk) * 4) red_bytes = (n_expert + tk) * 4;
-        o_red = o; o_cnt = o; o_ids = o + n_expert * 4;
-        o += (red_bytes + 15) / 16 * 16;
+        const int red_bytes = nred * CW * 16 * ncol * 4; // the K-split partial buffers
+        o_red = o; o += (red_bytes + 15) / 16 * 16;
+        // the routing scratch, the expert counts and the id list lie over the activation cache: it is staged again after they are dead
+        o_cnt = o_xc; o_ids = o_xc + n_expert * 4;
         o_bar = o; o += ((2 * nstage + 2 * nred) * 8 + 127) / 128 * 128;
         o_w = o; o += tk * 4;
-        o_off = o; o += (n_expert + 2) / 2 * 2 * 2;
+        o_off = o; o += (tk + 2) / 2 * 2 * 2;
         o_plist = o; o += (tk + 1) / 2 * 2 * 2;
         o_act = o; o += (tk + 2) / 2 * 2 * 2;
         o_ppre = o; o += (tk + 2) / 2 * 2 * 2;
@@ -150,15 +151,18 @@ __device__ __noinline__ void dec_bad_index(uint32_t *ctrl, uint32_t code, uint32
 }
 #define DEC_GUARD(cond, code, val) ((cond) ? true : (dec_bad_index(P.ctrl, (code), (uint32_t)(val)), false))
 
-// Grid-wide barrier among the consumer threads of all CTAs (thread 0 of each
-// CTA arrives).  `target` = arrivals expected so far in this launch.
-__device__ __forceinline__ void grid_barrier(uint32_t *ctrl, uint32_t *sync, uint32_t target, int tid, int cons_threads,
-                                             int first_id, int first_count) {
+// Grid-wide barrier among the consumer threads of all CTAs (thread 0 of each CTA arrives), in two halves so that work can
+// be done between them.  `target` = arrivals expected so far in this launch.
+__device__ __forceinline__ void grid_arrive(uint32_t *sync, int tid, int first_id, int first_count) {
     // the CTA barrier orders every thread's stores before thread 0's fence, which is cumulative: one fence per CTA
     bar_sync(first_id, first_count); // phases 1/2: the epilogue warp arrives here once its stores are fenced
     if (tid == 0) {
         __threadfence();
         atomicAdd(&sync[0], 1u);
+    }
+}
+__device__ __forceinline__ void grid_wait(uint32_t *ctrl, uint32_t *sync, uint32_t target, int tid, int cons_threads) {
+    if (tid == 0) {
         uint32_t i = 0;
         while (ld_acquire(&sync[0]) < target) {
             if ((i & 1023u) == 1023u && *reinterpret_cast<volatile uint32_t *>(ctrl) != 0u) break;
@@ -180,14 +184,40 @@ struct Pass {
     int tok[MAX_NTOK], pair[MAX_NTOK];
 };
 
-struct Tables {
+struct Tables { // per active expert: first entry in the pair list, expert id, first pass
     const uint16_t *off, *plist, *act, *ppre;
-    int n_active, routed_passes, shared_passes;
+    const int *n_active;
 };
 
 __device__ __forceinline__ void unit_range(int n_units, int &u0, int &u1) {
-    u0 = (int)((long long)blockIdx.x * n_units / gridDim.x);
-    u1 = (int)((long long)(blockIdx.x + 1) * n_units / gridDim.x);
+    if (n_units < (1 << 22)) { // the product fits 32 bits, whose division is a third of the 64-bit one's code
+        u0 = (int)((unsigned)blockIdx.x * (unsigned)n_units / gridDim.x);
+        u1 = (int)((unsigned)(blockIdx.x + 1) * (unsigned)n_units / gridDim.x);
+    } else {
+        u0 = (int)((long long)blockIdx.x * n_units / gridDim.x);
+        u1 = (int)((long long)(blockIdx.x + 1) * n_units / gridDim.x);
+    }
+}
+// The shared expert's phase-1 units.  The first t CTAs select the experts meanwhile and take none of them (they were 8 us
+// late for the routed units otherwise) unless they are more than half of all.
+__device__ __forceinline__ void unit_range_first(int n_units, int selecting, int &u0, int &u1) {
+    if (2 * selecting > (int)gridDim.x) selecting = 0;
+    const int c = (int)blockIdx.x - selecting, n = (int)gridDim.x - selecting;
+    u0 = c < 0 ? 0 : (int)((long long)c * n_units / n);
+    u1 = c < 0 ? 0 : (int)((long long)(c + 1) * n_units / n);
+}
+// Units of this CTA by section (phase 1 shared / routed, phase 2 shared / routed) as (first, end).  Each section is split
+// evenly by itself; only in phase 2, where a CTA has few units, shared and routed are split evenly TOGETHER: one token makes
+// 3.6 of them per CTA, and two separate splits gave some CTAs five.  (In phase 1 the shared units pass while the routing is
+// still on its way.)  A CTA's share of all must not be smaller than its part of the shared ones, which holds from one
+// routed unit per CTA on.
+__device__ __forceinline__ void dec_unit_range_of(int sec, int n_routed1, int n_shared2, int n_routed2, int2 *r) {
+    const int n = sec == 1 ? n_routed1 : (sec == 2 ? n_shared2 : n_routed2);
+    const bool together = sec == 3 && n_routed2 >= (int)gridDim.x && n_shared2 + n_routed2 <= 16 * (int)gridDim.x;
+    int a, b, c, d;
+    unit_range(together ? n_shared2 + n : n, a, b);
+    unit_range(together ? n_shared2 : 0, c, d);
+    r[sec] = make_int2(a - c, b - d);
 }
 
 // Resolve routed pass index -> active index (the expert it belongs to).
@@ -211,10 +241,9 @@ __device__ __forceinline__ void make_pass(Pass &U, int sh_t0, int sh_nt, int top
             U.pair[i] = U.tok[i] * (top_k + 1) + top_k;
         }
     } else {
-        const int a = find_active(T.ppre, T.n_active, q);
-        const int e = T.act[a];
+        const int a = find_active(T.ppre, *T.n_active, q);
         const int r = q - T.ppre[a];
-        const int o = T.off[e], n = T.off[e + 1] - o;
+        const int o = T.off[a], n = T.off[a + 1] - o;
         U.n_tok = min(NTOK, n - r * NTOK);
 #pragma unroll
         for (int i = 0; i < NTOK; i++) {
@@ -235,69 +264,90 @@ __device__ __forceinline__ void make_pass(Pass &U, int sh_t0, int sh_nt, int top
 // times 2^-9 (three digits) or 2^-4 (two), so they fit f16 for any input magnitude.  One warp per (token,
 // block): a lane owns 8 consecutive values.
 // FROM_X: phase 1, rows of x (global, read-only); else phase 2, SwiGLU activations written by other CTAs.
+// Three of a warp's blocks at a time: their loads are in flight together and their shuffle chains overlap (one at a time a
+// pass of two tokens took 3 us, during which the CTA multiplies nothing).  Out of line: it must not disturb the register
+// allocation of the unit loops.
 template <int NDIG, int NTOK, int SUB, bool FROM_X, int NCW>
-__device__ __forceinline__ void stage_rows(const DecodeParams &P, const Pass &U, int8_t *xc, __half *sh, float *sxs,
-                                           int xs, int ss, int warp, int lane) {
+__device__ __noinline__ void stage_rows(const float *rows, int k, int n_tok, int row0, int row1, int row2, int8_t *xc, __half *sh, float *sxs,
+                                        int xs, int ss, int warp, int lane) {
+    static_assert(NTOK <= 3, "rows of a pass");
     constexpr float QMAX = NDIG == 3 ? 524287.f : 16191.f;
-    const int k = FROM_X ? P.hidden : P.ff;
-    const int nblk = k / QK_K;
-    for (int it = warp; it < U.n_tok * nblk; it += NCW) {
-        const int tk = it / nblk, b = it - tk * nblk;
-        const float *src = (FROM_X ? P.x + (size_t)U.tok[tk] * P.hidden : P.act_f + (size_t)U.pair[tk] * P.ff) +
-                           b * QK_K + lane * 8;
-        float4 a, c;
-        if (FROM_X) {
-            a = __ldg(reinterpret_cast<const float4 *>(src));
-            c = __ldg(reinterpret_cast<const float4 *>(src) + 1);
-        } else {
-            a = __ldcg(reinterpret_cast<const float4 *>(src));
-            c = __ldcg(reinterpret_cast<const float4 *>(src) + 1);
-        }
-        const float v[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
-        float amax = 0.f;
+    constexpr int BATCH = 3;
+    const int nblk = k / QK_K, items = n_tok * nblk;
+    for (int it0 = warp; it0 < items; it0 += BATCH * NCW) {
+        float v[BATCH][8];
+        int tk[BATCH], blk[BATCH];
 #pragma unroll
-        for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(v[j]));
-#pragma unroll
-        for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        const float inv = amax > 0.f ? QMAX / amax : 0.f;
-        const float sx = amax * (1.0f / QMAX);
-        int sum = 0;
-        uint32_t dig[NDIG][2];
-#pragma unroll
-        for (int d = 0; d < NDIG; d++) dig[d][0] = dig[d][1] = 0u;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            int X = __float2int_rn(v[j] * inv);
-            sum += X;
-            // least significant digit first; the last digit takes what is left
-#pragma unroll
-            for (int d = NDIG - 1; d > 0; d--) {
-                const int dd = ((X + 64) & 127) - 64;
-                dig[d][j >> 2] |= (uint32_t)(dd & 255) << (8 * (j & 3));
-                X = (X - dd) >> 7;
+        for (int q = 0; q < BATCH; q++) {
+            const int it = min(it0 + q * NCW, items - 1); // past the end: repeat the last one, store nothing
+            tk[q] = (it >= nblk) + (it >= 2 * nblk);
+            blk[q] = it - tk[q] * nblk;
+            const float *src = rows + (size_t)(tk[q] == 0 ? row0 : (tk[q] == 1 ? row1 : row2)) * k + blk[q] * QK_K + lane * 8;
+            float4 a, c;
+            if (FROM_X) {
+                a = __ldg(reinterpret_cast<const float4 *>(src));
+                c = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+            } else {
+                a = __ldcg(reinterpret_cast<const float4 *>(src));
+                c = __ldcg(reinterpret_cast<const float4 *>(src) + 1);
             }
-            dig[0][j >> 2] |= (uint32_t)(X & 255) << (8 * (j & 3));
+            v[q][0] = a.x; v[q][1] = a.y; v[q][2] = a.z; v[q][3] = a.w;
+            v[q][4] = c.x; v[q][5] = c.y; v[q][6] = c.z; v[q][7] = c.w;
+        }
+        float amax[BATCH];
+#pragma unroll
+        for (int q = 0; q < BATCH; q++) {
+            amax[q] = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j++) amax[q] = fmaxf(amax[q], fabsf(v[q][j]));
         }
 #pragma unroll
-        for (int d = 0; d < NDIG; d++)
-            *reinterpret_cast<uint2 *>(xc + (NDIG * tk + d) * xs + b * QK_K + lane * 8) = make_uint2(dig[d][0], dig[d][1]);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        if (SUB == 32) sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        if ((lane & (SUB / 8 - 1)) == 0) {
-            // the integer sum, scaled into the f16 range whatever the magnitude of the row (|sum| <= 32 * QMAX);
-            // the block's scale comes back in through the column scales (see sum_ratio)
-            const float sf = (float)sum * (NDIG == 3 ? 0x1p-9f : 0x1p-4f);
-            const __half h = __float2half_rn(sf);
-            const int idx = b * (QK_K / SUB) + lane / (SUB / 8);
-            sh[(NDIG * tk) * ss + idx] = h;
-            sh[(NDIG * tk + 1) * ss + idx] = __float2half_rn(sf - __half2float(h));
-            if (NDIG == 3) sh[(NDIG * tk + 2) * ss + idx] = __float2half_rn(0.f);
-        }
-        if (lane < NDIG) {
-            // column scale: digit d (most significant first) weighs 128^(NDIG-1-d)
-            float f = sx;
-            for (int d = lane; d < NDIG - 1; d++) f *= 128.f;
-            sxs[b * 8 + NDIG * tk + lane] = f;
+        for (int o = 16; o; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < BATCH; q++) amax[q] = fmaxf(amax[q], __shfl_xor_sync(0xffffffffu, amax[q], o));
+#pragma unroll
+        for (int q = 0; q < BATCH; q++) {
+            const float inv = amax[q] > 0.f ? QMAX / amax[q] : 0.f;
+            const float sx = amax[q] * (1.0f / QMAX);
+            int sum = 0;
+            uint32_t dig[NDIG][2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                int X[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    X[j] = quant_int(v[q][4 * h + j], inv);
+                    sum += X[j];
+                }
+                uint32_t w[NDIG];
+                digits_of(X, w);
+#pragma unroll
+                for (int d = 0; d < NDIG; d++) dig[d][h] = w[d];
+            }
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            if (SUB == 32) sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            if (it0 + q * NCW < items) {
+                const int c0 = NDIG * tk[q], b = blk[q];
+#pragma unroll
+                for (int d = 0; d < NDIG; d++)
+                    *reinterpret_cast<uint2 *>(xc + (c0 + d) * xs + b * QK_K + lane * 8) = make_uint2(dig[d][0], dig[d][1]);
+                if ((lane & (SUB / 8 - 1)) == 0) {
+                    // the integer sum, scaled into the f16 range whatever the magnitude of the row (|sum| <= 32 * QMAX);
+                    // the block's scale comes back in through the column scales (see sum_ratio)
+                    const float sf = (float)sum * (NDIG == 3 ? 0x1p-9f : 0x1p-4f);
+                    const __half h = __float2half_rn(sf);
+                    const int idx = b * (QK_K / SUB) + lane / (SUB / 8);
+                    sh[c0 * ss + idx] = h;
+                    sh[(c0 + 1) * ss + idx] = __float2half_rn(sf - __half2float(h));
+                    if (NDIG == 3) sh[(c0 + 2) * ss + idx] = __float2half_rn(0.f);
+                }
+                if (lane < NDIG) {
+                    // column scale: digit d (most significant first) weighs 128^(NDIG-1-d)
+                    float f = sx;
+                    for (int d = lane; d < NDIG - 1; d++) f *= 128.f;
+                    sxs[b * 8 + c0 + lane] = f;
+                }
+            }
         }
     }
 }
@@ -417,6 +467,297 @@ __device__ __noinline__ void dec_wait_pass(const uint32_t *cnt, uint32_t need, u
     }
 }
 
+// The units n .. n1 - 1 of one pass (a unit is one fill of the ring, fills are counted through the launch).  A function of its
+// own, with everything in scalars: its registers are then its own, and no change around it moves them (the same loop inside
+// the kernel varied by 5 % with what stood beside it).
+template <int NDIG, int NTOK, int NG, int PHASE>
+__device__ __noinline__ void dec_units(uint32_t n, uint32_t n1, const uint8_t *ring, int stage_bytes, int row_bytes, int nb,
+                                       const int8_t *xcol, const __half *scol, const float *sxs, float r0, float r1, float *red,
+                                       uint64_t *full, uint32_t *ctrl) {
+    using C = Cfg<NG>;
+    constexpr int NCOL = NDIG * NTOK, NSTAGE = C::NSTAGE, NRED = C::NRED;
+    uint64_t *empty = full + NSTAGE, *red_full = empty + NSTAGE, *red_free = red_full + NRED;
+    const int lane = threadIdx.x & 31, wq = (threadIdx.x >> 5) % CW, g = lane >> 2, t4 = lane & 3;
+    bool have_data = false, have_buf = false;
+#pragma unroll 1
+    for (; n < n1; n++) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        const int s = n % NSTAGE;
+        // the answers about this unit's two barriers were asked for before the previous unit's arithmetic
+        if (!have_data) mbar_wait(&full[s], (n / NSTAGE) & 1, ctrl, 0x20 + PHASE);
+        const bool buf_free = have_buf;
+        have_data = mbar_test(&full[(n + 1) % NSTAGE], ((n + 1) / NSTAGE) & 1);
+        have_buf = mbar_test(&red_free[(n + 1) % NRED], (((n + 1) / NRED) & 1) ^ 1);
+        const uint8_t *stage = ring + (size_t)s * stage_bytes;
+        if (PHASE == 1) unit_q4k(stage, row_bytes, nb, wq, g, t4, xcol, scol, sxs, r0, r1, acc);
+        else unit_q6k(stage, row_bytes, nb, wq, g, t4, xcol, scol, sxs, r0, r1, acc);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
+        // K-split partials -> shared memory, handed to the epilogue warp
+        const int buf = n % NRED;
+        if (!buf_free) mbar_wait(&red_free[buf], ((n / NRED) & 1) ^ 1, ctrl, 0x28 + PHASE);
+        float *rb = red + buf * (CW * 16 * NCOL);
+        if (2 * t4 < NCOL) {
+            // accumulator rows: g and g+8 of the 16 (phase 1), 2g and 2g+1 (phase 2, see unit_q6k)
+            float *p = rb + (wq * 16 + (PHASE == 1 ? g : 2 * g)) * NCOL + 2 * t4;
+            const int second = PHASE == 1 ? 8 * NCOL : NCOL;
+            p[0] = acc[0]; p[1] = acc[1];
+            p[second] = acc[2]; p[second + 1] = acc[3];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&red_full[buf]);
+    }
+}
+
+// ---- routing: runs once per launch.  Functions that are not inlined take scalars, never the parameter block by reference:
+//      every access to it would then be a load from memory (the logits took 15 us instead of 5 that way). ----
+// Router logits (bit-specified reduction, see route_math.cuh).
+template <int NCW>
+__device__ __forceinline__ void dec_logits_rows(const DecodeParams &P, float *xs32, int tid, int warp, int lane) {
+    constexpr int CONS_THREADS = 32 * NCW;
+    const int E = P.n_expert, G = gridDim.x;
+    if (P.hidden == 128 * 24) {
+        // Work item = (expert, group of four tokens).  A CTA serves ONE token group (CTA c: group c mod
+        // #groups), so it stages only those four hidden states (as f32, in the not yet used weight ring);
+        // the CTAs of a group share out the experts, one per warp.  The router row is held in registers
+        // half a row at a time (all loads of a half in flight at once).  Each of the 128 partial chains
+        // still runs over its 24 elements in order.
+        constexpr int HH = 12;
+        const int H = P.hidden;
+        const int ngr = (P.t + 3) / 4;
+        const int cg = blockIdx.x % ngr, ci = blockIdx.x / ngr;
+        const int n_cta = (G - cg + ngr - 1) / ngr; // CTAs serving this group
+        const int t0 = 4 * cg, nt = min(4, P.t - t0);
+        float4 wv[HH];
+        bool preloaded = false;
+        {
+            // the first item's first half row is requested before the hidden states are staged
+            const int e = ci + n_cta * warp;
+            if (e < E) {
+                const float4 *wr = reinterpret_cast<const float4 *>(P.router + (size_t)e * H) + lane;
+#pragma unroll
+                for (int j = 0; j < HH; j++) wv[j] = __ldg(wr + 32 * j);
+                preloaded = true;
+            }
+        }
+        for (int i = tid; i < nt * (H / 4); i += CONS_THREADS)
+            reinterpret_cast<float4 *>(xs32)[i] = __ldg(reinterpret_cast<const float4 *>(P.x + (size_t)t0 * H) + i);
+        bar_sync(1, CONS_THREADS);
+        for (int e = ci + n_cta * warp; e < E; e += n_cta * NCW) {
+            const float4 *wr = reinterpret_cast<const float4 *>(P.router + (size_t)e * H) + lane;
+            float a[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i][0] = a[i][1] = a[i][2] = a[i][3] = 0.f;
+#pragma unroll 1
+            for (int half = 0; half < 2; half++) {
+                if (!(preloaded && half == 0)) {
+#pragma unroll
+                    for (int j = 0; j < HH; j++) wv[j] = __ldg(wr + 32 * (HH * half + j));
+                }
+                preloaded = false;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if (i < nt) {
+                        const float4 *xr = reinterpret_cast<const float4 *>(xs32 + i * H) + lane + 32 * HH * half;
+#pragma unroll
+                        for (int j = 0; j < HH; j++) {
+                            const float4 xv = xr[32 * j];
+                            a[i][0] = __fmaf_rn(xv.x, wv[j].x, a[i][0]);
+                            a[i][1] = __fmaf_rn(xv.y, wv[j].y, a[i][1]);
+                            a[i][2] = __fmaf_rn(xv.z, wv[j].z, a[i][2]);
+                            a[i][3] = __fmaf_rn(xv.w, wv[j].w, a[i][3]);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float v = lmoe_router_fold(a[i][0], a[i][1], a[i][2], a[i][3]);
+                if (lane == 0 && i < nt) P.logits[(size_t)(t0 + i) * E + e] = v;
+            }
+        }
+    } else {
+        const int ntt = (P.t + 3) / 4;
+        const int H = P.hidden;
+        for (int q = blockIdx.x * NCW + warp; q < E * ntt; q += G * NCW) {
+            const int e = q / ntt, t0 = (q - e * ntt) * 4;
+            const float *wr = P.router + (size_t)e * H;
+            float a[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i][0] = a[i][1] = a[i][2] = a[i][3] = 0.f;
+#pragma unroll 4
+            for (int base = 4 * lane; base < H; base += 128) {
+                const float4 wv = __ldg(reinterpret_cast<const float4 *>(wr + base));
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if (t0 + i < P.t) {
+                        const float4 xv = __ldg(reinterpret_cast<const float4 *>(P.x + (size_t)(t0 + i) * H + base));
+                        a[i][0] = __fmaf_rn(xv.x, wv.x, a[i][0]);
+                        a[i][1] = __fmaf_rn(xv.y, wv.y, a[i][1]);
+                        a[i][2] = __fmaf_rn(xv.z, wv.z, a[i][2]);
+                        a[i][3] = __fmaf_rn(xv.w, wv.w, a[i][3]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float v = lmoe_router_fold(a[i][0], a[i][1], a[i][2], a[i][3]);
+                if (lane == 0 && t0 + i < P.t) P.logits[(size_t)(t0 + i) * E + e] = v;
+            }
+        }
+    }
+}
+
+// Selection of token blockIdx.x: an expert's place in the stable descending order is the number of experts before it, and
+// the first top_k places are the decision.  One thread per expert counts over all keys: a short loop without a chain from
+// place to place.  (Everything before the first weights runs once per launch, from a cold instruction cache, and pays for
+// its code size: unrolled per-lane rounds took 7 us, a quarter of the experts per warp and a merge 3 us.)  The decision goes to
+// global memory; `sync[2]` counts the tokens that are done.  scratch: keys, scores, 32 selected scores.
+__device__ __noinline__ void dec_select_token(const float *logits, const float *bias, int E, int K, int norm, float scale, uint32_t *ids_row,
+                                              float *w_row, uint32_t *done, float *scratch, int tid, int threads) {
+    const int E4 = (E + 3) / 4 * 4;
+    uint32_t *keys = reinterpret_cast<uint32_t *>(scratch);
+    float *probs = scratch + E4, *top_p = probs + E;
+    // two experts per thread and step
+#pragma unroll 1
+    for (int e0 = tid; e0 < E4; e0 += 2 * threads) {
+        float lg[2], bs[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int e = min(e0 + i * threads, E - 1);
+            lg[i] = __ldcg(logits + e);
+            bs[i] = bias ? __ldg(bias + e) : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int e = e0 + i * threads;
+            const float p = lmoe_sigmoid_fixed(lg[i]);
+            const float sv = __fadd_rn(__fadd_rn(p, bs[i]), 0.0f); // -0 -> +0: integer order = float order
+            const uint32_t u = __float_as_uint(sv);
+            if (e < E) probs[e] = p;
+            if (e < E4) keys[e] = e < E ? max((u & 0x80000000u) ? ~u : (u | 0x80000000u), 1u) : 0u; // padding: before nobody
+        }
+    }
+    bar_sync(1, threads);
+#pragma unroll 1
+    for (int e0 = tid; e0 < E; e0 += 2 * threads) {
+        const int e1 = min(e0 + threads, E - 1);
+        const uint32_t m0 = keys[e0], m1 = keys[e1];
+        int place0 = 0, place1 = 0;
+#pragma unroll 4
+        for (int j = 0; j < E4; j += 4) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(keys + j);
+            const uint32_t l0 = j + 3 < e0 ? m0 - 1u : m0, l1 = j + 3 < e1 ? m1 - 1u : m1; // equal keys count where their index is lower
+            place0 += ((v.x > l0) + (v.y > l0)) + ((v.z > l0) + (v.w > l0));
+            place1 += ((v.x > l1) + (v.y > l1)) + ((v.z > l1) + (v.w > l1));
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int e = i ? e1 : e0;
+            int place = i ? place1 : place0;
+            const uint32_t me = i ? m1 : m0;
+            if (place >= K || (i && e0 + threads >= E)) continue;
+            for (int j = e & ~3; j < e; j++) place += keys[j] == me; // the four that hold e itself
+            if (place < K) {
+                ids_row[place] = (uint32_t)e;
+                top_p[place] = probs[e];
+            }
+        }
+    }
+    bar_sync(1, threads);
+    if (tid < 32) {
+        if (tid < K) {
+            float w = top_p[tid];
+            if (norm) {
+                float sum = 0.0f; // sequential in slot order, like a plain CPU sum
+                for (int k = 0; k < K; k++) sum = __fadd_rn(sum, top_p[k]);
+                sum = sum < 6.103515625e-5f ? 6.103515625e-5f : sum;
+                w = __fdiv_rn(w, sum);
+            }
+            if (scale != 0.0f && scale != 1.0f) w = __fmul_rn(w, scale);
+            w_row[tid] = w;
+        }
+        __syncwarp();
+        if (tid == 0) {
+            __threadfence(); // cumulative: the CTA barrier ordered the other warps' ids before it
+            atomicAdd(done, 1u);
+        }
+    }
+}
+
+// Per-expert token lists from the decision in ids_s (n pairs).
+template <int NTOK>
+__device__ __noinline__ void dec_lists(int n, int E, uint32_t *ctrl, const uint32_t *ids_s, uint32_t *cnt_s, uint16_t *plist_s, uint16_t *act_s,
+                                       uint16_t *off_s, uint16_t *ppre_s, int *n_active, int *routed_passes, int tid, int threads) {
+    const int warp = tid >> 5, lane = tid & 31;
+    for (int e = tid; e < E; e += threads) cnt_s[e] = 0;
+    bar_sync(1, threads);
+    for (int i = tid; i < n; i += threads)
+        if (ids_s[i] < (uint32_t)E) atomicAdd(&cnt_s[ids_s[i]], 1u);
+    bar_sync(1, threads);
+    if (warp == 0) {
+        // exclusive scans over experts: list offsets, active index, pass prefix
+        const int per = (E + 31) / 32;
+        const int e0 = lane * per, e1 = min(E, e0 + per);
+        int c_sum = 0, a_sum = 0, p_sum = 0;
+        for (int e = e0; e < e1; e++) {
+            const int c = (int)cnt_s[e];
+            c_sum += c;
+            a_sum += c > 0;
+            p_sum += (c + NTOK - 1) / NTOK;
+        }
+        int c_pre = c_sum, a_pre = a_sum, p_pre = p_sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int c2 = __shfl_up_sync(0xffffffffu, c_pre, o), a2 = __shfl_up_sync(0xffffffffu, a_pre, o);
+            const int p2 = __shfl_up_sync(0xffffffffu, p_pre, o);
+            if (lane >= o) { c_pre += c2; a_pre += a2; p_pre += p2; }
+        }
+        const int c_tot = __shfl_sync(0xffffffffu, c_pre, 31), a_tot = __shfl_sync(0xffffffffu, a_pre, 31);
+        const int p_tot = __shfl_sync(0xffffffffu, p_pre, 31);
+        c_pre -= c_sum; a_pre -= a_sum; p_pre -= p_sum;
+        for (int e = e0; e < e1; e++) {
+            const int c = (int)cnt_s[e];
+            cnt_s[e] = (uint32_t)c_pre; // where the expert's next pair goes
+            if (c > 0) {
+                act_s[a_pre] = (uint16_t)e;
+                off_s[a_pre] = (uint16_t)c_pre;
+                ppre_s[a_pre] = (uint16_t)p_pre;
+                a_pre++;
+                p_pre += (c + NTOK - 1) / NTOK;
+            }
+            c_pre += c;
+        }
+        if (lane == 31) {
+            off_s[a_tot] = (uint16_t)c_tot;
+            ppre_s[a_tot] = (uint16_t)p_tot;
+            *n_active = a_tot;
+            *routed_passes = p_tot;
+        }
+    }
+    bar_sync(1, threads);
+    for (int i = tid; i < n; i += threads) {
+        const uint32_t e = ids_s[i];
+        if (e < (uint32_t)E) {
+            const uint32_t pos = atomicAdd(&cnt_s[e], 1u);
+            if (pos < (uint32_t)n) plist_s[pos] = (uint16_t)i;
+            else dec_bad_index(ctrl, 0x506, pos);
+        }
+    }
+    bar_sync(1, threads);
+    // every CTA must see the same list order (passes are cut from it): sort each short list
+    for (int a = tid; a < *n_active; a += threads) {
+        const int o = off_s[a], c = off_s[a + 1] - o;
+        for (int i = 1; i < c; i++) {
+            const uint16_t v = plist_s[o + i];
+            int j = i - 1;
+            while (j >= 0 && plist_s[o + j] > v) { plist_s[o + j + 1] = plist_s[o + j]; j--; }
+            plist_s[o + j + 1] = v;
+        }
+    }
+    bar_sync(1, threads);
+}
+
 // ---- the kernel ---------------------------------------------------------------------
 template <int NDIG, int NTOK, int NG>
 __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decode_kernel(const __grid_constant__ DecodeParams P) {
@@ -441,6 +782,7 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
     uint16_t *act_s = reinterpret_cast<uint16_t *>(smem + L.o_act);
     uint16_t *ppre_s = reinterpret_cast<uint16_t *>(smem + L.o_ppre);
     __shared__ int s_n_active, s_routed_passes;
+    __shared__ int2 s_range[4];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = gridDim.x;
@@ -481,13 +823,11 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
             n++;
         };
         int u0, u1, u = 0;
-        // phase 1, shared expert: known before routing.  Only as many fills as the ring
-        // holds may be issued before the routing tables exist (consumers drain the ring
-        // only after they have built them).
-        unit_range(shared_passes * tiles1, u0, u1);
-        bar_sync(3, C::RING); // the consumers stage hidden states in the ring while they compute the logits
+        // phase 1, shared expert: known before routing, and consumed before it is complete
+        unit_range_first(shared_passes * tiles1, P.ext_ids ? 0 : P.t, u0, u1);
+        if (P.ext_ids == nullptr) bar_sync(3, C::RING); // the consumers stage hidden states in the ring while they compute the logits
         if (lane == 0) {
-            for (u = u0; u < u1 && u < u0 + NSTAGE; u++) {
+            for (u = u0; u < u1; u++) {
                 const int tile = u % tiles1;
                 fill(P.sh_gate + (size_t)tile * 8 * row4, P.sh_up + (size_t)tile * 8 * row4, 8 * row4);
             }
@@ -495,12 +835,9 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
         __syncwarp();
         bar_sync(2, C::THREADS); // routing tables are ready
         if (lane == 0) {
-            for (; u < u1; u++) {
-                const int tile = u % tiles1;
-                fill(P.sh_gate + (size_t)tile * 8 * row4, P.sh_up + (size_t)tile * 8 * row4, 8 * row4);
-            }
-            const int n_active = s_n_active, routed_passes = s_routed_passes;
-            unit_range(routed_passes * tiles1, u0, u1);
+            const int n_active = s_n_active;
+            u0 = s_range[1].x;
+            u1 = s_range[1].y;
             if (u0 < u1) {
                 int q = u0 / tiles1, tile = u0 - q * tiles1;
                 int e = act_s[find_active(ppre_s, n_active, q)];
@@ -514,9 +851,11 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
                 }
             }
             // phase 2 (weights do not depend on the grid barrier: keep streaming)
-            unit_range(shared_passes * tiles2, u0, u1);
+            u0 = s_range[2].x;
+            u1 = s_range[2].y;
             for (u = u0; u < u1; u++) fill(P.sh_down + (size_t)(u % tiles2) * DOWN_ROWS * row6, nullptr, DOWN_ROWS * row6);
-            unit_range(routed_passes * tiles2, u0, u1);
+            u0 = s_range[3].x;
+            u1 = s_range[3].y;
             if (u0 < u1) {
                 int q = u0 / tiles2, tile = u0 - q * tiles2;
                 int e = act_s[find_active(ppre_s, n_active, q)];
@@ -541,16 +880,16 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
         // ===================== epilogue warp =====================
         // Sums the K-split partials of each unit in a fixed order and writes the SwiGLU activation
         // (phase 1) or the weighted partial output row (phase 2), off the consumers' critical path.
-        bar_sync(2, C::THREADS);
-        const Tables T{off_s, plist_s, act_s, ppre_s, s_n_active, s_routed_passes, shared_passes};
+        const Tables T{off_s, plist_s, act_s, ppre_s, &s_n_active};
         uint32_t m = 0; // units handed over so far (the same sequence the consumers count)
-        for (int phase = 1; phase <= 2; phase++) {
+        for (int sec = 0; sec < 4; sec++) {
+            const int phase = 1 + (sec >> 1), shared = (sec & 1) ^ 1;
+            if (sec == 1) bar_sync(2, C::THREADS);
             const int tiles = phase == 1 ? tiles1 : tiles2;
-            for (int kind = 0; kind < 2; kind++) {
-                const int shared = kind == 0;
-                int u0, u1;
-                unit_range((shared ? shared_passes : T.routed_passes) * tiles, u0, u1);
-                if (u0 >= u1) continue;
+            int u0, u1;
+            if (sec == 0) unit_range_first(shared_passes * tiles, P.ext_ids ? 0 : P.t, u0, u1);
+            else u0 = s_range[sec].x, u1 = s_range[sec].y;
+            if (u0 < u1) {
                 int q = u0 / tiles, tile = u0 - q * tiles;
                 Pass U;
                 make_pass<NTOK>(U, P.sh_t0, P.sh_nt, K, T, shared, q);
@@ -615,7 +954,7 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
             }
             // the phase's results are complete: join the consumers' grid barrier (none after phase 1 when the
             // per-pass counters are in use)
-            if (phase == 2 || !pass_flags) {
+            if (sec == 3 || (sec == 1 && !pass_flags)) {
                 __threadfence();
                 bar_arrive(4, C::EPI);
             }
@@ -625,294 +964,60 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
 
     // ========================= consumer warps =========================
     const int g = lane >> 2, t4 = lane & 3;
-    const int grp = warp / CW, wq = warp % CW;
     uint32_t gb = 0; // grid barriers passed
 
     if (P.first_launch && blockIdx.x == 0 && tid < 4) P.ctrl[tid] = 0u; // a fresh device flag for this call
+    // ---- phase 0a: router logits, then token i's selection on CTA i.  The others do not wait for it here: the shared expert's
+    //      units, which do not depend on the routing, pass first. ----
     if (P.ext_ids == nullptr) {
-        // ---- phase 0a: router logits (bit-specified reduction, see route_math.cuh) ----
-        if (P.hidden == 128 * 24) {
-            // Work item = (expert, group of four tokens).  A CTA serves ONE token group (CTA c: group c mod
-            // #groups), so it stages only those four hidden states (as f32, in the not yet used weight ring);
-            // the CTAs of a group share out the experts, one per warp.  The router row is held in registers
-            // half a row at a time (all loads of a half in flight at once).  Each of the 128 partial chains
-            // still runs over its 24 elements in order.
-            constexpr int HH = 12;
-            const int H = P.hidden;
-            float *xs32 = reinterpret_cast<float *>(ring);
-            const int ngr = (P.t + 3) / 4;
-            const int cg = blockIdx.x % ngr, ci = blockIdx.x / ngr;
-            const int n_cta = (G - cg + ngr - 1) / ngr; // CTAs serving this group
-            const int t0 = 4 * cg, nt = min(4, P.t - t0);
-            float4 wv[HH];
-            bool preloaded = false;
-            {
-                // the first item's first half row is requested before the hidden states are staged
-                const int e = ci + n_cta * warp;
-                if (e < E) {
-                    const float4 *wr = reinterpret_cast<const float4 *>(P.router + (size_t)e * H) + lane;
-#pragma unroll
-                    for (int j = 0; j < HH; j++) wv[j] = __ldg(wr + 32 * j);
-                    preloaded = true;
-                }
-            }
-            for (int i = tid; i < nt * (H / 4); i += CONS_THREADS)
-                reinterpret_cast<float4 *>(xs32)[i] = __ldg(reinterpret_cast<const float4 *>(P.x + (size_t)t0 * H) + i);
-            bar_sync(1, CONS_THREADS);
-            for (int e = ci + n_cta * warp; e < E; e += n_cta * NCW) {
-                const float4 *wr = reinterpret_cast<const float4 *>(P.router + (size_t)e * H) + lane;
-                float a[4][4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) a[i][0] = a[i][1] = a[i][2] = a[i][3] = 0.f;
-#pragma unroll 1
-                for (int half = 0; half < 2; half++) {
-                    if (!(preloaded && half == 0)) {
-#pragma unroll
-                        for (int j = 0; j < HH; j++) wv[j] = __ldg(wr + 32 * (HH * half + j));
-                    }
-                    preloaded = false;
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        if (i < nt) {
-                            const float4 *xr = reinterpret_cast<const float4 *>(xs32 + i * H) + lane + 32 * HH * half;
-#pragma unroll
-                            for (int j = 0; j < HH; j++) {
-                                const float4 xv = xr[32 * j];
-                                a[i][0] = __fmaf_rn(xv.x, wv[j].x, a[i][0]);
-                                a[i][1] = __fmaf_rn(xv.y, wv[j].y, a[i][1]);
-                                a[i][2] = __fmaf_rn(xv.z, wv[j].z, a[i][2]);
-                                a[i][3] = __fmaf_rn(xv.w, wv[j].w, a[i][3]);
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float v = lmoe_router_fold(a[i][0], a[i][1], a[i][2], a[i][3]);
-                    if (lane == 0 && i < nt) P.logits[(size_t)(t0 + i) * E + e] = v;
-                }
-            }
-        } else {
-            const int ntt = (P.t + 3) / 4;
-            const int H = P.hidden;
-            for (int q = blockIdx.x * NCW + warp; q < E * ntt; q += G * NCW) {
-                const int e = q / ntt, t0 = (q - e * ntt) * 4;
-                const float *wr = P.router + (size_t)e * H;
-                float a[4][4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) a[i][0] = a[i][1] = a[i][2] = a[i][3] = 0.f;
-#pragma unroll 4
-                for (int base = 4 * lane; base < H; base += 128) {
-                    const float4 wv = __ldg(reinterpret_cast<const float4 *>(wr + base));
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        if (t0 + i < P.t) {
-                            const float4 xv = __ldg(reinterpret_cast<const float4 *>(P.x + (size_t)(t0 + i) * H + base));
-                            a[i][0] = __fmaf_rn(xv.x, wv.x, a[i][0]);
-                            a[i][1] = __fmaf_rn(xv.y, wv.y, a[i][1]);
-                            a[i][2] = __fmaf_rn(xv.z, wv.z, a[i][2]);
-                            a[i][3] = __fmaf_rn(xv.w, wv.w, a[i][3]);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float v = lmoe_router_fold(a[i][0], a[i][1], a[i][2], a[i][3]);
-                    if (lane == 0 && t0 + i < P.t) P.logits[(size_t)(t0 + i) * E + e] = v;
-                }
-            }
-        }
-        // selection bias -> shared memory (the expert-count table is not in use yet)
-        float *bias_s = reinterpret_cast<float *>(cnt_s);
-        for (int e = tid; e < E; e += CONS_THREADS) bias_s[e] = P.bias ? __ldg(P.bias + e) : 0.0f;
+        dec_logits_rows<NCW>(P, reinterpret_cast<float *>(ring), tid, warp, lane);
         bar_sync(3, C::RING); // the weight ring is free from here on: the producer may start
-        grid_barrier(P.ctrl, P.sync, (++gb) * (uint32_t)G, tid, CONS_THREADS, 1, CONS_THREADS);
-
-        // ---- phase 0b: selection.  Token i is handled by CTA i: each of the consumer warps ranks an equal share
-        //      of the experts (register-light, rolled loops: this code runs once), warp 0 merges the candidates;
-        //      ties always go to the lower expert index, so the result equals a stable descending sort.
-        //      Results travel through global memory and one more grid barrier. ----
+        grid_arrive(P.sync, tid, 1, CONS_THREADS);
+        gb++;
         if ((int)blockIdx.x < P.t) {
-            const int tok = blockIdx.x;
-            float *probs = reinterpret_cast<float *>(xc);
-            uint32_t *keys = reinterpret_cast<uint32_t *>(probs + E);
-            uint32_t *cand_key = keys + E, *cand_idx = cand_key + NCW * 32;
-            const int eq = (E + NCW - 1) / NCW, lo = warp * eq, hi = min(E, lo + eq);
-            uint32_t best = 0u;
-            int best_i = 0x7fffffff;
-            for (int e0 = lo; e0 < hi; e0 += 128) {
-                float lg[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int e = e0 + lane + 32 * i;
-                    lg[i] = e < hi ? __ldcg(P.logits + (size_t)tok * E + e) : 0.0f;
-                }
-#pragma unroll 1
-                for (int i = 0; i < 4; i++) {
-                    const int e = e0 + lane + 32 * i;
-                    if (e < hi) {
-                        const float p = lmoe_sigmoid_fixed(lg[i]);
-                        const float sv = __fadd_rn(__fadd_rn(p, bias_s[e]), 0.0f);
-                        const uint32_t u = __float_as_uint(sv);
-                        uint32_t kk = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-                        kk = kk == 0u ? 1u : kk;
-                        probs[e] = p;
-                        keys[e] = kk;
-                        if (kk > best) { best = kk; best_i = e; }
-                    }
-                }
-            }
-            __syncwarp();
-#pragma unroll 1
-            for (int k = 0; k < K; k++) {
-                const uint32_t m = __reduce_max_sync(0xffffffffu, best);
-                const uint32_t idx = __reduce_min_sync(0xffffffffu, best == m ? (uint32_t)best_i : 0xffffffffu);
-                if (lane == 0) { cand_key[warp * 32 + k] = m; cand_idx[warp * 32 + k] = idx; }
-                if (m != 0u && (int)idx == best_i && best == m) {
-                    keys[idx] = 0u;
-                    best = 0u;
-                    best_i = 0x7fffffff;
-#pragma unroll 1
-                    for (int e = lo + lane; e < hi; e += 32) {
-                        const uint32_t kk = keys[e];
-                        if (kk > best) { best = kk; best_i = e; }
-                    }
-                }
-            }
-            bar_sync(1, CONS_THREADS);
-            if (warp == 0) {
-                // lane l owns candidate l of every warp (K <= 32)
-                uint32_t ck[NCW], ci[NCW];
-#pragma unroll
-                for (int w = 0; w < NCW; w++) {
-                    ck[w] = lane < K ? cand_key[w * 32 + lane] : 0u;
-                    ci[w] = lane < K ? cand_idx[w * 32 + lane] : 0xffffffffu;
-                }
-                float my_w = 0.0f;
-#pragma unroll 1
-                for (int k = 0; k < K; k++) {
-                    uint32_t bk = 0u;
-#pragma unroll
-                    for (int w = 0; w < NCW; w++) bk = ck[w] > bk ? ck[w] : bk;
-                    const uint32_t m = __reduce_max_sync(0xffffffffu, bk);
-                    uint32_t bi = 0xffffffffu;
-#pragma unroll
-                    for (int w = 0; w < NCW; w++) bi = (ck[w] == m && ci[w] < bi) ? ci[w] : bi;
-                    const uint32_t idx = __reduce_min_sync(0xffffffffu, bi);
-#pragma unroll
-                    for (int w = 0; w < NCW; w++) if (ci[w] == idx) ck[w] = 0u;
-                    const float pw = probs[idx < (uint32_t)E ? idx : 0u];
-                    if (lane == k) my_w = pw;
-                    if (lane == 0) P.ids_ws[tok * K + k] = idx;
-                }
-                if (P.norm) {
-                    float sum = 0.0f;
-#pragma unroll 1
-                    for (int k = 0; k < K; k++) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, my_w, k));
-                    sum = sum < 6.103515625e-5f ? 6.103515625e-5f : sum;
-                    my_w = __fdiv_rn(my_w, sum);
-                }
-                if (P.scale != 0.0f && P.scale != 1.0f) my_w = __fmul_rn(my_w, P.scale);
-                if (lane < K) P.w_ws[tok * K + lane] = my_w;
-            }
-        }
-        grid_barrier(P.ctrl, P.sync, (++gb) * (uint32_t)G, tid, CONS_THREADS, 1, CONS_THREADS);
-        for (int i = tid; i < P.t * K; i += CONS_THREADS) {
-            const uint32_t id = __ldcg(P.ids_ws + i);
-            const float wv = __ldcg(P.w_ws + i);
-            ids_s[i] = id;
-            w_s[i] = wv;
-            if (blockIdx.x == 0) {
-                if (P.ids_out) P.ids_out[i] = id;
-                if (P.w_out) P.w_out[i] = wv;
-            }
-        }
-    } else {
-        // ---- the caller routed: take its decision as it is (an id >= n_expert marks an empty slot) ----
-        bar_sync(3, C::RING);
-        for (int i = tid; i < P.t * K; i += CONS_THREADS) {
-            ids_s[i] = __ldg(P.ext_ids + i);
-            w_s[i] = __ldg(P.ext_w + i);
+            grid_wait(P.ctrl, P.sync, (uint32_t)G, tid, CONS_THREADS);
+            dec_select_token(P.logits + (size_t)blockIdx.x * E, P.bias, E, K, P.norm, P.scale, P.ids_ws + blockIdx.x * K, P.w_ws + blockIdx.x * K,
+                             P.sync + 2, reinterpret_cast<float *>(xc), tid, CONS_THREADS);
         }
     }
-    for (int e = tid; e < E; e += CONS_THREADS) cnt_s[e] = 0;
-    bar_sync(1, CONS_THREADS);
-    // ---- phase 0c: per-expert token lists ----
-    for (int i = tid; i < P.t * K; i += CONS_THREADS)
-        if (ids_s[i] < (uint32_t)E) atomicAdd(&cnt_s[ids_s[i]], 1u);
-    bar_sync(1, CONS_THREADS);
-    if (warp == 0) {
-        // exclusive scans over experts: list offsets, active index, pass prefix
-        const int per = (E + 31) / 32;
-        const int e0 = lane * per, e1 = min(E, e0 + per);
-        int c_sum = 0, a_sum = 0, p_sum = 0;
-        for (int e = e0; e < e1; e++) {
-            const int c = (int)cnt_s[e];
-            c_sum += c;
-            a_sum += c > 0;
-            p_sum += (c + NTOK - 1) / NTOK;
-        }
-        int c_pre = c_sum, a_pre = a_sum, p_pre = p_sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int c2 = __shfl_up_sync(0xffffffffu, c_pre, o), a2 = __shfl_up_sync(0xffffffffu, a_pre, o);
-            const int p2 = __shfl_up_sync(0xffffffffu, p_pre, o);
-            if (lane >= o) { c_pre += c2; a_pre += a2; p_pre += p2; }
-        }
-        const int c_tot = __shfl_sync(0xffffffffu, c_pre, 31), a_tot = __shfl_sync(0xffffffffu, a_pre, 31);
-        const int p_tot = __shfl_sync(0xffffffffu, p_pre, 31);
-        c_pre -= c_sum; a_pre -= a_sum; p_pre -= p_sum;
-        for (int e = e0; e < e1; e++) {
-            const int c = (int)cnt_s[e];
-            off_s[e] = (uint16_t)c_pre;
-            if (c > 0) {
-                act_s[a_pre] = (uint16_t)e;
-                ppre_s[a_pre] = (uint16_t)p_pre;
-                a_pre++;
-                p_pre += (c + NTOK - 1) / NTOK;
-            }
-            c_pre += c;
-        }
-        if (lane == 31) {
-            off_s[E] = (uint16_t)c_tot;
-            ppre_s[a_tot] = (uint16_t)p_tot;
-            s_n_active = a_tot;
-            s_routed_passes = p_tot;
-        }
-    }
-    bar_sync(1, CONS_THREADS);
-    for (int e = tid; e < E; e += CONS_THREADS) cnt_s[e] = 0;
-    bar_sync(1, CONS_THREADS);
-    for (int i = tid; i < P.t * K; i += CONS_THREADS) {
-        const uint32_t e = ids_s[i];
-        if (e < (uint32_t)E) {
-            const uint32_t pos = atomicAdd(&cnt_s[e], 1u);
-            if (DEC_GUARD(off_s[e] + pos < (uint32_t)(P.t * K), 0x506, off_s[e] + pos)) plist_s[off_s[e] + pos] = (uint16_t)i;
-        }
-    }
-    bar_sync(1, CONS_THREADS);
-    // every CTA must see the same list order (passes are cut from it): sort each short list
-    for (int e = tid; e < E; e += CONS_THREADS) {
-        const int o = off_s[e], c = off_s[e + 1] - o;
-        for (int i = 1; i < c; i++) {
-            const uint16_t v = plist_s[o + i];
-            int j = i - 1;
-            while (j >= 0 && plist_s[o + j] > v) { plist_s[o + j + 1] = plist_s[o + j]; j--; }
-            plist_s[o + j + 1] = v;
-        }
-    }
-    bar_sync(1, CONS_THREADS);
-    bar_sync(2, C::THREADS); // release the producer and the epilogue warp: the routing tables are complete
-
-    const Tables T{off_s, plist_s, act_s, ppre_s, s_n_active, s_routed_passes, shared_passes};
+    const Tables T{off_s, plist_s, act_s, ppre_s, &s_n_active};
 
     uint32_t n_unit = 0; // units (= ring fills) before the current section, the same sequence as the producer's
-    uint32_t probed = 0xffffffffu; // unit whose barriers have been tested ahead (see the unit loop), and the answers
-    bool probe_data = false, probe_buf = false;
     unsigned long long xkey = ~0ull;
 
-    // ---- phases 1 and 2 ----
-    for (int phase = 1; phase <= 2; phase++) {
+    // ---- phases 1 and 2: the shared expert's units first, then the routed ones ----
+    for (int sec = 0; sec < 4; sec++) {
+        const int phase = 1 + (sec >> 1), shared = (sec & 1) ^ 1;
+        if (sec == 1) {
+            // ---- phase 0b: the routing decision, then the per-expert token lists ----
+            if (P.ext_ids == nullptr) {
+                if (tid == 0) dec_wait_pass(P.sync + 2, (uint32_t)P.t, P.ctrl, 0x180u);
+                bar_sync(1, CONS_THREADS);
+                for (int i = tid; i < P.t * K; i += CONS_THREADS) {
+                    ids_s[i] = __ldcg(P.ids_ws + i);
+                    w_s[i] = __ldcg(P.w_ws + i);
+                }
+            } else {
+                // the caller routed: take its decision as it is (an id >= n_expert marks an empty slot)
+                bar_sync(1, CONS_THREADS); // the list may lie over the activation cache
+                for (int i = tid; i < P.t * K; i += CONS_THREADS) {
+                    ids_s[i] = __ldg(P.ext_ids + i);
+                    w_s[i] = __ldg(P.ext_w + i);
+                }
+            }
+            bar_sync(1, CONS_THREADS);
+            if (blockIdx.x == 0 && P.ext_ids == nullptr) {
+                for (int i = tid; i < P.t * K; i += CONS_THREADS) {
+                    if (P.ids_out) P.ids_out[i] = ids_s[i];
+                    if (P.w_out) P.w_out[i] = w_s[i];
+                }
+            }
+            dec_lists<NTOK>(P.t * K, E, P.ctrl, ids_s, cnt_s, plist_s, act_s, off_s, ppre_s, &s_n_active, &s_routed_passes, tid, CONS_THREADS);
+            xkey = ~0ull; // the lists were built over the activation cache
+            if (tid >= 1 && tid < 4)
+                dec_unit_range_of(tid, s_routed_passes * tiles1, shared_passes * tiles2, s_routed_passes * tiles2, s_range);
+            bar_sync(2, C::THREADS); // release the producer and the epilogue warp: the routing tables are complete
+        }
         const int tiles = phase == 1 ? tiles1 : tiles2;
         // column pitch of the activation cache: 32 (mod 128) bytes for the 8-byte loads of phase 1, 16 for the
         // 4-byte loads of phase 2, so that the columns of one load instruction cover distinct banks
@@ -924,11 +1029,10 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
         // factors of the sub-block sum terms of this lane's two accumulator columns (x 32 for the Q6_K offset)
         const float r0 = sum_ratio<NDIG>(2 * t4) * (phase == 1 ? 1.0f : 32.0f);
         const float r1 = sum_ratio<NDIG>(2 * t4 + 1) * (phase == 1 ? 1.0f : 32.0f);
-        for (int kind = 0; kind < 2; kind++) { // shared units first, then routed
-            const int shared = kind == 0;
-            int u0, u1;
-            unit_range((shared ? shared_passes : T.routed_passes) * tiles, u0, u1);
-            if (u0 >= u1) continue;
+        int u0, u1;
+        if (sec == 0) unit_range_first(shared_passes * tiles, P.ext_ids ? 0 : P.t, u0, u1);
+        else u0 = s_range[sec].x, u1 = s_range[sec].y;
+        if (u0 < u1) {
             // the section is walked pass by pass: all consumer warps stage a pass's activations together,
             // then the two groups take alternate units of the pass's slice
             for (int q = u0 / tiles; q * tiles < u1; q++) {
@@ -945,46 +1049,25 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
                     if (phase == 2 && pass_flags && tid == 0)
                         dec_wait_pass(P.sync + SYNC_PASS0 + (shared ? q : shared_passes + q), (uint32_t)tiles1, P.ctrl, 0x200u + q);
                     bar_sync(1, CONS_THREADS); // everyone is done with the previous contents
-                    if (phase == 1) stage_rows<NDIG, NTOK, 32, true, NCW>(P, U, xc, sh, sxs, xs_ph, L.ss, warp, lane);
-                    else stage_rows<NDIG, NTOK, 16, false, NCW>(P, U, xc, sh, sxs, xs_ph, L.ss, warp, lane);
+                    if (phase == 1)
+                        stage_rows<NDIG, NTOK, 32, true, NCW>(P.x, P.hidden, U.n_tok, U.tok[0], U.tok[1], U.tok[NTOK - 1], xc, sh, sxs, xs_ph, L.ss, warp, lane);
+                    else
+                        stage_rows<NDIG, NTOK, 16, false, NCW>(P.act_f, P.ff, U.n_tok, U.pair[0], U.pair[1], U.pair[NTOK - 1], xc, sh, sxs, xs_ph, L.ss, warp, lane);
                     xkey = key;
                     bar_sync(1, CONS_THREADS);
                 }
-                for (int u = a; u < b; u++) {
-                    const uint32_t n = n_unit + (uint32_t)(u - u0);
-                    if ((int)(n % NG) != grp) continue;
-                    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                    const int s = n % NSTAGE; // one ring fill per unit
-                    // the answers about this unit's two barriers were asked for before the previous unit's arithmetic
-                    const bool have_data = probed == n && probe_data, have_buf = probed == n && probe_buf;
-                    if (!have_data) mbar_wait(&full[s], (n / NSTAGE) & 1, P.ctrl, 0x20 + phase);
-                    probed = n + 1;
-                    probe_data = mbar_test(&full[probed % NSTAGE], (probed / NSTAGE) & 1);
-                    probe_buf = mbar_test(&red_free[probed % NRED], ((probed / NRED) & 1) ^ 1);
-                    const uint8_t *stage = ring + (size_t)s * L.stage_bytes;
-                    if (phase == 1) unit_q4k(stage, row4, nb4, wq, g, t4, xcol, scol, sxs, r0, r1, acc);
-                    else unit_q6k(stage, row6, nb6, wq, g, t4, xcol, scol, sxs, r0, r1, acc);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&empty[s]);
-                    // K-split partials -> shared memory, handed to the epilogue warp
-                    const int buf = n % NRED;
-                    if (!have_buf) mbar_wait(&red_free[buf], ((n / NRED) & 1) ^ 1, P.ctrl, 0x28 + phase);
-                    float *rb = red + buf * (CW * 16 * NCOL);
-                    if (2 * t4 < NCOL) {
-                        // accumulator rows: g and g+8 of the 16 (phase 1), 2g and 2g+1 (phase 2, see unit_q6k)
-                        float *r0 = rb + (wq * 16 + (phase == 1 ? g : 2 * g)) * NCOL + 2 * t4;
-                        const int second = phase == 1 ? 8 * NCOL : NCOL;
-                        r0[0] = acc[0]; r0[1] = acc[1];
-                        r0[second] = acc[2]; r0[second + 1] = acc[3];
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&red_full[buf]);
-                }
+                const uint32_t n0 = n_unit + (uint32_t)(a - u0), n1 = n_unit + (uint32_t)(b - u0);
+                if (phase == 1)
+                    dec_units<NDIG, NTOK, NG, 1>(n0, n1, ring, L.stage_bytes, row4, nb4, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
+                else
+                    dec_units<NDIG, NTOK, NG, 2>(n0, n1, ring, L.stage_bytes, row6, nb6, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
             }
             n_unit += (uint32_t)(u1 - u0);
         }
-        if (phase == 2 || !pass_flags)
-            grid_barrier(P.ctrl, P.sync, (++gb) * (uint32_t)G, tid, CONS_THREADS, 4, C::EPI);
+        if (sec == 3 || (sec == 1 && !pass_flags)) {
+            grid_arrive(P.sync, tid, 4, C::EPI);
+            grid_wait(P.ctrl, P.sync, (++gb) * (uint32_t)G, tid, CONS_THREADS);
+        }
     }
 
     // ---- phase 3: out[t, :] = sum over slots (then the shared expert) of the weighted partial rows,
@@ -1030,7 +1113,8 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
         if (old == (uint32_t)(G - 1)) {
             P.sync[0] = 0u;
             P.sync[1] = 0u;
-            const int n_pass = shared_passes + T.routed_passes;
+            P.sync[2] = 0u;
+            const int n_pass = shared_passes + s_routed_passes;
             if (pass_flags)
                 for (int i = 0; i < n_pass && i < SYNC_WORDS - SYNC_PASS0; i++) P.sync[SYNC_PASS0 + i] = 0u;
             __threadfence();

@@ -76,18 +76,17 @@ __device__ __forceinline__ void mvs_stage_x(const float *__restrict__ x, int nb,
         int sum = 0;
         uint32_t dig[MVS_NDIG][2];
 #pragma unroll
-        for (int d = 0; d < MVS_NDIG; d++) dig[d][0] = dig[d][1] = 0u;
+        for (int h = 0; h < 2; h++) {
+            int X[4];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            int X = __float2int_rn(v[j] * inv);
-            sum += X;
-#pragma unroll
-            for (int d = MVS_NDIG - 1; d > 0; d--) { // least significant digit first; the last takes what is left
-                const int dd = ((X + 64) & 127) - 64;
-                dig[d][j >> 2] |= (uint32_t)(dd & 255) << (8 * (j & 3));
-                X = (X - dd) >> 7;
+            for (int j = 0; j < 4; j++) {
+                X[j] = quant_int(v[4 * h + j], inv);
+                sum += X[j];
             }
-            dig[0][j >> 2] |= (uint32_t)(X & 255) << (8 * (j & 3));
+            uint32_t w[MVS_NDIG];
+            digits_of(X, w);
+#pragma unroll
+            for (int d = 0; d < MVS_NDIG; d++) dig[d][h] = w[d];
         }
 #pragma unroll
         for (int d = 0; d < MVS_NDIG; d++)

@@ -81,6 +81,39 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
 }
 
 
+// round(v * inv) as an integer, for |v * inv| < 2^22: the sum with 1.5 * 2^23 holds it in its low mantissa bits.
+__device__ __forceinline__ int quant_int(float v, float inv) { return __float_as_int(__fmaf_rn(v, inv, 12582912.f)) - 0x4B400000; }
+
+// Four integers (|X| < 2^20) -> their signed base-128 digits, most significant first, one word of four bytes per digit.
+// With 64 + 64 * 128 added the two low digits are plain 7-bit fields plus 64; the digits of all four values are moved into
+// one word before the 64 comes off again (bytewise, no borrow crosses a byte), so a digit costs two operations.
+__device__ __forceinline__ uint32_t bytes_of(const uint32_t (&y)[4], uint32_t sel2) { // byte i of each word: sel2 = 0x(4+i)i
+    return __byte_perm(__byte_perm(y[0], y[1], sel2), __byte_perm(y[2], y[3], sel2), 0x5410u);
+}
+__device__ __forceinline__ uint32_t minus64(uint32_t v) { return (((v & 0x7F7F7F7Fu) | 0x80808080u) - 0x40404040u) ^ 0x80808080u; }
+__device__ __forceinline__ void digits_of(const int (&X)[4], uint32_t (&w)[3]) {
+    uint32_t y[4], z[4], u[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        y[j] = (uint32_t)(X[j] + 64 + 64 * 128);
+        z[j] = y[j] << 1; // bits 7..13 -> byte 1
+        u[j] = y[j] << 2; // bits 14..21 -> byte 2
+    }
+    w[2] = minus64(bytes_of(y, 0x40u));
+    w[1] = minus64(bytes_of(z, 0x51u));
+    w[0] = bytes_of(u, 0x62u);
+}
+__device__ __forceinline__ void digits_of(const int (&X)[4], uint32_t (&w)[2]) {
+    uint32_t y[4], z[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        y[j] = (uint32_t)(X[j] + 64);
+        z[j] = y[j] << 1; // bits 7..14 -> byte 1
+    }
+    w[1] = minus64(bytes_of(y, 0x40u));
+    w[0] = bytes_of(z, 0x51u);
+}
+
 // d = a*b (fresh accumulator: C is the zero register, no moves needed)
 __device__ __forceinline__ void mma16816_z(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                            uint32_t b0, uint32_t b1) {
