@@ -103,6 +103,7 @@ struct DecodeParams {
 // Shared-memory layout (bytes), computed identically on host and device.
 struct DecLayout {
     int stage_bytes, xs, ss;
+    bool lists_alias;
     int o_ring, o_xc, o_s, o_sx, o_red, o_bar, o_ids, o_w, o_cnt, o_off, o_plist, o_act, o_ppre, total;
     __host__ __device__ DecLayout(int hidden, int ff, int n_expert, int t, int top_k, int ncol, int ncw, int nstage, int nred) {
         const int row4 = hidden / QK_K * Q4K_BYTES, row6 = ff / QK_K * Q6K_BYTES;
@@ -117,8 +118,7 @@ struct DecLayout {
         o_ring = o; o += nstage * stage_bytes;
         o_xc = o;
         int xc_bytes = ncol * xs;
-        // scratch of the routing phase aliases the activation cache: keys, scores and the selected scores; later the expert counts
-        // and the id list of larger batches
+        // the selection's scratch aliases the activation cache: keys, scores and the selected scores
         const int sel_bytes = (2 * n_expert + 4 + 32) * 4, list_bytes = (n_expert + tk) * 4;
         if (sel_bytes > xc_bytes) xc_bytes = sel_bytes;
         if (list_bytes > xc_bytes) xc_bytes = list_bytes;
@@ -127,8 +127,11 @@ struct DecLayout {
         o_sx = o; o += (kmax / QK_K) * 8 * 4; // [256-block][8 columns] digit scales
         const int red_bytes = nred * CW * 16 * ncol * 4; // the K-split partial buffers
         o_red = o; o += (red_bytes + 15) / 16 * 16;
-        // the routing scratch, the expert counts and the id list lie over the activation cache: it is staged again after they are dead
-        o_cnt = o_xc; o_ids = o_xc + n_expert * 4;
+        // expert counts and id list: over the activation cache (which is staged again after they are dead) in larger batches
+        lists_alias = tk > 256;
+        o_cnt = lists_alias ? o_xc : o;
+        o_ids = o_cnt + n_expert * 4;
+        if (!lists_alias) o += (list_bytes + 15) / 16 * 16;
         o_bar = o; o += ((2 * nstage + 2 * nred) * 8 + 127) / 128 * 128;
         o_w = o; o += tk * 4;
         o_off = o; o += (tk + 2) / 2 * 2 * 2;
@@ -430,8 +433,9 @@ __device__ __forceinline__ void unit_q4k(const uint8_t *stage, int row_bytes, in
         q4k_block(rg + b * Q4K_BYTES, rG + b * Q4K_BYTES, t, xcol + 256 * b, scol + 8 * b, sxs + 8 * b, r0, r1, acc);
 }
 
-// 32 Q6_K rows: warp wq of the group takes row tile wq & 1 (16 rows) and every (CW/2)-th super-block of it.
-// Super-blocks are 210 bytes long, so every other one starts 2 bytes off a word boundary.
+// 32 Q6_K rows: warp wq of the group takes row tile wq & 1 (16 rows) and a contiguous half of its super-blocks.
+// Super-blocks are 210 bytes long, so every other one starts 2 bytes off a word boundary and costs twice the shared-memory
+// reads; neighbours share the expensive ones out evenly.
 __device__ __forceinline__ void unit_q6k(const uint8_t *stage, int row_bytes, int nb, int wq, int g, int t,
                                          const int8_t *xcol, const __half *scol, const float *sxs, float r0, float r1,
                                          float (&acc)[4]) {
@@ -439,7 +443,16 @@ __device__ __forceinline__ void unit_q6k(const uint8_t *stage, int row_bytes, in
     // disjoint shared-memory banks (rows g and g+8 would share two)
     const uint8_t *rg = stage + ((wq & 1) * 16 + 2 * g) * row_bytes;
     const uint8_t *rG = rg + row_bytes;
-    for (int b = wq >> 1; b < nb; b += CW / 2) {
+    if (nb == CW && !(row_bytes & 2)) {
+        // both of the warp's blocks in straight line: the second one's loads run under the first one's arithmetic (a unit is
+        // bound by its chains, with two warps per scheduler: 16 tokens 154 -> 148 us, 64 tokens 357 -> 342 us)
+        const int b = (wq >> 1) * 2;
+        q6k_block<0>(rg + b * Q6K_BYTES, rG + b * Q6K_BYTES, b, t, xcol, scol, sxs, r0, r1, acc);
+        q6k_block<1>(rg + (b + 1) * Q6K_BYTES, rG + (b + 1) * Q6K_BYTES, b + 1, t, xcol, scol, sxs, r0, r1, acc);
+        return;
+    }
+    const int per = (nb + CW / 2 - 1) / (CW / 2), b_end = min(nb, ((wq >> 1) + 1) * per);
+    for (int b = (wq >> 1) * per; b < b_end; b++) {
         const uint8_t *bg = rg + b * Q6K_BYTES, *bG = rG + b * Q6K_BYTES;
         if (row_bytes & 2) q6k_block<2>(bg, bG, b, t, xcol, scol, sxs, r0, r1, acc); // odd block count: rows alternate too
         else if (b & 1) q6k_block<1>(bg, bG, b, t, xcol, scol, sxs, r0, r1, acc);
@@ -683,6 +696,43 @@ __device__ __noinline__ void dec_select_token(const float *logits, const float *
             atomicAdd(done, 1u);
         }
     }
+}
+
+// The routing decision and the per-expert token lists of at most 32 (token, slot) pairs, by one warp without a barrier: lane i
+// holds pair i, and its place in (expert, pair) order is a count over the others.
+template <int NTOK>
+__device__ __noinline__ void dec_lists_warp(int n, int E, uint32_t id, uint16_t *plist_s, uint16_t *act_s, uint16_t *off_s, uint16_t *ppre_s,
+                                            int *n_active, int *routed_passes, int lane) {
+    const bool valid = lane < n && id < (uint32_t)E;
+    const uint32_t e = valid ? id : 0xffffff00u + lane; // empty slots come last, each by itself
+    const uint32_t same = __match_any_sync(0xffffffffu, e);
+    const int before = __popc(same & ((1u << lane) - 1u));
+    const int passes = valid && before == 0 ? (__popc(same) + NTOK - 1) / NTOK : 0; // of the expert, at its first pair
+    int less = 0, a_pre = 0, p_pre = 0;
+#pragma unroll 4
+    for (int j = 0; j < n; j++) {
+        const uint32_t ej = __shfl_sync(0xffffffffu, e, j);
+        const int pj = __shfl_sync(0xffffffffu, passes, j);
+        const bool lt = ej < e;
+        less += lt;
+        a_pre += lt && pj > 0;
+        p_pre += lt ? pj : 0;
+    }
+    if (valid) plist_s[less + before] = (uint16_t)lane;
+    if (passes > 0) {
+        act_s[a_pre] = (uint16_t)e;
+        off_s[a_pre] = (uint16_t)less;
+        ppre_s[a_pre] = (uint16_t)p_pre;
+    }
+    const int a_tot = __popc(__ballot_sync(0xffffffffu, passes > 0)), c_tot = __popc(__ballot_sync(0xffffffffu, valid));
+    const int p_tot = __reduce_add_sync(0xffffffffu, passes);
+    if (lane == 0) {
+        off_s[a_tot] = (uint16_t)c_tot;
+        ppre_s[a_tot] = (uint16_t)p_tot;
+        *n_active = a_tot;
+        *routed_passes = p_tot;
+    }
+    __syncwarp();
 }
 
 // Per-expert token lists from the decision in ids_s (n pairs).
@@ -990,30 +1040,38 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
         const int phase = 1 + (sec >> 1), shared = (sec & 1) ^ 1;
         if (sec == 1) {
             // ---- phase 0b: the routing decision, then the per-expert token lists ----
-            if (P.ext_ids == nullptr) {
-                if (tid == 0) dec_wait_pass(P.sync + 2, (uint32_t)P.t, P.ctrl, 0x180u);
-                bar_sync(1, CONS_THREADS);
-                for (int i = tid; i < P.t * K; i += CONS_THREADS) {
-                    ids_s[i] = __ldcg(P.ids_ws + i);
-                    w_s[i] = __ldcg(P.w_ws + i);
+            const uint32_t *ids_g = P.ext_ids ? P.ext_ids : P.ids_ws; // the caller's decision is taken as it is (an id >= n_expert:
+            const float *w_g = P.ext_ids ? P.ext_w : P.w_ws;          // an empty slot)
+            const int tk = P.t * K;
+            const bool write_out = blockIdx.x == 0 && P.ext_ids == nullptr;
+            if (tk <= 32) {
+                if (warp == 0) {
+                    if (P.ext_ids == nullptr && lane == 0) dec_wait_pass(P.sync + 2, (uint32_t)P.t, P.ctrl, 0x180u);
+                    __syncwarp();
+                    const uint32_t id = lane < tk ? __ldcg(ids_g + lane) : 0xffffffffu;
+                    if (lane < tk) {
+                        const float wv = __ldcg(w_g + lane);
+                        w_s[lane] = wv;
+                        if (write_out && P.ids_out) P.ids_out[lane] = id;
+                        if (write_out && P.w_out) P.w_out[lane] = wv;
+                    }
+                    dec_lists_warp<NTOK>(tk, E, id, plist_s, act_s, off_s, ppre_s, &s_n_active, &s_routed_passes, lane);
                 }
             } else {
-                // the caller routed: take its decision as it is (an id >= n_expert marks an empty slot)
-                bar_sync(1, CONS_THREADS); // the list may lie over the activation cache
-                for (int i = tid; i < P.t * K; i += CONS_THREADS) {
-                    ids_s[i] = __ldg(P.ext_ids + i);
-                    w_s[i] = __ldg(P.ext_w + i);
+                if (P.ext_ids == nullptr && tid == 0) dec_wait_pass(P.sync + 2, (uint32_t)P.t, P.ctrl, 0x180u);
+                bar_sync(1, CONS_THREADS); // (also: the lists may lie over the activation cache)
+                for (int i = tid; i < tk; i += CONS_THREADS) {
+                    const uint32_t id = __ldcg(ids_g + i);
+                    const float wv = __ldcg(w_g + i);
+                    ids_s[i] = id;
+                    w_s[i] = wv;
+                    if (write_out && P.ids_out) P.ids_out[i] = id;
+                    if (write_out && P.w_out) P.w_out[i] = wv;
                 }
+                bar_sync(1, CONS_THREADS);
+                dec_lists<NTOK>(tk, E, P.ctrl, ids_s, cnt_s, plist_s, act_s, off_s, ppre_s, &s_n_active, &s_routed_passes, tid, CONS_THREADS);
+                if (L.lists_alias) xkey = ~0ull; // they were built over the activation cache
             }
-            bar_sync(1, CONS_THREADS);
-            if (blockIdx.x == 0 && P.ext_ids == nullptr) {
-                for (int i = tid; i < P.t * K; i += CONS_THREADS) {
-                    if (P.ids_out) P.ids_out[i] = ids_s[i];
-                    if (P.w_out) P.w_out[i] = w_s[i];
-                }
-            }
-            dec_lists<NTOK>(P.t * K, E, P.ctrl, ids_s, cnt_s, plist_s, act_s, off_s, ppre_s, &s_n_active, &s_routed_passes, tid, CONS_THREADS);
-            xkey = ~0ull; // the lists were built over the activation cache
             if (tid >= 1 && tid < 4)
                 dec_unit_range_of(tid, s_routed_passes * tiles1, shared_passes * tiles2, s_routed_passes * tiles2, s_range);
             bar_sync(2, C::THREADS); // release the producer and the epilogue warp: the routing tables are complete
