@@ -24,8 +24,9 @@ DTYPE_NAME = {Q4_K: "Q4_K", Q6_K: "Q6_K"}
 
 
 def stream_ptr(stream=None) -> int:
-    s = torch.cuda.current_stream() if stream is None else stream
-    return s.cuda_stream
+    if stream is None:  # 0.4 us; building the `torch.cuda.Stream` object of the current stream costs 3.6
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return stream.cuda_stream
 
 
 class ExpertStack:
