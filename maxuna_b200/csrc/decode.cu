@@ -700,6 +700,8 @@ __device__ __noinline__ void dec_select_token(const float *logits, const float *
 
 // The routing decision and the per-expert token lists of at most 32 (token, slot) pairs, by one warp without a barrier: lane i
 // holds pair i, and its place in (expert, pair) order is a count over the others.
+// All of it is latency of code that runs once: the block-wide form below takes 3.4 us from the decision on at one token, this one
+// 1.5, and the staged activation stays where it is (one token 46.1 -> 42.0 us, four 78.6 -> 77).
 template <int NTOK>
 __device__ __noinline__ void dec_lists_warp(int n, int E, uint32_t id, uint16_t *plist_s, uint16_t *act_s, uint16_t *off_s, uint16_t *ppre_s,
                                             int *n_active, int *routed_passes, int lane) {

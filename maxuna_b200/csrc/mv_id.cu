@@ -2,15 +2,18 @@
 // Reference: `ops::mul_mv_id`, src/ops/mv_id.rs:37-45; kernels
 // kernel_mul_mv_id_q{4,6}_K_f32_v, src/ops/mv.metal:181-290, 413-504, 638-717.
 //
-// Two kernels.  Both carry the activations as three signed base-256 digits under the largest magnitude of every 256-wide
+// Three kernels.  All carry the activations as three signed base-256 digits under the largest magnitude of every 256-wide
 // block (24 bits: the resolution of f32 at that magnitude) and multiply them with the raw 4- and 6-bit fields on the integer
 // tensor-core path (mma.sync u8 x s8 -> s32, exact), as the fused decode kernel does; the scales come in once per
 // super-block.  A lane-per-16-bytes f32 dot product was bound by its conversions and multiply-adds.
-//   mv_pair_kernel   one (token, slot) pair per block row: the digits are MMA columns.  Weights go straight from global
-//                    memory into the A fragments (a fragment row is a whole 32-byte sector).
-//                    30 pairs of [1024 x 3072] Q4_K: 33 -> 20 us.
+//   mv_expert_kernel the ordinary case, bound by the weight stream: pairs of the same expert share a pass over its rows, which
+//                    come through shared memory in bulk copies.  Weights of 3 / 16 / 64 tokens with ten experts each, against
+//                    mv_pair_kernel: [1024 x 3072] Q4_K 17 / 78 / 290 -> 15 / 47 / 139 us, [3072 x 1024] Q6_K (whose 210-byte
+//                    super-blocks cost two loads a word from global memory) 39 / 203 / 810 -> 22 / 74 / 218 us.
+//   mv_pair_kernel   any shape, one (token, slot) pair per block row; what is left to it are rows too long for the ring and
+//                    matrices off a 16-byte boundary.  Weights go straight from global memory into the A fragments.
 //   mv_multi_kernel  many pairs of ONE weight matrix (the shared expert, a plain matrix): eight pairs are the columns of
-//                    an MMA, so a super-block is unpacked once for 32 pairs.  512 pairs of [1024 x 3072] Q4_K: 830 -> 84 us.
+//                    an MMA, so a super-block is unpacked once for 32 pairs.  512 pairs of [1024 x 3072] Q4_K: 830 -> 70 us.
 #include "common.cuh"
 #include "stream_math.cuh"
 
@@ -406,6 +409,363 @@ mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
     }
 }
 
+// ---- pairs grouped by expert ------------------------------------------------------------
+// grid (row splits, pairs): a block serves one expert's next 2 * NT pairs (its "leader" is the first of them; the blocks of
+// the others leave at once) on a range of row units.  A unit is 16 * m whole rows, contiguous in memory: a producer warp keeps
+// a ring of units filled with one bulk copy each, NG groups of four warps take them in turn and split a unit over K (and
+// over its row tiles when a row has fewer than four super-blocks).  Two pairs share one MMA (four columns each: the three
+// digits and a spare), so a super-block is unpacked once for 2 * NT pairs;
+// four pairs a block measured no better than two where the weights of the second pass come from the L2 cache.
+constexpr int MX_GW = 4;                                    // warps of a group
+constexpr int MX_STAGES = 8;                                // most ring stages
+constexpr int MX_WINDOW = 2048;                             // pairs of one expert are looked for among this many
+constexpr int MX_UNIT = 28 * 1024;                          // a unit has as many row tiles as fit here (at least what the warps need)
+constexpr int64_t MX_L2 = 100 << 20;                          // what of the 126 MB L2 cache a matrix may hope for
+constexpr int MX_SMEM_ONE = 226 * 1024, MX_SMEM_TWO = 112 * 1024; // dynamic shared memory of one / two blocks a SM
+
+struct MxLayout {
+    int pitch, ns, kw, m, unit_bytes, stride, nstage, o_sum, o_sx, o_red, o_bar, o_ring, total;
+    __host__ __device__ MxLayout(bool q4, int np, int ng, int nb, int smem_max) {
+        const int row_bytes = nb * (q4 ? Q4K_BYTES : Q6K_BYTES);
+        ns = q4 ? 8 : 16;
+        pitch = nb * QK_K + (q4 ? 32 : 16); // the columns of one load instruction cover distinct banks
+        kw = nb >= 4 ? 4 : (nb >= 2 ? 2 : 1); // warps along K; 4 / kw along the row tiles
+        m = 4 / kw;
+        while (2 * m * kw <= 8 && 32 * m * row_bytes <= MX_UNIT) m *= 2;
+        unit_bytes = 16 * m * row_bytes;
+        stride = (unit_bytes + 16 + 127) / 128 * 128; // 16 spare bytes: an aligned two-word read may end past the last block
+        int o = np * MV_NDIG * pitch;
+        o_sum = o; o += np * 2 * nb * ns * 2;
+        o_sx = o; o += (np * nb * 4 + 15) / 16 * 16;
+        o_red = o; o += ng * 2 * kw * np * 16 * m * 4;
+        o_bar = o; o += 2 * MX_STAGES * 8 + 16;
+        o_ring = (o + 127) / 128 * 128;
+        nstage = (smem_max - o_ring) / stride;
+        nstage = nstage > MX_STAGES ? MX_STAGES : (nstage < 0 ? 0 : nstage);
+        total = o_ring + nstage * stride;
+    }
+};
+
+// One super-block of two rows against the digits of 2 * NT pairs.  y[j]: this lane's pair of column tile j, rows g and G;
+// lanes of even t hold the two high digits (and the sums), lanes of odd t the low one.
+template <int NT>
+__device__ __forceinline__ void mx_finish(const int (&al)[NT][4], const float (&cm)[NT][4], float dg, float dG, float mg, float mG, int b, int t,
+                                          const float *const (&sxp)[NT], float (&y)[NT][2]) {
+    const float f0 = (t & 1) ? 1.f : 65536.f, f1 = (t & 1) ? 0.f : 256.f, fm = (t & 1) ? 0.f : 1.f;
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        const float sx = sxp[j][b];
+        y[j][0] += sx * (dg * (f0 * (float)al[j][0] + f1 * (float)al[j][1]) - mg * (fm * (cm[j][0] + cm[j][1])));
+        y[j][1] += sx * (dG * (f0 * (float)al[j][2] + f1 * (float)al[j][3]) - mG * (fm * (cm[j][2] + cm[j][3])));
+    }
+}
+template <int NT>
+__device__ __forceinline__ void mx_q4k(const uint8_t *bg, const uint8_t *bG, int b, int t, const int8_t *const (&xcol)[NT],
+                                       const __half *const (&scol)[NT], const float *const (&sxp)[NT], float (&y)[NT][2]) {
+    MvQ4 R;
+    R.hg = *reinterpret_cast<const uint4 *>(bg);
+    R.hG = *reinterpret_cast<const uint4 *>(bG);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        R.wg[j] = *reinterpret_cast<const uint2 *>(bg + 16 + 32 * j + 8 * t);
+        R.wG[j] = *reinterpret_cast<const uint2 *>(bG + 16 + 32 * j + 8 * t);
+    }
+    MvA<LMOE_Q4_K> A;
+    A.unpack(R, t);
+    int al[NT][4];
+    float cm[NT][4];
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        mma16816_z(cm[j], A.f[0], A.f[1], 0u, 0u, *reinterpret_cast<const uint32_t *>(scol[j] + b * 8 + 2 * t), 0u);
+#pragma unroll
+        for (int q = 0; q < 4; q++) al[j][q] = 0;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int sg = A.sg(i), sG = A.sG(i);
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            int f[4];
+            A.mma(i, f, xcol[j] + b * QK_K, t);
+            al[j][0] += sg * f[0]; al[j][1] += sg * f[1]; al[j][2] += sG * f[2]; al[j][3] += sG * f[3];
+        }
+    }
+    mx_finish<NT>(al, cm, A.dg, A.dG, A.mg, A.mG, b, t, sxp, y);
+}
+template <int NT, int MIS>
+__device__ __forceinline__ void mx_q6k(const uint8_t *bg, const uint8_t *bG, int b, int t, const int8_t *const (&xcol)[NT],
+                                       const __half *const (&scol)[NT], const float *const (&sxp)[NT], float (&y)[NT][2]) {
+    constexpr uint32_t M4 = 0x0F0F0F0Fu, M2 = 0x30303030u;
+    const int8_t *cg = reinterpret_cast<const int8_t *>(bg + 192), *cG = reinterpret_cast<const int8_t *>(bG + 192);
+    const float dg = lmoe_h2f(*reinterpret_cast<const uint16_t *>(bg + 208)), dG = lmoe_h2f(*reinterpret_cast<const uint16_t *>(bG + 208));
+    int al[NT][4];
+    float cm[NT][4];
+    {
+        const uint32_t f0 = sc_pair_half2(cg + 2 * t), f1 = sc_pair_half2(cG + 2 * t), f2 = sc_pair_half2(cg + 2 * t + 8), f3 = sc_pair_half2(cG + 2 * t + 8);
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            mma16816_z(cm[j], f0, f1, f2, f3, *reinterpret_cast<const uint32_t *>(scol[j] + b * 16 + 2 * t),
+                       *reinterpret_cast<const uint32_t *>(scol[j] + b * 16 + 2 * t + 8));
+#pragma unroll
+            for (int q = 0; q < 4; q++) al[j][q] = 0;
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+        const uint32_t wg0 = lds32<MIS>(bg, 192 + 8 * n), wg1 = lds32<MIS>(bg, 196 + 8 * n);
+        const uint32_t wG0 = lds32<MIS>(bG, 192 + 8 * n), wG1 = lds32<MIS>(bG, 196 + 8 * n);
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const int l0 = 16 * c + 4 * t;
+            const uint32_t qa_g = lds32<MIS>(bg, 64 * n + l0), qb_g = lds32<MIS>(bg, 64 * n + 32 + l0), qh_g = lds32<MIS>(bg, 128 + 32 * n + l0);
+            const uint32_t qa_G = lds32<MIS>(bG, 64 * n + l0), qb_G = lds32<MIS>(bG, 64 * n + 32 + l0), qh_G = lds32<MIS>(bG, 128 + 32 * n + l0);
+#pragma unroll
+            for (int i = 0; i < 4; i++) { // sub-block 8 n + 2 i + c: nibble i / 2 of ql run 2 (i & 1) + c, bits 2 i of qh run c
+                const uint32_t qg = (i & 1) ? qb_g : qa_g, qG = (i & 1) ? qb_G : qa_G;
+                const uint32_t lg = (i & 2) ? (qg >> 4) : qg, lG = (i & 2) ? (qG >> 4) : qG;
+                const uint32_t hg = i == 0 ? (qh_g << 4) : (i == 1 ? (qh_g << 2) : (i == 2 ? qh_g : (qh_g >> 2)));
+                const uint32_t hG = i == 0 ? (qh_G << 4) : (i == 1 ? (qh_G << 2) : (i == 2 ? qh_G : (qh_G >> 2)));
+                const uint32_t a0 = (lg & M4) | (hg & M2), a1 = (lG & M4) | (hG & M2);
+                const int sg = sbyte(i < 2 ? wg0 : wg1, 2 * (i & 1) + c), sG = sbyte(i < 2 ? wG0 : wG1, 2 * (i & 1) + c);
+#pragma unroll
+                for (int j = 0; j < NT; j++) {
+                    int f[4];
+                    imma16816_z(f, a0, a1, *reinterpret_cast<const uint32_t *>(xcol[j] + b * QK_K + 128 * n + 32 * i + l0));
+                    al[j][0] += sg * f[0]; al[j][1] += sg * f[1]; al[j][2] += sG * f[2]; al[j][3] += sG * f[3];
+                }
+            }
+        }
+    }
+    mx_finish<NT>(al, cm, dg, dG, dg * (32.f * MV_SUM_UNSCALE), dG * (32.f * MV_SUM_UNSCALE), b, t, sxp, y);
+}
+
+struct MxArgs {
+    const uint8_t *w; // the expert's rows
+    const uint8_t *ring;
+    const int8_t *xc;
+    const __half *sums;
+    const float *sxs;
+    float *red, *out;
+    uint64_t *full, *empty;
+    uint32_t *fail; // the block's failure words, then the count of units issued
+    const int *pairs;
+    int np, n_out, nb, u0, u1;
+};
+
+// The units of a block, by the consumer warps: columns of NT MMA tiles.
+template <int DT, int NT, int NG>
+__device__ __forceinline__ void mx_units(const MxArgs P, const MxLayout L, int warp_all, int lane) {
+    const int gi = warp_all / MX_GW, wq = warp_all % MX_GW, g = lane >> 2, t = lane & 3;
+    const int kq = wq % L.kw, tq = wq / L.kw, tstep = MX_GW / L.kw;
+    constexpr int TS = DT == LMOE_Q4_K ? Q4K_BYTES : Q6K_BYTES;
+    const int nb = P.nb, row_bytes = nb * TS, rows = 16 * L.m;
+    const int8_t *xcol[NT];
+    const __half *scol[NT];
+    const float *sxp[NT];
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        const int pb = 2 * j + (g >> 2), po = 2 * j + (t >> 1); // pair of this lane's B column, and of its accumulators
+        xcol[j] = P.xc + ((pb < P.np ? pb : 0) * MV_NDIG + min(g & 3, MV_NDIG - 1)) * L.pitch;
+        scol[j] = P.sums + ((pb < P.np ? pb : 0) * 2 + ((g & 3) == 1)) * nb * L.ns;
+        sxp[j] = P.sxs + (po < P.np ? po : 0) * nb;
+    }
+    // Q6_K rows 2g and 2g + 1 where they are word aligned: the eight rows of a load sit in disjoint banks
+    const bool inter = DT == LMOE_Q6_K && (row_bytes & 2) == 0;
+    const int rowA = inter ? 2 * g : g, rowB = inter ? 2 * g + 1 : g + 8;
+    int seq = gi; // of the block's unit sequence
+    for (int u = P.u0 + gi; u < P.u1; u += NG, seq += NG) {
+        const int s = seq % L.nstage;
+        wait_issued(P.fail + 3, (uint32_t)seq, P.fail, 1u);
+        mbar_wait(P.full + s, (uint32_t)((seq / L.nstage) & 1), P.fail, 1u);
+        float *rb = P.red + (gi * 2 + ((seq / NG) & 1)) * L.kw * 2 * NT * rows;
+        for (int tile = tq; tile < L.m; tile += tstep) {
+            const uint8_t *rg = P.ring + (size_t)s * L.stride + (16 * tile + rowA) * row_bytes;
+            const uint8_t *rG = P.ring + (size_t)s * L.stride + (16 * tile + rowB) * row_bytes;
+            float y[NT][2];
+#pragma unroll
+            for (int j = 0; j < NT; j++) y[j][0] = y[j][1] = 0.f;
+            for (int b = kq; b < nb; b += L.kw) {
+                if (DT == LMOE_Q4_K) mx_q4k<NT>(rg + b * TS, rG + b * TS, b, t, xcol, scol, sxp, y);
+                else if (row_bytes & 2) mx_q6k<NT, 2>(rg + b * TS, rG + b * TS, b, t, xcol, scol, sxp, y);
+                else if (b & 1) mx_q6k<NT, 1>(rg + b * TS, rG + b * TS, b, t, xcol, scol, sxp, y);
+                else mx_q6k<NT, 0>(rg + b * TS, rG + b * TS, b, t, xcol, scol, sxp, y);
+            }
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+                y[j][0] += __shfl_xor_sync(0xffffffffu, y[j][0], 1);
+                y[j][1] += __shfl_xor_sync(0xffffffffu, y[j][1], 1);
+                if ((t & 1) == 0) {
+                    float *r = rb + (kq * 2 * NT + 2 * j + (t >> 1)) * rows + 16 * tile;
+                    r[rowA] = y[j][0];
+                    r[rowB] = y[j][1];
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(P.empty + s);
+        // the buffer is written again two units of the group later, after the group's next barrier, which a warp reaches
+        // only when it has read this one
+        bar_sync(2 + gi, 32 * MX_GW);
+        const int r0 = u * rows, nr = min(rows, P.n_out - r0);
+        for (int i = wq * 32 + lane; i < P.np * rows; i += 32 * MX_GW) {
+            const int p = i / rows, r = i - p * rows;
+            float sum = 0.f;
+            for (int q = 0; q < L.kw; q++) sum += rb[(q * 2 * NT + p) * rows + r];
+            if (*reinterpret_cast<volatile uint32_t *>(P.fail) != 0u) sum = __int_as_float(0x7fc00000);
+            if (r < nr) P.out[(size_t)P.pairs[p] * P.n_out + r0 + r] = sum;
+        }
+    }
+}
+
+template <int DT, int NT, int NG, bool ODD>
+__global__ void __launch_bounds__(32 * (NG * MX_GW + 1), NG == 2 ? 2 : 1)
+mv_expert_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *__restrict__ x,
+                 int x_per_row, const uint32_t *__restrict__ ids, int top_k, int n_pairs, int smem_max, float *__restrict__ out) {
+    constexpr int SUB = DT == LMOE_Q4_K ? 32 : 16, NS = QK_K / SUB, NP = 2 * NT, CONS_WARPS = NG * MX_GW;
+    extern __shared__ __align__(128) uint8_t mx_smem[];
+    __shared__ int pairs_s[NP], np_s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, p0 = blockIdx.y;
+    const int nb = k / QK_K;
+    const MxLayout L(DT == LMOE_Q4_K, NP, NG, nb, smem_max);
+    const int rows = 16 * L.m, units = (n_out + rows - 1) / rows;
+    const int u0 = (int)((int64_t)units * blockIdx.x / gridDim.x), u1 = (int)((int64_t)units * (blockIdx.x + 1) / gridDim.x);
+    const uint32_t e = ids ? __ldg(ids + p0) : 0u;
+    if (e >= (uint32_t)n_expert) { // an out-of-range id produces a zero row
+        for (int i = u0 * rows + tid; i < min(u1 * rows, n_out); i += 32 * (CONS_WARPS + 1)) out[(size_t)p0 * n_out + i] = 0.f;
+        return;
+    }
+    uint64_t *full = reinterpret_cast<uint64_t *>(mx_smem + L.o_bar), *empty = full + MX_STAGES;
+    uint32_t *fail = reinterpret_cast<uint32_t *>(empty + MX_STAGES);
+    if (warp == 0) { // the expert's pairs: a count of those before p0 in the window, a list from p0 on
+        const int w0 = p0 / MX_WINDOW * MX_WINDOW, w1 = min(w0 + MX_WINDOW, n_pairs);
+        int before = 0, found = 0;
+        for (int i0 = w0; i0 < w1 && found < NP; i0 += 256) {
+            uint32_t id[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int i = i0 + 32 * j + lane;
+                id[j] = i < w1 ? (ids ? __ldg(ids + i) : 0u) : 0xffffffffu;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int i = i0 + 32 * j + lane;
+                const uint32_t hit = __ballot_sync(0xffffffffu, id[j] == e && i < w1), old = __ballot_sync(0xffffffffu, i < p0);
+                before += __popc(hit & old);
+                const uint32_t now = hit & ~old;
+                const int pos = found + __popc(now & ((1u << lane) - 1u));
+                if (((now >> lane) & 1u) && pos < NP) pairs_s[pos] = i;
+                found += __popc(now);
+            }
+            if (i0 + 256 > p0 && (before & (NP - 1))) break;
+        }
+        if (lane == 0) np_s = (before & (NP - 1)) ? 0 : min(found, NP);
+    } else if (tid == 32) {
+        for (int s = 0; s < L.nstage; s++) {
+            mbar_init(full + s, 1);
+            mbar_init(empty + s, MX_GW);
+        }
+        fail[0] = fail[1] = fail[2] = fail[3] = 0u;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    const int np = np_s;
+    if (np == 0) return; // an earlier pair's block serves this one
+    const uint8_t *we = w + (size_t)e * expert_bytes;
+    if (warp == CONS_WARPS) {
+        if (lane == 0) {
+            const int64_t row_bytes = (int64_t)nb * (DT == LMOE_Q4_K ? Q4K_BYTES : Q6K_BYTES);
+            int i = 0;
+            for (int u = u0; u < u1; u++, i++) {
+                const int s = i % L.nstage;
+                if (i >= L.nstage) mbar_wait<32>(empty + s, (uint32_t)((i / L.nstage - 1) & 1), fail, 2u);
+                copy_rows<ODD>(mx_smem + L.o_ring + (size_t)s * L.stride, we + (size_t)u * L.unit_bytes, (uint32_t)(min(rows, n_out - u * rows) * row_bytes), full + s);
+                set_issued(fail + 3, (uint32_t)i + 1);
+            }
+            // leave only when the last copies have landed (they have been waited for already unless a consumer gave up)
+            for (int j = i > L.nstage ? i - L.nstage : 0; j < i; j++)
+                mbar_wait<32>(full + j % L.nstage, (uint32_t)((j / L.nstage) & 1), fail, 3u);
+        }
+        return;
+    }
+    int8_t *xc = reinterpret_cast<int8_t *>(mx_smem);
+    __half *sums = reinterpret_cast<__half *>(mx_smem + L.o_sum);
+    float *sxs = reinterpret_cast<float *>(mx_smem + L.o_sx);
+    auto src = [&](int i) {
+        const int pair = pairs_s[i / nb];
+        return x + ((size_t)(pair / top_k) * x_per_row + (x_per_row == 1 ? 0 : pair % top_k)) * k + (size_t)(i % nb) * QK_K;
+    };
+    MvX in;
+    if (warp < np * nb) in.load(src(warp), true, lane);
+    for (int i = warp; i < np * nb; i += CONS_WARPS) {
+        const int p = i / nb, b = i - p * nb;
+        MvX next;
+        if (i + CONS_WARPS < np * nb) next.load(src(i + CONS_WARPS), true, lane);
+        uint2 dig[MV_NDIG];
+        float sx;
+        __half hi, lo;
+        mv_digits<SUB>(in, dig, sx, hi, lo);
+        in = next;
+#pragma unroll
+        for (int d = 0; d < MV_NDIG; d++) *reinterpret_cast<uint2 *>(xc + (p * MV_NDIG + d) * L.pitch + b * QK_K + lane * 8) = dig[d];
+        if ((lane & (SUB / 8 - 1)) == 0) {
+            sums[(2 * p) * nb * NS + b * NS + lane / (SUB / 8)] = hi;
+            sums[(2 * p + 1) * nb * NS + b * NS + lane / (SUB / 8)] = lo;
+        }
+        if (lane == 0) sxs[p * nb + b] = sx;
+    }
+    bar_sync(1, 32 * CONS_WARPS);
+    const MxArgs P = {we, mx_smem + L.o_ring, xc, sums, sxs, reinterpret_cast<float *>(mx_smem + L.o_red), out, full, empty, fail, pairs_s,
+                      np, n_out, nb, u0, u1};
+    mx_units<DT, NT, NG>(P, L, warp, lane);
+}
+
+template <int DT, int NT, int NG, bool ODD>
+cudaError_t launch_mv_expert(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs, int x_per_row,
+                             const uint32_t *ids, int top_k, float *out, int dev, int sms, cudaStream_t s) {
+    constexpr int smem_max = NG == 2 ? MX_SMEM_TWO : MX_SMEM_ONE;
+    const MxLayout L(DT == LMOE_Q4_K, 2 * NT, NG, k / QK_K, smem_max);
+    if (L.nstage < NG) return cudaErrorNotSupported; // rows too long for the ring
+    static thread_local int c_dev = -1;
+    if (dev != c_dev) {
+        const cudaError_t e = cudaFuncSetAttribute(mv_expert_kernel<DT, NT, NG, ODD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+        if (e != cudaSuccess) return e;
+        c_dev = dev;
+    }
+    const int64_t units = (n_out + 16 * L.m - 1) / (16 * L.m), slots = (NG == 2 ? 2 : 1) * (int64_t)sms;
+    const int64_t step = 65535 / top_k * top_k; // grid.y is limited to 65535
+    for (int64_t p = 0; p < pairs; p += step) {
+        const int64_t n = pairs - p < step ? pairs - p : step;
+        // Row splits: the blocks run in rounds of `slots`, and a block costs about three units of start-up.
+        const int64_t groups = n_expert == 1 ? (n + 2 * NT - 1) / (2 * NT) : n;
+        int64_t gx = 1, best = INT64_MAX;
+        for (int64_t rounds = 1; rounds <= 16; rounds++) {
+            int64_t g = rounds * slots / groups;
+            g = g < 1 ? 1 : (g > units ? units : g);
+            const int64_t cost = (groups * g + slots - 1) / slots * (3 + (units + g - 1) / g);
+            if (cost < best) best = cost, gx = g;
+        }
+        mv_expert_kernel<DT, NT, NG, ODD><<<dim3((unsigned)gx, (unsigned)n), 32 * (NG * MX_GW + 1), L.total, s>>>(
+            w, expert_bytes, n_expert, n_out, k, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k, (int)n,
+            smem_max, out + (size_t)p * n_out);
+    }
+    return cudaGetLastError();
+}
+
+// One block an SM, with twice the warps on the same digits: where a row is too long for two, and for a single matrix that is
+// larger than the L2 cache, so that up to four pairs cost one pass over it ([100352 x 3072] Q6_K, 2 / 4 pairs: 86 / 172 us in
+// passes of one pair, 55 / 91 with two blocks an SM, 47 / 72 so).
+template <int DT, bool ODD>
+cudaError_t launch_mv_by_expert(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs,
+                                int x_per_row, const uint32_t *ids, int top_k, float *out, int dev, int sms, cudaStream_t s) {
+    cudaError_t r = cudaErrorNotSupported;
+    if (n_expert == 1 && expert_bytes > MX_L2)
+        r = pairs > 2 ? launch_mv_expert<DT, 2, 4, ODD>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, dev, sms, s)
+                      : launch_mv_expert<DT, 1, 4, ODD>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, dev, sms, s);
+    if (r == cudaErrorNotSupported) r = launch_mv_expert<DT, 1, 2, ODD>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, dev, sms, s);
+    if (r == cudaErrorNotSupported) r = launch_mv_expert<DT, 1, 4, ODD>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, dev, sms, s);
+    return r;
+}
+
 template <int DT>
 cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs, int x_per_row,
                       const uint32_t *ids, int top_k, float *out, cudaStream_t s) {
@@ -414,8 +774,15 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    // one matrix for all pairs: from four pairs on the columns of one unpacked super-block pay for the 32-pair staging
-    if (n_expert == 1 && pairs >= 4) {
+    static thread_local int sms_dev = -1, sms = 0;
+    if (dev != sms_dev) {
+        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        sms_dev = dev;
+    }
+    // One matrix for all pairs: 32 pairs to an unpacked super-block, once such blocks cover every SM.  (Below that two pairs to a
+    // block win by parallelism: [1024 x 3072] Q4_K, 64 / 512 pairs 26 / 88 us against 55 / 70, [3072 x 1024] Q6_K, 32 / 128
+    // pairs 16 / 42 against 27 / 38.)
+    if (n_expert == 1 && (pairs + MM_COLS - 1) / MM_COLS * gx >= sms && pairs > 4) {
         constexpr int smem = MM_COLS * MM_PITCH<DT> + 2 * MM_COLS * (MM_KC / QK_K * NS + 8) * 2 + (MM_KC / QK_K) * MM_COLS * 4;
         static thread_local int c_dev = -1;
         if (dev != c_dev) {
@@ -430,6 +797,12 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
                 w, n_out, k, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k, (int)n, out + (size_t)p * n_out);
         }
         return cudaGetLastError();
+    }
+    // a bulk copy starts and ends on 16 bytes: every expert must; the end of a single matrix may be ragged
+    if ((reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (n_expert == 1 || expert_bytes % 16 == 0)) {
+        const cudaError_t r = expert_bytes % 16 ? launch_mv_by_expert<DT, true>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, dev, sms, s)
+                                                : launch_mv_by_expert<DT, false>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, dev, sms, s);
+        if (r != cudaErrorNotSupported) return r;
     }
     const int bc = k / QK_K < MV_PAIR_BLOCKS ? k / QK_K : MV_PAIR_BLOCKS;
     const int smem_pair = 3 * (bc * QK_K + 32) + 2 * bc * NS * 2 + bc * 4; // at most 27 KB

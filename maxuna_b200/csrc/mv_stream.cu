@@ -4,7 +4,7 @@
 // 253 MB that must all cross HBM, so the kernel is a pure bandwidth problem.
 //
 //   * One persistent CTA per SM.  A producer thread moves chunks of 16 weight rows (one MMA row tile,
-//     16 * row_bytes contiguous bytes, always a multiple of 16) into a shared-memory ring with one bulk copy
+//     16 * row_bytes contiguous bytes; the last may have fewer rows) into a shared-memory ring with one bulk copy
 //     each, completion counted on an mbarrier; as many stages as fit (five at k = 3072: 200 KB in flight per SM).
 //   * Three groups of four consumer warps take the chunks of the ring in turn; inside a group the four warps
 //     split the super-blocks of the chunk (the K dimension) and meet in a small shared array behind a named
@@ -49,7 +49,7 @@ struct MvsLayout {
         o_s = o; o += (MVS_NDIG * ss * 2 + 15) / 16 * 16;
         o_sx = o; o += nb * 8 * 4;
         o_red = o; o += 2 * MVS_NG * MVS_NCW * MVS_ROWS * 4;
-        o_bar = o; o += 2 * MVS_MAX_STAGES * 8 + 16; // full / empty barriers, then the CTA's failure word
+        o_bar = o; o += 2 * MVS_MAX_STAGES * 8 + 16; // full / empty barriers, then the CTA's failure words and the issue count
         o = (o + 127) / 128 * 128;
         o_ring = o;
         int n = (MVS_SMEM_MAX - o - 16) / stage_stride; // 16 spare bytes: an aligned two-word read may end past the last block
@@ -171,8 +171,10 @@ __device__ __forceinline__ void q6k_block_k32(const uint8_t *bg, const uint8_t *
     acc[3] += dG * (cs.y * ((float)al[3] - r1 * co[3]));
 }
 
+// ODD: the last chunk has fewer rows (code of its own: the few more instructions on the way to the first copies cost 2 of 43 us).
+template <bool ODD>
 __global__ void __launch_bounds__(MVS_THREADS, 1)
-mv_q6k_stream_kernel(const uint8_t *__restrict__ w, const float *__restrict__ x, float *__restrict__ out, int k, int n_chunks) {
+mv_q6k_stream_kernel(const uint8_t *__restrict__ w, const float *__restrict__ x, float *__restrict__ out, int n_out, int k, int n_chunks) {
     extern __shared__ __align__(128) uint8_t smem[];
     const MvsLayout L(k);
     const int nb = k / QK_K, row_bytes = nb * Q6K_BYTES, nstage = L.nstage;
@@ -182,7 +184,7 @@ mv_q6k_stream_kernel(const uint8_t *__restrict__ w, const float *__restrict__ x,
     float *red = reinterpret_cast<float *>(smem + L.o_red);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + L.o_bar);
     uint64_t *empty = full + MVS_MAX_STAGES;
-    uint32_t *fail = reinterpret_cast<uint32_t *>(empty + MVS_MAX_STAGES);
+    uint32_t *fail = reinterpret_cast<uint32_t *>(empty + MVS_MAX_STAGES), *issued = fail + 3;
     uint8_t *ring = smem + L.o_ring;
     const int tid = threadIdx.x, warp_all = tid >> 5, lane = tid & 31;
     const int gi = warp_all / MVS_NCW, warp = warp_all % MVS_NCW;
@@ -191,7 +193,7 @@ mv_q6k_stream_kernel(const uint8_t *__restrict__ w, const float *__restrict__ x,
             mbar_init(full + s, 1);
             mbar_init(empty + s, MVS_NCW);
         }
-        fail[0] = fail[1] = fail[2] = 0u;
+        fail[0] = fail[1] = fail[2] = *issued = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -202,8 +204,9 @@ mv_q6k_stream_kernel(const uint8_t *__restrict__ w, const float *__restrict__ x,
             for (int c = blockIdx.x; c < n_chunks; c += gridDim.x, i++) {
                 const int s = i % nstage;
                 if (i >= nstage) mbar_wait<32>(empty + s, (uint32_t)((i / nstage - 1) & 1), fail, 1u);
-                mbar_expect_tx(full + s, (uint32_t)L.chunk_bytes);
-                bulk_g2s(ring + (size_t)s * L.stage_stride, w + (size_t)c * L.chunk_bytes, (uint32_t)L.chunk_bytes, full + s);
+                copy_rows<ODD>(ring + (size_t)s * L.stage_stride, w + (size_t)c * L.chunk_bytes,
+                               (uint32_t)(ODD ? min(MVS_ROWS, n_out - c * MVS_ROWS) * row_bytes : L.chunk_bytes), full + s);
+                set_issued(issued, (uint32_t)i + 1);
             }
             // leave only when the last copies have landed (they have been waited for already unless a consumer gave up)
             for (int j = i > nstage ? i - nstage : 0; j < i; j++)
@@ -264,6 +267,7 @@ mv_q6k_stream_kernel(const uint8_t *__restrict__ w, const float *__restrict__ x,
     int i = gi;
     for (int c = blockIdx.x + gi * gridDim.x; c < n_chunks; c += MVS_NG * gridDim.x, i += MVS_NG) {
         const int s = i % nstage;
+        wait_issued(issued, (uint32_t)i, fail, 3u);
         mbar_wait(full + s, (uint32_t)((i / nstage) & 1), fail, 3u);
         const uint8_t *rg = ring + (size_t)s * L.stage_stride + rowA * row_bytes;
         const uint8_t *rG = ring + (size_t)s * L.stage_stride + rowB * row_bytes;
@@ -298,7 +302,7 @@ mv_q6k_stream_kernel(const uint8_t *__restrict__ w, const float *__restrict__ x,
 #pragma unroll
             for (int q = 0; q < MVS_NCW; q++) sum += rb[q * MVS_ROWS + lane];
             if (*reinterpret_cast<volatile uint32_t *>(fail) != 0u) sum = __int_as_float(0x7fc00000);
-            out[(size_t)c * MVS_ROWS + lane] = sum;
+            if (!ODD || c * MVS_ROWS + lane < n_out) out[(size_t)c * MVS_ROWS + lane] = sum;
         }
     }
 }
@@ -311,10 +315,9 @@ bool mv_q6k_stream_available(int64_t n_out, int64_t k) {
     if (k <= 0 || k % QK_K != 0 || n_out < MVS_ROWS) return false;
     if (k / QK_K > MVS_MAX_NB) return false;
     const MvsLayout L((int)k);
-    return L.nstage >= 3;
+    return L.nstage >= MVS_NG;
 }
 
-// Rows [0, n_out - n_out % 16) of one activation row; the caller serves the tail rows with the row-per-warp kernel.
 cudaError_t launch_mv_q6k_stream(const uint8_t *w, int n_out, int k, const float *x, float *out, cudaStream_t s) {
     static std::mutex mu;
     static bool ready[64] = {};
@@ -327,16 +330,16 @@ cudaError_t launch_mv_q6k_stream(const uint8_t *w, int n_out, int k, const float
     {
         std::lock_guard<std::mutex> lock(mu);
         if (!ready[dev]) {
-            e = cudaFuncSetAttribute(mv_q6k_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MVS_SMEM_MAX);
+            e = cudaFuncSetAttribute(mv_q6k_stream_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MVS_SMEM_MAX);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(mv_q6k_stream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MVS_SMEM_MAX);
             if (e != cudaSuccess) return e;
             e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
             if (e != cudaSuccess) return e;
             ready[dev] = true;
         }
     }
-    const int n_chunks = n_out / MVS_ROWS;
-    if (n_chunks == 0) return cudaSuccess;
+    const int n_chunks = (n_out + MVS_ROWS - 1) / MVS_ROWS;
     const int grid = n_chunks < sms[dev] ? n_chunks : sms[dev];
-    mv_q6k_stream_kernel<<<grid, MVS_THREADS, L.total, s>>>(w, x, out, k, n_chunks);
+    (n_out % MVS_ROWS ? mv_q6k_stream_kernel<true> : mv_q6k_stream_kernel<false>)<<<grid, MVS_THREADS, L.total, s>>>(w, x, out, n_out, k, n_chunks);
     return cudaGetLastError();
 }

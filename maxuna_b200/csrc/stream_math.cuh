@@ -68,6 +68,41 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                  "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
+// Several warp groups that share a ring: a stage's barrier tells its turns apart by parity only, and another group may have had
+// the stage last, so a group asks first whether the producer has issued unit `seq` (it does so in order, and only after the
+// stage's last turn is over).  A word in shared memory; asking the stage's other barrier instead cost 0.3 us a unit.
+__device__ __forceinline__ void set_issued(uint32_t *issued, uint32_t n) {
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(issued)), "r"(n) : "memory");
+}
+__device__ __forceinline__ uint32_t get_issued(const uint32_t *issued) {
+    uint32_t n;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(n) : "r"(smem_u32(issued)) : "memory");
+    return n;
+}
+static __device__ __noinline__ void poll_issued(const uint32_t *issued, uint32_t seq, uint32_t *ctrl, uint32_t where) {
+    for (uint32_t i = 0; i < SPIN_LIMIT; i++) {
+        if (get_issued(issued) > seq) return;
+        if ((i & 1023u) == 1023u && *reinterpret_cast<volatile uint32_t *>(ctrl) != 0u) return;
+        __nanosleep(64); // far below the copy's own flight time
+    }
+    if (atomicCAS(ctrl, 0u, (uint32_t)LMOE_FLAG_WAIT_TIMEOUT) == 0u) {
+        ctrl[1] = where;
+        ctrl[2] = blockIdx.x;
+    }
+}
+__device__ __forceinline__ void wait_issued(const uint32_t *issued, uint32_t seq, uint32_t *ctrl, uint32_t where) {
+    if (get_issued(issued) <= seq) poll_issued(issued, seq, ctrl, where);
+}
+// A run of rows global -> shared, by one thread: a bulk copy, and the bytes past the last multiple of 16 (an odd number of
+// rows at the end of a matrix) by plain stores that the arrival on `bar` publishes.  `src` on a 16-byte boundary, `bytes` even.
+template <bool ODD>
+__device__ __forceinline__ void copy_rows(uint8_t *dst, const uint8_t *src, uint32_t bytes, uint64_t *bar) {
+    const uint32_t body = ODD ? bytes & ~15u : bytes;
+    if (ODD)
+        for (uint32_t i = body; i < bytes; i += 2) *reinterpret_cast<uint16_t *>(dst + i) = __ldg(reinterpret_cast<const uint16_t *>(src + i));
+    mbar_expect_tx(bar, body);
+    bulk_g2s(dst, src, body, bar);
+}
 __device__ __forceinline__ void bar_sync(int id, int count) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }

@@ -123,6 +123,31 @@ def test_mv_tile_edges(orc, dev, dt, name, n_expert, n_out, k, t, top_k, xpr):
     assert np.array_equal(hole, got)
 
 
+@pytest.mark.parametrize("n_expert,n_out,k,t,top_k", [
+    (3, 8, 256, 2, 2),       # one super-block per row, one unit shorter than a row tile
+    (5, 72, 512, 7, 3),      # two; three to five pairs of an expert
+    (4, 200, 768, 9, 2),     # three: rows of odd word alignment (Q6_K), a tail unit
+    (2, 136, 1280, 6, 1),    # five: a second turn of the K split for one warp only
+    (7, 40, 256, 700, 3),    # more pairs than an expert's are looked for among, many blocks of each expert
+    (3, 1032, 4096, 3, 3),   # more shared memory than two blocks of an SM have
+])
+@pytest.mark.parametrize("dt,name", DTYPES)
+def test_mv_pairs_by_expert(orc, dev, dt, name, n_expert, n_out, k, t, top_k):
+    """Pairs grouped by expert: group, unit and K edges, repeated experts in any order, empty slots.  Bound as above."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    raw = orc.quantize(dt, orc.pseudo_random(n_expert * n_out * k, 0x700 + k, -1.0, 1.0))
+    stack = ExpertStack.from_bytes(raw, dt, n_expert, n_out, k, device=dev)
+    x = orc.pseudo_random(t * k, 0x35, -1.0, 1.0).reshape(t, 1, k)
+    ids = np.random.default_rng(t).integers(0, n_expert + 1, (t, top_k)).astype(np.uint32)  # n_expert: an empty slot
+    got = ops.mul_mv_id(stack, torch.from_numpy(x).to(dev), torch.from_numpy(ids.astype(np.int32)).to(dev)).cpu().numpy()
+    assert not got[ids == n_expert].any()
+    want = orc.mul_id(dt, raw, n_expert, n_out, k, x, np.minimum(ids, n_expert - 1))
+    want[ids == n_expert] = 0
+    assert orc.rel_l2(got, want) < 1e-5
+
+
 @pytest.mark.parametrize("dt,name", DTYPES)
 def test_plain_mv(orc, dev, dt, name):
     from maxuna_b200 import ops
