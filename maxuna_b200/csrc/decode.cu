@@ -214,13 +214,22 @@ __device__ __forceinline__ void unit_range_first(int n_units, int selecting, int
 // 3.6 of them per CTA, and two separate splits gave some CTAs five.  (In phase 1 the shared units pass while the routing is
 // still on its way.)  A CTA's share of all must not be smaller than its part of the shared ones, which holds from one
 // routed unit per CTA on.
-__device__ __forceinline__ void dec_unit_range_of(int sec, int n_routed1, int n_shared2, int n_routed2, int2 *r) {
-    const int n = sec == 1 ? n_routed1 : (sec == 2 ? n_shared2 : n_routed2);
-    const bool together = sec == 3 && n_routed2 >= (int)gridDim.x && n_shared2 + n_routed2 <= 16 * (int)gridDim.x;
+// The split is by cost, not by count: staging a pass's activations takes a CTA about as long as STAGE_UNITS units, so a CTA
+// whose range crosses into another pass gets that much less (3 tokens: 66.9 -> 64.3 us, 6: 95.5 -> 91.9, 16: 148 -> 145.5;
+// 64: no difference).
+constexpr int STAGE_UNITS = 2;
+__device__ __forceinline__ int unit_at(int v, int tiles) { // the real unit at position v of a section's cost line
+    const int q = v / (tiles + STAGE_UNITS), r = v - q * (tiles + STAGE_UNITS);
+    return q * tiles + max(r - STAGE_UNITS, 0);
+}
+__device__ __noinline__ int2 dec_unit_range_of(int sec, int routed, int shared, int tiles1, int tiles2) {
+    const int tiles = sec == 1 ? tiles1 : tiles2;
+    const int n_shared2 = shared * (tiles + STAGE_UNITS), n = (sec == 2 ? shared : routed) * (tiles + STAGE_UNITS);
+    const bool together = sec == 3 && n >= (int)gridDim.x && n_shared2 + n <= 16 * (int)gridDim.x;
     int a, b, c, d;
     unit_range(together ? n_shared2 + n : n, a, b);
     unit_range(together ? n_shared2 : 0, c, d);
-    r[sec] = make_int2(a - c, b - d);
+    return make_int2(unit_at(a - c, tiles), unit_at(b - d, tiles));
 }
 
 // Resolve routed pass index -> active index (the expert it belongs to).
@@ -1075,7 +1084,7 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
                 if (L.lists_alias) xkey = ~0ull; // they were built over the activation cache
             }
             if (tid >= 1 && tid < 4)
-                dec_unit_range_of(tid, s_routed_passes * tiles1, shared_passes * tiles2, s_routed_passes * tiles2, s_range);
+                s_range[tid] = dec_unit_range_of(tid, s_routed_passes, shared_passes, tiles1, tiles2);
             bar_sync(2, C::THREADS); // release the producer and the epilogue warp: the routing tables are complete
         }
         const int tiles = phase == 1 ? tiles1 : tiles2;
