@@ -199,6 +199,13 @@ lmoe_status lmoe_mul_mm_id(const lmoe_expert_stack *stack, const float *x, int64
  * src/ops/silu_mul.metal:57-72: out[i] = (g / (1 + exp(-g))) * u, the two
  * roundings kept separate. n <= INT32_MAX. */
 lmoe_status lmoe_silu_mul(const float *gate, const float *up, int64_t n, float *out, void *stream);
+
+/*
+ * The range guard of `FusedExperts::forward`, src/moe.rs:292-313, before the
+ * f16 down projection: l2[r] = clamp(||a[r]||, 1e-8, 1e30) and
+ * out[r] = a[r] * 2^15 / l2[r], rows [rows, n].
+ */
+lmoe_status lmoe_l2_rescale(const float *a, int64_t rows, int64_t n, float *out, float *l2, void *stream);
 /* `ops::combine`, src/ops/combine.rs:16 -> `run_combine`, src/ops/dispatch.rs:1366-1506
  * -> kernel_moe_combine{,_rescale}, src/ops/combine.metal:70-133:
  *   out[s, c] = sum_k down[s, k, c] * (col_l2[s, k] * 2^-15) * w[s, k]

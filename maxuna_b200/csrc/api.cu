@@ -246,6 +246,15 @@ extern "C" lmoe_status lmoe_silu_mul(const float *gate, const float *up, int64_t
     return LMOE_OK;
 }
 
+extern "C" lmoe_status lmoe_l2_rescale(const float *a, int64_t rows, int64_t n, float *out, float *l2, void *stream) {
+    lmoe_clear_error();
+    REQUIRE(a && out && l2, "a/out/l2 is NULL");
+    REQUIRE(rows >= 0 && n >= 1 && n <= INT32_MAX && rows <= INT64_MAX / 4 / n, "l2_rescale dims out of range");
+    REQUIRE((rows + 7) / 8 <= INT32_MAX, "l2_rescale rows (%lld) out of range", (long long)rows);
+    LMOE_CUDA(launch_l2_rescale(a, rows, (int)n, out, l2, (cudaStream_t)stream));
+    return LMOE_OK;
+}
+
 extern "C" lmoe_status lmoe_combine(const float *down, const float *col_l2, const float *weights, int64_t seq,
                                     int64_t top_k, int64_t n_out, float *out, void *stream) {
     lmoe_clear_error();

@@ -93,6 +93,7 @@ cudaError_t launch_mul_mv_id(int dtype, const uint8_t *w, int64_t expert_bytes, 
                              cudaStream_t s);
 // glue.cu
 cudaError_t launch_silu_mul(const float *g, const float *u, int64_t n, float *out, cudaStream_t s);
+cudaError_t launch_l2_rescale(const float *a, int64_t rows, int n, float *out, float *l2, cudaStream_t s);
 cudaError_t launch_combine(const float *down, const float *col_l2, const float *w, int seq, int top_k,
                            int n_out, float *out, cudaStream_t s);
 cudaError_t launch_add_inplace(float *out, const float *b, int64_t n, cudaStream_t s);

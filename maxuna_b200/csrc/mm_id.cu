@@ -186,8 +186,9 @@ __device__ __forceinline__ size_t tiled_off(int slot, int k_stages, int ks, int 
     return (((size_t)slot * k_stages + ks) * nt + rr) * 128 + ((size_t)(c ^ (rr & 7)) << 4);
 }
 
-// A block takes GT_ROWS rows of one row tile, one warp per row: the work is even however the rows fall to the experts.
-constexpr int GT_ROWS = 32;
+// A block takes GT_ROWS rows of one row tile, one warp per row: the work is even however the rows fall to the experts, and no
+// row waits behind another of its warp (5120 rows of 3072 in 256 tiles: 32 rows a block 25.6 us, 8 rows 12.7).
+constexpr int GT_ROWS = 8;
 template <bool XF16>
 __global__ void __launch_bounds__(256) gather_tiles_kernel(const void *__restrict__ xv, int x_per_row, int top_k, int k,
                                                            const int4 *__restrict__ tiles, const int32_t *__restrict__ n_tiles,

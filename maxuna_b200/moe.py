@@ -60,10 +60,9 @@ class FusedExperts(ExpertFfn):
         if use_mm:
             # the grouped GEMM stages the activation as f16: keep it in range with the
             # per-(token, slot) L2 rescale and undo it in the combine (src/moe.rs:292-313)
-            col_l2 = act.square().sum(2, keepdim=True).sqrt().clamp(1e-8, 1e30)
-            act_s = (act * 32768.0) / col_l2
-            down = matmul(self.down, act_s.contiguous())
-            return ops.combine(down, col_l2.contiguous(), w)
+            act_s, col_l2 = ops.l2_rescale(act)
+            down = matmul(self.down, act_s)
+            return ops.combine(down, col_l2, w)
         down = matmul(self.down, act)
         return ops.combine(down, None, w)
 
@@ -73,10 +72,12 @@ class SharedExpert:
 
     def __init__(self, gate: ExpertStack, up: ExpertStack, down: ExpertStack):
         self.gate, self.up, self.down = gate, up, down
+        # the expert index of a small batch, laid out once with the weights (a fill kernel and 6 us of host per call otherwise)
+        self._zeros = torch.zeros(64, 1, dtype=torch.int32, device=gate.buffer.device)
 
     def forward(self, x):
         seq, hidden = x.shape
-        zeros = torch.zeros(seq, 1, dtype=torch.int32, device=x.device)
+        zeros = self._zeros[:seq] if seq <= 64 else torch.zeros(seq, 1, dtype=torch.int32, device=x.device)
         xg = x.reshape(seq, 1, hidden).contiguous()
         g = ops.mul_mv_id(self.gate, xg, zeros)
         u = ops.mul_mv_id(self.up, xg, zeros)

@@ -47,6 +47,8 @@ def _require(cond, msg):
 
 
 def _f32_dev(name, t: torch.Tensor):
+    if isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float32 and t.is_contiguous():
+        return  # the messages below cost 1 us to build, a tenth of a call
     _require(isinstance(t, torch.Tensor), f"{name} must be a tensor")
     _require(t.is_cuda, f"{name} must be on a CUDA device")
     _require(t.dtype == torch.float32, f"{name} must be f32, got {t.dtype}")
@@ -54,6 +56,8 @@ def _f32_dev(name, t: torch.Tensor):
 
 
 def _ids_dev(ids: torch.Tensor):
+    if ids.is_cuda and ids.dtype == torch.int32 and ids.is_contiguous() and ids.dim() == 2:
+        return
     _require(ids.is_cuda, "ids must be on a CUDA device")
     # torch has no first-class u32 arithmetic; int32 storage carries the same bits
     _require(ids.dtype in (torch.int32, torch.uint32), f"ids must be u32, got {ids.dtype}")
@@ -82,7 +86,8 @@ def mul_mv(weight: torch.Tensor, dtype: int, n_out: int, k: int, x: torch.Tensor
     """Plain quantized mat-vec: weight = raw ``[n_out, k]`` super-blocks, x ``[t, k]`` -> ``[t, n_out]``."""
     _f32_dev("x", x)
     _require(x.dim() == 2, "x must be rank-2 [t, k]")
-    _require(x.shape[1] == k, f"x k ({x.shape[1]}) does not match weight k ({k})")
+    if x.shape[1] != k:
+        raise LmoeError(-1, f"x k ({x.shape[1]}) does not match weight k ({k})")
     _require(weight.is_cuda and weight.dtype == torch.uint8, "weight must be a CUDA uint8 buffer")
     out = torch.empty(x.shape[0], n_out, dtype=torch.float32, device=x.device)
     check(lib().lmoe_mul_mv(weight.data_ptr(), dtype, n_out, k, x.data_ptr(), x.shape[0], out.data_ptr(),
@@ -146,11 +151,22 @@ def mul_mm_id(stack: ExpertStack, x: torch.Tensor, ids: torch.Tensor) -> torch.T
 def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     _f32_dev("gate", gate)
     _f32_dev("up", up)
-    _require(gate.shape == up.shape, f"silu_mul shape mismatch: gate {tuple(gate.shape)}, up {tuple(up.shape)}")
+    if gate.shape != up.shape:
+        raise LmoeError(-1, f"silu_mul shape mismatch: gate {tuple(gate.shape)}, up {tuple(up.shape)}")
     _require(gate.device == up.device, "gate and up must be on the same device")
     out = torch.empty_like(gate)
     check(lib().lmoe_silu_mul(gate.data_ptr(), up.data_ptr(), gate.numel(), out.data_ptr(), stream_ptr()))
     return out
+
+
+def l2_rescale(a: torch.Tensor):
+    """a ``[t, top_k, n]`` -> (a * 2^15 / l2, l2 ``[t, top_k, 1]``), l2 the clamped norm of every row (src/moe.rs:292-313)."""
+    _f32_dev("a", a)
+    t, top_k, n = a.shape
+    out = torch.empty_like(a)
+    l2 = torch.empty(t, top_k, 1, dtype=torch.float32, device=a.device)
+    check(lib().lmoe_l2_rescale(a.data_ptr(), t * top_k, n, out.data_ptr(), l2.data_ptr(), stream_ptr()))
+    return out, l2
 
 
 def combine(down: torch.Tensor, col_l2, weights: torch.Tensor) -> torch.Tensor:
@@ -158,11 +174,13 @@ def combine(down: torch.Tensor, col_l2, weights: torch.Tensor) -> torch.Tensor:
     _require(down.dim() == 3, "down must be rank-3 [seq, top_k, n_out]")
     seq, top_k, n_out = down.shape
     _f32_dev("weights", weights)
-    _require(tuple(weights.shape) == (seq, top_k), f"weights shape {tuple(weights.shape)} must be [seq, top_k] = [{seq}, {top_k}]")
+    if weights.shape != (seq, top_k):
+        raise LmoeError(-1, f"weights shape {tuple(weights.shape)} must be [seq, top_k] = [{seq}, {top_k}]")
     l2p = None
     if col_l2 is not None:
         _f32_dev("col_l2", col_l2)
-        _require(tuple(col_l2.shape) == (seq, top_k, 1), f"col_l2 shape {tuple(col_l2.shape)} must be [seq, top_k, 1] = [{seq}, {top_k}, 1]")
+        if col_l2.shape != (seq, top_k, 1):
+            raise LmoeError(-1, f"col_l2 shape {tuple(col_l2.shape)} must be [seq, top_k, 1] = [{seq}, {top_k}, 1]")
         l2p = col_l2.data_ptr()
     out = torch.empty(seq, n_out, dtype=torch.float32, device=down.device)
     check(lib().lmoe_combine(down.data_ptr(), l2p, weights.data_ptr(), seq, top_k, n_out, out.data_ptr(), stream_ptr()))
@@ -175,7 +193,8 @@ def route(router: torch.Tensor, bias, x: torch.Tensor, top_k: int, scale: float 
     _f32_dev("x", x)
     _require(router.dim() == 2 and x.dim() == 2, "router must be [n_expert, hidden], x [t, hidden]")
     n_expert, hidden = router.shape
-    _require(x.shape[1] == hidden, f"x hidden ({x.shape[1]}) does not match router hidden ({hidden})")
+    if x.shape[1] != hidden:
+        raise LmoeError(-1, f"x hidden ({x.shape[1]}) does not match router hidden ({hidden})")
     t = x.shape[0]
     if bias is not None:
         _f32_dev("bias", bias)

@@ -269,6 +269,26 @@ def test_combine_and_silu_mul(orc, dev, seq):
     np.testing.assert_allclose(ops.silu_mul(td(g), td(u)).cpu().numpy(), orc.silu_mul(g, u), rtol=2e-6, atol=1e-7)
 
 
+@pytest.mark.parametrize("rows,top_k,n", [(3, 1, 97), (5, 6, 33), (2, 22, 132), (1, 64, 4)])
+def test_glue_edges(orc, dev, rows, top_k, n):
+    """Scalar and four-wide forms of combine and silu_mul, a row count off the block size, and the range guard: a zero row, and
+    both outputs within three roundings plus n/2 ulp of the sum of squares."""
+    from maxuna_b200 import ops
+
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((rows, top_k, n)).astype(np.float32)
+    a[0, 0] = 0
+    b, w = rng.standard_normal(a.shape).astype(np.float32), rng.uniform(0, 1, (rows, top_k)).astype(np.float32)
+    td = lambda v: torch.from_numpy(v).to(dev)
+    assert np.array_equal(ops.combine(td(a), None, td(w)).cpu().numpy(), orc.combine(a, None, w))
+    np.testing.assert_allclose(ops.silu_mul(td(a), td(b)).cpu().numpy(), orc.silu_mul(a, b), rtol=2e-6, atol=1e-7)
+    got, l2 = (v.cpu().numpy() for v in ops.l2_rescale(td(a)))
+    want = np.clip(np.sqrt((a.astype(np.float64) ** 2).sum(2, keepdims=True)), 1e-8, 1e30)
+    tol = (3 + n / 2) * 2.0 ** -24
+    np.testing.assert_allclose(l2, want, rtol=tol)
+    np.testing.assert_allclose(got, a * 32768.0 / want, rtol=tol)
+
+
 def test_map0_matches_oracle(orc, dev):
     from maxuna_b200 import ops
 
