@@ -234,6 +234,21 @@ def test_routing_bit_exact_vs_oracle(orc, dev, t):
     assert np.array_equal(w.cpu().numpy().view(np.uint32), w_o.view(np.uint32))  # weights bit-exact too
 
 
+@pytest.mark.parametrize("t,hidden,ne", [(65, 512, 20), (81, 2048, 130), (79, 3072, 17), (73, 4096, 70), (66, 6144, 33)])
+def test_routing_tiles_bit_exact(orc, dev, t, hidden, ne):
+    """The register-tiled router product at the edges of its token and expert tiles, in both tile shapes: same fixed summation
+    order, so ids and weights are bitwise the oracle's."""
+    from maxuna_b200 import ops
+
+    rng = np.random.default_rng(hidden)
+    router = (rng.standard_normal((ne, hidden)) * 0.02).astype(np.float32)
+    x = rng.standard_normal((t, hidden)).astype(np.float32)
+    ids, w = ops.route(torch.from_numpy(router).to(dev), None, torch.from_numpy(x).to(dev), 16)
+    ids_o, w_o = orc.route(router, None, x, 16)
+    assert np.array_equal(ids.cpu().numpy().astype(np.uint32), ids_o)
+    assert np.array_equal(w.cpu().numpy().view(np.uint32), w_o.view(np.uint32))
+
+
 def test_routing_odd_hidden_and_ties(orc, dev):
     from maxuna_b200 import ops
 
