@@ -14,6 +14,7 @@ __device__ __forceinline__ float silu_mul(float a, float u) {
 template <bool VEC>
 __global__ void silu_mul_kernel(const float *__restrict__ g, const float *__restrict__ u, int64_t n,
                                 float *__restrict__ out) {
+    pdl_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (VEC) {
@@ -29,6 +30,7 @@ __global__ void silu_mul_kernel(const float *__restrict__ g, const float *__rest
 // as six element-wise steps 47.
 __global__ void __launch_bounds__(256) l2_rescale_kernel(const float *__restrict__ a, int64_t rows, int n, float *__restrict__ out,
                                                          float *__restrict__ l2) {
+    pdl_begin();
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -46,6 +48,7 @@ __global__ void __launch_bounds__(256) l2_rescale_kernel(const float *__restrict
 }
 
 __global__ void add_inplace_kernel(float *__restrict__ out, const float *__restrict__ b, int64_t n) {
+    pdl_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = __fadd_rn(out[i], b[i]);
 }
@@ -56,6 +59,7 @@ template <int W, int V>
 __global__ void combine_kernel(const float *__restrict__ down, const float *__restrict__ col_l2,
                                const float *__restrict__ w, int seq, int top_k, int n_out,
                                float *__restrict__ out) {
+    pdl_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int nv = n_out / V;
     if (i >= (int64_t)seq * nv) return;
@@ -101,6 +105,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(256)
 map0_kernel(const uint32_t *__restrict__ ids, int t, int top_k, int n_expert, uint32_t *__restrict__ tpe,
             int32_t *__restrict__ ids_map) {
+    pdl_begin();
     __shared__ int warp_count[8];
     __shared__ int base;
     const int e = blockIdx.x;
@@ -172,6 +177,7 @@ map0_kernel(const uint32_t *__restrict__ ids, int t, int top_k, int n_expert, ui
 // router input - and with it the expert selection - does not depend on the launch geometry.
 __global__ void __launch_bounds__(256) rms_norm_kernel(const float *__restrict__ x, const float *__restrict__ w, float eps,
                                                        int t, int hidden, float *__restrict__ out) {
+    pdl_begin();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= t) return;
@@ -203,7 +209,7 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(const float *__restrict__
 
 cudaError_t launch_rms_norm(const float *x, const float *w, float eps, int64_t t, int hidden, float *out, cudaStream_t s) {
     if (t == 0) return cudaSuccess;
-    rms_norm_kernel<<<(unsigned)((t + 7) / 8), 256, 0, s>>>(x, w, eps, (int)t, hidden, out);
+    launch_pdl(rms_norm_kernel, (unsigned)((t + 7) / 8), 256, 0, s, x, w, eps, (int)t, hidden, out);
     return cudaGetLastError();
 }
 
@@ -213,20 +219,20 @@ static bool aligned16_all(const void *a, const void *b, const void *c) {
 
 cudaError_t launch_silu_mul(const float *g, const float *u, int64_t n, float *out, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    if (n % 4 == 0 && aligned16_all(g, u, out)) silu_mul_kernel<true><<<(unsigned)((n / 4 + 255) / 256), 256, 0, s>>>(g, u, n / 4, out);
-    else silu_mul_kernel<false><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, u, n, out);
+    if (n % 4 == 0 && aligned16_all(g, u, out)) launch_pdl(silu_mul_kernel<true>, (unsigned)((n / 4 + 255) / 256), 256, 0, s, g, u, n / 4, out);
+    else launch_pdl(silu_mul_kernel<false>, (unsigned)((n + 255) / 256), 256, 0, s, g, u, n, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_l2_rescale(const float *a, int64_t rows, int n, float *out, float *l2, cudaStream_t s) {
     if (rows == 0) return cudaSuccess;
-    l2_rescale_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(a, rows, n, out, l2);
+    launch_pdl(l2_rescale_kernel, (unsigned)((rows + 7) / 8), 256, 0, s, a, rows, n, out, l2);
     return cudaGetLastError();
 }
 
 cudaError_t launch_add_inplace(float *out, const float *b, int64_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    add_inplace_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, b, n);
+    launch_pdl(add_inplace_kernel, (unsigned)((n + 255) / 256), 256, 0, s, out, b, n);
     return cudaGetLastError();
 }
 
@@ -234,9 +240,9 @@ template <int W>
 static void combine_launch(const float *down, const float *col_l2, const float *w, int seq, int top_k, int n_out, float *out, cudaStream_t s) {
     const int64_t n = (int64_t)seq * n_out;
     if (n_out % 4 == 0 && aligned16_all(down, out, nullptr))
-        combine_kernel<W, 4><<<(unsigned)((n / 4 + 127) / 128), 128, 0, s>>>(down, col_l2, w, seq, top_k, n_out, out);
+        launch_pdl(combine_kernel<W, 4>, (unsigned)((n / 4 + 127) / 128), 128, 0, s, down, col_l2, w, seq, top_k, n_out, out);
     else
-        combine_kernel<W, 1><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(down, col_l2, w, seq, top_k, n_out, out);
+        launch_pdl(combine_kernel<W, 1>, (unsigned)((n + 255) / 256), 256, 0, s, down, col_l2, w, seq, top_k, n_out, out);
 }
 
 cudaError_t launch_combine(const float *down, const float *col_l2, const float *w, int seq, int top_k,
@@ -259,9 +265,9 @@ cudaError_t launch_map0(const uint32_t *ids, int t, int top_k, int n_expert, uin
                         cudaStream_t s) {
     if (n_expert == 0) return cudaSuccess;
     if (t % 4 == 0 && (reinterpret_cast<uintptr_t>(ids) & 15u) == 0)
-        map0_kernel<true><<<n_expert, 256, 0, s>>>(ids, t, top_k, n_expert, tpe, ids_map);
+        launch_pdl(map0_kernel<true>, n_expert, 256, 0, s, ids, t, top_k, n_expert, tpe, ids_map);
     else
-        map0_kernel<false><<<n_expert, 256, 0, s>>>(ids, t, top_k, n_expert, tpe, ids_map);
+        launch_pdl(map0_kernel<false>, n_expert, 256, 0, s, ids, t, top_k, n_expert, tpe, ids_map);
     return cudaGetLastError();
 }
 

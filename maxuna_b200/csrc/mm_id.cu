@@ -146,6 +146,7 @@ __device__ __forceinline__ uint32_t h2_sub_mul(uint32_t v, uint32_t base, uint32
 // With `extra` > 0 one more list follows the experts' ("expert" n_expert): the rows 0 .. extra-1 of the shared expert.
 __global__ void __launch_bounds__(1024) row_tiles_kernel(const uint32_t *__restrict__ tpe, int n_expert, int extra, int nt,
                                                          int4 *__restrict__ tiles, int32_t *__restrict__ n_tiles, int max_tiles) {
+    pdl_begin();
     __shared__ int2 warp_sum[32];
     const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
     const int rows = e < n_expert ? (int)tpe[e] : (e == n_expert ? extra : 0);
@@ -196,6 +197,7 @@ __global__ void __launch_bounds__(256) gather_tiles_kernel(const void *__restric
                                                            int routed_rows, int nt, uint8_t *__restrict__ xt,
                                                            int32_t *__restrict__ pos, int32_t *__restrict__ spos,
                                                            int32_t *__restrict__ sfid) {
+    pdl_begin();
     const int slot = blockIdx.x;
     if (slot >= *n_tiles) return;
     const int4 T = tiles[slot];
@@ -241,6 +243,7 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict_
                                                          const int32_t *__restrict__ ids_map, int map_stride, int n_expert,
                                                          int routed_rows, int nt, uint8_t *__restrict__ xh, int32_t *__restrict__ src,
                                                          int32_t *__restrict__ pos, int32_t *__restrict__ spos, int32_t *__restrict__ sfid) {
+    pdl_begin();
     if ((int)blockIdx.x < convert_blocks) {
         const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
         if (i >= x_chunks) return;
@@ -891,14 +894,14 @@ lmoe_status launch_gather_tiles(const MmRows &R, const void *x, int x_f16, int x
     if (R.n_expert > 512) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "grouped GEMM supports at most 512 experts");
     int4 *tiles = static_cast<int4 *>(tiles_ws);
     int32_t *n_tiles = mm_tile_count(R, tiles_ws);
-    row_tiles_kernel<<<1, 1024, 0, s>>>(tpe, R.n_expert, (int)R.extra, R.nt, tiles, n_tiles, (int)R.max_tiles);
+    launch_pdl(row_tiles_kernel, 1, 1024, 0, s, tpe, R.n_expert, (int)R.extra, R.nt, tiles, n_tiles, (int)R.max_tiles);
     LMOE_LAUNCH_CHECK("row_tiles_kernel");
     const dim3 grid((unsigned)R.max_tiles, (unsigned)((R.nt + GT_ROWS - 1) / GT_ROWS));
     if (x_f16)
-        gather_tiles_kernel<true><<<grid, 256, 0, s>>>(x, x_per_row, top_k, k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
+        launch_pdl(gather_tiles_kernel<true>, grid, 256, 0, s, x, x_per_row, top_k, k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
                                                        (int)R.rows, R.nt, static_cast<uint8_t *>(xt), pos, spos, sfid);
     else
-        gather_tiles_kernel<false><<<grid, 256, 0, s>>>(x, x_per_row, top_k, k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
+        launch_pdl(gather_tiles_kernel<false>, grid, 256, 0, s, x, x_per_row, top_k, k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
                                                         (int)R.rows, R.nt, static_cast<uint8_t *>(xt), pos, spos, sfid);
     LMOE_LAUNCH_CHECK("gather_tiles_kernel");
     return LMOE_OK;
@@ -912,16 +915,16 @@ lmoe_status launch_stage_rows(const MmRows &R, const void *x, int x_f16, int64_t
     if (R.n_expert > 512) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "grouped GEMM supports at most 512 experts");
     int4 *tiles = static_cast<int4 *>(tiles_ws);
     int32_t *n_tiles = mm_tile_count(R, tiles_ws);
-    row_tiles_kernel<<<1, 1024, 0, s>>>(tpe, R.n_expert, (int)R.extra, R.nt, tiles, n_tiles, (int)R.max_tiles);
+    launch_pdl(row_tiles_kernel, 1, 1024, 0, s, tpe, R.n_expert, (int)R.extra, R.nt, tiles, n_tiles, (int)R.max_tiles);
     LMOE_LAUNCH_CHECK("row_tiles_kernel");
     const int64_t chunks = x_rows * (k / 8);
     const int conv = (int)((chunks + 255) / 256);
     const unsigned grid = (unsigned)(conv + R.max_tiles);
     if (x_f16)
-        stage_rows_kernel<true><<<grid, 256, 0, s>>>(x, chunks, conv, top_k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
+        launch_pdl(stage_rows_kernel<true>, grid, 256, 0, s, x, chunks, conv, top_k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
                                                      (int)R.rows, R.nt, static_cast<uint8_t *>(xh), src, pos, spos, sfid);
     else
-        stage_rows_kernel<false><<<grid, 256, 0, s>>>(x, chunks, conv, top_k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
+        launch_pdl(stage_rows_kernel<false>, grid, 256, 0, s, x, chunks, conv, top_k, tiles, n_tiles, ids_map, (int)map_stride, R.n_expert,
                                                       (int)R.rows, R.nt, static_cast<uint8_t *>(xh), src, pos, spos, sfid);
     LMOE_LAUNCH_CHECK("stage_rows_kernel");
     return LMOE_OK;

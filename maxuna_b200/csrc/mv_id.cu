@@ -222,6 +222,7 @@ template <int DT>
 __global__ void __launch_bounds__(MV_THREADS, 2)
 mv_pair_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *__restrict__ x,
                int x_per_row, const uint32_t *__restrict__ ids, int top_k, float *__restrict__ out) {
+    pdl_begin();
     constexpr int SUB = DT == LMOE_Q4_K ? 32 : 16, NS = QK_K / SUB;
     constexpr int TS = DT == LMOE_Q4_K ? Q4K_BYTES : Q6K_BYTES;
     extern __shared__ __align__(16) uint8_t mv_smem[];
@@ -310,6 +311,7 @@ template <int DT>
 __global__ void __launch_bounds__(MV_THREADS, 2)
 mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__restrict__ x, int x_per_row,
                 const uint32_t *__restrict__ ids, int top_k, int pairs, float *__restrict__ out) {
+    pdl_begin();
     constexpr int SUB = DT == LMOE_Q4_K ? 32 : 16, NS = QK_K / SUB, BC = MM_KC / QK_K;
     constexpr int TS = DT == LMOE_Q4_K ? Q4K_BYTES : Q6K_BYTES;
     constexpr int SP = BC * NS + 8; // f16 sums of a pair and part, padded
@@ -621,6 +623,7 @@ template <int DT, int NT, int NG, bool ODD>
 __global__ void __launch_bounds__(32 * (NG * MX_GW + 1), NG == 2 ? 2 : 1)
 mv_expert_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *__restrict__ x,
                  int x_per_row, const uint32_t *__restrict__ ids, int top_k, int n_pairs, int smem_max, float *__restrict__ out) {
+    pdl_begin();
     constexpr int SUB = DT == LMOE_Q4_K ? 32 : 16, NS = QK_K / SUB, NP = 2 * NT, CONS_WARPS = NG * MX_GW;
     extern __shared__ __align__(128) uint8_t mx_smem[];
     __shared__ int pairs_s[NP], np_s;
@@ -744,7 +747,7 @@ cudaError_t launch_mv_expert(const uint8_t *w, int64_t expert_bytes, int n_exper
             const int64_t cost = (groups * g + slots - 1) / slots * (3 + (units + g - 1) / g);
             if (cost < best) best = cost, gx = g;
         }
-        mv_expert_kernel<DT, NT, NG, ODD><<<dim3((unsigned)gx, (unsigned)n), 32 * (NG * MX_GW + 1), L.total, s>>>(
+        launch_pdl(mv_expert_kernel<DT, NT, NG, ODD>, dim3((unsigned)gx, (unsigned)n), 32 * (NG * MX_GW + 1), L.total, s, 
             w, expert_bytes, n_expert, n_out, k, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k, (int)n,
             smem_max, out + (size_t)p * n_out);
     }
@@ -793,7 +796,7 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
         const int64_t step = (int64_t)65535 * MM_COLS / top_k * top_k;
         for (int64_t p = 0; p < pairs; p += step) {
             const int64_t n = pairs - p < step ? pairs - p : step;
-            mv_multi_kernel<DT><<<dim3(gx, (unsigned)((n + MM_COLS - 1) / MM_COLS)), MV_THREADS, smem, s>>>(
+            launch_pdl(mv_multi_kernel<DT>, dim3(gx, (unsigned)((n + MM_COLS - 1) / MM_COLS)), MV_THREADS, smem, s, 
                 w, n_out, k, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k, (int)n, out + (size_t)p * n_out);
         }
         return cudaGetLastError();
@@ -810,7 +813,7 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
     const int64_t step = 65535 / top_k * top_k;
     for (int64_t p = 0; p < pairs; p += step) {
         const int64_t n = pairs - p < step ? pairs - p : step;
-        mv_pair_kernel<DT><<<dim3(gx, (unsigned)n), MV_THREADS, smem_pair, s>>>(w, expert_bytes, n_expert, n_out, k,
+        launch_pdl(mv_pair_kernel<DT>, dim3(gx, (unsigned)n), MV_THREADS, smem_pair, s, w, expert_bytes, n_expert, n_out, k,
                                                                                 x + (size_t)(p / top_k) * x_per_row * k, x_per_row,
                                                                                 ids ? ids + p : nullptr, top_k, out + (size_t)p * n_out);
     }

@@ -400,9 +400,9 @@ lmoe_status launch_moe_prefill(const lmoe_layer *L, const float *x, const float 
     float *w = c.take<float>((size_t)rows);
     uint8_t *ex_ws = static_cast<uint8_t *>(workspace) + c.off;
 
-    LMOE_CUDA(cudaMemsetAsync(flag, 0, 16, s)); // a fresh device flag: the workspace needs no initialisation
     LMOE_CUDA(launch_route_logits(L->router, x, (int)t, (int)H, (int)L->n_expert, logits, s));
-    LMOE_CUDA(launch_route_select(logits, L->bias, (int)t, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, ids, w, s));
+    LMOE_CUDA(launch_route_select(logits, L->bias, (int)t, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, ids, w, s,
+                                  flag)); // a fresh device flag: the workspace needs no initialisation
     lmoe_status st = experts_prefill(L, x, 0, ids, w, t, L->top_k, 0, 1, residual, out, ex_ws, flag, s);
     if (st) return st;
     if (ids_out) LMOE_CUDA(cudaMemcpyAsync(ids_out, ids, (size_t)rows * 4, cudaMemcpyDeviceToDevice, s));

@@ -14,6 +14,7 @@ template <int TT>
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
 route_logits_kernel(const float *__restrict__ router, const float *__restrict__ x, int t, int hidden,
                     int n_expert, float *__restrict__ logits) {
+    pdl_begin();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int e = blockIdx.x * ROUTE_WARPS + warp;
     const int t0 = blockIdx.y * TT;
@@ -101,6 +102,7 @@ template <int T>
 __global__ void __launch_bounds__(RT_THREADS, 1)
 route_logits_tiled_kernel(const float *__restrict__ router, const float *__restrict__ x, int t, int hidden, int n_expert,
                           int experts_per_block, float *__restrict__ logits) {
+    pdl_begin();
     constexpr int TG = T / 8, EG = 4 / TG; // token and expert groups of the four sets
     typedef unsigned long long u64;
     extern __shared__ __align__(16) uint8_t rt_smem[];
@@ -201,10 +203,13 @@ route_logits_tiled_kernel(const float *__restrict__ router, const float *__restr
     }
 }
 
-// One warp per token; scores staged in shared memory (2 * n_expert floats per warp).
+// One warp per token; scores staged in shared memory (2 * n_expert floats per warp).  clear: four words to set to zero (a
+// call's device flag, which otherwise takes a launch of its own), or NULL.
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
 route_select_kernel(const float *__restrict__ logits, const float *__restrict__ bias, int t, int n_expert,
-                    int top_k, float scale, int norm, uint32_t *__restrict__ ids, float *__restrict__ weights) {
+                    int top_k, float scale, int norm, uint32_t *__restrict__ ids, float *__restrict__ weights, uint32_t *__restrict__ clear) {
+    pdl_begin();
+    if (clear && blockIdx.x == 0 && threadIdx.x < 4) clear[threadIdx.x] = 0u;
     extern __shared__ float smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int token = blockIdx.x * ROUTE_WARPS + warp;
@@ -257,24 +262,24 @@ cudaError_t launch_route_logits(const float *router, const float *x, int t, int 
         const dim3 grid((unsigned)((t + nt - 1) / nt), (unsigned)((n_expert + pass * ppb - 1) / (pass * ppb)));
         const int smem = nt * hidden * 4 + RT_FOLD;
         if (nt == 16)
-            route_logits_tiled_kernel<16><<<grid, RT_THREADS, smem, s>>>(router, x, t, hidden, n_expert, ppb * pass, logits);
+            launch_pdl(route_logits_tiled_kernel<16>, grid, RT_THREADS, smem, s, router, x, t, hidden, n_expert, ppb * pass, logits);
         else
-            route_logits_tiled_kernel<8><<<grid, RT_THREADS, smem, s>>>(router, x, t, hidden, n_expert, ppb * pass, logits);
+            launch_pdl(route_logits_tiled_kernel<8>, grid, RT_THREADS, smem, s, router, x, t, hidden, n_expert, ppb * pass, logits);
     } else if (t <= 2) {
-        route_logits_kernel<1><<<dim3(gx, t), ROUTE_WARPS * 32, 0, s>>>(router, x, t, hidden, n_expert, logits);
+        launch_pdl(route_logits_kernel<1>, dim3(gx, t), ROUTE_WARPS * 32, 0, s, router, x, t, hidden, n_expert, logits);
     } else {
-        route_logits_kernel<4><<<dim3(gx, (t + 3) / 4), ROUTE_WARPS * 32, 0, s>>>(router, x, t, hidden, n_expert, logits);
+        launch_pdl(route_logits_kernel<4>, dim3(gx, (t + 3) / 4), ROUTE_WARPS * 32, 0, s, router, x, t, hidden, n_expert, logits);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_route_select(const float *logits, const float *bias, int t, int n_expert, int top_k,
-                                float scale, int norm, uint32_t *ids, float *weights, cudaStream_t s) {
+                                float scale, int norm, uint32_t *ids, float *weights, cudaStream_t s, uint32_t *clear) {
     if (t == 0) return cudaSuccess;
     const size_t smem = (size_t)ROUTE_WARPS * 2 * n_expert * sizeof(float);
     const unsigned grid = (unsigned)((t + ROUTE_WARPS - 1) / ROUTE_WARPS);
-    route_select_kernel<<<grid, ROUTE_WARPS * 32, smem, s>>>(logits, bias, t, n_expert, top_k, scale, norm, ids,
-                                                             weights);
+    launch_pdl(route_select_kernel, grid, ROUTE_WARPS * 32, smem, s, logits, bias, t, n_expert, top_k, scale, norm, ids,
+                                                             weights, clear);
     return cudaGetLastError();
 }
 
