@@ -13,7 +13,8 @@
 //   mv_pair_kernel   any shape, one (token, slot) pair per block row; what is left to it are rows too long for the ring and
 //                    matrices off a 16-byte boundary.  Weights go straight from global memory into the A fragments.
 //   mv_multi_kernel  many pairs of ONE weight matrix (the shared expert, a plain matrix): eight pairs are the columns of
-//                    an MMA, so a super-block is unpacked once for 32 pairs.  512 pairs of [1024 x 3072] Q4_K: 830 -> 70 us.
+//                    an MMA, so a super-block is unpacked once for 32 pairs.  512 pairs of [1024 x 3072] Q4_K: 830 -> 52 us.
+#include <cooperative_groups.h>
 #include "common.cuh"
 #include "stream_math.cuh"
 
@@ -302,13 +303,15 @@ mv_pair_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert
 }
 
 // ---- many pairs of one matrix -----------------------------------------------------------
-// grid (ceil(n_out / 64), ceil(pairs / 32)); the same warp layout.  The digits of 32 pairs are staged 1024 k at a time.
+// grid (ceil(n_out / 64), ceil(pairs / 32)); the same warp layout.  The digits of 32 pairs are staged 1024 k at a time.  Making
+// them was half of the instructions, so the CS blocks of a cluster, row blocks of the same pairs, make a share each and store
+// it to all of them through distributed shared memory (512 pairs: CLNOW).
 constexpr int MM_COLS = 32, MM_KC = 1024;
 // bytes of a pair's digits: the columns of one load instruction (8 bytes a lane for Q4_K, 4 for Q6_K) cover distinct banks
 template <int DT>
 constexpr int MM_PITCH = MV_NDIG * MM_KC + (DT == LMOE_Q4_K ? 32 : 16);
-template <int DT>
-__global__ void __launch_bounds__(MV_THREADS, 2)
+template <int DT, int CS>
+__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(MV_THREADS, 2)
 mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__restrict__ x, int x_per_row,
                 const uint32_t *__restrict__ ids, int top_k, int pairs, float *__restrict__ out) {
     pdl_begin();
@@ -325,6 +328,13 @@ mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
     const int r_base = blockIdx.x * MV_ROWS, rt = warp & 3, ks = warp >> 2;
     const int rg = min(r_base + 16 * rt + g, n_out - 1), rG = min(r_base + 16 * rt + g + 8, n_out - 1);
     const uint8_t *pg = w + (size_t)rg * row_bytes, *pG = w + (size_t)rG * row_bytes;
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cl = cg::this_cluster();
+    const int rank = CS > 1 ? (int)cl.block_rank() : 0;
+    auto sync_all = [&]() {
+        if (CS > 1) cl.sync();
+        else __syncthreads();
+    };
     float acc[MM_COLS / 8][4];
 #pragma unroll
     for (int c = 0; c < MM_COLS / 8; c++)
@@ -334,8 +344,8 @@ mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
         const int bn = min(BC, nb - b0);
         typename MvRaw<DT>::T raw;
         if (ks < bn) raw.load(pg + (size_t)(b0 + ks) * TS, pG + (size_t)(b0 + ks) * TS, t);
-        __syncthreads(); // the previous chunk's digits have been read
-        for (int i = warp; i < np * bn; i += MV_THREADS / 32) {
+        sync_all(); // the previous chunk's digits have been read
+        for (int i = rank * (MV_THREADS / 32) + warp; i < np * bn; i += CS * (MV_THREADS / 32)) {
             const int p = i / bn, b = i - p * bn, pair = p0 + p;
             MvX in;
             in.load(x + ((size_t)(pair / top_k) * x_per_row + (x_per_row == 1 ? 0 : pair % top_k)) * k + (size_t)(b0 + b) * QK_K,
@@ -345,14 +355,20 @@ mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
             __half hi, lo;
             mv_digits<SUB>(in, dig, sx, hi, lo);
 #pragma unroll
-            for (int d = 0; d < MV_NDIG; d++) *reinterpret_cast<uint2 *>(xc + p * MM_PITCH<DT> + d * MM_KC + b * QK_K + lane * 8) = dig[d];
-            if ((lane & (SUB / 8 - 1)) == 0) {
-                sh[p * SP + b * NS + lane / (SUB / 8)] = hi;
-                sh[(MM_COLS + p) * SP + b * NS + lane / (SUB / 8)] = lo;
+            for (int r = 0; r < CS; r++) {
+                int8_t *xr = CS > 1 ? cl.map_shared_rank(xc, r) : xc;
+                __half *hr = CS > 1 ? cl.map_shared_rank(sh, r) : sh;
+                float *fr = CS > 1 ? cl.map_shared_rank(sxs, r) : sxs;
+#pragma unroll
+                for (int d = 0; d < MV_NDIG; d++) *reinterpret_cast<uint2 *>(xr + p * MM_PITCH<DT> + d * MM_KC + b * QK_K + lane * 8) = dig[d];
+                if ((lane & (SUB / 8 - 1)) == 0) {
+                    hr[p * SP + b * NS + lane / (SUB / 8)] = hi;
+                    hr[(MM_COLS + p) * SP + b * NS + lane / (SUB / 8)] = lo;
+                }
+                if (lane == 0) fr[b * MM_COLS + p] = sx;
             }
-            if (lane == 0) sxs[b * MM_COLS + p] = sx;
         }
-        __syncthreads();
+        sync_all();
         for (int b = ks; b < bn; b += 2) {
             MvA<DT> A;
             A.unpack(raw, t);
@@ -747,7 +763,7 @@ cudaError_t launch_mv_expert(const uint8_t *w, int64_t expert_bytes, int n_exper
             const int64_t cost = (groups * g + slots - 1) / slots * (3 + (units + g - 1) / g);
             if (cost < best) best = cost, gx = g;
         }
-        launch_pdl(mv_expert_kernel<DT, NT, NG, ODD>, dim3((unsigned)gx, (unsigned)n), 32 * (NG * MX_GW + 1), L.total, s, 
+        launch_pdl(mv_expert_kernel<DT, NT, NG, ODD>, dim3((unsigned)gx, (unsigned)n), 32 * (NG * MX_GW + 1), L.total, s,
             w, expert_bytes, n_expert, n_out, k, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k, (int)n,
             smem_max, out + (size_t)p * n_out);
     }
@@ -783,21 +799,26 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
         sms_dev = dev;
     }
     // One matrix for all pairs: 32 pairs to an unpacked super-block, once such blocks cover every SM.  (Below that two pairs to a
-    // block win by parallelism: [1024 x 3072] Q4_K, 64 / 512 pairs 26 / 88 us against 55 / 70, [3072 x 1024] Q6_K, 32 / 128
-    // pairs 16 / 42 against 27 / 38.)
+    // block win by parallelism: [1024 x 3072] Q4_K, 64 / 512 pairs 26 / 88 us against 55 / 52, [3072 x 1024] Q6_K, 32 / 128
+    // pairs 16 / 42 against 27 / 33.)
     if (n_expert == 1 && (pairs + MM_COLS - 1) / MM_COLS * gx >= sms && pairs > 4) {
         constexpr int smem = MM_COLS * MM_PITCH<DT> + 2 * MM_COLS * (MM_KC / QK_K * NS + 8) * 2 + (MM_KC / QK_K) * MM_COLS * 4;
+        constexpr int CS = 4;
         static thread_local int c_dev = -1;
         if (dev != c_dev) {
-            if ((e = cudaFuncSetAttribute(mv_multi_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+            if ((e = cudaFuncSetAttribute(mv_multi_kernel<DT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+            if ((e = cudaFuncSetAttribute(mv_multi_kernel<DT, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
             c_dev = dev;
         }
+        // clusters where the row blocks that fill up the last one are few (they only make digits)
+        const bool cluster = gx % CS == 0 || gx >= 4 * CS;
         // grid.y is limited to 65535 groups
         const int64_t step = (int64_t)65535 * MM_COLS / top_k * top_k;
         for (int64_t p = 0; p < pairs; p += step) {
             const int64_t n = pairs - p < step ? pairs - p : step;
-            launch_pdl(mv_multi_kernel<DT>, dim3(gx, (unsigned)((n + MM_COLS - 1) / MM_COLS)), MV_THREADS, smem, s, 
-                w, n_out, k, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k, (int)n, out + (size_t)p * n_out);
+            launch_pdl(cluster ? mv_multi_kernel<DT, CS> : mv_multi_kernel<DT, 1>,
+                       dim3(cluster ? (gx + CS - 1) / CS * CS : gx, (unsigned)((n + MM_COLS - 1) / MM_COLS)), MV_THREADS, smem, s, w, n_out, k,
+                       x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k, (int)n, out + (size_t)p * n_out);
         }
         return cudaGetLastError();
     }
