@@ -305,7 +305,8 @@ mv_pair_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert
 // ---- many pairs of one matrix -----------------------------------------------------------
 // grid (ceil(n_out / 64), ceil(pairs / 32)); the same warp layout.  The digits of 32 pairs are staged 1024 k at a time.  Making
 // them was half of the instructions, so the CS blocks of a cluster, row blocks of the same pairs, make a share each and store
-// it to all of them through distributed shared memory (512 pairs: CLNOW).
+// it to all of them through distributed shared memory (512 pairs: [1024 x 3072] Q4_K 70 -> 52 us,
+// [3072 x 1024] Q6_K 102 -> 90).
 constexpr int MM_COLS = 32, MM_KC = 1024;
 // bytes of a pair's digits: the columns of one load instruction (8 bytes a lane for Q4_K, 4 for Q6_K) cover distinct banks
 template <int DT>

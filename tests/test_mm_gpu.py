@@ -59,6 +59,17 @@ def test_mm_ragged_rows_multi_block_k_and_big_expert(orc, dev, dt, name):
     assert orc.rel_l2(got, want) < 1e-3
 
 
+@pytest.mark.parametrize("dt,name", DTYPES)
+@pytest.mark.parametrize("t,n_out,k", [(80, 128, 256), (82, 130, 1280), (257, 124, 512)])
+def test_mm_tile_shapes(orc, dev, dt, name, t, n_out, k):
+    """Both row-tile widths on either side of their rule (40 and 41 rows an expert), a row past a tile, row counts of the matrix
+    that are no multiple of the copy's eight rows or of four, more than four super-blocks.  Both operands are rounded to f16
+    (2^-11 each), sums are f32: well under 1e-3."""
+    ids = (np.arange(t, dtype=np.uint32) % 2)[:, None]
+    got, want = _case(orc, dev, dt, 2, n_out, k, t, 1, 1, ids, 0x90 + t)
+    assert orc.rel_l2(got, want) < 1e-3
+
+
 def test_mm_shared_map0_bitwise_equals_self_contained(orc, dev):
     ids = orc.distinct_ids(96, 4, 8, 0x61)
     a, _ = _case(orc, dev, 12, 8, 64, 512, 96, 4, 1, ids, 0x62, shared_map=False)

@@ -148,6 +148,27 @@ def test_mv_pairs_by_expert(orc, dev, dt, name, n_expert, n_out, k, t, top_k):
     assert orc.rel_l2(got, want) < 1e-5
 
 
+@pytest.mark.parametrize("n_out,k,pairs", [
+    (72, 256, 2369),    # row blocks by themselves, one pair in the last group
+    (256, 1280, 1185),  # one whole cluster of row blocks, a second staged run of k
+    (1100, 512, 285),   # the last cluster has blocks without rows
+])
+@pytest.mark.parametrize("dt,name", DTYPES)
+def test_mv_many_pairs_of_one_matrix(orc, dev, dt, name, n_out, k, pairs):
+    """The many-pair form at the edges of its row blocks, clusters and pair groups, and empty slots.  Bound as above."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    raw = orc.quantize(dt, orc.pseudo_random(n_out * k, 0x500 + k, -1.0, 1.0))
+    stack = ExpertStack.from_bytes(raw, dt, 1, n_out, k, device=dev)
+    x = orc.pseudo_random(pairs * k, 0x36, -1.0, 1.0).reshape(pairs, 1, k)
+    ids = (np.arange(pairs, dtype=np.uint32) % 7 == 3).astype(np.uint32)[:, None]  # 1: an empty slot
+    got = ops.mul_mv_id(stack, torch.from_numpy(x).to(dev), torch.from_numpy(ids.astype(np.int32)).to(dev)).cpu().numpy()
+    want = orc.mul_id(dt, raw, 1, n_out, k, x, np.zeros_like(ids))
+    want[ids == 1] = 0
+    assert not got[ids == 1].any() and orc.rel_l2(got, want) < 1e-5
+
+
 @pytest.mark.parametrize("dt,name", DTYPES)
 def test_plain_mv(orc, dev, dt, name):
     from maxuna_b200 import ops
