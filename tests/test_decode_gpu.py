@@ -50,6 +50,28 @@ def test_decode_two_blocks_per_row_and_repeatability(orc, dev):
     assert torch.equal(a, b)  # deterministic: fixed-order combine, no float atomics
 
 
+@pytest.mark.parametrize("hidden,ff,ne,k,ts", [
+    (512, 512, 5, 4, (1, 8, 9, 64)),       # two super-blocks a row; lists of 32 pairs and of 36
+    (768, 1024, 130, 6, (5, 6, 43)),       # expert count off four; four super-blocks in straight line; 256 pairs and more
+    (256, 1280, 33, 32, (1, 2, 9)),        # five super-blocks; 32 pairs of one token
+    (1024, 768, 12, 1, (2, 33)),           # three: rows of odd word alignment; one expert a token
+])
+def test_decode_list_and_row_forms(orc, dev, hidden, ff, ne, k, ts):
+    """The forms of the list build (by one warp, by the block, over the activation cache) and of the down units, with experts
+    that tie in every score: routing exact, output within the 21- and 15-bit activations' error."""
+    from maxuna_b200.moe import MoeBlock
+
+    blk = MoeBlock.random(hidden, ff, ne, k, seed=17, device=dev, weight_std=0.1)
+    blk.router[1] = blk.router[0]
+    blk.router[ne - 1] = blk.router[2]
+    blk.exp_probs_b[1], blk.exp_probs_b[ne - 1] = blk.exp_probs_b[0].item(), blk.exp_probs_b[2].item()
+    host = blk.host_layer(orc)
+    rng = np.random.default_rng(18)
+    for t in ts:
+        x = rng.standard_normal((t, hidden)).astype(np.float32)
+        _check(orc, blk, host, x, 1e-4 if t <= 8 else 5e-4)
+
+
 @pytest.fixture(scope="module")
 def full_block(dev):
     from maxuna_b200.moe import MoeBlock
