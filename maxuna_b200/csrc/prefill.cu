@@ -391,6 +391,7 @@ lmoe_status launch_moe_prefill(const lmoe_layer *L, const float *x, const float 
     if (!workspace || workspace_bytes < prefill_workspace_bytes(L, t))
         return lmoe_fail(LMOE_ERR_WORKSPACE, "prefill workspace needs %zu bytes, got %zu", prefill_workspace_bytes(L, t),
                          workspace_bytes);
+    if (L->n_expert > 512) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "grouped GEMM supports at most 512 experts");
     if (t * L->top_k > INT32_MAX / 2) return lmoe_fail(LMOE_ERR_INVALID, "too many routed rows");
     const int64_t rows = t * L->top_k, H = L->hidden;
     Carver c{static_cast<uint8_t *>(workspace), 65536};

@@ -7,18 +7,20 @@
 namespace {
 
 constexpr int ROUTE_WARPS = 8;
+constexpr int LOGIT_WARPS = 2; // few blocks are what a small batch has: 256 experts on 128 SMs instead of 32
 
-// grid (ceil(n_expert / ROUTE_WARPS), ceil(t / TT)); one warp per expert row,
+// grid (ceil(n_expert / LOGIT_WARPS), ceil(t / TT)); one warp per expert row,
 // TT tokens per pass so the router row is read once per token tile.
 template <int TT>
-__global__ void __launch_bounds__(ROUTE_WARPS * 32)
+__global__ void __launch_bounds__(LOGIT_WARPS * 32)
 route_logits_kernel(const float *__restrict__ router, const float *__restrict__ x, int t, int hidden,
                     int n_expert, float *__restrict__ logits) {
     pdl_begin();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int e = blockIdx.x * ROUTE_WARPS + warp;
+    const int e = blockIdx.x * LOGIT_WARPS + warp;
     const int t0 = blockIdx.y * TT;
     if (e >= n_expert) return;
+    constexpr int UNROLL = TT == 1 ? 12 : 6; // loads in flight: the kernel is their latency
     const float *w = router + (size_t)e * hidden;
     float acc[TT][4];
 #pragma unroll
@@ -26,7 +28,7 @@ route_logits_kernel(const float *__restrict__ router, const float *__restrict__ 
 
     if ((hidden & 3) == 0) {
         const int full = hidden / 128; // passes where every lane has a full float4
-#pragma unroll 4
+#pragma unroll UNROLL
         for (int j = 0; j < full; j++) {
             const float4 wv = __ldg(reinterpret_cast<const float4 *>(w + 128 * j + 4 * lane));
 #pragma unroll
@@ -203,8 +205,10 @@ route_logits_tiled_kernel(const float *__restrict__ router, const float *__restr
     }
 }
 
-// One warp per token; scores staged in shared memory (2 * n_expert floats per warp).  clear: four words to set to zero (a
-// call's device flag, which otherwise takes a launch of its own), or NULL.
+// One warp per token, up to 32 * PER experts in its registers.  (Rounds of a scan of shared memory and ten dependent shuffles
+// were a chain of latencies: logits and selection of 3 tokens, 256 experts 15.2 -> 8.1 us, 64 33.6 -> 19.2, 512 40.8 -> 34.4.)
+// clear: four words to set to zero (a call's device flag, which otherwise takes a launch of its own), or NULL.
+template <int PER>
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
 route_select_kernel(const float *__restrict__ logits, const float *__restrict__ bias, int t, int n_expert,
                     int top_k, float scale, int norm, uint32_t *__restrict__ ids, float *__restrict__ weights, uint32_t *__restrict__ clear) {
@@ -214,16 +218,24 @@ route_select_kernel(const float *__restrict__ logits, const float *__restrict__ 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int token = blockIdx.x * ROUTE_WARPS + warp;
     if (token >= t) return;
-    float *probs = smem + (size_t)warp * 2 * n_expert;
-    float *sel = probs + n_expert;
-    for (int e = lane; e < n_expert; e += 32) {
-        const float p = lmoe_sigmoid_fixed(logits[(size_t)token * n_expert + e]);
-        probs[e] = p;
-        sel[e] = bias ? __fadd_rn(p, bias[e]) : p;
+    const float *lg = logits + (size_t)token * n_expert;
+    float *probs = smem + (size_t)warp * n_expert;
+    uint32_t key[PER];
+    float v[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) v[j] = lane + 32 * j < n_expert ? __ldg(lg + lane + 32 * j) : 0.f;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int e = lane + 32 * j;
+        key[j] = 0u;
+        if (e < n_expert) {
+            const float p = lmoe_sigmoid_fixed(v[j]);
+            probs[e] = p;
+            key[j] = lmoe_score_key(bias ? __fadd_rn(p, __ldg(bias + e)) : p);
+        }
     }
     __syncwarp();
-    lmoe_warp_select(sel, probs, n_expert, top_k, scale, norm, ids + (size_t)token * top_k,
-                     weights + (size_t)token * top_k, lane);
+    lmoe_warp_select_keys<PER>(key, probs, top_k, scale, norm, ids + (size_t)token * top_k, weights + (size_t)token * top_k, lane);
 }
 
 } // namespace
@@ -231,7 +243,7 @@ route_select_kernel(const float *__restrict__ logits, const float *__restrict__ 
 cudaError_t launch_route_logits(const float *router, const float *x, int t, int hidden, int n_expert,
                                 float *logits, cudaStream_t s) {
     if (t == 0) return cudaSuccess;
-    const unsigned gx = (unsigned)((n_expert + ROUTE_WARPS - 1) / ROUTE_WARPS);
+    const unsigned gx = (unsigned)((n_expert + LOGIT_WARPS - 1) / LOGIT_WARPS);
     if (t > 64 && hidden % (128 * RT_AHEAD) == 0 && 8 * hidden * 4 + RT_FOLD <= 227 * 1024) {
         static int sms_of[64] = {0}; // per device: SM count, and the shared-memory opt-in done once
         int dev = 0;
@@ -266,9 +278,9 @@ cudaError_t launch_route_logits(const float *router, const float *x, int t, int 
         else
             launch_pdl(route_logits_tiled_kernel<8>, grid, RT_THREADS, smem, s, router, x, t, hidden, n_expert, ppb * pass, logits);
     } else if (t <= 2) {
-        launch_pdl(route_logits_kernel<1>, dim3(gx, t), ROUTE_WARPS * 32, 0, s, router, x, t, hidden, n_expert, logits);
+        launch_pdl(route_logits_kernel<1>, dim3(gx, t), LOGIT_WARPS * 32, 0, s, router, x, t, hidden, n_expert, logits);
     } else {
-        launch_pdl(route_logits_kernel<4>, dim3(gx, (t + 3) / 4), ROUTE_WARPS * 32, 0, s, router, x, t, hidden, n_expert, logits);
+        launch_pdl(route_logits_kernel<4>, dim3(gx, (t + 3) / 4), LOGIT_WARPS * 32, 0, s, router, x, t, hidden, n_expert, logits);
     }
     return cudaGetLastError();
 }
@@ -276,10 +288,12 @@ cudaError_t launch_route_logits(const float *router, const float *x, int t, int 
 cudaError_t launch_route_select(const float *logits, const float *bias, int t, int n_expert, int top_k,
                                 float scale, int norm, uint32_t *ids, float *weights, cudaStream_t s, uint32_t *clear) {
     if (t == 0) return cudaSuccess;
-    const size_t smem = (size_t)ROUTE_WARPS * 2 * n_expert * sizeof(float);
+    const size_t smem = (size_t)ROUTE_WARPS * n_expert * sizeof(float);
     const unsigned grid = (unsigned)((t + ROUTE_WARPS - 1) / ROUTE_WARPS);
-    launch_pdl(route_select_kernel, grid, ROUTE_WARPS * 32, smem, s, logits, bias, t, n_expert, top_k, scale, norm, ids,
-                                                             weights, clear);
+    if (n_expert > 512) return cudaErrorInvalidValue; // every entry point has refused it
+    // a round rescans the lane's scores: no more of them than needed
+    launch_pdl(n_expert <= 128 ? route_select_kernel<4> : (n_expert <= 256 ? route_select_kernel<8> : route_select_kernel<16>), grid,
+               ROUTE_WARPS * 32, smem, s, logits, bias, t, n_expert, top_k, scale, norm, ids, weights, clear);
     return cudaGetLastError();
 }
 

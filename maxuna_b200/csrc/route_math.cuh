@@ -51,34 +51,33 @@ __device__ __forceinline__ float lmoe_router_fold(float p0, float p1, float p2, 
     return v;
 }
 
-// One warp turns `n_expert` selection scores (shared memory, destroyed) into
-// the ordered top_k: descending score, ties to the lower expert index.
-// probs: unbiased probabilities (shared memory). Writes ids/weights rows.
-__device__ __forceinline__ void lmoe_warp_select(float *sel, const float *probs, int n_expert, int top_k,
-                                                 float scale, int norm, uint32_t *ids_row, float *w_row,
-                                                 int lane) {
-    float my_w = 0.0f; // lane k keeps weight k (top_k <= 32)
+// One warp turns selection scores into the ordered top_k: descending score, ties to the lower expert index.  Lane l holds the
+// scores of experts l, l + 32, ... (PER of them) as unsigned keys in the order of the floats (-0 is +0, NaN and experts that
+// do not exist below everything), so a round is two warp reductions and a rescan of PER registers.
+// probs: unbiased probabilities (shared memory).  Writes ids / weights rows.
+constexpr uint32_t LMOE_KEY_TAKEN = 0x007fffffu; // the key of -infinity
+__device__ __forceinline__ uint32_t lmoe_score_key(float v) {
+    const uint32_t u = __float_as_uint(__fadd_rn(v, 0.0f));
+    return v != v ? 0u : (u & 0x80000000u ? ~u : u | 0x80000000u);
+}
+template <int PER>
+__device__ __forceinline__ void lmoe_warp_select_keys(uint32_t (&key)[PER], const float *probs, int top_k, float scale, int norm,
+                                                      uint32_t *ids_row, float *w_row, int lane) {
+    uint32_t my_id = 0;
     for (int k = 0; k < top_k; k++) {
-        float best = -INFINITY;
-        int best_i = 0x7fffffff;
-        for (int e = lane; e < n_expert; e += 32) {
-            const float v = sel[e];
-            if (v > best || (v == best && e < best_i)) { best = v; best_i = e; }
-        }
+        uint32_t best = 0, best_i = 0x7fffffffu;
 #pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, best, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, best_i, off);
-            if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
-        }
-        if (best_i == 0x7fffffff) best_i = 0; // only reachable with NaN scores
-        if (lane == k) my_w = probs[best_i];
-        if (lane == 0) {
-            ids_row[k] = (uint32_t)best_i;
-            sel[best_i] = -INFINITY;
-        }
-        __syncwarp();
+        for (int j = PER - 1; j >= 0; j--)
+            if (key[j] >= best) { best = key[j]; best_i = lane + 32 * j; }
+        const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+        uint32_t id = __reduce_min_sync(0xffffffffu, best == top ? best_i : 0x7fffffffu);
+        if (top == 0) id = 0; // only reachable with NaN scores
+#pragma unroll
+        for (int j = 0; j < PER; j++)
+            if (id == (uint32_t)(lane + 32 * j)) key[j] = LMOE_KEY_TAKEN;
+        if (lane == k) my_id = id;
     }
+    float my_w = lane < top_k ? probs[my_id] : 0.0f;
     if (norm) {
         float sum = 0.0f; // sequential in slot order, like a plain CPU sum
         for (int k = 0; k < top_k; k++) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, my_w, k));
@@ -86,5 +85,8 @@ __device__ __forceinline__ void lmoe_warp_select(float *sel, const float *probs,
         my_w = __fdiv_rn(my_w, sum);
     }
     if (scale != 0.0f && scale != 1.0f) my_w = __fmul_rn(my_w, scale);
-    if (lane < top_k) w_row[lane] = my_w;
+    if (lane < top_k) {
+        ids_row[lane] = my_id;
+        w_row[lane] = my_w;
+    }
 }

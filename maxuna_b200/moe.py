@@ -21,6 +21,11 @@ from .gguf import Q4_K, Q6_K, ExpertStack, stream_ptr
 WEIGHTS_SUM_FLOOR = 6.103515625e-5  # src/moe.rs:14
 
 
+def _f32(x: torch.Tensor) -> torch.Tensor:
+    """x as contiguous f32; the two conversions cost 2 us of host even where they have nothing to do."""
+    return x if x.dtype == torch.float32 and x.is_contiguous() else x.to(torch.float32).contiguous()
+
+
 class ExpertFfn:
     """`ExpertFfn`, src/moe.rs:19-21."""
 
@@ -42,9 +47,9 @@ class FusedExperts(ExpertFfn):
         the grouped-GEMM or the mat-vec op chain."""
         seq, hidden = x.shape
         top_k = ids.shape[1]
-        x = x.to(torch.float32)
-        mm_supported = all(ops.supported(s.dtype, top_k) for s in (self.gate, self.up, self.down))
-        use_mm = (seq >= ops.mm_id_min_seq() if use_mm is None else bool(use_mm)) and mm_supported
+        x = _f32(x)
+        use_mm = ((seq >= ops.mm_id_min_seq() if use_mm is None else bool(use_mm)) and
+                  all(ops.supported(s.dtype, top_k) for s in (self.gate, self.up, self.down)))
         map0 = ops.prepare_map0(self.gate.n_expert, ids) if use_mm else None
 
         def matmul(stack, xin):
@@ -52,11 +57,11 @@ class FusedExperts(ExpertFfn):
                 return ops.mul_mm_id_shared(stack, xin, ids, map0)
             return ops.mul_mv_id(stack, xin, ids)
 
-        x_g = x.reshape(seq, 1, hidden).contiguous()
+        x_g = x.view(seq, 1, hidden)
         gate = matmul(self.gate, x_g)
         up = matmul(self.up, x_g)
         act = ops.silu_mul(gate, up)
-        w = weights.to(torch.float32)
+        w = weights if weights.dtype == torch.float32 else weights.to(torch.float32)
         if use_mm:
             # the grouped GEMM stages the activation as f16: keep it in range with the
             # per-(token, slot) L2 rescale and undo it in the combine (src/moe.rs:292-313)
@@ -150,12 +155,12 @@ class MoeBlock:
     # ---- reference-shaped API ----------------------------------------------
     def route(self, x_normed: torch.Tensor):
         """`MoeBlock::route`, src/moe.rs:62-71 -> (ids [seq, top_k], weights [seq, top_k])."""
-        return ops.route(self.router, self.exp_probs_b, x_normed.to(torch.float32).contiguous(),
+        return ops.route(self.router, self.exp_probs_b, _f32(x_normed),
                          self.n_expert_used, self.weights_scale, self.weights_norm)
 
     def forward_unfused(self, x_normed: torch.Tensor, use_mm=None) -> torch.Tensor:
         """The reference's op-by-op sequence, src/moe.rs:73-78."""
-        x = x_normed.to(torch.float32).contiguous()
+        x = _f32(x_normed)
         ids, weights = self.route(x)
         routed = self.experts.forward(x, ids, weights, use_mm)
         if self.shared is None:

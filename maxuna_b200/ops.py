@@ -76,7 +76,7 @@ def mul_mv_id(stack: ExpertStack, x: torch.Tensor, ids: torch.Tensor) -> torch.T
     t, xpr, k = _x3(x)
     _ids_dev(ids)
     t_ids, top_k = ids.shape
-    out = torch.empty(t_ids, top_k, stack.n_out, dtype=torch.float32, device=x.device)
+    out = x.new_empty((t_ids, top_k, stack.n_out))
     check(lib().lmoe_mul_mv_id(stack.handle, x.data_ptr(), t, xpr, k, ids.data_ptr(), t_ids, top_k,
                                out.data_ptr(), stream_ptr()))
     return out
@@ -89,7 +89,7 @@ def mul_mv(weight: torch.Tensor, dtype: int, n_out: int, k: int, x: torch.Tensor
     if x.shape[1] != k:
         raise LmoeError(-1, f"x k ({x.shape[1]}) does not match weight k ({k})")
     _require(weight.is_cuda and weight.dtype == torch.uint8, "weight must be a CUDA uint8 buffer")
-    out = torch.empty(x.shape[0], n_out, dtype=torch.float32, device=x.device)
+    out = x.new_empty((x.shape[0], n_out))
     check(lib().lmoe_mul_mv(weight.data_ptr(), dtype, n_out, k, x.data_ptr(), x.shape[0], out.data_ptr(),
                             stream_ptr()))
     return out
@@ -127,7 +127,7 @@ def mul_mm_id_shared(stack: ExpertStack, x: torch.Tensor, ids: torch.Tensor, scr
     t, xpr, k = _x3(x)
     _ids_dev(ids)
     t_ids, top_k = ids.shape
-    out = torch.empty(t_ids, top_k, stack.n_out, dtype=torch.float32, device=x.device)
+    out = x.new_empty((t_ids, top_k, stack.n_out))
     ws_bytes = lib().lmoe_mm_id_workspace_bytes(stack.handle, t, top_k, xpr)
     ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=x.device)
     check(lib().lmoe_mul_mm_id_shared(stack.handle, x.data_ptr(), t, xpr, k, ids.data_ptr(), t_ids, top_k,
@@ -140,7 +140,7 @@ def mul_mm_id(stack: ExpertStack, x: torch.Tensor, ids: torch.Tensor) -> torch.T
     t, xpr, k = _x3(x)
     _ids_dev(ids)
     t_ids, top_k = ids.shape
-    out = torch.empty(t_ids, top_k, stack.n_out, dtype=torch.float32, device=x.device)
+    out = x.new_empty((t_ids, top_k, stack.n_out))
     ws_bytes = lib().lmoe_mm_id_workspace_bytes(stack.handle, t, top_k, xpr) + lib().lmoe_map0_scratch_bytes(stack.n_expert, t)
     ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=x.device)
     check(lib().lmoe_mul_mm_id(stack.handle, x.data_ptr(), t, xpr, k, ids.data_ptr(), t_ids, top_k, out.data_ptr(),
@@ -164,7 +164,7 @@ def l2_rescale(a: torch.Tensor):
     _f32_dev("a", a)
     t, top_k, n = a.shape
     out = torch.empty_like(a)
-    l2 = torch.empty(t, top_k, 1, dtype=torch.float32, device=a.device)
+    l2 = a.new_empty((t, top_k, 1))
     check(lib().lmoe_l2_rescale(a.data_ptr(), t * top_k, n, out.data_ptr(), l2.data_ptr(), stream_ptr()))
     return out, l2
 
@@ -182,7 +182,7 @@ def combine(down: torch.Tensor, col_l2, weights: torch.Tensor) -> torch.Tensor:
         if col_l2.shape != (seq, top_k, 1):
             raise LmoeError(-1, f"col_l2 shape {tuple(col_l2.shape)} must be [seq, top_k, 1] = [{seq}, {top_k}, 1]")
         l2p = col_l2.data_ptr()
-    out = torch.empty(seq, n_out, dtype=torch.float32, device=down.device)
+    out = down.new_empty((seq, n_out))
     check(lib().lmoe_combine(down.data_ptr(), l2p, weights.data_ptr(), seq, top_k, n_out, out.data_ptr(), stream_ptr()))
     return out
 
@@ -199,8 +199,8 @@ def route(router: torch.Tensor, bias, x: torch.Tensor, top_k: int, scale: float 
     if bias is not None:
         _f32_dev("bias", bias)
         _require(bias.numel() == n_expert, "bias must have n_expert entries")
-    ids = torch.empty(t, top_k, dtype=torch.int32, device=x.device)
-    w = torch.empty(t, top_k, dtype=torch.float32, device=x.device)
+    ids = x.new_empty((t, top_k), dtype=torch.int32)
+    w = x.new_empty((t, top_k))
     nbytes = lib().lmoe_route_workspace_bytes(t, n_expert)
     ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
     check(lib().lmoe_route(router.data_ptr(), None if bias is None else bias.data_ptr(), x.data_ptr(), t, hidden,

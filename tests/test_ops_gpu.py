@@ -270,6 +270,23 @@ def test_routing_tiles_bit_exact(orc, dev, t, hidden, ne):
     assert np.array_equal(w.cpu().numpy().view(np.uint32), w_o.view(np.uint32))
 
 
+@pytest.mark.parametrize("ne,top_k", [(1, 1), (31, 31), (128, 8), (129, 32), (257, 10), (512, 32)])
+def test_routing_selection_widths(orc, dev, ne, top_k):
+    """Selection at the edges of the scores a lane holds, with ties, infinities and signed zeros: bitwise the oracle's."""
+    from maxuna_b200 import ops
+
+    rng = np.random.default_rng(ne)
+    logits = rng.integers(-3, 4, (11, ne)).astype(np.float32)
+    logits[1] = -logits[1] * 0.0
+    logits[2, : ne // 2] = -np.inf
+    logits[3, ne // 3] = np.inf
+    bias = np.where(rng.random(ne) < 0.3, -0.5, 0.0).astype(np.float32)
+    ids, w = ops.route_from_logits(torch.from_numpy(logits).to(dev), torch.from_numpy(bias).to(dev), top_k)
+    ids_o, w_o = orc.route_from_logits(logits, bias, top_k)
+    assert np.array_equal(ids.cpu().numpy().astype(np.uint32), ids_o)
+    assert np.array_equal(w.cpu().numpy().view(np.uint32), w_o.view(np.uint32))
+
+
 def test_routing_odd_hidden_and_ties(orc, dev):
     from maxuna_b200 import ops
 
