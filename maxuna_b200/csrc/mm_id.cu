@@ -144,14 +144,22 @@ __device__ __forceinline__ uint32_t h2_sub_mul(uint32_t v, uint32_t base, uint32
 // expert-sorted order}; i is also the slot of the tile in the tile-ordered operands.  A GEMM tile is (row tile, block of
 // 128 weight rows), the latter varying fastest, so CTAs running side by side share the same activation rows in L2.
 // With `extra` > 0 one more list follows the experts' ("expert" n_expert): the rows 0 .. extra-1 of the shared expert.
+// Full tiles come first, then the partial ones by falling height (in sixteens of rows): the CTAs take the tiles of a product
+// in turn, so each round has tiles of one cost and the last, incomplete one the cheapest (experts' order left the SMs idle for
+// 13 % of the gate/up product of 2048 tokens; the whole call 920 -> 892 us, 600 tokens with 128 experts of 768 217 -> 208).
 __global__ void __launch_bounds__(1024) row_tiles_kernel(const uint32_t *__restrict__ tpe, int n_expert, int extra, int nt,
                                                          int4 *__restrict__ tiles, int32_t *__restrict__ n_tiles, int max_tiles) {
     pdl_begin();
     __shared__ int2 warp_sum[32];
+    __shared__ int part_total, part_cnt[32][16]; // partial tiles by warp and by sixteens of rows
     const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
     const int rows = e < n_expert ? (int)tpe[e] : (e == n_expert ? extra : 0);
-    const int cnt = (rows + nt - 1) / nt;
-    int ct = cnt, cr = rows; // inclusive prefix sums
+    const int full = rows / nt, rest = rows - full * nt, bucket = (rest + 15) / 16; // bucket 0: no partial tile
+    if (lane < 16) part_cnt[warp][lane] = 0;
+    const uint32_t same = __match_any_sync(0xffffffffu, bucket), below = (1u << lane) - 1u;
+    __syncwarp();
+    if ((same & below) == 0) part_cnt[warp][bucket] = __popc(same);
+    int ct = full, cr = rows; // inclusive prefix sums
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int a = __shfl_up_sync(0xffffffffu, ct, o), b = __shfl_up_sync(0xffffffffu, cr, o);
@@ -167,12 +175,33 @@ __global__ void __launch_bounds__(1024) row_tiles_kernel(const uint32_t *__restr
             if (lane >= o) { v.x += a; v.y += b; }
         }
         warp_sum[lane] = v;
-        if (lane == 31) *n_tiles = min(v.x, max_tiles);
+    } else if (warp == 1 && lane < 16) { // partial tiles: the warps' counts of a bucket -> first places, the largest bucket first
+        const int warps = (n_expert + 32) / 32;
+        int n = 0;
+        for (int w = 0; w < warps; w++) n += part_cnt[w][lane];
+        if (lane == 0) n = 0;
+        int ge = n; // partial tiles of this bucket and the larger ones
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const int a = __shfl_down_sync(0x0000ffffu, ge, o, 16);
+            if (lane + o < 16) ge += a;
+        }
+        int first = ge - n;
+        for (int w = 0; w < warps; w++) {
+            const int c = part_cnt[w][lane];
+            part_cnt[w][lane] = first;
+            first += c;
+        }
+        if (lane == 1) part_total = ge;
     }
     __syncthreads();
-    const int t0 = ct - cnt + (warp ? warp_sum[warp - 1].x : 0), r0 = cr - rows + (warp ? warp_sum[warp - 1].y : 0);
-    for (int i = 0; i < cnt; i++)
-        if (t0 + i < max_tiles) tiles[t0 + i] = make_int4(e, i * nt, min(nt, rows - i * nt), r0 + i * nt);
+    const int n_full = warp_sum[31].x;
+    if (e == 0) *n_tiles = min(n_full + part_total, max_tiles);
+    const int t0 = ct - full + (warp ? warp_sum[warp - 1].x : 0), r0 = cr - rows + (warp ? warp_sum[warp - 1].y : 0);
+    for (int i = 0; i < full; i++)
+        if (t0 + i < max_tiles) tiles[t0 + i] = make_int4(e, i * nt, nt, r0 + i * nt);
+    const int tp = n_full + part_cnt[warp][bucket] + __popc(same & below);
+    if (rest && tp < max_tiles) tiles[tp] = make_int4(e, full * nt, rest, r0 + full * nt);
 }
 
 // Routed rows -> the f16 B operand in TILE ORDER.  Row tile `slot` (nt routed rows of one expert)
