@@ -244,18 +244,21 @@ cudaError_t launch_route_logits(const float *router, const float *x, int t, int 
                                 float *logits, cudaStream_t s) {
     if (t == 0) return cudaSuccess;
     const unsigned gx = (unsigned)((n_expert + LOGIT_WARPS - 1) / LOGIT_WARPS);
-    if (t > 64 && hidden % (128 * RT_AHEAD) == 0 && 8 * hidden * 4 + RT_FOLD <= 227 * 1024) {
-        static int sms_of[64] = {0}; // per device: SM count, and the shared-memory opt-in done once
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-        if (!sms_of[dev]) {
-            int n = 0;
-            if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
-            cudaFuncSetAttribute(route_logits_tiled_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            cudaFuncSetAttribute(route_logits_tiled_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            sms_of[dev] = n;
-        }
-        // (Up to 64 tokens a warp per expert row covers the device better: 7 us against 9 at 16 tokens.)
+    static int sms_of[64] = {0}; // per device: SM count, and the shared-memory opt-in done once
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (!sms_of[dev]) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+        cudaFuncSetAttribute(route_logits_tiled_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(route_logits_tiled_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        sms_of[dev] = n;
+    }
+    // A warp per expert row while its blocks are few, up to five an SM; beyond, their trips to the L2 cache take longer than a
+    // register-tiled pass, whose time is the same for any small batch (256 experts, 16 / 24 / 64 tokens: 11.0 / 12.8 / 19.1 us
+    // against 12.4 / 12.5 / 12.8; 64 experts of 4096, 64 tokens: 10.2 against 13.3).
+    const bool many = (int64_t)gx * ((t + 3) / 4) > 5 * sms_of[dev];
+    if (many && hidden % (128 * RT_AHEAD) == 0 && 8 * hidden * 4 + RT_FOLD <= 227 * 1024) {
         // One block per SM at a time: 16 tokens and 16 experts a pass where the rows fit (hidden <= 3072), or 8 tokens and 32
         // experts, in the same time.  The experts are split over blocks until the device is covered, and further where that
         // fills the last wave better; a block repeats the staging of its tokens, which for 16 costs about a pass.  Of equal

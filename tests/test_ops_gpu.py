@@ -255,7 +255,7 @@ def test_routing_bit_exact_vs_oracle(orc, dev, t):
     assert np.array_equal(w.cpu().numpy().view(np.uint32), w_o.view(np.uint32))  # weights bit-exact too
 
 
-@pytest.mark.parametrize("t,hidden,ne", [(65, 512, 20), (81, 2048, 130), (79, 3072, 17), (73, 4096, 70), (66, 6144, 33)])
+@pytest.mark.parametrize("t,hidden,ne", [(301, 512, 20), (81, 2048, 130), (335, 3072, 17), (90, 4096, 70), (23, 3072, 256), (179, 6144, 33)])
 def test_routing_tiles_bit_exact(orc, dev, t, hidden, ne):
     """The register-tiled router product at the edges of its token and expert tiles, in both tile shapes: same fixed summation
     order, so ids and weights are bitwise the oracle's."""
