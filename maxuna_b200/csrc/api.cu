@@ -359,8 +359,8 @@ extern "C" void lmoe_layer_destroy(lmoe_layer *layer) {
     if (!layer) return;
     cudaFree(layer->sync);
     if (layer->dec_event) cudaEventDestroy(layer->dec_event);
+    if (layer->host_x[0]) cudaFree(layer->host_x[0]); // both buffers are one allocation
     for (int i = 0; i < 2; i++) {
-        if (layer->host_x[i]) cudaFree(layer->host_x[i]);
         if (layer->host_copied[i]) cudaEventDestroy(layer->host_copied[i]);
         if (layer->host_slot_free[i]) cudaEventDestroy(layer->host_slot_free[i]);
     }

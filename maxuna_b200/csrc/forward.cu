@@ -198,8 +198,9 @@ static bool host_buffer_is_pinned(const void *p) {
 static bool host_staging_ready(const lmoe_layer *L) {
     if (L->host_failed) return false;
     if (L->host_copy_stream) return true;
-    const size_t bytes = (size_t)decode_max_tokens() * L->hidden * 4;
-    bool ok = cudaMalloc(&L->host_x[0], bytes) == cudaSuccess && cudaMalloc(&L->host_x[1], bytes) == cudaSuccess;
+    const size_t rows = (size_t)decode_max_tokens() * L->hidden;
+    bool ok = cudaMalloc(&L->host_x[0], 2 * rows * 4) == cudaSuccess; // one allocation, not two: they are most of a first call
+    if (ok) L->host_x[1] = L->host_x[0] + rows;
     for (int i = 0; i < 2 && ok; i++)
         ok = cudaEventCreateWithFlags(&L->host_copied[i], cudaEventDisableTiming) == cudaSuccess &&
              cudaEventCreateWithFlags(&L->host_slot_free[i], cudaEventDisableTiming) == cudaSuccess;
