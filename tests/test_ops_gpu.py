@@ -355,6 +355,20 @@ def test_map0_matches_oracle(orc, dev):
             assert np.array_equal(got[e, : tpe[e]], m[e, : tpe[e]])
 
 
+@pytest.mark.parametrize("t", [1024, 1025, 1028, 4096, 4097, 8196])
+def test_map0_chunk_edges(orc, dev, t):
+    """Block sizes, chunks and the vector and scalar loads of the token lists, with empty slots: bytes equal the oracle's."""
+    from maxuna_b200 import ops
+
+    ids = orc.distinct_ids(t, 3, 9, t)
+    ids[t - 1, 2] = 9
+    s = ops.prepare_map0(8, torch.from_numpy(ids.astype(np.int32)).to(dev))
+    for e in range(8):
+        want = np.flatnonzero(ids.reshape(-1) == e)
+        assert s.tpe()[e].item() == want.size
+        assert np.array_equal(s.ids_map()[e, : want.size].cpu().numpy(), want)
+
+
 def _tiny_block(dev, seed=3, hidden=256, ff=256, ne=8, top_k=3, shared=True):
     from maxuna_b200.moe import MoeBlock
 
