@@ -33,6 +33,7 @@ at batch <= 16 does not shard; weak scaling).
 from __future__ import annotations
 
 import argparse
+import gc
 import hashlib
 import json
 import os
@@ -391,6 +392,7 @@ def measure_lm_head(dev, steps=20, warmup=5):
         i[0] += 1
         _native.check(lib.lmoe_mul_mv(st.buffer.data_ptr() + st.base_off, Q6_K, n_out, k, x.data_ptr(), 1, out.data_ptr(), stream_ptr()))
 
+    gc.collect()  # a collection of what earlier measurements left would fall into these few launches
     ms = _time_gpu(run, steps, warmup, 1, dev)
     nbytes = n_out * (k // 256) * 210
     # parity: the last launch used stack (steps + warmup - 1) % copies; check 64 sampled rows of it
