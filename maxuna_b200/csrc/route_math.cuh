@@ -52,13 +52,14 @@ __device__ __forceinline__ float lmoe_router_fold(float p0, float p1, float p2, 
 }
 
 // One warp turns selection scores into the ordered top_k: descending score, ties to the lower expert index.  Lane l holds the
-// scores of experts l, l + 32, ... (PER of them) as unsigned keys in the order of the floats (-0 is +0, NaN and experts that
-// do not exist below everything), so a round is two warp reductions and a rescan of PER registers.
+// scores of experts l, l + 32, ... (PER of them) as unsigned keys in the order of the floats (-0 is +0, NaN below -infinity),
+// so a round is two warp reductions and a rescan of PER registers.  The key of an expert is never 0: that marks the taken ones
+// and those that do not exist, so the ids of a token are distinct whatever its scores are (the row lists and the sums of the
+// grouped products index by them); top_k <= n_expert keeps an untaken one for every round.
 // probs: unbiased probabilities (shared memory).  Writes ids / weights rows.
-constexpr uint32_t LMOE_KEY_TAKEN = 0x007fffffu; // the key of -infinity
 __device__ __forceinline__ uint32_t lmoe_score_key(float v) {
     const uint32_t u = __float_as_uint(__fadd_rn(v, 0.0f));
-    return v != v ? 0u : (u & 0x80000000u ? ~u : u | 0x80000000u);
+    return v != v ? 1u : (u & 0x80000000u ? ~u : u | 0x80000000u); // -infinity: 0x007fffff
 }
 template <int PER>
 __device__ __forceinline__ void lmoe_warp_select_keys(uint32_t (&key)[PER], const float *probs, int top_k, float scale, int norm,
@@ -70,11 +71,10 @@ __device__ __forceinline__ void lmoe_warp_select_keys(uint32_t (&key)[PER], cons
         for (int j = PER - 1; j >= 0; j--)
             if (key[j] >= best) { best = key[j]; best_i = lane + 32 * j; }
         const uint32_t top = __reduce_max_sync(0xffffffffu, best);
-        uint32_t id = __reduce_min_sync(0xffffffffu, best == top ? best_i : 0x7fffffffu);
-        if (top == 0) id = 0; // only reachable with NaN scores
+        const uint32_t id = __reduce_min_sync(0xffffffffu, best == top ? best_i : 0x7fffffffu);
 #pragma unroll
         for (int j = 0; j < PER; j++)
-            if (id == (uint32_t)(lane + 32 * j)) key[j] = LMOE_KEY_TAKEN;
+            if (id == (uint32_t)(lane + 32 * j)) key[j] = 0u;
         if (lane == k) my_id = id;
     }
     float my_w = lane < top_k ? probs[my_id] : 0.0f;

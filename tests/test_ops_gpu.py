@@ -287,6 +287,28 @@ def test_routing_selection_widths(orc, dev, ne, top_k):
     assert np.array_equal(w.cpu().numpy().view(np.uint32), w_o.view(np.uint32))
 
 
+@pytest.mark.parametrize("ne,top_k", [(5, 5), (64, 8), (200, 10), (512, 32)])
+def test_routing_ids_are_distinct(orc, dev, ne, top_k):
+    """A token's ids are distinct and in range whatever its scores are: all or some NaN, and a bias that leaves fewer finite
+    scores than slots (the row lists and sums behind them take distinct ids for granted).  Where no score is NaN, and where
+    all are, ids are the oracle's."""
+    from maxuna_b200 import ops
+
+    rng = np.random.default_rng(ne)
+    logits = rng.standard_normal((9, ne)).astype(np.float32)
+    logits[0] = np.nan
+    logits[1, 1:] = np.nan
+    logits[2, rng.random(ne) < 0.7] = np.nan
+    bias = np.zeros(ne, dtype=np.float32)
+    bias[top_k // 2:] = -np.inf
+    for b in (None, bias):
+        ids, _ = ops.route_from_logits(torch.from_numpy(logits).to(dev), None if b is None else torch.from_numpy(b).to(dev), top_k)
+        ids = ids.cpu().numpy().astype(np.uint32)
+        assert ids.max() < ne and all(len(set(r)) == top_k for r in ids.tolist())
+        want, _ = orc.route_from_logits(logits, b, top_k)
+        assert np.array_equal(ids[[0, *range(3, 9)]], want[[0, *range(3, 9)]])
+
+
 def test_routing_odd_hidden_and_ties(orc, dev):
     from maxuna_b200 import ops
 
@@ -367,6 +389,22 @@ def test_map0_chunk_edges(orc, dev, t):
         want = np.flatnonzero(ids.reshape(-1) == e)
         assert s.tpe()[e].item() == want.size
         assert np.array_equal(s.ids_map()[e, : want.size].cpu().numpy(), want)
+
+
+def test_prefill_with_a_nan_token(orc, dev):
+    """A token with a NaN in its hidden state goes through the grouped products beside others: its own row is NaN, the other
+    rows are what they are without it."""
+    blk = _tiny_block(dev)
+    x = torch.from_numpy(orc.pseudo_random(96 * 256, 5, -1.0, 1.0).reshape(96, 256)).to(dev)
+    want = blk.forward(x, path="prefill")
+    x[40, 7] = float("nan")
+    got, ids, _ = blk.forward(x, return_routing=True, path="prefill")
+    torch.cuda.synchronize()
+    blk.check_device_flag()
+    assert sorted(set(ids[40].tolist())) == sorted(ids[40].tolist())
+    keep = [i for i in range(96) if i != 40]
+    assert torch.isnan(got[40]).all() and torch.isfinite(got[keep]).all()
+    assert orc.rel_l2(got[keep].cpu().numpy(), want[keep].cpu().numpy()) < 1e-6  # the same products, other row tiles
 
 
 def _tiny_block(dev, seed=3, hidden=256, ff=256, ne=8, top_k=3, shared=True):
