@@ -442,9 +442,9 @@ __device__ __forceinline__ void unit_q4k(const uint8_t *stage, int row_bytes, in
         q4k_block(rg + b * Q4K_BYTES, rG + b * Q4K_BYTES, t, xcol + 256 * b, scol + 8 * b, sxs + 8 * b, r0, r1, acc);
 }
 
-// 32 Q6_K rows: warp wq of the group takes row tile wq & 1 (16 rows) and a contiguous half of its super-blocks.
-// Super-blocks are 210 bytes long, so every other one starts 2 bytes off a word boundary and costs twice the shared-memory
-// reads; neighbours share the expensive ones out evenly.
+// 32 Q6_K rows: warp wq of the group takes row tile wq & 1 (16 rows) and half of its super-blocks.  Super-blocks are 210 bytes
+// long, so every other one starts 2 bytes off a word boundary and costs twice the shared-memory reads.  With an even number of
+// them in a row the rows start alike, and contiguous halves share the expensive ones out evenly.
 __device__ __forceinline__ void unit_q6k(const uint8_t *stage, int row_bytes, int nb, int wq, int g, int t,
                                          const int8_t *xcol, const __half *scol, const float *sxs, float r0, float r1,
                                          float (&acc)[4]) {
@@ -452,21 +452,34 @@ __device__ __forceinline__ void unit_q6k(const uint8_t *stage, int row_bytes, in
     // disjoint shared-memory banks (rows g and g+8 would share two)
     const uint8_t *rg = stage + ((wq & 1) * 16 + 2 * g) * row_bytes;
     const uint8_t *rG = rg + row_bytes;
-    if (nb == CW && !(row_bytes & 2)) {
+    if (nb == CW) {
         // both of the warp's blocks in straight line: the second one's loads run under the first one's arithmetic (a unit is
         // bound by its chains, with two warps per scheduler: 16 tokens 154 -> 148 us, 64 tokens 357 -> 342 us)
         const int b = (wq >> 1) * 2;
-        q6k_block<0>(rg + b * Q6K_BYTES, rG + b * Q6K_BYTES, b, t, xcol, scol, sxs, r0, r1, acc);
-        q6k_block<1>(rg + (b + 1) * Q6K_BYTES, rG + (b + 1) * Q6K_BYTES, b + 1, t, xcol, scol, sxs, r0, r1, acc);
+        q6k_block<0, 0>(rg + b * Q6K_BYTES, rG + b * Q6K_BYTES, b, t, xcol, scol, sxs, r0, r1, acc);
+        q6k_block<1, 1>(rg + (b + 1) * Q6K_BYTES, rG + (b + 1) * Q6K_BYTES, b + 1, t, xcol, scol, sxs, r0, r1, acc);
         return;
     }
-    const int per = (nb + CW / 2 - 1) / (CW / 2), b_end = min(nb, ((wq >> 1) + 1) * per);
+    const int per = nb / (CW / 2), b_end = ((wq >> 1) + 1) * per;
     for (int b = (wq >> 1) * per; b < b_end; b++) {
         const uint8_t *bg = rg + b * Q6K_BYTES, *bG = rG + b * Q6K_BYTES;
-        if (row_bytes & 2) q6k_block<2>(bg, bG, b, t, xcol, scol, sxs, r0, r1, acc); // odd block count: rows alternate too
-        else if (b & 1) q6k_block<1>(bg, bG, b, t, xcol, scol, sxs, r0, r1, acc);
-        else q6k_block<0>(bg, bG, b, t, xcol, scol, sxs, r0, r1, acc);
+        if (b & 1) q6k_block<1, 1>(bg, bG, b, t, xcol, scol, sxs, r0, r1, acc);
+        else q6k_block<0, 0>(bg, bG, b, t, xcol, scol, sxs, r0, r1, acc);
     }
+}
+
+// The same for an odd number of super-blocks: a row and the next one have opposite alignment, and so have neighbouring blocks.
+// The warps take alternate blocks, which fixes both for the whole unit.  (A choice per lane at every word instead: expert
+// width 768, hidden 4096, 7 / 16 / 64 tokens 169 / 271 / 720 us, so 124 / 186 / 481.)
+__device__ __forceinline__ void unit_q6k_odd(const uint8_t *stage, int row_bytes, int nb, int wq, int g, int t,
+                                             const int8_t *xcol, const __half *scol, const float *sxs, float r0, float r1,
+                                             float (&acc)[4]) {
+    const uint8_t *rg = stage + ((wq & 1) * 16 + 2 * g) * row_bytes;
+    const uint8_t *rG = rg + row_bytes;
+    if (wq >> 1)
+        for (int b = 1; b < nb; b += 2) q6k_block<1, 0>(rg + b * Q6K_BYTES, rG + b * Q6K_BYTES, b, t, xcol, scol, sxs, r0, r1, acc);
+    else
+        for (int b = 0; b < nb; b += 2) q6k_block<0, 1>(rg + b * Q6K_BYTES, rG + b * Q6K_BYTES, b, t, xcol, scol, sxs, r0, r1, acc);
 }
 
 // Per-pass hand-over between phases 1 and 2 (small batches).  Out of line on purpose: they run once per
@@ -489,7 +502,8 @@ __device__ __noinline__ void dec_wait_pass(const uint32_t *cnt, uint32_t need, u
     }
 }
 
-// The units n .. n1 - 1 of one pass (a unit is one fill of the ring, fills are counted through the launch).  A function of its
+// The units n .. n1 - 1 of one pass (a unit is one fill of the ring, fills are counted through the launch); PHASE 3 is the
+// second one for rows of an odd number of super-blocks.  A function of its
 // own, with everything in scalars: its registers are then its own, and no change around it moves them (the same loop inside
 // the kernel varied by 5 % with what stood beside it).
 template <int NDIG, int NTOK, int NG, int PHASE>
@@ -512,7 +526,8 @@ __device__ __noinline__ void dec_units(uint32_t n, uint32_t n1, const uint8_t *r
         have_buf = mbar_test(&red_free[(n + 1) % NRED], (((n + 1) / NRED) & 1) ^ 1);
         const uint8_t *stage = ring + (size_t)s * stage_bytes;
         if (PHASE == 1) unit_q4k(stage, row_bytes, nb, wq, g, t4, xcol, scol, sxs, r0, r1, acc);
-        else unit_q6k(stage, row_bytes, nb, wq, g, t4, xcol, scol, sxs, r0, r1, acc);
+        else if (PHASE == 2) unit_q6k(stage, row_bytes, nb, wq, g, t4, xcol, scol, sxs, r0, r1, acc);
+        else unit_q6k_odd(stage, row_bytes, nb, wq, g, t4, xcol, scol, sxs, r0, r1, acc);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
         // K-split partials -> shared memory, handed to the epilogue warp
@@ -1128,6 +1143,8 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
                 const uint32_t n0 = n_unit + (uint32_t)(a - u0), n1 = n_unit + (uint32_t)(b - u0);
                 if (phase == 1)
                     dec_units<NDIG, NTOK, NG, 1>(n0, n1, ring, L.stage_bytes, row4, nb4, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
+                else if (row6 & 2)
+                    dec_units<NDIG, NTOK, NG, 3>(n0, n1, ring, L.stage_bytes, row6, nb6, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
                 else
                     dec_units<NDIG, NTOK, NG, 2>(n0, n1, ring, L.stage_bytes, row6, nb6, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
             }

@@ -199,10 +199,10 @@ __device__ __forceinline__ uint32_t sc_pair_half2(const int8_t *p) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// One Q6_K super-block of two rows (bg -> accumulators 0/1, bG -> 2/3) that have the same alignment.  The six-bit value of a
+// One Q6_K super-block of two rows (bg -> accumulators 0/1, bG -> 2/3), MIS / MIS2: their alignment.  The six-bit value of a
 // weight (low nibble | two high bits << 4, 0..63) is one byte of a k = 16 integer MMA: one MMA per 16-wide
 // sub-block, whose signed scale multiplies the exact integer sum.
-template <int MIS>
+template <int MIS, int MIS2>
 __device__ __forceinline__ void q6k_block(const uint8_t *bg, const uint8_t *bG, int b, int t, const int8_t *xcol,
                                           const __half *scol, const float *sxs, float r0, float r1, float (&acc)[4]) {
     constexpr uint32_t M4 = 0x0F0F0F0Fu, M2 = 0x30303030u;
@@ -222,14 +222,14 @@ __device__ __forceinline__ void q6k_block(const uint8_t *bg, const uint8_t *bG, 
 #pragma unroll
     for (int n = 0; n < 2; n++) {
         const uint32_t swg0 = lds32<MIS>(bg, 192 + 8 * n), swg1 = lds32<MIS>(bg, 196 + 8 * n);
-        const uint32_t swG0 = lds32<MIS>(bG, 192 + 8 * n), swG1 = lds32<MIS>(bG, 196 + 8 * n);
+        const uint32_t swG0 = lds32<MIS2>(bG, 192 + 8 * n), swG1 = lds32<MIS2>(bG, 196 + 8 * n);
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             const int l0 = 16 * c + 4 * t;
             const uint32_t qa_g = lds32<MIS>(bg, 64 * n + l0), qb_g = lds32<MIS>(bg, 64 * n + 32 + l0);
             const uint32_t qh_g = lds32<MIS>(bg, 128 + 32 * n + l0);
-            const uint32_t qa_G = lds32<MIS>(bG, 64 * n + l0), qb_G = lds32<MIS>(bG, 64 * n + 32 + l0);
-            const uint32_t qh_G = lds32<MIS>(bG, 128 + 32 * n + l0);
+            const uint32_t qa_G = lds32<MIS2>(bG, 64 * n + l0), qb_G = lds32<MIS2>(bG, 64 * n + 32 + l0);
+            const uint32_t qh_G = lds32<MIS2>(bG, 128 + 32 * n + l0);
             const int8_t *xp = xcol + 256 * b + 128 * n + l0;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
