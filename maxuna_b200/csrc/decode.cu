@@ -88,7 +88,7 @@ struct DecodeParams {
     const uint8_t *gate, *up, *down, *sh_gate, *sh_up, *sh_down;
     int t, hidden, ff, n_expert, top_k;
     float scale;
-    int norm, has_shared;
+    int norm, has_shared, lists_alias;
     int sh_t0, sh_nt; // the shared expert serves tokens [sh_t0, sh_t0 + sh_nt) (all of them unless the caller narrows it)
     uint32_t *ctrl;   // workspace: [0..3] device flag (zeroed by the launch with first_launch set)
     uint32_t *sync;   // owned by the layer, zero between launches: [0] grid barrier, [1] exit count, [32..] per-pass counts
@@ -102,10 +102,12 @@ struct DecodeParams {
 
 // Shared-memory layout (bytes), computed identically on host and device.
 struct DecLayout {
-    int stage_bytes, xs, ss;
-    bool lists_alias;
-    int o_ring, o_xc, o_s, o_sx, o_red, o_bar, o_ids, o_w, o_cnt, o_off, o_plist, o_act, o_ppre, total;
-    __host__ __device__ DecLayout(int hidden, int ff, int n_expert, int t, int top_k, int ncol, int ncw, int nstage, int nred) {
+    int stage_bytes = 0, xs = 0, ss = 0;
+    int o_ring = 0, o_xc = 0, o_s = 0, o_sx = 0, o_red = 0, o_bar = 0, o_ids = 0, o_w = 0, o_cnt = 0, o_off = 0, o_plist = 0, o_act = 0,
+        o_ppre = 0, total = 0;
+    // lists_alias: the list build's counts and ids lie over the activation cache (see dec_lists_alias)
+    constexpr __host__ __device__ DecLayout(int hidden, int ff, int n_expert, int t, int top_k, int ncol, int nstage, int nred,
+                                            bool lists_alias) {
         const int row4 = hidden / QK_K * Q4K_BYTES, row6 = ff / QK_K * Q6K_BYTES;
         int sb = 16 * row4 > DOWN_ROWS * row6 ? 16 * row4 : DOWN_ROWS * row6;
         stage_bytes = (sb + 127) / 128 * 128;
@@ -119,28 +121,43 @@ struct DecLayout {
         o_xc = o;
         int xc_bytes = ncol * xs;
         // the selection's scratch aliases the activation cache: keys, scores and the selected scores
-        const int sel_bytes = (2 * n_expert + 4 + 32) * 4, list_bytes = (n_expert + tk) * 4;
+        const int sel_bytes = (2 * n_expert + 4 + 32) * 4, list_bytes = tk <= 32 ? 0 : (n_expert + tk) * 4; // (32: dec_lists_warp)
         if (sel_bytes > xc_bytes) xc_bytes = sel_bytes;
-        if (list_bytes > xc_bytes) xc_bytes = list_bytes;
+        if (lists_alias && list_bytes > xc_bytes) xc_bytes = list_bytes;
         o += (xc_bytes + 15) / 16 * 16;
         o_s = o; o += ncol * ss * 2;
         o_sx = o; o += (kmax / QK_K) * 8 * 4; // [256-block][8 columns] digit scales
         const int red_bytes = nred * CW * 16 * ncol * 4; // the K-split partial buffers
         o_red = o; o += (red_bytes + 15) / 16 * 16;
-        // expert counts and id list: over the activation cache (which is staged again after they are dead) in larger batches
-        lists_alias = tk > 256;
         o_cnt = lists_alias ? o_xc : o;
         o_ids = o_cnt + n_expert * 4;
         if (!lists_alias) o += (list_bytes + 15) / 16 * 16;
         o_bar = o; o += ((2 * nstage + 2 * nred) * 8 + 127) / 128 * 128;
         o_w = o; o += tk * 4;
-        o_off = o; o += (tk + 2) / 2 * 2 * 2;
+        const int na = n_expert < tk ? n_expert : tk; // most experts a launch can select
+        o_off = o; o += (na + 2) / 2 * 2 * 2;
         o_plist = o; o += (tk + 1) / 2 * 2 * 2;
-        o_act = o; o += (tk + 2) / 2 * 2 * 2;
-        o_ppre = o; o += (tk + 2) / 2 * 2 * 2;
+        o_act = o; o += (na + 2) / 2 * 2 * 2;
+        o_ppre = o; o += (na + 2) / 2 * 2 * 2;
         total = (o + 15) / 16 * 16;
     }
+    // CTAs of an SM, of at most two: 228 KB a SM and 227 a CTA, each CTA with 1 KB of its own and the kernel's static arrays
+    constexpr __host__ __device__ int ctas() const {
+        return 2 * (total + 1024 + 128) <= 228 * 1024 ? 2 : (total + 128 <= 227 * 1024 ? 1 : 0);
+    }
 };
+// Where the list build's counts and ids go: over the activation cache, which then has to be staged again, in batches of more
+// than 256 pairs, and in smaller ones where space of their own would cost a CTA of the SM or the whole launch (hidden 1280,
+// expert width 1280, 40 experts, 64 pairs: 103 us with one CTA, 78 with two and the unit code of the time).
+constexpr bool dec_lists_alias(int hidden, int ff, int n_expert, int t, int top_k, int ncol, int nstage, int nred) {
+    return t * top_k > 256 || DecLayout(hidden, ff, n_expert, t, top_k, ncol, nstage, nred, true).ctas() >
+                                  DecLayout(hidden, ff, n_expert, t, top_k, ncol, nstage, nred, false).ctas();
+}
+constexpr int dec_ctas(int hidden, int ff, int n_expert, int t, int top_k) {
+    return DecLayout(hidden, ff, n_expert, t, top_k, 6, 3, 3, dec_lists_alias(hidden, ff, n_expert, t, top_k, 6, 3, 3)).ctas();
+}
+static_assert(dec_ctas(256, 2560, 64, 25, 32) == 1 && dec_ctas(256, 1280, 16, 9, 8) == 2 && dec_ctas(1280, 1280, 40, 2, 32) == 2 &&
+                  dec_ctas(3072, 1024, 256, 16, 10) == 2, "shapes just below a limit");
 
 // Index guard for values read back from the routing tables, on the paths that run once per unit or less
 // (the producer's source addresses, the list build): a value outside its range is recorded in the device
@@ -841,7 +858,7 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
     constexpr int NCOL = NDIG * NTOK; // MMA columns in use: (token, digit)
     constexpr int NSTAGE = C::NSTAGE, NRED = C::NRED, NCW = C::NCW, CONS_THREADS = C::CONS;
     extern __shared__ __align__(128) uint8_t smem[];
-    const DecLayout L(P.hidden, P.ff, P.n_expert, P.t, P.top_k, NCOL, NCW, NSTAGE, NRED);
+    const DecLayout L(P.hidden, P.ff, P.n_expert, P.t, P.top_k, NCOL, NSTAGE, NRED, P.lists_alias);
     uint8_t *ring = smem + L.o_ring;
     int8_t *xc = reinterpret_cast<int8_t *>(smem + L.o_xc);
     __half *sh = reinterpret_cast<__half *>(smem + L.o_s);
@@ -1096,7 +1113,7 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
                 }
                 bar_sync(1, CONS_THREADS);
                 dec_lists<NTOK>(tk, E, P.ctrl, ids_s, cnt_s, plist_s, act_s, off_s, ppre_s, &s_n_active, &s_routed_passes, tid, CONS_THREADS);
-                if (L.lists_alias) xkey = ~0ull; // they were built over the activation cache
+                if (P.lists_alias) xkey = ~0ull; // they were built over the activation cache
             }
             if (tid >= 1 && tid < 4)
                 s_range[tid] = dec_unit_range_of(tid, s_routed_passes, shared_passes, tiles1, tiles2);
@@ -1258,7 +1275,8 @@ lmoe_status launch_moe_decode(const lmoe_layer *Ly, const float *x, int t, float
     static thread_local DecVariant v_small = make_variant<3, 2, 1>();
     static thread_local DecVariant v_23 = make_variant<2, 3, 1>();
     DecVariant &V = t >= LMOE_DEC_V23_FROM_T ? v_23 : v_small;
-    const DecLayout L(H, F, E, t, K, V.ncol, V.ncw, V.nstage, V.nred);
+    const bool lists_alias = dec_lists_alias(H, F, E, t, K, V.ncol, V.nstage, V.nred);
+    const DecLayout L(H, F, E, t, K, V.ncol, V.nstage, V.nred, lists_alias);
     static thread_local int c_dev = -1, c_sms = 0, c_max_smem = 0;
     int dev = 0;
     LMOE_CUDA(cudaGetDevice(&dev));
@@ -1298,6 +1316,7 @@ lmoe_status launch_moe_decode(const lmoe_layer *Ly, const float *x, int t, float
     P.sh_down = P.has_shared ? Ly->sh_down->blocks() : nullptr;
     P.t = t; P.hidden = H; P.ff = F; P.n_expert = E; P.top_k = K;
     P.scale = Ly->scale; P.norm = Ly->norm;
+    P.lists_alias = lists_alias;
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     P.ctrl = reinterpret_cast<uint32_t *>(ws);
     P.sync = Ly->sync;

@@ -72,6 +72,17 @@ def test_decode_list_and_row_forms(orc, dev, hidden, ff, ne, k, ts):
         _check(orc, blk, host, x, 1e-4 if t <= 8 else 5e-4)
 
 
+@pytest.mark.parametrize("hidden,ff,ne,k,t", [(256, 2560, 64, 32, 25), (1280, 1280, 40, 16, 4)])
+def test_decode_at_the_shared_memory_limits(orc, dev, hidden, ff, ne, k, t):
+    """A launch that needs all of an SM's shared memory, and one whose lists only fit over the activation cache beside a second
+    CTA: served, with the routing exact and the output within the 21- and 15-bit activations' error."""
+    from maxuna_b200.moe import MoeBlock
+
+    blk = MoeBlock.random(hidden, ff, ne, k, seed=21, device=dev, weight_std=0.1)
+    x = np.random.default_rng(22).standard_normal((t, hidden)).astype(np.float32)
+    _check(orc, blk, blk.host_layer(orc), x, 1e-4 if t <= 8 else 5e-4)
+
+
 @pytest.fixture(scope="module")
 def full_block(dev):
     from maxuna_b200.moe import MoeBlock
