@@ -43,6 +43,8 @@
 //   * The down projection writes weighted partial rows; a last phase sums the
 //     K+1 partials of every output element in slot order, so the result is
 //     deterministic without float atomics.
+#include <type_traits>
+
 #include "fused.cuh"
 #include "kquant.cuh"
 #include "route_math.cuh"
@@ -226,27 +228,28 @@ __device__ __forceinline__ void unit_range_first(int n_units, int selecting, int
     u0 = c < 0 ? 0 : (int)((long long)c * n_units / n);
     u1 = c < 0 ? 0 : (int)((long long)(c + 1) * n_units / n);
 }
-// Units of this CTA by section (phase 1 shared / routed, phase 2 shared / routed) as (first, end).  Each section is split
-// evenly by itself; only in phase 2, where a CTA has few units, shared and routed are split evenly TOGETHER: one token makes
-// 3.6 of them per CTA, and two separate splits gave some CTAs five.  (In phase 1 the shared units pass while the routing is
-// still on its way.)  A CTA's share of all must not be smaller than its part of the shared ones, which holds from one
-// routed unit per CTA on.
+// Units of this CTA by section (phase 1 shared / routed, phase 2 shared / routed) as (first, end).  Where a CTA has few units,
+// shared and routed are split evenly TOGETHER: one token makes 3.6 of phase 2 per CTA, and two separate splits gave some
+// CTAs five.  (In phase 1 the shared units pass while the routing is still on its way, and each section is split by itself;
+// where the lists come first, `whole`, it is split like phase 2: one token, hidden 2048, expert width 512 24.9 -> 22.7 us.)
+// A CTA's share of all must not be smaller than its part of the shared ones, which holds from one routed unit per CTA on.
 // The split is by cost, not by count: staging a pass's activations takes a CTA about as long as STAGE_UNITS units, so a CTA
 // whose range crosses into another pass gets that much less (3 tokens: 66.9 -> 64.3 us, 6: 95.5 -> 91.9, 16: 148 -> 145.5;
 // 64: no difference).
+// In phase 1 all passes of one token share what is staged.
 constexpr int STAGE_UNITS = 2;
-__device__ __forceinline__ int unit_at(int v, int tiles) { // the real unit at position v of a section's cost line
-    const int q = v / (tiles + STAGE_UNITS), r = v - q * (tiles + STAGE_UNITS);
-    return q * tiles + max(r - STAGE_UNITS, 0);
+__device__ __forceinline__ int unit_at(int v, int tiles, int stage) { // the real unit at position v of a section's cost line
+    const int q = v / (tiles + stage), r = v - q * (tiles + stage);
+    return q * tiles + max(r - stage, 0);
 }
-__device__ __noinline__ int2 dec_unit_range_of(int sec, int routed, int shared, int tiles1, int tiles2) {
-    const int tiles = sec == 1 ? tiles1 : tiles2;
-    const int n_shared2 = shared * (tiles + STAGE_UNITS), n = (sec == 2 ? shared : routed) * (tiles + STAGE_UNITS);
-    const bool together = sec == 3 && n >= (int)gridDim.x && n_shared2 + n <= 16 * (int)gridDim.x;
+__device__ __noinline__ int2 dec_unit_range_of(int sec, bool whole, int t, int routed, int shared, int tiles1, int tiles2) {
+    const int tiles = sec < 2 ? tiles1 : tiles2, stage = sec < 2 && t == 1 ? 0 : STAGE_UNITS;
+    const int n_shared = shared * (tiles + stage), n = (sec & 1 ? routed : shared) * (tiles + stage);
+    const bool together = (sec == 3 || (sec == 1 && whole)) && n >= (int)gridDim.x && n_shared + n <= 16 * (int)gridDim.x;
     int a, b, c, d;
-    unit_range(together ? n_shared2 + n : n, a, b);
-    unit_range(together ? n_shared2 : 0, c, d);
-    return make_int2(unit_at(a - c, tiles), unit_at(b - d, tiles));
+    unit_range(together ? n_shared + n : n, a, b);
+    unit_range(together ? n_shared : 0, c, d);
+    return make_int2(unit_at(a - c, tiles, stage), unit_at(b - d, tiles, stage));
 }
 
 // Resolve routed pass index -> active index (the expert it belongs to).
@@ -294,14 +297,14 @@ __device__ __forceinline__ void make_pass(Pass &U, int sh_t0, int sh_nt, int top
 // block): a lane owns 8 consecutive values.
 // FROM_X: phase 1, rows of x (global, read-only); else phase 2, SwiGLU activations written by other CTAs.
 // Three of a warp's blocks at a time: their loads are in flight together and their shuffle chains overlap (one at a time a
-// pass of two tokens took 3 us, during which the CTA multiplies nothing).  Out of line: it must not disturb the register
-// allocation of the unit loops.
-template <int NDIG, int NTOK, int SUB, bool FROM_X, int NCW>
+// pass of two tokens took 3 us, during which the CTA multiplies nothing); one where a warp has no more (hidden 512, expert
+// width 256, 1 / 7 tokens: 22.9 / 24.6 -> 22.1 / 23.9 us).  Out of line: it must not disturb the register allocation of the
+// unit loops.
+template <int BATCH, int NDIG, int NTOK, int SUB, bool FROM_X, int NCW>
 __device__ __noinline__ void stage_rows(const float *rows, int k, int n_tok, int row0, int row1, int row2, int8_t *xc, __half *sh, float *sxs,
                                         int xs, int ss, int warp, int lane) {
     static_assert(NTOK <= 3, "rows of a pass");
     constexpr float QMAX = NDIG == 3 ? 524287.f : 16191.f;
-    constexpr int BATCH = 3;
     const int nblk = k / QK_K, items = n_tok * nblk;
     for (int it0 = warp; it0 < items; it0 += BATCH * NCW) {
         float v[BATCH][8];
@@ -888,6 +891,10 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
     // Between phases 1 and 2: per-pass completion counters up to 16 tokens (no grid barrier, early passes start
     // early: a few per cent at 4 and 8 tokens), a grid barrier for larger batches.
     const bool pass_flags = P.t <= LMOE_DEC_PASS_FLAG_MAX_T;
+    // A caller's decision of few pairs is made into lists before anything else (they take one warp 1.5 us), and phase 1 is then
+    // split as a whole; of more pairs behind the shared expert's units, which even out the CTAs' starts (64 tokens 344 us, lists
+    // first 357).
+    const bool lists_first = P.ext_ids != nullptr && P.t * P.top_k <= 32;
 
     if (tid == 0) {
         for (int s = 0; s < NSTAGE; s++) {
@@ -916,18 +923,28 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
             n++;
         };
         int u0, u1, u = 0;
-        // phase 1, shared expert: known before routing, and consumed before it is complete
-        unit_range_first(shared_passes * tiles1, P.ext_ids ? 0 : P.t, u0, u1);
-        if (P.ext_ids == nullptr) bar_sync(3, C::RING); // the consumers stage hidden states in the ring while they compute the logits
-        if (lane == 0) {
-            for (u = u0; u < u1; u++) {
+        // phase 1, shared expert: known before routing, and consumed before it is complete; where the lists come first, only
+        // what the ring holds can be issued before them
+        if (lists_first) {
+            const int2 r = dec_unit_range_of(0, true, P.t, 0, shared_passes, tiles1, tiles2);
+            u0 = r.x;
+            u1 = r.y;
+        } else {
+            unit_range_first(shared_passes * tiles1, P.ext_ids ? 0 : P.t, u0, u1);
+            if (P.ext_ids == nullptr) bar_sync(3, C::RING); // the consumers stage hidden states in the ring while they compute the logits
+        }
+        auto shared_fills = [&](int end) {
+            for (; u < end; u++) {
                 const int tile = u % tiles1;
                 fill(P.sh_gate + (size_t)tile * 8 * row4, P.sh_up + (size_t)tile * 8 * row4, 8 * row4);
             }
-        }
+        };
+        u = u0;
+        if (lane == 0) shared_fills(lists_first ? min(u1, u0 + NSTAGE) : u1);
         __syncwarp();
         bar_sync(2, C::THREADS); // routing tables are ready
         if (lane == 0) {
+            shared_fills(u1);
             const int n_active = s_n_active;
             u0 = s_range[1].x;
             u1 = s_range[1].y;
@@ -977,10 +994,10 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
         uint32_t m = 0; // units handed over so far (the same sequence the consumers count)
         for (int sec = 0; sec < 4; sec++) {
             const int phase = 1 + (sec >> 1), shared = (sec & 1) ^ 1;
-            if (sec == 1) bar_sync(2, C::THREADS);
+            if (sec == (lists_first ? 0 : 1)) bar_sync(2, C::THREADS);
             const int tiles = phase == 1 ? tiles1 : tiles2;
             int u0, u1;
-            if (sec == 0) unit_range_first(shared_passes * tiles, P.ext_ids ? 0 : P.t, u0, u1);
+            if (sec == 0 && !lists_first) unit_range_first(shared_passes * tiles, P.ext_ids ? 0 : P.t, u0, u1);
             else u0 = s_range[sec].x, u1 = s_range[sec].y;
             if (u0 < u1) {
                 int q = u0 / tiles, tile = u0 - q * tiles;
@@ -1081,7 +1098,7 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
     // ---- phases 1 and 2: the shared expert's units first, then the routed ones ----
     for (int sec = 0; sec < 4; sec++) {
         const int phase = 1 + (sec >> 1), shared = (sec & 1) ^ 1;
-        if (sec == 1) {
+        if (sec == (lists_first ? 0 : 1)) {
             // ---- phase 0b: the routing decision, then the per-expert token lists ----
             const uint32_t *ids_g = P.ext_ids ? P.ext_ids : P.ids_ws; // the caller's decision is taken as it is (an id >= n_expert:
             const float *w_g = P.ext_ids ? P.ext_w : P.w_ws;          // an empty slot)
@@ -1115,8 +1132,7 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
                 dec_lists<NTOK>(tk, E, P.ctrl, ids_s, cnt_s, plist_s, act_s, off_s, ppre_s, &s_n_active, &s_routed_passes, tid, CONS_THREADS);
                 if (P.lists_alias) xkey = ~0ull; // they were built over the activation cache
             }
-            if (tid >= 1 && tid < 4)
-                s_range[tid] = dec_unit_range_of(tid, s_routed_passes, shared_passes, tiles1, tiles2);
+            if (tid < 4) s_range[tid] = dec_unit_range_of(tid, lists_first, P.t, s_routed_passes, shared_passes, tiles1, tiles2);
             bar_sync(2, C::THREADS); // release the producer and the epilogue warp: the routing tables are complete
         }
         const int tiles = phase == 1 ? tiles1 : tiles2;
@@ -1131,7 +1147,7 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
         const float r0 = sum_ratio<NDIG>(2 * t4) * (phase == 1 ? 1.0f : 32.0f);
         const float r1 = sum_ratio<NDIG>(2 * t4 + 1) * (phase == 1 ? 1.0f : 32.0f);
         int u0, u1;
-        if (sec == 0) unit_range_first(shared_passes * tiles, P.ext_ids ? 0 : P.t, u0, u1);
+        if (sec == 0 && !lists_first) unit_range_first(shared_passes * tiles, P.ext_ids ? 0 : P.t, u0, u1);
         else u0 = s_range[sec].x, u1 = s_range[sec].y;
         if (u0 < u1) {
             // the section is walked pass by pass: all consumer warps stage a pass's activations together,
@@ -1150,10 +1166,15 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
                     if (phase == 2 && pass_flags && tid == 0)
                         dec_wait_pass(P.sync + SYNC_PASS0 + (shared ? q : shared_passes + q), (uint32_t)tiles1, P.ctrl, 0x200u + q);
                     bar_sync(1, CONS_THREADS); // everyone is done with the previous contents
-                    if (phase == 1)
-                        stage_rows<NDIG, NTOK, 32, true, NCW>(P.x, P.hidden, U.n_tok, U.tok[0], U.tok[1], U.tok[NTOK - 1], xc, sh, sxs, xs_ph, L.ss, warp, lane);
-                    else
-                        stage_rows<NDIG, NTOK, 16, false, NCW>(P.act_f, P.ff, U.n_tok, U.pair[0], U.pair[1], U.pair[NTOK - 1], xc, sh, sxs, xs_ph, L.ss, warp, lane);
+                    auto stage = [&](auto batch) {
+                        constexpr int B = decltype(batch)::value;
+                        if (phase == 1)
+                            stage_rows<B, NDIG, NTOK, 32, true, NCW>(P.x, P.hidden, U.n_tok, U.tok[0], U.tok[1], U.tok[NTOK - 1], xc, sh, sxs, xs_ph, L.ss, warp, lane);
+                        else
+                            stage_rows<B, NDIG, NTOK, 16, false, NCW>(P.act_f, P.ff, U.n_tok, U.pair[0], U.pair[1], U.pair[NTOK - 1], xc, sh, sxs, xs_ph, L.ss, warp, lane);
+                    };
+                    if (U.n_tok * (phase == 1 ? nb4 : nb6) <= NCW) stage(std::integral_constant<int, 1>());
+                    else stage(std::integral_constant<int, 3>());
                     xkey = key;
                     bar_sync(1, CONS_THREADS);
                 }
