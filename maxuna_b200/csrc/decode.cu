@@ -288,7 +288,7 @@ __device__ __forceinline__ void make_pass(Pass &U, int sh_t0, int sh_nt, int top
 
 // ---- activation cache staging --------------------------------------------------
 // Each value of a token's row becomes NDIG signed base-128 digits of X = round(v * QMAX / amax), amax
-// taken per 256-wide block (QMAX = 2^19 - 1 for three digits, 16191 for two: the top digit stays inside a
+// taken per 256-wide block, at least 2^-107 (QMAX = 2^19 - 1 for three digits, 16191 for two: the top digit stays inside a
 // signed byte).  Digit d (most significant first) of token tk is int8 column NDIG*tk + d of the cache, in
 // natural k order, and sxs[block][column] is the float that turns the column's integer dot product back
 // into the row's scale.  sh: SUB-wide sums of the quantized values, as f16 hi/lo pairs in columns NDIG*tk and
@@ -339,8 +339,9 @@ __device__ __noinline__ void stage_rows(const float *rows, int k, int n_tok, int
             for (int q = 0; q < BATCH; q++) amax[q] = fmaxf(amax[q], __shfl_xor_sync(0xffffffffu, amax[q], o));
 #pragma unroll
         for (int q = 0; q < BATCH; q++) {
-            const float inv = amax[q] > 0.f ? QMAX / amax[q] : 0.f;
-            const float sx = amax[q] * (1.0f / QMAX);
+            const float top = fmaxf(amax[q], 0x1p-107f); // below it the quotient is infinite; the scale is still a normal number
+            const float inv = QMAX / top;
+            const float sx = top * (1.0f / QMAX);
             int sum = 0;
             uint32_t dig[NDIG][2];
 #pragma unroll

@@ -71,7 +71,8 @@ __device__ __forceinline__ void mvs_stage_x(const float *__restrict__ x, int nb,
         for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(v[j]));
 #pragma unroll
         for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        const float inv = amax > 0.f ? QMAX / amax : 0.f;
+        amax = fmaxf(amax, 0x1p-107f); // below it the quotient is infinite; the scale is still a normal number
+        const float inv = QMAX / amax;
         const float sx = amax * (1.0f / QMAX);
         int sum = 0;
         uint32_t dig[MVS_NDIG][2];

@@ -83,6 +83,23 @@ def test_decode_at_the_shared_memory_limits(orc, dev, hidden, ff, ne, k, t):
     _check(orc, blk, blk.host_layer(orc), x, 1e-4 if t <= 8 else 5e-4)
 
 
+@pytest.mark.parametrize("t", [3, 12])
+def test_decode_tiny_activations(orc, dev, t):
+    """Blocks whose largest magnitude is near the end of the f32 range (one value among zeros, many, a subnormal): a token whose
+    whole row is that small has a result below 1e-30, and a row with one such block is served like any other."""
+    from maxuna_b200.moe import MoeBlock
+
+    blk = MoeBlock.random(512, 256, 8, 3, seed=23, device=dev, weight_std=0.2)
+    host = blk.host_layer(orc)
+    x = np.random.default_rng(24).standard_normal((t, 512)).astype(np.float32)
+    x[0] *= np.float32(1e-34)
+    x[1] = 0
+    x[1, 7], x[1, 300] = 1e-33, 1e-42
+    x[2, 256:] *= np.float32(1e-35)
+    out, _ = _check(orc, blk, host, x, 1e-4 if t <= 8 else 5e-4)
+    assert np.abs(out[:2].cpu().numpy()).max() < 1e-30
+
+
 @pytest.fixture(scope="module")
 def full_block(dev):
     from maxuna_b200.moe import MoeBlock

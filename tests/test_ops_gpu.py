@@ -202,6 +202,25 @@ def test_plain_mv_q6k_streamed(orc, dev, n_out, k, t):
     assert np.abs(got - want).max() < 1e-5 * np.abs(want).max() * 10
 
 
+@pytest.mark.parametrize("n_out,k", [(4097, 512), (4104, 256), (4111, 768), (4100, 1280), (4096 + 16 * 150 + 7, 2816)])
+def test_plain_mv_q6k_streamed_ragged(orc, dev, n_out, k):
+    """The streamed kernel, one token, with a last chunk of fewer than sixteen rows (all remainders of its bytes by 16) and odd
+    block counts of several blocks; then blocks near the end of the f32 range, as exact as 21 bits above 2^-126 are."""
+    from maxuna_b200 import ops
+
+    raw = orc.quantize(14, orc.pseudo_random(n_out * k, 71 + k, -1.0, 1.0))
+    buf = torch.zeros(raw.size + 128, dtype=torch.uint8, device=dev)
+    buf[: raw.size] = torch.from_numpy(raw).to(dev)
+    x = orc.pseudo_random(k, 9, -1.0, 1.0).reshape(1, k)
+    tiny = np.zeros_like(x)
+    tiny[0, 5], tiny[0, k - 1] = 1e-33, -3e-33
+    for v, tol in ((x, 1e-5), (tiny, 1e-4)):
+        got = ops.mul_mv(buf, 14, n_out, k, torch.from_numpy(v).to(dev)).cpu().numpy()
+        want = orc.mul_mv(14, raw, n_out, k, v)
+        scale = np.float64(1e30) if tol == 1e-4 else 1.0
+        assert np.isfinite(got).all() and orc.rel_l2(got * scale, want * scale) < tol
+
+
 @pytest.mark.parametrize("dt,name", DTYPES)
 def test_device_codec_matches_oracle(orc, dev, dt, name):
     from maxuna_b200.gguf import ExpertStack
