@@ -2,10 +2,14 @@
 // Reference: `ops::mul_mv_id`, src/ops/mv_id.rs:37-45; kernels
 // kernel_mul_mv_id_q{4,6}_K_f32_v, src/ops/mv.metal:181-290, 413-504, 638-717.
 //
-// Three kernels.  All carry the activations as three signed base-256 digits under the largest magnitude of every 256-wide
-// block (24 bits: the resolution of f32 at that magnitude) and multiply them with the raw 4- and 6-bit fields on the integer
-// tensor-core path (mma.sync u8 x s8 -> s32, exact), as the fused decode kernel does; the scales come in once per
-// super-block.  A lane-per-16-bytes f32 dot product was bound by its conversions and multiply-adds.
+// Three kernels.  All carry the activations as four signed base-256 digits of 30-bit integers under a power of two per
+// 256-wide block, and multiply them with the raw 4- and 6-bit fields on the integer tensor-core path (mma.sync u8 x s8 -> s32,
+// exact), as the fused decode kernel does; the scales come in once per super-block.  The integers hold every value within 2^6
+// of the block's largest exactly and the others to 2^-30 of it, so a product is no further from 64 bits than one of f32
+// values and sums (relative error Q4_K 0.6e-7 to 1.4e-7 against 1.7e-7 to 2.9e-7, Q6_K 0.6e-7 to 0.8e-7 against 0.8e-7 to
+// 1.0e-7, for normal and log-normal values, products of two, and one value of a block or row 100 or 10^4 times the others;
+// three digits, 24 bits under the largest magnitude: up to 13e-7, and NaN below 2.5e-32).
+// A lane-per-16-bytes f32 dot product was bound by its conversions and multiply-adds.
 //   mv_expert_kernel the ordinary case, bound by the weight stream: pairs of the same expert share a pass over its rows, which
 //                    come through shared memory in bulk copies.  Weights of 3 / 16 / 64 tokens with ten experts each, against
 //                    mv_pair_kernel: [1024 x 3072] Q4_K 17 / 78 / 290 -> 15 / 47 / 139 us, [3072 x 1024] Q6_K (whose 210-byte
@@ -21,14 +25,18 @@
 namespace {
 
 constexpr int MV_THREADS = 256, MV_ROWS = 64; // rows of a block: four MMA row tiles, the K dimension in two halves
-constexpr int MV_NDIG = 3;
-// Largest quantized magnitude: digits 127, 127, 127 is 127 * 65793; a little below, so that every digit stays in a byte.
-constexpr float MV_QMAX = 8355000.f;
-// The SUB-wide sums (|sum| <= 32 * QMAX < 2^28) enter an f16 product times 2^-13, as a high and a low part.
-constexpr float MV_SUM_SCALE = 0x1p-13f, MV_SUM_UNSCALE = 0x1p13f;
+constexpr int MV_NDIG = 4;
+// A value is an integer of magnitude <= 2^30 (the top digit stays within +-64) times its block's scale, 2^29 integers to the
+// power of two at or below the largest magnitude.
+constexpr int MV_BITS = 29;
+// The SUB-wide sums (|sum| <= 2^35) enter an f16 product times 2^-20, in three parts of eleven bits: multiples of 2^5, 2^-6 and
+// 2^-17.  With one quantum for all sub-blocks the product with the integer mins or scales is exact, a part at a time.
+constexpr int MV_PARTS = 3;
+constexpr float MV_SUM_UNSCALE = 0x1p20f;
+constexpr float MV_OFFSET = 32.f * MV_SUM_UNSCALE; // Q6_K: what the product of scales and sums stands for, in units of the integers
 
 // One 256-wide block of an activation row, by one warp (eight consecutive values per lane): digits, the block's scale, and
-// the SUB-wide sums of the quantized values as f16 high and low parts.
+// the SUB-wide sums of the quantized values as f16 parts, most significant first.
 struct MvX {
     float4 a, c;
     __device__ __forceinline__ void load(const float *__restrict__ src, bool want, int lane) { // a row not wanted counts as zero
@@ -45,40 +53,55 @@ __device__ __forceinline__ float max_nan(float a, float b) {
     return r;
 }
 template <int SUB>
-__device__ __forceinline__ void mv_digits(const MvX &in, uint2 (&dig)[MV_NDIG], float &sx, __half &hi, __half &lo) {
+__device__ __forceinline__ void mv_digits(const MvX &in, uint2 (&dig)[MV_NDIG], float &sx, __half (&part)[MV_PARTS]) {
     const float v[8] = {in.a.x, in.a.y, in.a.z, in.a.w, in.c.x, in.c.y, in.c.z, in.c.w};
     float amax = 0.f; // NaN if any value is: the block's scale, and with it the result, then is NaN too
 #pragma unroll
     for (int j = 0; j < 8; j++) amax = max_nan(amax, fabsf(v[j]));
 #pragma unroll
     for (int o = 16; o; o >>= 1) amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float inv = amax > 0.f ? MV_QMAX / amax : 0.f;
-    sx = amax * (1.0f / MV_QMAX);
-    int sum = 0;
+    // 2^e <= amax < 2^(e + 1); below 2^-97 the scale stays at the smallest normal number, so that its reciprocal exists
+    const int e = max((int)(__float_as_uint(amax) >> 23) - 127, -97);
+    const float inv = __int_as_float((127 + MV_BITS - e) << 23);
+    sx = e == 128 ? amax : __int_as_float((127 - MV_BITS + e) << 23);
+    int X[8], sum_h = 0, sum_l = 0; // sums of the upper and the lower 15 bits
+#pragma unroll
+    for (int j = 0; j < 8; j++) X[j] = __float2int_rn(v[j] * inv);
+    if (e == 128) { // an infinite value times an infinite scale; the others count nothing beside it
+#pragma unroll
+        for (int j = 0; j < 8; j++) X[j] = fabsf(v[j]) == INFINITY ? (v[j] > 0.f ? 1 << MV_BITS : -(1 << MV_BITS)) : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        sum_h += X[j] >> 15;
+        sum_l += X[j] & 0x7fff;
+    }
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         uint32_t y[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int X = __float2int_rn(v[4 * h + j] * inv);
-            sum += X;
-            y[j] = (uint32_t)(X + 0x8080); // the two low digits become plain bytes plus 128
-        }
+        for (int j = 0; j < 4; j++) y[j] = (uint32_t)(X[4 * h + j] + 0x808080); // the three low digits become plain bytes plus 128
         // byte d of the four values side by side; the 128 comes off again with the sign bit
-        const uint32_t d2 = __byte_perm(__byte_perm(y[0], y[1], 0x40), __byte_perm(y[2], y[3], 0x40), 0x5410) ^ 0x80808080u;
-        const uint32_t d1 = __byte_perm(__byte_perm(y[0], y[1], 0x51), __byte_perm(y[2], y[3], 0x51), 0x5410) ^ 0x80808080u;
-        const uint32_t d0 = __byte_perm(__byte_perm(y[0], y[1], 0x62), __byte_perm(y[2], y[3], 0x62), 0x5410);
-        if (h == 0) { dig[0].x = d0; dig[1].x = d1; dig[2].x = d2; }
-        else { dig[0].y = d0; dig[1].y = d1; dig[2].y = d2; }
+        const uint32_t d3 = __byte_perm(__byte_perm(y[0], y[1], 0x40), __byte_perm(y[2], y[3], 0x40), 0x5410) ^ 0x80808080u;
+        const uint32_t d2 = __byte_perm(__byte_perm(y[0], y[1], 0x51), __byte_perm(y[2], y[3], 0x51), 0x5410) ^ 0x80808080u;
+        const uint32_t d1 = __byte_perm(__byte_perm(y[0], y[1], 0x62), __byte_perm(y[2], y[3], 0x62), 0x5410) ^ 0x80808080u;
+        const uint32_t d0 = __byte_perm(__byte_perm(y[0], y[1], 0x73), __byte_perm(y[2], y[3], 0x73), 0x5410);
+        if (h == 0) { dig[0].x = d0; dig[1].x = d1; dig[2].x = d2; dig[3].x = d3; }
+        else { dig[0].y = d0; dig[1].y = d1; dig[2].y = d2; dig[3].y = d3; }
     }
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    if (SUB == 32) sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    const float sf = (float)sum * MV_SUM_SCALE;
-    hi = __float2half_rn(sf);
-    lo = __float2half_rn(sf - __half2float(hi));
+#pragma unroll
+    for (int o = 1; o < SUB / 8; o <<= 1) {
+        sum_h += __shfl_xor_sync(0xffffffffu, sum_h, o);
+        sum_l += __shfl_xor_sync(0xffffffffu, sum_l, o);
+    }
+    const int q0 = (sum_h + (1 << 9)) >> 10, r0 = (sum_h - (q0 << 10)) * (1 << 15) + sum_l; // |sum_h|, sum_l <= 2^20
+    const int q1 = (r0 + (1 << 13)) >> 14, r1 = r0 - (q1 << 14);
+    part[0] = __float2half_rn((float)q0 * 0x1p5f);
+    part[1] = __float2half_rn((float)q1 * 0x1p-6f);
+    part[2] = __float2half_rn((float)((r1 + 4) >> 3) * 0x1p-17f);
 }
 // weight of digit d (most significant first)
-__device__ __forceinline__ float mv_digit_weight(int d) { return d == 0 ? 65536.f : (d == 1 ? 256.f : 1.f); }
+__device__ __forceinline__ float mv_digit_weight(int d) { return d == 0 ? 16777216.f : (d == 1 ? 65536.f : (d == 2 ? 256.f : 1.f)); }
 
 // ---- raw fields of two rows of one super-block, as this lane's part of the MMA A fragments --------------------------
 // Q4_K: bytes 8t .. 8t+7 of each 32-byte run (low nibbles: sub-block 2j, high: 2j+1), and the 16-byte header.
@@ -173,8 +196,8 @@ struct MvA<LMOE_Q6_K> {
 #pragma unroll
         for (int q = 0; q < 4; q++) { scg[q] = R.sg[q]; scG[q] = R.sG[q]; }
         dg = R.dg; dG = R.dG;
-        mg = dg * (32.f * MV_SUM_UNSCALE);
-        mG = dG * (32.f * MV_SUM_UNSCALE);
+        mg = dg * MV_OFFSET;
+        mG = dG * MV_OFFSET;
         // scales 2t, 2t+1 and 2t+8, 2t+9 of each row, as f16 pairs
         auto pair = [&](const uint32_t (&s)[4], int w) {
             const uint32_t v = t >= 2 ? s[2 * w + 1] : s[2 * w];
@@ -218,7 +241,7 @@ constexpr int MV_PAIR_BLOCKS = 32; // super-blocks of the activation row staged 
 
 // ---- one pair -------------------------------------------------------------------------
 // grid (ceil(n_out / 64), pairs), eight warps: row tile = warp % 4, K half = warp / 4.
-// MMA columns 0-2: the digits; 3-7 repeat column 0 and are not read.
+// MMA columns 0-3: the digits; 4-7 repeat column 0 and are not read.
 template <int DT>
 __global__ void __launch_bounds__(MV_THREADS, 2)
 mv_pair_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *__restrict__ x,
@@ -239,15 +262,15 @@ mv_pair_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert
     }
     const int bc = min(nb, MV_PAIR_BLOCKS), pitch = bc * QK_K + 32; // super-blocks staged at a time, bytes of a digit column
     int8_t *xc = reinterpret_cast<int8_t *>(mv_smem);
-    __half *sh = reinterpret_cast<__half *>(mv_smem + 3 * pitch);
-    float *sxs = reinterpret_cast<float *>(mv_smem + 3 * pitch + 2 * bc * NS * 2);
+    __half *sh = reinterpret_cast<__half *>(mv_smem + MV_NDIG * pitch);
+    float *sxs = reinterpret_cast<float *>(mv_smem + MV_NDIG * pitch + MV_PARTS * bc * NS * 2);
     const int rt = warp & 3, ks = warp >> 2;
     const int rg = min(r_base + 16 * rt + g, n_out - 1), rG = min(r_base + 16 * rt + g + 8, n_out - 1);
     const uint8_t *wb = w + (size_t)e * expert_bytes;
     const uint8_t *pg = wb + (size_t)rg * row_bytes, *pG = wb + (size_t)rG * row_bytes;
     const float *xr = x + ((size_t)(pair / top_k) * x_per_row + (x_per_row == 1 ? 0 : pair % top_k)) * k;
-    const int8_t *xcol = xc + (g < 3 ? g : 0) * pitch;
-    const __half *scol = sh + (g == 1 ? bc * NS : 0); // column 0: high parts, column 1: low parts
+    const int8_t *xcol = xc + (g < MV_NDIG ? g : 0) * pitch;
+    const __half *scol = sh + (g < MV_PARTS ? g : 0) * bc * NS; // columns 0-2: the parts of the sums
     float yg = 0.f, yG = 0.f;
     for (int c0 = 0; c0 < nb; c0 += bc) {
         const int bn = min(bc, nb - c0);
@@ -257,15 +280,15 @@ mv_pair_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert
         for (int b = warp; b < bn; b += MV_THREADS / 32) {
             uint2 dig[MV_NDIG];
             float sx;
-            __half hi, lo;
+            __half part[MV_PARTS];
             MvX in;
             in.load(xr + (size_t)(c0 + b) * QK_K, true, lane);
-            mv_digits<SUB>(in, dig, sx, hi, lo);
+            mv_digits<SUB>(in, dig, sx, part);
 #pragma unroll
             for (int d = 0; d < MV_NDIG; d++) *reinterpret_cast<uint2 *>(xc + d * pitch + b * QK_K + lane * 8) = dig[d];
             if ((lane & (SUB / 8 - 1)) == 0) {
-                sh[b * NS + lane / (SUB / 8)] = hi;
-                sh[bc * NS + b * NS + lane / (SUB / 8)] = lo;
+#pragma unroll
+                for (int h = 0; h < MV_PARTS; h++) sh[(h * bc + b) * NS + lane / (SUB / 8)] = part[h];
             }
             if (lane == 0) sxs[b] = sx;
         }
@@ -286,10 +309,11 @@ mv_pair_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert
                 const int sg = A.sg(i), sG = A.sG(i);
                 al[0] += sg * f[0]; al[1] += sg * f[1]; al[2] += sG * f[2]; al[3] += sG * f[3];
             }
-            // lane t = 0 holds columns 0, 1 (and both halves of the sums), lane t = 1 column 2
-            const float f0 = t == 0 ? 65536.f : (t == 1 ? 1.f : 0.f), f1 = t == 0 ? 256.f : 0.f, fm = t == 0 ? 1.f : 0.f, sx = sxs[b];
-            yg += sx * (A.dg * (f0 * (float)al[0] + f1 * (float)al[1]) - A.mg * (fm * (cm[0] + cm[1])));
-            yG += sx * (A.dG * (f0 * (float)al[2] + f1 * (float)al[3]) - A.mG * (fm * (cm[2] + cm[3])));
+            // lane t = 0 holds columns 0, 1, lane t = 1 columns 2, 3 (no part of the sums in 3)
+            const float f0 = t == 0 ? 16777216.f : (t == 1 ? 256.f : 0.f), f1 = t == 0 ? 65536.f : (t == 1 ? 1.f : 0.f), sx = sxs[b];
+            const float m0 = t < 2 ? 1.f : 0.f, m1 = t == 0 ? 1.f : 0.f;
+            yg += sx * (A.dg * (f0 * (float)al[0] + f1 * (float)al[1]) - A.mg * (m0 * cm[0] + m1 * cm[1]));
+            yG += sx * (A.dG * (f0 * (float)al[2] + f1 * (float)al[3]) - A.mG * (m0 * cm[2] + m1 * cm[3]));
         }
     }
     yg += __shfl_xor_sync(0xffffffffu, yg, 1);
@@ -303,11 +327,11 @@ mv_pair_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert
 }
 
 // ---- many pairs of one matrix -----------------------------------------------------------
-// grid (ceil(n_out / 64), ceil(pairs / 32)); the same warp layout.  The digits of 32 pairs are staged 1024 k at a time.  Making
+// grid (ceil(n_out / 64), ceil(pairs / 32)); the same warp layout.  The digits of 32 pairs are staged 512 k at a time.  Making
 // them was half of the instructions, so the CS blocks of a cluster, row blocks of the same pairs, make a share each and store
 // it to all of them through distributed shared memory (512 pairs: [1024 x 3072] Q4_K 70 -> 52 us,
 // [3072 x 1024] Q6_K 102 -> 90).
-constexpr int MM_COLS = 32, MM_KC = 1024;
+constexpr int MM_COLS = 32, MM_KC = 512;
 // bytes of a pair's digits: the columns of one load instruction (8 bytes a lane for Q4_K, 4 for Q6_K) cover distinct banks
 template <int DT>
 constexpr int MM_PITCH = MV_NDIG * MM_KC + (DT == LMOE_Q4_K ? 32 : 16);
@@ -322,7 +346,7 @@ mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
     extern __shared__ __align__(16) uint8_t mv_smem[];
     int8_t *xc = reinterpret_cast<int8_t *>(mv_smem);                                                    // [pair][digit][k]
     __half *sh = reinterpret_cast<__half *>(mv_smem + MM_COLS * MM_PITCH<DT>);                           // [part][pair][SP]
-    float *sxs = reinterpret_cast<float *>(mv_smem + MM_COLS * MM_PITCH<DT> + 2 * MM_COLS * SP * 2);     // [block][pair]
+    float *sxs = reinterpret_cast<float *>(mv_smem + MM_COLS * MM_PITCH<DT> + MV_PARTS * MM_COLS * SP * 2); // [block][pair]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int p0 = blockIdx.y * MM_COLS, np = min(MM_COLS, pairs - p0), nb = k / QK_K;
     const int64_t row_bytes = (int64_t)nb * TS;
@@ -353,8 +377,8 @@ mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
                     ids == nullptr || ids[pair] == 0u, lane);
             uint2 dig[MV_NDIG];
             float sx;
-            __half hi, lo;
-            mv_digits<SUB>(in, dig, sx, hi, lo);
+            __half part[MV_PARTS];
+            mv_digits<SUB>(in, dig, sx, part);
 #pragma unroll
             for (int r = 0; r < CS; r++) {
                 int8_t *xr = CS > 1 ? cl.map_shared_rank(xc, r) : xc;
@@ -363,29 +387,26 @@ mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
 #pragma unroll
                 for (int d = 0; d < MV_NDIG; d++) *reinterpret_cast<uint2 *>(xr + p * MM_PITCH<DT> + d * MM_KC + b * QK_K + lane * 8) = dig[d];
                 if ((lane & (SUB / 8 - 1)) == 0) {
-                    hr[p * SP + b * NS + lane / (SUB / 8)] = hi;
-                    hr[(MM_COLS + p) * SP + b * NS + lane / (SUB / 8)] = lo;
+#pragma unroll
+                    for (int h = 0; h < MV_PARTS; h++) hr[(h * MM_COLS + p) * SP + b * NS + lane / (SUB / 8)] = part[h];
                 }
                 if (lane == 0) fr[b * MM_COLS + p] = sx;
             }
         }
         sync_all();
-        for (int b = ks; b < bn; b += 2) {
+        static_assert(BC == 2, "a block for each half");
+        if (const int b = ks; b < bn) {
             MvA<DT> A;
             A.unpack(raw, t);
-            if (b + 2 < bn) raw.load(pg + (size_t)(b0 + b + 2) * TS, pG + (size_t)(b0 + b + 2) * TS, t);
 #pragma unroll
             for (int c = 0; c < MM_COLS / 8; c++) {
                 if (8 * c < np) { // columns past the last pair hold whatever was there: their results are not written
                     const int8_t *xp = xc + (8 * c + g) * MM_PITCH<DT> + b * QK_K;
-                    float cm[4] = {0.f, 0.f, 0.f, 0.f}, tot[4] = {0.f, 0.f, 0.f, 0.f};
+                    // digits from the least significant on, so that only the last addition rounds at the size of the sum.  The
+                    // Q6_K offset comes off digit by digit: both terms are exact, and larger than their difference.
+                    float sum[4] = {0.f, 0.f, 0.f, 0.f}, tot[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const __half *sp = sh + (h * MM_COLS + 8 * c + g) * SP + b * NS + 2 * t;
-                        mma16816_acc(cm, A.f, *reinterpret_cast<const uint32_t *>(sp), NS == 16 ? *reinterpret_cast<const uint32_t *>(sp + 8) : 0u);
-                    }
-#pragma unroll
-                    for (int d = 0; d < MV_NDIG; d++) {
+                    for (int d = MV_NDIG - 1; d >= 0; d--) {
                         int al[4] = {0, 0, 0, 0};
 #pragma unroll
                         for (int i = 0; i < MvA<DT>::N; i++) {
@@ -394,14 +415,22 @@ mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
                             const int sg = A.sg(i), sG = A.sG(i);
                             al[0] += sg * f[0]; al[1] += sg * f[1]; al[2] += sG * f[2]; al[3] += sG * f[3];
                         }
+                        float cm[4] = {0.f, 0.f, 0.f, 0.f};
+                        if (d < MV_PARTS) {
+                            const __half *sp = sh + (d * MM_COLS + 8 * c + g) * SP + b * NS + 2 * t;
+                            mma16816_acc(cm, A.f, *reinterpret_cast<const uint32_t *>(sp), NS == 16 ? *reinterpret_cast<const uint32_t *>(sp + 8) : 0u);
+                        }
 #pragma unroll
-                        for (int i = 0; i < 4; i++) tot[i] += mv_digit_weight(d) * (float)al[i];
+                        for (int i = 0; i < 4; i++) {
+                            if (DT == LMOE_Q6_K) tot[i] += __fmaf_rn(mv_digit_weight(d), (float)al[i], -MV_OFFSET * cm[i]);
+                            else tot[i] += mv_digit_weight(d) * (float)al[i], sum[i] += cm[i];
+                        }
                     }
                     const float2 sx = *reinterpret_cast<const float2 *>(sxs + b * MM_COLS + 8 * c + 2 * t);
-                    acc[c][0] += sx.x * (A.dg * tot[0] - A.mg * cm[0]);
-                    acc[c][1] += sx.y * (A.dg * tot[1] - A.mg * cm[1]);
-                    acc[c][2] += sx.x * (A.dG * tot[2] - A.mG * cm[2]);
-                    acc[c][3] += sx.y * (A.dG * tot[3] - A.mG * cm[3]);
+                    acc[c][0] += sx.x * (A.dg * tot[0] - A.mg * sum[0]);
+                    acc[c][1] += sx.y * (A.dg * tot[1] - A.mg * sum[1]);
+                    acc[c][2] += sx.x * (A.dG * tot[2] - A.mG * sum[2]);
+                    acc[c][3] += sx.y * (A.dG * tot[3] - A.mG * sum[3]);
                 }
             }
         }
@@ -432,15 +461,15 @@ mv_multi_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
 // grid (row splits, pairs): a block serves one expert's next 2 * NT pairs (its "leader" is the first of them; the blocks of
 // the others leave at once) on a range of row units.  A unit is 16 * m whole rows, contiguous in memory: a producer warp keeps
 // a ring of units filled with one bulk copy each, NG groups of four warps take them in turn and split a unit over K (and
-// over its row tiles when a row has fewer than four super-blocks).  Two pairs share one MMA (four columns each: the three
-// digits and a spare), so a super-block is unpacked once for 2 * NT pairs;
+// over its row tiles when a row has fewer than four super-blocks).  Two pairs share one MMA (four columns each: their
+// digits), so a super-block is unpacked once for 2 * NT pairs;
 // four pairs a block measured no better than two where the weights of the second pass come from the L2 cache.
 constexpr int MX_GW = 4;                                    // warps of a group
 constexpr int MX_STAGES = 8;                                // most ring stages
 constexpr int MX_WINDOW = 2048;                             // pairs of one expert are looked for among this many
 constexpr int MX_UNIT = 28 * 1024;                          // a unit has as many row tiles as fit here (at least what the warps need)
 constexpr int64_t MX_L2 = 100 << 20;                          // what of the 126 MB L2 cache a matrix may hope for
-constexpr int MX_SMEM_ONE = 226 * 1024, MX_SMEM_TWO = 112 * 1024; // dynamic shared memory of one / two blocks a SM
+constexpr int MX_SMEM_ONE = 227 * 1024 - 128, MX_SMEM_TWO = 112 * 1024; // dynamic shared memory of one / two blocks a SM
 
 struct MxLayout {
     int pitch, ns, kw, m, unit_bytes, stride, nstage, o_sum, o_sx, o_red, o_bar, o_ring, total;
@@ -452,9 +481,9 @@ struct MxLayout {
         m = 4 / kw;
         while (2 * m * kw <= 8 && 32 * m * row_bytes <= MX_UNIT) m *= 2;
         unit_bytes = 16 * m * row_bytes;
-        stride = (unit_bytes + 16 + 127) / 128 * 128; // 16 spare bytes: an aligned two-word read may end past the last block
+        stride = (unit_bytes + (q4 ? 0 : 16) + 127) / 128 * 128; // Q6_K: an aligned two-word read may end past the last block
         int o = np * MV_NDIG * pitch;
-        o_sum = o; o += np * 2 * nb * ns * 2;
+        o_sum = o; o += np * MV_PARTS * nb * ns * 2;
         o_sx = o; o += (np * nb * 4 + 15) / 16 * 16;
         o_red = o; o += ng * 2 * kw * np * 16 * m * 4;
         o_bar = o; o += 2 * MX_STAGES * 8 + 16;
@@ -466,16 +495,22 @@ struct MxLayout {
 };
 
 // One super-block of two rows against the digits of 2 * NT pairs.  y[j]: this lane's pair of column tile j, rows g and G;
-// lanes of even t hold the two high digits (and the sums), lanes of odd t the low one.
-template <int NT>
+// lanes of even t hold the two high digits and parts of the sums, lanes of odd t the low ones (no part in the last column).
+template <int DT, int NT>
 __device__ __forceinline__ void mx_finish(const int (&al)[NT][4], const float (&cm)[NT][4], float dg, float dG, float mg, float mG, int b, int t,
                                           const float *const (&sxp)[NT], float (&y)[NT][2]) {
-    const float f0 = (t & 1) ? 1.f : 65536.f, f1 = (t & 1) ? 0.f : 256.f, fm = (t & 1) ? 0.f : 1.f;
+    const float f0 = (t & 1) ? 256.f : 16777216.f, f1 = (t & 1) ? 1.f : 65536.f, m1 = (t & 1) ? 0.f : 1.f;
 #pragma unroll
     for (int j = 0; j < NT; j++) {
         const float sx = sxp[j][b];
-        y[j][0] += sx * (dg * (f0 * (float)al[j][0] + f1 * (float)al[j][1]) - mg * (fm * (cm[j][0] + cm[j][1])));
-        y[j][1] += sx * (dG * (f0 * (float)al[j][2] + f1 * (float)al[j][3]) - mG * (fm * (cm[j][2] + cm[j][3])));
+        if (DT == LMOE_Q6_K) { // the offset comes off digit by digit: both terms are exact, and larger than their difference
+            const float k1 = m1 * -MV_OFFSET;
+            y[j][0] += sx * dg * (__fmaf_rn(f0, (float)al[j][0], -MV_OFFSET * cm[j][0]) + __fmaf_rn(f1, (float)al[j][1], k1 * cm[j][1]));
+            y[j][1] += sx * dG * (__fmaf_rn(f0, (float)al[j][2], -MV_OFFSET * cm[j][2]) + __fmaf_rn(f1, (float)al[j][3], k1 * cm[j][3]));
+        } else {
+            y[j][0] += sx * (dg * (f0 * (float)al[j][0] + f1 * (float)al[j][1]) - mg * (cm[j][0] + m1 * cm[j][1]));
+            y[j][1] += sx * (dG * (f0 * (float)al[j][2] + f1 * (float)al[j][3]) - mG * (cm[j][2] + m1 * cm[j][3]));
+        }
     }
 }
 template <int NT>
@@ -509,7 +544,7 @@ __device__ __forceinline__ void mx_q4k(const uint8_t *bg, const uint8_t *bG, int
             al[j][0] += sg * f[0]; al[j][1] += sg * f[1]; al[j][2] += sG * f[2]; al[j][3] += sG * f[3];
         }
     }
-    mx_finish<NT>(al, cm, A.dg, A.dG, A.mg, A.mG, b, t, sxp, y);
+    mx_finish<LMOE_Q4_K, NT>(al, cm, A.dg, A.dG, A.mg, A.mG, b, t, sxp, y);
 }
 template <int NT, int MIS>
 __device__ __forceinline__ void mx_q6k(const uint8_t *bg, const uint8_t *bG, int b, int t, const int8_t *const (&xcol)[NT],
@@ -555,7 +590,7 @@ __device__ __forceinline__ void mx_q6k(const uint8_t *bg, const uint8_t *bG, int
             }
         }
     }
-    mx_finish<NT>(al, cm, dg, dG, dg * (32.f * MV_SUM_UNSCALE), dG * (32.f * MV_SUM_UNSCALE), b, t, sxp, y);
+    mx_finish<LMOE_Q6_K, NT>(al, cm, dg, dG, 0.f, 0.f, b, t, sxp, y);
 }
 
 struct MxArgs {
@@ -584,8 +619,8 @@ __device__ __forceinline__ void mx_units(const MxArgs P, const MxLayout L, int w
 #pragma unroll
     for (int j = 0; j < NT; j++) {
         const int pb = 2 * j + (g >> 2), po = 2 * j + (t >> 1); // pair of this lane's B column, and of its accumulators
-        xcol[j] = P.xc + ((pb < P.np ? pb : 0) * MV_NDIG + min(g & 3, MV_NDIG - 1)) * L.pitch;
-        scol[j] = P.sums + ((pb < P.np ? pb : 0) * 2 + ((g & 3) == 1)) * nb * L.ns;
+        xcol[j] = P.xc + ((pb < P.np ? pb : 0) * MV_NDIG + (g & 3)) * L.pitch;
+        scol[j] = P.sums + ((pb < P.np ? pb : 0) * MV_PARTS + min(g & 3, MV_PARTS - 1)) * nb * L.ns;
         sxp[j] = P.sxs + (po < P.np ? po : 0) * nb;
     }
     // Q6_K rows 2g and 2g + 1 where they are word aligned: the eight rows of a load sit in disjoint banks
@@ -722,14 +757,14 @@ mv_expert_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expe
         if (i + CONS_WARPS < np * nb) next.load(src(i + CONS_WARPS), true, lane);
         uint2 dig[MV_NDIG];
         float sx;
-        __half hi, lo;
-        mv_digits<SUB>(in, dig, sx, hi, lo);
+        __half part[MV_PARTS];
+        mv_digits<SUB>(in, dig, sx, part);
         in = next;
 #pragma unroll
         for (int d = 0; d < MV_NDIG; d++) *reinterpret_cast<uint2 *>(xc + (p * MV_NDIG + d) * L.pitch + b * QK_K + lane * 8) = dig[d];
         if ((lane & (SUB / 8 - 1)) == 0) {
-            sums[(2 * p) * nb * NS + b * NS + lane / (SUB / 8)] = hi;
-            sums[(2 * p + 1) * nb * NS + b * NS + lane / (SUB / 8)] = lo;
+#pragma unroll
+            for (int h = 0; h < MV_PARTS; h++) sums[((MV_PARTS * p + h) * nb + b) * NS + lane / (SUB / 8)] = part[h];
         }
         if (lane == 0) sxs[p * nb + b] = sx;
     }
@@ -803,7 +838,7 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
     // block win by parallelism: [1024 x 3072] Q4_K, 64 / 512 pairs 26 / 88 us against 55 / 52, [3072 x 1024] Q6_K, 32 / 128
     // pairs 16 / 42 against 27 / 33.)
     if (n_expert == 1 && (pairs + MM_COLS - 1) / MM_COLS * gx >= sms && pairs > 4) {
-        constexpr int smem = MM_COLS * MM_PITCH<DT> + 2 * MM_COLS * (MM_KC / QK_K * NS + 8) * 2 + (MM_KC / QK_K) * MM_COLS * 4;
+        constexpr int smem = MM_COLS * MM_PITCH<DT> + MV_PARTS * MM_COLS * (MM_KC / QK_K * NS + 8) * 2 + (MM_KC / QK_K) * MM_COLS * 4;
         constexpr int CS = 4;
         static thread_local int c_dev = -1;
         if (dev != c_dev) {
@@ -830,7 +865,7 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
         if (r != cudaErrorNotSupported) return r;
     }
     const int bc = k / QK_K < MV_PAIR_BLOCKS ? k / QK_K : MV_PAIR_BLOCKS;
-    const int smem_pair = 3 * (bc * QK_K + 32) + 2 * bc * NS * 2 + bc * 4; // at most 27 KB
+    const int smem_pair = MV_NDIG * (bc * QK_K + 32) + MV_PARTS * bc * NS * 2 + bc * 4; // at most 36 KB
     // grid.y is limited to 65535: fold large pair counts over several launches
     const int64_t step = 65535 / top_k * top_k;
     for (int64_t p = 0; p < pairs; p += step) {

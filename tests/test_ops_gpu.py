@@ -169,6 +169,39 @@ def test_mv_many_pairs_of_one_matrix(orc, dev, dt, name, n_out, k, pairs):
     assert not got[ids == 1].any() and orc.rel_l2(got, want) < 1e-5
 
 
+@pytest.mark.parametrize("n_expert,n_out,k,t,top_k", [(4, 512, 768, 17, 2), (1, 1100, 512, 285, 1), (1, 64, 8192, 40, 1)])
+@pytest.mark.parametrize("dt,name", DTYPES)
+def test_mv_range_and_resolution(orc, dev, dt, name, n_expert, n_out, k, t, top_k):
+    """The forms for pairs by expert, for one matrix and for long rows, with activations that have one value of a block 10^4
+    times the others, that are products (as SwiGLU's are), and that span the range of f32.  Bound against 64-bit sums: values
+    are held to 2^-30 of their block's largest, and a result is some eight f32 roundings away from exact sums of up to twice
+    its size; blocks below 2^-97 are held to 2^-126.  Infinities and NaN stay in their rows."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    raw = orc.quantize(dt, orc.pseudo_random(n_expert * n_out * k, 0xA00 + k, -1.0, 1.0))
+    stack = ExpertStack.from_bytes(raw, dt, n_expert, n_out, k, device=dev)
+    rng = np.random.default_rng(k)
+    ids = (np.arange(t * top_k, dtype=np.uint32) % n_expert).reshape(t, top_k)
+    run = lambda v: ops.mul_mv_id(stack, torch.from_numpy(v).to(dev), torch.from_numpy(ids.astype(np.int32)).to(dev)).cpu().numpy()
+    x = rng.standard_normal((t, 1, k)).astype(np.float32)
+    x[0::3, 0, 7::256] *= 1e4
+    x[1::3] *= rng.standard_normal(x[1::3].shape).astype(np.float32)
+    x[2::3] *= (2.0 ** rng.integers(-60, 60, (len(x[2::3]), 1, 1))).astype(np.float32)
+    got, want = run(x), orc.mul_id(dt, raw, n_expert, n_out, k, x, ids, accum64=True)
+    for r in range(t):
+        scale = 1.0 / np.abs(want[r]).max()
+        assert orc.rel_l2(got[r] * scale, want[r] * scale) < 8 * 2.0 ** -24
+    tiny = np.zeros_like(x)
+    tiny[:, 0, 5], tiny[0, 0, 300], tiny[1, 0, 9] = 1e-33, 1e-42, 3e-34
+    got, want = run(tiny), orc.mul_id(dt, raw, n_expert, n_out, k, tiny, ids, accum64=True)
+    assert np.isfinite(got).all() and orc.rel_l2(got * np.float64(1e30), want * np.float64(1e30)) < 1e-4
+    base = run(x)
+    x[3, 0, 40], x[5, 0, 11] = np.inf, np.nan
+    got, keep = run(x), [r for r in range(t) if r not in (3, 5)]
+    assert not np.isfinite(got[3]).any() and np.isnan(got[5]).all() and np.array_equal(got[keep], base[keep])
+
+
 @pytest.mark.parametrize("dt,name", DTYPES)
 def test_plain_mv(orc, dev, dt, name):
     from maxuna_b200 import ops
