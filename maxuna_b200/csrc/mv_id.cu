@@ -2,20 +2,23 @@
 // Reference: `ops::mul_mv_id`, src/ops/mv_id.rs:37-45; kernels
 // kernel_mul_mv_id_q{4,6}_K_f32_v, src/ops/mv.metal:181-290, 413-504, 638-717.
 //
-// Three kernels.  All carry the activations as four signed base-256 digits of 30-bit integers under a power of two per
+// Four kernels.  Three carry the activations as four signed base-256 digits of 30-bit integers under a power of two per
 // 256-wide block, and multiply them with the raw 4- and 6-bit fields on the integer tensor-core path (mma.sync u8 x s8 -> s32,
 // exact), as the fused decode kernel does; the scales come in once per super-block.  The integers hold every value within 2^6
 // of the block's largest exactly and the others to 2^-30 of it, so a product is no further from 64 bits than one of f32
 // values and sums (relative error Q4_K 0.6e-7 to 1.4e-7 against 1.7e-7 to 2.9e-7, Q6_K 0.6e-7 to 0.8e-7 against 0.8e-7 to
 // 1.0e-7, for normal and log-normal values, products of two, and one value of a block or row 100 or 10^4 times the others;
 // three digits, 24 bits under the largest magnitude: up to 13e-7, and NaN below 2.5e-32).
-// A lane-per-16-bytes f32 dot product was bound by its conversions and multiply-adds.
+// A lane-per-16-bytes f32 dot product is bound by its conversions and multiply-adds, but has nothing to set up:
+//   mv_row_kernel    f32 activations and sums, a warp per row: little work, few rows, and Q6_K rows that the ring does not
+//                    take (see mv_rows_better).
+// The others:
 //   mv_expert_kernel the ordinary case, bound by the weight stream: pairs of the same expert share a pass over its rows, which
 //                    come through shared memory in bulk copies.  Weights of 3 / 16 / 64 tokens with ten experts each, against
 //                    mv_pair_kernel: [1024 x 3072] Q4_K 17 / 78 / 290 -> 15 / 47 / 139 us, [3072 x 1024] Q6_K (whose 210-byte
 //                    super-blocks cost two loads a word from global memory) 39 / 203 / 810 -> 22 / 74 / 218 us.
-//   mv_pair_kernel   any shape, one (token, slot) pair per block row; what is left to it are rows too long for the ring and
-//                    matrices off a 16-byte boundary.  Weights go straight from global memory into the A fragments.
+//   mv_pair_kernel   Q4_K of any shape, one (token, slot) pair per block row; what is left to it are rows too long for the
+//                    ring.  Weights go straight from global memory into the A fragments.
 //   mv_multi_kernel  many pairs of ONE weight matrix (the shared expert, a plain matrix): eight pairs are the columns of
 //                    an MMA, so a super-block is unpacked once for 32 pairs.  512 pairs of [1024 x 3072] Q4_K: 830 -> 52 us.
 #include <cooperative_groups.h>
@@ -238,6 +241,91 @@ __device__ __forceinline__ void mma16816_acc(float (&d)[4], const uint32_t (&a)[
 }
 
 constexpr int MV_PAIR_BLOCKS = 32; // super-blocks of the activation row staged at a time (8192 values)
+
+// ---- a warp per row -------------------------------------------------------------------
+// grid (ceil(n_out / 8), pairs): lanes stride over 16-byte pieces of the row, decode in registers, multiply f32 activations.
+constexpr int MR_WARPS = 4, MR_ROWS = 2; // rows of a warp
+
+__device__ __forceinline__ float dot_row_q4k(const uint8_t *__restrict__ row, const float *__restrict__ x, int nb, int lane) {
+    float acc = 0.f;
+    for (int u = lane; u < nb * 8; u += 32) {
+        const int b = u >> 3, c = u & 7, j = c >> 1, h = c & 1;
+        const uint8_t *blk = row + (size_t)b * Q4K_BYTES;
+        const uint32_t dm = __ldg(reinterpret_cast<const uint32_t *>(blk));
+        const float d = lmoe_h2f((uint16_t)(dm & 0xffff)), dmin = lmoe_h2f((uint16_t)(dm >> 16));
+        int sc0, mn0, sc1, mn1;
+        q4k_scale_min(blk + 4, 2 * j, sc0, mn0);
+        q4k_scale_min(blk + 4, 2 * j + 1, sc1, mn1);
+        const uint4 qv = __ldg(reinterpret_cast<const uint4 *>(blk + 16 + 16 * c));
+        const uint32_t qw[4] = {qv.x, qv.y, qv.z, qv.w};
+        const float *xl = x + (size_t)b * QK_K + 64 * j + 16 * h, *xh = xl + 32;
+        float slo = 0.f, shi = 0.f, xsl = 0.f, xsh = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            const float4 a = __ldg(reinterpret_cast<const float4 *>(xl + 4 * w)), g = __ldg(reinterpret_cast<const float4 *>(xh + 4 * w));
+            const uint32_t q = qw[w];
+            slo += a.x * (float)(q & 15) + a.y * (float)((q >> 8) & 15) + a.z * (float)((q >> 16) & 15) + a.w * (float)((q >> 24) & 15);
+            shi += g.x * (float)((q >> 4) & 15) + g.y * (float)((q >> 12) & 15) + g.z * (float)((q >> 20) & 15) + g.w * (float)(q >> 28);
+            xsl += a.x + a.y + a.z + a.w;
+            xsh += g.x + g.y + g.z + g.w;
+        }
+        acc += d * ((float)sc0 * slo + (float)sc1 * shi) - dmin * ((float)mn0 * xsl + (float)mn1 * xsh);
+    }
+    return acc;
+}
+
+__device__ __forceinline__ float dot_row_q6k(const uint8_t *__restrict__ row, const float *__restrict__ x, int nb, int lane) {
+    float acc = 0.f;
+    for (int u = lane; u < nb * 16; u += 32) {
+        const int b = u >> 4, n = (u >> 3) & 1, lg = u & 7;
+        const uint8_t *blk = row + (size_t)b * Q6K_BYTES;
+        const uint32_t qa = ld_u32_unaligned2(blk + 64 * n + 4 * lg), qb = ld_u32_unaligned2(blk + 64 * n + 32 + 4 * lg);
+        const uint32_t qh = ld_u32_unaligned2(blk + 128 + 32 * n + 4 * lg);
+        const int8_t *sc = reinterpret_cast<const int8_t *>(blk + 192) + 8 * n + (lg >> 2);
+        const float d = lmoe_h2f(*reinterpret_cast<const uint16_t *>(blk + 208));
+        const float *xp = x + (size_t)b * QK_K + 128 * n + 4 * lg;
+        float xa[4][4], s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(xp + 32 * g));
+            xa[g][0] = v.x; xa[g][1] = v.y; xa[g][2] = v.z; xa[g][3] = v.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int h = (qh >> (8 * i)) & 0xff, a = (qa >> (8 * i)) & 0xff, c = (qb >> (8 * i)) & 0xff;
+            s[0] += xa[0][i] * (float)(((a & 15) | ((h & 3) << 4)) - 32);
+            s[1] += xa[1][i] * (float)(((c & 15) | (((h >> 2) & 3) << 4)) - 32);
+            s[2] += xa[2][i] * (float)(((a >> 4) | (((h >> 4) & 3) << 4)) - 32);
+            s[3] += xa[3][i] * (float)(((c >> 4) | (((h >> 6) & 3) << 4)) - 32);
+        }
+        acc += d * ((float)sc[0] * s[0] + (float)sc[2] * s[1] + (float)sc[4] * s[2] + (float)sc[6] * s[3]);
+    }
+    return acc;
+}
+
+template <int DT>
+__global__ void __launch_bounds__(MR_WARPS * 32)
+mv_row_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *__restrict__ x,
+              int x_per_row, const uint32_t *__restrict__ ids, int top_k, float *__restrict__ out) {
+    pdl_begin();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pair = blockIdx.y, nb = k / QK_K;
+    const uint32_t e = ids ? ids[pair] : 0u;
+    const int64_t row_bytes = (int64_t)nb * (DT == LMOE_Q4_K ? Q4K_BYTES : Q6K_BYTES);
+    const float *xr = x + ((size_t)(pair / top_k) * x_per_row + (x_per_row == 1 ? 0 : pair % top_k)) * k;
+    const int r0 = (blockIdx.x * MR_WARPS + warp) * MR_ROWS;
+#pragma unroll
+    for (int r = 0; r < MR_ROWS; r++) {
+        if (r0 + r >= n_out) break;
+        float v = 0.f;
+        if (e < (uint32_t)n_expert) { // an out-of-range id produces a zero row
+            const uint8_t *row = w + (size_t)e * expert_bytes + (size_t)(r0 + r) * row_bytes;
+            v = DT == LMOE_Q4_K ? dot_row_q4k(row, xr, nb, lane) : dot_row_q6k(row, xr, nb, lane);
+#pragma unroll
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        }
+        if (lane == 0) out[(size_t)pair * n_out + r0 + r] = v;
+    }
+}
 
 // ---- one pair -------------------------------------------------------------------------
 // grid (ceil(n_out / 64), pairs), eight warps: row tile = warp % 4, K half = warp / 4.
@@ -821,9 +909,36 @@ cudaError_t launch_mv_by_expert(const uint8_t *w, int64_t expert_bytes, int n_ex
     return r;
 }
 
+// Where the warp-per-row kernel is the faster one.  The others begin with 2 us of setting up digits, ring and barriers, which
+// pays from a number of rows (pairs times rows of the matrix) on that falls with a row's length, and they work on 16 rows or
+// more at a time.  Row kernel against the others: Q4_K [1024 x 512], 4 / 8 pairs 3.7 / 5.0 us against 4.2 / 4.3,
+// [1024 x 3072], 1 / 4 pairs 5.0 / 9.7 against 5.2 / 7.3, [7 x 512], 1024 pairs 4.7 against 14.4; Q6_K [1024 x 1024],
+// 4 / 16 pairs 4.3 / 9.6 against 5.2 / 8.6, [256 x 2048], 1 / 64 pairs 5.4 / 15.6 against 5.0 / 13.4.
+template <int DT>
+bool mv_rows_better(int64_t pairs, int n_out, int k) {
+    const int64_t rows = pairs * n_out;
+    if (DT == LMOE_Q4_K)
+        return rows < (k < 1024 ? 8192 : (k < 2048 ? 4096 : (k < 3072 ? 2560 : 2048))) || n_out < (k < 2048 ? 32 : 16);
+    return k < 2048 ? rows < (k < 1024 ? 16384 : 8193) || n_out < 64 : n_out < 32;
+}
+
+template <int DT>
+cudaError_t launch_mv_rows(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs, int x_per_row,
+                           const uint32_t *ids, int top_k, float *out, cudaStream_t s) {
+    const int64_t step = 65535 / top_k * top_k; // grid.y is limited to 65535
+    for (int64_t p = 0; p < pairs; p += step) {
+        const int64_t n = pairs - p < step ? pairs - p : step;
+        launch_pdl(mv_row_kernel<DT>, dim3((unsigned)((n_out + MR_WARPS * MR_ROWS - 1) / (MR_WARPS * MR_ROWS)), (unsigned)n), MR_WARPS * 32, 0, s, w,
+                   expert_bytes, n_expert, n_out, k, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k,
+                   out + (size_t)p * n_out);
+    }
+    return cudaGetLastError();
+}
+
 template <int DT>
 cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs, int x_per_row,
                       const uint32_t *ids, int top_k, float *out, cudaStream_t s) {
+    if (mv_rows_better<DT>(pairs, n_out, k)) return launch_mv_rows<DT>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, s);
     constexpr int NS = DT == LMOE_Q4_K ? 8 : 16;
     const unsigned gx = (unsigned)((n_out + MV_ROWS - 1) / MV_ROWS);
     int dev = 0;
@@ -864,13 +979,16 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
                                                 : launch_mv_by_expert<DT, false>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, dev, sms, s);
         if (r != cudaErrorNotSupported) return r;
     }
+    // Q6_K straight from global memory takes two loads a word, which the matrix instructions do not make up for: 16 experts of
+    // [256 x 8192], 64 pairs 61.2 us that way, 53.9 by rows, of [4096 x 8192], 8 pairs 125 and 107
+    if (DT == LMOE_Q6_K) return launch_mv_rows<DT>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, s);
     const int bc = k / QK_K < MV_PAIR_BLOCKS ? k / QK_K : MV_PAIR_BLOCKS;
     const int smem_pair = MV_NDIG * (bc * QK_K + 32) + MV_PARTS * bc * NS * 2 + bc * 4; // at most 36 KB
     // grid.y is limited to 65535: fold large pair counts over several launches
     const int64_t step = 65535 / top_k * top_k;
     for (int64_t p = 0; p < pairs; p += step) {
         const int64_t n = pairs - p < step ? pairs - p : step;
-        launch_pdl(mv_pair_kernel<DT>, dim3(gx, (unsigned)n), MV_THREADS, smem_pair, s, w, expert_bytes, n_expert, n_out, k,
+        launch_pdl(mv_pair_kernel<LMOE_Q4_K>, dim3(gx, (unsigned)n), MV_THREADS, smem_pair, s, w, expert_bytes, n_expert, n_out, k,
                                                                                 x + (size_t)(p / top_k) * x_per_row * k, x_per_row,
                                                                                 ids ? ids + p : nullptr, top_k, out + (size_t)p * n_out);
     }

@@ -217,18 +217,19 @@ def test_decode_entry_takes_more_than_64_tokens(orc, dev):
     assert orc.rel_l2(out.cpu().numpy(), want) < 2e-3
 
 
-def test_lm_head_shape_plain_mv(orc, dev):
+@pytest.mark.parametrize("n_out,t", [(100352, 1), (100352, 2), (100352, 3), (100353, 1), (100353, 4)])
+def test_lm_head_shape_plain_mv(orc, dev, n_out, t):
     """`ops::mul_mv` at the shape the model calls it on, once per decoded token (src/model.rs:388-403):
-    Q6_K [100352 x 3072].  256 sampled rows against the oracle, the first and the last chunk among them, and
-    every row finite; a second activation row checks the per-token loop."""
+    Q6_K [100352 x 3072], and with an odd row more.  256 sampled rows against the oracle, the first and the last
+    chunk among them, and every row finite; one token is streamed, two and up to four share a pass over the matrix."""
     from maxuna_b200 import ops
     from maxuna_b200.gguf import Q6_K, ExpertStack
 
-    n_out, k = 100352, 3072
+    k = 3072
     st = ExpertStack.random(Q6_K, 1, n_out, k, std=0.02, seed=4242, device=dev, chunk_experts=1)
     gen = torch.Generator(device=dev)
     gen.manual_seed(9)
-    x = torch.randn(2, k, generator=gen, device=dev)
+    x = torch.randn(t, k, generator=gen, device=dev)
     x[0, 100] = 40.0  # an outlier channel, as the hidden state has them
     w = st.buffer[st.base_off:st.base_off + st.nbytes]
     got = ops.mul_mv(w, Q6_K, n_out, k, x)

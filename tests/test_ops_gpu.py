@@ -104,8 +104,8 @@ def test_mv_shape_mismatch_errors(orc, dev):
     (1, 64, 256, 3, 1, 1), (1, 65, 512, 4, 1, 1), (1, 63, 1280, 33, 1, 1), (1, 130, 3072, 5, 13, 13),  # one matrix: 3 / 4 / 33 / 65 pairs
     (3, 127, 768, 2, 3, 3), (2, 16, 8192 + 256, 1, 2, 1)])                                            # odd block counts, two staged chunks
 def test_mv_tile_edges(orc, dev, dt, name, n_expert, n_out, k, t, top_k, xpr):
-    """Row, pair and K edges of the two mat-vec kernels, an empty slot and an outlier channel.  Bound: activations and sums
-    carry at least 22 bits per 256-wide block and the oracle's own f32 sums err by about sqrt(k) * 2^-24 (5e-6 at 8448)."""
+    """Row, pair and K edges of little work, an empty slot and an outlier channel.  Bound: activations and sums are f32 or better
+    and the oracle's own f32 sums err by about sqrt(k) * 2^-24 (5e-6 at 8448)."""
     from maxuna_b200 import ops
     from maxuna_b200.gguf import ExpertStack
 
@@ -130,10 +130,14 @@ def test_mv_tile_edges(orc, dev, dt, name, n_expert, n_out, k, t, top_k, xpr):
     (2, 136, 1280, 6, 1),    # five: a second turn of the K split for one warp only
     (7, 40, 256, 700, 3),    # more pairs than an expert's are looked for among, many blocks of each expert
     (3, 1032, 4096, 3, 3),   # more shared memory than two blocks of an SM have
+    # the same edges with as many rows as the form needs in order to be taken
+    (3, 64, 256, 130, 2), (5, 72, 512, 80, 3), (4, 200, 768, 41, 2), (2, 136, 1280, 61, 1), (7, 72, 256, 700, 3),
+    (3, 520, 3584, 3, 3), (3, 520, 5120, 3, 3),  # one block an SM: Q6_K, Q4_K
 ])
 @pytest.mark.parametrize("dt,name", DTYPES)
 def test_mv_pairs_by_expert(orc, dev, dt, name, n_expert, n_out, k, t, top_k):
-    """Pairs grouped by expert: group, unit and K edges, repeated experts in any order, empty slots.  Bound as above."""
+    """Pairs grouped by expert, and the same by rows where that is the faster form: group, unit and K edges, repeated experts in
+    any order, empty slots.  Bound as above."""
     from maxuna_b200 import ops
     from maxuna_b200.gguf import ExpertStack
 
@@ -202,6 +206,27 @@ def test_mv_range_and_resolution(orc, dev, dt, name, n_expert, n_out, k, t, top_
     assert not np.isfinite(got[3]).any() and np.isnan(got[5]).all() and np.array_equal(got[keep], base[keep])
 
 
+@pytest.mark.parametrize("n_expert,n_out,k,pairs", [
+    (3, 1024, 256, (7, 8, 15, 16)), (2, 1024, 1024, (3, 4, 8, 9)), (2, 512, 2048, (4, 5)), (2, 512, 3072, (3, 4)),  # rows by length
+    (1, 31, 512, (600,)), (1, 32, 512, (600,)), (1, 63, 768, (300,)), (1, 64, 768, (300,)), (2, 15, 2048, (300,)), (2, 16, 2048, (300,)),
+    (3, 100, 768, (200,)), (2, 64, 8192, (31, 32, 40)), (1, 7, 32768 + 256, (2,))])                              # ring misses
+@pytest.mark.parametrize("dt,name", DTYPES)
+def test_mv_forms_agree(orc, dev, dt, name, n_expert, n_out, k, pairs):
+    """Both sides of every line between the mat-vec forms: the same product, to the roundings of the two evaluations."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    raw = orc.quantize(dt, orc.pseudo_random(n_expert * n_out * k, 0xB00 + k, -1.0, 1.0))
+    stack = ExpertStack.from_bytes(raw, dt, n_expert, n_out, k, device=dev)
+    for t in pairs:
+        x = orc.pseudo_random(t * k, 0x38, -1.0, 1.0).reshape(t, 1, k)
+        ids = (np.arange(t, dtype=np.uint32) * 7 % (n_expert + 1))[:, None]
+        got = ops.mul_mv_id(stack, torch.from_numpy(x).to(dev), torch.from_numpy(ids.astype(np.int32)).to(dev)).cpu().numpy()
+        want = orc.mul_id(dt, raw, n_expert, n_out, k, x, np.minimum(ids, n_expert - 1), accum64=True)
+        want[ids == n_expert] = 0
+        assert not got[ids == n_expert].any() and orc.rel_l2(got, want) < 8 * 2.0 ** -24
+
+
 @pytest.mark.parametrize("dt,name", DTYPES)
 def test_plain_mv(orc, dev, dt, name):
     from maxuna_b200 import ops
@@ -218,8 +243,8 @@ def test_plain_mv(orc, dev, dt, name):
 @pytest.mark.parametrize("n_out,k,t", [(4096, 256, 1), (4104, 512, 3), (4112, 768, 2), (4096 + 16 * 150, 3072, 1)])
 def test_plain_mv_q6k_streamed(orc, dev, n_out, k, t):
     """The streamed Q6_K kernel behind `lmoe_mul_mv` (rows in 16-row chunks through shared memory, integer tensor
-    cores): odd and even super-block counts per row (the 210-byte blocks change word alignment), a row count
-    with a tail, more than one chunk per CTA, several tokens, and an outlier channel.  Same oracle and a tighter
+    cores; one token) and the forms behind it for more tokens: odd and even super-block counts per row (the 210-byte
+    blocks change word alignment), more than one chunk per CTA, and an outlier channel.  Same oracle and a tighter
     bound than the reference's 1e-3 (src/ops/mv_id.rs:300-330): the activations carry 21 bits."""
     from maxuna_b200 import ops
 
