@@ -7,17 +7,16 @@
 namespace {
 
 constexpr int ROUTE_WARPS = 8;
-constexpr int LOGIT_WARPS = 2; // few blocks are what a small batch has: 256 experts on 128 SMs instead of 32
 
-// grid (ceil(n_expert / LOGIT_WARPS), ceil(t / TT)); one warp per expert row,
+// grid (ceil(n_expert / WARPS), ceil(t / TT)); one warp per expert row,
 // TT tokens per pass so the router row is read once per token tile.
-template <int TT>
-__global__ void __launch_bounds__(LOGIT_WARPS * 32)
+template <int TT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 route_logits_kernel(const float *__restrict__ router, const float *__restrict__ x, int t, int hidden,
                     int n_expert, float *__restrict__ logits) {
     pdl_begin();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int e = blockIdx.x * LOGIT_WARPS + warp;
+    const int e = blockIdx.x * WARPS + warp;
     const int t0 = blockIdx.y * TT;
     if (e >= n_expert) return;
     constexpr int UNROLL = TT == 1 ? 12 : 6; // loads in flight: the kernel is their latency
@@ -243,6 +242,7 @@ route_select_kernel(const float *__restrict__ logits, const float *__restrict__ 
 cudaError_t launch_route_logits(const float *router, const float *x, int t, int hidden, int n_expert,
                                 float *logits, cudaStream_t s) {
     if (t == 0) return cudaSuccess;
+    constexpr int LOGIT_WARPS = 2; // few blocks are what a small batch has: 256 experts on 128 SMs instead of 32
     const unsigned gx = (unsigned)((n_expert + LOGIT_WARPS - 1) / LOGIT_WARPS);
     static int sms_of[64] = {0}; // per device: SM count, and the shared-memory opt-in done once
     int dev = 0;
@@ -257,7 +257,9 @@ cudaError_t launch_route_logits(const float *router, const float *x, int t, int 
     // A warp per expert row while its blocks are few, up to five an SM; beyond, their trips to the L2 cache take longer than a
     // register-tiled pass, whose time is the same for any small batch (256 experts, 16 / 24 / 64 tokens: 11.0 / 12.8 / 19.1 us
     // against 12.4 / 12.5 / 12.8; 64 experts of 4096, 64 tokens: 10.2 against 13.3).
-    const bool many = (int64_t)gx * ((t + 3) / 4) > 5 * sms_of[dev];
+    // The tile is padded to 16 experts: up to eight are better off untiled until the tokens are many (8 experts of 4096, 1024 /
+    // 2048 / 4096 tokens: 16.9 / 26.9 / 48 us tiled, 11.1 / 19.4 / 36 so).
+    const bool many = (int64_t)gx * ((t + 3) / 4) > 5 * sms_of[dev] && (n_expert > 8 || t > 4096);
     if (many && hidden % (128 * RT_AHEAD) == 0 && 8 * hidden * 4 + RT_FOLD <= 227 * 1024) {
         // One block per SM at a time: 16 tokens and 16 experts a pass where the rows fit (hidden <= 3072), or 8 tokens and 32
         // experts, in the same time.  The experts are split over blocks until the device is covered, and further where that
@@ -281,9 +283,21 @@ cudaError_t launch_route_logits(const float *router, const float *x, int t, int 
         else
             launch_pdl(route_logits_tiled_kernel<8>, grid, RT_THREADS, smem, s, router, x, t, hidden, n_expert, ppb * pass, logits);
     } else if (t <= 2) {
-        launch_pdl(route_logits_kernel<1>, dim3(gx, t), LOGIT_WARPS * 32, 0, s, router, x, t, hidden, n_expert, logits);
+        launch_pdl(route_logits_kernel<1, LOGIT_WARPS>, dim3(gx, t), LOGIT_WARPS * 32, 0, s, router, x, t, hidden, n_expert, logits);
     } else {
-        launch_pdl(route_logits_kernel<4>, dim3(gx, (t + 3) / 4), LOGIT_WARPS * 32, 0, s, router, x, t, hidden, n_expert, logits);
+        // Rows of two or three steps are mostly fold: in very large numbers twice the warps a block, and the plain launch, which
+        // spreads them evenly (hidden 256, 256 experts, 2048 / 16384 tokens 73 / 563 us as below, 51 / 351 so).
+        const bool short_rows = hidden % 4 == 0 && hidden <= 384 && (int64_t)gx * ((t + 3) / 4) > 100 * (int64_t)sms_of[dev];
+        constexpr int TOKENS = 65535 * 4; // grid.y is limited to 65535
+        for (int t0 = 0; t0 < t; t0 += TOKENS) {
+            const int n = t - t0 < TOKENS ? t - t0 : TOKENS;
+            const float *xs = x + (size_t)t0 * hidden;
+            float *ls = logits + (size_t)t0 * n_expert;
+            if (short_rows)
+                route_logits_kernel<4, 4><<<dim3((unsigned)((n_expert + 3) / 4), (n + 3) / 4), 128, 0, s>>>(router, xs, n, hidden, n_expert, ls);
+            else
+                launch_pdl(route_logits_kernel<4, LOGIT_WARPS>, dim3(gx, (n + 3) / 4), LOGIT_WARPS * 32, 0, s, router, xs, n, hidden, n_expert, ls);
+        }
     }
     return cudaGetLastError();
 }

@@ -347,6 +347,33 @@ def test_routing_tiles_bit_exact(orc, dev, t, hidden, ne):
     assert np.array_equal(w.cpu().numpy().view(np.uint32), w_o.view(np.uint32))
 
 
+@pytest.mark.parametrize("t,hidden,ne", [(2048, 256, 64), (2051, 384, 61), (2600, 3072, 8), (4099, 512, 7)])
+def test_routing_many_tokens_bit_exact(orc, dev, t, hidden, ne):
+    """Short router rows in large numbers, and few experts on either side of the tiled form: bitwise the oracle's."""
+    from maxuna_b200 import ops
+
+    rng = np.random.default_rng(t)
+    router = (rng.standard_normal((ne, hidden)) * 0.02).astype(np.float32)
+    x = rng.standard_normal((t, hidden)).astype(np.float32)
+    ids, w = ops.route(torch.from_numpy(router).to(dev), None, torch.from_numpy(x).to(dev), 4)
+    ids_o, w_o = orc.route(router, None, x, 4)
+    assert np.array_equal(ids.cpu().numpy().astype(np.uint32), ids_o)
+    assert np.array_equal(w.cpu().numpy().view(np.uint32), w_o.view(np.uint32))
+
+
+@pytest.mark.parametrize("hidden", [256, 260])
+def test_routing_beyond_one_grid(dev, hidden):
+    """More tokens than the rows of one grid serve: the same bits as in two calls."""
+    from maxuna_b200 import ops
+
+    t, cut = 65535 * 4 + 7, 131072
+    router, x = torch.randn(5, hidden, device=dev) * 0.02, torch.randn(t, hidden, device=dev)
+    ids, w = ops.route(router, None, x, 2)
+    for part in (slice(0, cut), slice(cut, t)):
+        i, v = ops.route(router, None, x[part], 2)
+        assert torch.equal(ids[part], i) and torch.equal(w[part], v)
+
+
 @pytest.mark.parametrize("ne,top_k", [(1, 1), (31, 31), (128, 8), (129, 32), (257, 10), (512, 32)])
 def test_routing_selection_widths(orc, dev, ne, top_k):
     """Selection at the edges of the scores a lane holds, with ties, infinities and signed zeros: bitwise the oracle's."""
