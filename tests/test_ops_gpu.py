@@ -448,6 +448,23 @@ def test_combine_and_silu_mul(orc, dev, seq):
     np.testing.assert_allclose(ops.silu_mul(td(g), td(u)).cpu().numpy(), orc.silu_mul(g, u), rtol=2e-6, atol=1e-7)
 
 
+@pytest.mark.parametrize("n", [1, 3, 1025, (1 << 18) - 1, 1 << 18, (1 << 18) + 3])
+def test_silu_mul_counts_and_alignment(orc, dev, n):
+    """Counts off a multiple of four and rows off a 16-byte boundary: the same values, and nothing written past the last one."""
+    from maxuna_b200._native import check, lib
+    from maxuna_b200.gguf import stream_ptr
+
+    rng = np.random.default_rng(n)
+    g, u = (rng.standard_normal(n).astype(np.float32) * 3 for _ in range(2))
+    want = orc.silu_mul(g, u)
+    for off in (0, 1):
+        bg, bu = (torch.from_numpy(np.concatenate([np.zeros(off, np.float32), v])).to(dev) for v in (g, u))
+        out = torch.full((n + off + 4,), 7.0, device=dev)
+        check(lib().lmoe_silu_mul(bg.data_ptr() + 4 * off, bu.data_ptr() + 4 * off, n, out.data_ptr() + 4 * off, stream_ptr()))
+        np.testing.assert_allclose(out[off:off + n].cpu().numpy(), want, rtol=2e-6, atol=1e-7)
+        assert (out[off + n:] == 7).all() and (out[:off] == 7).all()
+
+
 @pytest.mark.parametrize("rows,top_k,n", [(3, 1, 97), (5, 6, 33), (2, 22, 132), (1, 64, 4)])
 def test_glue_edges(orc, dev, rows, top_k, n):
     """Scalar and four-wide forms of combine and silu_mul, a row count off the block size, and the range guard: a zero row, and
