@@ -321,7 +321,7 @@ lmoe_status lmoe_moe_layer_forward(const lmoe_layer *layer, const float *ffn_inp
  * run the routed experts of pre-routed, pre-dispatched rows.
  *   x [rows, hidden] f32, local_ids [rows] u32 (expert id relative to the
  *   layer's first expert), row_weights [rows] f32 -> out [rows, hidden] f32
- *   = row_weights[r] * FFN_{local_ids[r]}(x[r]). */
+ *   = row_weights[r] * FFN_{local_ids[r]}(x[r]); a row whose id names no expert of the layer is a zero row. */
 lmoe_status lmoe_experts_forward_rows(const lmoe_layer *layer, const float *x, const uint32_t *local_ids,
                                       const float *row_weights, int64_t rows, float *out, void *workspace,
                                       size_t workspace_bytes, void *stream);
@@ -346,6 +346,7 @@ lmoe_status lmoe_experts_forward_tokens_f16(const lmoe_layer *layer, const void 
  * ids / weights [t, top_k], writes the t * top_k routed rows grouped by destination rank (by expert inside a
  * rank): rows_f16 [t*top_k, hidden] half, local_ids [t*top_k] (expert id relative to the destination's first
  * expert), row_weights [t*top_k], row_pos [t*top_k] = position of flat id (token * top_k + slot) in that order,
+ * -1 for an id >= n_expert,
  * and send_counts [world] (int64, device).  Workspace: lmoe_ep_pack_workspace_bytes(n_expert, t). */
 size_t lmoe_ep_pack_workspace_bytes(int64_t n_expert, int64_t t);
 lmoe_status lmoe_ep_pack(const float *x, const uint32_t *ids, const float *weights, int64_t t, int64_t hidden,

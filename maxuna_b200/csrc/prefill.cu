@@ -30,13 +30,19 @@ namespace {
 // order (row tile pos / nt, row pos % nt, 128-byte swizzle, groups of 8 as [0 2 1 3 4 6 5 7]);
 // scale[row] = l2 * 2^-15 * weight[row] undoes it in the down epilogue together with the
 // routing weight (src/ops/combine.metal:102-133).
+// A row that no list names (pos < 0) is a zero row of `y`.
+__device__ __forceinline__ void zero_row(float *y, int hidden, int lane) {
+    for (int i = lane; i < hidden; i += 32) y[i] = 0.f;
+}
 __global__ void __launch_bounds__(256) swiglu_rows_kernel(const float *__restrict__ g, const float *__restrict__ u,
                                                           const float *__restrict__ w, const int32_t *__restrict__ pos,
                                                           int64_t rows, int ff, int nt, uint8_t *__restrict__ act,
-                                                          float *__restrict__ scale) {
+                                                          float *__restrict__ scale, float *__restrict__ y, int hidden) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
+    const int p = pos[row];
+    if (p < 0) { zero_row(y + row * hidden, hidden, lane); return; }
     const float *gr = g + row * ff, *ur = u + row * ff;
     float ss = 0.f;
     for (int i = lane * 8; i < ff; i += 256) {
@@ -54,7 +60,6 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const float *__restric
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float l2 = fminf(fmaxf(sqrtf(ss), 1e-8f), 1e30f);
     const float k = 32768.0f / l2;
-    const int p = pos[row];
     for (int i = lane * 8; i < ff; i += 256) {
         const float4 g0 = *reinterpret_cast<const float4 *>(gr + i), g1 = *reinterpret_cast<const float4 *>(gr + i + 4);
         const float4 u0 = *reinterpret_cast<const float4 *>(ur + i), u1 = *reinterpret_cast<const float4 *>(ur + i + 4);
@@ -79,12 +84,14 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const float *__restric
 __global__ void __launch_bounds__(256) rescale_rows_kernel(const float *__restrict__ a, const float *__restrict__ w,
                                                            const int32_t *__restrict__ pos, const int32_t *__restrict__ sfid,
                                                            int64_t rows, int64_t routed, int ff, int nt, uint8_t *__restrict__ act,
-                                                           float *__restrict__ scale) {
+                                                           float *__restrict__ scale, float *__restrict__ y, int hidden) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int64_t fid = sfid ? sfid[row] : row;
     if (fid < 0) return;                                   // no routed row here (masked slots leave a tail unused)
+    const int p = pos[fid];
+    if (p < 0) { zero_row(y + row * hidden, hidden, lane); return; } // (rows by flat id only)
     const float *ar = a + row * ff;
     float ss = 0.f;
     for (int i = lane * 8; i < ff; i += 256) {
@@ -95,7 +102,6 @@ __global__ void __launch_bounds__(256) rescale_rows_kernel(const float *__restri
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const float l2 = fminf(fmaxf(sqrtf(ss), 1e-8f), 1e30f);
     const float k = 32768.0f / l2;
-    const int p = pos[fid];
     for (int i = lane * 8; i < ff; i += 256) {
         const float4 a0 = *reinterpret_cast<const float4 *>(ar + i), a1 = *reinterpret_cast<const float4 *>(ar + i + 4);
         __align__(16) __half2 h[4] = {__floats2half2_rn(a0.x * k, a0.z * k), __floats2half2_rn(a0.y * k, a0.w * k),
@@ -263,13 +269,15 @@ size_t ffn_bytes(const MmRows &R, int64_t hidden, int64_t ff) {
 // UNSCALED rows in expert-sorted order: row spos[flat id], to be multiplied by scale_out[that row]; the
 // tensor-core epilogues then store whole tile columns side by side instead of scattering by flat id.  Only in that form
 // can R.extra rows of the shared expert (`sh`: its gate, up, down) ride along: one launch of each kernel serves both.
-// `masked`: ids >= n_expert were left out of the lists.
+// The lists must name every flat id, but for these: SLOTS_MAY_BE_EMPTY (sorted form), ids >= n_expert are empty slots;
+// ROWS_MAY_BE_UNLISTED (unsorted), a row whose id is none of the experts' is a zero row.
+enum Gaps { COMPLETE = 0, SLOTS_MAY_BE_EMPTY = 1, ROWS_MAY_BE_UNLISTED = 2 };
 bool ffn_sorts(const lmoe_expert_stack *gate, const lmoe_expert_stack *up) { return gate->dtype == LMOE_Q4_K && up->dtype == LMOE_Q4_K; }
 
 lmoe_status ffn_grouped(const MmRows &R, const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *down,
                         const lmoe_expert_stack *const (&sh)[3], const void *x, int top_k, const uint32_t *tpe, const int32_t *ids_map,
                         int64_t map_stride, const float *row_w, float *y, uint8_t *ws, uint32_t *flag, cudaStream_t s,
-                        int32_t *spos = nullptr, float *scale_out = nullptr, int x_f16 = 0, int masked = 0) {
+                        int32_t *spos = nullptr, float *scale_out = nullptr, int x_f16 = 0, int gaps = COMPLETE) {
     const int64_t all = R.rows + R.extra, ff = gate->n_out, hidden = gate->k;
     Carver c{ws, 0};
     uint8_t *xt = c.take<uint8_t>(mm_tiled_bytes(R, hidden));
@@ -282,7 +290,8 @@ lmoe_status ffn_grouped(const MmRows &R, const lmoe_expert_stack *gate, const lm
     void *tiles = ws + c.off;
     lmoe_status st;
     const bool fused_gu = ffn_sorts(gate, up), sorted = spos && scale_out && fused_gu;
-    if (masked) {
+    if (gaps == ROWS_MAY_BE_UNLISTED) LMOE_CUDA(cudaMemsetAsync(pos, 0xFF, (size_t)all * 4, s));
+    if (gaps == SLOTS_MAY_BE_EMPTY) {
         // some (token, slot) pairs name no expert: the lists skip them, and the per-row arrays mark them
         if (!sorted) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "masked slots need the fused Q4_K gate/up kernel");
         LMOE_CUDA(cudaMemsetAsync(spos, 0xFF, (size_t)all * 4, s));
@@ -296,14 +305,14 @@ lmoe_status ffn_grouped(const MmRows &R, const lmoe_expert_stack *gate, const lm
             return st;
         if ((st = launch_mm_gateup(R, gate, up, sh[0], sh[1], xt, src, ids_map, map_stride, g, sorted, tiles, flag, s))) return st;
         rescale_rows_kernel<<<row_blocks, 256, 0, s>>>(g, row_w, pos, sorted ? sfid : nullptr, all, R.rows, (int)ff, R.nt, act,
-                                                       sorted ? scale_out : rs);
+                                                       sorted ? scale_out : rs, y, (int)hidden);
         LMOE_LAUNCH_CHECK("rescale_rows_kernel");
     } else {
         if ((st = launch_gather_tiles(R, x, x_f16, 1, top_k, (int)hidden, tpe, ids_map, map_stride, tiles, xt, pos, nullptr, nullptr, s)))
             return st;
         if ((st = launch_mm_id(R, gate, nullptr, xt, ids_map, map_stride, nullptr, g, 0, tiles, flag, s))) return st;
         if ((st = launch_mm_id(R, up, nullptr, xt, ids_map, map_stride, nullptr, u, 0, tiles, flag, s))) return st;
-        swiglu_rows_kernel<<<row_blocks, 256, 0, s>>>(g, u, row_w, pos, all, (int)ff, R.nt, act, rs);
+        swiglu_rows_kernel<<<row_blocks, 256, 0, s>>>(g, u, row_w, pos, all, (int)ff, R.nt, act, rs, y, (int)hidden);
         LMOE_LAUNCH_CHECK("swiglu_rows_kernel");
     }
     return launch_mm_id(R, down, sh[2], act, ids_map, map_stride, sorted ? nullptr : rs, y, sorted, tiles, flag, s);
@@ -530,7 +539,7 @@ static lmoe_status experts_rows_run(const lmoe_layer *L, const void *x, int x_f1
     LMOE_CUDA(cudaMemsetAsync(flag, 0, 16, s));
     LMOE_CUDA(launch_map0(local_ids, (int)rows, 1, (int)L->n_expert, tpe, ids_map, s));
     return ffn_grouped(mm_rows(rows, 0, L->n_expert), L->gate, L->up, L->down, {nullptr, nullptr, nullptr}, x, 1, tpe, ids_map, rows,
-                       row_weights, out, ffn_ws, flag, s, nullptr, nullptr, x_f16);
+                       row_weights, out, ffn_ws, flag, s, nullptr, nullptr, x_f16, ROWS_MAY_BE_UNLISTED);
 }
 
 extern "C" lmoe_status lmoe_experts_forward_rows(const lmoe_layer *L, const float *x, const uint32_t *local_ids,
@@ -619,6 +628,7 @@ extern "C" lmoe_status lmoe_ep_pack(const float *x, const uint32_t *ids, const f
     cudaStream_t s = (cudaStream_t)stream;
     uint32_t *tpe = static_cast<uint32_t *>(workspace);
     int32_t *ids_map = reinterpret_cast<int32_t *>(static_cast<uint8_t *>(workspace) + n_expert * 4);
+    LMOE_CUDA(cudaMemsetAsync(row_pos, 0xFF, (size_t)(t * top_k) * 4, s)); // an id that names no expert: an empty slot
     LMOE_CUDA(launch_map0(ids, (int)t, (int)top_k, (int)n_expert, tpe, ids_map, s));
     const int e_local = (int)(n_expert / world);
     ep_counts_kernel<<<(unsigned)world, 32, 0, s>>>(tpe, (int)n_expert, e_local, reinterpret_cast<long long *>(send_counts));

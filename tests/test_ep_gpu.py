@@ -89,6 +89,41 @@ def test_tokens_entry_matches_rows_entry(t, k):
     blk.check_device_flag()
 
 
+@pytest.mark.parametrize("gate_dtype", [12, 14])
+def test_rows_whose_id_names_no_expert(gate_dtype):
+    """A row with an id outside the layer's experts is a zero row and leaves the others as they are; packed for the exchange,
+    such a slot is empty."""
+    from maxuna_b200._native import check, lib
+    from maxuna_b200.gguf import stream_ptr
+    from maxuna_b200.moe import MoeBlock
+
+    dev = torch.device("cuda:0")
+    ne, rows, H = 8, 90, 256
+    blk = MoeBlock.random(H, 512, ne, 2, seed=49, device=dev, weight_std=0.25, gate_dtype=gate_dtype)
+    x = torch.randn(rows, H, device=dev)
+    ids = torch.randint(0, ne, (rows,), device=dev, dtype=torch.int32)
+    w = torch.rand(rows, device=dev)
+    want = blk.experts_forward_rows(x, ids, w)
+    gone = torch.zeros(rows, dtype=torch.bool, device=dev)
+    gone[[0, 7, 50, 89]] = True
+    ids[gone] = torch.tensor([ne, -1, 2 ** 31 - 1, 1000], dtype=torch.int32, device=dev)
+    blk._rws.fill_(0x7f)  # what an earlier call may have left
+    got = blk.experts_forward_rows(x, ids, w)
+    assert not got[gone].any() and torch.equal(got[~gone], want[~gone])
+    # two slots a token through the exchange's packing
+    t, k = rows // 2, 2
+    sent, li = torch.empty(rows, H, dtype=torch.float16, device=dev), torch.empty(rows, dtype=torch.int32, device=dev)
+    rw, pos = torch.empty(rows, device=dev), torch.full((rows,), 10 ** 9, dtype=torch.int32, device=dev)
+    counts = torch.empty(2, dtype=torch.int64, device=dev)
+    nb = lib().lmoe_ep_pack_workspace_bytes(ne, t)
+    ws = torch.empty(nb, dtype=torch.uint8, device=dev)
+    distinct = (torch.arange(t, device=dev, dtype=torch.int32)[:, None] + torch.tensor([0, 3], dtype=torch.int32, device=dev)) % ne
+    distinct.view(-1)[gone] = ids[gone]
+    check(lib().lmoe_ep_pack(x.data_ptr(), distinct.data_ptr(), w.data_ptr(), t, H, k, ne, 2, sent.data_ptr(), li.data_ptr(), rw.data_ptr(),
+                             pos.data_ptr(), counts.data_ptr(), ws.data_ptr(), nb, stream_ptr()))
+    assert (pos[gone] == -1).all() and sorted(pos[~gone].tolist()) == list(range(rows - 4)) and counts.sum().item() == rows - 4
+
+
 @pytest.mark.parametrize("world", [2, 4])
 def test_ep_pack_and_combine_match_the_index_arithmetic(world):
     """lmoe_ep_pack / lmoe_ep_combine against the torch plan they replace (one device, any world size)."""
