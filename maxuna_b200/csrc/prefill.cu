@@ -249,14 +249,20 @@ struct Carver {
     }
 };
 
-// Scratch of one grouped SwiGLU FFN.
-size_t ffn_bytes(const MmRows &R, int64_t hidden, int64_t ff) {
+bool ffn_sorts(const lmoe_expert_stack *gate, const lmoe_expert_stack *up) { return gate->dtype == LMOE_Q4_K && up->dtype == LMOE_Q4_K; }
+
+// The f16 activations of a grouped SwiGLU FFN: x_rows rows in token order for the fused gate/up kernel, else in tile order.
+size_t ffn_x_bytes(const MmRows &R, int64_t x_rows, int64_t hidden, bool fused) {
+    return fused ? lmoe_align_up((size_t)x_rows * hidden * 2, 256) : mm_tiled_bytes(R, hidden);
+}
+// Its scratch, by the form that `fused` takes.
+size_t ffn_bytes(const MmRows &R, int64_t x_rows, int64_t hidden, int64_t ff, bool fused) {
     const size_t all = (size_t)(R.rows + R.extra);
     size_t o = 0;
-    o += mm_tiled_bytes(R, hidden);                          // x in tile order, or in token order (never more)
-    o += mm_src_bytes(R);                                    // source row of every tile row
+    o += ffn_x_bytes(R, x_rows, hidden, fused);
+    o += fused ? mm_src_bytes(R) : 0;                        // source row of every tile row
     o += lmoe_align_up(all * 4, 256);                        // position of every flat id
-    o += 2 * lmoe_align_up(all * ff * 4, 256);               // gate, up
+    o += (fused ? 1 : 2) * lmoe_align_up(all * ff * 4, 256); // SwiGLU activations, or gate and up
     o += mm_tiled_bytes(R, ff);                              // f16 activation in tile order
     o += lmoe_align_up(all * 4, 256);                        // row scale
     o += lmoe_align_up(all * 4, 256);                        // flat id of every sorted row
@@ -272,24 +278,23 @@ size_t ffn_bytes(const MmRows &R, int64_t hidden, int64_t ff) {
 // The lists must name every flat id, but for these: SLOTS_MAY_BE_EMPTY (sorted form), ids >= n_expert are empty slots;
 // ROWS_MAY_BE_UNLISTED (unsorted), a row whose id is none of the experts' is a zero row.
 enum Gaps { COMPLETE = 0, SLOTS_MAY_BE_EMPTY = 1, ROWS_MAY_BE_UNLISTED = 2 };
-bool ffn_sorts(const lmoe_expert_stack *gate, const lmoe_expert_stack *up) { return gate->dtype == LMOE_Q4_K && up->dtype == LMOE_Q4_K; }
 
 lmoe_status ffn_grouped(const MmRows &R, const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *down,
                         const lmoe_expert_stack *const (&sh)[3], const void *x, int top_k, const uint32_t *tpe, const int32_t *ids_map,
                         int64_t map_stride, const float *row_w, float *y, uint8_t *ws, uint32_t *flag, cudaStream_t s,
                         int32_t *spos = nullptr, float *scale_out = nullptr, int x_f16 = 0, int gaps = COMPLETE) {
     const int64_t all = R.rows + R.extra, ff = gate->n_out, hidden = gate->k;
+    const bool fused_gu = ffn_sorts(gate, up), sorted = spos && scale_out && fused_gu;
     Carver c{ws, 0};
-    uint8_t *xt = c.take<uint8_t>(mm_tiled_bytes(R, hidden));
-    int32_t *src = reinterpret_cast<int32_t *>(c.take<uint8_t>(mm_src_bytes(R)));
+    uint8_t *xt = c.take<uint8_t>(ffn_x_bytes(R, R.rows / top_k, hidden, fused_gu));
+    int32_t *src = reinterpret_cast<int32_t *>(c.take<uint8_t>(fused_gu ? mm_src_bytes(R) : 0));
     int32_t *pos = c.take<int32_t>((size_t)all);
-    float *g = c.take<float>((size_t)all * ff), *u = c.take<float>((size_t)all * ff);
+    float *g = c.take<float>((size_t)all * ff), *u = c.take<float>(fused_gu ? 0 : (size_t)all * ff);
     uint8_t *act = c.take<uint8_t>(mm_tiled_bytes(R, ff));
     float *rs = c.take<float>((size_t)all);
     int32_t *sfid = c.take<int32_t>((size_t)all);
     void *tiles = ws + c.off;
     lmoe_status st;
-    const bool fused_gu = ffn_sorts(gate, up), sorted = spos && scale_out && fused_gu;
     if (gaps == ROWS_MAY_BE_UNLISTED) LMOE_CUDA(cudaMemsetAsync(pos, 0xFF, (size_t)all * 4, s));
     if (gaps == SLOTS_MAY_BE_EMPTY) {
         // some (token, slot) pairs name no expert: the lists skip them, and the per-row arrays mark them
@@ -338,7 +343,8 @@ static size_t experts_ws_bytes(const lmoe_layer *L, int64_t t, int64_t top_k) {
     o += lmoe_align_up(all * L->hidden * 4, 256);                    // partial rows
     o += lmoe_align_up((size_t)(t + 64) * 4, 256);                   // identity list
     o += 2 * lmoe_align_up(all * 4, 256);                            // sorted position and scale of every row
-    const size_t a = ffn_bytes(R, L->hidden, L->expert_ff), b = ffn_bytes(mm_rows(t, 0, 1), L->hidden, L->expert_ff);
+    const bool fused = ffn_sorts(L->gate, L->up);
+    const size_t a = ffn_bytes(R, t, L->hidden, L->expert_ff, fused), b = ffn_bytes(mm_rows(t, 0, 1), t, L->hidden, L->expert_ff, fused);
     o += a > b ? a : b;
     return o;
 }
@@ -510,7 +516,9 @@ extern "C" lmoe_status lmoe_mul_mm_id(const lmoe_expert_stack *stack, const floa
 // ---- expert-parallel pieces -------------------------------------------------------------
 // (the same entries serve the shared expert alone, whose single list may take another tile size)
 static size_t rows_ffn_bytes(const lmoe_layer *L, int64_t rows) {
-    const size_t a = ffn_bytes(mm_rows(rows, 0, L->n_expert), L->hidden, L->expert_ff), b = ffn_bytes(mm_rows(rows, 0, 1), L->hidden, L->expert_ff);
+    const bool fused = ffn_sorts(L->gate, L->up);
+    const size_t a = ffn_bytes(mm_rows(rows, 0, L->n_expert), rows, L->hidden, L->expert_ff, fused);
+    const size_t b = ffn_bytes(mm_rows(rows, 0, 1), rows, L->hidden, L->expert_ff, fused);
     return a > b ? a : b;
 }
 static size_t rows_ws_bytes(const lmoe_layer *L, int64_t rows) {

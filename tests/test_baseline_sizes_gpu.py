@@ -177,6 +177,35 @@ def test_prefill_entries_clear_the_device_flag(dev, entry):
     assert torch.isfinite(out).all()
 
 
+@pytest.mark.parametrize("gate_dtype,t", [(12, 70), (14, 70), (12, 700), (14, 700)])
+def test_prefill_stays_inside_its_workspace(dev, gate_dtype, t):
+    """A workspace of exactly the stated size is enough for both forms of the grouped path, whichever row tiles they take."""
+    from maxuna_b200._native import check, lib
+    from maxuna_b200.gguf import stream_ptr
+    from maxuna_b200.moe import MoeBlock
+
+    blk = MoeBlock.random(256, 512, 8, 3, seed=96, device=dev, weight_std=0.25, gate_dtype=gate_dtype)
+    x, outs = torch.randn(t, 256, device=dev), []
+    for more in (0, 1 << 26):
+        n = lib().lmoe_layer_workspace_bytes(blk.handle, t) + more
+        ws = torch.full((n + 4096,), 0xA5, dtype=torch.uint8, device=dev)
+        out = torch.empty(t, 256, device=dev)
+        check(lib().lmoe_moe_forward_prefill(blk.handle, x.data_ptr(), t, out.data_ptr(), None, None, ws.data_ptr(), n, stream_ptr()))
+        assert (ws[n:] == 0xA5).all()
+        outs.append(out)
+    assert torch.equal(*outs)
+
+
+def test_prefill_workspace_holds_what_is_used(zipf_block):
+    """2048 tokens of the production shape: the f32 rows of every (token, slot), their f32 and f16 activations, the tokens in
+    f16 and the staging of host buffers (input and result), with 5 % for the lists and what the row tiles round up; no tile-ordered copy of the tokens and no second f32 activation."""
+    from maxuna_b200._native import lib
+
+    t, k, e, h, f = 2048, zipf_block.n_expert_used, zipf_block.n_expert, zipf_block.hidden, zipf_block.expert_ff
+    used = t * (k + 1) * (h * 4 + f * 4) + (t * (k + 1) + 192 * (e + 1)) * f * 2 + t * h * 2 + 2 * t * h * 4
+    assert lib().lmoe_layer_workspace_bytes(zipf_block.handle, t) <= 1.05 * used
+
+
 def test_second_decode_call_in_flight_is_refused(dev, zipf_block):
     """One decode call at a time per layer handle: a call on a second stream while the first is still
     running is an error, not silent corruption; after the first has finished the second stream may call."""
