@@ -12,9 +12,8 @@
 //
 // Structure (the path is HBM-bound: 70.5 MB per token at the production shape)
 //   * grid = every SM x 2 CTAs, launched cooperatively so all CTAs are resident;
-//     CTA = 4 consumer warps + 1 producer warp + 1 epilogue warp.  (The kernel is written for NG groups of
-//     four consumer warps per CTA; geometries with two to four groups in one CTA per SM were measured and did
-//     not beat one group in each of two CTAs up to 16 tokens, so only NG = 1 is instantiated.)
+//     CTA = 4 consumer warps + 1 producer warp + 1 epilogue warp.  (Two to four groups of four consumer warps in
+//     one CTA per SM were measured and did not beat one group in each of two CTAs up to 16 tokens.)
 //   * The producer streams raw super-blocks global -> shared with 1-D bulk
 //     copies (cp.async.bulk + mbarrier) through a 3-stage ring: each DISTINCT
 //     selected expert (and the shared expert) is read from HBM exactly once per
@@ -52,21 +51,17 @@
 
 namespace {
 
-constexpr int CW = 4;             // consumer warps of a group: the K split of one unit
+constexpr int CW = 4;             // consumer warps: the K split of one unit
 constexpr int DOWN_ROWS = 32;     // rows of a down-projection unit: two MMA row tiles
-// Launch geometry by the number of groups NG (units a CTA works on at the same time): one group means two
-// CTAs per SM with a 3-stage ring each; more groups share one CTA per SM, one activation cache and a longer ring.
-template <int NG_>
+// Launch geometry: two CTAs per SM, a 3-stage ring each.
 struct Cfg {
-    static constexpr int NG = NG_;
-    static constexpr int NCW = CW * NG;                 // consumer warps
-    static constexpr int THREADS = 32 * (NCW + 2);      // + producer warp + epilogue warp
-    static constexpr int CONS = 32 * NCW;
-    static constexpr int RING = 32 * (NCW + 1);         // consumers + producer
-    static constexpr int EPI = 32 * (NCW + 1);          // consumers + epilogue warp
-    static constexpr int NSTAGE = NG == 1 ? 3 : (NG == 2 ? 4 : 6);
-    static constexpr int NRED = NG == 1 ? 3 : 2 * NG;   // K-split partial buffers between the consumers and the epilogue warp
-    static constexpr int MIN_CTAS = NG == 1 ? 2 : 1;
+    static constexpr int THREADS = 32 * (CW + 2);       // + producer warp + epilogue warp
+    static constexpr int CONS = 32 * CW;
+    static constexpr int RING = 32 * (CW + 1);          // consumers + producer
+    static constexpr int EPI = 32 * (CW + 1);           // consumers + epilogue warp
+    static constexpr int NSTAGE = 3;
+    static constexpr int NRED = 3;                      // K-split partial buffers between the consumers and the epilogue warp
+    static constexpr int MIN_CTAS = 2;
 };
 constexpr int SYNC_PASS0 = 32;   // layer sync words: [0] grid barrier, [1] exit count, [2] tokens routed, [32 + pass] phase-1 units done
 constexpr int SYNC_WORDS = SYNC_PASS0 + 1024;
@@ -453,7 +448,7 @@ __device__ __forceinline__ void q4k_block(const uint8_t *bg, const uint8_t *bG, 
     acc[2] += cs.x * (dG * (float)al[2] - mG * (r0 * cm[2]));
     acc[3] += cs.y * (dG * (float)al[3] - mG * (r1 * cm[3]));}
 
-// 16 Q4_K rows (8 gate + 8 up): warp wq of the group takes every CW-th super-block.
+// 16 Q4_K rows (8 gate + 8 up): warp wq takes every CW-th super-block.
 __device__ __forceinline__ void unit_q4k(const uint8_t *stage, int row_bytes, int nb, int wq, int g, int t,
                                          const int8_t *xcol, const __half *scol, const float *sxs, float r0, float r1,
                                          float (&acc)[4]) {
@@ -463,7 +458,7 @@ __device__ __forceinline__ void unit_q4k(const uint8_t *stage, int row_bytes, in
         q4k_block(rg + b * Q4K_BYTES, rG + b * Q4K_BYTES, t, xcol + 256 * b, scol + 8 * b, sxs + 8 * b, r0, r1, acc);
 }
 
-// 32 Q6_K rows: warp wq of the group takes row tile wq & 1 (16 rows) and half of its super-blocks.  Super-blocks are 210 bytes
+// 32 Q6_K rows: warp wq takes row tile wq & 1 (16 rows) and half of its super-blocks.  Super-blocks are 210 bytes
 // long, so every other one starts 2 bytes off a word boundary and costs twice the shared-memory reads.  With an even number of
 // them in a row the rows start alike, and contiguous halves share the expensive ones out evenly.
 __device__ __forceinline__ void unit_q6k(const uint8_t *stage, int row_bytes, int nb, int wq, int g, int t,
@@ -527,11 +522,11 @@ __device__ __noinline__ void dec_wait_pass(const uint32_t *cnt, uint32_t need, u
 // second one for rows of an odd number of super-blocks.  A function of its
 // own, with everything in scalars: its registers are then its own, and no change around it moves them (the same loop inside
 // the kernel varied by 5 % with what stood beside it).
-template <int NDIG, int NTOK, int NG, int PHASE>
+template <int NDIG, int NTOK, int PHASE>
 __device__ __noinline__ void dec_units(uint32_t n, uint32_t n1, const uint8_t *ring, int stage_bytes, int row_bytes, int nb,
                                        const int8_t *xcol, const __half *scol, const float *sxs, float r0, float r1, float *red,
                                        uint64_t *full, uint32_t *ctrl) {
-    using C = Cfg<NG>;
+    using C = Cfg;
     constexpr int NCOL = NDIG * NTOK, NSTAGE = C::NSTAGE, NRED = C::NRED;
     uint64_t *empty = full + NSTAGE, *red_full = empty + NSTAGE, *red_free = red_full + NRED;
     const int lane = threadIdx.x & 31, wq = (threadIdx.x >> 5) % CW, g = lane >> 2, t4 = lane & 3;
@@ -856,11 +851,11 @@ __device__ __noinline__ void dec_lists(int n, int E, uint32_t *ctrl, const uint3
 }
 
 // ---- the kernel ---------------------------------------------------------------------
-template <int NDIG, int NTOK, int NG>
-__global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decode_kernel(const __grid_constant__ DecodeParams P) {
-    using C = Cfg<NG>;
+template <int NDIG, int NTOK>
+__global__ void __launch_bounds__(Cfg::THREADS, Cfg::MIN_CTAS) moe_decode_kernel(const __grid_constant__ DecodeParams P) {
+    using C = Cfg;
     constexpr int NCOL = NDIG * NTOK; // MMA columns in use: (token, digit)
-    constexpr int NSTAGE = C::NSTAGE, NRED = C::NRED, NCW = C::NCW, CONS_THREADS = C::CONS;
+    constexpr int NSTAGE = C::NSTAGE, NRED = C::NRED, NCW = CW, CONS_THREADS = C::CONS;
     extern __shared__ __align__(128) uint8_t smem[];
     const DecLayout L(P.hidden, P.ff, P.n_expert, P.t, P.top_k, NCOL, NSTAGE, NRED, P.lists_alias);
     uint8_t *ring = smem + L.o_ring;
@@ -1152,7 +1147,7 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
         else u0 = s_range[sec].x, u1 = s_range[sec].y;
         if (u0 < u1) {
             // the section is walked pass by pass: all consumer warps stage a pass's activations together,
-            // then the two groups take alternate units of the pass's slice
+            // then the units of the pass's slice
             for (int q = u0 / tiles; q * tiles < u1; q++) {
                 const int a = max(u0, q * tiles), b = min(u1, (q + 1) * tiles);
                 Pass U;
@@ -1181,11 +1176,11 @@ __global__ void __launch_bounds__(Cfg<NG>::THREADS, Cfg<NG>::MIN_CTAS) moe_decod
                 }
                 const uint32_t n0 = n_unit + (uint32_t)(a - u0), n1 = n_unit + (uint32_t)(b - u0);
                 if (phase == 1)
-                    dec_units<NDIG, NTOK, NG, 1>(n0, n1, ring, L.stage_bytes, row4, nb4, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
+                    dec_units<NDIG, NTOK, 1>(n0, n1, ring, L.stage_bytes, row4, nb4, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
                 else if (row6 & 2)
-                    dec_units<NDIG, NTOK, NG, 3>(n0, n1, ring, L.stage_bytes, row6, nb6, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
+                    dec_units<NDIG, NTOK, 3>(n0, n1, ring, L.stage_bytes, row6, nb6, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
                 else
-                    dec_units<NDIG, NTOK, NG, 2>(n0, n1, ring, L.stage_bytes, row6, nb6, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
+                    dec_units<NDIG, NTOK, 2>(n0, n1, ring, L.stage_bytes, row6, nb6, xcol, scol, sxs, r0, r1, red, full, P.ctrl);
             }
             n_unit += (uint32_t)(u1 - u0);
         }
@@ -1267,13 +1262,13 @@ namespace {
 // (device, shared-memory size).
 struct DecVariant {
     const void *fn;
-    int ncol, ng, threads, ncw, nstage, nred, min_ctas;
+    int ncol, threads, nstage, nred, min_ctas;
     int c_dev = -1, c_total = -1, c_occ = 0;
 };
-template <int NDIG, int NTOK, int NG>
+template <int NDIG, int NTOK>
 DecVariant make_variant() {
-    using C = Cfg<NG>;
-    return DecVariant{(const void *)moe_decode_kernel<NDIG, NTOK, NG>, NDIG * NTOK, NG, C::THREADS, C::NCW, C::NSTAGE, C::NRED, C::MIN_CTAS};
+    using C = Cfg;
+    return DecVariant{(const void *)moe_decode_kernel<NDIG, NTOK>, NDIG * NTOK, C::THREADS, C::NSTAGE, C::NRED, C::MIN_CTAS};
 }
 } // namespace
 
@@ -1290,12 +1285,12 @@ lmoe_status launch_moe_decode(const lmoe_layer *Ly, const float *x, int t, float
         return lmoe_fail(LMOE_ERR_UNSUPPORTED, "fused decode needs hidden %% 128 == 0 and expert_ff %% 16 == 0");
     if (t * K > 4095 || t * (K + 1) > 4095 || (t + 1) / 2 + t * K > SYNC_WORDS - SYNC_PASS0)
         return lmoe_fail(LMOE_ERR_UNSUPPORTED, "t*top_k too large");
-    // One group per CTA, two CTAs per SM.  Up to 8 tokens: three digits per activation (21 bits) and two tokens
+    // Two CTAs per SM.  Up to 8 tokens: three digits per activation (21 bits) and two tokens
     // per pass.  From 9 tokens on: two digits (15 bits) and three tokens per pass - the same six MMA columns and
     // the same shared memory, but an expert selected by three tokens, and the shared expert, need a third fewer
     // passes (16 tokens: 187 -> 178 us, 64 tokens: 512 -> 397 us per launch).
-    static thread_local DecVariant v_small = make_variant<3, 2, 1>();
-    static thread_local DecVariant v_23 = make_variant<2, 3, 1>();
+    static thread_local DecVariant v_small = make_variant<3, 2>();
+    static thread_local DecVariant v_23 = make_variant<2, 3>();
     DecVariant &V = t >= LMOE_DEC_V23_FROM_T ? v_23 : v_small;
     const bool lists_alias = dec_lists_alias(H, F, E, t, K, V.ncol, V.nstage, V.nred);
     const DecLayout L(H, F, E, t, K, V.ncol, V.nstage, V.nred, lists_alias);
