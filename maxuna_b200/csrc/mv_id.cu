@@ -865,6 +865,7 @@ template <int DT, int NT, int NG, bool ODD>
 cudaError_t launch_mv_expert(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs, int x_per_row,
                              const uint32_t *ids, int top_k, float *out, int dev, int sms, cudaStream_t s) {
     constexpr int smem_max = NG == 2 ? MX_SMEM_TWO : MX_SMEM_ONE;
+    if (k > smem_max) return cudaErrorNotSupported; // the digits alone are longer, and the layout's sums stay within 32 bits
     const MxLayout L(DT == LMOE_Q4_K, 2 * NT, NG, k / QK_K, smem_max);
     if (L.nstage < NG) return cudaErrorNotSupported; // rows too long for the ring
     static thread_local int c_dev = -1;
