@@ -60,7 +60,7 @@ def test_mm_ragged_rows_multi_block_k_and_big_expert(orc, dev, dt, name):
 
 
 @pytest.mark.parametrize("dt,name", DTYPES)
-@pytest.mark.parametrize("t,n_out,k", [(80, 128, 256), (82, 130, 1280), (257, 124, 512)])
+@pytest.mark.parametrize("t,n_out,k", [(80, 128, 256), (82, 130, 1280), (257, 124, 512), (81, 131, 768)])
 def test_mm_tile_shapes(orc, dev, dt, name, t, n_out, k):
     """Both row-tile widths on either side of their rule (40 and 41 rows an expert), a row past a tile, row counts of the matrix
     that are no multiple of the copy's eight rows or of four, more than four super-blocks.  Both operands are rounded to f16
