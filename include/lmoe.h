@@ -127,9 +127,8 @@ lmoe_status lmoe_route(const float *router, const float *bias, const float *x, i
  * library instead of a workspace.  It has no counterpart in the reference.
  *   - limit: t * n_expert <= 32768 (128 KB of scratch held by every GPU that loads the
  *     library, until exit); larger requests are rejected with LMOE_ERR_INVALID;
- *   - the first call on each device looks up the array's device address, and the first call with
- *     more than 64 tokens and hidden = 3072 also sets a kernel attribute (cudaFuncSetAttribute):
- *     make one call of each kind you will use before starting any stream capture;
+ *   - the first call on each device, of any size, looks up the array's device address and sets kernel
+ *     attributes (cudaFuncSetAttribute): make one call per device before starting any stream capture;
  *   - all calls share the one array (it keeps the previous call's logits; nothing needs
  *     clearing because each call overwrites what it reads): calls that overlap on the GPU,
  *     e.g. on two streams, race.

@@ -326,7 +326,10 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict_
 //   two projections: warps 4-7 B loaders (rows in token order), the epilogue falls to the dequantising warps
 constexpr int GM_DQ_WARPS = 16, GM_DQ0 = 8; // number of dequantising warps, the first of them
 constexpr int GM_THREADS = (GM_DQ_WARPS + 8) * 32;
-constexpr int GM_Q6_PITCH = 240; // a 210-byte block inside its 224-byte aligned window; 60 words: rows spread over the banks
+// A 210-byte block inside its 224-byte aligned window.  Neighbouring lines lie in different banks (60 words), but neighbouring
+// rows lie 16 lines apart, in the same ones, and only a block's offset in its granule spreads them: the reads are 4-way at k =
+// 1024 and 3072, 8-way at 2048 and 4096, 2-way at 512 and 768.
+constexpr int GM_Q6_PITCH = 240;
 constexpr int GM_Q6_COPY = 224;
 constexpr int GM_EPI_BYTES = 1024; // one epilogue warp's staging: 8 tile columns (output rows) x 32 weight rows, f32
 constexpr int GM_BOX_ROWS = 16;    // single projection: tile stores of 16 output rows x 32 weight rows, two in flight per warp
@@ -881,8 +884,9 @@ static int mm_m_tiles(int64_t n_out) { return (int)((n_out + MM_M - 1) / MM_M); 
 
 // Routed rows per tile.  192 fills the tensor memory beside two accumulators with two operand stages and converts each
 // weight least often; with a few dozen rows per expert every tile is thin whatever its limit, and 128 leaves room for four
-// operand stages (gate/up + down, 256 experts: 16 rows per expert 417 us against 431; 80: 550 against 531; 160: 1027
-// against 739; 640: 3192 against 2790).
+// operand stages.  A block of 256 experts, evenly routed, 128 against 192, by rows per expert: 16 489 us against 497, 24 545 / 552,
+// 32 572 / 576, 40 602 / 604, 44 628 / 628, 48 688 / 663, 56 745 / 695, 80 940 / 877; of 128 experts of 768: 32 187 / 189,
+// 40 200 / 201, 48 213 / 211, 64 244 / 227.
 int mm_tile_rows(int64_t rows, int64_t n_expert) { return rows <= 40 * n_expert ? 128 : 192; }
 
 // Row tiles that `rows` routed rows over n_lists lists can make.

@@ -15,12 +15,12 @@
 // The others:
 //   mv_expert_kernel the ordinary case, bound by the weight stream: pairs of the same expert share a pass over its rows, which
 //                    come through shared memory in bulk copies.  Weights of 3 / 16 / 64 tokens with ten experts each, against
-//                    mv_pair_kernel: [1024 x 3072] Q4_K 17 / 78 / 290 -> 15 / 47 / 139 us, [3072 x 1024] Q6_K (whose 210-byte
-//                    super-blocks cost two loads a word from global memory) 39 / 203 / 810 -> 22 / 74 / 218 us.
+//                    mv_pair_kernel: [1024 x 3072] Q4_K 17 / 78 / 290 -> 15 / 55 / 144 us, [3072 x 1024] Q6_K (whose 210-byte
+//                    super-blocks cost two loads a word from global memory) 39 / 203 / 810 -> 21 / 84 / 221 us.
 //   mv_pair_kernel   Q4_K of any shape, one (token, slot) pair per block row; what is left to it are rows too long for the
 //                    ring.  Weights go straight from global memory into the A fragments.
 //   mv_multi_kernel  many pairs of ONE weight matrix (the shared expert, a plain matrix): eight pairs are the columns of
-//                    an MMA, so a super-block is unpacked once for 32 pairs.  512 pairs of [1024 x 3072] Q4_K: 830 -> 52 us.
+//                    an MMA, so a super-block is unpacked once for 32 pairs.  512 pairs of [1024 x 3072] Q4_K: 816 -> 68 us.
 #include <cooperative_groups.h>
 #include "common.cuh"
 #include "stream_math.cuh"
@@ -416,8 +416,8 @@ mv_pair_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert
 // ---- many pairs of one matrix -----------------------------------------------------------
 // grid (ceil(n_out / 64), ceil(pairs / 32)); the same warp layout.  The digits of 32 pairs are staged 512 k at a time.  Making
 // them was half of the instructions, so the CS blocks of a cluster, row blocks of the same pairs, make a share each and store
-// it to all of them through distributed shared memory (512 pairs: [1024 x 3072] Q4_K 70 -> 52 us,
-// [3072 x 1024] Q6_K 102 -> 90).
+// it to all of them through distributed shared memory (512 pairs: [1024 x 3072] Q4_K 79 -> 68 us,
+// [3072 x 1024] Q6_K 114 -> 108).
 constexpr int MM_COLS = 32, MM_KC = 512;
 // bytes of a pair's digits: the columns of one load instruction (8 bytes a lane for Q4_K, 4 for Q6_K) cover distinct banks
 template <int DT>
@@ -896,7 +896,7 @@ cudaError_t launch_mv_expert(const uint8_t *w, int64_t expert_bytes, int n_exper
 
 // One block an SM, with twice the warps on the same digits: where a row is too long for two, and for a single matrix that is
 // larger than the L2 cache, so that up to four pairs cost one pass over it ([100352 x 3072] Q6_K, 2 / 4 pairs: 86 / 172 us in
-// passes of one pair, 55 / 91 with two blocks an SM, 47 / 72 so).
+// passes of one pair, 52 / 72 so; with three digits a value 47 / 72, and 55 / 91 with two blocks an SM).
 template <int DT, bool ODD>
 cudaError_t launch_mv_by_expert(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs,
                                 int x_per_row, const uint32_t *ids, int top_k, float *out, int dev, int sms, cudaStream_t s) {
@@ -952,8 +952,8 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
         sms_dev = dev;
     }
     // One matrix for all pairs: 32 pairs to an unpacked super-block, once such blocks cover every SM.  (Below that two pairs to a
-    // block win by parallelism: [1024 x 3072] Q4_K, 64 / 512 pairs 26 / 88 us against 55 / 52, [3072 x 1024] Q6_K, 32 / 128
-    // pairs 16 / 42 against 27 / 33.)
+    // block win by parallelism: [1024 x 3072] Q4_K, 64 / 512 pairs 26 / 92 us against 44 / 68, [3072 x 1024] Q6_K, 32 / 128
+    // pairs 19 / 44 against 26 / 39.)
     if (n_expert == 1 && (pairs + MM_COLS - 1) / MM_COLS * gx >= sms && pairs > 4) {
         constexpr int smem = MM_COLS * MM_PITCH<DT> + MV_PARTS * MM_COLS * (MM_KC / QK_K * NS + 8) * 2 + (MM_KC / QK_K) * MM_COLS * 4;
         constexpr int CS = 4;
