@@ -58,11 +58,11 @@ EXPERT_BYTES = 2 * F * (H // 256) * 144 + H * (F // 256) * 210  # 6 119 424
 ROUTER_BYTES = E * H * 4
 WORKLOAD = "config2: single MoE layer decode sweep B=1/2/4/8/16 (31 tokens per step)"
 # DRAM traffic of one decode sweep (B = 1, 2, 4, 8, 16) from an ncu capture of the five launches
-# (dram__bytes_read.sum + dram__bytes_write.sum: 71.9 + 132.7 + 219.6 + 408.8 + 699.7 MB; the algorithmic figure is
+# (dram__bytes_read.sum + dram__bytes_write.sum: 71.6 + 133.7 + 220.0 + 408.8 + 700.0 MB; the algorithmic figure is
 # the mean over the three sweeps of that run).  The figure belongs to the kernel source it was captured on: when
 # csrc/decode.cu has changed since, the line reports null.
-NCU_TRAFFIC = {"bytes_per_sweep": 1.5325e9, "algorithmic_bytes_of_that_sweep": 1.4648e9,
-               "decode_cu_sha256_16": "0d41629bcc8f671b"}
+NCU_TRAFFIC = {"bytes_per_sweep": 1.5341e9, "algorithmic_bytes_of_that_sweep": 1.4648e9,
+               "decode_cu_sha256_16": "df503bb54f35ccb2"}
 NVSMI_Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
            "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,"
            "clocks_event_reasons.sw_power_cap")
