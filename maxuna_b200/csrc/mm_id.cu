@@ -326,11 +326,14 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict_
 //   two projections: warps 4-7 B loaders (rows in token order), the epilogue falls to the dequantising warps
 constexpr int GM_DQ_WARPS = 16, GM_DQ0 = 8; // number of dequantising warps, the first of them
 constexpr int GM_THREADS = (GM_DQ_WARPS + 8) * 32;
-// A 210-byte block inside its 224-byte aligned window.  Neighbouring lines lie in different banks (60 words), but neighbouring
-// rows lie 16 lines apart, in the same ones, and only a block's offset in its granule spreads them: the reads are 4-way at k =
-// 1024 and 3072, 8-way at 2048 and 4096, 2-way at 512 and 768.
+// A 210-byte block inside its 224-byte aligned window; neighbouring lines lie in different banks (60 words).
 constexpr int GM_Q6_PITCH = 240;
 constexpr int GM_Q6_COPY = 224;
+// 2^lg rows of n_blk 210-byte blocks are the least that a multiple of 16 bytes holds: the lines of the tile loads.  As few as
+// that, because 2^lg - 1 neighbours of a row lie 128 / 2^lg lines away, in its own banks but for the block's offset in its granule.
+__host__ __device__ __forceinline__ int gm_q6_lg(int n_blk) { return n_blk & 1 ? 3 : (n_blk & 2 ? 2 : (n_blk & 4 ? 1 : 0)); }
+// the line of row r of a tile
+__device__ __forceinline__ int gm_q6_line(int r, int lg) { return ((r & ((1 << lg) - 1)) << (7 - lg)) + (r >> lg); }
 constexpr int GM_EPI_BYTES = 1024; // one epilogue warp's staging: 8 tile columns (output rows) x 32 weight rows, f32
 constexpr int GM_BOX_ROWS = 16;    // single projection: tile stores of 16 output rows x 32 weight rows, two in flight per warp
 
@@ -353,12 +356,12 @@ struct GmCfg {
 
 struct GmParams {
     // Q4_K: 2-D byte views [n_expert * n_out rows][row_bytes], box = 144 bytes x 128 rows.
-    // Q6_K (n_out a multiple of 8): eight rows as one line, [rows / 8][8 * row_bytes], box = 240 bytes x 16 lines
+    // Q6_K (n_out a multiple of 2^lg, see gm_q6_lg): 2^lg rows as one line, box = 240 bytes x 128 / 2^lg lines
     // [0, 1]: the experts' stacks (gate / up, or one projection), [2, 3]: the shared expert's
     CUtensorMap map[4];
     CUtensorMap map_out;     // NPROJ = 1, sorted rows: `out` as [rows][n_out] f32, box = 32 values x 16 rows
-    int rows8;
-    const uint8_t *w[2];     // Q6_K, n_out not a multiple of 8: stack blocks, shared expert's blocks
+    int lines, lg;           // Q6_K: the views exist; lg
+    const uint8_t *w[2];     // Q6_K without them: stack blocks, shared expert's blocks
     int n_expert, m_tiles;   // list number of the shared expert; blocks of 128 weight rows
     int64_t expert_bytes;
     int n_out, k;
@@ -425,6 +428,38 @@ __device__ __forceinline__ void q6k_fields(const uint8_t *base4, int sh, int n, 
     F.s0 = __funnelshift_r(w0, w1, s);
     F.s1 = __funnelshift_r(w1, w2, s);
     F.d2 = prmt(reinterpret_cast<const uint32_t *>(base4)[(sh + 208) >> 2], 0u, (sh & 2) ? 0x3232u : 0x1010u);
+}
+// The same where a row's blocks are a multiple of 8 bytes (rows of 4 i blocks): the offset of block b in its granule is 2 b bytes
+// modulo 8 for every row of the tile, so the words come in pairs and a branch that all lanes take alike picks them.  The tile's
+// lines (gm_q6_line) then put sixteen lanes' pairs into different banks at k = 1024 and 3072 (two lanes' into the same at 2048
+// and 4096): 24 shared-memory passes a warp and block where single words of lines of eight rows took 76 (at 2048: 152), beside
+// the tensor core's own reads the bound of the down product.
+__device__ __forceinline__ void q6k_fields_paired(const uint8_t *base8, int sh, int b, int n, int lh, Q6Fields &F) {
+    const uint2 *w = reinterpret_cast<const uint2 *>(base8) + ((sh & 8) >> 3) + 8 * n + 2 * lh;
+    const uint2 *ws = reinterpret_cast<const uint2 *>(base8) + ((sh & 8) >> 3) + 24 + n;
+    const uint2 a0 = w[0], a1 = w[1], a2 = w[2], b0 = w[4], b1 = w[5], b2 = w[6];
+    const uint2 *wh = w + 16 - 4 * n;
+    const uint2 h0 = wh[0], h1 = wh[1], h2 = wh[2], s0 = ws[0], s1 = ws[1], s2 = ws[n ? 1 : 2];
+    const uint32_t s = (uint32_t)(b & 1) * 16u, dsel = (b & 1) ? 0x3232u : 0x1010u;
+    if (b & 2) {
+        F.qa[0] = __funnelshift_r(a0.y, a1.x, s); F.qa[1] = __funnelshift_r(a1.x, a1.y, s);
+        F.qa[2] = __funnelshift_r(a1.y, a2.x, s); F.qa[3] = __funnelshift_r(a2.x, a2.y, s);
+        F.qb[0] = __funnelshift_r(b0.y, b1.x, s); F.qb[1] = __funnelshift_r(b1.x, b1.y, s);
+        F.qb[2] = __funnelshift_r(b1.y, b2.x, s); F.qb[3] = __funnelshift_r(b2.x, b2.y, s);
+        F.qh[0] = __funnelshift_r(h0.y, h1.x, s); F.qh[1] = __funnelshift_r(h1.x, h1.y, s);
+        F.qh[2] = __funnelshift_r(h1.y, h2.x, s); F.qh[3] = __funnelshift_r(h2.x, h2.y, s);
+        F.s0 = __funnelshift_r(s0.y, s1.x, s); F.s1 = __funnelshift_r(s1.x, s1.y, s);
+        F.d2 = prmt(s2.y, 0u, dsel);
+    } else {
+        F.qa[0] = __funnelshift_r(a0.x, a0.y, s); F.qa[1] = __funnelshift_r(a0.y, a1.x, s);
+        F.qa[2] = __funnelshift_r(a1.x, a1.y, s); F.qa[3] = __funnelshift_r(a1.y, a2.x, s);
+        F.qb[0] = __funnelshift_r(b0.x, b0.y, s); F.qb[1] = __funnelshift_r(b0.y, b1.x, s);
+        F.qb[2] = __funnelshift_r(b1.x, b1.y, s); F.qb[3] = __funnelshift_r(b1.y, b2.x, s);
+        F.qh[0] = __funnelshift_r(h0.x, h0.y, s); F.qh[1] = __funnelshift_r(h0.y, h1.x, s);
+        F.qh[2] = __funnelshift_r(h1.x, h1.y, s); F.qh[3] = __funnelshift_r(h1.y, h2.x, s);
+        F.s0 = __funnelshift_r(s0.x, s0.y, s); F.s1 = __funnelshift_r(s0.y, s1.x, s);
+        F.d2 = prmt(s2.x, 0u, dsel);
+    }
 }
 // 16 weights of each of the half's four 32-wide groups -> o[8 g .. 8 g + 7] = group g's values 16 lh .. 16 lh + 15,
 // 8-value chunks as [0 2 1 3 4 6 5 7].  Four six-bit values are put together per word (low nibble | two high bits << 4),
@@ -633,7 +668,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         uint4 hdr, qa0, qb0, qa1, qb1;
         Q6Fields F;
         int sh = 0; // Q6_K: offset of the block inside its 16-byte granule
-        auto load = [&]() {
+        const uint32_t line = DT == LMOE_Q6_K ? (uint32_t)gm_q6_line(r, P.lg) * GM_Q6_PITCH : 0u;
+        auto load = [&](int b) {
             ok &= mb_wait(&raw_full[slot], rph);
             const uint8_t *rs = raw + (size_t)slot * C::RAW_SLOT;
             if (DT == LMOE_Q4_K) {
@@ -643,7 +679,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                 qb0 = blk[2 + 2 * j0];
                 if (NPROJ == 2) { qa1 = blk[5 + 2 * j0]; qb1 = blk[6 + 2 * j0]; }
             } else {
-                q6k_fields(rs + ((r & 7) * 16 + (r >> 3)) * GM_Q6_PITCH, sh & 15, grp, part, F);
+                if (P.lg <= 1) q6k_fields_paired(rs + line, sh, b, grp, part, F);
+                else q6k_fields(rs + line, sh & 15, grp, part, F);
                 sh += Q6K_BYTES;
             }
             __syncwarp();
@@ -656,9 +693,9 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             next = gm_tile(P, tile + gridDim.x, n_tiles);
             // (rows past the last one convert whatever the slot holds: their accumulator rows are never read)
             if (DT == LMOE_Q6_K) sh = (int)(((int64_t)T.e * P.expert_bytes + (int64_t)(T.m0 + r) * row_bytes) & 15);
-            if (NPROJ == 1) load();
+            if (NPROJ == 1) load(0);
             for (int b = 0; b < n_blk && ok; b++) {
-                if (NPROJ == 2) load();
+                if (NPROJ == 2) load(b);
                 uint32_t o[32];
                 uint32_t last = NPROJ == 2 ? 1u : use & 1;
                 if (DT == LMOE_Q4_K) {
@@ -673,7 +710,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                 }
                 store(o, last);
                 // the next column's words arrive while the store completes (two projections have no registers left for that)
-                if (NPROJ == 1 && b + 1 < n_blk) load();
+                if (NPROJ == 1 && b + 1 < n_blk) load(b + 1);
                 stored(last);
             }
             if (NPROJ == 2) {
@@ -710,17 +747,16 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                         for (int p = 0; p < NPROJ; p++)
                             tma_load_2d(dst + p * MM_M * Q4K_BYTES, &P.map[2 * T.sh + p], b * Q4K_BYTES, T.e * P.n_out + T.m0, &raw_full[slot]);
                     }
-                } else if (P.rows8) {
-                    // 210-byte blocks start at any even address, and a row is not a multiple of 16 bytes long, but eight rows
-                    // are: one tile load per row of a group of eight takes that row's block of all sixteen groups, each
+                } else if (P.lines) {
+                    // 210-byte blocks start at any even address, and a row need not be a multiple of 16 bytes long, but 2^lg rows
+                    // are: one tile load per row of a group of 2^lg takes that row's block of all groups, each
                     // inside a 240-byte window that starts on a 16-byte boundary.  (128 bulk copies of one window each
-                    // cost 65 cycles apiece: 4180 cycles per stage; these eight loads keep ahead of the conversion.)
+                    // cost 65 cycles apiece: 4180 cycles per stage; these at most eight loads keep ahead of the conversion.)
                     if (el) {
                         mb_expect_tx(&raw_full[slot], (uint32_t)C::RAW_SLOT);
-#pragma unroll
-                        for (int r8 = 0; r8 < 8; r8++)
-                            tma_load_2d(dst + r8 * 16 * GM_Q6_PITCH, &P.map[2 * T.sh], (r8 * row_bytes + b * Q6K_BYTES) & ~15,
-                                        (T.e * P.n_out + T.m0) >> 3, &raw_full[slot]);
+                        for (int i = 0; i < 1 << P.lg; i++)
+                            tma_load_2d(dst + (i << (7 - P.lg)) * GM_Q6_PITCH, &P.map[2 * T.sh], (i * row_bytes + b * Q6K_BYTES) & ~15,
+                                        (T.e * P.n_out + T.m0) >> P.lg, &raw_full[slot]);
                     }
                 } else {
                     // other row counts: each row's block inside its 224-byte aligned window (the last 16-byte granule holds
@@ -729,7 +765,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                     __syncwarp();
                     const int64_t o0 = (int64_t)T.e * P.expert_bytes + (int64_t)T.m0 * row_bytes + b * Q6K_BYTES;
                     for (int r = lane; r < vrows; r += 32)
-                        bulk_g2s(dst + ((r & 7) * 16 + (r >> 3)) * GM_Q6_PITCH, P.w[T.sh] + ((o0 + (int64_t)r * row_bytes) & ~(int64_t)15),
+                        bulk_g2s(dst + gm_q6_line(r, P.lg) * GM_Q6_PITCH, P.w[T.sh] + ((o0 + (int64_t)r * row_bytes) & ~(int64_t)15),
                                  GM_Q6_COPY, &raw_full[slot]);
                 }
                 __syncwarp();
@@ -1003,7 +1039,8 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
                                   float *out, int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
     using C = GmCfg<DT, NPROJ, NT>;
     GmParams P;
-    P.rows8 = st[0]->n_out % 8 == 0;
+    P.lg = gm_q6_lg((int)(st[0]->k / QK_K));
+    P.lines = (st[0]->n_out & ((1 << P.lg) - 1)) == 0;
     for (int p = 0; p < 2 * NPROJ; p++) {
         const lmoe_expert_stack *s = p < NPROJ ? st[p] : sh[p - NPROJ];
         if (!s) continue;
@@ -1011,8 +1048,8 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
         lmoe_status mst = LMOE_OK;
         if (DT == LMOE_Q4_K)
             mst = make_rows_map(map, s->blocks(), (uint64_t)s->row_bytes(), (uint64_t)s->n_expert * s->n_out, Q4K_BYTES, MM_M);
-        else if (P.rows8)
-            mst = make_rows_map(map, s->blocks(), 8 * (uint64_t)s->row_bytes(), (uint64_t)s->n_expert * s->n_out / 8, GM_Q6_PITCH, MM_M / 8);
+        else if (P.lines)
+            mst = make_rows_map(map, s->blocks(), (uint64_t)s->row_bytes() << P.lg, (uint64_t)(s->n_expert * s->n_out) >> P.lg, GM_Q6_PITCH, MM_M >> P.lg);
         if (mst) return mst;
     }
     P.w[0] = st[0]->blocks();

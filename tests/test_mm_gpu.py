@@ -70,6 +70,15 @@ def test_mm_tile_shapes(orc, dev, dt, name, t, n_out, k):
     assert orc.rel_l2(got, want) < 1e-3
 
 
+@pytest.mark.parametrize("n_out,k", [(6, 256), (130, 512), (128, 512), (131, 1024), (198, 1024), (129, 2048), (256, 2048), (64, 3072)])
+def test_mm_q6k_row_groups(orc, dev, n_out, k):
+    """Q6_K rows of one to twelve blocks: lines of one, two, four and eight rows, row counts that they divide and that they do
+    not.  The first expert's list is a row longer than a row tile (rows 129 of 5 experts, then 193 of 2).  f16 operands, f32 sums."""
+    for ne, t in ((5, 129), (2, 193)):
+        got, want = _case(orc, dev, 14, ne, n_out, k, t, 1, 1, np.zeros((t, 1), np.uint32) + (ne == 5), 0xA0 + k)
+        assert orc.rel_l2(got, want) < 1e-3
+
+
 def test_mm_shared_map0_bitwise_equals_self_contained(orc, dev):
     ids = orc.distinct_ids(96, 4, 8, 0x61)
     a, _ = _case(orc, dev, 12, 8, 64, 512, 96, 4, 1, ids, 0x62, shared_map=False)
