@@ -5,7 +5,7 @@
 // kernel_mul_mm_id_q{4,6}_K_f32_t, src/ops/mm_id.metal:492-647 (f16 operand
 // tiles, f32 accumulation); per-expert lists from map0, src/ops/mm_id.metal:207-269.
 //
-// One persistent CTA per SM, warp-specialised around tcgen05.mma; see grouped_mm_kernel.  The weight tile is the
+// Persistent pairs of CTAs, one CTA per SM, warp-specialised around tcgen05.mma; see grouped_mm_kernel.  The weight tile is the
 // A operand (M = 128 output features) and the routed rows are the N dimension, so ragged per-expert row counts cost
 // only a rounding to 16.  Every wait is bounded; a wait that runs out records a flag and the kernel drains and exits.
 #include <cuda.h> // CUtensorMap (types only; the encoder is fetched through the runtime)
@@ -15,7 +15,7 @@
 
 namespace {
 
-constexpr int MM_M = 128;      // weight rows per tile
+constexpr int MM_M = 128;      // weight rows per CTA; a pair's tile has twice as many
 constexpr int MM_K = 64;       // k per pipeline stage (one 128-byte swizzle row of f16)
 constexpr int MM_WAIT_HINT_NS = 1000, MM_WAIT_TRIES = 1 << 22;
 
@@ -43,6 +43,11 @@ __device__ __forceinline__ bool mb_wait(uint64_t *b, uint32_t parity) {
                  : "=r"(ok) : "r"(s32(b)), "r"(parity), "n"(MM_WAIT_HINT_NS), "n"(MM_WAIT_TRIES) : "memory");
     return ok != 0;
 }
+// Arrival at a barrier of the pair's first CTA.
+__device__ __forceinline__ void mb_arrive_first(uint64_t *b) {
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\t"
+                 "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(s32(b)) : "memory");
+}
 __device__ __noinline__ void mm_timeout(uint32_t *flag, uint32_t where) {
     if (atomicCAS(flag, 0u, (uint32_t)LMOE_FLAG_WAIT_TIMEOUT) == 0u) {
         flag[1] = 0x1000u + where;
@@ -62,14 +67,17 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Arrives, once the multiplies issued so far are done, at the barrier at this place in both CTAs of the pair.
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(bar)) : "memory");
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(s32(bar)),
+                 "h"((uint16_t)3) : "memory");
 }
-// D += A * B with the A operand in tensor memory: 128 lanes (weight rows) x 8 columns (K = 16 as f16 pairs).
+// D += A * B for both CTAs of a pair; the A operand lies in tensor memory, in each CTA its own 128 lanes (weight rows) x 8 columns
+// (K = 16 as f16 pairs), and each CTA's shared memory holds half of B's rows at the place the descriptor names.
 __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc),
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc),
         "r"(accum) : "memory");
 }
 // 32 registers of every lane -> 32 columns of the warp's 32 tensor-memory lanes; complete after tc_wait_st().
@@ -142,7 +150,7 @@ __device__ __forceinline__ uint32_t h2_sub_mul(uint32_t v, uint32_t base, uint32
 // ---- row tiles -----------------------------------------------------------------------
 // The routed rows of an expert are cut into tiles of nt.  tiles[i] = {expert, first list index, valid rows, first row in
 // expert-sorted order}; i is also the slot of the tile in the tile-ordered operands.  A GEMM tile is (row tile, block of
-// 128 weight rows), the latter varying fastest, so CTAs running side by side share the same activation rows in L2.
+// 256 weight rows), the latter varying fastest, so CTAs running side by side share the same activation rows in L2.
 // With `extra` > 0 one more list follows the experts' ("expert" n_expert): the rows 0 .. extra-1 of the shared expert.
 // Full tiles come first, then the partial ones by falling height (in sixteens of rows): the CTAs take the tiles of a product
 // in turn, so each round has tiles of one cost and the last, incomplete one the cheapest (experts' order left the SMs idle for
@@ -314,6 +322,13 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict_
 // so the dequantised tile never passes through shared memory.  A thread converts its next stage's weights BEFORE it
 // waits for the stage to be free, so the wait covers only the store.
 //
+// Two CTAs on neighbouring SMs share a tile (cta_group::2): each converts 128 of its 256 weight rows and keeps their accumulators,
+// and each loads half of the tile's activation rows, which the tensor cores of both read.  One SM alone loads 24 KB of
+// activations for 768 cycles of multiplies in gate/up, 48 KB in down, and with the weights that is more than the L2 cache hands
+// out: down of 8192 tokens took the same 990 thousand cycles without its conversions or with 16-column multiplies.  The first CTA's
+// warp 0 issues for both; whatever it waits for is signalled at its barriers by both CTAs (arrivals of the default scope: with
+// release and acquire at cluster scope a signal took over a thousand cycles), and its commits arrive in both.
+//
 // The multiplies are issued by an elected lane inside a loop that the whole warp runs: the operand addresses then
 // stay in uniform registers.  Issued from a lane == 0 branch a tcgen05.mma costs 46 cycles of issue whatever its
 // width; this way a 16-column one takes 10 and an N-column one N/2, the tensor core's own rate.
@@ -321,7 +336,7 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict_
 // Tensor-memory columns: [0, NT) and [NT, 2 NT): the gate and up accumulators, or the two accumulator
 // buffers of a single projection (its epilogue runs beside the next tile's multiplies); the rest holds the operand
 // stages, 64 columns each: two beside 192-row tiles, four beside 128-row tiles.
-//   warp 0    MMA issuer    warp 2 loader of the quantized columns    warps 8-23 dequant
+//   warp 0    MMA issuer (second CTA, single projection: relay)    warp 2 loader of the quantized columns    warps 8-23 dequant
 //   single projection: warp 1 B loader (bulk copies of the tile-ordered operand), warps 4-7 epilogue
 //   two projections: warps 4-7 B loaders (rows in token order), the epilogue falls to the dequantising warps
 constexpr int GM_DQ_WARPS = 16, GM_DQ0 = 8; // number of dequantising warps, the first of them
@@ -343,11 +358,12 @@ struct GmCfg {
     static constexpr int RAW_SLOT = NPROJ * MM_M * (DT == LMOE_Q4_K ? Q4K_BYTES : GM_Q6_PITCH);
     static constexpr int RAW_SLOTS = DT == LMOE_Q4_K && NPROJ == 1 ? 4 : 3;
     static constexpr int EPI_BYTES = NPROJ == 2 ? GM_EPI_BYTES : 2 * GM_BOX_ROWS * 128;
-    static constexpr int B_BLK = NT * MM_K * 2;         // a 64-k block of the B operand
-    static constexpr int NB = 96 * 1024 / B_BLK;        // ring of them
+    static constexpr int B_ROWS = NT / 2;
+    static constexpr int B_BLK = B_ROWS * MM_K * 2;     // a CTA's half of a 64-k block of the B operand
+    static constexpr int NB = 96 * 1024 / B_BLK < 8 ? 96 * 1024 / B_BLK : 8; // ring of them
     static constexpr int NA = (512 - 2 * NT) / 64 >= 4 ? 4 : 2, A_COL0 = 2 * NT;
     static constexpr int EPI_WARPS = NPROJ == 2 ? GM_DQ_WARPS : 4;
-    static constexpr int B_ARRIVALS = NPROJ == 2 ? 4 : 1; // per ring slot
+    static constexpr int B_ARRIVALS = NPROJ == 2 ? 8 : 1; // per ring slot (the first CTA's of a single projection: one more, see the relay)
     static constexpr int O_RAW = NB * B_BLK, O_EPI = O_RAW + RAW_SLOTS * RAW_SLOT, O_BAR = O_EPI + EPI_WARPS * EPI_BYTES;
     static constexpr int SMEM = O_BAR + 512 + 1024; // barriers, slack to align the base to 1024 bytes
     static_assert(A_COL0 + 64 * NA <= 512, "tensor memory");
@@ -362,7 +378,7 @@ struct GmParams {
     CUtensorMap map_out;     // NPROJ = 1, sorted rows: `out` as [rows][n_out] f32, box = 32 values x 16 rows
     int lines, lg;           // Q6_K: the views exist; lg
     const uint8_t *w[2];     // Q6_K without them: stack blocks, shared expert's blocks
-    int n_expert, m_tiles;   // list number of the shared expert; blocks of 128 weight rows
+    int n_expert, m_tiles;   // list number of the shared expert; blocks of 256 weight rows
     int64_t expert_bytes;
     int n_out, k;
     const uint8_t *xt;       // NPROJ = 1: f16 activations in tile order (see gather_tiles_kernel); 2: in token order
@@ -491,13 +507,13 @@ struct GmTile {
     int e, sh; // expert; 1 for the shared expert (then e is 0)
     int l0, nv, m0, slot, srow;
 };
-__device__ __forceinline__ GmTile gm_tile(const GmParams &P, int tile, int n_tiles) {
+__device__ __forceinline__ GmTile gm_tile(const GmParams &P, int tile, int n_tiles, int rank) {
     GmTile T = {0, 0, 0, 0, 0, 0, 0};
     if (tile < n_tiles) {
         const int slot = tile / P.m_tiles;
         const int4 a = __ldg(P.tiles + slot);
         const int sh = a.x == P.n_expert;
-        T = {sh ? 0 : a.x, sh, a.y, a.z, (tile - slot * P.m_tiles) * MM_M, slot, a.w};
+        T = {sh ? 0 : a.x, sh, a.y, a.z, (tile - slot * P.m_tiles) * (2 * MM_M) + rank * MM_M, slot, a.w};
     }
     return T;
 }
@@ -505,6 +521,12 @@ __device__ __forceinline__ GmTile gm_tile(const GmParams &P, int tile, int n_til
 // hides the copies' latency there.
 template <int NT>
 __device__ __forceinline__ int gm_b_group(int nv) { return nv > NT / 2 ? 1 : (nv > NT / 4 ? 2 : 4); }
+
+// rows of a tile that each CTA of a pair holds of the B operand (of the padded tile: a multiple of 8)
+__device__ __forceinline__ int gm_half(int nv) { return ((nv + 15) & ~15) >> 1; }
+__device__ __forceinline__ void pair_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 // Epilogue of the 16-column chunks c0, c0 + cs, ... of a tile for the 32 weight rows of tensor-memory quadrant q: one
 // output row per tile column.  NPROJ = 2: out = silu(gate) * up.  A lane holds one weight row, so eight columns at a
@@ -605,20 +627,21 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n_tiles = *P.n_tiles * P.m_tiles;
+    const int rank = blockIdx.x & 1, tile0 = blockIdx.x >> 1, tile_step = gridDim.x >> 1; // place in the pair; the pair's tiles
     const int n_blk = P.k / QK_K, k_blocks = P.k / MM_K;
     const int row_bytes = n_blk * (DT == LMOE_Q4_K ? Q4K_BYTES : Q6K_BYTES);
 
     if (tid == 0) {
         for (int s = 0; s < C::NA; s++) {
-            mb_init(&a_full[s], GM_DQ_WARPS / 2);
+            mb_init(&a_full[s], GM_DQ_WARPS);
             mb_init(&a_empty[s], 1);
         }
         for (int s = 0; s < 2; s++) {
             mb_init(&acc_full[s], 1);
-            mb_init(&acc_empty[s], C::EPI_WARPS);
+            mb_init(&acc_empty[s], 2 * C::EPI_WARPS);
         }
         for (int i = 0; i < C::NB; i++) {
-            mb_init(&b_full[i], C::B_ARRIVALS);
+            mb_init(&b_full[i], C::B_ARRIVALS + (NPROJ == 1 && rank == 0 ? 1 : 0));
             mb_init(&b_empty[i], 1);
         }
         for (int i = 0; i < C::RAW_SLOTS; i++) {
@@ -628,11 +651,12 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
+    pair_sync(); // the other CTA's barriers are initialised
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true; // false once a wait of this warp has run out
@@ -660,12 +684,12 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mb_arrive(&a_full[C::NA == 4 ? 2 * i + grp : grp]);
+            if (lane == 0) mb_arrive_first(&a_full[C::NA == 4 ? 2 * i + grp : grp]);
             use++;
         };
-        // the thread's part of one column: out of shared memory, then the slot goes back to the loader
+        // single projection: the thread's part of one column, out of shared memory; then the slot goes back to the loader
         const int j0 = NPROJ == 2 ? grp : 2 * grp + part;
-        uint4 hdr, qa0, qb0, qa1, qb1;
+        uint4 hdr, qa, qb;
         Q6Fields F;
         int sh = 0; // Q6_K: offset of the block inside its 16-byte granule
         const uint32_t line = DT == LMOE_Q6_K ? (uint32_t)gm_q6_line(r, P.lg) * GM_Q6_PITCH : 0u;
@@ -673,11 +697,10 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             ok &= mb_wait(&raw_full[slot], rph);
             const uint8_t *rs = raw + (size_t)slot * C::RAW_SLOT;
             if (DT == LMOE_Q4_K) {
-                const uint4 *blk = reinterpret_cast<const uint4 *>(rs + (NPROJ == 2 ? part * MM_M + r : r) * Q4K_BYTES);
+                const uint4 *blk = reinterpret_cast<const uint4 *>(rs + r * Q4K_BYTES);
                 hdr = blk[0];
-                qa0 = blk[1 + 2 * j0];
-                qb0 = blk[2 + 2 * j0];
-                if (NPROJ == 2) { qa1 = blk[5 + 2 * j0]; qb1 = blk[6 + 2 * j0]; }
+                qa = blk[1 + 2 * j0];
+                qb = blk[2 + 2 * j0];
             } else {
                 if (P.lg <= 1) q6k_fields_paired(rs + line, sh, b, grp, part, F);
                 else q6k_fields(rs + line, sh & 15, grp, part, F);
@@ -687,31 +710,49 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             if (lane == 0) mb_arrive(&raw_empty[slot]);
             if (++slot == C::RAW_SLOTS) { slot = 0; rph ^= 1; }
         };
-        GmTile T, next = gm_tile(P, blockIdx.x, n_tiles);
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, it++) {
+        // two projections: the first or second of this group's stages of a column
+        auto half = [&](uint32_t i) {
+            if (i == 0) ok &= mb_wait(&raw_full[slot], rph);
+            const uint4 *blk = reinterpret_cast<const uint4 *>(raw + (size_t)slot * C::RAW_SLOT + (part * MM_M + r) * Q4K_BYTES);
+            hdr = blk[0];
+            qa = blk[1 + 2 * j0 + 4 * i];
+            qb = blk[2 + 2 * j0 + 4 * i];
+            if (i == 1) {
+                __syncwarp();
+                if (lane == 0) mb_arrive(&raw_empty[slot]);
+                if (++slot == C::RAW_SLOTS) { slot = 0; rph ^= 1; }
+            }
+            uint32_t o[32];
+            dequant_q4k_regs(hdr, qa, qb, j0 + 2 * i, o);
+            store(o, i);
+            stored(i);
+        };
+        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        if (NPROJ == 2 && tile0 < n_tiles) half(0);
+        for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, it++) {
             T = next;
-            next = gm_tile(P, tile + gridDim.x, n_tiles);
+            next = gm_tile(P, tile + tile_step, n_tiles, rank);
             // (rows past the last one convert whatever the slot holds: their accumulator rows are never read)
             if (DT == LMOE_Q6_K) sh = (int)(((int64_t)T.e * P.expert_bytes + (int64_t)(T.m0 + r) * row_bytes) & 15);
-            if (NPROJ == 1) load(0);
-            for (int b = 0; b < n_blk && ok; b++) {
-                if (NPROJ == 2) load(b);
-                uint32_t o[32];
-                uint32_t last = NPROJ == 2 ? 1u : use & 1;
-                if (DT == LMOE_Q4_K) {
-                    dequant_q4k_regs(hdr, qa0, qb0, j0, o);
-                    if (NPROJ == 2) {
-                        store(o, 0);
-                        stored(0);
-                        dequant_q4k_regs(hdr, qa1, qb1, j0 + 2, o);
-                    }
-                } else {
-                    dequant_q6k_regs(F, part, o);
+            if (NPROJ == 1) {
+                load(0);
+                for (int b = 0; b < n_blk && ok; b++) {
+                    uint32_t o[32];
+                    const uint32_t last = use & 1;
+                    if (DT == LMOE_Q4_K) dequant_q4k_regs(hdr, qa, qb, j0, o);
+                    else dequant_q6k_regs(F, part, o);
+                    store(o, last);
+                    if (b + 1 < n_blk) load(b + 1); // the next column's words arrive while the store completes
+                    stored(last);
                 }
-                store(o, last);
-                // the next column's words arrive while the store completes (two projections have no registers left for that)
-                if (NPROJ == 1 && b + 1 < n_blk) load(b + 1);
-                stored(last);
+            } else {
+                // a column's second stage, then the first one of the next column, which may be the next tile's: it is there when
+                // that tile's multiplies may begin (96 / 512 / 4096 / 16384 tokens 391 / 526 / 1343 / 4487 us without, 387 / 521 /
+                // 1329 / 4447 so)
+                for (int b = 0; b < n_blk && ok; b++) {
+                    half(1);
+                    if (b + 1 < n_blk || tile + tile_step < n_tiles) half(0);
+                }
             }
             if (NPROJ == 2) {
                 // this warp's share of the tile's epilogue: there is one accumulator set, so nothing is multiplied meanwhile
@@ -724,18 +765,18 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                     tc_fence_before();
                 }
                 __syncwarp();
-                if (lane == 0) mb_arrive(&acc_empty[0]);
+                if (lane == 0) mb_arrive_first(&acc_empty[0]);
             }
         }
     } else if (warp == 2) {
         // ---------------- loader of the quantized columns ----------------
         const bool el = elect_one();
         uint32_t slot = 0, rph = 0;
-        GmTile T, next = gm_tile(P, blockIdx.x, n_tiles);
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             T = next;
-            next = gm_tile(P, tile + gridDim.x, n_tiles);
-            const int vrows = min(MM_M, P.n_out - T.m0);
+            next = gm_tile(P, tile + tile_step, n_tiles, rank);
+            const int vrows = max(0, min(MM_M, P.n_out - T.m0));
             for (int b = 0; b < n_blk && ok; b++) {
                 ok &= mb_wait(&raw_empty[slot], rph ^ 1);
                 uint8_t *dst = raw + (size_t)slot * C::RAW_SLOT;
@@ -776,35 +817,51 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         // ---------------- B loader: one bulk copy per 64-k block (the operand is stored in tile order) ----------------
         const bool el = elect_one();
         uint32_t slot = 0, ph = 0;
-        GmTile T, next = gm_tile(P, blockIdx.x, n_tiles);
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             T = next;
-            next = gm_tile(P, tile + gridDim.x, n_tiles);
-            const uint32_t bytes = (uint32_t)T.nv * 128u, grp = (uint32_t)gm_b_group<NT>(T.nv), sub = C::B_BLK / grp;
-            const uint8_t *src = P.xt + (size_t)T.slot * k_blocks * C::B_BLK;
+            next = gm_tile(P, tile + tile_step, n_tiles, rank);
+            const int first = rank * gm_half(T.nv), brows = max(0, min(gm_half(T.nv), T.nv - first));
+            const uint32_t bytes = (uint32_t)brows * 128u, grp = (uint32_t)gm_b_group<NT>(T.nv), sub = C::B_BLK / grp;
+            const uint8_t *src = P.xt + ((size_t)T.slot * k_blocks * NT + first) * 128;
             for (int kb = 0; kb < k_blocks && ok; kb += (int)grp) {
                 ok &= mb_wait(&b_empty[slot], ph ^ 1);
                 if (el) {
                     mb_expect_tx(&b_full[slot], bytes * grp);
-                    for (uint32_t i = 0; i < grp; i++)
-                        bulk_g2s(b_st + slot * C::B_BLK + i * sub, src + (size_t)(kb + (int)i) * C::B_BLK, bytes, &b_full[slot]);
+                    for (uint32_t i = 0; i < grp && bytes; i++)
+                        bulk_g2s(b_st + slot * C::B_BLK + i * sub, src + (size_t)(kb + (int)i) * (NT * 128), bytes, &b_full[slot]);
                 }
                 __syncwarp();
                 if (++slot == C::NB) { slot = 0; ph ^= 1; }
             }
         }
-    } else if (warp == 0) {
-        // ---------------- MMA issuer: the whole warp walks the loop, one elected lane issues ----------------
+    } else if (NPROJ == 1 && warp == 0 && rank == 1) {
+        // ---------------- relay: a bulk copy signals its own CTA only; the issuer is told that this half of a slot has landed ----------------
+        uint32_t slot = 0, ph = 0;
+        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
+            T = next;
+            next = gm_tile(P, tile + tile_step, n_tiles, rank);
+            const int grp = gm_b_group<NT>(T.nv);
+            for (int kb = 0; kb < k_blocks && ok; kb += grp) {
+                ok &= mb_wait(&b_full[slot], ph);
+                __syncwarp();
+                if (lane == 0) mb_arrive_first(&b_full[slot]);
+                if (++slot == C::NB) { slot = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 0 && rank == 0) {
+        // ---------------- MMA issuer of the pair: the whole warp walks the loop, one elected lane issues ----------------
         const bool el = elect_one();
         const uint64_t bd0 = umma_desc(s32(b_st));
         uint32_t it = 0, bs = 0, bph = 0, as = 0, aph = 0; // tiles; slot and phase of the B ring and of the operand stages
-        GmTile T, next = gm_tile(P, blockIdx.x, n_tiles);
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, it++) {
+        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, it++) {
             T = next;
-            next = gm_tile(P, tile + gridDim.x, n_tiles);
+            next = gm_tile(P, tile + tile_step, n_tiles, rank);
             const int npad = (T.nv + 15) & ~15;
             const uint32_t grp = (uint32_t)gm_b_group<NT>(T.nv), sub = (C::B_BLK >> 4) / grp;
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(MM_M >> 4) << 24);
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(2 * MM_M >> 4) << 24);
             const uint32_t buf = NPROJ == 2 ? 0u : it & 1, cph = NPROJ == 2 ? it & 1 : (it >> 1) & 1;
             ok &= mb_wait(&acc_empty[buf], cph ^ 1);
             const uint32_t d = tmem_base + buf * NT;
@@ -848,24 +905,29 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         auto announce = [&]() {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mb_arrive(&b_full[done]);
+            if (lane == 0) mb_arrive_first(&b_full[done]);
             if (++done == C::NB) done = 0;
             behind--;
         };
-        GmTile T, next = gm_tile(P, blockIdx.x, n_tiles);
-        int nsrc[NT / 16];
+        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        constexpr int RPT = C::B_ROWS / 16; // rows of a thread
+        int nsrc[RPT];
+        auto brows = [&](const GmTile &N) { return min(gm_half(N.nv), N.nv - rank * gm_half(N.nv)); };
         auto rows = [&](const GmTile &N) {
+            const int n = brows(N);
+            const int32_t *src = P.src + N.slot * NT + rank * gm_half(N.nv);
 #pragma unroll
-            for (int i = 0; i < NT / 16; i++) nsrc[i] = r0 + 16 * i < N.nv ? __ldg(P.src + N.slot * NT + r0 + 16 * i) : 0;
+            for (int i = 0; i < RPT; i++) nsrc[i] = r0 + 16 * i < n ? __ldg(src + r0 + 16 * i) : 0;
         };
         rows(next);
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+        for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             T = next;
-            next = gm_tile(P, tile + gridDim.x, n_tiles);
-            uint32_t off[NT / 16];
+            next = gm_tile(P, tile + tile_step, n_tiles, rank);
+            uint32_t off[RPT];
 #pragma unroll
-            for (int i = 0; i < NT / 16; i++) off[i] = (uint32_t)nsrc[i] * row16 + ch;
+            for (int i = 0; i < RPT; i++) off[i] = (uint32_t)nsrc[i] * row16 + ch;
             rows(next);
+            const int n = brows(T);
             const int grp = gm_b_group<NT>(T.nv);
             const uint32_t sub = C::B_BLK / grp;
             for (int kb = 0; kb < k_blocks && ok; kb += grp) {
@@ -874,8 +936,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                     const uint32_t dst = dst0 + slot * C::B_BLK + g * sub;
                     const uint4 *base = reinterpret_cast<const uint4 *>(P.xt) + (size_t)(kb + g) * 8;
 #pragma unroll
-                    for (int i = 0; i < NT / 16; i++)
-                        if (r0 + 16 * i < T.nv)
+                    for (int i = 0; i < RPT; i++)
+                        if (r0 + 16 * i < n)
                             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 2048), "l"(base + off[i]) : "memory");
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
@@ -892,32 +954,31 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         // ---------------- epilogue ----------------
         float *stage = reinterpret_cast<float *>(smem + C::O_EPI + (warp - 4) * C::EPI_BYTES);
         uint32_t it = 0;
-        GmTile T, next = gm_tile(P, blockIdx.x, n_tiles);
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, it++) {
+        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, it++) {
             T = next;
-            next = gm_tile(P, tile + gridDim.x, n_tiles);
+            next = gm_tile(P, tile + tile_step, n_tiles, rank);
             const uint32_t buf = it & 1;
             ok &= mb_wait(&acc_full[buf], (it >> 1) & 1);
             tc_fence_after();
             gm_epilogue<NPROJ, NT>(P, T, tmem_base + buf * NT, stage, warp & 3, lane, 0, 1);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mb_arrive(&acc_empty[buf]);
+            if (lane == 0) mb_arrive_first(&acc_empty[buf]);
         }
     }
     if (NPROJ == 1 && warp >= 4 && warp < GM_DQ0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (!ok && lane == 0) mm_timeout(P.flag, warp);
     tc_fence_before();
     __syncthreads();
+    pair_sync(); // neither CTA leaves while the other may signal it or multiply its operands
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
 }
 
 } // namespace
 
 // ---- host side ---------------------------------------------------------------------------
-static int mm_m_tiles(int64_t n_out) { return (int)((n_out + MM_M - 1) / MM_M); }
-
 // Routed rows per tile.  192 fills the tensor memory beside two accumulators with two operand stages and converts each
 // weight least often; with a few dozen rows per expert every tile is thin whatever its limit, and 128 leaves room for four
 // operand stages.  A block of 256 experts, evenly routed, 128 against 192, by rows per expert: 16 489 us against 497, 24 545 / 552,
@@ -1055,7 +1116,7 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
     P.w[0] = st[0]->blocks();
     P.w[1] = sh[0] ? sh[0]->blocks() : nullptr;
     P.expert_bytes = st[0]->expert_bytes(); P.n_out = (int)st[0]->n_out; P.k = (int)st[0]->k;
-    P.n_expert = R.n_expert; P.m_tiles = mm_m_tiles(st[0]->n_out);
+    P.n_expert = R.n_expert; P.m_tiles = (int)((st[0]->n_out + 2 * MM_M - 1) / (2 * MM_M));
     P.xt = static_cast<const uint8_t *>(xt); P.src = src; P.ids_map = ids_map; P.map_stride = (int)map_stride;
     P.tiles = static_cast<const int4 *>(tiles_ws); P.n_tiles = mm_tile_count(R, tiles_ws);
     P.row_scale = row_scale; P.out = out; P.sorted = sorted; P.flag = flag;
@@ -1065,15 +1126,32 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
                                       32, GM_BOX_ROWS);
         if (mst) return mst;
     }
-    static thread_local int c_dev = -1, c_sms = 0;
+    auto kernel = grouped_mm_kernel<DT, NPROJ, NT>;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(GM_THREADS);
+    cfg.dynamicSmemBytes = C::SMEM;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    static thread_local int c_dev = -1, c_grid = 0;
     int dev = 0;
     LMOE_CUDA(cudaGetDevice(&dev));
     if (dev != c_dev) {
-        LMOE_CUDA(cudaDeviceGetAttribute(&c_sms, cudaDevAttrMultiProcessorCount, dev));
-        LMOE_CUDA(cudaFuncSetAttribute(grouped_mm_kernel<DT, NPROJ, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+        int sms = 0, pairs = 0;
+        LMOE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        LMOE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+        cfg.gridDim = dim3((unsigned)(sms & ~1));
+        LMOE_CUDA(cudaOccupancyMaxActiveClusters(&pairs, kernel, &cfg));
+        if (pairs < 1) return lmoe_fail(LMOE_ERR_CUDA, "no two multiprocessors to pair");
+        c_grid = 2 * pairs < sms ? 2 * pairs : sms & ~1;
         c_dev = dev;
     }
-    grouped_mm_kernel<DT, NPROJ, NT><<<c_sms, GM_THREADS, C::SMEM, stream>>>(P);
+    cfg.gridDim = dim3((unsigned)c_grid);
+    LMOE_CUDA(cudaLaunchKernelEx(&cfg, kernel, P));
     LMOE_LAUNCH_CHECK("grouped_mm_kernel");
     return LMOE_OK;
 }
