@@ -43,6 +43,13 @@ __device__ __forceinline__ bool mb_wait(uint64_t *b, uint32_t parity) {
                  : "=r"(ok) : "r"(s32(b)), "r"(parity), "n"(MM_WAIT_HINT_NS), "n"(MM_WAIT_TRIES) : "memory");
     return ok != 0;
 }
+// Whether that phase is over, without waiting.
+__device__ __forceinline__ bool mb_test(uint64_t *b, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(s32(b)), "r"(parity) : "memory");
+    return ok != 0;
+}
 // Arrival at a barrier of the pair's first CTA.
 __device__ __forceinline__ void mb_arrive_first(uint64_t *b) {
     asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\t"
@@ -360,11 +367,12 @@ struct GmCfg {
     static constexpr int EPI_BYTES = NPROJ == 2 ? GM_EPI_BYTES : 2 * GM_BOX_ROWS * 128;
     static constexpr int B_ROWS = NT / 2;
     static constexpr int B_BLK = B_ROWS * MM_K * 2;     // a CTA's half of a 64-k block of the B operand
-    static constexpr int NB = 96 * 1024 / B_BLK < 8 ? 96 * 1024 / B_BLK : 8; // ring of them
+    static constexpr int B_SLOT = NPROJ == 2 ? B_BLK : 2 * B_BLK; // ring slot: as much as an operand stage multiplies
+    static constexpr int NB = 96 * 1024 / B_SLOT < 8 ? 96 * 1024 / B_SLOT : 8;
     static constexpr int NA = (512 - 2 * NT) / 64 >= 4 ? 4 : 2, A_COL0 = 2 * NT;
     static constexpr int EPI_WARPS = NPROJ == 2 ? GM_DQ_WARPS : 4;
     static constexpr int B_ARRIVALS = NPROJ == 2 ? 8 : 1; // per ring slot (the first CTA's of a single projection: one more, see the relay)
-    static constexpr int O_RAW = NB * B_BLK, O_EPI = O_RAW + RAW_SLOTS * RAW_SLOT, O_BAR = O_EPI + EPI_WARPS * EPI_BYTES;
+    static constexpr int O_RAW = NB * B_SLOT, O_EPI = O_RAW + RAW_SLOTS * RAW_SLOT, O_BAR = O_EPI + EPI_WARPS * EPI_BYTES;
     static constexpr int SMEM = O_BAR + 512 + 1024; // barriers, slack to align the base to 1024 bytes
     static_assert(A_COL0 + 64 * NA <= 512, "tensor memory");
     static_assert(SMEM <= 227 * 1024, "shared memory");
@@ -519,8 +527,8 @@ __device__ __forceinline__ GmTile gm_tile(const GmParams &P, int tile, int n_til
 }
 // 64-k blocks of the B operand that share one ring slot: a thin tile's blocks do not fill it, and a deeper ring is what
 // hides the copies' latency there.
-template <int NT>
-__device__ __forceinline__ int gm_b_group(int nv) { return nv > NT / 2 ? 1 : (nv > NT / 4 ? 2 : 4); }
+template <int NPROJ, int NT>
+__device__ __forceinline__ int gm_b_group(int nv) { return nv > NT / 2 ? (NPROJ == 2 ? 1 : 2) : (NPROJ == 2 && nv > NT / 4 ? 2 : 4); }
 
 // rows of a tile that each CTA of a pair holds of the B operand (of the padded tile: a multiple of 8)
 __device__ __forceinline__ int gm_half(int nv) { return ((nv + 15) & ~15) >> 1; }
@@ -822,14 +830,14 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             T = next;
             next = gm_tile(P, tile + tile_step, n_tiles, rank);
             const int first = rank * gm_half(T.nv), brows = max(0, min(gm_half(T.nv), T.nv - first));
-            const uint32_t bytes = (uint32_t)brows * 128u, grp = (uint32_t)gm_b_group<NT>(T.nv), sub = C::B_BLK / grp;
+            const uint32_t bytes = (uint32_t)brows * 128u, grp = (uint32_t)gm_b_group<NPROJ, NT>(T.nv), sub = C::B_SLOT / grp;
             const uint8_t *src = P.xt + ((size_t)T.slot * k_blocks * NT + first) * 128;
             for (int kb = 0; kb < k_blocks && ok; kb += (int)grp) {
                 ok &= mb_wait(&b_empty[slot], ph ^ 1);
                 if (el) {
                     mb_expect_tx(&b_full[slot], bytes * grp);
                     for (uint32_t i = 0; i < grp && bytes; i++)
-                        bulk_g2s(b_st + slot * C::B_BLK + i * sub, src + (size_t)(kb + (int)i) * (NT * 128), bytes, &b_full[slot]);
+                        bulk_g2s(b_st + slot * C::B_SLOT + i * sub, src + (size_t)(kb + (int)i) * (NT * 128), bytes, &b_full[slot]);
                 }
                 __syncwarp();
                 if (++slot == C::NB) { slot = 0; ph ^= 1; }
@@ -842,7 +850,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             T = next;
             next = gm_tile(P, tile + tile_step, n_tiles, rank);
-            const int grp = gm_b_group<NT>(T.nv);
+            const int grp = gm_b_group<NPROJ, NT>(T.nv);
             for (int kb = 0; kb < k_blocks && ok; kb += grp) {
                 ok &= mb_wait(&b_full[slot], ph);
                 __syncwarp();
@@ -852,15 +860,19 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         }
     } else if (warp == 0 && rank == 0) {
         // ---------------- MMA issuer of the pair: the whole warp walks the loop, one elected lane issues ----------------
+        // A wait that finds its barrier complete still takes over a hundred cycles beside the converting warps, two or three of
+        // them more than a thin tile's multiplies.  So the next stage's barriers are asked, without waiting, before this stage's
+        // multiplies are issued (512 tokens 514 -> 504 us, 1024 594 -> 581, op by op 512 849 -> 808).
         const bool el = elect_one();
         const uint64_t bd0 = umma_desc(s32(b_st));
         uint32_t it = 0, bs = 0, bph = 0, as = 0, aph = 0; // tiles; slot and phase of the B ring and of the operand stages
+        bool b_here = false, a_here = false; // they were seen to be full
         GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, it++) {
             T = next;
             next = gm_tile(P, tile + tile_step, n_tiles, rank);
             const int npad = (T.nv + 15) & ~15;
-            const uint32_t grp = (uint32_t)gm_b_group<NT>(T.nv), sub = (C::B_BLK >> 4) / grp;
+            const uint32_t grp = (uint32_t)gm_b_group<NPROJ, NT>(T.nv), sub = (C::B_SLOT >> 4) / grp;
             const uint32_t idesc = (1u << 4) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(2 * MM_M >> 4) << 24);
             const uint32_t buf = NPROJ == 2 ? 0u : it & 1, cph = NPROJ == 2 ? it & 1 : (it >> 1) & 1;
             ok &= mb_wait(&acc_empty[buf], cph ^ 1);
@@ -871,12 +883,21 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                 for (int u = 0; u < 4; u++) {
                     const bool a_first = NPROJ == 2 || (u & 1) == 0, a_last = NPROJ == 2 || (u & 1) == 1;
                     const uint32_t in = (uint32_t)u & (grp - 1); // block within its slot
-                    if (in == 0) ok &= mb_wait(&b_full[bs], bph);
-                    if (a_first) ok &= mb_wait(&a_full[as], aph);
+                    if (in == 0 && !b_here) ok &= mb_wait(&b_full[bs], bph);
+                    if (a_first && !a_here) ok &= mb_wait(&a_full[as], aph);
                     tc_fence_after();
                     const uint32_t a = tmem_base + C::A_COL0 + 64u * as + (a_first ? 0u : 32u);
-                    const uint64_t bd = bd0 + (uint64_t)(bs * (C::B_BLK >> 4) + in * sub);
+                    const uint64_t bd = bd0 + (uint64_t)(bs * (C::B_SLOT >> 4) + in * sub);
                     const bool b_last = in == grp - 1;
+                    uint64_t *const b_done = &b_empty[bs], *const a_done = &a_empty[as];
+                    if (b_last) {
+                        if (++bs == C::NB) { bs = 0; bph ^= 1; }
+                        b_here = mb_test(&b_full[bs], bph);
+                    }
+                    if (a_last) {
+                        if (++as == C::NA) { as = 0; aph ^= 1; }
+                        a_here = mb_test(&a_full[as], aph);
+                    }
                     if (el) {
 #pragma unroll
                         for (int kk = 0; kk < 4; kk++) {
@@ -884,12 +905,10 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                             tc_mma_f16_ts(d, a + 8 * kk, bd + 2 * kk, idesc, acc);
                             if (NPROJ == 2) tc_mma_f16_ts(d + NT, a + 32 + 8 * kk, bd + 2 * kk, idesc, acc);
                         }
-                        if (b_last) tc_commit(&b_empty[bs]);
-                        if (a_last) tc_commit(&a_empty[as]);
+                        if (b_last) tc_commit(b_done);
+                        if (a_last) tc_commit(a_done);
                     }
                     __syncwarp();
-                    if (b_last && ++bs == C::NB) { bs = 0; bph ^= 1; }
-                    if (a_last && ++as == C::NA) { as = 0; aph ^= 1; }
                 }
             }
             if (el) tc_commit(&acc_full[buf]);
@@ -928,12 +947,12 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             for (int i = 0; i < RPT; i++) off[i] = (uint32_t)nsrc[i] * row16 + ch;
             rows(next);
             const int n = brows(T);
-            const int grp = gm_b_group<NT>(T.nv);
-            const uint32_t sub = C::B_BLK / grp;
+            const int grp = gm_b_group<NPROJ, NT>(T.nv);
+            const uint32_t sub = C::B_SLOT / grp;
             for (int kb = 0; kb < k_blocks && ok; kb += grp) {
                 ok &= mb_wait(&b_empty[slot], ph ^ 1);
                 for (int g = 0; g < grp; g++) {
-                    const uint32_t dst = dst0 + slot * C::B_BLK + g * sub;
+                    const uint32_t dst = dst0 + slot * C::B_SLOT + g * sub;
                     const uint4 *base = reinterpret_cast<const uint4 *>(P.xt) + (size_t)(kb + g) * 8;
 #pragma unroll
                     for (int i = 0; i < RPT; i++)
