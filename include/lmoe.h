@@ -205,6 +205,20 @@ lmoe_status lmoe_silu_mul(const float *gate, const float *up, int64_t n, float *
  * out[r] = a[r] * 2^15 / l2[r], rows [rows, n].
  */
 lmoe_status lmoe_l2_rescale(const float *a, int64_t rows, int64_t n, float *out, float *l2, void *stream);
+/* The mat-vec branch of `FusedExperts::forward`, src/moe.rs:221-323, and `SharedExpert::forward`, src/moe.rs:342-344, as one
+ * call: mul_mv_id (gate, up), silu_mul, mul_mv_id (down), combine, plus the shared expert's rows, with the results of those
+ * ops called one by one and their errors.  Products that do not depend on one another share a launch.  gate / up / down, ids
+ * [t_ids, top_k] and weights [t, top_k]: the routed experts, all NULL for none; sh_*: the shared expert, all NULL for none.
+ * x [t, k]; out [t, down n_out].  Workspace: lmoe_ffn_mv_workspace_bytes, contents undefined before and after. */
+size_t lmoe_ffn_mv_workspace_bytes(const lmoe_expert_stack *gate, const lmoe_expert_stack *down,
+                                   const lmoe_expert_stack *sh_gate, const lmoe_expert_stack *sh_down,
+                                   int64_t t, int64_t top_k);
+lmoe_status lmoe_ffn_mv(const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *down,
+                        const uint32_t *ids, int64_t t_ids, int64_t top_k, const float *weights,
+                        const lmoe_expert_stack *sh_gate, const lmoe_expert_stack *sh_up,
+                        const lmoe_expert_stack *sh_down, const float *x, int64_t t, int64_t k, float *out,
+                        void *workspace, size_t workspace_bytes, void *stream);
+
 /* `ops::combine`, src/ops/combine.rs:16 -> `run_combine`, src/ops/dispatch.rs:1366-1506
  * -> kernel_moe_combine{,_rescale}, src/ops/combine.metal:70-133:
  *   out[s, c] = sum_k down[s, k, c] * (col_l2[s, k] * 2^-15) * w[s, k]

@@ -255,17 +255,121 @@ extern "C" lmoe_status lmoe_l2_rescale(const float *a, int64_t rows, int64_t n, 
     return LMOE_OK;
 }
 
-extern "C" lmoe_status lmoe_combine(const float *down, const float *col_l2, const float *weights, int64_t seq,
-                                    int64_t top_k, int64_t n_out, float *out, void *stream) {
-    lmoe_clear_error();
-    REQUIRE(down && weights && out, "down/weights/out is NULL");
+static lmoe_status combine_check(int64_t seq, int64_t top_k, int64_t n_out) {
     REQUIRE(seq >= 0 && top_k >= 1 && n_out >= 1, "combine dims must be positive");
     int64_t width = 1;
     while (width < top_k / 2) width <<= 1;
     REQUIRE(width <= 32, "combine top_k (%lld) needs a reduction width %lld > 32", (long long)top_k, (long long)width);
     REQUIRE(seq * top_k * n_out <= INT32_MAX, "combine seq*top_k*n_out (%lld) exceeds i32::MAX",
             (long long)(seq * top_k * n_out));
+    return LMOE_OK;
+}
+
+extern "C" lmoe_status lmoe_combine(const float *down, const float *col_l2, const float *weights, int64_t seq,
+                                    int64_t top_k, int64_t n_out, float *out, void *stream) {
+    lmoe_clear_error();
+    REQUIRE(down && weights && out, "down/weights/out is NULL");
+    const lmoe_status st = combine_check(seq, top_k, n_out);
+    if (st) return st;
     LMOE_CUDA(launch_combine(down, col_l2, weights, (int)seq, (int)top_k, (int)n_out, out, (cudaStream_t)stream));
+    return LMOE_OK;
+}
+
+// ---------------------------------------------------------- FFN by mat-vecs ----
+namespace {
+struct FfnRows {
+    int64_t routed, shared, ff, sh_ff, n_out; // rows and widths of the routed and the shared experts' activations
+    size_t act_bytes() const { return lmoe_align_up((size_t)(routed * ff + shared * sh_ff) * 4, 256); }
+    size_t bytes() const { return 3 * act_bytes() + (routed ? lmoe_align_up((size_t)(routed + shared) * n_out * 4, 256) : 0); }
+};
+FfnRows ffn_rows(const lmoe_expert_stack *gate, const lmoe_expert_stack *down, const lmoe_expert_stack *sh_gate, const lmoe_expert_stack *sh_down,
+                 int64_t t, int64_t top_k) {
+    return {gate ? t * top_k : 0, sh_gate ? t : 0, gate ? gate->n_out : 0, sh_gate ? sh_gate->n_out : 0, gate ? down->n_out : (sh_gate ? sh_down->n_out : 0)};
+}
+// The products of one stage of an FFN, those of one type and shape together.
+struct FfnProducts {
+    const lmoe_expert_stack *st[MV_JOBS];
+    MvJob job[MV_JOBS];
+    int n = 0;
+    void add(const lmoe_expert_stack *s, const float *x, int64_t x_per_row, const uint32_t *ids, int64_t top_k, int64_t pairs, float *out) {
+        st[n] = s;
+        job[n++] = {s->blocks(), s->expert_bytes(), (int)s->n_expert, x, (int)x_per_row, ids, (int)top_k, (int)pairs, out};
+    }
+    cudaError_t launch(cudaStream_t s) const {
+        bool done[MV_JOBS] = {};
+        for (int i = 0; i < n; i++) {
+            if (done[i]) continue;
+            MvJob same[MV_JOBS];
+            int m = 0;
+            for (int j = i; j < n; j++)
+                if (!done[j] && st[j]->dtype == st[i]->dtype && st[j]->n_out == st[i]->n_out && st[j]->k == st[i]->k) same[m++] = job[j], done[j] = true;
+            const cudaError_t e = launch_mul_mv_id_jobs(st[i]->dtype, same, m, (int)st[i]->n_out, (int)st[i]->k, s);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+};
+} // namespace
+
+extern "C" size_t lmoe_ffn_mv_workspace_bytes(const lmoe_expert_stack *gate, const lmoe_expert_stack *down, const lmoe_expert_stack *sh_gate,
+                                              const lmoe_expert_stack *sh_down, int64_t t, int64_t top_k) {
+    if ((!gate && !sh_gate) || (gate && !down) || (sh_gate && !sh_down) || t < 0 || top_k < 1 || t * top_k > INT32_MAX) return 0;
+    return ffn_rows(gate, down, sh_gate, sh_down, t, top_k).bytes();
+}
+
+extern "C" lmoe_status lmoe_ffn_mv(const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *down, const uint32_t *ids,
+                                   int64_t t_ids, int64_t top_k, const float *weights, const lmoe_expert_stack *sh_gate,
+                                   const lmoe_expert_stack *sh_up, const lmoe_expert_stack *sh_down, const float *x, int64_t t, int64_t k,
+                                   float *out, void *workspace, size_t workspace_bytes, void *stream) {
+    lmoe_clear_error();
+    cudaStream_t s = (cudaStream_t)stream;
+    REQUIRE(gate || sh_gate, "neither routed nor shared experts given");
+    REQUIRE((!gate || (up && down && weights)) && (!sh_gate || (sh_up && sh_down)), "an expert stack or the weights are NULL");
+    lmoe_status st;
+    if (gate) {
+        if ((st = lmoe_id_shape_check(gate, x, t, 1, k, ids, t_ids, top_k, out)) || (st = lmoe_id_shape_check(up, x, t, 1, k, ids, t_ids, top_k, out)) ||
+            (st = lmoe_id_shape_check(down, x, t, top_k, gate->n_out, ids, t_ids, top_k, out)))
+            return st;
+        REQUIRE(gate->n_out == up->n_out, "silu_mul shape mismatch: gate has %lld columns, up %lld", (long long)gate->n_out, (long long)up->n_out);
+        REQUIRE(t * top_k * gate->n_out <= INT32_MAX, "silu_mul n (%lld) must be in [0, i32::MAX]", (long long)(t * top_k * gate->n_out));
+        if ((st = combine_check(t, top_k, down->n_out))) return st;
+    }
+    if (sh_gate) { // its one expert's index is 0 for every token
+        if ((st = lmoe_id_shape_check(sh_gate, x, t, 1, k, x, t, 1, out)) || (st = lmoe_id_shape_check(sh_up, x, t, 1, k, x, t, 1, out)) ||
+            (st = lmoe_id_shape_check(sh_down, x, t, 1, sh_gate->n_out, x, t, 1, out)))
+            return st;
+        REQUIRE(sh_gate->n_out == sh_up->n_out, "silu_mul shape mismatch: shared gate has %lld columns, up %lld", (long long)sh_gate->n_out,
+                (long long)sh_up->n_out);
+        REQUIRE(t * sh_gate->n_out <= INT32_MAX, "silu_mul n (%lld) must be in [0, i32::MAX]", (long long)(t * sh_gate->n_out));
+        REQUIRE(!gate || sh_down->n_out == down->n_out, "shared expert width %lld does not match the experts' %lld", (long long)sh_down->n_out,
+                (long long)(gate ? down->n_out : 0));
+    }
+    const FfnRows R = ffn_rows(gate, down, sh_gate, sh_down, t, top_k);
+    REQUIRE(workspace && aligned16(workspace), "the workspace must be 16-byte aligned");
+    if (workspace_bytes < R.bytes()) return lmoe_fail(LMOE_ERR_WORKSPACE, "ffn_mv workspace needs %zu bytes, got %zu", R.bytes(), workspace_bytes);
+    if (t == 0) return LMOE_OK;
+    const size_t act_floats = R.act_bytes() / 4;
+    float *g = static_cast<float *>(workspace), *u = g + act_floats, *a = u + act_floats, *d = a + act_floats;
+    const size_t sh = (size_t)(R.routed * R.ff); // the shared expert's rows behind the routed ones
+    FfnProducts in, outp;
+    if (gate) {
+        in.add(gate, x, 1, ids, top_k, R.routed, g);
+        in.add(up, x, 1, ids, top_k, R.routed, u);
+        outp.add(down, a, top_k, ids, top_k, R.routed, d);
+    }
+    float *d_sh = gate ? d + (size_t)(R.routed * R.n_out) : out;
+    if (sh_gate) {
+        in.add(sh_gate, x, 1, nullptr, 1, t, g + sh);
+        in.add(sh_up, x, 1, nullptr, 1, t, u + sh);
+        outp.add(sh_down, a + sh, 1, nullptr, 1, t, d_sh);
+    }
+    LMOE_CUDA(in.launch(s));
+    LMOE_CUDA(launch_silu_mul(g, u, (int64_t)(sh + (size_t)(R.shared * R.sh_ff)), a, s));
+    LMOE_CUDA(outp.launch(s));
+    if (gate) {
+        LMOE_CUDA(launch_combine(d, nullptr, weights, (int)t, (int)top_k, (int)R.n_out, out, s));
+        if (sh_gate) LMOE_CUDA(launch_add_inplace(out, d_sh, t * R.n_out, s));
+    }
     return LMOE_OK;
 }
 

@@ -119,6 +119,20 @@ cudaError_t launch_mul_mv_id(int dtype, const uint8_t *w, int64_t expert_bytes, 
                              const float *x, int t, int x_per_row, const uint32_t *ids, int top_k, float *out,
                              cudaStream_t s);
 // glue.cu
+// One product of launch_mul_mv_id_jobs: `pairs` = tokens times top_k; ids NULL = expert 0 for every pair.
+constexpr int MV_JOBS = 4;
+struct MvJob {
+    const uint8_t *w;
+    int64_t expert_bytes;
+    int n_expert;
+    const float *x;
+    int x_per_row;
+    const uint32_t *ids;
+    int top_k, pairs;
+    float *out;
+};
+// Products of the same type, row count and k that do not depend on one another.
+cudaError_t launch_mul_mv_id_jobs(int dtype, const MvJob *job, int jobs, int n_out, int k, cudaStream_t s);
 cudaError_t launch_silu_mul(const float *g, const float *u, int64_t n, float *out, cudaStream_t s);
 cudaError_t launch_l2_rescale(const float *a, int64_t rows, int n, float *out, float *l2, cudaStream_t s);
 cudaError_t launch_combine(const float *down, const float *col_l2, const float *w, int seq, int top_k,

@@ -758,11 +758,22 @@ __device__ __forceinline__ void mx_units(const MxArgs P, const MxLayout L, int w
     }
 }
 
+// Up to four products of the same shape in one launch, blockIdx.z each (see launch_mul_mv_id_jobs).
+struct MxJobs {
+    MvJob job[MV_JOBS];
+};
 template <int DT, int NT, int NG, bool ODD>
 __global__ void __launch_bounds__(32 * (NG * MX_GW + 1), NG == 2 ? 2 : 1)
-mv_expert_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *__restrict__ x,
-                 int x_per_row, const uint32_t *__restrict__ ids, int top_k, int n_pairs, int smem_max, float *__restrict__ out) {
+mv_expert_kernel(const __grid_constant__ MxJobs jobs, int n_out, int k, int smem_max) {
     pdl_begin();
+    const MvJob &J = jobs.job[blockIdx.z];
+    const uint8_t *__restrict__ w = J.w;
+    const int64_t expert_bytes = J.expert_bytes;
+    const float *__restrict__ x = J.x;
+    const uint32_t *__restrict__ ids = J.ids;
+    float *__restrict__ out = J.out;
+    const int n_expert = J.n_expert, x_per_row = J.x_per_row, top_k = J.top_k, n_pairs = J.pairs;
+    if ((int)blockIdx.y >= n_pairs) return;
     constexpr int SUB = DT == LMOE_Q4_K ? 32 : 16, NS = QK_K / SUB, NP = 2 * NT, CONS_WARPS = NG * MX_GW;
     extern __shared__ __align__(128) uint8_t mx_smem[];
     __shared__ int pairs_s[NP], np_s;
@@ -862,8 +873,7 @@ mv_expert_kernel(const uint8_t *__restrict__ w, int64_t expert_bytes, int n_expe
 }
 
 template <int DT, int NT, int NG, bool ODD>
-cudaError_t launch_mv_expert(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs, int x_per_row,
-                             const uint32_t *ids, int top_k, float *out, int dev, int sms, cudaStream_t s) {
+cudaError_t launch_mv_expert_jobs(const MvJob *job, int jobs, int n_out, int k, int dev, int sms, cudaStream_t s) {
     constexpr int smem_max = NG == 2 ? MX_SMEM_TWO : MX_SMEM_ONE;
     if (k > smem_max) return cudaErrorNotSupported; // the digits alone are longer, and the layout's sums stay within 32 bits
     const MxLayout L(DT == LMOE_Q4_K, 2 * NT, NG, k / QK_K, smem_max);
@@ -875,23 +885,37 @@ cudaError_t launch_mv_expert(const uint8_t *w, int64_t expert_bytes, int n_exper
         c_dev = dev;
     }
     const int64_t units = (n_out + 16 * L.m - 1) / (16 * L.m), slots = (NG == 2 ? 2 : 1) * (int64_t)sms;
+    // Row splits: the blocks run in rounds of `slots`, and a block costs about three units of start-up.
+    MxJobs P = {};
+    int64_t groups = 0, most = 0;
+    for (int j = 0; j < jobs; j++) {
+        P.job[j] = job[j];
+        groups += job[j].n_expert == 1 ? (job[j].pairs + 2 * NT - 1) / (2 * NT) : job[j].pairs;
+        most = job[j].pairs > most ? job[j].pairs : most;
+    }
+    int64_t gx = 1, best = INT64_MAX;
+    for (int64_t rounds = 1; rounds <= 16; rounds++) {
+        int64_t g = rounds * slots / groups;
+        g = g < 1 ? 1 : (g > units ? units : g);
+        const int64_t cost = (groups * g + slots - 1) / slots * (3 + (units + g - 1) / g);
+        if (cost < best) best = cost, gx = g;
+    }
+    launch_pdl(mv_expert_kernel<DT, NT, NG, ODD>, dim3((unsigned)gx, (unsigned)most, (unsigned)jobs), 32 * (NG * MX_GW + 1), L.total, s, P, n_out, k,
+               smem_max);
+    return cudaGetLastError();
+}
+
+template <int DT, int NT, int NG, bool ODD>
+cudaError_t launch_mv_expert(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs, int x_per_row,
+                             const uint32_t *ids, int top_k, float *out, int dev, int sms, cudaStream_t s) {
     const int64_t step = 65535 / top_k * top_k; // grid.y is limited to 65535
     for (int64_t p = 0; p < pairs; p += step) {
-        const int64_t n = pairs - p < step ? pairs - p : step;
-        // Row splits: the blocks run in rounds of `slots`, and a block costs about three units of start-up.
-        const int64_t groups = n_expert == 1 ? (n + 2 * NT - 1) / (2 * NT) : n;
-        int64_t gx = 1, best = INT64_MAX;
-        for (int64_t rounds = 1; rounds <= 16; rounds++) {
-            int64_t g = rounds * slots / groups;
-            g = g < 1 ? 1 : (g > units ? units : g);
-            const int64_t cost = (groups * g + slots - 1) / slots * (3 + (units + g - 1) / g);
-            if (cost < best) best = cost, gx = g;
-        }
-        launch_pdl(mv_expert_kernel<DT, NT, NG, ODD>, dim3((unsigned)gx, (unsigned)n), 32 * (NG * MX_GW + 1), L.total, s,
-            w, expert_bytes, n_expert, n_out, k, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k, (int)n,
-            smem_max, out + (size_t)p * n_out);
+        const MvJob job = {w, expert_bytes, n_expert, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k,
+                           (int)(pairs - p < step ? pairs - p : step), out + (size_t)p * n_out};
+        const cudaError_t r = launch_mv_expert_jobs<DT, NT, NG, ODD>(&job, 1, n_out, k, dev, sms, s);
+        if (r != cudaSuccess) return r;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 // One block an SM, with twice the warps on the same digits: where a row is too long for two, and for a single matrix that is
@@ -937,24 +961,34 @@ cudaError_t launch_mv_rows(const uint8_t *w, int64_t expert_bytes, int n_expert,
     return cudaGetLastError();
 }
 
+cudaError_t mv_device(int &dev, int &sms) {
+    cudaError_t e = cudaGetDevice(&dev);
+    static thread_local int c_dev = -1, c_sms = 0;
+    if (e == cudaSuccess && dev != c_dev && (e = cudaDeviceGetAttribute(&c_sms, cudaDevAttrMultiProcessorCount, dev)) == cudaSuccess) c_dev = dev;
+    sms = c_sms;
+    return e;
+}
+bool mv_multi_better(int n_expert, int n_out, int64_t pairs, int sms) {
+    return n_expert == 1 && (pairs + MM_COLS - 1) / MM_COLS * ((n_out + MV_ROWS - 1) / MV_ROWS) >= sms && pairs > 4;
+}
+// a bulk copy starts and ends on 16 bytes: every expert must; the end of a single matrix may be ragged
+bool mv_copies(const uint8_t *w, int n_expert, int64_t expert_bytes) {
+    return (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (n_expert == 1 || expert_bytes % 16 == 0);
+}
+
 template <int DT>
 cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k, const float *x, int64_t pairs, int x_per_row,
                       const uint32_t *ids, int top_k, float *out, cudaStream_t s) {
     if (mv_rows_better<DT>(pairs, n_out, k)) return launch_mv_rows<DT>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, s);
     constexpr int NS = DT == LMOE_Q4_K ? 8 : 16;
     const unsigned gx = (unsigned)((n_out + MV_ROWS - 1) / MV_ROWS);
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    int dev, sms;
+    cudaError_t e = mv_device(dev, sms);
     if (e != cudaSuccess) return e;
-    static thread_local int sms_dev = -1, sms = 0;
-    if (dev != sms_dev) {
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        sms_dev = dev;
-    }
     // One matrix for all pairs: 32 pairs to an unpacked super-block, once such blocks cover every SM.  (Below that two pairs to a
     // block win by parallelism: [1024 x 3072] Q4_K, 64 / 512 pairs 26 / 92 us against 44 / 68, [3072 x 1024] Q6_K, 32 / 128
     // pairs 19 / 44 against 26 / 39.)
-    if (n_expert == 1 && (pairs + MM_COLS - 1) / MM_COLS * gx >= sms && pairs > 4) {
+    if (mv_multi_better(n_expert, n_out, pairs, sms)) {
         constexpr int smem = MM_COLS * MM_PITCH<DT> + MV_PARTS * MM_COLS * (MM_KC / QK_K * NS + 8) * 2 + (MM_KC / QK_K) * MM_COLS * 4;
         constexpr int CS = 4;
         static thread_local int c_dev = -1;
@@ -975,8 +1009,7 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
         }
         return cudaGetLastError();
     }
-    // a bulk copy starts and ends on 16 bytes: every expert must; the end of a single matrix may be ragged
-    if ((reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (n_expert == 1 || expert_bytes % 16 == 0)) {
+    if (mv_copies(w, n_expert, expert_bytes)) {
         const cudaError_t r = expert_bytes % 16 ? launch_mv_by_expert<DT, true>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, dev, sms, s)
                                                 : launch_mv_by_expert<DT, false>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, dev, sms, s);
         if (r != cudaErrorNotSupported) return r;
@@ -997,6 +1030,38 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
     return cudaGetLastError();
 }
 
+// Several products of one shape, those that mv_expert_kernel serves in one launch: a launch of it begins with 2 us of digits,
+// ring and barriers on every SM and ends with the slowest block, and the products of an expert FFN that do not depend on one
+// another share both.  (3 tokens op by op, ten of 256 experts [1024 x 3072] and the shared one: 112 us with twelve launches and
+// eleven calls from the host, 74 with seven and two.)
+template <int DT>
+cudaError_t launch_mv_jobs(const MvJob *job, int jobs, int n_out, int k, cudaStream_t s) {
+    int dev, sms, n = 0;
+    const cudaError_t e = mv_device(dev, sms);
+    if (e != cudaSuccess) return e;
+    MvJob together[MV_JOBS], alone[MV_JOBS];
+    int rest = 0;
+    for (int j = 0; j < jobs; j++) {
+        const MvJob &J = job[j];
+        const bool one = J.pairs > 0 && J.pairs <= 65535 && !mv_rows_better<DT>(J.pairs, n_out, k) && !mv_multi_better(J.n_expert, n_out, J.pairs, sms) &&
+                         mv_copies(J.w, J.n_expert, J.expert_bytes) && J.expert_bytes % 16 == 0 && !(J.n_expert == 1 && J.expert_bytes > MX_L2);
+        if (one) together[n++] = J;
+        else alone[rest++] = J;
+    }
+    if (n > 1) {
+        const cudaError_t r = launch_mv_expert_jobs<DT, 1, 2, false>(together, n, n_out, k, dev, sms, s);
+        if (r == cudaSuccess) n = 0;
+        else if (r != cudaErrorNotSupported) return r;
+    }
+    for (int j = 0; j < n + rest; j++) {
+        const MvJob &J = j < n ? together[j] : alone[j - n];
+        if (J.pairs == 0) continue;
+        const cudaError_t r = launch_mv<DT>(J.w, J.expert_bytes, J.n_expert, n_out, k, J.x, J.pairs, J.x_per_row, J.ids, J.top_k, J.out, s);
+        if (r != cudaSuccess) return r;
+    }
+    return cudaSuccess;
+}
+
 } // namespace
 
 cudaError_t launch_mul_mv_id(int dtype, const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k,
@@ -1006,4 +1071,10 @@ cudaError_t launch_mul_mv_id(int dtype, const uint8_t *w, int64_t expert_bytes, 
     const int64_t pairs = (int64_t)t * top_k;
     return dtype == LMOE_Q4_K ? launch_mv<LMOE_Q4_K>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, s)
                               : launch_mv<LMOE_Q6_K>(w, expert_bytes, n_expert, n_out, k, x, pairs, x_per_row, ids, top_k, out, s);
+}
+
+cudaError_t launch_mul_mv_id_jobs(int dtype, const MvJob *job, int jobs, int n_out, int k, cudaStream_t s) {
+    if (jobs > MV_JOBS) return cudaErrorInvalidValue;
+    if (n_out == 0) return cudaSuccess;
+    return dtype == LMOE_Q4_K ? launch_mv_jobs<LMOE_Q4_K>(job, jobs, n_out, k, s) : launch_mv_jobs<LMOE_Q6_K>(job, jobs, n_out, k, s);
 }

@@ -42,34 +42,28 @@ class FusedExperts(ExpertFfn):
                                 f"up={up.n_expert}, down={down.n_expert}")
         self.gate, self.up, self.down = gate, up, down
 
+    def uses_mm(self, seq, top_k, use_mm=None):
+        return ((seq >= ops.mm_id_min_seq() if use_mm is None else bool(use_mm)) and
+                all(ops.supported(s.dtype, top_k) for s in (self.gate, self.up, self.down)))
+
     def forward(self, x, ids, weights, use_mm=None):
         """`use_mm`: None applies the `seq >= mm_id_min_seq()` rule of src/moe.rs:236-240; True / False force
         the grouped-GEMM or the mat-vec op chain."""
         seq, hidden = x.shape
         top_k = ids.shape[1]
         x = _f32(x)
-        use_mm = ((seq >= ops.mm_id_min_seq() if use_mm is None else bool(use_mm)) and
-                  all(ops.supported(s.dtype, top_k) for s in (self.gate, self.up, self.down)))
-        map0 = ops.prepare_map0(self.gate.n_expert, ids) if use_mm else None
-
-        def matmul(stack, xin):
-            if map0 is not None:
-                return ops.mul_mm_id_shared(stack, xin, ids, map0)
-            return ops.mul_mv_id(stack, xin, ids)
-
-        x_g = x.view(seq, 1, hidden)
-        gate = matmul(self.gate, x_g)
-        up = matmul(self.up, x_g)
-        act = ops.silu_mul(gate, up)
         w = weights if weights.dtype == torch.float32 else weights.to(torch.float32)
-        if use_mm:
-            # the grouped GEMM stages the activation as f16: keep it in range with the
-            # per-(token, slot) L2 rescale and undo it in the combine (src/moe.rs:292-313)
-            act_s, col_l2 = ops.l2_rescale(act)
-            down = matmul(self.down, act_s)
-            return ops.combine(down, col_l2, w)
-        down = matmul(self.down, act)
-        return ops.combine(down, None, w)
+        if not self.uses_mm(seq, top_k, use_mm):
+            return ops.ffn_mv((self.gate, self.up, self.down), ids, w, None, x)
+        map0 = ops.prepare_map0(self.gate.n_expert, ids)
+        x_g = x.view(seq, 1, hidden)
+        gate = ops.mul_mm_id_shared(self.gate, x_g, ids, map0)
+        up = ops.mul_mm_id_shared(self.up, x_g, ids, map0)
+        act = ops.silu_mul(gate, up)
+        # the grouped GEMM stages the activation as f16: keep it in range with the
+        # per-(token, slot) L2 rescale and undo it in the combine (src/moe.rs:292-313)
+        act_s, col_l2 = ops.l2_rescale(act)
+        return ops.combine(ops.mul_mm_id_shared(self.down, act_s, ids, map0), col_l2, w)
 
 
 class SharedExpert:
@@ -77,17 +71,9 @@ class SharedExpert:
 
     def __init__(self, gate: ExpertStack, up: ExpertStack, down: ExpertStack):
         self.gate, self.up, self.down = gate, up, down
-        # the expert index of a small batch, laid out once with the weights (a fill kernel and 6 us of host per call otherwise)
-        self._zeros = torch.zeros(64, 1, dtype=torch.int32, device=gate.buffer.device)
 
     def forward(self, x):
-        seq, hidden = x.shape
-        zeros = self._zeros[:seq] if seq <= 64 else torch.zeros(seq, 1, dtype=torch.int32, device=x.device)
-        xg = x.reshape(seq, 1, hidden).contiguous()
-        g = ops.mul_mv_id(self.gate, xg, zeros)
-        u = ops.mul_mv_id(self.up, xg, zeros)
-        h = ops.silu_mul(g, u)
-        return ops.mul_mv_id(self.down, h, zeros).reshape(seq, hidden)
+        return ops.ffn_mv(None, None, None, (self.gate, self.up, self.down), x.contiguous())
 
 
 class MoeBlock:
@@ -162,10 +148,11 @@ class MoeBlock:
         """The reference's op-by-op sequence, src/moe.rs:73-78."""
         x = _f32(x_normed)
         ids, weights = self.route(x)
-        routed = self.experts.forward(x, ids, weights, use_mm)
-        if self.shared is None:
-            return routed
-        return routed + self.shared.forward(x)
+        e, sh = self.experts, self.shared
+        if sh is not None and not e.uses_mm(x.shape[0], ids.shape[1], use_mm):
+            return ops.ffn_mv((e.gate, e.up, e.down), ids, weights, (sh.gate, sh.up, sh.down), x)
+        routed = e.forward(x, ids, weights, use_mm)
+        return routed if sh is None else routed + sh.forward(x)
 
     def workspace(self, tokens: int) -> torch.Tensor:
         if self._ws is None or tokens > self._ws_tokens:

@@ -169,6 +169,32 @@ def l2_rescale(a: torch.Tensor):
     return out, l2
 
 
+def ffn_mv(experts, ids, weights, shared, x: torch.Tensor) -> torch.Tensor:
+    """The mat-vec op chain of an expert FFN in one call (`lmoe_ffn_mv`): x ``[t, k]`` -> ``[t, n_out]``.  ``experts``: (gate, up,
+    down) with ids ``[t, top_k]`` and f32 weights of that shape, or None; ``shared``: the shared expert's three stacks, or None.
+    Bit for bit what the ops give one by one; a call of eleven ops from Python is bound by the host."""
+    _f32_dev("x", x)
+    _require(x.dim() == 2, "x must be rank-2 [t, k]")
+    t, k = x.shape
+    g = u = d = sg = su = sd = idp = wp = None
+    t_ids, top_k = t, 1
+    if experts is not None:
+        _ids_dev(ids)
+        t_ids, top_k = ids.shape
+        _f32_dev("weights", weights)
+        if weights.shape != (t, top_k):
+            raise LmoeError(-1, f"weights shape {tuple(weights.shape)} must be [seq, top_k] = [{t}, {top_k}]")
+        g, u, d = experts[0].handle, experts[1].handle, experts[2].handle
+        idp, wp = ids.data_ptr(), weights.data_ptr()
+    if shared is not None:
+        sg, su, sd = shared[0].handle, shared[1].handle, shared[2].handle
+    out = x.new_empty((t, (experts or shared)[2].n_out))
+    n = lib().lmoe_ffn_mv_workspace_bytes(g, d, sg, sd, t, top_k)
+    ws = torch.empty(max(n, 16), dtype=torch.uint8, device=x.device)
+    check(lib().lmoe_ffn_mv(g, u, d, idp, t_ids, top_k, wp, sg, su, sd, x.data_ptr(), t, k, out.data_ptr(), ws.data_ptr(), n, stream_ptr()))
+    return out
+
+
 def combine(down: torch.Tensor, col_l2, weights: torch.Tensor) -> torch.Tensor:
     _f32_dev("down", down)
     _require(down.dim() == 3, "down must be rank-3 [seq, top_k, n_out]")

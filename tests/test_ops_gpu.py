@@ -544,3 +544,48 @@ def test_unfused_block_vs_oracle(orc, dev):
     assert np.array_equal(ids.cpu().numpy().astype(np.uint32), ids_o)
     got = blk.forward_unfused(xd).cpu().numpy()
     assert orc.rel_l2(got, want) < 1e-3
+
+
+@pytest.mark.parametrize("hidden,ff,sh_ff,ne,top_k,up_dt", [(256, 256, 256, 4, 2, 12), (2048, 768, 768, 16, 4, 12), (3072, 1024, 512, 24, 10, 12),
+                                                            (1024, 2048, 2048, 3, 3, 14)])
+def test_ffn_mv_equals_the_ops(dev, hidden, ff, sh_ff, ne, top_k, up_dt):
+    """One call for the mat-vec chain gives the bits of its ops one by one: products that share a launch and that do not (few
+    rows; another type; a shared expert of another width; many pairs of one matrix), an id that names no expert, no shared or
+    no routed experts."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    mk = lambda dt, n, o, k, s: ExpertStack.random(dt, n, o, k, seed=s, device=dev)
+    e = (mk(12, ne, ff, hidden, 1), mk(up_dt, ne, ff, hidden, 2), mk(14, ne, hidden, ff, 3))
+    sh = (mk(12, 1, sh_ff, hidden, 4), mk(12, 1, sh_ff, hidden, 5), mk(14, 1, hidden, sh_ff, 6))
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(7)
+    for t in (1, 2, 3, 9, 64, 130):
+        x = torch.randn(t, hidden, generator=gen, device=dev)
+        ids = torch.stack([torch.randperm(ne, generator=gen, device=dev)[:top_k] for _ in range(t)]).to(torch.int32)
+        ids[t // 2, 0] = ne + 5
+        w = torch.rand(t, top_k, generator=gen, device=dev)
+
+        def chain(stacks, idx):
+            xg = x.view(t, 1, hidden)
+            return ops.mul_mv_id(stacks[2], ops.silu_mul(ops.mul_mv_id(stacks[0], xg, idx), ops.mul_mv_id(stacks[1], xg, idx)), idx)
+
+        routed = ops.combine(chain(e, ids), None, w)
+        shared = chain(sh, torch.zeros(t, 1, dtype=torch.int32, device=dev)).view(t, hidden)
+        for got, want in ((ops.ffn_mv(e, ids, w, sh, x), routed + shared), (ops.ffn_mv(e, ids, w, None, x), routed),
+                          (ops.ffn_mv(None, None, None, sh, x), shared)):
+            assert torch.equal(got.view(torch.int32), want.view(torch.int32)), t
+
+
+def test_ffn_mv_errors(dev):
+    from maxuna_b200 import LmoeError, ops
+    from maxuna_b200.gguf import ExpertStack
+
+    mk = lambda dt, n, o, k: ExpertStack.random(dt, n, o, k, device=dev)
+    e = (mk(12, 4, 256, 512), mk(12, 4, 256, 512), mk(14, 4, 512, 256))
+    x, ids, w = torch.zeros(2, 512, device=dev), torch.zeros(2, 2, dtype=torch.int32, device=dev), torch.zeros(2, 2, device=dev)
+    for bad in ((e, ids, w, None, torch.zeros(2, 256, device=dev)), (e, ids, w[:1], None, x), (e, ids[:1], w, None, x),
+                ((e[0], mk(12, 4, 128, 512), e[2]), ids, w, None, x), ((e[0], e[1], mk(14, 4, 512, 512)), ids, w, None, x),
+                (e, ids, w, (e[0], e[1], mk(14, 1, 256, 256)), x), (e, ids, w.double(), None, x)):
+        with pytest.raises(LmoeError):
+            ops.ffn_mv(*bad)
