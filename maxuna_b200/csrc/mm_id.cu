@@ -155,68 +155,96 @@ __device__ __forceinline__ uint32_t h2_sub_mul(uint32_t v, uint32_t base, uint32
 }
 
 // ---- row tiles -----------------------------------------------------------------------
-// The routed rows of an expert are cut into tiles of nt.  tiles[i] = {expert, first list index, valid rows, first row in
-// expert-sorted order}; i is also the slot of the tile in the tile-ordered operands.  A GEMM tile is (row tile, block of
-// 256 weight rows), the latter varying fastest, so CTAs running side by side share the same activation rows in L2.
+// The routed rows of an expert are cut into as few tiles as nt rows each allow, of even height: sixteens of rows, a tile one
+// more or less than another.  A stage of a tile takes the multiplies' time, but from about 150 rows down the conversion's, which
+// is the same for any height, so a full tile and a thin one cost more than two even ones (256 experts, 8192 tokens 2383 us
+// with full tiles and a rest, 2348 so; Zipf, 6000 tokens 1935 and 1888).  tiles[i] = {expert, first list index,
+// valid rows, first row in expert-sorted order}; i is also the slot of the tile in the tile-ordered operands.  A GEMM tile is (row
+// tile, block of 256 weight rows), the latter varying fastest, so CTAs running side by side share the same activation rows in L2.
 // With `extra` > 0 one more list follows the experts' ("expert" n_expert): the rows 0 .. extra-1 of the shared expert.
-// Full tiles come first, then the partial ones by falling height (in sixteens of rows): the CTAs take the tiles of a product
-// in turn, so each round has tiles of one cost and the last, incomplete one the cheapest (experts' order left the SMs idle for
-// 13 % of the gate/up product of 2048 tokens; the whole call 920 -> 892 us, 600 tokens with 128 experts of 768 217 -> 208).
+// The tiles stand by falling height: the CTAs take the tiles of a product in turn, so each round has tiles of one cost and the
+// last, incomplete one the cheapest (experts' order left the SMs idle for 13 % of the gate/up product of 2048 tokens; the whole
+// call 920 -> 892 us, 600 tokens with 128 experts of 768 217 -> 208).
 __global__ void __launch_bounds__(1024) row_tiles_kernel(const uint32_t *__restrict__ tpe, int n_expert, int extra, int nt,
                                                          int4 *__restrict__ tiles, int32_t *__restrict__ n_tiles, int max_tiles) {
     pdl_begin();
-    __shared__ int2 warp_sum[32];
-    __shared__ int part_total, part_cnt[32][16]; // partial tiles by warp and by sixteens of rows
+    __shared__ int warp_sum[32];
+    __shared__ int2 of_height[1024];  // an expert's tiles of its larger and its smaller height: height << 24 | count
+    __shared__ int first[32][16];     // tiles by warp and height, then the place of the first of them
     const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
     const int rows = e < n_expert ? (int)tpe[e] : (e == n_expert ? extra : 0);
-    const int full = rows / nt, rest = rows - full * nt, bucket = (rest + 15) / 16; // bucket 0: no partial tile
-    if (lane < 16) part_cnt[warp][lane] = 0;
-    const uint32_t same = __match_any_sync(0xffffffffu, bucket), below = (1u << lane) - 1u;
-    __syncwarp();
-    if ((same & below) == 0) part_cnt[warp][bucket] = __popc(same);
-    int ct = full, cr = rows; // inclusive prefix sums
+    const int n16 = (rows + 15) / 16, n = (rows + nt - 1) / nt, low = n ? n16 / n : 0, high_n = n ? n16 - low * n : 0;
+    int cr = rows; // inclusive prefix sum
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int a = __shfl_up_sync(0xffffffffu, ct, o), b = __shfl_up_sync(0xffffffffu, cr, o);
-        if (lane >= o) { ct += a; cr += b; }
+        const int v = __shfl_up_sync(0xffffffffu, cr, o);
+        if (lane >= o) cr += v;
     }
-    if (lane == 31) warp_sum[warp] = make_int2(ct, cr);
+    if (lane == 31) warp_sum[warp] = cr;
+    // the warp's tiles by height, and how many of a lane's height are before its own
+    int at_high = 0, at_low;
+    if (lane < 16) first[warp][lane] = 0;
+    __syncwarp();
+    if (!__any_sync(0xffffffffu, n > 1)) { // one tile each
+        const uint32_t same = __match_any_sync(0xffffffffu, low);
+        at_low = __popc(same & ((1u << lane) - 1u));
+        if (at_low == 0) first[warp][low] = __popc(same);
+    } else { // the larger heights first, then the smaller ones
+        of_height[e] = make_int2((low + 1) << 24 | high_n, low << 24 | (n - high_n)); // a list has fewer than 2^24 tiles
+        __syncwarp();
+        int all = 0;
+        at_low = 0;
+        for (uint32_t left = __ballot_sync(0xffffffffu, n > 0); left; left &= left - 1u) {
+            const int l = __ffs(left) - 1;
+            const int2 h = of_height[32 * warp + l];
+            const int hh = h.x >> 24, hn = h.x & 0xffffff, lh = h.y >> 24, ln = h.y & 0xffffff;
+            all += (hh == lane ? hn : 0) + (lh == lane ? ln : 0);
+            at_high += l < lane && hh == low + 1 ? hn : 0;
+            at_low += (hh == low ? hn : 0) + (l < lane && lh == low ? ln : 0);
+        }
+        if (lane < 16) first[warp][lane] = all;
+    }
     __syncthreads();
     if (warp == 0) {
-        int2 v = warp_sum[lane];
+        int v = warp_sum[lane];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int a = __shfl_up_sync(0xffffffffu, v.x, o), b = __shfl_up_sync(0xffffffffu, v.y, o);
-            if (lane >= o) { v.x += a; v.y += b; }
+            const int a = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += a;
         }
         warp_sum[lane] = v;
-    } else if (warp == 1 && lane < 16) { // partial tiles: the warps' counts of a bucket -> first places, the largest bucket first
+    } else if (warp == 1 && lane < 16) { // the warps' counts of a height -> places, the largest height first
         const int warps = (n_expert + 32) / 32;
-        int n = 0;
-        for (int w = 0; w < warps; w++) n += part_cnt[w][lane];
-        if (lane == 0) n = 0;
-        int ge = n; // partial tiles of this bucket and the larger ones
+        int c = 0;
+        for (int w = 0; w < warps; w++) c += first[w][lane];
+        if (lane == 0) c = 0;
+        int ge = c; // tiles of this height and the larger ones
 #pragma unroll
         for (int o = 1; o < 16; o <<= 1) {
             const int a = __shfl_down_sync(0x0000ffffu, ge, o, 16);
             if (lane + o < 16) ge += a;
         }
-        int first = ge - n;
+        int at = ge - c;
         for (int w = 0; w < warps; w++) {
-            const int c = part_cnt[w][lane];
-            part_cnt[w][lane] = first;
-            first += c;
+            const int m = first[w][lane];
+            first[w][lane] = at;
+            at += m;
         }
-        if (lane == 1) part_total = ge;
+        if (lane == 0) *n_tiles = min(ge, max_tiles);
     }
     __syncthreads();
-    const int n_full = warp_sum[31].x;
-    if (e == 0) *n_tiles = min(n_full + part_total, max_tiles);
-    const int t0 = ct - full + (warp ? warp_sum[warp - 1].x : 0), r0 = cr - rows + (warp ? warp_sum[warp - 1].y : 0);
-    for (int i = 0; i < full; i++)
-        if (t0 + i < max_tiles) tiles[t0 + i] = make_int4(e, i * nt, nt, r0 + i * nt);
-    const int tp = n_full + part_cnt[warp][bucket] + __popc(same & below);
-    if (rest && tp < max_tiles) tiles[tp] = make_int4(e, full * nt, rest, r0 + full * nt);
+    const int r0 = cr - rows + (warp ? warp_sum[warp - 1] : 0);
+    if (n == 1) { // (the whole list, whatever the height)
+        const int t = first[warp][low] + at_low;
+        if (t < max_tiles) tiles[t] = make_int4(e, 0, rows, r0);
+        return;
+    }
+    for (int i = 0; i < n; i++) {
+        const bool high = i < high_n;
+        const int t = high ? first[warp][low + 1] + at_high + i : first[warp][low] + at_low + i - high_n;
+        const int l0 = 16 * (i * low + min(i, high_n));
+        if (t < max_tiles) tiles[t] = make_int4(e, l0, min(16 * (low + high), rows - l0), r0 + l0);
+    }
 }
 
 // Routed rows -> the f16 B operand in TILE ORDER.  Row tile `slot` (nt routed rows of one expert)

@@ -79,6 +79,15 @@ def test_mm_q6k_row_groups(orc, dev, n_out, k):
         assert orc.rel_l2(got, want) < 1e-3
 
 
+@pytest.mark.parametrize("counts", [(193, 385, 577, 0, 1), (192, 384, 208, 16, 17), (129, 0, 0, 31, 0, 257, 1, 0, 16, 33, 0, 0, 47, 0, 0)])
+def test_mm_even_row_tiles(orc, dev, counts):
+    """Lists of zero to four row tiles, of heights that do and do not divide, of 192 rows a tile (the first two) and 128.  Bound as in
+    test_mm_tile_shapes."""
+    ids = np.repeat(np.arange(len(counts), dtype=np.uint32), counts)[np.random.default_rng(len(counts)).permutation(sum(counts))][:, None]
+    got, want = _case(orc, dev, 12, len(counts), 64, 256, sum(counts), 1, 1, ids, 0xB0)
+    assert orc.rel_l2(got, want) < 1e-3
+
+
 def test_mm_shared_map0_bitwise_equals_self_contained(orc, dev):
     ids = orc.distinct_ids(96, 4, 8, 0x61)
     a, _ = _case(orc, dev, 12, 8, 64, 512, 96, 4, 1, ids, 0x62, shared_map=False)
