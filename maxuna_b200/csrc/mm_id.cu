@@ -361,8 +361,10 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict_
 // and each loads half of the tile's activation rows, which the tensor cores of both read.  One SM alone loads 24 KB of
 // activations for 768 cycles of multiplies in gate/up, 48 KB in down, and with the weights that is more than the L2 cache hands
 // out: down of 8192 tokens took the same 990 thousand cycles without its conversions or with 16-column multiplies.  The first CTA's
-// warp 0 issues for both; whatever it waits for is signalled at its barriers by both CTAs (arrivals of the default scope: with
-// release and acquire at cluster scope a signal took over a thousand cycles), and its commits arrive in both.
+// warp 0 issues for both; whatever it waits for is signalled at its barriers by both CTAs, and its commits arrive in both.  (What is
+// handed over lies in tensor memory, behind tcgen05 fences, or in a CTA's own shared memory, behind a proxy fence or a bulk copy's
+// completion, so the arrivals are of the default scope: with release and acquire at cluster scope a signal took over a thousand
+// cycles.)
 //
 // The multiplies are issued by an elected lane inside a loop that the whole warp runs: the operand addresses then
 // stay in uniform registers.  Issued from a lane == 0 branch a tcgen05.mma costs 46 cycles of issue whatever its
@@ -654,7 +656,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *b_st = smem, *raw = smem + C::O_RAW;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + C::O_BAR);
-    // a_full[s]: the eight warps of the stage's group; a_empty[s]: one commit; b_full[i]: the copy's bytes; b_empty[i]: one commit;
+    // a_full[s]: the eight warps of the stage's group, of both CTAs; a_empty[s]: one commit; b_full[i]: the copies' bytes, or both CTAs'
+    // loaders; b_empty[i]: one commit;
     // raw_full[i]: the copies' bytes; raw_empty[i]: all sixteen dequantising warps; acc_*: per accumulator buffer
     uint64_t *a_full = bars, *a_empty = bars + 4, *b_full = bars + 8, *b_empty = bars + 16, *raw_full = bars + 24,
              *raw_empty = bars + 28, *acc_full = bars + 32, *acc_empty = bars + 34;
@@ -662,7 +665,6 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
     static_assert(C::NB <= 8 && C::RAW_SLOTS <= 4 && C::NA <= 4, "barrier table");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n_tiles = *P.n_tiles * P.m_tiles;
     const int rank = blockIdx.x & 1, tile0 = blockIdx.x >> 1, tile_step = gridDim.x >> 1; // place in the pair; the pair's tiles
     const int n_blk = P.k / QK_K, k_blocks = P.k / MM_K;
     const int row_bytes = n_blk * (DT == LMOE_Q4_K ? Q4K_BYTES : Q6K_BYTES);
@@ -695,6 +697,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
     pair_sync(); // the other CTA's barriers are initialised
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    asm volatile("griddepcontrol.wait;" ::: "memory"); // what earlier kernels wrote is read from here on
+    const int n_tiles = *P.n_tiles * P.m_tiles;
     bool ok = true; // false once a wait of this warp has run out
 
     if (warp >= GM_DQ0) {
@@ -1028,9 +1032,9 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
 // ---- host side ---------------------------------------------------------------------------
 // Routed rows per tile.  192 fills the tensor memory beside two accumulators with two operand stages and converts each
 // weight least often; with a few dozen rows per expert every tile is thin whatever its limit, and 128 leaves room for four
-// operand stages.  A block of 256 experts, evenly routed, 128 against 192, by rows per expert: 16 489 us against 497, 24 545 / 552,
-// 32 572 / 576, 40 602 / 604, 44 628 / 628, 48 688 / 663, 56 745 / 695, 80 940 / 877; of 128 experts of 768: 32 187 / 189,
-// 40 200 / 201, 48 213 / 211, 64 244 / 227.
+// operand stages.  A call of 256 experts [3072 x 1024], evenly routed, 128 against 192, by rows per expert: 8 461 us against 460,
+// 16 490 / 472, 24 516 / 513, 32 525 / 523, 40 547 / 544, 48 586 / 555, 64 620 / 613, 80 683 / 670; of 128 experts [2048 x 768]: 8
+// 183 / 190, 16 192 / 198, 24 199 / 209, 32 200 / 211, 40 209 / 215, 48 212 / 226, 64 217 / 219, 80 224 / 230.
 int mm_tile_rows(int64_t rows, int64_t n_expert) { return rows <= 40 * n_expert ? 128 : 192; }
 
 // Row tiles that `rows` routed rows over n_lists lists can make.
@@ -1174,16 +1178,20 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
         if (mst) return mst;
     }
     auto kernel = grouped_mm_kernel<DT, NPROJ, NT>;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GM_THREADS);
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    // With thin tiles the launch (barriers, tensor memory, the pair's meeting) overlaps the end of the kernel before: 70 to 600 tokens
+    // on 64 to 256 experts 3 to 5 us less of 95 to 640.  From 2048 tokens on that cost 2 to 4 %.
+    cfg.numAttrs = NT == 128 ? 2 : 1;
     static thread_local int c_dev = -1, c_grid = 0;
     int dev = 0;
     LMOE_CUDA(cudaGetDevice(&dev));
