@@ -219,6 +219,15 @@ lmoe_status lmoe_ffn_mv(const lmoe_expert_stack *gate, const lmoe_expert_stack *
                         const lmoe_expert_stack *sh_down, const float *x, int64_t t, int64_t k, float *out,
                         void *workspace, size_t workspace_bytes, void *stream);
 
+/* The grouped-GEMM branch of `FusedExperts::forward`, src/moe.rs:236-323, as one call: prepare_map0, mul_mm_id (gate, up),
+ * silu_mul, l2_rescale, mul_mm_id (down), combine, with the results of those ops called one by one and their errors; a
+ * (token, slot) whose id names no expert counts nothing.  Expert widths up to 12288.  Workspace: lmoe_ffn_mm_workspace_bytes,
+ * 256-byte aligned, contents undefined before and after. */
+size_t lmoe_ffn_mm_workspace_bytes(const lmoe_expert_stack *gate, const lmoe_expert_stack *down, int64_t t, int64_t top_k);
+lmoe_status lmoe_ffn_mm(const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *down,
+                        const uint32_t *ids, int64_t t_ids, int64_t top_k, const float *weights, const float *x,
+                        int64_t t, int64_t k, float *out, void *workspace, size_t workspace_bytes, void *stream);
+
 /* `ops::combine`, src/ops/combine.rs:16 -> `run_combine`, src/ops/dispatch.rs:1366-1506
  * -> kernel_moe_combine{,_rescale}, src/ops/combine.metal:70-133:
  *   out[s, c] = sum_k down[s, k, c] * (col_l2[s, k] * 2^-15) * w[s, k]

@@ -44,6 +44,8 @@ PROTOTYPES = {
     "lmoe_l2_rescale": (c_i32, [c_vp, c_i64, c_i64, c_vp, c_vp, c_vp]),
     "lmoe_ffn_mv_workspace_bytes": (c_sz, [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64]),
     "lmoe_ffn_mv": (c_i32, [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_sz, c_vp]),
+    "lmoe_ffn_mm_workspace_bytes": (c_sz, [c_vp, c_vp, c_i64, c_i64]),
+    "lmoe_ffn_mm": (c_i32, [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_sz, c_vp]),
     "lmoe_combine": (c_i32, [c_vp, c_vp, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp]),
     "lmoe_layer_create": (c_i32, [c_i64, c_i64, c_i64, c_i64, c_f32, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp,
                                   c_vp, c_vp, C.POINTER(c_vp)]),

@@ -255,7 +255,7 @@ extern "C" lmoe_status lmoe_l2_rescale(const float *a, int64_t rows, int64_t n, 
     return LMOE_OK;
 }
 
-static lmoe_status combine_check(int64_t seq, int64_t top_k, int64_t n_out) {
+lmoe_status lmoe_combine_check(int64_t seq, int64_t top_k, int64_t n_out) {
     REQUIRE(seq >= 0 && top_k >= 1 && n_out >= 1, "combine dims must be positive");
     int64_t width = 1;
     while (width < top_k / 2) width <<= 1;
@@ -269,7 +269,7 @@ extern "C" lmoe_status lmoe_combine(const float *down, const float *col_l2, cons
                                     int64_t top_k, int64_t n_out, float *out, void *stream) {
     lmoe_clear_error();
     REQUIRE(down && weights && out, "down/weights/out is NULL");
-    const lmoe_status st = combine_check(seq, top_k, n_out);
+    const lmoe_status st = lmoe_combine_check(seq, top_k, n_out);
     if (st) return st;
     LMOE_CUDA(launch_combine(down, col_l2, weights, (int)seq, (int)top_k, (int)n_out, out, (cudaStream_t)stream));
     return LMOE_OK;
@@ -332,7 +332,7 @@ extern "C" lmoe_status lmoe_ffn_mv(const lmoe_expert_stack *gate, const lmoe_exp
             return st;
         REQUIRE(gate->n_out == up->n_out, "silu_mul shape mismatch: gate has %lld columns, up %lld", (long long)gate->n_out, (long long)up->n_out);
         REQUIRE(t * top_k * gate->n_out <= INT32_MAX, "silu_mul n (%lld) must be in [0, i32::MAX]", (long long)(t * top_k * gate->n_out));
-        if ((st = combine_check(t, top_k, down->n_out))) return st;
+        if ((st = lmoe_combine_check(t, top_k, down->n_out))) return st;
     }
     if (sh_gate) { // its one expert's index is 0 for every token
         if ((st = lmoe_id_shape_check(sh_gate, x, t, 1, k, x, t, 1, out)) || (st = lmoe_id_shape_check(sh_up, x, t, 1, k, x, t, 1, out)) ||

@@ -14,6 +14,8 @@ enum {
 lmoe_status lmoe_id_shape_check(const lmoe_expert_stack *stack, const void *x, int64_t t, int64_t x_per_row,
                                 int64_t k, const void *ids, int64_t t_ids, int64_t top_k, const void *out);
 
+lmoe_status lmoe_combine_check(int64_t seq, int64_t top_k, int64_t n_out);
+
 // Rows of one grouped product (mm_id.cu): `rows` routed rows over n_expert lists, `extra` rows of the shared expert behind
 // them, row tiles of nt rows.
 struct MmRows {

@@ -54,6 +54,51 @@ __global__ void __launch_bounds__(256) l2_rescale_kernel(const float *__restrict
     if (lane == 0) l2[row] = norm;
 }
 
+// Both steps at once, a warp a row: the bits of silu_mul_kernel and l2_rescale_kernel, rounded to f16 as gather_tiles_kernel
+// does.  The activations stay in shared memory between the two passes instead of going through memory three times (5120 x 1024
+// values, with a cold cache: 12 + 16 + 11 us in three kernels).
+__global__ void __launch_bounds__(256) silu_rescale_tiles_kernel(const float *__restrict__ g, const float *__restrict__ u,
+                                                                 const int32_t *__restrict__ pos, int64_t rows, int n, int nt,
+                                                                 uint8_t *__restrict__ act, float *__restrict__ l2, float *__restrict__ y, int n_y) {
+    pdl_begin();
+    extern __shared__ __align__(16) float sr_rows[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
+    if (row >= rows) return;
+    const int p = pos[row];
+    if (p < 0) {
+        for (int i = lane; i < n_y; i += 32) y[row * n_y + i] = 0.f;
+        if (lane == 0) l2[row] = 1.0f;
+        return;
+    }
+    const float *gr = g + row * n, *ur = u + row * n;
+    float *a = sr_rows + (size_t)warp * n;
+    float ss = 0.f;
+#pragma unroll 4
+    for (int i = lane; i < n; i += 32) {
+        const float v = silu_mul(__ldg(gr + i), __ldg(ur + i));
+        a[i] = v;
+        ss = __fmaf_rn(v, v, ss);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float norm = isnan(ss) ? ss : fminf(fmaxf(sqrtf(ss), 1e-8f), 1e30f);
+    __syncwarp();
+    for (int i = lane * 8; i < n; i += 256) {
+        const float4 b = *reinterpret_cast<const float4 *>(a + i), c = *reinterpret_cast<const float4 *>(a + i + 4);
+        const float v[8] = {b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+        float q[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) q[j] = __fdiv_rn(__fmul_rn(v[j], 32768.0f), norm);
+        __align__(16) __half2 h[4] = {__floats2half2_rn(q[0], q[2]), __floats2half2_rn(q[1], q[3]), __floats2half2_rn(q[4], q[6]),
+                                      __floats2half2_rn(q[5], q[7])};
+        const int ci = i >> 3;
+        const size_t off = (((size_t)(p / nt) * (n / 64) + (ci >> 3)) * nt + (p % nt)) * 128 + ((size_t)((ci & 7) ^ (p & 7)) << 4);
+        *reinterpret_cast<uint4 *>(act + off) = *reinterpret_cast<const uint4 *>(h);
+    }
+    if (lane == 0) l2[row] = norm;
+}
+
 __global__ void add_inplace_kernel(float *__restrict__ out, const float *__restrict__ b, int64_t n) {
     pdl_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -230,6 +275,17 @@ cudaError_t launch_silu_mul(const float *g, const float *u, int64_t n, float *ou
     if (aligned16_all(g, u, out)) launch_pdl(silu_mul_kernel<true, 4>, g4, 256, 0, s, g, u, n, out);
     else if (n >= 1 << 18) launch_pdl(silu_mul_kernel<false, 4>, g4, 256, 0, s, g, u, n, out);
     else launch_pdl(silu_mul_kernel<false, 1>, (unsigned)((n + 255) / 256), 256, 0, s, g, u, n, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_silu_rescale_tiles(const float *g, const float *u, const int32_t *pos, int64_t rows, int n, int nt, void *act, float *l2,
+                                      float *y, int n_y, cudaStream_t s) {
+    if (rows == 0) return cudaSuccess;
+    int warps = 48 * 1024 / (4 * n); // whole rows in the shared memory that needs no opt-in
+    warps = warps > 8 ? 8 : warps;
+    if (warps < 1) return cudaErrorInvalidValue;
+    launch_pdl(silu_rescale_tiles_kernel, (unsigned)((rows + warps - 1) / warps), 32 * warps, (size_t)warps * n * 4, s, g, u, pos, rows, n, nt,
+               static_cast<uint8_t *>(act), l2, y, n_y);
     return cudaGetLastError();
 }
 

@@ -513,6 +513,75 @@ extern "C" lmoe_status lmoe_mul_mm_id(const lmoe_expert_stack *stack, const floa
     return mm_id_run(stack, x, t, x_per_row, k, ids, t_ids, top_k, map0, out, workspace, mm, (cudaStream_t)stream);
 }
 
+// The grouped-GEMM branch of `FusedExperts::forward` as one call: map0, mul_mm_id (gate, up), silu_mul, l2_rescale, mul_mm_id
+// (down), combine, with the bits of the ops one by one.  The tables and the f16 copy of x are made once for both projections,
+// and the activations go straight into the down product's operand.
+struct FfnMmLayout {
+    MmRows R;
+    size_t map0, tiles, xt, pos, g, u, act, l2, d, total;
+    FfnMmLayout(const lmoe_expert_stack *gate, const lmoe_expert_stack *down, int64_t t, int64_t top_k) : R(mm_rows(t * top_k, 0, gate->n_expert)) {
+        const size_t rows = (size_t)R.rows;
+        size_t o = 256; // device flag
+        auto take = [&](size_t n) { const size_t at = o; o += lmoe_align_up(n, 256); return at; };
+        map0 = take(lmoe_map0_scratch_bytes(gate->n_expert, t));
+        tiles = take(mm_tiles_bytes(R));
+        xt = take(mm_tiled_bytes(R, gate->k));
+        pos = take(rows * 4);
+        g = take(rows * gate->n_out * 4);
+        u = take(rows * gate->n_out * 4);
+        act = take(mm_tiled_bytes(R, gate->n_out));
+        l2 = take(rows * 4);
+        d = take(rows * down->n_out * 4);
+        total = o;
+    }
+};
+
+extern "C" size_t lmoe_ffn_mm_workspace_bytes(const lmoe_expert_stack *gate, const lmoe_expert_stack *down, int64_t t, int64_t top_k) {
+    if (!gate || !down || t < 0 || top_k < 1 || t * top_k > INT32_MAX / 2) return 0;
+    return FfnMmLayout(gate, down, t, top_k).total;
+}
+
+extern "C" lmoe_status lmoe_ffn_mm(const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *down, const uint32_t *ids,
+                                   int64_t t_ids, int64_t top_k, const float *weights, const float *x, int64_t t, int64_t k, float *out,
+                                   void *workspace, size_t workspace_bytes, void *stream) {
+    lmoe_clear_error();
+    cudaStream_t s = (cudaStream_t)stream;
+    if (!gate || !up || !down || !weights) return lmoe_fail(LMOE_ERR_INVALID, "an expert stack or the weights are NULL");
+    lmoe_status st;
+    if ((st = lmoe_id_shape_check(gate, x, t, 1, k, ids, t_ids, top_k, out)) || (st = lmoe_id_shape_check(up, x, t, 1, k, ids, t_ids, top_k, out)) ||
+        (st = lmoe_id_shape_check(down, x, t, top_k, gate->n_out, ids, t_ids, top_k, out)) || (st = lmoe_combine_check(t, top_k, down->n_out)))
+        return st;
+    if (gate->n_out != up->n_out || gate->n_expert != up->n_expert || gate->n_expert != down->n_expert)
+        return lmoe_fail(LMOE_ERR_INVALID, "the stacks disagree: gate %lld x %lld, up %lld x %lld, down %lld experts", (long long)gate->n_expert,
+                         (long long)gate->n_out, (long long)up->n_expert, (long long)up->n_out, (long long)down->n_expert);
+    for (const lmoe_expert_stack *e : {gate, up, down})
+        if (!mm_id_kernel_available(e->dtype, e->n_out, e->k))
+            return lmoe_fail(LMOE_ERR_UNSUPPORTED, "no grouped-GEMM kernel for dtype %d, n_out %lld, k %lld", e->dtype, (long long)e->n_out,
+                             (long long)e->k);
+    if (t * top_k > INT32_MAX / 2 || t * top_k * gate->n_out > INT32_MAX)
+        return lmoe_fail(LMOE_ERR_INVALID, "silu_mul n (%lld) must be in [0, i32::MAX]", (long long)(t * top_k * gate->n_out));
+    if (gate->n_out > 48 * 1024 / 4) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "expert width %lld: call the ops one by one", (long long)gate->n_out);
+    const FfnMmLayout L(gate, down, t, top_k);
+    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255u) || workspace_bytes < L.total)
+        return lmoe_fail(LMOE_ERR_WORKSPACE, "ffn_mm workspace needs %zu bytes, 256-byte aligned, got %zu", L.total, workspace_bytes);
+    if (t == 0) return LMOE_OK;
+    uint8_t *ws = static_cast<uint8_t *>(workspace);
+    uint32_t *flag = reinterpret_cast<uint32_t *>(ws), *tpe = reinterpret_cast<uint32_t *>(ws + L.map0);
+    int32_t *ids_map = reinterpret_cast<int32_t *>(ws + L.map0 + gate->n_expert * 4), *pos = reinterpret_cast<int32_t *>(ws + L.pos);
+    float *g = reinterpret_cast<float *>(ws + L.g), *u = reinterpret_cast<float *>(ws + L.u), *l2 = reinterpret_cast<float *>(ws + L.l2);
+    float *d = reinterpret_cast<float *>(ws + L.d);
+    LMOE_CUDA(cudaMemsetAsync(flag, 0, 16, s));
+    LMOE_CUDA(cudaMemsetAsync(pos, 0xFF, (size_t)L.R.rows * 4, s)); // an id that names no expert
+    LMOE_CUDA(launch_map0(ids, (int)t, (int)top_k, (int)gate->n_expert, tpe, ids_map, s));
+    if ((st = launch_gather_tiles(L.R, x, 0, 1, (int)top_k, (int)k, tpe, ids_map, t, ws + L.tiles, ws + L.xt, pos, nullptr, nullptr, s))) return st;
+    if ((st = launch_mm_id(L.R, gate, nullptr, ws + L.xt, ids_map, t, nullptr, g, 0, ws + L.tiles, flag, s))) return st;
+    if ((st = launch_mm_id(L.R, up, nullptr, ws + L.xt, ids_map, t, nullptr, u, 0, ws + L.tiles, flag, s))) return st;
+    LMOE_CUDA(launch_silu_rescale_tiles(g, u, pos, L.R.rows, (int)gate->n_out, L.R.nt, ws + L.act, l2, d, (int)down->n_out, s));
+    if ((st = launch_mm_id(L.R, down, nullptr, ws + L.act, ids_map, t, nullptr, d, 0, ws + L.tiles, flag, s))) return st;
+    LMOE_CUDA(launch_combine(d, l2, weights, (int)t, (int)top_k, (int)down->n_out, out, s));
+    return LMOE_OK;
+}
+
 // ---- expert-parallel pieces -------------------------------------------------------------
 // (the same entries serve the shared expert alone, whose single list may take another tile size)
 static size_t rows_ffn_bytes(const lmoe_layer *L, int64_t rows) {

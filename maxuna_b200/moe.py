@@ -55,6 +55,8 @@ class FusedExperts(ExpertFfn):
         w = weights if weights.dtype == torch.float32 else weights.to(torch.float32)
         if not self.uses_mm(seq, top_k, use_mm):
             return ops.ffn_mv((self.gate, self.up, self.down), ids, w, None, x)
+        if self.gate.n_out <= ops.FFN_MM_MAX_FF:
+            return ops.ffn_mm((self.gate, self.up, self.down), ids, w, x)
         map0 = ops.prepare_map0(self.gate.n_expert, ids)
         x_g = x.view(seq, 1, hidden)
         gate = ops.mul_mm_id_shared(self.gate, x_g, ids, map0)

@@ -195,6 +195,29 @@ def ffn_mv(experts, ids, weights, shared, x: torch.Tensor) -> torch.Tensor:
     return out
 
 
+FFN_MM_MAX_FF = 12288  # expert width up to which `lmoe_ffn_mm` takes the chain
+
+
+def ffn_mm(experts, ids, weights, x: torch.Tensor) -> torch.Tensor:
+    """The grouped-GEMM op chain of the routed experts in one call (`lmoe_ffn_mm`), bit for bit what the ops give one by one:
+    experts (gate, up, down), ids and f32 weights ``[t, top_k]``, x ``[t, k]`` -> ``[t, n_out]``."""
+    _f32_dev("x", x)
+    _require(x.dim() == 2, "x must be rank-2 [t, k]")
+    t, k = x.shape
+    _ids_dev(ids)
+    t_ids, top_k = ids.shape
+    _f32_dev("weights", weights)
+    if weights.shape != (t, top_k):
+        raise LmoeError(-1, f"weights shape {tuple(weights.shape)} must be [seq, top_k] = [{t}, {top_k}]")
+    gate, up, down = experts
+    out = x.new_empty((t, down.n_out))
+    n = lib().lmoe_ffn_mm_workspace_bytes(gate.handle, down.handle, t, top_k)
+    ws = torch.empty(max(n, 16), dtype=torch.uint8, device=x.device)
+    check(lib().lmoe_ffn_mm(gate.handle, up.handle, down.handle, ids.data_ptr(), t_ids, top_k, weights.data_ptr(), x.data_ptr(), t, k,
+                            out.data_ptr(), ws.data_ptr(), n, stream_ptr()))
+    return out
+
+
 def combine(down: torch.Tensor, col_l2, weights: torch.Tensor) -> torch.Tensor:
     _f32_dev("down", down)
     _require(down.dim() == 3, "down must be rank-3 [seq, top_k, n_out]")

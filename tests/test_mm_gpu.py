@@ -157,3 +157,28 @@ def test_prefill_block_production_shape(orc, dev):
     host = blk.host_layer(orc)
     x = np.random.default_rng(23).standard_normal((48, 3072)).astype(np.float32)
     _check_block(orc, blk, host, x, 2e-3)
+
+
+@pytest.mark.parametrize("hidden,ff,ne,top_k,up_dt,t", [(256, 256, 4, 2, 12, 7), (512, 1536, 8, 3, 12, 100), (1024, 768, 16, 4, 14, 333),
+                                                        (256, 2048, 3, 2, 12, 300)])
+def test_ffn_mm_equals_the_ops(dev, hidden, ff, ne, top_k, up_dt, t):
+    """One call for the grouped-GEMM chain gives the bits of its ops one by one: both tile widths, rows of one to eight blocks,
+    widths that take eight and fewer warps a block, and an id that names no expert (which counts nothing here)."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    mk = lambda dt, o, k, s: ExpertStack.random(dt, ne, o, k, seed=s, device=dev)
+    e = (mk(12, ff, hidden, 1), mk(up_dt, ff, hidden, 2), mk(14, hidden, ff, 3))
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(t)
+    x = torch.randn(t, hidden, generator=gen, device=dev)
+    x[t // 2] *= 1e4
+    ids = torch.stack([torch.randperm(ne, generator=gen, device=dev)[:top_k] for _ in range(t)]).to(torch.int32)
+    w = torch.rand(t, top_k, generator=gen, device=dev)
+    m, xg = ops.prepare_map0(ne, ids), x.view(t, 1, hidden)
+    act, l2 = ops.l2_rescale(ops.silu_mul(ops.mul_mm_id_shared(e[0], xg, ids, m), ops.mul_mm_id_shared(e[1], xg, ids, m)))
+    want = ops.combine(ops.mul_mm_id_shared(e[2], act, ids, m), l2, w)
+    assert torch.equal(ops.ffn_mm(e, ids, w, x).view(torch.int32), want.view(torch.int32))
+    ids[0, 0] = ne + 1
+    got = ops.ffn_mm(e, ids, w, x)
+    assert torch.isfinite(got).all() and torch.equal(got[1:], want[1:])
