@@ -133,7 +133,7 @@ struct MvJob {
 };
 // Products of the same type, row count and k that do not depend on one another.
 cudaError_t launch_mul_mv_id_jobs(int dtype, const MvJob *job, int jobs, int n_out, int k, cudaStream_t s);
-// silu_mul and l2_rescale of rows of n values (a multiple of 256, at most 12288), straight into the grouped GEMM's tile order as f16
+// silu_mul and l2_rescale of rows of n values (a multiple of 256, at most LMOE_FFN_MM_MAX_FF), straight into the grouped GEMM's tile order as f16
 // (row of the tile order pos[row], tiles of nt rows); a row that no list names (pos < 0) is a zero row of y instead.
 cudaError_t launch_silu_rescale_tiles(const float *g, const float *u, const int32_t *pos, int64_t rows, int n, int nt, void *act, float *l2,
                                       float *y, int n_y, cudaStream_t s);

@@ -54,49 +54,71 @@ __global__ void __launch_bounds__(256) l2_rescale_kernel(const float *__restrict
     if (lane == 0) l2[row] = norm;
 }
 
-// Both steps at once, a warp a row: the bits of silu_mul_kernel and l2_rescale_kernel, rounded to f16 as gather_tiles_kernel
-// does.  The activations stay in shared memory between the two passes instead of going through memory three times (5120 x 1024
-// values, with a cold cache: 12 + 16 + 11 us in three kernels).
-__global__ void __launch_bounds__(256) silu_rescale_tiles_kernel(const float *__restrict__ g, const float *__restrict__ u,
-                                                                 const int32_t *__restrict__ pos, int64_t rows, int n, int nt,
-                                                                 uint8_t *__restrict__ act, float *__restrict__ l2, float *__restrict__ y, int n_y) {
-    pdl_begin();
-    extern __shared__ __align__(16) float sr_rows[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-    if (row >= rows) return;
-    const int p = pos[row];
-    if (p < 0) {
-        for (int i = lane; i < n_y; i += 32) y[row * n_y + i] = 0.f;
-        if (lane == 0) l2[row] = 1.0f;
-        return;
-    }
-    const float *gr = g + row * n, *ur = u + row * n;
-    float *a = sr_rows + (size_t)warp * n;
-    float ss = 0.f;
-#pragma unroll 4
-    for (int i = lane; i < n; i += 32) {
-        const float v = silu_mul(__ldg(gr + i), __ldg(ur + i));
-        a[i] = v;
-        ss = __fmaf_rn(v, v, ss);
-    }
+// Eight values of a row -> their place in the tile order, divided by the row's norm and rounded to f16 as gather_tiles_kernel does.
+__device__ __forceinline__ void rescale_chunk(const float *a, int ci, float norm, int p, int n, int nt, uint8_t *__restrict__ act) {
+    const float4 b = *reinterpret_cast<const float4 *>(a + ci * 8), c = *reinterpret_cast<const float4 *>(a + ci * 8 + 4);
+    const float v[8] = {b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+    float q[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) q[j] = __fdiv_rn(__fmul_rn(v[j], 32768.0f), norm);
+    __align__(16) __half2 h[4] = {__floats2half2_rn(q[0], q[2]), __floats2half2_rn(q[1], q[3]), __floats2half2_rn(q[4], q[6]),
+                                  __floats2half2_rn(q[5], q[7])};
+    const size_t off = (((size_t)(p / nt) * (n / 64) + (ci >> 3)) * nt + (p % nt)) * 128 + ((size_t)((ci & 7) ^ (p & 7)) << 4);
+    *reinterpret_cast<uint4 *>(act + off) = *reinterpret_cast<const uint4 *>(h);
+}
+__device__ __forceinline__ float row_norm(float ss) { // of a lane's share of the squares
 #pragma unroll
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float norm = isnan(ss) ? ss : fminf(fmaxf(sqrtf(ss), 1e-8f), 1e30f);
-    __syncwarp();
-    for (int i = lane * 8; i < n; i += 256) {
-        const float4 b = *reinterpret_cast<const float4 *>(a + i), c = *reinterpret_cast<const float4 *>(a + i + 4);
+    return isnan(ss) ? ss : fminf(fmaxf(sqrtf(ss), 1e-8f), 1e30f);
+}
+
+// Both steps at once, a block a row: the bits of silu_mul_kernel and l2_rescale_kernel.  The activations stay in shared memory
+// between the two passes instead of going through memory three times (5120 x 1024 values, with a cold cache: 12 + 16 + 11 us in
+// three kernels, 25 here).  Bound by memory from rows of 4096 on; below, by the chain load, sum, divide of a block.  The squares are
+// summed by one warp, in l2_rescale_kernel's order.  (A warp a row left the wide rows few loads in flight, as a warp's row stays
+// in shared memory: 5120 rows of 256 / 1024 / 4096 / 12288 values 14 / 33 / 237 / 2006 us, a block a row 12 / 25 / 61 / 177.)
+__global__ void __launch_bounds__(256) silu_rescale_tiles_kernel(const float *__restrict__ g, const float *__restrict__ u,
+                                                                 const int32_t *__restrict__ pos, int n, int nt, uint8_t *__restrict__ act,
+                                                                 float *__restrict__ l2, float *__restrict__ y, int n_y) {
+    pdl_begin();
+    extern __shared__ __align__(16) float sr_row[];
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    const int64_t row = blockIdx.x;
+    const int p = pos[row];
+    if (p < 0) {
+        for (int i = tid; i < n_y; i += nthr) y[row * n_y + i] = 0.f;
+        if (tid == 0) l2[row] = 1.0f;
+        return;
+    }
+    const float4 *gr = reinterpret_cast<const float4 *>(g + row * n), *ur = reinterpret_cast<const float4 *>(u + row * n);
+#pragma unroll 2
+    for (int i = tid; i < n / 4; i += nthr) {
+        const float4 b = __ldg(gr + i), c = __ldg(ur + i);
+        reinterpret_cast<float4 *>(sr_row)[i] = make_float4(silu_mul(b.x, c.x), silu_mul(b.y, c.y), silu_mul(b.z, c.z), silu_mul(b.w, c.w));
+    }
+    __syncthreads();
+    if (tid < 32) {
+        float ss = 0.f;
+#pragma unroll 8
+        for (int i = tid; i < n; i += 32) ss = __fmaf_rn(sr_row[i], sr_row[i], ss);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (tid == 0) l2[row] = isnan(ss) ? ss : fminf(fmaxf(sqrtf(ss), 1e-8f), 1e30f);
+    }
+    __syncthreads();
+    const float norm = l2[row]; // (shared memory may be the row's to the last byte)
+    for (int ci = tid; ci < n / 8; ci += nthr) {
+        const float4 b = *reinterpret_cast<const float4 *>(sr_row + ci * 8), c = *reinterpret_cast<const float4 *>(sr_row + ci * 8 + 4);
         const float v[8] = {b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
         float q[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) q[j] = __fdiv_rn(__fmul_rn(v[j], 32768.0f), norm);
+        // rounded to f16 as gather_tiles_kernel does
         __align__(16) __half2 h[4] = {__floats2half2_rn(q[0], q[2]), __floats2half2_rn(q[1], q[3]), __floats2half2_rn(q[4], q[6]),
                                       __floats2half2_rn(q[5], q[7])};
-        const int ci = i >> 3;
         const size_t off = (((size_t)(p / nt) * (n / 64) + (ci >> 3)) * nt + (p % nt)) * 128 + ((size_t)((ci & 7) ^ (p & 7)) << 4);
         *reinterpret_cast<uint4 *>(act + off) = *reinterpret_cast<const uint4 *>(h);
     }
-    if (lane == 0) l2[row] = norm;
 }
 
 __global__ void add_inplace_kernel(float *__restrict__ out, const float *__restrict__ b, int64_t n) {
@@ -281,11 +303,9 @@ cudaError_t launch_silu_mul(const float *g, const float *u, int64_t n, float *ou
 cudaError_t launch_silu_rescale_tiles(const float *g, const float *u, const int32_t *pos, int64_t rows, int n, int nt, void *act, float *l2,
                                       float *y, int n_y, cudaStream_t s) {
     if (rows == 0) return cudaSuccess;
-    int warps = 48 * 1024 / (4 * n); // whole rows in the shared memory that needs no opt-in
-    warps = warps > 8 ? 8 : warps;
-    if (warps < 1) return cudaErrorInvalidValue;
-    launch_pdl(silu_rescale_tiles_kernel, (unsigned)((rows + warps - 1) / warps), 32 * warps, (size_t)warps * n * 4, s, g, u, pos, rows, n, nt,
-               static_cast<uint8_t *>(act), l2, y, n_y);
+    if (n > LMOE_FFN_MM_MAX_FF) return cudaErrorInvalidValue; // a row in the shared memory that needs no opt-in
+    launch_pdl(silu_rescale_tiles_kernel, (unsigned)rows, n < 1024 ? n / 4 : 256, (size_t)n * 4, s, g, u, pos, n, nt, static_cast<uint8_t *>(act),
+               l2, y, n_y);
     return cudaGetLastError();
 }
 

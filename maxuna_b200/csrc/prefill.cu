@@ -560,7 +560,7 @@ extern "C" lmoe_status lmoe_ffn_mm(const lmoe_expert_stack *gate, const lmoe_exp
                              (long long)e->k);
     if (t * top_k > INT32_MAX / 2 || t * top_k * gate->n_out > INT32_MAX)
         return lmoe_fail(LMOE_ERR_INVALID, "silu_mul n (%lld) must be in [0, i32::MAX]", (long long)(t * top_k * gate->n_out));
-    if (gate->n_out > 48 * 1024 / 4) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "expert width %lld: call the ops one by one", (long long)gate->n_out);
+    if (gate->n_out > LMOE_FFN_MM_MAX_FF) return lmoe_fail(LMOE_ERR_UNSUPPORTED, "expert width %lld: call the ops one by one", (long long)gate->n_out);
     const FfnMmLayout L(gate, down, t, top_k);
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255u) || workspace_bytes < L.total)
         return lmoe_fail(LMOE_ERR_WORKSPACE, "ffn_mm workspace needs %zu bytes, 256-byte aligned, got %zu", L.total, workspace_bytes);

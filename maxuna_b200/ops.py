@@ -195,7 +195,7 @@ def ffn_mv(experts, ids, weights, shared, x: torch.Tensor) -> torch.Tensor:
     return out
 
 
-FFN_MM_MAX_FF = 12288  # expert width up to which `lmoe_ffn_mm` takes the chain
+FFN_MM_MAX_FF = 12288  # LMOE_FFN_MM_MAX_FF: expert width up to which `lmoe_ffn_mm` takes the chain
 
 
 def ffn_mm(experts, ids, weights, x: torch.Tensor) -> torch.Tensor:

@@ -27,6 +27,13 @@ def test_header_symbols_exported():
     assert b"sm_100a" in lib.lmoe_version()
 
 
+def test_ffn_mm_width_limit_is_the_headers():
+    from maxuna_b200 import ops
+
+    text = open(os.path.join(ROOT, "include", "lmoe.h")).read()
+    assert ops.FFN_MM_MAX_FF == int(re.search(r"#define LMOE_FFN_MM_MAX_FF (\d+)", text).group(1))
+
+
 def test_argument_errors_without_cuda():
     from maxuna_b200 import _native
 

@@ -182,3 +182,27 @@ def test_ffn_mm_equals_the_ops(dev, hidden, ff, ne, top_k, up_dt, t):
     ids[0, 0] = ne + 1
     got = ops.ffn_mm(e, ids, w, x)
     assert torch.isfinite(got).all() and torch.equal(got[1:], want[1:])
+
+
+@pytest.mark.parametrize("ff", [256, 768, 1024, 1792, 4096, 12288])
+def test_ffn_mm_wide_rows(dev, ff):
+    """Activation rows from one warp pair a block to the widest that fits, whole and broken turns of its threads: the bits of the
+    ops one by one, and a slot whose id names no expert is a zero row."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    ne, t, top_k, hidden = 3, 70, 2, 256
+    mk = lambda dt, o, k, s: ExpertStack.random(dt, ne, o, k, seed=s, device=dev)
+    e = (mk(12, ff, hidden, 1), mk(12, ff, hidden, 2), mk(14, hidden, ff, 3))
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(ff)
+    x = torch.randn(t, hidden, generator=gen, device=dev)
+    ids = torch.stack([torch.randperm(ne, generator=gen, device=dev)[:top_k] for _ in range(t)]).to(torch.int32)
+    ids[5, 1] = ne
+    w = torch.rand(t, top_k, generator=gen, device=dev)
+    m, xg = ops.prepare_map0(ne, ids), x.view(t, 1, hidden)
+    act, l2 = ops.l2_rescale(ops.silu_mul(ops.mul_mm_id_shared(e[0], xg, ids, m), ops.mul_mm_id_shared(e[1], xg, ids, m)))
+    down = ops.mul_mm_id_shared(e[2], act, ids, m)
+    down[5, 1], l2[5, 1] = 0.0, 1.0
+    want = ops.combine(down, l2, w)
+    assert torch.equal(ops.ffn_mm(e, ids, w, x).view(torch.int32), want.view(torch.int32))
