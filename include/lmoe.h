@@ -222,7 +222,8 @@ lmoe_status lmoe_ffn_mv(const lmoe_expert_stack *gate, const lmoe_expert_stack *
 /* The grouped-GEMM branch of `FusedExperts::forward`, src/moe.rs:236-323, as one call: prepare_map0, mul_mm_id (gate, up),
  * silu_mul, l2_rescale, mul_mm_id (down), combine, with the results of those ops called one by one and their errors; a
  * (token, slot) whose id names no expert counts nothing.  Expert widths up to LMOE_FFN_MM_MAX_FF.  Workspace:
- * lmoe_ffn_mm_workspace_bytes, 256-byte aligned, contents undefined before and after. */
+ * lmoe_ffn_mm_workspace_bytes, 256-byte aligned, contents undefined before; its first bytes hold the call's device flag after it
+ * (lmoe_check_device_flag), and `out` is NaN where a product's bounded wait ran out. */
 #define LMOE_FFN_MM_MAX_FF 12288 /* an f32 row in 48 KB of shared memory */
 size_t lmoe_ffn_mm_workspace_bytes(const lmoe_expert_stack *gate, const lmoe_expert_stack *down, int64_t t, int64_t top_k);
 lmoe_status lmoe_ffn_mm(const lmoe_expert_stack *gate, const lmoe_expert_stack *up, const lmoe_expert_stack *down,

@@ -140,7 +140,7 @@ cudaError_t launch_silu_rescale_tiles(const float *g, const float *u, const int3
 cudaError_t launch_silu_mul(const float *g, const float *u, int64_t n, float *out, cudaStream_t s);
 cudaError_t launch_l2_rescale(const float *a, int64_t rows, int n, float *out, float *l2, cudaStream_t s);
 cudaError_t launch_combine(const float *down, const float *col_l2, const float *w, int seq, int top_k,
-                           int n_out, float *out, cudaStream_t s);
+                           int n_out, float *out, cudaStream_t s, const uint32_t *flag = nullptr);
 cudaError_t launch_add_inplace(float *out, const float *b, int64_t n, cudaStream_t s);
 cudaError_t launch_ep_localize_ids(const uint32_t *ids, int64_t n, uint32_t first, uint32_t count, uint32_t *out,
                                    cudaStream_t s);

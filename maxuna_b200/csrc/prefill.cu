@@ -578,7 +578,7 @@ extern "C" lmoe_status lmoe_ffn_mm(const lmoe_expert_stack *gate, const lmoe_exp
     if ((st = launch_mm_id(L.R, up, nullptr, ws + L.xt, ids_map, t, nullptr, u, 0, ws + L.tiles, flag, s))) return st;
     LMOE_CUDA(launch_silu_rescale_tiles(g, u, pos, L.R.rows, (int)gate->n_out, L.R.nt, ws + L.act, l2, d, (int)down->n_out, s));
     if ((st = launch_mm_id(L.R, down, nullptr, ws + L.act, ids_map, t, nullptr, d, 0, ws + L.tiles, flag, s))) return st;
-    LMOE_CUDA(launch_combine(d, l2, weights, (int)t, (int)top_k, (int)down->n_out, out, s));
+    LMOE_CUDA(launch_combine(d, l2, weights, (int)t, (int)top_k, (int)down->n_out, out, s, flag));
     return LMOE_OK;
 }
 

@@ -206,3 +206,22 @@ def test_ffn_mm_wide_rows(dev, ff):
     down[5, 1], l2[5, 1] = 0.0, 1.0
     want = ops.combine(down, l2, w)
     assert torch.equal(ops.ffn_mm(e, ids, w, x).view(torch.int32), want.view(torch.int32))
+
+
+def test_combine_after_a_wait_that_ran_out(dev):
+    """The sum that ends `lmoe_ffn_mm` on products whose device flag is set: NaN, not a wrong finite row; on a clean flag the sum."""
+    import ctypes as C
+
+    from maxuna_b200 import ops
+    from maxuna_b200._native import lib
+    from maxuna_b200.gguf import stream_ptr
+
+    # launch_combine(down, col_l2, w, seq, top_k, n_out, out, stream, flag) of csrc/glue.cu
+    f = lib()._Z14launch_combinePKfS0_S0_iiiPfP11CUstream_stPKj
+    f.argtypes = [C.c_void_p] * 3 + [C.c_int] * 3 + [C.c_void_p] * 3
+    for n_out in (64, 65):  # four columns a thread, and one
+        down, w = torch.randn(5, 3, n_out, device=dev), torch.rand(5, 3, device=dev)
+        for flag in (0, 2):
+            word, out = torch.tensor([flag, 0, 0, 0], dtype=torch.int32, device=dev), torch.zeros(5, n_out, device=dev)
+            assert f(down.data_ptr(), None, w.data_ptr(), 5, 3, n_out, out.data_ptr(), stream_ptr(), word.data_ptr()) == 0
+            assert torch.isnan(out).all() if flag else torch.equal(out, ops.combine(down, None, w))
