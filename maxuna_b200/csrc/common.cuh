@@ -30,8 +30,9 @@ void lmoe_clear_error();
 // kernel begins with pdl_begin(): it waits until the kernel before it is complete and visible, and only then lets the one
 // after it start, so that never more than two overlap.  Where there is nothing to wait for the two instructions do nothing.
 // (70 tokens: 374 -> 364 us, 200: 446 -> 432; 130 tokens of a layer with 128 experts of 768: 181 -> 167; op by op, 3 tokens:
-// 134 -> 118.)  The grouped products and the two kernels that stream their results are launched the plain way: overlapping
-// those cost 2 to 4 % from 2048 tokens on.
+// 134 -> 118.)  The grouped products set up their barriers and tensor memory before they wait, and do not let the next kernel
+// start early.  The two kernels that stream their results and the warp-per-row mat-vec are launched the plain way: overlapping
+// those cost 2 to 4 % from 2048 tokens on, and up to half as much again.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");

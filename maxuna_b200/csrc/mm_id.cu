@@ -1189,9 +1189,11 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = stream;
     cfg.attrs = attr;
-    // With thin tiles the launch (barriers, tensor memory, the pair's meeting) overlaps the end of the kernel before: 70 to 600 tokens
-    // on 64 to 256 experts 3 to 5 us less of 95 to 640.  From 2048 tokens on that cost 2 to 4 %.
-    cfg.numAttrs = NT == 128 ? 2 : 1;
+    // The launch (barriers, tensor memory, the pair's meeting) overlaps the end of the kernel before.  Plain against so, a layer of 8
+    // experts of 256, 400 / 1228 / 3000 tokens: 61.7 / 69.9 / 96.5 us, 56.3 / 67.6 / 92.2; 64 of 512, 640 / 3000 tokens: 127 / 305,
+    // 122 / 299; a single product of 8 experts [3072 x 1024], 256 tokens: 24.7, 22.7.  From 2048 tokens of the large layers on the two
+    // differ by less than two runs of one of them.
+    cfg.numAttrs = 2;
     static thread_local int c_dev = -1, c_grid = 0;
     int dev = 0;
     LMOE_CUDA(cudaGetDevice(&dev));
