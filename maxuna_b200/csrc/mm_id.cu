@@ -6,7 +6,7 @@
 // tiles, f32 accumulation); per-expert lists from map0, src/ops/mm_id.metal:207-269.
 //
 // Persistent pairs of CTAs, one CTA per SM, warp-specialised around tcgen05.mma; see grouped_mm_kernel.  The weight tile is the
-// A operand (M = 128 output features) and the routed rows are the N dimension, so ragged per-expert row counts cost
+// A operand (M = 256 output features, 128 in each CTA) and the routed rows are the N dimension, so ragged per-expert row counts cost
 // only a rounding to 16.  Every wait is bounded; a wait that runs out records a flag and the kernel drains and exits.
 #include <cuda.h> // CUtensorMap (types only; the encoder is fetched through the runtime)
 
@@ -16,6 +16,7 @@
 namespace {
 
 constexpr int MM_M = 128;      // weight rows per CTA; a pair's tile has twice as many
+// CG below: the CTAs that share a tile, 2 (a pair) or 1
 constexpr int MM_K = 64;       // k per pipeline stage (one 128-byte swizzle row of f16)
 constexpr int MM_WAIT_HINT_NS = 1000, MM_WAIT_TRIES = 1 << 22;
 
@@ -50,8 +51,11 @@ __device__ __forceinline__ bool mb_test(uint64_t *b, uint32_t parity) {
                  : "=r"(ok) : "r"(s32(b)), "r"(parity) : "memory");
     return ok != 0;
 }
-// Arrival at a barrier of the pair's first CTA.
+// Arrival at a barrier of the pair's first CTA.  Of the default scope: it may announce what lies in tensor memory, behind the tcgen05
+// fence, or in this CTA's own shared memory, behind a proxy fence or a bulk copy's completion; nothing else that the other CTA reads.
+template <int CG>
 __device__ __forceinline__ void mb_arrive_first(uint64_t *b) {
+    if (CG == 1) return mb_arrive(b);
     asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\t"
                  "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(s32(b)) : "memory");
 }
@@ -75,17 +79,26 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // Arrives, once the multiplies issued so far are done, at the barrier at this place in both CTAs of the pair.
+template <int CG>
 __device__ __forceinline__ void tc_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(s32(bar)),
+    if (CG == 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(bar)) : "memory");
+    else asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(s32(bar)),
                  "h"((uint16_t)3) : "memory");
 }
 // D += A * B for both CTAs of a pair; the A operand lies in tensor memory, in each CTA its own 128 lanes (weight rows) x 8 columns
 // (K = 16 as f16 pairs), and each CTA's shared memory holds half of B's rows at the place the descriptor names.
+template <int CG>
 __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc),
-        "r"(accum) : "memory");
+    if (CG == 1)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc),
+            "r"(accum) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc),
+            "r"(accum) : "memory");
 }
 // 32 registers of every lane -> 32 columns of the warp's 32 tensor-memory lanes; complete after tc_wait_st().
 __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -160,7 +173,7 @@ __device__ __forceinline__ uint32_t h2_sub_mul(uint32_t v, uint32_t base, uint32
 // is the same for any height, so a full tile and a thin one cost more than two even ones (256 experts, 8192 tokens 2383 us
 // with full tiles and a rest, 2348 so; Zipf, 6000 tokens 1935 and 1888).  tiles[i] = {expert, first list index,
 // valid rows, first row in expert-sorted order}; i is also the slot of the tile in the tile-ordered operands.  A GEMM tile is (row
-// tile, block of 256 weight rows), the latter varying fastest, so CTAs running side by side share the same activation rows in L2.
+// tile, block of CG x 128 weight rows), the latter varying fastest, so CTAs running side by side share the same activation rows in L2.
 // With `extra` > 0 one more list follows the experts' ("expert" n_expert): the rows 0 .. extra-1 of the shared expert.
 // The tiles stand by falling height: the CTAs take the tiles of a product in turn, so each round has tiles of one cost and the
 // last, incomplete one the cheapest (experts' order left the SMs idle for 13 % of the gate/up product of 2048 tokens; the whole
@@ -357,8 +370,8 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict_
 // so the dequantised tile never passes through shared memory.  A thread converts its next stage's weights BEFORE it
 // waits for the stage to be free, so the wait covers only the store.
 //
-// Two CTAs on neighbouring SMs share a tile (cta_group::2): each converts 128 of its 256 weight rows and keeps their accumulators,
-// and each loads half of the tile's activation rows, which the tensor cores of both read.  One SM alone loads 24 KB of
+// Two CTAs on neighbouring SMs share a tile (CG = 2, cta_group::2; with CG = 1 a CTA has a tile of 128 weight rows for itself): each
+// converts 128 of its 256 weight rows and keeps their accumulators, and each loads half of the tile's activation rows, which the tensor cores of both read.  One SM alone loads 24 KB of
 // activations for 768 cycles of multiplies in gate/up, 48 KB in down, and with the weights that is more than the L2 cache hands
 // out: down of 8192 tokens took the same 990 thousand cycles without its conversions or with 16-column multiplies.  The first CTA's
 // warp 0 issues for both; whatever it waits for is signalled at its barriers by both CTAs, and its commits arrive in both.  (What is
@@ -389,19 +402,19 @@ __device__ __forceinline__ int gm_q6_line(int r, int lg) { return ((r & ((1 << l
 constexpr int GM_EPI_BYTES = 1024; // one epilogue warp's staging: 8 tile columns (output rows) x 32 weight rows, f32
 constexpr int GM_BOX_ROWS = 16;    // single projection: tile stores of 16 output rows x 32 weight rows, two in flight per warp
 
-template <int DT, int NPROJ, int NT>
+template <int DT, int NPROJ, int NT, int CG>
 struct GmCfg {
     // one 256-wide column of quantized blocks of all the tile's weight rows
     static constexpr int RAW_SLOT = NPROJ * MM_M * (DT == LMOE_Q4_K ? Q4K_BYTES : GM_Q6_PITCH);
     static constexpr int RAW_SLOTS = DT == LMOE_Q4_K && NPROJ == 1 ? 4 : 3;
     static constexpr int EPI_BYTES = NPROJ == 2 ? GM_EPI_BYTES : 2 * GM_BOX_ROWS * 128;
-    static constexpr int B_ROWS = NT / 2;
+    static constexpr int B_ROWS = NT / CG;
     static constexpr int B_BLK = B_ROWS * MM_K * 2;     // a CTA's half of a 64-k block of the B operand
-    static constexpr int B_SLOT = NPROJ == 2 ? B_BLK : 2 * B_BLK; // ring slot: as much as an operand stage multiplies
+    static constexpr int B_SLOT = NPROJ == 2 || CG == 1 ? B_BLK : 2 * B_BLK; // ring slot: as much as an operand stage multiplies (a CTA alone: half of that)
     static constexpr int NB = 96 * 1024 / B_SLOT < 8 ? 96 * 1024 / B_SLOT : 8;
     static constexpr int NA = (512 - 2 * NT) / 64 >= 4 ? 4 : 2, A_COL0 = 2 * NT;
     static constexpr int EPI_WARPS = NPROJ == 2 ? GM_DQ_WARPS : 4;
-    static constexpr int B_ARRIVALS = NPROJ == 2 ? 8 : 1; // per ring slot (the first CTA's of a single projection: one more, see the relay)
+    static constexpr int B_ARRIVALS = NPROJ == 2 ? 4 * CG : 1; // per ring slot (the first CTA's of a single projection: one more, see the relay)
     static constexpr int O_RAW = NB * B_SLOT, O_EPI = O_RAW + RAW_SLOTS * RAW_SLOT, O_BAR = O_EPI + EPI_WARPS * EPI_BYTES;
     static constexpr int SMEM = O_BAR + 512 + 1024; // barriers, slack to align the base to 1024 bytes
     static_assert(A_COL0 + 64 * NA <= 512, "tensor memory");
@@ -416,7 +429,7 @@ struct GmParams {
     CUtensorMap map_out;     // NPROJ = 1, sorted rows: `out` as [rows][n_out] f32, box = 32 values x 16 rows
     int lines, lg;           // Q6_K: the views exist; lg
     const uint8_t *w[2];     // Q6_K without them: stack blocks, shared expert's blocks
-    int n_expert, m_tiles;   // list number of the shared expert; blocks of 256 weight rows
+    int n_expert, m_tiles;   // list number of the shared expert; blocks of CG x 128 weight rows
     int64_t expert_bytes;
     int n_out, k;
     const uint8_t *xt;       // NPROJ = 1: f16 activations in tile order (see gather_tiles_kernel); 2: in token order
@@ -545,23 +558,28 @@ struct GmTile {
     int e, sh; // expert; 1 for the shared expert (then e is 0)
     int l0, nv, m0, slot, srow;
 };
+template <int CG>
 __device__ __forceinline__ GmTile gm_tile(const GmParams &P, int tile, int n_tiles, int rank) {
     GmTile T = {0, 0, 0, 0, 0, 0, 0};
     if (tile < n_tiles) {
         const int slot = tile / P.m_tiles;
         const int4 a = __ldg(P.tiles + slot);
         const int sh = a.x == P.n_expert;
-        T = {sh ? 0 : a.x, sh, a.y, a.z, (tile - slot * P.m_tiles) * (2 * MM_M) + rank * MM_M, slot, a.w};
+        T = {sh ? 0 : a.x, sh, a.y, a.z, (tile - slot * P.m_tiles) * (CG * MM_M) + rank * MM_M, slot, a.w};
     }
     return T;
 }
 // 64-k blocks of the B operand that share one ring slot: a thin tile's blocks do not fill it, and a deeper ring is what
 // hides the copies' latency there.
-template <int NPROJ, int NT>
-__device__ __forceinline__ int gm_b_group(int nv) { return nv > NT / 2 ? (NPROJ == 2 ? 1 : 2) : (NPROJ == 2 && nv > NT / 4 ? 2 : 4); }
+template <int NPROJ, int NT, int CG>
+__device__ __forceinline__ int gm_b_group(int nv) {
+    constexpr bool one = NPROJ == 2 || CG == 1; // a slot holds one block of a full tile, else two
+    return nv > NT / 2 ? (one ? 1 : 2) : (one && nv > NT / 4 ? 2 : 4);
+}
 
 // rows of a tile that each CTA of a pair holds of the B operand (of the padded tile: a multiple of 8)
-__device__ __forceinline__ int gm_half(int nv) { return ((nv + 15) & ~15) >> 1; }
+template <int CG>
+__device__ __forceinline__ int gm_half(int nv) { return ((nv + 15) & ~15) / CG; }
 __device__ __forceinline__ void pair_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -649,9 +667,9 @@ __device__ __forceinline__ void gm_epilogue(const GmParams &P, const GmTile &T, 
     }
 }
 
-template <int DT, int NPROJ, int NT>
+template <int DT, int NPROJ, int NT, int CG>
 __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_constant__ GmParams P) {
-    using C = GmCfg<DT, NPROJ, NT>;
+    using C = GmCfg<DT, NPROJ, NT, CG>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *b_st = smem, *raw = smem + C::O_RAW;
@@ -665,21 +683,21 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
     static_assert(C::NB <= 8 && C::RAW_SLOTS <= 4 && C::NA <= 4, "barrier table");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int rank = blockIdx.x & 1, tile0 = blockIdx.x >> 1, tile_step = gridDim.x >> 1; // place in the pair; the pair's tiles
+    const int rank = CG == 2 ? blockIdx.x & 1 : 0, tile0 = blockIdx.x / CG, tile_step = gridDim.x / CG; // place in the pair; the pair's tiles
     const int n_blk = P.k / QK_K, k_blocks = P.k / MM_K;
     const int row_bytes = n_blk * (DT == LMOE_Q4_K ? Q4K_BYTES : Q6K_BYTES);
 
     if (tid == 0) {
         for (int s = 0; s < C::NA; s++) {
-            mb_init(&a_full[s], GM_DQ_WARPS);
+            mb_init(&a_full[s], GM_DQ_WARPS / 2 * CG);
             mb_init(&a_empty[s], 1);
         }
         for (int s = 0; s < 2; s++) {
             mb_init(&acc_full[s], 1);
-            mb_init(&acc_empty[s], 2 * C::EPI_WARPS);
+            mb_init(&acc_empty[s], CG * C::EPI_WARPS);
         }
         for (int i = 0; i < C::NB; i++) {
-            mb_init(&b_full[i], C::B_ARRIVALS + (NPROJ == 1 && rank == 0 ? 1 : 0));
+            mb_init(&b_full[i], C::B_ARRIVALS + (NPROJ == 1 && CG == 2 && rank == 0 ? 1 : 0));
             mb_init(&b_empty[i], 1);
         }
         for (int i = 0; i < C::RAW_SLOTS; i++) {
@@ -689,12 +707,17 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        if (CG == 1) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
-    pair_sync(); // the other CTA's barriers are initialised
+    if (CG == 2) pair_sync(); // the other CTA's barriers are initialised
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     asm volatile("griddepcontrol.wait;" ::: "memory"); // what earlier kernels wrote is read from here on
@@ -724,7 +747,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mb_arrive_first(&a_full[C::NA == 4 ? 2 * i + grp : grp]);
+            if (lane == 0) mb_arrive_first<CG>(&a_full[C::NA == 4 ? 2 * i + grp : grp]);
             use++;
         };
         // single projection: the thread's part of one column, out of shared memory; then the slot goes back to the loader
@@ -767,11 +790,11 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             store(o, i);
             stored(i);
         };
-        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        GmTile T, next = gm_tile<CG>(P, tile0, n_tiles, rank);
         if (NPROJ == 2 && tile0 < n_tiles) half(0);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, it++) {
             T = next;
-            next = gm_tile(P, tile + tile_step, n_tiles, rank);
+            next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
             // (rows past the last one convert whatever the slot holds: their accumulator rows are never read)
             if (DT == LMOE_Q6_K) sh = (int)(((int64_t)T.e * P.expert_bytes + (int64_t)(T.m0 + r) * row_bytes) & 15);
             if (NPROJ == 1) {
@@ -805,17 +828,17 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                     tc_fence_before();
                 }
                 __syncwarp();
-                if (lane == 0) mb_arrive_first(&acc_empty[0]);
+                if (lane == 0) mb_arrive_first<CG>(&acc_empty[0]);
             }
         }
     } else if (warp == 2) {
         // ---------------- loader of the quantized columns ----------------
         const bool el = elect_one();
         uint32_t slot = 0, rph = 0;
-        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        GmTile T, next = gm_tile<CG>(P, tile0, n_tiles, rank);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             T = next;
-            next = gm_tile(P, tile + tile_step, n_tiles, rank);
+            next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
             const int vrows = max(0, min(MM_M, P.n_out - T.m0));
             for (int b = 0; b < n_blk && ok; b++) {
                 ok &= mb_wait(&raw_empty[slot], rph ^ 1);
@@ -857,12 +880,12 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         // ---------------- B loader: one bulk copy per 64-k block (the operand is stored in tile order) ----------------
         const bool el = elect_one();
         uint32_t slot = 0, ph = 0;
-        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        GmTile T, next = gm_tile<CG>(P, tile0, n_tiles, rank);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             T = next;
-            next = gm_tile(P, tile + tile_step, n_tiles, rank);
-            const int first = rank * gm_half(T.nv), brows = max(0, min(gm_half(T.nv), T.nv - first));
-            const uint32_t bytes = (uint32_t)brows * 128u, grp = (uint32_t)gm_b_group<NPROJ, NT>(T.nv), sub = C::B_SLOT / grp;
+            next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
+            const int first = rank * gm_half<CG>(T.nv), brows = max(0, min(gm_half<CG>(T.nv), T.nv - first));
+            const uint32_t bytes = (uint32_t)brows * 128u, grp = (uint32_t)gm_b_group<NPROJ, NT, CG>(T.nv), sub = C::B_SLOT / grp;
             const uint8_t *src = P.xt + ((size_t)T.slot * k_blocks * NT + first) * 128;
             for (int kb = 0; kb < k_blocks && ok; kb += (int)grp) {
                 ok &= mb_wait(&b_empty[slot], ph ^ 1);
@@ -875,18 +898,18 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                 if (++slot == C::NB) { slot = 0; ph ^= 1; }
             }
         }
-    } else if (NPROJ == 1 && warp == 0 && rank == 1) {
+    } else if (NPROJ == 1 && CG == 2 && warp == 0 && rank == 1) {
         // ---------------- relay: a bulk copy signals its own CTA only; the issuer is told that this half of a slot has landed ----------------
         uint32_t slot = 0, ph = 0;
-        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        GmTile T, next = gm_tile<CG>(P, tile0, n_tiles, rank);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             T = next;
-            next = gm_tile(P, tile + tile_step, n_tiles, rank);
-            const int grp = gm_b_group<NPROJ, NT>(T.nv);
+            next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
+            const int grp = gm_b_group<NPROJ, NT, CG>(T.nv);
             for (int kb = 0; kb < k_blocks && ok; kb += grp) {
                 ok &= mb_wait(&b_full[slot], ph);
                 __syncwarp();
-                if (lane == 0) mb_arrive_first(&b_full[slot]);
+                if (lane == 0) mb_arrive_first<CG>(&b_full[slot]);
                 if (++slot == C::NB) { slot = 0; ph ^= 1; }
             }
         }
@@ -899,13 +922,13 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         const uint64_t bd0 = umma_desc(s32(b_st));
         uint32_t it = 0, bs = 0, bph = 0, as = 0, aph = 0; // tiles; slot and phase of the B ring and of the operand stages
         bool b_here = false, a_here = false; // they were seen to be full
-        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        GmTile T, next = gm_tile<CG>(P, tile0, n_tiles, rank);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, it++) {
             T = next;
-            next = gm_tile(P, tile + tile_step, n_tiles, rank);
+            next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
             const int npad = (T.nv + 15) & ~15;
-            const uint32_t grp = (uint32_t)gm_b_group<NPROJ, NT>(T.nv), sub = (C::B_SLOT >> 4) / grp;
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(2 * MM_M >> 4) << 24);
+            const uint32_t grp = (uint32_t)gm_b_group<NPROJ, NT, CG>(T.nv), sub = (C::B_SLOT >> 4) / grp;
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(CG * MM_M >> 4) << 24);
             const uint32_t buf = NPROJ == 2 ? 0u : it & 1, cph = NPROJ == 2 ? it & 1 : (it >> 1) & 1;
             ok &= mb_wait(&acc_empty[buf], cph ^ 1);
             const uint32_t d = tmem_base + buf * NT;
@@ -934,16 +957,16 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
 #pragma unroll
                         for (int kk = 0; kk < 4; kk++) {
                             const uint32_t acc = (u | kk) != 0 ? 1u : (kb != 0 ? 1u : 0u);
-                            tc_mma_f16_ts(d, a + 8 * kk, bd + 2 * kk, idesc, acc);
-                            if (NPROJ == 2) tc_mma_f16_ts(d + NT, a + 32 + 8 * kk, bd + 2 * kk, idesc, acc);
+                            tc_mma_f16_ts<CG>(d, a + 8 * kk, bd + 2 * kk, idesc, acc);
+                            if (NPROJ == 2) tc_mma_f16_ts<CG>(d + NT, a + 32 + 8 * kk, bd + 2 * kk, idesc, acc);
                         }
-                        if (b_last) tc_commit(b_done);
-                        if (a_last) tc_commit(a_done);
+                        if (b_last) tc_commit<CG>(b_done);
+                        if (a_last) tc_commit<CG>(a_done);
                     }
                     __syncwarp();
                 }
             }
-            if (el) tc_commit(&acc_full[buf]);
+            if (el) tc_commit<CG>(&acc_full[buf]);
             __syncwarp();
         }
     } else if (NPROJ == 2 && warp >= 4) {
@@ -956,30 +979,30 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         auto announce = [&]() {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mb_arrive_first(&b_full[done]);
+            if (lane == 0) mb_arrive_first<CG>(&b_full[done]);
             if (++done == C::NB) done = 0;
             behind--;
         };
-        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        GmTile T, next = gm_tile<CG>(P, tile0, n_tiles, rank);
         constexpr int RPT = C::B_ROWS / 16; // rows of a thread
         int nsrc[RPT];
-        auto brows = [&](const GmTile &N) { return min(gm_half(N.nv), N.nv - rank * gm_half(N.nv)); };
+        auto brows = [&](const GmTile &N) { return min(gm_half<CG>(N.nv), N.nv - rank * gm_half<CG>(N.nv)); };
         auto rows = [&](const GmTile &N) {
             const int n = brows(N);
-            const int32_t *src = P.src + N.slot * NT + rank * gm_half(N.nv);
+            const int32_t *src = P.src + N.slot * NT + rank * gm_half<CG>(N.nv);
 #pragma unroll
             for (int i = 0; i < RPT; i++) nsrc[i] = r0 + 16 * i < n ? __ldg(src + r0 + 16 * i) : 0;
         };
         rows(next);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             T = next;
-            next = gm_tile(P, tile + tile_step, n_tiles, rank);
+            next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
             uint32_t off[RPT];
 #pragma unroll
             for (int i = 0; i < RPT; i++) off[i] = (uint32_t)nsrc[i] * row16 + ch;
             rows(next);
             const int n = brows(T);
-            const int grp = gm_b_group<NPROJ, NT>(T.nv);
+            const int grp = gm_b_group<NPROJ, NT, CG>(T.nv);
             const uint32_t sub = C::B_SLOT / grp;
             for (int kb = 0; kb < k_blocks && ok; kb += grp) {
                 ok &= mb_wait(&b_empty[slot], ph ^ 1);
@@ -1005,26 +1028,28 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         // ---------------- epilogue ----------------
         float *stage = reinterpret_cast<float *>(smem + C::O_EPI + (warp - 4) * C::EPI_BYTES);
         uint32_t it = 0;
-        GmTile T, next = gm_tile(P, tile0, n_tiles, rank);
+        GmTile T, next = gm_tile<CG>(P, tile0, n_tiles, rank);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, it++) {
             T = next;
-            next = gm_tile(P, tile + tile_step, n_tiles, rank);
+            next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
             const uint32_t buf = it & 1;
             ok &= mb_wait(&acc_full[buf], (it >> 1) & 1);
             tc_fence_after();
             gm_epilogue<NPROJ, NT>(P, T, tmem_base + buf * NT, stage, warp & 3, lane, 0, 1);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mb_arrive_first(&acc_empty[buf]);
+            if (lane == 0) mb_arrive_first<CG>(&acc_empty[buf]);
         }
     }
     if (NPROJ == 1 && warp >= 4 && warp < GM_DQ0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (!ok && lane == 0) mm_timeout(P.flag, warp);
     tc_fence_before();
     __syncthreads();
-    pair_sync(); // neither CTA leaves while the other may signal it or multiply its operands
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    if (CG == 2) pair_sync(); // neither CTA leaves while the other may signal it or multiply its operands
+    if (warp == 0) {
+        if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
 }
 
 } // namespace
@@ -1145,11 +1170,11 @@ static lmoe_status make_rows_map(CUtensorMap *map, const void *base, uint64_t ro
 }
 
 // st / sh: the stacks of the one or two projections, of the experts and (NULL without extra rows) of the shared expert.
-template <int DT, int NPROJ, int NT>
+template <int DT, int NPROJ, int NT, int CG>
 static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *const (&st)[2], const lmoe_expert_stack *const (&sh)[2],
                                   const void *xt, const int32_t *src, const int32_t *ids_map, int64_t map_stride, const float *row_scale,
                                   float *out, int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
-    using C = GmCfg<DT, NPROJ, NT>;
+    using C = GmCfg<DT, NPROJ, NT, CG>;
     GmParams P;
     P.lg = gm_q6_lg((int)(st[0]->k / QK_K));
     P.lines = (st[0]->n_out & ((1 << P.lg) - 1)) == 0;
@@ -1167,7 +1192,7 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
     P.w[0] = st[0]->blocks();
     P.w[1] = sh[0] ? sh[0]->blocks() : nullptr;
     P.expert_bytes = st[0]->expert_bytes(); P.n_out = (int)st[0]->n_out; P.k = (int)st[0]->k;
-    P.n_expert = R.n_expert; P.m_tiles = (int)((st[0]->n_out + 2 * MM_M - 1) / (2 * MM_M));
+    P.n_expert = R.n_expert; P.m_tiles = (int)((st[0]->n_out + CG * MM_M - 1) / (CG * MM_M));
     P.xt = static_cast<const uint8_t *>(xt); P.src = src; P.ids_map = ids_map; P.map_stride = (int)map_stride;
     P.tiles = static_cast<const int4 *>(tiles_ws); P.n_tiles = mm_tile_count(R, tiles_ws);
     P.row_scale = row_scale; P.out = out; P.sorted = sorted; P.flag = flag;
@@ -1177,10 +1202,10 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
                                       32, GM_BOX_ROWS);
         if (mst) return mst;
     }
-    auto kernel = grouped_mm_kernel<DT, NPROJ, NT>;
+    auto kernel = grouped_mm_kernel<DT, NPROJ, NT, CG>;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.x = CG;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
@@ -1201,10 +1226,10 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
         int sms = 0, pairs = 0;
         LMOE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         LMOE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-        cfg.gridDim = dim3((unsigned)(sms & ~1));
+        cfg.gridDim = dim3((unsigned)(sms / CG * CG));
         LMOE_CUDA(cudaOccupancyMaxActiveClusters(&pairs, kernel, &cfg));
-        if (pairs < 1) return lmoe_fail(LMOE_ERR_CUDA, "no two multiprocessors to pair");
-        c_grid = 2 * pairs < sms ? 2 * pairs : sms & ~1;
+        if (pairs < 1) return lmoe_fail(LMOE_ERR_CUDA, "no place for a tile's CTAs");
+        c_grid = CG * pairs < sms ? CG * pairs : sms / CG * CG;
         c_dev = dev;
     }
     cfg.gridDim = dim3((unsigned)c_grid);
@@ -1213,13 +1238,27 @@ static lmoe_status launch_grouped(const MmRows &R, const lmoe_expert_stack *cons
     return LMOE_OK;
 }
 
+// Up to this many blocks of 128 weight rows, an odd number of them goes to single CTAs: a pair's tile is two blocks high, and the
+// second CTA of the last one would convert rows of no use.  Q4_K, pairs against single CTAs: 512 tokens, ten of 256 experts
+// [128 x 1024] 37.1 us against 28.9, [128 x 3072] 58.2 / 42.0, [640 x 3072] 119 / 109; 64 experts, 8 a token, [1152 x 1024] 37.0 / 32.9;
+// Q6_K, 8192 rows of 4 experts, [384 x 1024] 37.0 / 29.0, [1664 x 1024] 67.7 / 60.5.  Where both take as many rounds over the SMs, long rows
+// in pairs are up to 10 % shorter ([1152 x 3072] of 4 experts 81.2 / 90.0); from 17 blocks on that is the rule ([2176 x 3072] of 64
+// experts 102 / 107).
+constexpr int GM_SINGLE_BLOCKS = 13;
+
 // One grouped projection on the row tiles that launch_gather_tiles made (`xt`: the f16 operand in tile order; `flag`: 4 device
 // words, zero = clean).  Rows of `out` by flat id, times row_scale when given, or (`sorted`) unscaled in expert-sorted order.
 lmoe_status launch_mm_id(const MmRows &R, const lmoe_expert_stack *st, const lmoe_expert_stack *shared, const void *xt,
                          const int32_t *ids_map, int64_t map_stride, const float *row_scale, float *out, int sorted, void *tiles_ws,
                          uint32_t *flag, cudaStream_t stream) {
-    auto fn = R.nt == 128 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128> : launch_grouped<LMOE_Q6_K, 1, 128>)
-                          : (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 192> : launch_grouped<LMOE_Q6_K, 1, 192>);
+    const int64_t blocks = (st->n_out + MM_M - 1) / MM_M;
+    if ((blocks & 1) && blocks <= GM_SINGLE_BLOCKS) {
+        auto fn = R.nt == 128 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128, 1> : launch_grouped<LMOE_Q6_K, 1, 128, 1>)
+                              : (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 192, 1> : launch_grouped<LMOE_Q6_K, 1, 192, 1>);
+        return fn(R, {st, nullptr}, {shared, nullptr}, xt, nullptr, ids_map, map_stride, row_scale, out, sorted, tiles_ws, flag, stream);
+    }
+    auto fn = R.nt == 128 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128, 2> : launch_grouped<LMOE_Q6_K, 1, 128, 2>)
+                          : (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 192, 2> : launch_grouped<LMOE_Q6_K, 1, 192, 2>);
     return fn(R, {st, nullptr}, {shared, nullptr}, xt, nullptr, ids_map, map_stride, row_scale, out, sorted, tiles_ws, flag, stream);
 }
 
@@ -1229,6 +1268,6 @@ lmoe_status launch_mm_gateup(const MmRows &R, const lmoe_expert_stack *gate, con
                              int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
     if (gate->dtype != LMOE_Q4_K || up->dtype != LMOE_Q4_K)
         return lmoe_fail(LMOE_ERR_UNSUPPORTED, "the fused gate/up kernel is built for Q4_K stacks");
-    auto fn = R.nt == 128 ? launch_grouped<LMOE_Q4_K, 2, 128> : launch_grouped<LMOE_Q4_K, 2, 192>;
+    auto fn = R.nt == 128 ? launch_grouped<LMOE_Q4_K, 2, 128, 2> : launch_grouped<LMOE_Q4_K, 2, 192, 2>;
     return fn(R, {gate, up}, {sh_gate, sh_up}, xh, src, ids_map, map_stride, nullptr, act, sorted, tiles_ws, flag, stream);
 }

@@ -225,3 +225,14 @@ def test_combine_after_a_wait_that_ran_out(dev):
             word, out = torch.tensor([flag, 0, 0, 0], dtype=torch.int32, device=dev), torch.zeros(5, n_out, device=dev)
             assert f(down.data_ptr(), None, w.data_ptr(), 5, 3, n_out, out.data_ptr(), stream_ptr(), word.data_ptr()) == 0
             assert torch.isnan(out).all() if flag else torch.equal(out, ops.combine(down, None, w))
+
+
+@pytest.mark.parametrize("dt,name", DTYPES)
+@pytest.mark.parametrize("n_out", [1, 128, 129, 257, 640, 1664, 1665, 1800, 1921])
+def test_mm_single_and_paired_ctas(orc, dev, dt, name, n_out):
+    """Odd numbers of blocks of 128 weight rows go to single CTAs up to 13, the others to pairs: either side of the rule, last blocks of
+    one row and full ones, a pair whose second CTA has no row, both row-tile heights.  Bound as in test_mm_tile_shapes."""
+    for t, k in ((70, 512), (200, 256)):
+        ids = (np.arange(t, dtype=np.uint32) % 2)[:, None]
+        got, want = _case(orc, dev, dt, 2, n_out, k, t, 1, 1, ids, 0xC0 + n_out)
+        assert orc.rel_l2(got, want) < 1e-3
