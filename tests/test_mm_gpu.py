@@ -236,3 +236,23 @@ def test_mm_single_and_paired_ctas(orc, dev, dt, name, n_out):
         ids = (np.arange(t, dtype=np.uint32) % 2)[:, None]
         got, want = _case(orc, dev, dt, 2, n_out, k, t, 1, 1, ids, 0xC0 + n_out)
         assert orc.rel_l2(got, want) < 1e-3
+
+
+@pytest.mark.parametrize("dt,name", DTYPES)
+@pytest.mark.parametrize("n_out,k,t", [(384, 256, 100), (384, 512, 700), (512, 256, 700), (512, 512, 100)])
+def test_mm_repeated_calls_are_bitwise_equal(dev, dt, name, n_out, k, t):
+    """Many tiles of few stages, so that every hand-over between the warps and the CTAs of a pair comes round often: a stale operand
+    would show as a difference between calls on the same inputs."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    ne, top_k = 48, 8
+    st = ExpertStack.random(dt, ne, n_out, k, seed=7, device=dev)
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(t)
+    x = torch.randn(t, 1, k, generator=gen, device=dev)
+    ids = torch.rand(t, ne, generator=gen, device=dev).argsort(1)[:, :top_k].to(torch.int32).contiguous()
+    m = ops.prepare_map0(ne, ids)
+    want = ops.mul_mm_id_shared(st, x, ids, m).view(torch.int32)
+    for _ in range(50):
+        assert torch.equal(ops.mul_mm_id_shared(st, x, ids, m).view(torch.int32), want)
