@@ -68,6 +68,43 @@ def test_argument_errors_without_cuda():
     assert lib.lmoe_map0_scratch_bytes(256, 512) >= 256 * 4 + 256 * 512 * 4
 
 
+def test_ffn_mm_argument_errors_without_cuda():
+    from maxuna_b200 import _native
+
+    lib = _native.lib()
+    fake, keep = C.c_void_p(4096), []
+
+    def stack(ne, n_out, k, dt=12):
+        h = C.c_void_p()
+        assert lib.lmoe_expert_stack_wrap(dt, ne, n_out, k, 4096, ne * n_out * k // 256 * (144 if dt == 12 else 210), 0, C.byref(h)) == 0
+        keep.append(h)
+        return h
+
+    def call(g, u, d, t=4, t_ids=4, top_k=2, k=512, ids=fake, w=fake, x=fake, ws=fake, n=None, out=fake):
+        n = lib.lmoe_ffn_mm_workspace_bytes(g, d, t, top_k) if n is None else n
+        return lib.lmoe_ffn_mm(g, u, d, ids, t_ids, top_k, w, x, t, k, out, ws, n, None)
+
+    g, u, d = stack(4, 256, 512), stack(4, 256, 512), stack(4, 512, 256, 14)
+    need = lib.lmoe_ffn_mm_workspace_bytes(g, d, 4, 2)
+    assert need > 0 and lib.lmoe_ffn_mm_workspace_bytes(g, None, 4, 2) == 0 and lib.lmoe_ffn_mm_workspace_bytes(g, d, -1, 2) == 0
+    for bad in (dict(k=256), dict(t_ids=3), dict(ids=None), dict(w=None), dict(x=None), dict(out=None), dict(x=C.c_void_p(4100)), dict(top_k=0)):
+        assert call(g, u, d, **bad) == -1, bad
+    # stacks that disagree: widths, numbers of experts, the down product's k
+    assert call(g, stack(4, 128, 512), d) == -1
+    assert call(g, stack(3, 256, 512), d) == -1 and b"disagree" in lib.lmoe_last_error()
+    assert call(g, u, stack(3, 512, 256, 14)) == -1 and b"disagree" in lib.lmoe_last_error()
+    assert call(g, u, stack(4, 512, 512, 14)) == -1
+    assert call(g, None, d) == -1
+    # more activations than the separate silu_mul takes
+    assert call(g, u, d, t=1 << 22, t_ids=1 << 22) == -1 and b"i32::MAX" in lib.lmoe_last_error()
+    # workspace: missing, a byte short, not on 256 bytes
+    assert call(g, u, d, ws=None) == -4 and call(g, u, d, n=need - 1) == -4 and call(g, u, d, ws=C.c_void_p(4096 + 128)) == -4
+    # a row that does not fit into shared memory: the ops one by one take it
+    assert call(stack(1, 12544, 512), stack(1, 12544, 512), stack(1, 512, 12544, 14)) == -2 and b"one by one" in lib.lmoe_last_error()
+    for h in keep:
+        lib.lmoe_expert_stack_destroy(h)
+
+
 def test_expert_parallel_argument_errors_without_cuda():
     from maxuna_b200 import _native
 

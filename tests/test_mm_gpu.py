@@ -163,7 +163,7 @@ def test_prefill_block_production_shape(orc, dev):
                                                         (256, 2048, 3, 2, 12, 300)])
 def test_ffn_mm_equals_the_ops(dev, hidden, ff, ne, top_k, up_dt, t):
     """One call for the grouped-GEMM chain gives the bits of its ops one by one: both tile widths, rows of one to eight blocks,
-    widths that take eight and fewer warps a block, and an id that names no expert (which counts nothing here)."""
+    several widths, and an id that names no expert (which counts nothing here)."""
     from maxuna_b200 import ops
     from maxuna_b200.gguf import ExpertStack
 
@@ -256,3 +256,44 @@ def test_mm_repeated_calls_are_bitwise_equal(dev, dt, name, n_out, k, t):
     want = ops.mul_mm_id_shared(st, x, ids, m).view(torch.int32)
     for _ in range(50):
         assert torch.equal(ops.mul_mm_id_shared(st, x, ids, m).view(torch.int32), want)
+
+
+def test_ffn_mm_id_without_expert_in_a_stale_workspace(dev):
+    """A slot whose id names no expert is a zero row of the sum, whatever the workspace held: all bytes 0xFF (NaN, and positions that
+    the lists would have to overwrite) and all zero (positions of the first row)."""
+    from maxuna_b200 import ops
+    from maxuna_b200._native import check, lib
+    from maxuna_b200.gguf import ExpertStack, stream_ptr
+
+    ne, t, top_k, hidden, ff = 4, 40, 2, 256, 512
+    mk = lambda dt, o, k, s: ExpertStack.random(dt, ne, o, k, seed=s, device=dev)
+    g, u, d = mk(12, ff, hidden, 1), mk(12, ff, hidden, 2), mk(14, hidden, ff, 3)
+    x, w = torch.randn(t, hidden, device=dev), torch.rand(t, top_k, device=dev)
+    ids = torch.stack([torch.randperm(ne, device=dev)[:top_k] for _ in range(t)]).to(torch.int32)
+    ids[0, 0], ids[7, 1], ids[9] = ne, -1, ne + 3
+    m, xg = ops.prepare_map0(ne, ids), x.view(t, 1, hidden)
+    act, l2 = ops.l2_rescale(ops.silu_mul(ops.mul_mm_id_shared(g, xg, ids, m), ops.mul_mm_id_shared(u, xg, ids, m)))
+    down = ops.mul_mm_id_shared(d, act, ids, m)
+    gone = (ids < 0) | (ids >= ne)
+    down[gone], l2[gone] = 0.0, 1.0
+    want = ops.combine(down, l2, w)
+    n = lib().lmoe_ffn_mm_workspace_bytes(g.handle, d.handle, t, top_k)
+    for fill in (0xFF, 0):
+        ws, out = torch.full((n,), fill, dtype=torch.uint8, device=dev), torch.empty(t, hidden, device=dev)
+        check(lib().lmoe_ffn_mm(g.handle, u.handle, d.handle, ids.data_ptr(), t, top_k, w.data_ptr(), x.data_ptr(), t, hidden, out.data_ptr(),
+                                ws.data_ptr(), n, stream_ptr()))
+        assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+        check(lib().lmoe_check_device_flag(ws.data_ptr(), stream_ptr()))
+
+
+def test_fused_experts_wider_than_the_one_call(dev, monkeypatch):
+    """`FusedExperts.forward` calls the ops one by one for experts wider than `lmoe_ffn_mm` takes: the same bits."""
+    from maxuna_b200 import ops
+    from maxuna_b200.moe import MoeBlock
+
+    blk = MoeBlock.random(512, 768, 8, 3, seed=4, device=dev)
+    x = torch.randn(90, 512, device=dev)
+    want = blk.forward_unfused(x, use_mm=True)
+    monkeypatch.setattr(ops, "FFN_MM_MAX_FF", 512)
+    monkeypatch.setattr(ops, "ffn_mm", None)
+    assert torch.equal(blk.forward_unfused(x, use_mm=True).view(torch.int32), want.view(torch.int32))
