@@ -758,22 +758,24 @@ __device__ __forceinline__ void mx_units(const MxArgs P, const MxLayout L, int w
     }
 }
 
-// Up to four products of the same shape in one launch, blockIdx.z each (see launch_mul_mv_id_jobs).
+// N = MV_JOBS: up to as many products of the same shape in one launch, blockIdx.z each (see launch_mul_mv_id_jobs).  N = 1: one, its
+// job at a place known to the compiler (Q6_K [4096 x 1024], 16 pairs: 14.5 us, with the job behind blockIdx.z 15.5).
+template <int N>
 struct MxJobs {
-    MvJob job[MV_JOBS];
+    MvJob job[N];
 };
-template <int DT, int NT, int NG, bool ODD>
+template <int DT, int NT, int NG, bool ODD, int N>
 __global__ void __launch_bounds__(32 * (NG * MX_GW + 1), NG == 2 ? 2 : 1)
-mv_expert_kernel(const __grid_constant__ MxJobs jobs, int n_out, int k, int smem_max) {
+mv_expert_kernel(const __grid_constant__ MxJobs<N> jobs, int n_out, int k, int smem_max) {
     pdl_begin();
-    const MvJob &J = jobs.job[blockIdx.z];
+    const MvJob &J = jobs.job[N == 1 ? 0 : blockIdx.z];
     const uint8_t *__restrict__ w = J.w;
     const int64_t expert_bytes = J.expert_bytes;
     const float *__restrict__ x = J.x;
     const uint32_t *__restrict__ ids = J.ids;
     float *__restrict__ out = J.out;
     const int n_expert = J.n_expert, x_per_row = J.x_per_row, top_k = J.top_k, n_pairs = J.pairs;
-    if ((int)blockIdx.y >= n_pairs) return;
+    if (N > 1 && (int)blockIdx.y >= n_pairs) return;
     constexpr int SUB = DT == LMOE_Q4_K ? 32 : 16, NS = QK_K / SUB, NP = 2 * NT, CONS_WARPS = NG * MX_GW;
     extern __shared__ __align__(128) uint8_t mx_smem[];
     __shared__ int pairs_s[NP], np_s;
@@ -872,7 +874,7 @@ mv_expert_kernel(const __grid_constant__ MxJobs jobs, int n_out, int k, int smem
     mx_units<DT, NT, NG>(P, L, warp, lane);
 }
 
-template <int DT, int NT, int NG, bool ODD>
+template <int DT, int NT, int NG, bool ODD, int N>
 cudaError_t launch_mv_expert_jobs(const MvJob *job, int jobs, int n_out, int k, int dev, int sms, cudaStream_t s) {
     constexpr int smem_max = NG == 2 ? MX_SMEM_TWO : MX_SMEM_ONE;
     if (k > smem_max) return cudaErrorNotSupported; // the digits alone are longer, and the layout's sums stay within 32 bits
@@ -880,13 +882,13 @@ cudaError_t launch_mv_expert_jobs(const MvJob *job, int jobs, int n_out, int k, 
     if (L.nstage < NG) return cudaErrorNotSupported; // rows too long for the ring
     static thread_local int c_dev = -1;
     if (dev != c_dev) {
-        const cudaError_t e = cudaFuncSetAttribute(mv_expert_kernel<DT, NT, NG, ODD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+        const cudaError_t e = cudaFuncSetAttribute(mv_expert_kernel<DT, NT, NG, ODD, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
         if (e != cudaSuccess) return e;
         c_dev = dev;
     }
     const int64_t units = (n_out + 16 * L.m - 1) / (16 * L.m), slots = (NG == 2 ? 2 : 1) * (int64_t)sms;
     // Row splits: the blocks run in rounds of `slots`, and a block costs about three units of start-up.
-    MxJobs P = {};
+    MxJobs<N> P = {};
     int64_t groups = 0, most = 0;
     for (int j = 0; j < jobs; j++) {
         P.job[j] = job[j];
@@ -900,7 +902,7 @@ cudaError_t launch_mv_expert_jobs(const MvJob *job, int jobs, int n_out, int k, 
         const int64_t cost = (groups * g + slots - 1) / slots * (3 + (units + g - 1) / g);
         if (cost < best) best = cost, gx = g;
     }
-    launch_pdl(mv_expert_kernel<DT, NT, NG, ODD>, dim3((unsigned)gx, (unsigned)most, (unsigned)jobs), 32 * (NG * MX_GW + 1), L.total, s, P, n_out, k,
+    launch_pdl(mv_expert_kernel<DT, NT, NG, ODD, N>, dim3((unsigned)gx, (unsigned)most, (unsigned)jobs), 32 * (NG * MX_GW + 1), L.total, s, P, n_out, k,
                smem_max);
     return cudaGetLastError();
 }
@@ -912,7 +914,7 @@ cudaError_t launch_mv_expert(const uint8_t *w, int64_t expert_bytes, int n_exper
     for (int64_t p = 0; p < pairs; p += step) {
         const MvJob job = {w, expert_bytes, n_expert, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k,
                            (int)(pairs - p < step ? pairs - p : step), out + (size_t)p * n_out};
-        const cudaError_t r = launch_mv_expert_jobs<DT, NT, NG, ODD>(&job, 1, n_out, k, dev, sms, s);
+        const cudaError_t r = launch_mv_expert_jobs<DT, NT, NG, ODD, 1>(&job, 1, n_out, k, dev, sms, s);
         if (r != cudaSuccess) return r;
     }
     return cudaSuccess;
@@ -1049,7 +1051,7 @@ cudaError_t launch_mv_jobs(const MvJob *job, int jobs, int n_out, int k, cudaStr
         else alone[rest++] = J;
     }
     if (n > 1) {
-        const cudaError_t r = launch_mv_expert_jobs<DT, 1, 2, false>(together, n, n_out, k, dev, sms, s);
+        const cudaError_t r = launch_mv_expert_jobs<DT, 1, 2, false, MV_JOBS>(together, n, n_out, k, dev, sms, s);
         if (r == cudaSuccess) n = 0;
         else if (r != cudaErrorNotSupported) return r;
     }
