@@ -129,8 +129,8 @@ __global__ void add_inplace_kernel(float *__restrict__ out, const float *__restr
 
 // V consecutive columns of one row per thread (four where rows are whole 16-byte words). The top_k terms are summed in the
 // order of the reference's launch geometry: k strided over W lanes, then a butterfly. 512 rows of 10 x 3072: 43 -> 20 us.
-// `flag` (may be NULL): a device flag of the products summed here; once it is set the rows are NaN, never a wrong finite sum.
-template <int W, int V>
+// CHECKED: `flag` is the device flag of the products summed here; once it is set the rows are NaN, never a wrong finite sum.
+template <int W, int V, bool CHECKED>
 __global__ void combine_kernel(const float *__restrict__ down, const float *__restrict__ col_l2,
                                const float *__restrict__ w, int seq, int top_k, int n_out,
                                float *__restrict__ out, const uint32_t *flag) {
@@ -138,6 +138,11 @@ __global__ void combine_kernel(const float *__restrict__ down, const float *__re
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int nv = n_out / V;
     if (i >= (int64_t)seq * nv) return;
+    if (CHECKED && *flag != 0u) {
+#pragma unroll
+        for (int q = 0; q < V; q++) out[i * V + q] = __int_as_float(0x7fc00000);
+        return;
+    }
     const int s = (int)(i / nv), c = (int)(i % nv) * V;
     const float *dp = down + (size_t)s * top_k * n_out + c, *wp = w + (size_t)s * top_k;
     alignas(16) float v[W][V];
@@ -169,10 +174,6 @@ __global__ void combine_kernel(const float *__restrict__ down, const float *__re
         for (int l = 0; l < off; l++)
 #pragma unroll
             for (int q = 0; q < V; q++) v[l][q] = __fadd_rn(v[l][q], v[l + off][q]);
-    if (flag && *flag != 0u) {
-#pragma unroll
-        for (int q = 0; q < V; q++) v[0][q] = __int_as_float(0x7fc00000);
-    }
     if (V == 4) reinterpret_cast<float4 *>(out)[i] = *reinterpret_cast<const float4 *>(v[0]);
     else out[i] = v[0][0];
 }
@@ -326,14 +327,14 @@ cudaError_t launch_add_inplace(float *out, const float *b, int64_t n, cudaStream
     return cudaGetLastError();
 }
 
-template <int W>
+template <int W, bool CHECKED>
 static void combine_launch(const float *down, const float *col_l2, const float *w, int seq, int top_k, int n_out, float *out, cudaStream_t s,
                            const uint32_t *flag) {
     const int64_t n = (int64_t)seq * n_out;
     if (n_out % 4 == 0 && aligned16_all(down, out, nullptr))
-        launch_pdl(combine_kernel<W, 4>, (unsigned)((n / 4 + 127) / 128), 128, 0, s, down, col_l2, w, seq, top_k, n_out, out, flag);
+        launch_pdl(combine_kernel<W, 4, CHECKED>, (unsigned)((n / 4 + 127) / 128), 128, 0, s, down, col_l2, w, seq, top_k, n_out, out, flag);
     else
-        launch_pdl(combine_kernel<W, 1>, (unsigned)((n + 255) / 256), 256, 0, s, down, col_l2, w, seq, top_k, n_out, out, flag);
+        launch_pdl(combine_kernel<W, 1, CHECKED>, (unsigned)((n + 255) / 256), 256, 0, s, down, col_l2, w, seq, top_k, n_out, out, flag);
 }
 
 cudaError_t launch_combine(const float *down, const float *col_l2, const float *w, int seq, int top_k,
@@ -341,14 +342,16 @@ cudaError_t launch_combine(const float *down, const float *col_l2, const float *
     if ((int64_t)seq * n_out == 0) return cudaSuccess;
     int width = 1;
     while (width < top_k / 2) width <<= 1;
+#define COMBINE(W) (flag ? combine_launch<W, true> : combine_launch<W, false>)(down, col_l2, w, seq, top_k, n_out, out, s, flag)
     switch (width) {
-    case 1: combine_launch<1>(down, col_l2, w, seq, top_k, n_out, out, s, flag); break;
-    case 2: combine_launch<2>(down, col_l2, w, seq, top_k, n_out, out, s, flag); break;
-    case 4: combine_launch<4>(down, col_l2, w, seq, top_k, n_out, out, s, flag); break;
-    case 8: combine_launch<8>(down, col_l2, w, seq, top_k, n_out, out, s, flag); break;
-    case 16: combine_launch<16>(down, col_l2, w, seq, top_k, n_out, out, s, flag); break;
-    default: combine_launch<32>(down, col_l2, w, seq, top_k, n_out, out, s, flag); break;
+    case 1: COMBINE(1); break;
+    case 2: COMBINE(2); break;
+    case 4: COMBINE(4); break;
+    case 8: COMBINE(8); break;
+    case 16: COMBINE(16); break;
+    default: COMBINE(32); break;
     }
+#undef COMBINE
     return cudaGetLastError();
 }
 
