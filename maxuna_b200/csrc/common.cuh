@@ -112,14 +112,14 @@ cudaError_t launch_route_logits(const float *router, const float *x, int t, int 
                                 float *logits, cudaStream_t s);
 cudaError_t launch_route_select(const float *logits, const float *bias, int t, int n_expert, int top_k,
                                 float scale, int norm, uint32_t *ids, float *weights, cudaStream_t s, uint32_t *clear = nullptr);
-// mv_id.cu
-// Streamed Q6_K mat-vec (mv_stream.cu): one activation row, all rows of the matrix.
+// mv_stream.cu
+// Streamed Q6_K mat-vec: one activation row, all rows of the matrix.
 bool mv_q6k_stream_available(int64_t n_out, int64_t k);
 cudaError_t launch_mv_q6k_stream(const uint8_t *w, int n_out, int k, const float *x, float *out, cudaStream_t s);
+// mv_id.cu
 cudaError_t launch_mul_mv_id(int dtype, const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k,
                              const float *x, int t, int x_per_row, const uint32_t *ids, int top_k, float *out,
                              cudaStream_t s);
-// glue.cu
 // One product of launch_mul_mv_id_jobs: `pairs` = tokens times top_k; ids NULL = expert 0 for every pair.
 constexpr int MV_JOBS = 4;
 struct MvJob {
@@ -134,6 +134,7 @@ struct MvJob {
 };
 // Products of the same type, row count and k that do not depend on one another.
 cudaError_t launch_mul_mv_id_jobs(int dtype, const MvJob *job, int jobs, int n_out, int k, cudaStream_t s);
+// glue.cu
 // silu_mul and l2_rescale of rows of n values (a multiple of 256, at most LMOE_FFN_MM_MAX_FF), straight into the grouped GEMM's tile order as f16
 // (row of the tile order pos[row], tiles of nt rows); a row that no list names (pos < 0) is a zero row of y instead.
 cudaError_t launch_silu_rescale_tiles(const float *g, const float *u, const int32_t *pos, int64_t rows, int n, int nt, void *act, float *l2,

@@ -1057,9 +1057,16 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
 // ---- host side ---------------------------------------------------------------------------
 // Routed rows per tile.  192 fills the tensor memory beside two accumulators with two operand stages and converts each
 // weight least often; with a few dozen rows per expert every tile is thin whatever its limit, and 128 leaves room for four
-// operand stages.  A call of 256 experts [3072 x 1024], evenly routed, 128 against 192, by rows per expert: 8 461 us against 460,
-// 16 490 / 472, 24 516 / 513, 32 525 / 523, 40 547 / 544, 48 586 / 555, 64 620 / 613, 80 683 / 670; of 128 experts [2048 x 768]: 8
-// 183 / 190, 16 192 / 198, 24 199 / 209, 32 200 / 211, 40 209 / 215, 48 212 / 226, 64 217 / 219, 80 224 / 230.
+// operand stages.  A block's forward with its shared expert, evenly routed, cold L2, both launches overlapped, us with 128 / 192 by rows
+// per expert:
+//                              8         16         24         32         40         48         64         80        160
+//   256 experts, 3072, 1024  423 / 422  479 / 478  528 / 508  563 / 561  594 / 603  675 / 636  768 / 740  869 / 821  1431 / 1282
+//   128 experts, 2048, 768   167 / 166  179 / 178  188 / 188  195 / 195  205 / 205  217 / 216  246 / 229  272 / 257   426 / 382
+//   64 experts, 4096, 1536   289 / 286  295 / 293  299 / 302  307 / 303  311 / 310  316 / 321  336 / 335  393 / 360   638 / 601
+//   64 experts, 2048, 512     96 / 96    96 / 96    97 / 100  100 / 100  100 / 102  104 / 107  113 / 112  131 / 120   188 / 173
+//   16 experts, 4096, 2048   148 / 145  150 / 150  148 / 156  154 / 154  184 / 160  180 / 160  188 / 193  201 / 199   315 / 287
+// From some 60 rows on 192 is the shorter one.  Below, most differ by less than 2 % and the others go either way, as the tallest lists
+// happen to fill a tile of one height or the other; the line lies where 128 no longer gains anything.
 int mm_tile_rows(int64_t rows, int64_t n_expert) { return rows <= 40 * n_expert ? 128 : 192; }
 
 // Row tiles that `rows` routed rows over n_lists lists can make.

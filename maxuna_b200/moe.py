@@ -2,11 +2,13 @@
 
   ExpertFfn       src/moe.rs:19-21   forward(x, ids, weights) -> [seq, hidden]
   MoeBlock        src/moe.rs:28-79   route -> experts -> + shared expert
-  FusedExperts    src/moe.rs:194-324 op-by-op runner over ``ops`` (mv_id / mm_id)
+  FusedExperts    src/moe.rs:194-324 the op chain of ``ops`` (mv_id / mm_id), one C call each way
   SharedExpert    src/moe.rs:327-345 the always-on SwiGLU expert
 ``MoeBlock.forward`` runs the whole block through the fused CUDA entry points
 (``lmoe_moe_forward_decode`` / ``_prefill``); ``MoeBlock.forward_unfused``
-follows the reference's op-by-op sequence and exists for op-level parity.
+follows the reference's sequence of ops (``lmoe_route``, then ``lmoe_ffn_mv`` or
+``lmoe_ffn_mm``, which give the bits of the ops called one by one) and exists for
+op-level parity.
 """
 from __future__ import annotations
 
@@ -147,7 +149,8 @@ class MoeBlock:
                          self.n_expert_used, self.weights_scale, self.weights_norm)
 
     def forward_unfused(self, x_normed: torch.Tensor, use_mm=None) -> torch.Tensor:
-        """The reference's op-by-op sequence, src/moe.rs:73-78."""
+        """The reference's sequence of ops, src/moe.rs:73-78: routing, then the experts' op chain as one call (`ops.ffn_mv` /
+        `ops.ffn_mm`: the bits of the ops one by one, with fewer launches)."""
         x = _f32(x_normed)
         ids, weights = self.route(x)
         e, sh = self.experts, self.shared
