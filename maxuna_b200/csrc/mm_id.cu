@@ -723,6 +723,13 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
     asm volatile("griddepcontrol.wait;" ::: "memory"); // what earlier kernels wrote is read from here on
     const int n_tiles = *P.n_tiles * P.m_tiles;
     bool ok = true; // false once a wait of this warp has run out
+    // A loader leaves when its copies have landed, also where their readers have given up: slot i < next was filled in the present turn of
+    // the ring (its parity), the others in the turn before (a barrier never used counts as complete).
+    auto landed = [&](uint64_t *full, int n, uint32_t next, uint32_t parity) {
+        bool here = true;
+        for (int i = 0; i < n && here; i++) here = mb_wait(&full[i], (uint32_t)i < next ? parity : parity ^ 1);
+        ok &= here;
+    };
 
     if (warp >= GM_DQ0) {
         // ---------------- dequant: thread = (part, weight row), group = stage parity ----------------
@@ -876,6 +883,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                 if (++slot == C::RAW_SLOTS) { slot = 0; rph ^= 1; }
             }
         }
+        landed(raw_full, C::RAW_SLOTS, slot, rph);
     } else if (NPROJ == 1 && warp == 1) {
         // ---------------- B loader: one bulk copy per 64-k block (the operand is stored in tile order) ----------------
         const bool el = elect_one();
@@ -898,6 +906,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
                 if (++slot == C::NB) { slot = 0; ph ^= 1; }
             }
         }
+        landed(b_full, C::NB, slot, ph);
     } else if (NPROJ == 1 && CG == 2 && warp == 0 && rank == 1) {
         // ---------------- relay: a bulk copy signals its own CTA only; the issuer is told that this half of a slot has landed ----------------
         uint32_t slot = 0, ph = 0;
@@ -969,6 +978,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             if (el) tc_commit<CG>(&acc_full[buf]);
             __syncwarp();
         }
+        // the last tile's commit covers all multiplies: none is in flight when the tensor memory is given back
+        if (it) ok &= mb_wait(&acc_full[NPROJ == 2 ? 0u : (it - 1) & 1], NPROJ == 2 ? (it - 1) & 1 : ((it - 1) >> 1) & 1);
     } else if (NPROJ == 2 && warp >= 4) {
         // ---------------- B loaders: thread = (16-byte chunk of the 128-byte row piece, every 16th row) ----------------
         const int lt = tid - 128, ch = lt & 7, r0 = lt >> 3;
