@@ -8,6 +8,8 @@
 // Persistent pairs of CTAs, one CTA per SM, warp-specialised around tcgen05.mma; see grouped_mm_kernel.  The weight tile is the
 // A operand (M = 256 output features, 128 in each CTA) and the routed rows are the N dimension, so ragged per-expert row counts cost
 // only a rounding to 16.  Every wait is bounded; a wait that runs out records a flag and the kernel drains and exits.
+#include <type_traits>
+
 #include <cuda.h> // CUtensorMap (types only; the encoder is fetched through the runtime)
 
 #include "fused.cuh"
@@ -87,18 +89,35 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar) {
 }
 // D += A * B for both CTAs of a pair; the A operand lies in tensor memory, in each CTA its own 128 lanes (weight rows) x 8 columns
 // (K = 16 as f16 pairs), and each CTA's shared memory holds half of B's rows at the place the descriptor names.
-template <int CG>
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
-    if (CG == 1)
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc),
-            "r"(accum) : "memory");
+// The four K = 16 steps of a 64-k block, of one projection or (d1 != d0) two: one piece of assembly of 32-bit additions, as the issuing
+// warp's own instructions are what a thin tile's stage takes.  `first`: the block starts the accumulators.
+template <int CG, bool TWO>
+__device__ __forceinline__ void tc_mma_block(uint32_t d0, uint32_t d1, uint32_t a, uint32_t blo, uint32_t bhi, uint32_t idesc, uint32_t first) {
+    if (CG == 1 && !TWO)
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t.reg .b32 l, t;\n\tsetp.eq.b32 p, %6, 0;\n\t"
+                     "mov.b64 b, {%3, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%2], b, %5, p;\n\t"
+                     "add.u32 l, %3, 2;\n\tadd.u32 t, %2, 8;\n\tmov.b64 b, {l, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [t], b, %5, 1;\n\t"
+                     "add.u32 l, %3, 4;\n\tadd.u32 t, %2, 16;\n\tmov.b64 b, {l, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [t], b, %5, 1;\n\t"
+                     "add.u32 l, %3, 6;\n\tadd.u32 t, %2, 24;\n\tmov.b64 b, {l, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [t], b, %5, 1;\n\t}"
+                     ::"r"(d0), "r"(d1), "r"(a), "r"(blo), "r"(bhi), "r"(idesc), "r"(first) : "memory");
+    else if (CG == 2 && !TWO)
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t.reg .b32 l, t;\n\tsetp.eq.b32 p, %6, 0;\n\t"
+                     "mov.b64 b, {%3, %4};\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%2], b, %5, p;\n\t"
+                     "add.u32 l, %3, 2;\n\tadd.u32 t, %2, 8;\n\tmov.b64 b, {l, %4};\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [t], b, %5, 1;\n\t"
+                     "add.u32 l, %3, 4;\n\tadd.u32 t, %2, 16;\n\tmov.b64 b, {l, %4};\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [t], b, %5, 1;\n\t"
+                     "add.u32 l, %3, 6;\n\tadd.u32 t, %2, 24;\n\tmov.b64 b, {l, %4};\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [t], b, %5, 1;\n\t}"
+                     ::"r"(d0), "r"(d1), "r"(a), "r"(blo), "r"(bhi), "r"(idesc), "r"(first) : "memory");
     else
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc),
-            "r"(accum) : "memory");
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t.reg .b32 l, t;\n\tsetp.eq.b32 p, %6, 0;\n\t"
+                     "mov.b64 b, {%3, %4};\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%2], b, %5, p;\n\t"
+                     "add.u32 t, %2, 32;\n\ttcgen05.mma.cta_group::2.kind::f16 [%1], [t], b, %5, p;\n\t"
+                     "add.u32 l, %3, 2;\n\tadd.u32 t, %2, 8;\n\tmov.b64 b, {l, %4};\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [t], b, %5, 1;\n\t"
+                     "add.u32 t, %2, 40;\n\ttcgen05.mma.cta_group::2.kind::f16 [%1], [t], b, %5, 1;\n\t"
+                     "add.u32 l, %3, 4;\n\tadd.u32 t, %2, 16;\n\tmov.b64 b, {l, %4};\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [t], b, %5, 1;\n\t"
+                     "add.u32 t, %2, 48;\n\ttcgen05.mma.cta_group::2.kind::f16 [%1], [t], b, %5, 1;\n\t"
+                     "add.u32 l, %3, 6;\n\tadd.u32 t, %2, 24;\n\tmov.b64 b, {l, %4};\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [t], b, %5, 1;\n\t"
+                     "add.u32 t, %2, 56;\n\ttcgen05.mma.cta_group::2.kind::f16 [%1], [t], b, %5, 1;\n\t}"
+                     ::"r"(d0), "r"(d1), "r"(a), "r"(blo), "r"(bhi), "r"(idesc), "r"(first) : "memory");
 }
 // 32 registers of every lane -> 32 columns of the warp's 32 tensor-memory lanes; complete after tc_wait_st().
 __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -164,6 +183,17 @@ __device__ __forceinline__ uint32_t h2_sub_fma(uint32_t v, uint32_t base, uint32
 __device__ __forceinline__ uint32_t h2_sub_mul(uint32_t v, uint32_t base, uint32_t s) {
     uint32_t r;
     asm("{\n\t.reg .b32 t;\n\tsub.rn.f16x2 t, %1, %2;\n\tmul.rn.f16x2 %0, t, %3;\n\t}" : "=r"(r) : "r"(v), "r"(base), "r"(s));
+    return r;
+}
+
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
     return r;
 }
 
@@ -365,10 +395,18 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict_
 // projection (the down projection, and the op-level `mul_mm_id` of either format).
 //
 // Sixteen dequantising warps in two groups of eight take the pipeline stages in turn.  A stage is 64 weights for
-// each of a group's 256 threads: 2 projections x 128 rows x 64 k, or 128 rows x 128 k.  The f16 values go straight
+// each of a group's 256 threads, 2 projections x 128 rows x 64 k or 128 rows x 128 k, and with tiles of up to 128 rows
+// (WIDE) twice that.  The f16 values go straight
 // into TENSOR MEMORY (tcgen05.st: lane = weight row) and the tensor core takes its A operand from there (TS form),
 // so the dequantised tile never passes through shared memory.  A thread converts its next stage's weights BEFORE it
 // waits for the stage to be free, so the wait covers only the store.
+// A thin tile is bound by instructions, on the converting warps' schedulers as a whole (70 % of the issue slots, of the integer pipe
+// 64) and one by one in the warp that issues the multiplies (450 to 560 cycles a stage where its multiplies take 100): hence the wide stages, which halve
+// what is done once a stage, tc_mma_block's assembly, and subnormal operands in the conversion.  A block's forward with its shared
+// expert, 128 / 512 / 1024 / 2048 tokens on 256 experts of 1024, cold L2: 402 / 489 / 591 / 840 us with stages of 64 weights and the
+// plain conversion, 382 / 470 / 579 / 813 with wide stages and lean issue, 365 / 452 / 554 / 800 with the subnormal conversion
+// too; 318 without conversions at 128 tokens, 240 the weights at the copy rate.  Four groups of four warps (396 / 483 / 589), the next
+// stage's words loaded ahead (411 / 517 / 623: the operand slots are held for longer) and other ways of waiting (none shorter) were tried.
 //
 // Two CTAs on neighbouring SMs share a tile (CG = 2, cta_group::2; with CG = 1 a CTA has a tile of 128 weight rows for itself): each
 // converts 128 of its 256 weight rows and keeps their accumulators, and each loads half of the tile's activation rows, which the tensor cores of both read.  One SM alone loads 24 KB of
@@ -385,7 +423,7 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const void *__restrict_
 //
 // Tensor-memory columns: [0, NT) and [NT, 2 NT): the gate and up accumulators, or the two accumulator
 // buffers of a single projection (its epilogue runs beside the next tile's multiplies); the rest holds the operand
-// stages, 64 columns each: two beside 192-row tiles, four beside 128-row tiles.
+// stages: two of 64 columns beside 192-row tiles, of 128 columns two beside 128-row and three beside 64-row tiles.
 //   warp 0    MMA issuer (second CTA, single projection: relay)    warp 2 loader of the quantized columns    warps 8-23 dequant
 //   single projection: warp 1 B loader (bulk copies of the tile-ordered operand), warps 4-7 epilogue
 //   two projections: warps 4-7 B loaders (rows in token order), the epilogue falls to the dequantising warps
@@ -410,14 +448,18 @@ struct GmCfg {
     static constexpr int EPI_BYTES = NPROJ == 2 ? GM_EPI_BYTES : 2 * GM_BOX_ROWS * 128;
     static constexpr int B_ROWS = NT / CG;
     static constexpr int B_BLK = B_ROWS * MM_K * 2;     // a CTA's half of a 64-k block of the B operand
-    static constexpr int B_SLOT = NPROJ == 2 || CG == 1 ? B_BLK : 2 * B_BLK; // ring slot: as much as an operand stage multiplies (a CTA alone: half of that)
+    static constexpr int B_FULL = (NPROJ == 2 || CG == 1 ? 1 : 2) * (NT == 64 ? 2 : 1); // blocks of a full tile in a ring slot
+    static constexpr int B_SLOT = B_FULL * B_BLK;
     static constexpr int NB = 96 * 1024 / B_SLOT < 8 ? 96 * 1024 / B_SLOT : 8;
-    static constexpr int NA = (512 - 2 * NT) / 64 >= 4 ? 4 : 2, A_COL0 = 2 * NT;
+    static constexpr bool WIDE = NT <= 128;             // operand stages of 128 weights a thread, else 64
+    static constexpr int A_COLS = WIDE ? 128 : 64, NA = (512 - 2 * NT) / A_COLS, A_COL0 = 2 * NT;
+    static constexpr int A_BLKS = (WIDE ? 2 : 1) * (NPROJ == 2 ? 1 : 2); // 64-k blocks of an operand stage
+    static constexpr int RAW_READERS = WIDE && NPROJ == 1 ? GM_DQ_WARPS / 2 : GM_DQ_WARPS;
     static constexpr int EPI_WARPS = NPROJ == 2 ? GM_DQ_WARPS : 4;
     static constexpr int B_ARRIVALS = NPROJ == 2 ? 4 * CG : 1; // per ring slot (the first CTA's of a single projection: one more, see the relay)
     static constexpr int O_RAW = NB * B_SLOT, O_EPI = O_RAW + RAW_SLOTS * RAW_SLOT, O_BAR = O_EPI + EPI_WARPS * EPI_BYTES;
     static constexpr int SMEM = O_BAR + 512 + 1024; // barriers, slack to align the base to 1024 bytes
-    static_assert(A_COL0 + 64 * NA <= 512, "tensor memory");
+    static_assert(A_COL0 + A_COLS * NA <= 512 && NA >= 2, "tensor memory");
     static_assert(SMEM <= 227 * 1024, "shared memory");
 };
 
@@ -448,19 +490,38 @@ struct GmParams {
 // 64 weights (sub-block pair j) of one Q4_K row -> 32 words, in the order the activation rows are stored
 // (8-value chunks as [0 2 1 3 4 6 5 7]): word 4c + i = chunk c, pair i.
 // The scale d * sc and the offset -dmin * m are products of an f16 and a six-bit integer, rounded once to f16.
-__device__ __forceinline__ void dequant_q4k_regs(const uint4 hdr, const uint4 qa, const uint4 qb, int j, uint32_t (&o)[32]) {
+// `small` (|d| < 2^-10, so that every scale is below 2^-4): a nibble in bits 4 to 7 of a half is the subnormal q * 2^-20, and the fma
+// takes it as it is with the scale times 2^20: the same product, so the same value, without the subtraction that makes a plain q.
+constexpr uint32_t Q4K_SMALL_D = 0x1400; // f16 bits of 2^-10
+__device__ __forceinline__ void dequant_q4k_regs(const uint4 hdr, const uint4 qa, const uint4 qb, int j, bool small, uint32_t (&o)[32]) {
     uint32_t sc[2], mn[2];
     q4k_unpack_scales(hdr.y, hdr.z, hdr.w, sc[0], sc[1], mn[0], mn[1]);
     // bytes 2 (j & 1), 2 (j & 1) + 1 of word j >> 1 -> 1024 + value, as an f16 pair
     const uint32_t sel = (j & 1) ? 0x4342u : 0x4140u;
-    const uint32_t s2 = h2_sub_mul(prmt((j & 2) ? sc[1] : sc[0], 0x64646464u, sel), 0x64006400u, prmt(hdr.x, 0u, 0x1010u));
+    const uint32_t d2 = prmt(hdr.x, 0u, 0x1010u);
+    uint32_t s2 = h2_sub_mul(prmt((j & 2) ? sc[1] : sc[0], 0x64646464u, sel), 0x64006400u, small ? h2_mul(d2, 0x64006400u) : d2);
     const uint32_t m2 = h2_sub_mul(prmt((j & 2) ? mn[1] : mn[0], 0x64646464u, sel), 0x64006400u, prmt(hdr.x ^ 0x80000000u, 0u, 0x3232u));
-    const uint32_t s_lo = prmt(s2, 0u, 0x1010u), s_hi = prmt(s2, 0u, 0x3232u), m_lo = prmt(m2, 0u, 0x1010u), m_hi = prmt(m2, 0u, 0x3232u);
+    const uint32_t m_lo = prmt(m2, 0u, 0x1010u), m_hi = prmt(m2, 0u, 0x3232u);
     const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+    if (small) {
+        s2 = h2_mul(s2, 0x64006400u);
+        const uint32_t s_lo = prmt(s2, 0u, 0x1010u), s_hi = prmt(s2, 0u, 0x3232u);
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const uint32_t v = w[c];
+            // low nibbles (sub-block 2j): chunks 0-3; high nibbles (sub-block 2j+1): chunks 4-7
+            o[2 * c] = h2_fma((v << 4) & 0x00F000F0u, s_lo, m_lo);
+            o[2 * c + 1] = h2_fma((v >> 4) & 0x00F000F0u, s_lo, m_lo);
+            o[16 + 2 * c] = h2_fma(v & 0x00F000F0u, s_hi, m_hi);
+            o[16 + 2 * c + 1] = h2_fma((v >> 8) & 0x00F000F0u, s_hi, m_hi);
+        }
+        return;
+    }
+    const uint32_t s_lo = prmt(s2, 0u, 0x1010u), s_hi = prmt(s2, 0u, 0x3232u);
 #pragma unroll
     for (int c = 0; c < 8; c++) {
         const uint32_t v = w[c], v8 = v >> 8;
-        // low nibbles (sub-block 2j): chunks 0-3, as 1024 + q; high nibbles in place (sub-block 2j+1): chunks 4-7, as 64 + q
+        // the same nibbles as 1024 + q and, in place, 64 + q
         o[2 * c] = h2_sub_fma(and_or(v, 0x000F000Fu, 0x64006400u), 0x64006400u, s_lo, m_lo);
         o[2 * c + 1] = h2_sub_fma(and_or(v8, 0x000F000Fu, 0x64006400u), 0x64006400u, s_lo, m_lo);
         o[16 + 2 * c] = h2_sub_fma(and_or(v, 0x00F000F0u, 0x54005400u), 0x54005400u, s_hi, m_hi);
@@ -531,12 +592,34 @@ __device__ __forceinline__ void q6k_fields_paired(const uint8_t *base8, int sh, 
 // 16 weights of each of the half's four 32-wide groups -> o[8 g .. 8 g + 7] = group g's values 16 lh .. 16 lh + 15,
 // 8-value chunks as [0 2 1 3 4 6 5 7].  Four six-bit values are put together per word (low nibble | two high bits << 4),
 // then spread two at a time into f16 pairs 1024 + q by one byte permute; q - 32 is exact and the scale rounds once.
-__device__ __forceinline__ void dequant_q6k_regs(const Q6Fields &F, int lh, uint32_t (&o)[32]) {
-    const uint32_t off = 0x64206420u; // 1024 + 32
+// `small` (|d| < 2^-13, so that every scale is below 2^-6): the values stand two bits higher in their bytes, as the subnormals q * 2^-22,
+// and one fma with the scale times 2^22 and -32 scales gives the same value.
+constexpr uint32_t Q6K_SMALL_D = 0x0800; // f16 bits of 2^-13
+__device__ __forceinline__ void dequant_q6k_regs(const Q6Fields &F, int lh, bool small, uint32_t (&o)[32]) {
     // the four groups' scales are bytes lh, 2 + lh of s0 and of s1, signed: (s ^ 0x80) + 1024 - 1152
     const uint32_t selp = lh ? 0x4341u : 0x4240u;
-    const uint32_t sc01 = h2_sub_mul(prmt(F.s0 ^ 0x80808080u, 0x64646464u, selp), 0x64806480u, F.d2);
-    const uint32_t sc23 = h2_sub_mul(prmt(F.s1 ^ 0x80808080u, 0x64646464u, selp), 0x64806480u, F.d2);
+    const uint32_t d2 = small ? h2_mul(F.d2, 0x78007800u) : F.d2; // * 2^15
+    const uint32_t sc01 = h2_sub_mul(prmt(F.s0 ^ 0x80808080u, 0x64646464u, selp), 0x64806480u, d2);
+    const uint32_t sc23 = h2_sub_mul(prmt(F.s1 ^ 0x80808080u, 0x64646464u, selp), 0x64806480u, d2);
+    if (small) {
+        const uint32_t b01 = h2_mul(sc01, 0x94009400u), b23 = h2_mul(sc23, 0x94009400u); // * -2^-10: -32 scales
+        const uint32_t m01 = h2_mul(sc01, 0x58005800u), m23 = h2_mul(sc23, 0x58005800u); // * 2^7
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            const uint32_t sel = (g & 1) ? 0x3232u : 0x1010u;
+            const uint32_t sc = prmt(g < 2 ? m01 : m23, 0u, sel), off = prmt(g < 2 ? b01 : b23, 0u, sel);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint32_t q = (g & 1) ? F.qb[j] : F.qa[j], ql = g < 2 ? q << 2 : q >> 2;
+                const uint32_t h = g == 0 ? F.qh[j] << 6 : (g == 1 ? F.qh[j] << 4 : (g == 2 ? F.qh[j] << 2 : F.qh[j]));
+                const uint32_t q6 = and_or(ql, 0x3C3C3C3Cu, h & 0xC0C0C0C0u);
+                o[8 * g + 2 * j] = h2_fma(prmt(q6, 0u, 0x4240u), sc, off);
+                o[8 * g + 2 * j + 1] = h2_fma(prmt(q6, 0u, 0x4341u), sc, off);
+            }
+        }
+        return;
+    }
+    const uint32_t off = 0x64206420u; // 1024 + 32
 #pragma unroll
     for (int g = 0; g < 4; g++) {
         // groups 0, 1: low nibbles of qa, qb; groups 2, 3: their high nibbles
@@ -571,10 +654,9 @@ __device__ __forceinline__ GmTile gm_tile(const GmParams &P, int tile, int n_til
 }
 // 64-k blocks of the B operand that share one ring slot: a thin tile's blocks do not fill it, and a deeper ring is what
 // hides the copies' latency there.
-template <int NPROJ, int NT, int CG>
+template <int FULL, int NT>
 __device__ __forceinline__ int gm_b_group(int nv) {
-    constexpr bool one = NPROJ == 2 || CG == 1; // a slot holds one block of a full tile, else two
-    return nv > NT / 2 ? (one ? 1 : 2) : (one && nv > NT / 4 ? 2 : 4);
+    return nv > NT / 2 ? FULL : (FULL == 1 && nv > NT / 4 ? 2 : 4);
 }
 
 // rows of a tile that each CTA of a pair holds of the B operand (of the padded tile: a multiple of 8)
@@ -702,7 +784,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         }
         for (int i = 0; i < C::RAW_SLOTS; i++) {
             mb_init(&raw_full[i], 1);
-            mb_init(&raw_empty[i], GM_DQ_WARPS);
+            mb_init(&raw_empty[i], C::RAW_READERS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -737,98 +819,119 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         const int grp = (warp - GM_DQ0) >> 3, part = (warp >> 2) & 1, q = warp & 3, r = 32 * q + lane;
         const uint32_t ta = tmem_base + ((uint32_t)(32 * q) << 16) + C::A_COL0;
         float *stage = reinterpret_cast<float *>(smem + C::O_EPI + (NPROJ == 2 ? (warp - GM_DQ0) * C::EPI_BYTES : 0));
-        uint32_t use = 0, slot = 0, rph = 0, it = 0; // stages of this group, ring slot and its phase, tiles
-        // the group's stage number `use` goes to operand slot (2 use + grp) mod NA; with two stages per column, i = use mod 2
-        auto store = [&](const uint32_t (&o)[32], uint32_t i) {
-            const uint32_t as = C::NA == 4 ? 2 * i + grp : grp, ph = C::NA == 4 ? (use >> 1) & 1 : i;
-            ok &= mb_wait(&a_empty[as], ph ^ 1);
+        uint32_t slot = C::WIDE && NPROJ == 1 ? grp : 0, rph = 0, it = 0; // raw ring slot and its phase, tiles
+        uint32_t as = grp, aph = 0;                                      // operand slot of the group's next stage: every second one
+        auto slot_free = [&]() {
+            ok &= mb_wait(&a_empty[as], aph ^ 1);
             tc_fence_after();
-            if (DT == LMOE_Q4_K) {
-                tc_st32(ta + 64u * as + 32u * part, o);
-            } else {
-#pragma unroll
-                for (int g = 0; g < 4; g++) tc_st8(ta + 64u * as + 16u * g + 8u * part, o + 8 * g);
-            }
         };
-        auto stored = [&](uint32_t i) {
+        auto stored = [&]() {
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mb_arrive_first<CG>(&a_full[C::NA == 4 ? 2 * i + grp : grp]);
-            use++;
+            if (lane == 0) mb_arrive_first<CG>(&a_full[as]);
+            if ((as += 2) >= C::NA) { as -= C::NA; aph ^= 1; }
         };
-        // single projection: the thread's part of one column, out of shared memory; then the slot goes back to the loader
-        const int j0 = NPROJ == 2 ? grp : 2 * grp + part;
-        uint4 hdr, qa, qb;
-        Q6Fields F;
-        int sh = 0; // Q6_K: offset of the block inside its 16-byte granule
-        const uint32_t line = DT == LMOE_Q6_K ? (uint32_t)gm_q6_line(r, P.lg) * GM_Q6_PITCH : 0u;
-        auto load = [&](int b) {
-            ok &= mb_wait(&raw_full[slot], rph);
-            const uint8_t *rs = raw + (size_t)slot * C::RAW_SLOT;
-            if (DT == LMOE_Q4_K) {
-                const uint4 *blk = reinterpret_cast<const uint4 *>(rs + r * Q4K_BYTES);
-                hdr = blk[0];
-                qa = blk[1 + 2 * j0];
-                qb = blk[2 + 2 * j0];
-            } else {
-                if (P.lg <= 1) q6k_fields_paired(rs + line, sh, b, grp, part, F);
-                else q6k_fields(rs + line, sh & 15, grp, part, F);
-                sh += Q6K_BYTES;
-            }
+        auto read = [&]() { // this warp is done with the ring slot
             __syncwarp();
             if (lane == 0) mb_arrive(&raw_empty[slot]);
-            if (++slot == C::RAW_SLOTS) { slot = 0; rph ^= 1; }
+            if ((slot += C::WIDE && NPROJ == 1 ? 2 : 1) >= C::RAW_SLOTS) { slot -= C::RAW_SLOTS; rph ^= 1; }
         };
-        // two projections: the first or second of this group's stages of a column
-        auto half = [&](uint32_t i) {
-            if (i == 0) ok &= mb_wait(&raw_full[slot], rph);
-            const uint4 *blk = reinterpret_cast<const uint4 *>(raw + (size_t)slot * C::RAW_SLOT + (part * MM_M + r) * Q4K_BYTES);
-            hdr = blk[0];
-            qa = blk[1 + 2 * j0 + 4 * i];
-            qb = blk[2 + 2 * j0 + 4 * i];
-            if (i == 1) {
-                __syncwarp();
-                if (lane == 0) mb_arrive(&raw_empty[slot]);
-                if (++slot == C::RAW_SLOTS) { slot = 0; rph ^= 1; }
+        int sh = 0; // Q6_K: offset of the block inside its 16-byte granule
+        const uint32_t line = DT == LMOE_Q6_K ? (uint32_t)gm_q6_line(r, P.lg) * GM_Q6_PITCH : 0u;
+        auto q6_fields = [&](int b, int n, Q6Fields &F) {
+            const uint8_t *rs = raw + (size_t)slot * C::RAW_SLOT + line;
+            if (P.lg <= 1) q6k_fields_paired(rs, sh, b, n, part, F);
+            else q6k_fields(rs, sh & 15, n, part, F);
+        };
+        const uint32_t blk0 = (uint32_t)((NPROJ == 2 ? part * MM_M : 0) + r) * Q4K_BYTES;
+        uint4 hdr, qw[C::WIDE ? 4 : 2];
+        Q6Fields F[C::WIDE ? 2 : 1];
+        // sub-block pair of the thread's first 64 weights of a column; a wide stage takes the next pair too
+        const int j0 = C::WIDE ? 2 * (NPROJ == 2 ? grp : part) : (NPROJ == 2 ? grp : 2 * grp + part);
+        // the thread's part of a stage, out of shared memory: sub-block pair j (and the next), or half n (both)
+        auto fetch = [&](int j, int b) {
+            if (DT == LMOE_Q4_K) {
+                const uint4 *blk = reinterpret_cast<const uint4 *>(raw + (size_t)slot * C::RAW_SLOT + blk0);
+                hdr = blk[0];
+#pragma unroll
+                for (int i = 0; i < (C::WIDE ? 4 : 2); i++) qw[i] = blk[1 + 2 * j + i];
+            } else {
+#pragma unroll
+                for (int n = 0; n < (C::WIDE ? 2 : 1); n++) q6_fields(b, C::WIDE ? n : grp, F[n]);
             }
+        };
+        // 64 of its weights (half i of a wide stage) into the operand slot
+        auto put = [&](const uint32_t (&o)[32], int i) {
+            const uint32_t a = ta + (uint32_t)C::A_COLS * as;
+            if (DT == LMOE_Q4_K) {
+                tc_st32(a + (C::WIDE && NPROJ == 1 ? 64u * part + 32u * i : 64u * i + 32u * part), o);
+            } else {
+#pragma unroll
+                for (int g = 0; g < 4; g++) tc_st8(a + 64u * i + 16u * g + 8u * part, o + 8 * g);
+            }
+        };
+        bool small = false; // all the warp's rows have small scales in this column
+        auto convert = [&](int j, int i, uint32_t (&o)[32]) {
+            if (DT == LMOE_Q4_K) dequant_q4k_regs(hdr, qw[2 * i], qw[2 * i + 1], j + i, small, o);
+            else dequant_q6k_regs(F[i], part, small, o);
+        };
+        auto stage_in = [&](int j) {
+            small = __all_sync(0xffffffffu, DT == LMOE_Q4_K ? (hdr.x & 0x7FFFu) < Q4K_SMALL_D : (F[0].d2 & 0x7FFFu) < Q6K_SMALL_D);
             uint32_t o[32];
-            dequant_q4k_regs(hdr, qa, qb, j0 + 2 * i, o);
-            store(o, i);
-            stored(i);
+            convert(j, 0, o);
+            slot_free();
+            put(o, 0);
+            if (C::WIDE) {
+                uint32_t p[32];
+                convert(j, C::WIDE ? 1 : 0, p);
+                put(p, 1);
+            }
+        };
+        // two projections: stage i of the group's one (wide) or two of a column
+        auto part_of_column = [&](int i) {
+            if (i == 0) ok &= mb_wait(&raw_full[slot], rph);
+            fetch(j0 + 2 * i, 0);
+            if (C::WIDE || i == 1) read();
+            stage_in(j0 + 2 * i);
+            stored();
         };
         GmTile T, next = gm_tile<CG>(P, tile0, n_tiles, rank);
-        if (NPROJ == 2 && tile0 < n_tiles) half(0);
+        if (NPROJ == 2 && tile0 < n_tiles) part_of_column(0);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, it++) {
             T = next;
             next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
             // (rows past the last one convert whatever the slot holds: their accumulator rows are never read)
-            if (DT == LMOE_Q6_K) sh = (int)(((int64_t)T.e * P.expert_bytes + (int64_t)(T.m0 + r) * row_bytes) & 15);
             if (NPROJ == 1) {
-                load(0);
-                for (int b = 0; b < n_blk && ok; b++) {
-                    uint32_t o[32];
-                    const uint32_t last = use & 1;
-                    if (DT == LMOE_Q4_K) dequant_q4k_regs(hdr, qa, qb, j0, o);
-                    else dequant_q6k_regs(F, part, o);
-                    store(o, last);
-                    if (b + 1 < n_blk) load(b + 1); // the next column's words arrive while the store completes
-                    stored(last);
+                // a wide stage is a whole column, and the groups take the columns in turn; else each takes its half of every column
+                const int b0 = C::WIDE ? (grp ^ ((int)it * n_blk)) & 1 : 0, bs = C::WIDE ? 2 : 1;
+                if (DT == LMOE_Q6_K) sh = (int)(((int64_t)T.e * P.expert_bytes + (int64_t)(T.m0 + r) * row_bytes) & 15) + b0 * Q6K_BYTES;
+                auto load = [&](int b) {
+                    ok &= mb_wait(&raw_full[slot], rph);
+                    fetch(j0, b);
+                    sh += bs * Q6K_BYTES;
+                    read();
+                };
+                if (b0 < n_blk) load(b0);
+                for (int b = b0; b < n_blk && ok; b += bs) {
+                    stage_in(j0);
+                    if (b + bs < n_blk) load(b + bs); // the next column's words arrive while the store completes
+                    stored();
                 }
             } else {
-                // a column's second stage, then the first one of the next column, which may be the next tile's: it is there when
+                // the rest of the tile's stages, then the first one of the next tile: it is there when
                 // that tile's multiplies may begin (96 / 512 / 4096 / 16384 tokens 391 / 526 / 1343 / 4487 us without, 387 / 521 /
                 // 1329 / 4447 so)
                 for (int b = 0; b < n_blk && ok; b++) {
-                    half(1);
-                    if (b + 1 < n_blk || tile + tile_step < n_tiles) half(0);
+                    if (!C::WIDE) part_of_column(1);
+                    if (b + 1 < n_blk || tile + tile_step < n_tiles) part_of_column(0);
                 }
             }
             if (NPROJ == 2) {
                 // this warp's share of the tile's epilogue: there is one accumulator set, so nothing is multiplied meanwhile
                 const int c0 = (warp - GM_DQ0) >> 2;
-                // (k = 256: a group could run a whole tile ahead, so every warp waits here)
-                if ((16 * c0 < T.nv || k_blocks <= 4) && ok) {
+                // (short rows: a group could run a whole tile ahead, so every warp waits here)
+                if ((16 * c0 < T.nv || k_blocks <= 8) && ok) {
                     ok &= mb_wait(&acc_full[0], it & 1);
                     tc_fence_after();
                     gm_epilogue<NPROJ, NT>(P, T, tmem_base, stage, q, lane, c0, 4);
@@ -893,7 +996,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             T = next;
             next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
             const int first = rank * gm_half<CG>(T.nv), brows = max(0, min(gm_half<CG>(T.nv), T.nv - first));
-            const uint32_t bytes = (uint32_t)brows * 128u, grp = (uint32_t)gm_b_group<NPROJ, NT, CG>(T.nv), sub = C::B_SLOT / grp;
+            const uint32_t bytes = (uint32_t)brows * 128u, grp = (uint32_t)gm_b_group<C::B_FULL, NT>(T.nv), sub = C::B_SLOT / grp;
             const uint8_t *src = P.xt + ((size_t)T.slot * k_blocks * NT + first) * 128;
             for (int kb = 0; kb < k_blocks && ok; kb += (int)grp) {
                 ok &= mb_wait(&b_empty[slot], ph ^ 1);
@@ -914,7 +1017,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             T = next;
             next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
-            const int grp = gm_b_group<NPROJ, NT, CG>(T.nv);
+            const int grp = gm_b_group<C::B_FULL, NT>(T.nv);
             for (int kb = 0; kb < k_blocks && ok; kb += grp) {
                 ok &= mb_wait(&b_full[slot], ph);
                 __syncwarp();
@@ -926,55 +1029,64 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
         // ---------------- MMA issuer of the pair: the whole warp walks the loop, one elected lane issues ----------------
         // A wait that finds its barrier complete still takes over a hundred cycles beside the converting warps, two or three of
         // them more than a thin tile's multiplies.  So the next stage's barriers are asked, without waiting, before this stage's
-        // multiplies are issued (512 tokens 514 -> 504 us, 1024 594 -> 581, op by op 512 849 -> 808).
+        // multiplies are issued (512 tokens 514 -> 504 us, 1024 594 -> 581, op by op 512 849 -> 808).  The blocks of a ring slot are
+        // a constant of the loop (there are up to three of it): with that and tc_mma_block, 512 tokens 475 -> 470, 1024 586 -> 579.
         const bool el = elect_one();
         const uint64_t bd0 = umma_desc(s32(b_st));
+        const uint32_t blo = (uint32_t)bd0, bhi = (uint32_t)(bd0 >> 32), a0 = tmem_base + C::A_COL0;
         uint32_t it = 0, bs = 0, bph = 0, as = 0, aph = 0; // tiles; slot and phase of the B ring and of the operand stages
         bool b_here = false, a_here = false; // they were seen to be full
         GmTile T, next = gm_tile<CG>(P, tile0, n_tiles, rank);
         for (int tile = tile0; tile < n_tiles && ok; tile += tile_step, it++) {
             T = next;
             next = gm_tile<CG>(P, tile + tile_step, n_tiles, rank);
-            const int npad = (T.nv + 15) & ~15;
-            const uint32_t grp = (uint32_t)gm_b_group<NPROJ, NT, CG>(T.nv), sub = (C::B_SLOT >> 4) / grp;
+            // (of one lane, so that the loop's operands are known to be the warp's)
+            const int nv = __shfl_sync(0xffffffffu, T.nv, 0);
+            const int npad = (nv + 15) & ~15;
             const uint32_t idesc = (1u << 4) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(CG * MM_M >> 4) << 24);
             const uint32_t buf = NPROJ == 2 ? 0u : it & 1, cph = NPROJ == 2 ? it & 1 : (it >> 1) & 1;
             ok &= mb_wait(&acc_empty[buf], cph ^ 1);
             const uint32_t d = tmem_base + buf * NT;
             // k is a multiple of 256: a tile has a multiple of four 64-k blocks
-            for (int kb = 0; kb < k_blocks && ok; kb += 4) {
+            auto multiply = [&](auto group) {
+                constexpr uint32_t GRP = decltype(group)::value, AB = C::A_BLKS, STEP = AB < GRP ? AB : GRP; // blocks between two waits
+                uint32_t first = 1;
+                for (int kb = 0; kb < k_blocks && ok; kb += 4) {
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const bool a_first = NPROJ == 2 || (u & 1) == 0, a_last = NPROJ == 2 || (u & 1) == 1;
-                    const uint32_t in = (uint32_t)u & (grp - 1); // block within its slot
-                    if (in == 0 && !b_here) ok &= mb_wait(&b_full[bs], bph);
-                    if (a_first && !a_here) ok &= mb_wait(&a_full[as], aph);
-                    tc_fence_after();
-                    const uint32_t a = tmem_base + C::A_COL0 + 64u * as + (a_first ? 0u : 32u);
-                    const uint64_t bd = bd0 + (uint64_t)(bs * (C::B_SLOT >> 4) + in * sub);
-                    const bool b_last = in == grp - 1;
-                    uint64_t *const b_done = &b_empty[bs], *const a_done = &a_empty[as];
-                    if (b_last) {
-                        if (++bs == C::NB) { bs = 0; bph ^= 1; }
-                        b_here = mb_test(&b_full[bs], bph);
-                    }
-                    if (a_last) {
-                        if (++as == C::NA) { as = 0; aph ^= 1; }
-                        a_here = mb_test(&a_full[as], aph);
-                    }
-                    if (el) {
-#pragma unroll
-                        for (int kk = 0; kk < 4; kk++) {
-                            const uint32_t acc = (u | kk) != 0 ? 1u : (kb != 0 ? 1u : 0u);
-                            tc_mma_f16_ts<CG>(d, a + 8 * kk, bd + 2 * kk, idesc, acc);
-                            if (NPROJ == 2) tc_mma_f16_ts<CG>(d + NT, a + 32 + 8 * kk, bd + 2 * kk, idesc, acc);
+                    for (uint32_t u = 0; u < 4; u += STEP) {
+                        if (C::NA * AB == 4) as = u / AB;
+                        if (u % GRP == 0 && !b_here) ok &= mb_wait(&b_full[bs], bph);
+                        if (u % AB == 0 && !a_here) ok &= mb_wait(&a_full[as], aph);
+                        tc_fence_after();
+                        const uint32_t a = a0 + C::A_COLS * as + (NPROJ == 2 ? 64u : 32u) * (u % AB);
+                        const uint32_t bl = blo + bs * (C::B_SLOT >> 4) + u % GRP * ((C::B_SLOT >> 4) / GRP);
+                        uint64_t *const b_done = &b_empty[bs], *const a_done = &a_empty[as];
+                        const bool b_last = (u + STEP) % GRP == 0, a_last = (u + STEP) % AB == 0;
+                        if (b_last) {
+                            if (++bs == C::NB) { bs = 0; bph ^= 1; }
+                            b_here = mb_test(&b_full[bs], bph);
                         }
-                        if (b_last) tc_commit<CG>(b_done);
-                        if (a_last) tc_commit<CG>(a_done);
+                        if (a_last) {
+                            if (++as == C::NA) { as = 0; aph ^= 1; }
+                            a_here = mb_test(&a_full[as], aph);
+                        }
+                        if (el) {
+#pragma unroll
+                            for (uint32_t i = 0; i < STEP; i++)
+                                tc_mma_block<CG, NPROJ == 2>(d, d + NT, a + (NPROJ == 2 ? 64u : 32u) * i, bl + i * ((C::B_SLOT >> 4) / GRP), bhi, idesc, u + i == 0 ? first : 0u);
+                            if (b_last) tc_commit<CG>(b_done);
+                            if (a_last) tc_commit<CG>(a_done);
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
+                    first = 0;
                 }
-            }
+            };
+            const int grp = gm_b_group<C::B_FULL, NT>(nv);
+            if (grp == 4) multiply(std::integral_constant<uint32_t, 4>{});
+            else if (C::B_FULL == 4) {}
+            else if (grp == 2) multiply(std::integral_constant<uint32_t, 2>{});
+            else if (C::B_FULL == 1) multiply(std::integral_constant<uint32_t, 1>{});
             if (el) tc_commit<CG>(&acc_full[buf]);
             __syncwarp();
         }
@@ -1013,7 +1125,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
             for (int i = 0; i < RPT; i++) off[i] = (uint32_t)nsrc[i] * row16 + ch;
             rows(next);
             const int n = brows(T);
-            const int grp = gm_b_group<NPROJ, NT, CG>(T.nv);
+            const int grp = gm_b_group<C::B_FULL, NT>(T.nv);
             const uint32_t sub = C::B_SLOT / grp;
             for (int kb = 0; kb < k_blocks && ok; kb += grp) {
                 ok &= mb_wait(&b_empty[slot], ph ^ 1);
@@ -1067,18 +1179,17 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
 
 // ---- host side ---------------------------------------------------------------------------
 // Routed rows per tile.  192 fills the tensor memory beside two accumulators with two operand stages and converts each
-// weight least often; with a few dozen rows per expert every tile is thin whatever its limit, and 128 leaves room for four
-// operand stages.  A block's forward with its shared expert, evenly routed, cold L2, both launches overlapped, us with 128 / 192 by rows
-// per expert:
-//                              8         16         24         32         40         48         64         80        160
-//   256 experts, 3072, 1024  423 / 422  479 / 478  528 / 508  563 / 561  594 / 603  675 / 636  768 / 740  869 / 821  1431 / 1282
-//   128 experts, 2048, 768   167 / 166  179 / 178  188 / 188  195 / 195  205 / 205  217 / 216  246 / 229  272 / 257   426 / 382
-//   64 experts, 4096, 1536   289 / 286  295 / 293  299 / 302  307 / 303  311 / 310  316 / 321  336 / 335  393 / 360   638 / 601
-//   64 experts, 2048, 512     96 / 96    96 / 96    97 / 100  100 / 100  100 / 102  104 / 107  113 / 112  131 / 120   188 / 173
-//   16 experts, 4096, 2048   148 / 145  150 / 150  148 / 156  154 / 154  184 / 160  180 / 160  188 / 193  201 / 199   315 / 287
-// From some 60 rows on 192 is the shorter one.  Below, most differ by less than 2 % and the others go either way, as the tallest lists
-// happen to fill a tile of one height or the other; the line lies where 128 no longer gains anything.
-int mm_tile_rows(int64_t rows, int64_t n_expert) { return rows <= 40 * n_expert ? 128 : 192; }
+// weight least often; with fewer rows per expert every tile is thin whatever its limit, and lower tiles leave room for wide operand
+// stages: two beside 128 rows, three beside 64.  A block's forward with its shared expert, evenly routed, cold L2, us with
+// 64 / 128 / 192 by rows per expert:
+//                              8                12                20                32                48                64                80
+//   256 experts, 3072, 1024  380 / 386 / 409  415 / 404 / 429  447 / 447 / 476  568 / 526 / 548  748 / 640 / 689  861 / 726 / 697  1033 / 863 / 818
+//   128 experts, 2048, 768   163 / 169 / 175  165 / 169 / 169  177 / 179 / 185  200 / 185 / 194  241 / 208 / 214  269 / 235 / 226  323 / 265 / 255
+//   64 experts, 4096, 1536         -          263 / 269 / 279  269 / 273 / 290  277 / 283 / 298  349 / 298 / 314  403 / 327 / 331  466 / 380 / 357
+//   64 experts, 2048, 512          -           93 / 95 / 97     93 / 93 / 98     99 / 97 / 101   116 / 101 / 107  124 / 110 / 112  142 / 128 / 120
+//   16 experts, 4096, 2048         -                 -         136 / 142 / 144  138 / 146 / 150  167 / 148 / 159  206 / 157 / 161  216 / 189 / 167
+// (Near the lines the tallest lists decide: how many of them just pass a tile's height.)
+int mm_tile_rows(int64_t rows, int64_t n_expert) { return rows <= 20 * n_expert ? 64 : (rows <= 50 * n_expert ? 128 : 192); }
 
 // Row tiles that `rows` routed rows over n_lists lists can make.
 static int64_t mm_max_row_tiles(int64_t rows, int64_t n_lists, int nt) { return (rows + nt - 1) / nt + n_lists; }
@@ -1271,11 +1382,13 @@ lmoe_status launch_mm_id(const MmRows &R, const lmoe_expert_stack *st, const lmo
                          uint32_t *flag, cudaStream_t stream) {
     const int64_t blocks = (st->n_out + MM_M - 1) / MM_M;
     if ((blocks & 1) && blocks <= GM_SINGLE_BLOCKS) {
-        auto fn = R.nt == 128 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128, 1> : launch_grouped<LMOE_Q6_K, 1, 128, 1>)
+        auto fn = R.nt == 64 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 64, 1> : launch_grouped<LMOE_Q6_K, 1, 64, 1>)
+                  : R.nt == 128 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128, 1> : launch_grouped<LMOE_Q6_K, 1, 128, 1>)
                               : (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 192, 1> : launch_grouped<LMOE_Q6_K, 1, 192, 1>);
         return fn(R, {st, nullptr}, {shared, nullptr}, xt, nullptr, ids_map, map_stride, row_scale, out, sorted, tiles_ws, flag, stream);
     }
-    auto fn = R.nt == 128 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128, 2> : launch_grouped<LMOE_Q6_K, 1, 128, 2>)
+    auto fn = R.nt == 64 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 64, 2> : launch_grouped<LMOE_Q6_K, 1, 64, 2>)
+              : R.nt == 128 ? (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 128, 2> : launch_grouped<LMOE_Q6_K, 1, 128, 2>)
                           : (st->dtype == LMOE_Q4_K ? launch_grouped<LMOE_Q4_K, 1, 192, 2> : launch_grouped<LMOE_Q6_K, 1, 192, 2>);
     return fn(R, {st, nullptr}, {shared, nullptr}, xt, nullptr, ids_map, map_stride, row_scale, out, sorted, tiles_ws, flag, stream);
 }
@@ -1286,6 +1399,6 @@ lmoe_status launch_mm_gateup(const MmRows &R, const lmoe_expert_stack *gate, con
                              int sorted, void *tiles_ws, uint32_t *flag, cudaStream_t stream) {
     if (gate->dtype != LMOE_Q4_K || up->dtype != LMOE_Q4_K)
         return lmoe_fail(LMOE_ERR_UNSUPPORTED, "the fused gate/up kernel is built for Q4_K stacks");
-    auto fn = R.nt == 128 ? launch_grouped<LMOE_Q4_K, 2, 128, 2> : launch_grouped<LMOE_Q4_K, 2, 192, 2>;
+    auto fn = R.nt == 64 ? launch_grouped<LMOE_Q4_K, 2, 64, 2> : R.nt == 128 ? launch_grouped<LMOE_Q4_K, 2, 128, 2> : launch_grouped<LMOE_Q4_K, 2, 192, 2>;
     return fn(R, {gate, up}, {sh_gate, sh_up}, xh, src, ids_map, map_stride, nullptr, act, sorted, tiles_ws, flag, stream);
 }

@@ -62,12 +62,70 @@ def test_mm_ragged_rows_multi_block_k_and_big_expert(orc, dev, dt, name):
 @pytest.mark.parametrize("dt,name", DTYPES)
 @pytest.mark.parametrize("t,n_out,k", [(80, 128, 256), (82, 130, 1280), (257, 124, 512), (81, 131, 768)])
 def test_mm_tile_shapes(orc, dev, dt, name, t, n_out, k):
-    """Both row-tile widths on either side of their rule (40 and 41 rows an expert), a row past a tile, row counts of the matrix
+    """40 and 41 rows an expert and a row past a tile, row counts of the matrix
     that are no multiple of the copy's eight rows or of four, more than four super-blocks.  Both operands are rounded to f16
     (2^-11 each), sums are f32: well under 1e-3."""
     ids = (np.arange(t, dtype=np.uint32) % 2)[:, None]
     got, want = _case(orc, dev, dt, 2, n_out, k, t, 1, 1, ids, 0x90 + t)
     assert orc.rel_l2(got, want) < 1e-3
+
+
+@pytest.mark.parametrize("dt,name", DTYPES)
+@pytest.mark.parametrize("per_expert", [20, 21, 50, 51])
+@pytest.mark.parametrize("n_out,k", [(128, 256), (256, 768), (384, 512)])
+def test_mm_tile_heights(orc, dev, dt, name, per_expert, n_out, k):
+    """Row tiles of 64, 128 and 192 rows on either side of their rule, in single CTAs (odd numbers of 128 weight rows) and in pairs, rows
+    of one, two and three blocks (which the groups of a wide stage take in turn), lists that just fit a tile and that just do not.  Bound as in
+    test_mm_tile_shapes."""
+    counts = [63, 64, 65, 1, 0, 16, 17, 129]
+    counts += [0] * 4
+    counts[-1] = per_expert * len(counts) - sum(counts) if per_expert * len(counts) >= sum(counts) else 0
+    counts += [0] * (-(-sum(counts) // per_expert) - len(counts))
+    ids = np.repeat(np.arange(len(counts), dtype=np.uint32), counts)[np.random.default_rng(per_expert).permutation(sum(counts))][:, None]
+    got, want = _case(orc, dev, dt, len(counts), n_out, k, sum(counts), 1, 1, ids, 0xC0)
+    assert orc.rel_l2(got, want) < 1e-3
+
+
+@pytest.mark.parametrize("ne", [16, 8, 2])
+@pytest.mark.parametrize("dt,name", DTYPES)
+def test_mm_operand_bits(dev, dt, name, ne):
+    """One-hot activations give the f16 operands themselves.  Both forms of the conversion: a warp's 32 rows all with a small d, all but
+    one (at the line itself), all just below the line, all large and of either sign.  Scale and offset are rounded to f16 once and the
+    weight once, so the bits are known.  Tiles of 64, 128 and 192 rows."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    rng = np.random.default_rng(dt)
+    line = 2.0 ** -10 if dt == 12 else 2.0 ** -13
+    below = np.nextafter(np.float16(line), np.float16(0))
+    d = np.concatenate([rng.uniform(0.55, 0.95, 32) * line, rng.uniform(0.55, 0.95, 32) * line, np.full(32, below),
+                        rng.uniform(1.0, 64.0, 32) * line * rng.choice([-1.0, 1.0], 32)]).astype(np.float16)
+    d[40] = line
+    b = rng.integers(0, 256, (128, 144 if dt == 12 else 210), dtype=np.uint8)
+    w = np.zeros((128, 256))
+    if dt == 12:
+        b[:, 0:2] = d[:, None].view(np.uint8)
+        dmin = (rng.uniform(-1.0, 1.0, 128) * 0.01).astype(np.float16)
+        b[:, 2:4] = dmin[:, None].view(np.uint8)
+        q = b[:, 4:16].astype(np.int32)
+        for j in range(8):
+            sc, mn = (q[:, j] & 63, q[:, j + 4] & 63) if j < 4 else ((q[:, j + 4] & 15) | (q[:, j - 4] >> 6) << 4, (q[:, j + 4] >> 4) | (q[:, j] >> 6) << 4)
+            s, m = (d.astype(np.float64) * sc).astype(np.float16), (-dmin.astype(np.float64) * mn).astype(np.float16)
+            n = (b[:, 16 + 32 * (j // 2):48 + 32 * (j // 2)] >> (4 * (j & 1))) & 15
+            w[:, 32 * j:32 * j + 32] = n * s.astype(np.float64)[:, None] + m.astype(np.float64)[:, None]
+    else:
+        b[:, 208:210] = d[:, None].view(np.uint8)
+        for n in range(2):
+            for g in range(4):
+                lo = (b[:, 64 * n + 32 * (g & 1):64 * n + 32 * (g & 1) + 32] >> (4 * (g >> 1))) & 15
+                hi = (b[:, 128 + 32 * n:160 + 32 * n] >> (2 * g)) & 3
+                sc = np.repeat(b[:, 192 + 8 * n + 2 * g:194 + 8 * n + 2 * g].view(np.int8).astype(np.float64), 16, axis=1)
+                s = (d.astype(np.float64)[:, None] * sc).astype(np.float16).astype(np.float64)
+                w[:, 128 * n + 32 * g:128 * n + 32 * g + 32] = ((lo | hi << 4).astype(np.float64) - 32.0) * s
+    want = w.astype(np.float16).astype(np.float32)
+    st = ExpertStack.from_bytes(np.concatenate([b.reshape(-1)] * ne), dt, ne, 128, 256, device=dev)
+    got = ops.mul_mm_id(st, torch.eye(256, device=dev).view(256, 1, 256), torch.zeros(256, 1, dtype=torch.int32, device=dev))
+    assert np.array_equal(got.cpu().numpy()[:, 0].T, want)
 
 
 @pytest.mark.parametrize("n_out,k", [(6, 256), (130, 512), (128, 512), (131, 1024), (198, 1024), (129, 2048), (256, 2048), (64, 3072)])
@@ -137,6 +195,17 @@ def test_prefill_block_tiny(orc, dev):
     want, _, _ = host.forward(x)
     got = blk.forward_unfused(torch.from_numpy(x).to(dev), use_mm=True).cpu().numpy()
     assert orc.rel_l2(got, want) < 2e-3
+
+
+@pytest.mark.parametrize("hidden,ff", [(256, 256), (512, 768), (768, 256)])
+@pytest.mark.parametrize("t", [80, 81, 200, 201])
+def test_prefill_block_tile_heights(orc, dev, hidden, ff, t):
+    """The fused gate/up product on either side of the rule for row tiles (20 and 50 rows an expert), with rows of one, two and three
+    blocks in both products.  Bound as above."""
+    from maxuna_b200.moe import MoeBlock
+
+    blk = MoeBlock.random(hidden, ff, 8, 2, seed=hidden + ff, device=dev, weight_std=0.1)
+    _check_block(orc, blk, blk.host_layer(orc), np.random.default_rng(t).standard_normal((t, hidden)).astype(np.float32), 2e-3)
 
 
 def test_prefill_block_wide_ff(orc, dev):
