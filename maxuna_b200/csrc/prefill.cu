@@ -390,12 +390,20 @@ static lmoe_status experts_prefill(const lmoe_layer *L, const void *x, int x_f16
     return LMOE_OK;
 }
 
+// Routing through route_filter.cu once the f32 product is the longer one (a block's forward, cold L2, us without / with: hidden 3072, 256
+// experts, 512 / 768 / 1024 / 2048 / 4096 / 16384 tokens 463 / 465, 512 / 500, 557 / 536, 806 / 745, 1295 / 1194, 4550 / 3919; hidden 2048,
+// 128 experts, 800 / 1600 / 4000 tokens 257 / 289, 352 / 325, 570 / 554).
+static bool prefill_filters(const lmoe_layer *L, int64_t t) {
+    return (double)t * L->n_expert * L->hidden >= 5e8 && route_filter_available(L->hidden, L->n_expert, L->top_k);
+}
+
 size_t prefill_workspace_bytes(const lmoe_layer *L, int64_t t) {
     if (t < 1) t = 1;
     const int64_t rows = t * L->top_k;
     size_t o = 65536;
     o += lmoe_align_up((size_t)t * L->n_expert * 4, 256);            // logits
     o += 2 * lmoe_align_up((size_t)rows * 4, 256);                   // ids, weights
+    if (prefill_filters(L, t)) o += route_filter_bytes(t, L->hidden, L->n_expert);
     o += experts_ws_bytes(L, t, L->top_k);
     return o;
 }
@@ -414,11 +422,17 @@ lmoe_status launch_moe_prefill(const lmoe_layer *L, const float *x, const float 
     float *logits = c.take<float>((size_t)t * L->n_expert);
     uint32_t *ids = c.take<uint32_t>((size_t)rows);
     float *w = c.take<float>((size_t)rows);
+    uint8_t *rf_ws = c.take<uint8_t>(prefill_filters(L, t) ? route_filter_bytes(t, H, L->n_expert) : 0);
+    const bool filter = prefill_filters(L, t) && ((reinterpret_cast<uintptr_t>(L->router) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0;
     uint8_t *ex_ws = static_cast<uint8_t *>(workspace) + c.off;
 
-    LMOE_CUDA(launch_route_logits(L->router, x, (int)t, (int)H, (int)L->n_expert, logits, s));
-    LMOE_CUDA(launch_route_select(logits, L->bias, (int)t, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, ids, w, s,
-                                  flag)); // a fresh device flag: the workspace needs no initialisation
+    // (both begin with a fresh device flag: the workspace needs no initialisation)
+    if (filter) {
+        LMOE_CUDA(launch_route_filter(L->router, L->bias, x, (int)t, (int)H, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, logits, rf_ws, ids, w, flag, s));
+    } else {
+        LMOE_CUDA(launch_route_logits(L->router, x, (int)t, (int)H, (int)L->n_expert, logits, s));
+        LMOE_CUDA(launch_route_select(logits, L->bias, (int)t, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, ids, w, s, flag));
+    }
     lmoe_status st = experts_prefill(L, x, 0, ids, w, t, L->top_k, 0, 1, residual, out, ex_ws, flag, s);
     if (st) return st;
     if (ids_out) LMOE_CUDA(cudaMemcpyAsync(ids_out, ids, (size_t)rows * 4, cudaMemcpyDeviceToDevice, s));

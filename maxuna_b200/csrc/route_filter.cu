@@ -1,0 +1,455 @@
+// Routing of long prompts: the tensor core says which experts can be among a token's top_k, and only those get the specified
+// f32 logit.  Ids and weights are those of route.cu to the bit.
+// Reference: `route_logits` and `route_from_logits`, src/moe.rs:84-119.
+//
+// The specified logits (route_math.cuh) are f32 products in a fixed order: for 16384 tokens, 256 experts and hidden 3072 they and the selection
+// take 730 us at half of the f32 rate, for 2048 tokens 115.  This takes 290 and 65: 5 for the router's f16 image, 43 / 22 for the approximate product
+// (16384 tokens: the tokens from memory at 4.7 TB/s), 240 / 38 for the rest (the router rows from the L2 cache).  A product of the operands rounded to f16 differs from it by at most
+//   |x| |w| (2^-10 + 2^-12) + 2^-25 sqrt(hidden) (|x| + |w|)
+// (2^-11 for the rounding of either operand by Cauchy's inequality, 2^-12 for the f32 sums of 3072 products in the tensor core, which rounds
+// or cuts once in 16, and for the specified sum, whose own error is 2^-19; the last term for values below the f16 range), so it bounds every score, and an expert whose
+// upper bound is below the top_k-th largest lower bound is out.  13 of 256 experts are left for a token of the benchmark's
+// router.  A token with a bound that is not finite (an operand beyond the f16 range, an infinity, NaN) keeps all its experts.
+#include <math.h>
+#include <type_traits>
+
+#include "fused.cuh"
+#include "route_math.cuh"
+#include "tc.cuh"
+
+namespace {
+
+constexpr int RF_A_BYTES = 128 * 128; // 128 tokens x 64 values as f16
+__host__ __device__ constexpr int rf_stages(int tm) { return tm == 64 ? 6 : 4; }
+constexpr int RF_AHEAD = 3; // stages whose words a producing thread has in flight
+
+// The router as f16 in the order of the B operand's stages (64 values of all experts: a 128-byte-swizzled tile), and its rows' norms.
+// A block per expert.  clear: the call's device flag.
+__global__ void __launch_bounds__(128) route_prep_kernel(const float *__restrict__ router, int hidden, int n_expert, uint8_t *__restrict__ img,
+                                                         float *__restrict__ wnorm, uint32_t *__restrict__ clear) {
+    pdl_begin();
+    const int e = blockIdx.x;
+    if (clear && e == 0 && threadIdx.x < 4) clear[threadIdx.x] = 0u;
+    const float4 *w = reinterpret_cast<const float4 *>(router + (size_t)e * hidden);
+    float ss = 0.f;
+    for (int ci = threadIdx.x; ci < hidden / 8; ci += 128) {
+        const float4 a = __ldg(w + 2 * ci), b = __ldg(w + 2 * ci + 1);
+        ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w + b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
+        __align__(16) __half2 h[4] = {__floats2half2_rn(a.x, a.y), __floats2half2_rn(a.z, a.w), __floats2half2_rn(b.x, b.y),
+                                      __floats2half2_rn(b.z, b.w)};
+        *reinterpret_cast<uint4 *>(img + ((size_t)(ci >> 3) * n_expert + e) * 128 + (((ci & 7) ^ (e & 7)) << 4)) = *reinterpret_cast<const uint4 *>(h);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    __shared__ float part[4];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    if (threadIdx.x == 0) wnorm[e] = sqrtf(part[0] + part[1] + part[2] + part[3]);
+}
+
+// Approximate logits of TM tokens (the M of the multiplies is 128; rows past the last token are whatever lies there, and nothing reads
+// their results) and `ne` experts from blockIdx.y * ne on: eight warps round the tokens to f16 and put them into the A stages, warp 8
+// issues the multiplies, warp 9 copies the B stages, warps 0-3 take the results out of tensor memory.  blockIdx.y = 0 writes the tokens' norms.
+template <int TM>
+__global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__restrict__ x, const uint8_t *__restrict__ img, int t, int hidden, int n_expert,
+                                                              int ne, float *__restrict__ logits, float *__restrict__ xnorm, uint32_t *__restrict__ flag) {
+    constexpr int RF_STAGES = rf_stages(TM), GROUPS = TM == 64 ? 2 : 1; // groups of producing warps, which take the stages in turn
+    extern __shared__ uint8_t rf_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(rf_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t a_full[RF_STAGES], b_full[RF_STAGES], empty[RF_STAGES], done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ float sums[TM];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, steps = hidden / 64;
+    const int t0 = blockIdx.x * TM, nt = min(TM, t - t0), e0 = blockIdx.y * ne;
+    const uint32_t b_bytes = (uint32_t)ne * 128u;
+    uint8_t *a_st = smem, *b_st = smem + RF_STAGES * RF_A_BYTES;
+    if (tid == 0) {
+        for (int s = 0; s < RF_STAGES; s++) {
+            mb_init(&a_full[s], 8 / GROUPS);
+            mb_init(&b_full[s], 1);
+            mb_init(&empty[s], 1);
+        }
+        mb_init(&done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 8) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&tmem_slot)), "r"(256u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_begin();
+    bool ok = true;
+    if (warp < 8) {
+        constexpr int THREADS = 256 / GROUPS, RS = THREADS / 8, NC = TM / RS; // 8-value chunks of a thread and stage: one of rows r0, r0 + RS, ...
+        const int grp = tid / THREADS, ch = tid & 7, r0 = tid % THREADS >> 3;
+        const float4 *src[NC];
+        uint8_t *dst[NC];
+        float ss[NC];
+#pragma unroll
+        for (int i = 0; i < NC; i++) {
+            const int r = r0 + RS * i;
+            src[i] = reinterpret_cast<const float4 *>(x + (size_t)(t0 + min(r, nt - 1)) * hidden) + 2 * ch;
+            dst[i] = a_st + r * 128 + ((ch ^ (r & 7)) << 4);
+            ss[i] = 0.f;
+        }
+        float4 v[RF_AHEAD][NC][2];
+        auto load = [&](int u, int s) {
+#pragma unroll
+            for (int i = 0; i < NC; i++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) v[u][i][h] = s < steps ? __ldg(src[i] + 16 * s + h) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+#pragma unroll
+        for (int u = 0; u < RF_AHEAD; u++) load(u, grp + GROUPS * u);
+        uint32_t st = grp, ph = 0;
+        for (int s0 = grp; s0 < steps && ok; s0 += GROUPS * RF_AHEAD) {
+#pragma unroll
+            for (int u = 0; u < RF_AHEAD; u++) {
+                if (s0 + GROUPS * u >= steps) break;
+                ok &= mb_wait(&empty[st], ph ^ 1);
+#pragma unroll
+                for (int i = 0; i < NC; i++) {
+                    const float4 a = v[u][i][0], b = v[u][i][1];
+                    ss[i] += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w + b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
+                    __align__(16) __half2 h[4] = {__floats2half2_rn(a.x, a.y), __floats2half2_rn(a.z, a.w), __floats2half2_rn(b.x, b.y),
+                                                  __floats2half2_rn(b.z, b.w)};
+                    *reinterpret_cast<uint4 *>(dst[i] + st * RF_A_BYTES) = *reinterpret_cast<const uint4 *>(h);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mb_arrive(&a_full[st]);
+                if ((st += GROUPS) >= RF_STAGES) { st -= RF_STAGES; ph ^= 1; }
+                load(u, s0 + GROUPS * (u + RF_AHEAD));
+            }
+        }
+        if (blockIdx.y == 0) { // (the groups' shares meet in shared memory)
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+#pragma unroll
+                for (int o = 4; o; o >>= 1) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o);
+                if (GROUPS == 2 && grp == 1 && ch == 0) sums[r0 + RS * i] = ss[i];
+            }
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+                const int r = r0 + RS * i;
+                if (grp == 0 && ch == 0 && r < nt) xnorm[t0 + r] = sqrtf(GROUPS == 2 ? ss[i] + sums[r] : ss[i]);
+            }
+        }
+        if (warp < 4) { // a lane is a token
+            ok &= mb_wait(&done, 0);
+            tc_fence_after();
+            const int r = 32 * warp + lane;
+            float *dstl = logits + (size_t)(t0 + r) * n_expert + e0;
+            if (32 * warp < nt)
+                for (int c = 0; c < ne; c += 16) {
+                    uint32_t o[16];
+                    tc_ld16(tmem + ((uint32_t)(32 * warp) << 16) + c, o);
+                    tc_wait_ld();
+                    if (r < nt) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) *reinterpret_cast<uint4 *>(dstl + c + 4 * i) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+                    }
+                }
+            tc_fence_before();
+        }
+    } else if (warp == 8) {
+        const bool el = elect_one();
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(ne >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        uint32_t st = 0, ph = 0;
+        for (int s = 0; s < steps && ok; s++) {
+            ok &= mb_wait(&b_full[st], ph);
+            ok &= mb_wait(&a_full[st], ph);
+            tc_fence_after();
+            if (el) {
+                const uint64_t ad = umma_desc(s32(a_st + st * RF_A_BYTES)), bd = umma_desc(s32(b_st + st * b_bytes));
+#pragma unroll
+                for (int kk = 0; kk < 4; kk++)
+                    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem), "l"(ad + 2 * kk), "l"(bd + 2 * kk), "r"(idesc),
+                                 "r"((uint32_t)(s | kk)) : "memory");
+                tc_commit<1>(&empty[st]);
+            }
+            __syncwarp();
+            if (++st == RF_STAGES) { st = 0; ph ^= 1; }
+        }
+        if (el) tc_commit<1>(&done);
+        __syncwarp();
+        ok &= mb_wait(&done, 0); // none is in flight when the tensor memory is given back
+    } else if (warp == 9) {
+        const bool el = elect_one();
+        uint32_t st = 0, ph = 0;
+        for (int s = 0; s < steps && ok; s++) {
+            ok &= mb_wait(&empty[st], ph ^ 1);
+            if (el) {
+                mb_expect_tx(&b_full[st], b_bytes);
+                bulk_g2s(b_st + st * b_bytes, img + ((size_t)s * n_expert + e0) * 128, b_bytes, &b_full[st]);
+            }
+            __syncwarp();
+            if (++st == RF_STAGES) { st = 0; ph ^= 1; }
+        }
+        // the copies have landed: slots below st in the present turn of the ring, the others in the turn before
+        for (uint32_t i = 0; i < RF_STAGES; i++) {
+            const bool here = mb_wait(&b_full[i], i < st ? ph : ph ^ 1);
+            ok &= here;
+            if (!here) break;
+        }
+    }
+    if (!ok && lane == 0 && atomicCAS(flag, 0u, (uint32_t)LMOE_FLAG_WAIT_TIMEOUT) == 0u) {
+        flag[1] = 0x2000u + warp;
+        flag[2] = blockIdx.x;
+    }
+    __syncthreads();
+    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+}
+
+// The specified logits of the experts that the approximate ones leave, then the selection: a block of TB tokens, whose rows lie in
+// shared memory.  The experts left for any of them are taken in turn by sixteen warps, each router row once for up to
+// four tokens: 146 rows for the 212 logits of sixteen tokens.  The rows from the L2 cache are what bounds it (16384 tokens: 1.8 GB; with each piece
+// of a row waited for before the next is asked for 424 us; with sixteen exact sigmoids a lane for the bounds and selection by rounds 297; so 240).
+constexpr int RV_WARPS = 16, RV_TOKENS = 4, RV_PIECE = 8;
+constexpr uint32_t RV_OUT = 0xffa5a5a5u; // in place of the logit of an expert that is out: a NaN that no operation results in
+
+template <int TB, int PER>
+__global__ void __launch_bounds__(RV_WARPS * 32, 1)
+route_verify_kernel(const float *__restrict__ router, const float *__restrict__ x, const float *__restrict__ bias, const float *__restrict__ approx,
+                    const float *__restrict__ xnorm, const float *__restrict__ wnorm, int t, int hidden, int n_expert, int top_k, float scale, int norm,
+                    uint32_t *__restrict__ ids, float *__restrict__ weights) {
+    extern __shared__ __align__(16) uint8_t rv_raw[];
+    float4 *xs = reinterpret_cast<float4 *>(rv_raw);
+    float *lg = reinterpret_cast<float *>(rv_raw + (size_t)TB * hidden * 4); // [token][expert]
+    uint32_t *items = reinterpret_cast<uint32_t *>(lg + TB * n_expert);        // expert << 16 | tokens
+    uint32_t *mask = items + (TB + RV_TOKENS - 1) / RV_TOKENS * n_expert;    // by expert: the tokens it is left for
+    __shared__ int n_items;
+    __shared__ __align__(16) uint16_t cand[TB][32 + 64]; // by token: the experts left, up to 32, and room for their probabilities
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row4 = hidden / 4;
+    const int t0 = blockIdx.x * TB, nt = min(TB, t - t0);
+    if (tid == 0) n_items = 0;
+    for (int e = tid; e < n_expert; e += RV_WARPS * 32) mask[e] = 0u;
+    pdl_begin();
+    for (int i = tid; i < nt * row4; i += RV_WARPS * 32)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s32(xs + i)), "l"(reinterpret_cast<const float4 *>(x + (size_t)t0 * hidden) + i) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    __syncthreads();
+    int left = 0; // experts left for the warp's token
+    if (warp < nt) { // a warp's token: bounds of its scores
+        const int tok = t0 + warp;
+        float lo[PER], hi[PER], l[PER], W[PER], b[PER];
+        bool finite = true;
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const int e = min(lane + 32 * j, n_expert - 1);
+            l[j] = approx[(size_t)tok * n_expert + e];
+            W[j] = wnorm[e] * 1.001f;
+            b[j] = bias ? __ldg(bias + e) : 0.f;
+        }
+        const float X = xnorm[tok] * 1.001f, sub = 0x1p-25f * 1.01f * sqrtf((float)hidden);
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            // (a sigmoid from the hardware's exponential and reciprocal is good to 1e-6, sums round by less)
+            const float d = X * W[j] * (0x1p-10f + 0x1p-12f) + sub * (X + W[j]), eps = 4e-6f * (1.f + fabsf(b[j]));
+            lo[j] = __fdividef(1.f, 1.f + __expf(d - l[j])) + b[j] - eps;
+            hi[j] = __fdividef(1.f, 1.f + __expf(-d - l[j])) + b[j] + eps;
+            finite = finite && isfinite(l[j]) && isfinite(d) && isfinite(lo[j]) && isfinite(hi[j]);
+        }
+        const bool all = !__all_sync(0xffffffffu, finite);
+        uint32_t key[PER], kth = 0u; // the top_k-th largest lower bound
+#pragma unroll
+        for (int j = 0; j < PER; j++) key[j] = lane + 32 * j < n_expert ? lmoe_score_key(lo[j]) : 0u;
+        for (int k = 0; k < top_k; k++) {
+            uint32_t best = 0u;
+#pragma unroll
+            for (int j = 0; j < PER; j++) best = max(best, key[j]);
+            kth = __reduce_max_sync(0xffffffffu, best);
+            bool take = lane == __ffs(__ballot_sync(0xffffffffu, best == kth)) - 1; // one of them is taken
+#pragma unroll
+            for (int j = 0; j < PER; j++) {
+                const bool hit = take && key[j] == kth;
+                key[j] = hit ? 0u : key[j];
+                take = take && !hit;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const int e = lane + 32 * j;
+            const bool in = e < n_expert && (all || lmoe_score_key(hi[j]) >= kth);
+            const uint32_t who = __ballot_sync(0xffffffffu, in);
+            if (e < n_expert && !in) lg[warp * n_expert + e] = __uint_as_float(RV_OUT);
+            if (in) {
+                const int at = left + __popc(who & ((1u << lane) - 1u));
+                if (at < 32) cand[warp][at] = (uint16_t)e;
+                atomicOr(&mask[e], 1u << warp);
+            }
+            left += __popc(who);
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < n_expert; e += RV_WARPS * 32) {
+        uint32_t m = mask[e];
+        const int groups = (__popc(m) + RV_TOKENS - 1) / RV_TOKENS;
+        if (!groups) continue;
+        const int at = atomicAdd(&n_items, groups);
+        for (int g = 0; g < groups; g++) {
+            uint32_t part = 0u;
+            for (int i = 0; i < RV_TOKENS && m; i++) {
+                part |= m & (0u - m);
+                m &= m - 1u;
+            }
+            items[at + g] = (uint32_t)e << 16 | part;
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // A warp's items in turn, a router row in pieces of RV_PIECE passes: the next piece, this item's or the next one's first, is on its way while
+    // one is multiplied.  The specified order: chains 4 lane .. 4 lane + 3, their elements in turn.
+    const int n = n_items, steps = hidden / 128, pieces = (steps + RV_PIECE - 1) / RV_PIECE;
+    if (warp < n) {
+        float4 wa[RV_PIECE], wb[RV_PIECE];
+        float acc[RV_TOKENS][4];
+        int i = warp, piece = 0;
+        uint32_t item = items[i];
+        const float4 *w = reinterpret_cast<const float4 *>(router + (size_t)(item >> 16) * hidden) + lane;
+        auto load = [&](float4 (&v)[RV_PIECE], const float4 *row, int p) {
+#pragma unroll
+            for (int u = 0; u < RV_PIECE; u++)
+                if (p * RV_PIECE + u < steps) v[u] = __ldg(row + 32 * (p * RV_PIECE + u));
+        };
+        auto multiply = [&](const float4 (&v)[RV_PIECE], float4 (&after)[RV_PIECE]) { // false: that was the last piece
+            const bool last = piece + 1 == pieces, more = i + RV_WARPS < n;
+            const uint32_t now = item;
+            const int p = piece;
+            if (!last) {
+                load(after, w, ++piece);
+            } else if (more) {
+                item = items[i += RV_WARPS];
+                w = reinterpret_cast<const float4 *>(router + (size_t)(item >> 16) * hidden) + lane;
+                load(after, w, piece = 0);
+            }
+            uint32_t m = now & 0xffffu;
+#pragma unroll
+            for (int c = 0; c < RV_TOKENS; c++) {
+                if (m) {
+                    const int tk = __ffs(m) - 1;
+                    m &= m - 1u;
+                    const float4 *xp = xs + tk * row4 + 32 * p * RV_PIECE + lane;
+                    if (p == 0) acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0.f;
+#pragma unroll
+                    for (int u = 0; u < RV_PIECE; u++)
+                        if (p * RV_PIECE + u < steps) {
+                            const float4 xv = xp[32 * u];
+                            acc[c][0] = __fmaf_rn(xv.x, v[u].x, acc[c][0]);
+                            acc[c][1] = __fmaf_rn(xv.y, v[u].y, acc[c][1]);
+                            acc[c][2] = __fmaf_rn(xv.z, v[u].z, acc[c][2]);
+                            acc[c][3] = __fmaf_rn(xv.w, v[u].w, acc[c][3]);
+                        }
+                    if (last) {
+                        const float l = lmoe_router_fold(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+                        if (lane == 0) lg[tk * n_expert + (now >> 16)] = l;
+                    }
+                }
+            }
+            return !last || more;
+        };
+        load(wa, w, 0);
+        while (multiply(wa, wb) && multiply(wb, wa)) {}
+    }
+    __syncthreads();
+    if (warp >= nt) return;
+    uint32_t *ids_row = ids + (size_t)(t0 + warp) * top_k;
+    float *w_row = weights + (size_t)(t0 + warp) * top_k, *probs = lg + warp * n_expert;
+    if (left <= 32) {
+        // a lane an expert: its slot is the number of those before it (a larger score, or the same and a lower index)
+        const int e = lane < left ? cand[warp][lane] : 0;
+        const float p = lane < left ? lmoe_sigmoid_fixed(probs[e]) : 0.f;
+        const uint32_t key = lane < left ? lmoe_score_key(bias ? __fadd_rn(p, __ldg(bias + e)) : p) : 0u;
+        int slot = 0;
+        for (int i = 0; i < left; i++) { // (the list is in the order of the indices)
+            const uint32_t other = __shfl_sync(0xffffffffu, key, i);
+            slot += other > key || (other == key && i < lane);
+        }
+        const bool mine = lane < left && slot < top_k;
+        float *by_slot = reinterpret_cast<float *>(cand[warp]) + 16; // behind the list: 32 floats
+        if (mine) by_slot[slot] = p;
+        __syncwarp();
+        float w = p;
+        if (norm) {
+            float sum = 0.0f;
+            for (int k = 0; k < top_k; k++) sum = __fadd_rn(sum, by_slot[k]);
+            sum = sum < 6.103515625e-5f ? 6.103515625e-5f : sum;
+            w = __fdiv_rn(w, sum);
+        }
+        if (scale != 0.0f && scale != 1.0f) w = __fmul_rn(w, scale);
+        if (mine) {
+            ids_row[slot] = (uint32_t)e;
+            w_row[slot] = w;
+        }
+        return;
+    }
+    // as in route_select_kernel; the experts that are out do not exist
+    uint32_t key[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int e = lane + 32 * j;
+        key[j] = 0u;
+        if (e < n_expert) {
+            const float v = probs[e];
+            if (__float_as_uint(v) != RV_OUT) {
+                const float p = lmoe_sigmoid_fixed(v);
+                probs[e] = p;
+                key[j] = lmoe_score_key(bias ? __fadd_rn(p, __ldg(bias + e)) : p);
+            }
+        }
+    }
+    __syncwarp();
+    lmoe_warp_select_keys<PER>(key, probs, top_k, scale, norm, ids_row, w_row, lane);
+}
+
+int rv_smem(int tb, int64_t hidden, int64_t n_expert) { return (int)(tb * hidden * 4 + tb * n_expert * 4 + (tb + RV_TOKENS - 1) / RV_TOKENS * n_expert * 4 + n_expert * 4); }
+
+} // namespace
+
+// Whether the filter serves these sizes (hidden a whole number of the specified passes, experts a whole tile of the tensor core).
+bool route_filter_available(int64_t hidden, int64_t n_expert, int64_t top_k) {
+    return hidden % 128 == 0 && hidden >= 512 && hidden <= 4096 && n_expert % 32 == 0 && n_expert >= 64 && n_expert <= 256 && top_k <= 32 && top_k * 8 <= n_expert &&
+           rv_smem(8, hidden, n_expert) <= 227 * 1024 - 4096;
+}
+// Scratch beside the logits: the router's f16 image and the norms.
+size_t route_filter_bytes(int64_t t, int64_t hidden, int64_t n_expert) {
+    return lmoe_align_up((size_t)n_expert * hidden * 2, 256) + lmoe_align_up((size_t)n_expert * 4, 256) + lmoe_align_up((size_t)t * 4, 256);
+}
+
+cudaError_t launch_route_filter(const float *router, const float *bias, const float *x, int t, int hidden, int n_expert, int top_k, float scale, int norm,
+                                float *logits, void *scratch, uint32_t *ids, float *weights, uint32_t *flag, cudaStream_t s) {
+    uint8_t *img = static_cast<uint8_t *>(scratch);
+    float *wnorm = reinterpret_cast<float *>(img + lmoe_align_up((size_t)n_expert * hidden * 2, 256));
+    float *xnorm = wnorm + lmoe_align_up((size_t)n_expert * 4, 256) / 4;
+    const int most = 227 * 1024 - 4096;
+    static thread_local int c_dev = -1, c_sms = 0;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev != c_dev) {
+        if ((e = cudaDeviceGetAttribute(&c_sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        for (auto f : {route_approx_kernel<128>, route_approx_kernel<64>})
+            if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most - 1024)) != cudaSuccess) return e;
+        for (auto f : {route_verify_kernel<16, 4>, route_verify_kernel<16, 8>, route_verify_kernel<8, 4>, route_verify_kernel<8, 8>})
+            if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most)) != cudaSuccess) return e;
+        c_dev = dev;
+    }
+    launch_pdl(route_prep_kernel, n_expert, 128, 0, s, router, hidden, n_expert, img, wnorm, flag);
+    // 128 tokens and all experts a block where that covers two thirds of the device, else 64 tokens and half of the experts
+    const bool large = (t + 127) / 128 * 3 >= 2 * c_sms;
+    const int tm = large ? 128 : 64, ne = large || n_expert % 64 ? n_expert : n_expert / 2;
+    launch_pdl(large ? route_approx_kernel<128> : route_approx_kernel<64>, dim3((unsigned)((t + tm - 1) / tm), (unsigned)(n_expert / ne)), 320,
+               rf_stages(tm) * (RF_A_BYTES + ne * 128) + 1024, s, x, img, t, hidden, n_expert, ne, logits, xnorm, flag);
+    // sixteen tokens a block where the rows fit and the blocks are enough for the device
+    const int tb = rv_smem(16, hidden, n_expert) <= most && (t + 15) / 16 * 5 >= 4 * c_sms ? 16 : 8;
+    auto verify = n_expert <= 128 ? (tb == 16 ? route_verify_kernel<16, 4> : route_verify_kernel<8, 4>)
+                                  : (tb == 16 ? route_verify_kernel<16, 8> : route_verify_kernel<8, 8>);
+    launch_pdl(verify, (unsigned)((t + tb - 1) / tb), RV_WARPS * 32, rv_smem(tb, hidden, n_expert), s, router, x, bias, logits, xnorm, wnorm, t, hidden,
+               n_expert, top_k, scale, norm, ids, weights);
+    return cudaGetLastError();
+}

@@ -208,6 +208,37 @@ def test_prefill_block_tile_heights(orc, dev, hidden, ff, t):
     _check_block(orc, blk, blk.host_layer(orc), np.random.default_rng(t).standard_normal((t, hidden)).astype(np.float32), 2e-3)
 
 
+@pytest.mark.parametrize("hidden,ne,top_k,t,bias", [(3072, 256, 10, 640, False), (3072, 256, 10, 2501, True), (4096, 96, 12, 1283, True),
+                                                    (1024, 256, 32, 1921, False), (512, 64, 8, 15361, True), (768, 128, 1, 5089, False)])
+def test_prefill_routing_through_the_filter(dev, hidden, ne, top_k, t, bias):
+    """Long prompts take the tensor core's bounds first: ids and weights are those of the stand-alone routing, which are the oracle's, to
+    the bit.  Both token tiles of either kernel, ragged counts; tokens that keep all experts (an infinity, NaN, values beyond the f16
+    range, zeros: every score ties), tiny and large ones, router rows that are equal and a bias that excludes an expert."""
+    from maxuna_b200.moe import MoeBlock
+
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(t)
+    b = 0.2 * torch.rand(ne, generator=gen, device=dev) - 0.1 if bias else None
+    if bias:
+        b[3], b[5], b[7] = float("-inf"), b[6], 40.0
+    blk = MoeBlock.random(hidden, 256, ne, top_k, seed=hidden + ne, device=dev, bias=b)
+    blk.router[6] = blk.router[5]
+    blk.router[ne - 1] = blk.router[0]
+    x = torch.randn(t, hidden, generator=gen, device=dev)
+    x[2] = 0.0
+    x[3] *= 1e-6
+    x[5] *= 300.0
+    x[7, 11] = 1e6
+    x[t // 2, 4] = float("inf")
+    x[t // 2 + 1, 9] = float("nan")
+    x[t - 1, 0] = 7e4
+    _, ids, w = blk.forward(x, return_routing=True, path="prefill")
+    ids2, w2 = blk.route(x)
+    torch.cuda.synchronize()
+    blk.check_device_flag()
+    assert torch.equal(ids, ids2) and torch.equal(w.view(torch.int32), w2.view(torch.int32))
+
+
 def test_prefill_block_wide_ff(orc, dev):
     # expert_ff = 512: two Q6_K super-blocks per down row (the 256-row down kernel), ragged row tiles
     from maxuna_b200.moe import MoeBlock
