@@ -126,6 +126,9 @@ cudaError_t launch_mv_q6k_stream(const uint8_t *w, int n_out, int k, const float
 cudaError_t launch_mul_mv_id(int dtype, const uint8_t *w, int64_t expert_bytes, int n_expert, int n_out, int k,
                              const float *x, int t, int x_per_row, const uint32_t *ids, int top_k, float *out,
                              cudaStream_t s);
+// mv_dense.cu
+cudaError_t launch_mv_dense(int dtype, const uint8_t *w, int n_out, int k, const float *x, int64_t pairs, int x_per_row, const uint32_t *ids, int top_k,
+                            float *out, cudaStream_t s);
 // One product of launch_mul_mv_id_jobs: `pairs` = tokens times top_k; ids NULL = expert 0 for every pair.
 constexpr int MV_JOBS = 4;
 struct MvJob {

@@ -1,0 +1,331 @@
+// Many rows times ONE quantized matrix, as exact as the mat-vec kernels, on the 5th-generation tensor cores.
+// Reference: the plain quantized product of `QMatMul`, src/ops/mv_id.rs:54-56, for a prompt chunk (the shared expert op by op).
+//
+// The operands are exact in f16: a weight is its sub-block's integer scale times its integer, up to 945 for Q4_K and for Q6_K, up to 4096, in two
+// parts, scale / 8 and scale % 8; an activation is four base-256 digits of a 30-bit integer (mv_digits.cuh), which are columns of the B operand.
+// Over a super-block the sums stay below 2^24 where they count (the top digit is within +-64), so the f32 accumulators hold
+// integers; the float factors, the weights of the digits and the Q4_K mins (a product of their own, against the sub-block sums in
+// three exact parts) come in once a super-block, as in mv_multi_kernel, whose integer products need their scales after every 32 or 16 values.
+// A super-block of 128 rows and 32 tokens takes 3.4 us (Q4_K; Q6_K 5.2), where its multiplies take 0.6 (1.2): the digits are made anew for every
+// 128 rows, 1700 of some 4300 cycles beside 1000 for storing them and 750 for the weights.  512 tokens [1024 x 3072] Q4_K 70 -> 47 us,
+// [3072 x 1024] Q6_K 113 -> 68, with the same error against 64 bits.
+#include "common.cuh"
+#include "kquant.cuh"
+#include "mv_digits.cuh"
+#include "tc.cuh"
+
+namespace {
+
+constexpr int MD_ROWS = 128, MD_TOK = 32, MD_COLS = MV_NDIG * MD_TOK; // a block's weight rows and tokens; column 32 d + i: digit d of token i
+constexpr int MD_WORK = 512, MD_THREADS = MD_WORK + 32; // sixteen warps make operands and take results, one issues
+constexpr int MD_Q6_WORDS = 53, MD_Q6_PITCH = 55;       // words that hold a 210-byte block at an even address; of a row of the staged blocks
+constexpr int MD_TILE = 128 * 128; // an operand tile of 128 rows x 64 values
+constexpr int MD_B = 4 * MD_TILE, MD_SUMS = 3 * MD_TOK * 128;
+
+template <int DT>
+struct MdCfg {
+    static constexpr bool Q4 = DT == LMOE_Q4_K;
+    static constexpr int O_LOW = 4 * MD_TILE, O_B = (Q4 ? 4 : 8) * MD_TILE, O_MINS = O_B + MD_B, O_SUMS = O_MINS + MD_TILE;
+    static constexpr int O_RAW = O_MINS; // Q6_K: the super-block's bytes of all rows
+    static constexpr int SMEM = (Q4 ? O_SUMS + MD_SUMS : O_RAW + MD_ROWS * MD_Q6_PITCH * 4) + 1024;
+};
+
+__device__ __forceinline__ uint32_t md_lop(uint32_t v, uint32_t mask, uint32_t magic) { // (v & mask) | magic
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(magic));
+    return r;
+}
+__device__ __forceinline__ uint32_t md_sub(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t md_mul(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t md_fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+__device__ __forceinline__ uint32_t md_twice(float v) { // f16 pair (v, v)
+    const uint32_t h = __half_as_ushort(__float2half_rn(v));
+    return h | h << 16;
+}
+__device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+__device__ __forceinline__ void md_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a),
+                 "l"(b), "r"(idesc), "r"(accum) : "memory");
+}
+// place of 16-byte chunk c of row r of an operand tile
+__device__ __forceinline__ int md_at(int r, int c) { return r * 128 + ((c ^ (r & 7)) << 4); }
+
+// Sixteen warps make the operands of a super-block, another one issues its multiplies, and while these run the sixteen take the super-block before out of tensor
+// memory and turn the next one's activations into digits (registers).  (With the roles given to different warps each of them waits for its
+// instructions: 512 tokens [1024 x 3072] Q4_K 59 us.)
+template <int DT>
+__global__ void __launch_bounds__(MD_THREADS, 1)
+mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__restrict__ x, int x_per_row, const uint32_t *__restrict__ ids, int top_k,
+                int pairs, float *__restrict__ out) {
+    using C = MdCfg<DT>;
+    constexpr int TS = C::Q4 ? Q4K_BYTES : Q6K_BYTES, SUB = C::Q4 ? 32 : 16;
+    extern __shared__ uint8_t md_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(md_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *a_st = smem, *b_st = smem + C::O_B, *mins = smem + C::O_MINS, *sums = smem + C::O_SUMS;
+    __shared__ uint64_t done;
+    __shared__ float sxs[4][MD_TOK];
+    __shared__ uint32_t tmem_slot;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = k / QK_K;
+    const int r0 = blockIdx.x * MD_ROWS, p0 = blockIdx.y * MD_TOK;
+    const int64_t row_bytes = (int64_t)nb * TS;
+    if (tid == 0) {
+        mb_init(&done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == MD_WORK / 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (C::Q4) { // the second half of the mins' 16 k is zero
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        if (tid < MD_ROWS) *reinterpret_cast<uint4 *>(mins + md_at(tid, 1)) = zero;
+        else if (tid < MD_ROWS + 3 * MD_TOK) *reinterpret_cast<uint4 *>(sums + md_at(tid - MD_ROWS, 1)) = zero;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_begin();
+    // weights: thread = (row, 64-k tile); activations: a warp has tokens warp and warp + 16; results: the same row, eight tokens
+    const int r = tid & (MD_ROWS - 1), j = (tid >> 7) & 3, q = warp & 3, part8 = (warp >> 2) & 3;
+    const uint8_t *row = w + (size_t)min(r0 + r, n_out - 1) * row_bytes;
+    const float *src[2];
+    bool want[2];
+#pragma unroll
+    for (int v = 0; v < 2; v++) {
+        const int p = p0 + (warp & 15) + 16 * v;
+        want[v] = p < pairs && (ids == nullptr || ids[p] == 0u); // another id names no matrix of this stack: a zero row
+        src[v] = x + (want[v] ? ((size_t)(p / top_k) * x_per_row + (x_per_row == 1 ? 0 : p % top_k)) * k : 0);
+    }
+    MvX in[2];
+    uint4 hdr, qa, qb;          // Q4_K: this tile's words
+    auto load_x = [&](int b) {
+#pragma unroll
+        for (int v = 0; v < 2; v++) in[v].load(src[v] + (want[v] ? (size_t)b * QK_K : 0), want[v], lane);
+    };
+    auto load_w = [&](int b) {
+        const uint8_t *blk = row + (size_t)b * TS;
+        if (C::Q4) {
+            hdr = __ldg(reinterpret_cast<const uint4 *>(blk));
+            qa = __ldg(reinterpret_cast<const uint4 *>(blk) + 1 + 2 * j);
+            qb = __ldg(reinterpret_cast<const uint4 *>(blk) + 2 + 2 * j);
+        } else { // whole rows, a word a lane (word by word of its own row a thread took 14 thousand cycles a super-block)
+            for (int i = 0; i < MD_ROWS / 16; i++) {
+                const int rr = warp * (MD_ROWS / 16) + i;
+                const uint8_t *g = w + (size_t)min(r0 + rr, n_out - 1) * row_bytes + (size_t)b * TS;
+                const uint32_t *g4 = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(g) & ~(uintptr_t)3);
+                uint32_t *to = reinterpret_cast<uint32_t *>(smem + C::O_RAW) + rr * MD_Q6_PITCH;
+#pragma unroll
+                for (int o = 0; o < 64; o += 32)
+                    if (lane + o < MD_Q6_WORDS) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s32(to + lane + o)), "l"(g4 + lane + o) : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+    };
+    float acc[8], odd[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) acc[i] = odd[i] = 0.f;
+    auto take = [&](int b, float d, float m) { // of super-block b: d, dmin of the row
+        const uint32_t t0 = tmem + 256u * (b & 1) + ((uint32_t)(32 * q) << 16) + 8u * part8;
+        uint32_t v[MV_NDIG][8], s[MV_PARTS][8];
+#pragma unroll
+        for (int e = 0; e < MV_NDIG; e++) tc_ld8(t0 + MD_TOK * e, v[e]);
+        if (C::Q4) {
+#pragma unroll
+            for (int e = 0; e < MV_PARTS; e++) tc_ld8(t0 + MD_COLS + MD_TOK * e, s[e]);
+        }
+        tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            // digits from the least significant on, so that only the last addition rounds at the size of the sum
+            float tot = __uint_as_float(v[MV_NDIG - 1][i]);
+#pragma unroll
+            for (int e = MV_NDIG - 2; e >= 0; e--) tot = __fmaf_rn(mv_digit_weight(e), __uint_as_float(v[e][i]), tot);
+            const float off = C::Q4 ? __uint_as_float(s[0][i]) + (__uint_as_float(s[1][i]) + __uint_as_float(s[2][i])) : 0.f;
+            // (two sums of half of the super-blocks, in turn, round less than one of all)
+            const float o = acc[i] + sxs[b & 3][8 * part8 + i] * (C::Q4 ? d * tot - m * off : d * tot);
+            acc[i] = odd[i];
+            odd[i] = o;
+        }
+        tc_fence_before();
+    };
+    bool ok = true;
+    if (warp == MD_WORK / 32) {
+        const bool el = elect_one();
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(MD_COLS >> 3) << 17) | ((uint32_t)(MD_ROWS >> 4) << 24);
+        const uint32_t idesc_m = (1u << 4) | ((uint32_t)(3 * MD_TOK >> 3) << 17) | ((uint32_t)(MD_ROWS >> 4) << 24);
+        const uint64_t ad = umma_desc(s32(a_st)), bd = umma_desc(s32(b_st)), md = umma_desc(s32(mins)), sd = umma_desc(s32(sums));
+        for (int b = 0; b < nb; b++) {
+            __syncthreads(); // the operands are there
+            tc_fence_after();
+            const uint32_t d = tmem + 256u * (b & 1);
+            if (el) {
+                if (C::Q4) md_mma(d + MD_COLS, md, sd, idesc_m, 0u);
+#pragma unroll
+                for (uint32_t t = 0; t < 4; t++) {
+#pragma unroll
+                    for (uint32_t kk = 0; kk < 4; kk++) {
+                        md_mma(d, ad + t * (MD_TILE >> 4) + 2 * kk, bd + t * (MD_TILE >> 4) + 2 * kk, idesc, t | kk);
+                        if (!C::Q4) md_mma(d, ad + ((C::O_LOW + t * MD_TILE) >> 4) + 2 * kk, bd + t * (MD_TILE >> 4) + 2 * kk, idesc, 1u);
+                    }
+                }
+                tc_commit<1>(&done);
+            }
+            __syncwarp();
+        }
+        ok = mb_wait(&done, (uint32_t)(nb - 1) & 1u); // none is in flight when the tensor memory is given back
+    }
+    float d = 0.f, m = 0.f;
+    if (warp < MD_WORK / 32) {
+        load_x(0);
+        load_w(0);
+    }
+    for (int b = 0; b < nb && warp < MD_WORK / 32; b++) {
+        uint2 dig[2][MV_NDIG];
+        float sx[2];
+        __half sub[2][MV_PARTS];
+#pragma unroll
+        for (int v = 0; v < 2; v++) mv_digits<SUB>(in[v], dig[v], sx[v], sub[v]);
+        if (b + 1 < nb) load_x(b + 1);
+        if (!C::Q4) asm volatile("cp.async.wait_group 0;\n\tbar.sync 1, 512;" ::: "memory"); // all rows' bytes are there
+        if (b && ok) ok = mb_wait(&done, (uint32_t)(b - 1) & 1u); // the operands of the super-block before have been multiplied
+        tc_fence_after();
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+            const int i = warp + 16 * v;
+#pragma unroll
+            for (int d = 0; d < MV_NDIG; d++) { // bytes as f16 pairs, in the order of the weights' chunks: 0 2 1 3 4 6 5 7
+                const uint32_t lo = dig[v][d].x ^ 0x80808080u, hi = dig[v][d].y ^ 0x80808080u, one = 0x64646464u, off = 0x64806480u;
+                *reinterpret_cast<uint4 *>(b_st + (lane >> 3) * MD_TILE + md_at(MD_TOK * d + i, lane & 7)) =
+                    make_uint4(md_sub(__byte_perm(lo, one, 0x4240), off), md_sub(__byte_perm(lo, one, 0x4341), off),
+                               md_sub(__byte_perm(hi, one, 0x4240), off), md_sub(__byte_perm(hi, one, 0x4341), off));
+            }
+            if (C::Q4 && (lane & 3) == 0) {
+#pragma unroll
+                for (int h = 0; h < MV_PARTS; h++)
+                    *reinterpret_cast<__half *>(sums + md_at(MD_TOK * h + i, 0) + 2 * (lane >> 2)) = sub[v][h];
+            }
+            if (lane == 0) sxs[b & 3][i] = sx[v];
+        }
+        uint8_t *a = a_st + j * MD_TILE;
+        uint16_t d6 = 0;
+        if constexpr (C::Q4) {
+            uint32_t scs[2], mn[2];
+            q4k_unpack_scales(hdr.y, hdr.z, hdr.w, scs[0], scs[1], mn[0], mn[1]);
+            if (j == 0) {
+                const uint32_t one = 0x64646464u, off = 0x64006400u;
+                *reinterpret_cast<uint4 *>(mins + md_at(r, 0)) =
+                    make_uint4(md_sub(__byte_perm(mn[0], one, 0x4140), off), md_sub(__byte_perm(mn[0], one, 0x4342), off),
+                               md_sub(__byte_perm(mn[1], one, 0x4140), off), md_sub(__byte_perm(mn[1], one, 0x4342), off));
+            }
+            const uint32_t pair = md_sub(__byte_perm((j & 2) ? scs[1] : scs[0], 0x64646464u, (j & 1) ? 0x4342u : 0x4140u), 0x64006400u);
+            const uint32_t v[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t s = __byte_perm(pair, 0u, h ? 0x3232u : 0x1010u), c0 = md_mul(s, 0xE400E400u); // - 1024 scales
+#pragma unroll
+                for (int c = 0; c < 4; c++) { // (1024 + q) scale - 1024 scale: exact
+                    const uint32_t u0 = v[2 * c] >> (4 * h), u1 = v[2 * c + 1] >> (4 * h);
+                    *reinterpret_cast<uint4 *>(a + md_at(r, 4 * h + c)) =
+                        make_uint4(md_fma(md_lop(u0, 0x000F000Fu, 0x64006400u), s, c0), md_fma(md_lop(u0 >> 8, 0x000F000Fu, 0x64006400u), s, c0),
+                                   md_fma(md_lop(u1, 0x000F000Fu, 0x64006400u), s, c0), md_fma(md_lop(u1 >> 8, 0x000F000Fu, 0x64006400u), s, c0));
+                }
+            }
+        } else {
+            // half j / 2, groups 2 (j % 2) + h
+            const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(row + (size_t)b * TS) & 2) * 8u;
+            const uint32_t *st = reinterpret_cast<const uint32_t *>(smem + C::O_RAW) + r * MD_Q6_PITCH;
+            auto word = [&](int i) { return __funnelshift_r(st[i], st[i + 1], off); }; // bytes 4 i .. 4 i + 3 of the block
+            const uint32_t scs = word(48 + 2 * (j >> 1) + (j & 1));
+            d6 = (uint16_t)(off ? st[52] >> 16 : st[52]);
+#pragma unroll
+            for (int h = 0; h < 2; h++) { // group 2 (j % 2) + h: its two scales are side by side
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int s = (int8_t)(scs >> (16 * h + (c < 2 ? 0 : 8)));
+                    const uint32_t hi = md_twice((float)(s >> 3)), lo = md_twice((float)(s & 7) * 0.125f);
+                    uint32_t e[4];
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        const uint32_t ql = word(16 * (j >> 1) + 8 * h + 2 * c + i) >> (4 * (j & 1));
+                        const uint32_t t = (word(32 + 8 * (j >> 1) + 2 * c + i) >> (4 * (j & 1) + 2 * h) & 0x03030303u) << 4;
+                        const uint32_t q6 = md_lop(ql, 0x0F0F0F0Fu, t);
+                        e[2 * i] = md_sub(__byte_perm(q6, 0x64646464u, 0x4240), 0x64206420u);
+                        e[2 * i + 1] = md_sub(__byte_perm(q6, 0x64646464u, 0x4341), 0x64206420u);
+                    }
+                    *reinterpret_cast<uint4 *>(a + md_at(r, 4 * h + c)) = make_uint4(md_mul(e[0], hi), md_mul(e[1], hi), md_mul(e[2], hi), md_mul(e[3], hi));
+                    *reinterpret_cast<uint4 *>(a + C::O_LOW + md_at(r, 4 * h + c)) = make_uint4(md_mul(e[0], lo), md_mul(e[1], lo), md_mul(e[2], lo), md_mul(e[3], lo));
+                }
+            }
+        }
+        const float d_now = C::Q4 ? lmoe_h2f((uint16_t)(hdr.x & 0xffff)) : 8.f * lmoe_h2f(d6);
+        const float m_now = C::Q4 ? lmoe_h2f((uint16_t)(hdr.x >> 16)) * MV_SUM_UNSCALE : 0.f;
+        if (C::Q4 && b + 1 < nb) load_w(b + 1);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (!C::Q4 && b + 1 < nb) load_w(b + 1); // (all have read this one's bytes)
+        if (b) take(b - 1, d, m);
+        d = d_now;
+        m = m_now;
+    }
+    if (warp < MD_WORK / 32) {
+        if (ok) ok = mb_wait(&done, (uint32_t)(nb - 1) & 1u);
+        tc_fence_after();
+        take(nb - 1, d, m);
+    }
+    const int bad = __syncthreads_or(!ok);
+    const int ro = r0 + 32 * q + lane;
+    if (ro < n_out && warp < MD_WORK / 32) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) { // (a wait that ran out leaves NaN, not a wrong number)
+            const int p = p0 + 8 * part8 + i;
+            if (p < pairs) out[(size_t)p * n_out + ro] = bad ? __int_as_float(0x7fffffff) : acc[i] + odd[i];
+        }
+    }
+    if (warp == MD_WORK / 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+}
+
+template <int DT>
+cudaError_t launch_dense(const uint8_t *w, int n_out, int k, const float *x, int64_t pairs, int x_per_row, const uint32_t *ids, int top_k, float *out,
+                         cudaStream_t s) {
+    static thread_local int c_dev = -1;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev != c_dev) {
+        if ((e = cudaFuncSetAttribute(mv_dense_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, MdCfg<DT>::SMEM)) != cudaSuccess) return e;
+        c_dev = dev;
+    }
+    // grid.y is limited to 65535 groups
+    const int64_t step = (int64_t)65535 * MD_TOK / top_k * top_k;
+    for (int64_t p = 0; p < pairs; p += step) {
+        const int64_t n = pairs - p < step ? pairs - p : step;
+        launch_pdl(mv_dense_kernel<DT>, dim3((unsigned)((n_out + MD_ROWS - 1) / MD_ROWS), (unsigned)((n + MD_TOK - 1) / MD_TOK)), MD_THREADS, MdCfg<DT>::SMEM, s,
+                   w, n_out, k, x + (size_t)(p / top_k) * x_per_row * k, x_per_row, ids ? ids + p : nullptr, top_k, (int)n, out + (size_t)p * n_out);
+    }
+    return cudaGetLastError();
+}
+
+} // namespace
+
+// out[pair][n_out] = the matrix times the pair's row of x; ids as in launch_mul_mv_id for a stack of one.
+cudaError_t launch_mv_dense(int dtype, const uint8_t *w, int n_out, int k, const float *x, int64_t pairs, int x_per_row, const uint32_t *ids, int top_k,
+                            float *out, cudaStream_t s) {
+    return dtype == LMOE_Q4_K ? launch_dense<LMOE_Q4_K>(w, n_out, k, x, pairs, x_per_row, ids, top_k, out, s)
+                              : launch_dense<LMOE_Q6_K>(w, n_out, k, x, pairs, x_per_row, ids, top_k, out, s);
+}

@@ -21,91 +21,15 @@
 //                    ring.  Weights go straight from global memory into the A fragments.
 //   mv_multi_kernel  many pairs of ONE weight matrix (the shared expert, a plain matrix): eight pairs are the columns of
 //                    an MMA, so a super-block is unpacked once for 32 pairs.  512 pairs of [1024 x 3072] Q4_K: 816 -> 68 us.
+//                    From where it is the shorter one, mv_dense.cu serves these.
 #include <cooperative_groups.h>
 #include "common.cuh"
+#include "mv_digits.cuh"
 #include "stream_math.cuh"
 
 namespace {
 
 constexpr int MV_THREADS = 256, MV_ROWS = 64; // rows of a block: four MMA row tiles, the K dimension in two halves
-constexpr int MV_NDIG = 4;
-// A value is an integer of magnitude <= 2^30 (the top digit stays within +-64) times its block's scale, 2^29 integers to the
-// power of two at or below the largest magnitude.
-constexpr int MV_BITS = 29;
-// The SUB-wide sums (|sum| <= 2^35) enter an f16 product times 2^-20, in three parts of eleven bits: multiples of 2^5, 2^-6 and
-// 2^-17.  With one quantum for all sub-blocks the product with the integer mins or scales is exact, a part at a time.
-constexpr int MV_PARTS = 3;
-constexpr float MV_SUM_UNSCALE = 0x1p20f;
-constexpr float MV_OFFSET = 32.f * MV_SUM_UNSCALE; // Q6_K: what the product of scales and sums stands for, in units of the integers
-
-// One 256-wide block of an activation row, by one warp (eight consecutive values per lane): digits, the block's scale, and
-// the SUB-wide sums of the quantized values as f16 parts, most significant first.
-struct MvX {
-    float4 a, c;
-    __device__ __forceinline__ void load(const float *__restrict__ src, bool want, int lane) { // a row not wanted counts as zero
-        a = c = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (want) {
-            a = __ldg(reinterpret_cast<const float4 *>(src + lane * 8));
-            c = __ldg(reinterpret_cast<const float4 *>(src + lane * 8) + 1);
-        }
-    }
-};
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-template <int SUB>
-__device__ __forceinline__ void mv_digits(const MvX &in, uint2 (&dig)[MV_NDIG], float &sx, __half (&part)[MV_PARTS]) {
-    const float v[8] = {in.a.x, in.a.y, in.a.z, in.a.w, in.c.x, in.c.y, in.c.z, in.c.w};
-    float amax = 0.f; // NaN if any value is: the block's scale, and with it the result, then is NaN too
-#pragma unroll
-    for (int j = 0; j < 8; j++) amax = max_nan(amax, fabsf(v[j]));
-#pragma unroll
-    for (int o = 16; o; o >>= 1) amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    // 2^e <= amax < 2^(e + 1); below 2^-97 the scale stays at the smallest normal number, so that its reciprocal exists
-    const int e = max((int)(__float_as_uint(amax) >> 23) - 127, -97);
-    const float inv = __int_as_float((127 + MV_BITS - e) << 23);
-    sx = e == 128 ? amax : __int_as_float((127 - MV_BITS + e) << 23);
-    int X[8], sum_h = 0, sum_l = 0; // sums of the upper and the lower 15 bits
-#pragma unroll
-    for (int j = 0; j < 8; j++) X[j] = __float2int_rn(v[j] * inv);
-    if (e == 128) { // an infinite value times an infinite scale; the others count nothing beside it
-#pragma unroll
-        for (int j = 0; j < 8; j++) X[j] = fabsf(v[j]) == INFINITY ? (v[j] > 0.f ? 1 << MV_BITS : -(1 << MV_BITS)) : 0;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        sum_h += X[j] >> 15;
-        sum_l += X[j] & 0x7fff;
-    }
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        uint32_t y[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) y[j] = (uint32_t)(X[4 * h + j] + 0x808080); // the three low digits become plain bytes plus 128
-        // byte d of the four values side by side; the 128 comes off again with the sign bit
-        const uint32_t d3 = __byte_perm(__byte_perm(y[0], y[1], 0x40), __byte_perm(y[2], y[3], 0x40), 0x5410) ^ 0x80808080u;
-        const uint32_t d2 = __byte_perm(__byte_perm(y[0], y[1], 0x51), __byte_perm(y[2], y[3], 0x51), 0x5410) ^ 0x80808080u;
-        const uint32_t d1 = __byte_perm(__byte_perm(y[0], y[1], 0x62), __byte_perm(y[2], y[3], 0x62), 0x5410) ^ 0x80808080u;
-        const uint32_t d0 = __byte_perm(__byte_perm(y[0], y[1], 0x73), __byte_perm(y[2], y[3], 0x73), 0x5410);
-        if (h == 0) { dig[0].x = d0; dig[1].x = d1; dig[2].x = d2; dig[3].x = d3; }
-        else { dig[0].y = d0; dig[1].y = d1; dig[2].y = d2; dig[3].y = d3; }
-    }
-#pragma unroll
-    for (int o = 1; o < SUB / 8; o <<= 1) {
-        sum_h += __shfl_xor_sync(0xffffffffu, sum_h, o);
-        sum_l += __shfl_xor_sync(0xffffffffu, sum_l, o);
-    }
-    const int q0 = (sum_h + (1 << 9)) >> 10, r0 = (sum_h - (q0 << 10)) * (1 << 15) + sum_l; // |sum_h|, sum_l <= 2^20
-    const int q1 = (r0 + (1 << 13)) >> 14, r1 = r0 - (q1 << 14);
-    part[0] = __float2half_rn((float)q0 * 0x1p5f);
-    part[1] = __float2half_rn((float)q1 * 0x1p-6f);
-    part[2] = __float2half_rn((float)((r1 + 4) >> 3) * 0x1p-17f);
-}
-// weight of digit d (most significant first)
-__device__ __forceinline__ float mv_digit_weight(int d) { return d == 0 ? 16777216.f : (d == 1 ? 65536.f : (d == 2 ? 256.f : 1.f)); }
-
 // ---- raw fields of two rows of one super-block, as this lane's part of the MMA A fragments --------------------------
 // Q4_K: bytes 8t .. 8t+7 of each 32-byte run (low nibbles: sub-block 2j, high: 2j+1), and the 16-byte header.
 struct MvQ4 {
@@ -973,6 +897,21 @@ cudaError_t mv_device(int &dev, int &sms) {
 bool mv_multi_better(int n_expert, int n_out, int64_t pairs, int sms) {
     return n_expert == 1 && (pairs + MM_COLS - 1) / MM_COLS * ((n_out + MV_ROWS - 1) / MV_ROWS) >= sms && pairs > 4;
 }
+// The tensor-core kernel of mv_dense.cu takes a super-block of 128 rows and 32 pairs at a time, 3.4 us Q4_K, 5.2 Q6_K, whatever the number
+// of blocks on the device; these kernels' time goes with the work.  us here / there, cold L2:
+//   pairs                      32           64          128          256          512         1024         4096
+//   [1024 x 3072] Q4_K  20.5 / 43.1  30.8 / 45.0  34.8 / 45.1  55.5 / 45.1  69.7 / 47.1   135 / 86.0    459 / 285
+//   [768 x 2048] Q4_K   18.4 / 32.8  22.5 / 32.8  26.7 / 32.8  43.0 / 34.8  47.1 / 34.8  74.8 / 63.5    239 / 179
+//   [3072 x 1024] Q6_K  22.6 / 26.6  41.0 / 26.6  43.0 / 26.6  66.6 / 47.1   113 / 67.6   201 / 128     773 / 428
+//   [2048 x 768] Q6_K   21.5 / 21.4  34.8 / 22.5  45.1 / 22.5  38.9 / 22.5  67.6 / 38.9   127 / 71.7    436 / 231
+// Below 64 pairs a chain's shared product is better off in the launch of the routed ones (48 tokens op by op, 256 experts: 443 us so, 460 apart).
+bool mv_dense_better(int dt, const uint8_t *w, int n_expert, int n_out, int k, int64_t pairs, int sms) {
+    if (n_expert != 1 || pairs < 64 || (reinterpret_cast<uintptr_t>(w) & 15u)) return false;
+    const bool q4 = dt == LMOE_Q4_K, multi = mv_multi_better(n_expert, n_out, pairs, sms);
+    const int64_t rounds = (((int64_t)n_out + 127) / 128 * ((pairs + 31) / 32) + sms - 1) / sms;
+    const double there = 5.0 + (double)rounds * (k / QK_K) * (q4 ? 3.4 : 5.2);
+    return there < 7.0 + (double)pairs * n_out * k * (multi ? (q4 ? 4.2e-8 : 6.8e-8) : (q4 ? 6.0e-8 : 1.5e-7));
+}
 // a bulk copy starts and ends on 16 bytes: every expert must; the end of a single matrix may be ragged
 bool mv_copies(const uint8_t *w, int n_expert, int64_t expert_bytes) {
     return (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (n_expert == 1 || expert_bytes % 16 == 0);
@@ -990,6 +929,7 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
     // One matrix for all pairs: 32 pairs to an unpacked super-block, once such blocks cover every SM.  (Below that two pairs to a
     // block win by parallelism: [1024 x 3072] Q4_K, 64 / 512 pairs 26 / 92 us against 44 / 68, [3072 x 1024] Q6_K, 32 / 128
     // pairs 19 / 44 against 26 / 39.)
+    if (mv_dense_better(DT, w, n_expert, n_out, k, pairs, sms)) return launch_mv_dense(DT, w, n_out, k, x, pairs, x_per_row, ids, top_k, out, s);
     if (mv_multi_better(n_expert, n_out, pairs, sms)) {
         constexpr int smem = MM_COLS * MM_PITCH<DT> + MV_PARTS * MM_COLS * (MM_KC / QK_K * NS + 8) * 2 + (MM_KC / QK_K) * MM_COLS * 4;
         constexpr int CS = 4;
@@ -1045,7 +985,7 @@ cudaError_t launch_mv_jobs(const MvJob *job, int jobs, int n_out, int k, cudaStr
     int rest = 0;
     for (int j = 0; j < jobs; j++) {
         const MvJob &J = job[j];
-        const bool one = J.pairs > 0 && J.pairs <= 65535 && !mv_rows_better<DT>(J.pairs, n_out, k) && !mv_multi_better(J.n_expert, n_out, J.pairs, sms) &&
+        const bool one = J.pairs > 0 && J.pairs <= 65535 && !mv_rows_better<DT>(J.pairs, n_out, k) && !mv_multi_better(J.n_expert, n_out, J.pairs, sms) && !mv_dense_better(DT, J.w, J.n_expert, n_out, k, J.pairs, sms) &&
                          mv_copies(J.w, J.n_expert, J.expert_bytes) && J.expert_bytes % 16 == 0 && !(J.n_expert == 1 && J.expert_bytes > MX_L2);
         if (one) together[n++] = J;
         else alone[rest++] = J;

@@ -173,6 +173,40 @@ def test_mv_many_pairs_of_one_matrix(orc, dev, dt, name, n_out, k, pairs):
     assert not got[ids == 1].any() and orc.rel_l2(got, want) < 1e-5
 
 
+@pytest.mark.parametrize("n_out,k,t,top_k,xpr", [
+    (130, 256, 2001, 1, 1),   # one super-block, two rows in the last block, one token in the last group
+    (1000, 1280, 167, 2, 2),  # an odd number of super-blocks; a row of x for every slot
+    (390, 768, 513, 2, 1),    # slots that share a row of x
+    (128, 512, 8200, 1, 1),   # several rounds over the device
+])
+@pytest.mark.parametrize("dt,name", DTYPES)
+def test_mv_dense(orc, dev, dt, name, n_out, k, t, top_k, xpr):
+    """One matrix and many pairs on the tensor cores: ragged rows and pairs, empty slots, values that span the range of f32, an infinity
+    and NaN that stay in their rows.  Exact products and sums but for the f32 roundings once a super-block: bound as in
+    test_mv_range_and_resolution, against 64-bit sums."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    raw = orc.quantize(dt, orc.pseudo_random(n_out * k, 0xD00 + k, -1.0, 1.0))
+    stack = ExpertStack.from_bytes(raw, dt, 1, n_out, k, device=dev)
+    rng = np.random.default_rng(t)
+    ids = (np.arange(t * top_k, dtype=np.uint32) % 11 == 4).astype(np.uint32).reshape(t, top_k)  # 1: an empty slot
+    run = lambda v: ops.mul_mv_id(stack, torch.from_numpy(v).to(dev), torch.from_numpy(ids.astype(np.int32)).to(dev)).cpu().numpy()
+    x = rng.standard_normal((t, xpr, k)).astype(np.float32)
+    x[0::3, :, 7::256] *= 1e4
+    x[2::3] *= (2.0 ** rng.integers(-60, 60, (len(x[2::3]), 1, 1))).astype(np.float32)
+    got = run(x)
+    w = stack.dequantize()[0].double()
+    want = torch.from_numpy(x).to(dev).double() @ w.T  # [t, xpr, n_out]
+    want = want.expand(t, top_k, n_out).cpu().numpy() if xpr == 1 else want.cpu().numpy()
+    assert not got[ids == 1].any()
+    err = np.linalg.norm(got - want, axis=2) / np.linalg.norm(want, axis=2)
+    assert err[ids == 0].max() < 8 * 2.0 ** -24
+    x[3, 0, 40], x[5, 0, 11] = np.inf, np.nan
+    bad, keep = run(x), [r for r in range(t) if r not in (3, 5)]
+    assert not np.isfinite(bad[3, 0]).any() and np.isnan(bad[5, 0]).all() and np.array_equal(bad[keep], got[keep])
+
+
 @pytest.mark.parametrize("n_expert,n_out,k,t,top_k", [(4, 512, 768, 17, 2), (1, 1100, 512, 285, 1), (1, 64, 8192, 40, 1)])
 @pytest.mark.parametrize("dt,name", DTYPES)
 def test_mv_range_and_resolution(orc, dev, dt, name, n_expert, n_out, k, t, top_k):
