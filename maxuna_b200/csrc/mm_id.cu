@@ -381,7 +381,8 @@ struct GmCfg {
     static constexpr int EPI_BYTES = NPROJ == 2 ? GM_EPI_BYTES : 2 * GM_BOX_ROWS * 128;
     static constexpr int B_ROWS = NT / CG;
     static constexpr int B_BLK = B_ROWS * MM_K * 2;     // a CTA's half of a 64-k block of the B operand
-    static constexpr int B_FULL = (NPROJ == 2 || CG == 1 ? 1 : 2) * (NT == 64 ? 2 : 1); // blocks of a full tile in a ring slot
+    // blocks of a full tile in a ring slot (two in the slots of gate/up's 128-row tiles: 768 / 1024 tokens 500 / 536 -> 497 / 529 us)
+    static constexpr int B_FULL = (NPROJ == 2 || CG == 1 ? 1 : 2) * (NT == 64 || (NPROJ == 2 && NT == 128) ? 2 : 1);
     static constexpr int B_SLOT = B_FULL * B_BLK;
     static constexpr int NB = 96 * 1024 / B_SLOT < 8 ? 96 * 1024 / B_SLOT : 8;
     static constexpr bool WIDE = NT <= 128;             // operand stages of 128 weights a thread, else 64
