@@ -113,11 +113,11 @@ cudaError_t launch_route_logits(const float *router, const float *x, int t, int 
 cudaError_t launch_route_select(const float *logits, const float *bias, int t, int n_expert, int top_k,
                                 float scale, int norm, uint32_t *ids, float *weights, cudaStream_t s, uint32_t *clear = nullptr);
 // route_filter.cu
-// Logits and selection in one, for long prompts: the same ids and weights.  `logits` ([t, n_expert]) is scratch; `flag` is cleared first.
+// Logits and selection in one, for long prompts: the same ids and weights.  `flag` is cleared first.
 bool route_filter_available(int64_t hidden, int64_t n_expert, int64_t top_k);
 size_t route_filter_bytes(int64_t t, int64_t hidden, int64_t n_expert);
 cudaError_t launch_route_filter(const float *router, const float *bias, const float *x, int t, int hidden, int n_expert, int top_k, float scale, int norm,
-                                float *logits, void *scratch, uint32_t *ids, float *weights, uint32_t *flag, cudaStream_t s);
+                                void *scratch, uint32_t *ids, float *weights, uint32_t *flag, cudaStream_t s);
 // mv_stream.cu
 // Streamed Q6_K mat-vec: one activation row, all rows of the matrix.
 bool mv_q6k_stream_available(int64_t n_out, int64_t k);

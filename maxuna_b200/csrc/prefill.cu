@@ -427,10 +427,11 @@ static lmoe_status experts_prefill(const lmoe_layer *L, const void *x, int x_f16
 }
 
 // Routing through route_filter.cu once the f32 product is the longer one (a block's forward, cold L2, us without / with: hidden 3072, 256
-// experts, 512 / 768 / 1024 / 2048 / 4096 / 16384 tokens 463 / 465, 512 / 500, 557 / 536, 806 / 745, 1295 / 1194, 4550 / 3919; hidden 2048,
-// 128 experts, 800 / 1600 / 4000 tokens 257 / 289, 352 / 325, 570 / 554).
+// experts, 256 / 384 / 512 / 640 / 2048 / 4096 / 16384 tokens 379 / 386, 421 / 417, 456 / 450, 482 / 466, 806 / 728, 1295 / 1166, 4550 / 3920; hidden 2048,
+// 128 experts, 400 / 800 / 1200 / 2400 tokens 175 / 180, 207 / 204, 248 / 241, 366 / 351; of 64 experts more are left: hidden 4096, 1200 / 2400 tokens
+// 245 / 248, 373 / 370).
 static bool prefill_filters(const lmoe_layer *L, int64_t t) {
-    return (double)t * L->n_expert * L->hidden >= 5e8 && route_filter_available(L->hidden, L->n_expert, L->top_k);
+    return (double)t * L->n_expert * L->hidden >= (L->n_expert >= 128 ? 3e8 : 6e8) && route_filter_available(L->hidden, L->n_expert, L->top_k);
 }
 
 size_t prefill_workspace_bytes(const lmoe_layer *L, int64_t t) {
@@ -464,7 +465,7 @@ lmoe_status launch_moe_prefill(const lmoe_layer *L, const float *x, const float 
 
     // (both begin with a fresh device flag: the workspace needs no initialisation)
     if (filter) {
-        LMOE_CUDA(launch_route_filter(L->router, L->bias, x, (int)t, (int)H, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, logits, rf_ws, ids, w, flag, s));
+        LMOE_CUDA(launch_route_filter(L->router, L->bias, x, (int)t, (int)H, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, rf_ws, ids, w, flag, s));
     } else {
         LMOE_CUDA(launch_route_logits(L->router, x, (int)t, (int)H, (int)L->n_expert, logits, s));
         LMOE_CUDA(launch_route_select(logits, L->bias, (int)t, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, ids, w, s, flag));

@@ -3,8 +3,8 @@
 // Reference: `route_logits` and `route_from_logits`, src/moe.rs:84-119.
 //
 // The specified logits (route_math.cuh) are f32 products in a fixed order: for 16384 tokens, 256 experts and hidden 3072 they and the selection
-// take 730 us at half of the f32 rate, for 2048 tokens 115.  This takes 290 and 65: 5 for the router's f16 image, 43 / 22 for the approximate product
-// (16384 tokens: the tokens from memory at 4.7 TB/s), 240 / 38 for the rest (the router rows from the L2 cache).  A product of the operands rounded to f16 differs from it by at most
+// take 730 us at half of the f32 rate, for 2048 tokens 115.  This takes 290 and 57: 5 for the router's f16 image, 42 / 13 for the approximate product
+// (16384 tokens: the tokens from memory at 4.8 TB/s), 240 / 38 for the rest (the router rows from the L2 cache).  A product of the operands rounded to f16 differs from it by at most
 //   |x| |w| (2^-10 + 2^-12) + 2^-25 sqrt(hidden) (|x| + |w|)
 // (2^-11 for the rounding of either operand by Cauchy's inequality, 2^-12 for the f32 sums of 3072 products in the tensor core, which rounds
 // or cuts once in 16, and for the specified sum, whose own error is 2^-19; the last term for values below the f16 range), so it bounds every score, and an expert whose
@@ -20,7 +20,8 @@
 namespace {
 
 constexpr int RF_A_BYTES = 128 * 128; // 128 tokens x 64 values as f16
-__host__ __device__ constexpr int rf_stages(int tm) { return tm == 64 ? 6 : 4; }
+constexpr int RF_STAGES = 4;
+constexpr int RF_SPLITS = 4; // most parts that hidden is cut into
 constexpr int RF_AHEAD = 3; // stages whose words a producing thread has in flight
 
 // The router as f16 in the order of the B operand's stages (64 values of all experts: a 128-byte-swizzled tile), and its rows' norms.
@@ -48,20 +49,22 @@ __global__ void __launch_bounds__(128) route_prep_kernel(const float *__restrict
 }
 
 // Approximate logits of TM tokens (the M of the multiplies is 128; rows past the last token are whatever lies there, and nothing reads
-// their results) and `ne` experts from blockIdx.y * ne on: eight warps round the tokens to f16 and put them into the A stages, warp 8
-// issues the multiplies, warp 9 copies the B stages, warps 0-3 take the results out of tensor memory.  blockIdx.y = 0 writes the tokens' norms.
+// their results) and all experts, over part blockIdx.y of hidden (the parts' results follow one another, t x n_expert each): eight warps round the tokens to f16 and put them into the A stages, warp 8
+// issues the multiplies, warp 9 copies the B stages, warps 0-3 take the results out of tensor memory.  xss: the tokens' squared norms, by part.
+// What a block reads bounds it, some 60 bytes a cycle and SM from the L2 cache: for few tokens the parts of hidden cut that, where parts of the experts would
+// read the tokens again (2048 tokens: 64 blocks of half of the experts 21 us, 128 of a quarter of hidden 13).
 template <int TM>
 __global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__restrict__ x, const uint8_t *__restrict__ img, int t, int hidden, int n_expert,
-                                                              int ne, float *__restrict__ logits, float *__restrict__ xnorm, uint32_t *__restrict__ flag) {
-    constexpr int RF_STAGES = rf_stages(TM), GROUPS = TM == 64 ? 2 : 1; // groups of producing warps, which take the stages in turn
+                                                              float *__restrict__ logits, float *__restrict__ xss, uint32_t *__restrict__ flag) {
+    constexpr int GROUPS = TM == 64 ? 2 : 1; // groups of producing warps, which take the stages in turn
     extern __shared__ uint8_t rf_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(rf_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t a_full[RF_STAGES], b_full[RF_STAGES], empty[RF_STAGES], done;
     __shared__ uint32_t tmem_slot;
     __shared__ float sums[TM];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, steps = hidden / 64;
-    const int t0 = blockIdx.x * TM, nt = min(TM, t - t0), e0 = blockIdx.y * ne;
-    const uint32_t b_bytes = (uint32_t)ne * 128u;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, steps = hidden / 64 / (int)gridDim.y, s00 = (int)blockIdx.y * steps;
+    const int t0 = blockIdx.x * TM, nt = min(TM, t - t0);
+    const uint32_t b_bytes = (uint32_t)n_expert * 128u;
     uint8_t *a_st = smem, *b_st = smem + RF_STAGES * RF_A_BYTES;
     if (tid == 0) {
         for (int s = 0; s < RF_STAGES; s++) {
@@ -91,7 +94,7 @@ __global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__res
 #pragma unroll
         for (int i = 0; i < NC; i++) {
             const int r = r0 + RS * i;
-            src[i] = reinterpret_cast<const float4 *>(x + (size_t)(t0 + min(r, nt - 1)) * hidden) + 2 * ch;
+            src[i] = reinterpret_cast<const float4 *>(x + (size_t)(t0 + min(r, nt - 1)) * hidden) + 16 * s00 + 2 * ch;
             dst[i] = a_st + r * 128 + ((ch ^ (r & 7)) << 4);
             ss[i] = 0.f;
         }
@@ -125,7 +128,7 @@ __global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__res
                 load(u, s0 + GROUPS * (u + RF_AHEAD));
             }
         }
-        if (blockIdx.y == 0) { // (the groups' shares meet in shared memory)
+        { // (the groups' shares meet in shared memory)
 #pragma unroll
             for (int i = 0; i < NC; i++) {
 #pragma unroll
@@ -136,16 +139,16 @@ __global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__res
 #pragma unroll
             for (int i = 0; i < NC; i++) {
                 const int r = r0 + RS * i;
-                if (grp == 0 && ch == 0 && r < nt) xnorm[t0 + r] = sqrtf(GROUPS == 2 ? ss[i] + sums[r] : ss[i]);
+                if (grp == 0 && ch == 0 && r < nt) xss[(size_t)blockIdx.y * t + t0 + r] = GROUPS == 2 ? ss[i] + sums[r] : ss[i];
             }
         }
         if (warp < 4) { // a lane is a token
             ok &= mb_wait(&done, 0);
             tc_fence_after();
             const int r = 32 * warp + lane;
-            float *dstl = logits + (size_t)(t0 + r) * n_expert + e0;
+            float *dstl = logits + ((size_t)blockIdx.y * t + t0 + r) * n_expert;
             if (32 * warp < nt)
-                for (int c = 0; c < ne; c += 16) {
+                for (int c = 0; c < n_expert; c += 16) {
                     uint32_t o[16];
                     tc_ld16(tmem + ((uint32_t)(32 * warp) << 16) + c, o);
                     tc_wait_ld();
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__res
         }
     } else if (warp == 8) {
         const bool el = elect_one();
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(ne >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(n_expert >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         uint32_t st = 0, ph = 0;
         for (int s = 0; s < steps && ok; s++) {
             ok &= mb_wait(&b_full[st], ph);
@@ -186,7 +189,7 @@ __global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__res
             ok &= mb_wait(&empty[st], ph ^ 1);
             if (el) {
                 mb_expect_tx(&b_full[st], b_bytes);
-                bulk_g2s(b_st + st * b_bytes, img + ((size_t)s * n_expert + e0) * 128, b_bytes, &b_full[st]);
+                bulk_g2s(b_st + st * b_bytes, img + (size_t)(s00 + s) * n_expert * 128, b_bytes, &b_full[st]);
             }
             __syncwarp();
             if (++st == RF_STAGES) { st = 0; ph ^= 1; }
@@ -216,7 +219,7 @@ constexpr uint32_t RV_OUT = 0xffa5a5a5u; // in place of the logit of an expert t
 template <int TB, int PER>
 __global__ void __launch_bounds__(RV_WARPS * 32, 1)
 route_verify_kernel(const float *__restrict__ router, const float *__restrict__ x, const float *__restrict__ bias, const float *__restrict__ approx,
-                    const float *__restrict__ xnorm, const float *__restrict__ wnorm, int t, int hidden, int n_expert, int top_k, float scale, int norm,
+                    const float *__restrict__ xss, int splits, const float *__restrict__ wnorm, int t, int hidden, int n_expert, int top_k, float scale, int norm,
                     uint32_t *__restrict__ ids, float *__restrict__ weights) {
     extern __shared__ __align__(16) uint8_t rv_raw[];
     float4 *xs = reinterpret_cast<float4 *>(rv_raw);
@@ -242,11 +245,16 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
 #pragma unroll
         for (int j = 0; j < PER; j++) {
             const int e = min(lane + 32 * j, n_expert - 1);
-            l[j] = approx[(size_t)tok * n_expert + e];
+            l[j] = 0.f;
+#pragma unroll
+            for (int p = 0; p < RF_SPLITS; p++)
+                if (p < splits) l[j] += approx[((size_t)p * t + tok) * n_expert + e];
             W[j] = wnorm[e] * 1.001f;
             b[j] = bias ? __ldg(bias + e) : 0.f;
         }
-        const float X = xnorm[tok] * 1.001f, sub = 0x1p-25f * 1.01f * sqrtf((float)hidden);
+        float x2 = 0.f;
+        for (int p = 0; p < splits; p++) x2 += xss[(size_t)p * t + tok];
+        const float X = sqrtf(x2) * 1.001f, sub = 0x1p-25f * 1.01f * sqrtf((float)hidden);
 #pragma unroll
         for (int j = 0; j < PER; j++) {
             // (a sigmoid from the hardware's exponential and reciprocal is good to 1e-6, sums round by less)
@@ -416,16 +424,19 @@ bool route_filter_available(int64_t hidden, int64_t n_expert, int64_t top_k) {
     return hidden % 128 == 0 && hidden >= 512 && hidden <= 4096 && n_expert % 32 == 0 && n_expert >= 64 && n_expert <= 256 && top_k <= 32 && top_k * 8 <= n_expert &&
            rv_smem(8, hidden, n_expert) <= 227 * 1024 - 4096;
 }
-// Scratch beside the logits: the router's f16 image and the norms.
+// Scratch: the router's f16 image, the norms, and the approximate logits by part of hidden, for at most this many token rows (never fewer for more
+// tokens: a workspace for t tokens serves any smaller number).
+static int64_t rf_rows(int64_t t) { return t > 16384 ? t : (RF_SPLITS * t < 16384 ? RF_SPLITS * t : 16384); }
 size_t route_filter_bytes(int64_t t, int64_t hidden, int64_t n_expert) {
-    return lmoe_align_up((size_t)n_expert * hidden * 2, 256) + lmoe_align_up((size_t)n_expert * 4, 256) + lmoe_align_up((size_t)t * 4, 256);
+    return lmoe_align_up((size_t)n_expert * hidden * 2, 256) + lmoe_align_up((size_t)n_expert * 4, 256) + lmoe_align_up((size_t)rf_rows(t) * 4, 256) +
+           (size_t)rf_rows(t) * n_expert * 4;
 }
 
 cudaError_t launch_route_filter(const float *router, const float *bias, const float *x, int t, int hidden, int n_expert, int top_k, float scale, int norm,
-                                float *logits, void *scratch, uint32_t *ids, float *weights, uint32_t *flag, cudaStream_t s) {
+                                void *scratch, uint32_t *ids, float *weights, uint32_t *flag, cudaStream_t s) {
     uint8_t *img = static_cast<uint8_t *>(scratch);
     float *wnorm = reinterpret_cast<float *>(img + lmoe_align_up((size_t)n_expert * hidden * 2, 256));
-    float *xnorm = wnorm + lmoe_align_up((size_t)n_expert * 4, 256) / 4;
+    float *xss = wnorm + lmoe_align_up((size_t)n_expert * 4, 256) / 4, *logits = xss + lmoe_align_up((size_t)rf_rows(t) * 4, 256) / 4;
     const int most = 227 * 1024 - 4096;
     static thread_local int c_dev = -1, c_sms = 0;
     int dev = 0;
@@ -440,16 +451,18 @@ cudaError_t launch_route_filter(const float *router, const float *bias, const fl
         c_dev = dev;
     }
     launch_pdl(route_prep_kernel, n_expert, 128, 0, s, router, hidden, n_expert, img, wnorm, flag);
-    // 128 tokens and all experts a block where that covers two thirds of the device, else 64 tokens and half of the experts
+    // 128 tokens a block where that covers two thirds of the device, else 64 and hidden in as many parts as there are SMs for
     const bool large = (t + 127) / 128 * 3 >= 2 * c_sms;
-    const int tm = large ? 128 : 64, ne = large || n_expert % 64 ? n_expert : n_expert / 2;
-    launch_pdl(large ? route_approx_kernel<128> : route_approx_kernel<64>, dim3((unsigned)((t + tm - 1) / tm), (unsigned)(n_expert / ne)), 320,
-               rf_stages(tm) * (RF_A_BYTES + ne * 128) + 1024, s, x, img, t, hidden, n_expert, ne, logits, xnorm, flag);
+    const int tiles = large ? (t + 127) / 128 : (t + 63) / 64;
+    int splits = 1;
+    while (!large && splits < RF_SPLITS && tiles * splits * 2 <= c_sms && (int64_t)t * splits * 2 <= rf_rows(t) && hidden / 64 % (2 * splits) == 0) splits *= 2;
+    launch_pdl(large ? route_approx_kernel<128> : route_approx_kernel<64>, dim3((unsigned)tiles, (unsigned)splits), 320,
+               RF_STAGES * (RF_A_BYTES + n_expert * 128) + 1024, s, x, img, t, hidden, n_expert, logits, xss, flag);
     // sixteen tokens a block where the rows fit and the blocks are enough for the device
     const int tb = rv_smem(16, hidden, n_expert) <= most && (t + 15) / 16 * 5 >= 4 * c_sms ? 16 : 8;
     auto verify = n_expert <= 128 ? (tb == 16 ? route_verify_kernel<16, 4> : route_verify_kernel<8, 4>)
                                   : (tb == 16 ? route_verify_kernel<16, 8> : route_verify_kernel<8, 8>);
-    launch_pdl(verify, (unsigned)((t + tb - 1) / tb), RV_WARPS * 32, rv_smem(tb, hidden, n_expert), s, router, x, bias, logits, xnorm, wnorm, t, hidden,
+    launch_pdl(verify, (unsigned)((t + tb - 1) / tb), RV_WARPS * 32, rv_smem(tb, hidden, n_expert), s, router, x, bias, logits, xss, splits, wnorm, t, hidden,
                n_expert, top_k, scale, norm, ids, weights);
     return cudaGetLastError();
 }
