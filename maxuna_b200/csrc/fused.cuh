@@ -9,6 +9,9 @@ enum {
     LMOE_FLAG_WAIT_TIMEOUT = 0x2,
     LMOE_FLAG_BAD_INDEX = 0x4,
 };
+// What follows it when a prompt's routing went through the filter (route_filter.cu): [LMOE_CONTROL_LEFT] the experts that
+// the bounds left, over all tokens of the call.
+enum { LMOE_CONTROL_LEFT = 4, LMOE_CONTROL_WORDS = 8 };
 
 // seam checks shared by the mat-vec and grouped-GEMM entry points (api.cu)
 lmoe_status lmoe_id_shape_check(const lmoe_expert_stack *stack, const void *x, int64_t t, int64_t x_per_row,

@@ -25,12 +25,12 @@ constexpr int RF_SPLITS = 4; // most parts that hidden is cut into
 constexpr int RF_AHEAD = 3; // stages whose words a producing thread has in flight
 
 // The router as f16 in the order of the B operand's stages (64 values of all experts: a 128-byte-swizzled tile), and its rows' norms.
-// A block per expert.  clear: the call's device flag.
+// A block per expert.  clear: the call's control words.
 __global__ void __launch_bounds__(128) route_prep_kernel(const float *__restrict__ router, int hidden, int n_expert, uint8_t *__restrict__ img,
                                                          float *__restrict__ wnorm, uint32_t *__restrict__ clear) {
     pdl_begin();
     const int e = blockIdx.x;
-    if (clear && e == 0 && threadIdx.x < 4) clear[threadIdx.x] = 0u;
+    if (e == 0 && threadIdx.x < LMOE_CONTROL_WORDS) clear[threadIdx.x] = 0u;
     const float4 *w = reinterpret_cast<const float4 *>(router + (size_t)e * hidden);
     float ss = 0.f;
     for (int ci = threadIdx.x; ci < hidden / 8; ci += 128) {
@@ -216,21 +216,29 @@ __global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__res
 constexpr int RV_WARPS = 16, RV_TOKENS = 4, RV_PIECE = 8;
 constexpr uint32_t RV_OUT = 0xffa5a5a5u; // in place of the logit of an expert that is out: a NaN that no operation results in
 
+// A bound below (side = -1) or above (1) of the specified sigmoid (route_math.cuh) of v, from the hardware's exponential and reciprocal.  These are
+// off by 2 + 1.2 |v| units in the last place (2^-23) of the exponential, which count (1 - sigmoid) times, and by three of the quotient; the specified one, which stops at
+// |v| = 87, by less.  The last term is for values below the normal range and for quotients that the hardware's division gives as 0.
+__device__ __forceinline__ float route_bound(float v, float side) {
+    const float a = fminf(fmaxf(-v, -88.f), 88.f), p = __fdividef(1.f, 1.f + __expf(a));
+    return p + side * (p * (8e-7f + (1e-6f + 2e-7f * fabsf(a)) * (1.f - p)) + 1e-37f);
+}
+
 template <int TB, int PER>
 __global__ void __launch_bounds__(RV_WARPS * 32, 1)
 route_verify_kernel(const float *__restrict__ router, const float *__restrict__ x, const float *__restrict__ bias, const float *__restrict__ approx,
                     const float *__restrict__ xss, int splits, const float *__restrict__ wnorm, int t, int hidden, int n_expert, int top_k, float scale, int norm,
-                    uint32_t *__restrict__ ids, float *__restrict__ weights) {
+                    uint32_t *__restrict__ ids, float *__restrict__ weights, uint32_t *__restrict__ control) {
     extern __shared__ __align__(16) uint8_t rv_raw[];
     float4 *xs = reinterpret_cast<float4 *>(rv_raw);
     float *lg = reinterpret_cast<float *>(rv_raw + (size_t)TB * hidden * 4); // [token][expert]
     uint32_t *items = reinterpret_cast<uint32_t *>(lg + TB * n_expert);        // expert << 16 | tokens
     uint32_t *mask = items + (TB + RV_TOKENS - 1) / RV_TOKENS * n_expert;    // by expert: the tokens it is left for
-    __shared__ int n_items;
+    __shared__ int n_items, n_left;
     __shared__ __align__(16) uint16_t cand[TB][32 + 64]; // by token: the experts left, up to 32, and room for their probabilities
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row4 = hidden / 4;
     const int t0 = blockIdx.x * TB, nt = min(TB, t - t0);
-    if (tid == 0) n_items = 0;
+    if (tid == 0) n_items = n_left = 0;
     for (int e = tid; e < n_expert; e += RV_WARPS * 32) mask[e] = 0u;
     pdl_begin();
     for (int i = tid; i < nt * row4; i += RV_WARPS * 32)
@@ -257,11 +265,12 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
         const float X = sqrtf(x2) * 1.001f, sub = 0x1p-25f * 1.01f * sqrtf((float)hidden);
 #pragma unroll
         for (int j = 0; j < PER; j++) {
-            // (a sigmoid from the hardware's exponential and reciprocal is good to 1e-6, sums round by less)
-            const float d = X * W[j] * (0x1p-10f + 0x1p-12f) + sub * (X + W[j]), eps = 4e-6f * (1.f + fabsf(b[j]));
-            lo[j] = __fdividef(1.f, 1.f + __expf(d - l[j])) + b[j] - eps;
-            hi[j] = __fdividef(1.f, 1.f + __expf(-d - l[j])) + b[j] + eps;
-            finite = finite && isfinite(l[j]) && isfinite(d) && isfinite(lo[j]) && isfinite(hi[j]);
+            const float d = X * W[j] * (0x1p-10f + 0x1p-12f) + sub * (X + W[j]);
+            // the bias comes in by the addition of the specified score, which keeps the order whatever the bias is: an infinite one, which
+            // excludes an expert or fixes it, and the type's lowest value bound the score as any other does
+            lo[j] = __fadd_rn(route_bound(l[j] - d, -1.f), b[j]);
+            hi[j] = __fadd_rn(route_bound(l[j] + d, 1.f), b[j]);
+            finite = finite && isfinite(l[j]) && isfinite(d);
         }
         const bool all = !__all_sync(0xffffffffu, finite);
         uint32_t key[PER], kth = 0u; // the top_k-th largest lower bound
@@ -293,8 +302,10 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
             }
             left += __popc(who);
         }
+        if (lane == 0) atomicAdd(&n_left, left);
     }
     __syncthreads();
+    if (tid == 0) atomicAdd(control + LMOE_CONTROL_LEFT, (uint32_t)n_left);
     for (int e = tid; e < n_expert; e += RV_WARPS * 32) {
         uint32_t m = mask[e];
         const int groups = (__popc(m) + RV_TOKENS - 1) / RV_TOKENS;
@@ -463,6 +474,6 @@ cudaError_t launch_route_filter(const float *router, const float *bias, const fl
     auto verify = n_expert <= 128 ? (tb == 16 ? route_verify_kernel<16, 4> : route_verify_kernel<8, 4>)
                                   : (tb == 16 ? route_verify_kernel<16, 8> : route_verify_kernel<8, 8>);
     launch_pdl(verify, (unsigned)((t + tb - 1) / tb), RV_WARPS * 32, rv_smem(tb, hidden, n_expert), s, router, x, bias, logits, xss, splits, wnorm, t, hidden,
-               n_expert, top_k, scale, norm, ids, weights);
+               n_expert, top_k, scale, norm, ids, weights, flag);
     return cudaGetLastError();
 }

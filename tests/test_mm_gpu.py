@@ -232,11 +232,52 @@ def test_prefill_routing_through_the_filter(dev, hidden, ne, top_k, t, bias):
     x[t // 2, 4] = float("inf")
     x[t // 2 + 1, 9] = float("nan")
     x[t - 1, 0] = 7e4
+    left = _check_routing(blk, x)
+    # ordinary tokens keep little more than top_k; about a dozen here keep them all
+    assert t * top_k <= left <= t * (1.5 * top_k + 3) + 12 * ne
+
+
+def _check_routing(blk, x):
+    """Ids and weights of a prompt against the stand-alone routing, to the bit; returns the count of experts that the filter left
+    (0: the filter did not run)."""
+    blk.workspace(x.shape[0])[:32].zero_()
     _, ids, w = blk.forward(x, return_routing=True, path="prefill")
     ids2, w2 = blk.route(x)
     torch.cuda.synchronize()
+    left = int(blk.workspace(x.shape[0])[16:20].view(torch.int32))
     blk.check_device_flag()
     assert torch.equal(ids, ids2) and torch.equal(w.view(torch.int32), w2.view(torch.int32))
+    return left
+
+
+@pytest.mark.parametrize("value", [float("-inf"), torch.finfo(torch.float32).min, -1e9, float("inf"), float("nan")])
+@pytest.mark.parametrize("hidden,ne,top_k,t", [(3072, 256, 10, 2048), (4096, 64, 8, 2500)])
+def test_prefill_routing_filter_with_any_bias(dev, hidden, ne, top_k, t, value):
+    """An expert that its bias excludes or fixes, by an infinity, the type's lowest value or NaN, leaves the other experts' bounds as they
+    are."""
+    from maxuna_b200.moe import MoeBlock
+
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(t)
+    b = 0.2 * torch.rand(ne, generator=gen, device=dev) - 0.1
+    b[3] = value
+    blk = MoeBlock.random(hidden, 256, ne, top_k, seed=hidden + ne, device=dev, bias=b)
+    left = _check_routing(blk, torch.randn(t, hidden, generator=gen, device=dev))
+    assert t * top_k <= left <= t * (1.5 * top_k + 3)
+
+
+def test_prefill_routing_filter_with_small_scores(dev):
+    """Scores near 1e-6 are told apart as well as others: the bounds are relative."""
+    from maxuna_b200.moe import MoeBlock
+
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(14)
+    blk = MoeBlock.random(3072, 256, 256, 10, seed=14, device=dev, bias=torch.zeros(256, device=dev))
+    x = torch.randn(2048, 3072, generator=gen, device=dev)
+    x[:, 0] = 10.0
+    blk.router[:, 0] = -1.4
+    left = _check_routing(blk, x)
+    assert 2048 * 10 <= left <= 2048 * 30
 
 
 def test_prefill_block_wide_ff(orc, dev):
