@@ -1,14 +1,15 @@
 // Many rows times ONE quantized matrix, as exact as the mat-vec kernels, on the 5th-generation tensor cores.
 // Reference: the plain quantized product of `QMatMul`, src/ops/mv_id.rs:54-56, for a prompt chunk (the shared expert op by op).
 //
-// The operands are exact in f16: a weight is its sub-block's integer scale times its integer, up to 945 for Q4_K and for Q6_K, up to 4096, in two
-// parts, scale / 8 and scale % 8; an activation is four base-256 digits of a 30-bit integer (mv_digits.cuh), which are columns of the B operand.
-// Over a super-block the sums stay below 2^24 where they count (the top digit is within +-64), so the f32 accumulators hold
-// integers; the float factors, the weights of the digits and the Q4_K mins (a product of their own, against the sub-block sums in
+// The operands are exact in f16, and so are the sums over a super-block in the f32 accumulators: integers of up to 2^24, whatever the values.  A Q4_K weight is its
+// sub-block's integer scale times its integer, up to 63 x 15, and an activation five digits within +-64, in base 128, of a 30-bit integer (mv_digits.cuh):
+// 256 x 945 x 64 = 0.92 x 2^24.  A Q6_K weight, up to 128 x 32, is in two parts with accumulators of their own, 8 x round(scale / 8) and the rest of the scale, up to 16 and 4 times 32, against
+// four base-256 digits within +-128: 256 x 512 x 128 = 2^24.  (With both parts in one accumulator, in eighths, and four digits for Q4_K, operands of one sign lost up
+// to five bits.)  The digits are columns of the B operand; the float factors, the weights of the digits and the Q4_K mins (a product of their own, against the sub-block sums in
 // three exact parts) come in once a super-block, as in mv_multi_kernel, whose integer products need their scales after every 32 or 16 values.
-// A super-block of 128 rows and 32 tokens takes 3.4 us (Q4_K; Q6_K 5.2), where its multiplies take 0.6 (1.2): the digits are made anew for every
-// 128 rows, 1700 of some 4300 cycles beside 1000 for storing them and 750 for the weights.  512 tokens [1024 x 3072] Q4_K 70 -> 47 us,
-// [3072 x 1024] Q6_K 113 -> 68, with the same error against 64 bits.
+// A super-block of 128 rows and 32 tokens takes 3.7 us (Q4_K; Q6_K 4.3 to 4.9), where its multiplies take 0.8 (1.2): the digits are made anew for every
+// 128 rows, and with the storing of them and of the weights they fill the issue slots.  512 tokens [1024 x 3072] Q4_K 72 -> 49 us,
+// [3072 x 1024] Q6_K 115 -> 66, with the same error against 64 bits.
 #include "common.cuh"
 #include "kquant.cuh"
 #include "mv_digits.cuh"
@@ -16,16 +17,18 @@
 
 namespace {
 
-constexpr int MD_ROWS = 128, MD_TOK = 32, MD_COLS = MV_NDIG * MD_TOK; // a block's weight rows and tokens; column 32 d + i: digit d of token i
+constexpr int MD_ROWS = 128, MD_TOK = 32; // a block's weight rows and tokens
 constexpr int MD_WORK = 512, MD_THREADS = MD_WORK + 32; // sixteen warps make operands and take results, one issues
 constexpr int MD_Q6_WORDS = 53, MD_Q6_PITCH = 55;       // words that hold a 210-byte block at an even address; of a row of the staged blocks
 constexpr int MD_TILE = 128 * 128; // an operand tile of 128 rows x 64 values
-constexpr int MD_B = 4 * MD_TILE, MD_SUMS = 3 * MD_TOK * 128;
+constexpr int MD_SUMS = 3 * MD_TOK * 128;
 
 template <int DT>
 struct MdCfg {
     static constexpr bool Q4 = DT == LMOE_Q4_K;
-    static constexpr int O_LOW = 4 * MD_TILE, O_B = (Q4 ? 4 : 8) * MD_TILE, O_MINS = O_B + MD_B, O_SUMS = O_MINS + MD_TILE;
+    static constexpr int NDIG = Q4 ? 5 : MV_NDIG, COLS = NDIG * MD_TOK; // digits of an activation; column 32 d + i: digit d of token i
+    static constexpr int B_TILE = COLS * 128;
+    static constexpr int O_LOW = 4 * MD_TILE, O_B = (Q4 ? 4 : 8) * MD_TILE, O_MINS = O_B + 4 * B_TILE, O_SUMS = O_MINS + MD_TILE;
     static constexpr int O_RAW = O_MINS; // Q6_K: the super-block's bytes of all rows
     static constexpr int SMEM = (Q4 ? O_SUMS + MD_SUMS : O_RAW + MD_ROWS * MD_Q6_PITCH * 4) + 1024;
 };
@@ -54,13 +57,23 @@ __device__ __forceinline__ uint32_t md_twice(float v) { // f16 pair (v, v)
     const uint32_t h = __half_as_ushort(__float2half_rn(v));
     return h | h << 16;
 }
-__device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+__device__ __forceinline__ void tc_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
 }
 __device__ __forceinline__ void md_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a),
                  "l"(b), "r"(idesc), "r"(accum) : "memory");
+}
+// A Q4_K activation as fields of 7, 7, 7, 7 and 4 bits from the lowest on, made positive by 64 and 8: f[p] holds, for the two values of pair p, fields 0 and 1 and the upper
+// two bits of the last one, f[4 + p] fields 2 and 3 and its lower two.
+__device__ __forceinline__ void md_fields(const int (&X)[8], uint32_t (&f)[8]) {
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        const int i = (p & 1) + 4 * (p >> 1);
+        const uint32_t a = (uint32_t)X[i] + 0x88102040u, c = (uint32_t)X[i + 2] + 0x88102040u, ah = a >> 14, ch = c >> 14;
+        f[p] = __byte_perm((a & 0x3FFFu) | (ah >> 2 & 0xC000u), (c & 0x3FFFu) | (ch >> 2 & 0xC000u), 0x5410);
+        f[4 + p] = __byte_perm(ah, ch, 0x5410);
+    }
 }
 // place of 16-byte chunk c of row r of an operand tile
 __device__ __forceinline__ int md_at(int r, int c) { return r * 128 + ((c ^ (r & 7)) << 4); }
@@ -75,7 +88,7 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
     using C = MdCfg<DT>;
     constexpr int TS = C::Q4 ? Q4K_BYTES : Q6K_BYTES, SUB = C::Q4 ? 32 : 16;
     extern __shared__ uint8_t md_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(md_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = md_raw + (0u - s32(md_raw) & 1023u); // (an offset: the compiler goes on knowing it as shared memory)
     uint8_t *a_st = smem, *b_st = smem + C::O_B, *mins = smem + C::O_MINS, *sums = smem + C::O_SUMS;
     __shared__ uint64_t done;
     __shared__ float sxs[4][MD_TOK];
@@ -103,23 +116,22 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
     pdl_begin();
     // weights: thread = (row, 64-k tile); activations: a warp has tokens warp and warp + 16; results: the same row, eight tokens
     const int r = tid & (MD_ROWS - 1), j = (tid >> 7) & 3, q = warp & 3, part8 = (warp >> 2) & 3;
-    const uint8_t *row = w + (size_t)min(r0 + r, n_out - 1) * row_bytes;
-    const float *src[2];
-    bool want[2];
+    const int row = min(r0 + r, n_out - 1);
+    int src[2]; // rows of x, or -1
 #pragma unroll
     for (int v = 0; v < 2; v++) {
         const int p = p0 + (warp & 15) + 16 * v;
-        want[v] = p < pairs && (ids == nullptr || ids[p] == 0u); // another id names no matrix of this stack: a zero row
-        src[v] = x + (want[v] ? ((size_t)(p / top_k) * x_per_row + (x_per_row == 1 ? 0 : p % top_k)) * k : 0);
+        const bool want = p < pairs && (ids == nullptr || ids[p] == 0u); // another id names no matrix of this stack: a zero row
+        src[v] = want ? (x_per_row == 1 ? p / top_k : p) : -1;           // (x_per_row is 1 or top_k)
     }
     MvX in[2];
     uint4 hdr, qa, qb;          // Q4_K: this tile's words
     auto load_x = [&](int b) {
 #pragma unroll
-        for (int v = 0; v < 2; v++) in[v].load(src[v] + (want[v] ? (size_t)b * QK_K : 0), want[v], lane);
+        for (int v = 0; v < 2; v++) in[v].load(x + (size_t)max(src[v], 0) * k + b * QK_K, src[v] >= 0, lane);
     };
     auto load_w = [&](int b) {
-        const uint8_t *blk = row + (size_t)b * TS;
+        const uint8_t *blk = w + (row * row_bytes + (int64_t)b * TS);
         if (C::Q4) {
             hdr = __ldg(reinterpret_cast<const uint4 *>(blk));
             qa = __ldg(reinterpret_cast<const uint4 *>(blk) + 1 + 2 * j);
@@ -142,32 +154,50 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
     for (int i = 0; i < 8; i++) acc[i] = odd[i] = 0.f;
     auto take = [&](int b, float d, float m) { // of super-block b: d, dmin of the row
         const uint32_t t0 = tmem + 256u * (b & 1) + ((uint32_t)(32 * q) << 16) + 8u * part8;
-        uint32_t v[MV_NDIG][8], s[MV_PARTS][8];
+        constexpr int MORE = C::Q4 ? MV_PARTS : C::NDIG; // parts of the mins' sums, or the low parts of the weights
 #pragma unroll
-        for (int e = 0; e < MV_NDIG; e++) tc_ld8(t0 + MD_TOK * e, v[e]);
-        if (C::Q4) {
+        for (int h = 0; h < 8; h += 4) {
+            float tot[4], off[4];
+            { // digits from the least significant on, so that only the last addition rounds at the size of the sum
+                uint32_t v[C::NDIG][4];
 #pragma unroll
-            for (int e = 0; e < MV_PARTS; e++) tc_ld8(t0 + MD_COLS + MD_TOK * e, s[e]);
-        }
-        tc_wait_ld();
+                for (int e = 0; e < C::NDIG; e++) tc_ld4(t0 + MD_TOK * e + h, v[e]);
+                tc_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            // digits from the least significant on, so that only the last addition rounds at the size of the sum
-            float tot = __uint_as_float(v[MV_NDIG - 1][i]);
+                for (int i = 0; i < 4; i++) {
+                    tot[i] = __uint_as_float(v[C::NDIG - 1][i]);
 #pragma unroll
-            for (int e = MV_NDIG - 2; e >= 0; e--) tot = __fmaf_rn(mv_digit_weight(e), __uint_as_float(v[e][i]), tot);
-            const float off = C::Q4 ? __uint_as_float(s[0][i]) + (__uint_as_float(s[1][i]) + __uint_as_float(s[2][i])) : 0.f;
-            // (two sums of half of the super-blocks, in turn, round less than one of all)
-            const float o = acc[i] + sxs[b & 3][8 * part8 + i] * (C::Q4 ? d * tot - m * off : d * tot);
-            acc[i] = odd[i];
-            odd[i] = o;
+                    for (int e = C::NDIG - 2; e >= 0; e--)
+                        tot[i] = __fmaf_rn(C::Q4 ? (float)(1 << 7 * (C::NDIG - 1 - e)) : mv_digit_weight(e), __uint_as_float(v[e][i]), tot[i]);
+                }
+            }
+            {
+                uint32_t v[MORE][4];
+#pragma unroll
+                for (int e = 0; e < MORE; e++) tc_ld4(t0 + C::COLS + MD_TOK * e + h, v[e]);
+                tc_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    off[i] = __uint_as_float(v[MORE - 1][i]);
+#pragma unroll
+                    for (int e = MORE - 2; e >= 0; e--)
+                        off[i] = C::Q4 ? __uint_as_float(v[e][i]) + off[i] : __fmaf_rn(mv_digit_weight(e), __uint_as_float(v[e][i]), off[i]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                // (two sums of half of the super-blocks, in turn, round less than one of all)
+                const float o = acc[h + i] + sxs[b & 3][8 * part8 + h + i] * (C::Q4 ? d * tot[i] - m * off[i] : d * __fmaf_rn(8.f, tot[i], off[i]));
+                acc[h + i] = odd[h + i];
+                odd[h + i] = o;
+            }
         }
         tc_fence_before();
     };
     bool ok = true;
     if (warp == MD_WORK / 32) {
         const bool el = elect_one();
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(MD_COLS >> 3) << 17) | ((uint32_t)(MD_ROWS >> 4) << 24);
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(C::COLS >> 3) << 17) | ((uint32_t)(MD_ROWS >> 4) << 24);
         const uint32_t idesc_m = (1u << 4) | ((uint32_t)(3 * MD_TOK >> 3) << 17) | ((uint32_t)(MD_ROWS >> 4) << 24);
         const uint64_t ad = umma_desc(s32(a_st)), bd = umma_desc(s32(b_st)), md = umma_desc(s32(mins)), sd = umma_desc(s32(sums));
         for (int b = 0; b < nb; b++) {
@@ -175,13 +205,14 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
             tc_fence_after();
             const uint32_t d = tmem + 256u * (b & 1);
             if (el) {
-                if (C::Q4) md_mma(d + MD_COLS, md, sd, idesc_m, 0u);
+                if (C::Q4) md_mma(d + C::COLS, md, sd, idesc_m, 0u);
 #pragma unroll
                 for (uint32_t t = 0; t < 4; t++) {
 #pragma unroll
                     for (uint32_t kk = 0; kk < 4; kk++) {
-                        md_mma(d, ad + t * (MD_TILE >> 4) + 2 * kk, bd + t * (MD_TILE >> 4) + 2 * kk, idesc, t | kk);
-                        if (!C::Q4) md_mma(d, ad + ((C::O_LOW + t * MD_TILE) >> 4) + 2 * kk, bd + t * (MD_TILE >> 4) + 2 * kk, idesc, 1u);
+                        const uint64_t bt = bd + t * (C::B_TILE >> 4) + 2 * kk;
+                        md_mma(d, ad + t * (MD_TILE >> 4) + 2 * kk, bt, idesc, t | kk);
+                        if (!C::Q4) md_mma(d + C::COLS, ad + ((C::O_LOW + t * MD_TILE) >> 4) + 2 * kk, bt, idesc, t | kk);
                     }
                 }
                 tc_commit<1>(&done);
@@ -196,11 +227,22 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
         load_w(0);
     }
     for (int b = 0; b < nb && warp < MD_WORK / 32; b++) {
-        uint2 dig[2][MV_NDIG];
+        uint32_t dig[2][8]; // Q4_K: words (0 2), (1 3), (4 6), (5 7) of the lower 14 bits and of the others, see md_fields; Q6_K: two words a digit
         float sx[2];
         __half sub[2][MV_PARTS];
 #pragma unroll
-        for (int v = 0; v < 2; v++) mv_digits<SUB>(in[v], dig[v], sx[v], sub[v]);
+        for (int v = 0; v < 2; v++) {
+            int X[8];
+            mv_integers<SUB>(in[v], X, sx[v], sub[v]);
+            if constexpr (C::Q4) {
+                md_fields(X, dig[v]);
+            } else {
+                uint2 d[MV_NDIG];
+                mv_bytes(X, d);
+#pragma unroll
+                for (int e = 0; e < MV_NDIG; e++) dig[v][2 * e] = d[e].x, dig[v][2 * e + 1] = d[e].y;
+            }
+        }
         if (b + 1 < nb) load_x(b + 1);
         if (!C::Q4) asm volatile("cp.async.wait_group 0;\n\tbar.sync 1, 512;" ::: "memory"); // all rows' bytes are there
         if (b && ok) ok = mb_wait(&done, (uint32_t)(b - 1) & 1u); // the operands of the super-block before have been multiplied
@@ -208,12 +250,30 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
 #pragma unroll
         for (int v = 0; v < 2; v++) {
             const int i = warp + 16 * v;
+            uint8_t *to = b_st + (lane >> 3) * C::B_TILE;
+            auto put = [&](int d, const uint32_t (&h)[4]) { *reinterpret_cast<uint4 *>(to + md_at(MD_TOK * d + i, lane & 7)) = make_uint4(h[0], h[1], h[2], h[3]); };
+            // f16 pairs in the order of the weights' chunks: 0 2 1 3 4 6 5 7
+            uint32_t h[4];
+            if constexpr (C::Q4) {
+                const uint32_t seven = 0x007F007Fu, off = 0x64406440u;
 #pragma unroll
-            for (int d = 0; d < MV_NDIG; d++) { // bytes as f16 pairs, in the order of the weights' chunks: 0 2 1 3 4 6 5 7
-                const uint32_t lo = dig[v][d].x ^ 0x80808080u, hi = dig[v][d].y ^ 0x80808080u, one = 0x64646464u, off = 0x64806480u;
-                *reinterpret_cast<uint4 *>(b_st + (lane >> 3) * MD_TILE + md_at(MD_TOK * d + i, lane & 7)) =
-                    make_uint4(md_sub(__byte_perm(lo, one, 0x4240), off), md_sub(__byte_perm(lo, one, 0x4341), off),
-                               md_sub(__byte_perm(hi, one, 0x4240), off), md_sub(__byte_perm(hi, one, 0x4341), off));
+                for (int d = 1; d < 5; d++) {
+#pragma unroll
+                    for (int p = 0; p < 4; p++) h[p] = md_sub(md_lop((d < 3 ? dig[v][4 + p] : dig[v][p]) >> ((d & 1) ? 7 : 0), seven, 0x64006400u), off);
+                    put(d, h);
+                }
+#pragma unroll
+                for (int p = 0; p < 4; p++)
+                    h[p] = md_sub(md_lop(dig[v][p] >> 12, 0x000C000Cu, md_lop(dig[v][4 + p] >> 14, 0x00030003u, 0x64006400u)), 0x64086408u);
+                put(0, h);
+            } else {
+#pragma unroll
+                for (int d = 0; d < MV_NDIG; d++) {
+                    const uint32_t lo = dig[v][2 * d] ^ 0x80808080u, hi = dig[v][2 * d + 1] ^ 0x80808080u, one = 0x64646464u, off = 0x64806480u;
+                    h[0] = md_sub(__byte_perm(lo, one, 0x4240), off), h[1] = md_sub(__byte_perm(lo, one, 0x4341), off);
+                    h[2] = md_sub(__byte_perm(hi, one, 0x4240), off), h[3] = md_sub(__byte_perm(hi, one, 0x4341), off);
+                    put(d, h);
+                }
             }
             if (C::Q4 && (lane & 3) == 0) {
 #pragma unroll
@@ -223,6 +283,8 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
             if (lane == 0) sxs[b & 3][i] = sx[v];
         }
         uint8_t *a = a_st + j * MD_TILE;
+        int rr = r;
+        asm volatile("" : "+r"(rr)); // the places of the eight stores are worked out here and not kept in registers
         uint16_t d6 = 0;
         if constexpr (C::Q4) {
             uint32_t scs[2], mn[2];
@@ -241,14 +303,14 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
 #pragma unroll
                 for (int c = 0; c < 4; c++) { // (1024 + q) scale - 1024 scale: exact
                     const uint32_t u0 = v[2 * c] >> (4 * h), u1 = v[2 * c + 1] >> (4 * h);
-                    *reinterpret_cast<uint4 *>(a + md_at(r, 4 * h + c)) =
+                    *reinterpret_cast<uint4 *>(a + md_at(rr, 4 * h + c)) =
                         make_uint4(md_fma(md_lop(u0, 0x000F000Fu, 0x64006400u), s, c0), md_fma(md_lop(u0 >> 8, 0x000F000Fu, 0x64006400u), s, c0),
                                    md_fma(md_lop(u1, 0x000F000Fu, 0x64006400u), s, c0), md_fma(md_lop(u1 >> 8, 0x000F000Fu, 0x64006400u), s, c0));
                 }
             }
         } else {
             // half j / 2, groups 2 (j % 2) + h
-            const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(row + (size_t)b * TS) & 2) * 8u;
+            const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(w + (row * row_bytes + (int64_t)b * TS)) & 2) * 8u;
             const uint32_t *st = reinterpret_cast<const uint32_t *>(smem + C::O_RAW) + r * MD_Q6_PITCH;
             auto word = [&](int i) { return __funnelshift_r(st[i], st[i + 1], off); }; // bytes 4 i .. 4 i + 3 of the block
             const uint32_t scs = word(48 + 2 * (j >> 1) + (j & 1));
@@ -258,7 +320,7 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     const int s = (int8_t)(scs >> (16 * h + (c < 2 ? 0 : 8)));
-                    const uint32_t hi = md_twice((float)(s >> 3)), lo = md_twice((float)(s & 7) * 0.125f);
+                    const uint32_t hi = md_twice((float)((s + 4) >> 3)), lo = md_twice((float)(s - ((s + 4) & ~7)));
                     uint32_t e[4];
 #pragma unroll
                     for (int i = 0; i < 2; i++) {
@@ -268,12 +330,12 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
                         e[2 * i] = md_sub(__byte_perm(q6, 0x64646464u, 0x4240), 0x64206420u);
                         e[2 * i + 1] = md_sub(__byte_perm(q6, 0x64646464u, 0x4341), 0x64206420u);
                     }
-                    *reinterpret_cast<uint4 *>(a + md_at(r, 4 * h + c)) = make_uint4(md_mul(e[0], hi), md_mul(e[1], hi), md_mul(e[2], hi), md_mul(e[3], hi));
-                    *reinterpret_cast<uint4 *>(a + C::O_LOW + md_at(r, 4 * h + c)) = make_uint4(md_mul(e[0], lo), md_mul(e[1], lo), md_mul(e[2], lo), md_mul(e[3], lo));
+                    *reinterpret_cast<uint4 *>(a + md_at(rr, 4 * h + c)) = make_uint4(md_mul(e[0], hi), md_mul(e[1], hi), md_mul(e[2], hi), md_mul(e[3], hi));
+                    *reinterpret_cast<uint4 *>(a + C::O_LOW + md_at(rr, 4 * h + c)) = make_uint4(md_mul(e[0], lo), md_mul(e[1], lo), md_mul(e[2], lo), md_mul(e[3], lo));
                 }
             }
         }
-        const float d_now = C::Q4 ? lmoe_h2f((uint16_t)(hdr.x & 0xffff)) : 8.f * lmoe_h2f(d6);
+        const float d_now = C::Q4 ? lmoe_h2f((uint16_t)(hdr.x & 0xffff)) : lmoe_h2f(d6);
         const float m_now = C::Q4 ? lmoe_h2f((uint16_t)(hdr.x >> 16)) * MV_SUM_UNSCALE : 0.f;
         if (C::Q4 && b + 1 < nb) load_w(b + 1);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

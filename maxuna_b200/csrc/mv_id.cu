@@ -897,19 +897,21 @@ cudaError_t mv_device(int &dev, int &sms) {
 bool mv_multi_better(int n_expert, int n_out, int64_t pairs, int sms) {
     return n_expert == 1 && (pairs + MM_COLS - 1) / MM_COLS * ((n_out + MV_ROWS - 1) / MV_ROWS) >= sms && pairs > 4;
 }
-// The tensor-core kernel of mv_dense.cu takes a super-block of 128 rows and 32 pairs at a time, 3.4 us Q4_K, 5.2 Q6_K, whatever the number
+// The tensor-core kernel of mv_dense.cu takes a super-block of 128 rows and 32 pairs at a time, 3.7 us Q4_K, 4.9 Q6_K, whatever the number
 // of blocks on the device; these kernels' time goes with the work.  us here / there, cold L2:
 //   pairs                      32           64          128          256          512         1024         4096
-//   [1024 x 3072] Q4_K  20.5 / 43.1  30.8 / 45.0  34.8 / 45.1  55.5 / 45.1  69.7 / 47.1   135 / 86.0    459 / 285
-//   [768 x 2048] Q4_K   18.4 / 32.8  22.5 / 32.8  26.7 / 32.8  43.0 / 34.8  47.1 / 34.8  74.8 / 63.5    239 / 179
-//   [3072 x 1024] Q6_K  22.6 / 26.6  41.0 / 26.6  43.0 / 26.6  66.6 / 47.1   113 / 67.6   201 / 128     773 / 428
-//   [2048 x 768] Q6_K   21.5 / 21.4  34.8 / 22.5  45.1 / 22.5  38.9 / 22.5  67.6 / 38.9   127 / 71.7    436 / 231
+//   [1024 x 3072] Q4_K  21.5 / 48.1  31.8 / 49.2  34.8 / 49.2  55.5 / 49.2  71.7 / 49.3   137 / 94.2    473 / 309
+//   [768 x 2048] Q4_K   18.5 / 36.9  22.6 / 36.9  27.6 / 36.9  42.0 / 36.9  49.2 / 37.1  76.8 / 69.6    244 / 195
+//   [3072 x 1024] Q6_K  23.5 / 24.6  41.0 / 24.6  43.0 / 25.6  67.6 / 45.1   115 / 65.5   206 / 122     787 / 410
+//   [2048 x 768] Q6_K   22.6 / 20.6  34.8 / 20.7  45.1 / 20.5  37.9 / 22.5  69.6 / 36.9   129 / 68.7    442 / 224
+// Of 264 matrices and counts that the rule sends there, drawn from 5 to 100352 rows of 256 to 12288 and 64 to 16384 pairs, one is longer there
+// ([768 x 2048] Q6_K, 160 pairs: 38.9 / 41.0), the rest take 0.2 to 1.0 times as long.
 // Below 64 pairs a chain's shared product is better off in the launch of the routed ones (48 tokens op by op, 256 experts: 443 us so, 460 apart).
 bool mv_dense_better(int dt, const uint8_t *w, int n_expert, int n_out, int k, int64_t pairs, int sms) {
     if (n_expert != 1 || pairs < 64 || (reinterpret_cast<uintptr_t>(w) & 15u)) return false;
     const bool q4 = dt == LMOE_Q4_K, multi = mv_multi_better(n_expert, n_out, pairs, sms);
     const int64_t rounds = (((int64_t)n_out + 127) / 128 * ((pairs + 31) / 32) + sms - 1) / sms;
-    const double there = 5.0 + (double)rounds * (k / QK_K) * (q4 ? 3.4 : 5.2);
+    const double there = 5.0 + (double)rounds * (k / QK_K) * (q4 ? 3.7 : 4.9);
     return there < 7.0 + (double)pairs * n_out * k * (multi ? (q4 ? 4.2e-8 : 6.8e-8) : (q4 ? 6.0e-8 : 1.5e-7));
 }
 // a bulk copy starts and ends on 16 bytes: every expert must; the end of a single matrix may be ragged

@@ -207,6 +207,42 @@ def test_mv_dense(orc, dev, dt, name, n_out, k, t, top_k, xpr):
     assert not np.isfinite(bad[3, 0]).any() and np.isnan(bad[5, 0]).all() and np.array_equal(bad[keep], got[keep])
 
 
+@pytest.mark.parametrize("case", ["top", "low", "negative"])
+@pytest.mark.parametrize("dt,name", DTYPES)
+def test_mv_dense_large_sums(dev, dt, name, case):
+    """A super-block's sums at their largest: weights of one sign and near the largest integers, activations of one sign whose leading
+    (`top`) or lower (`low`) bits are nearly all set, an odd number of weight rows and of super-blocks.  The sums of a super-block are exact, d and the
+    scale of the activations are powers of two and the mins are zero, so what rounds, by 2^-24 of its own size, are the additions of the digits' sums: two at up to the size of the
+    result, the lower ones a hundredth of that; for Q6_K these two in the part that comes in eight times (at most 1 + 4 / 121 of the result), and then the
+    addition of the other part."""
+    from maxuna_b200 import ops
+    from maxuna_b200.gguf import ExpertStack
+
+    n_out, k, t = 131, 256, 2001
+    rng = np.random.default_rng(dt)
+    b = np.zeros((n_out, 144 if dt == 12 else 210), dtype=np.uint8)
+    if dt == 12:
+        b[:, 0:2] = np.float16(2.0 ** -7).reshape(1).view(np.uint8)
+        sc = rng.integers(58, 64, (n_out, 8))  # scales; the mins are zero
+        b[:, 4:8] = sc[:, :4] | (sc[:, 4:] >> 4) << 6
+        b[:, 12:16] = sc[:, 4:] & 15
+        q = rng.integers(13, 16, (n_out, 8, 32))
+        b[:, 16:144] = (q[:, 0::2] | q[:, 1::2] << 4).reshape(n_out, 128)
+    else:
+        b[:, 208:210] = np.float16(2.0 ** -7).reshape(1).view(np.uint8)
+        b[:, 192:208] = rng.integers(-128, -120, (n_out, 16)).astype(np.int8).view(np.uint8)  # times values of -32 to -29
+        b[:, 0:128] = rng.integers(0, 4, (n_out, 128)) * 0x11
+    stack = ExpertStack.from_bytes(b.reshape(-1), dt, 1, n_out, k, device=dev)
+    bits = rng.integers(0, 1 << 5, (t, k)) * 0x010101  # five low bits of every byte at random, the others set
+    x = (0x7F0000 | 0x6060 | bits & 0x1F1F1F if case == "low" else 0xE06060 | bits).astype(np.int64)
+    x = (x if case == "low" else x << 6).astype(np.float64) * 2.0 ** -29
+    x[:, 17] = 1.0 if case == "low" else 1.96875  # the block's scale: 2^29 integers to 1
+    x = (-x if case == "negative" else x).astype(np.float32).reshape(t, 1, k)
+    got = ops.mul_mv_id(stack, torch.from_numpy(x).to(dev), torch.zeros(t, 1, dtype=torch.int32, device=dev)).cpu().numpy()[:, 0]
+    want = (torch.from_numpy(x).to(dev).double()[:, 0] @ stack.dequantize()[0].double().T).cpu().numpy()
+    assert np.abs(got / want - 1).max() < (2.1 if dt == 12 else 3.2) * 2.0 ** -24
+
+
 @pytest.mark.parametrize("n_expert,n_out,k,t,top_k", [(4, 512, 768, 17, 2), (1, 1100, 512, 285, 1), (1, 64, 8192, 40, 1)])
 @pytest.mark.parametrize("dt,name", DTYPES)
 def test_mv_range_and_resolution(orc, dev, dt, name, n_expert, n_out, k, t, top_k):
