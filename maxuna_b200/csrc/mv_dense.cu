@@ -144,7 +144,10 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
                 uint32_t *to = reinterpret_cast<uint32_t *>(smem + C::O_RAW) + rr * MD_Q6_PITCH;
 #pragma unroll
                 for (int o = 0; o < 64; o += 32)
-                    if (lane + o < MD_Q6_WORDS) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s32(to + lane + o)), "l"(g4 + lane + o) : "memory");
+                    if (lane + o < MD_Q6_WORDS) { // (of the last word of a block at a word's start only two bytes are the block's, and may be the matrix's last)
+                        const uint32_t n = lane + o == MD_Q6_WORDS - 1 && !(reinterpret_cast<uintptr_t>(g) & 2) ? 2u : 4u;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(s32(to + lane + o)), "l"(g4 + lane + o), "r"(n) : "memory");
+                    }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         }

@@ -178,6 +178,7 @@ def test_mv_many_pairs_of_one_matrix(orc, dev, dt, name, n_out, k, pairs):
     (1000, 1280, 167, 2, 2),  # an odd number of super-blocks; a row of x for every slot
     (390, 768, 513, 2, 1),    # slots that share a row of x
     (128, 512, 8200, 1, 1),   # several rounds over the device
+    (131, 768, 1201, 1, 1),   # an odd number of blocks in all: the last Q6_K one ends in the middle of a word
 ])
 @pytest.mark.parametrize("dt,name", DTYPES)
 def test_mv_dense(orc, dev, dt, name, n_out, k, t, top_k, xpr):
