@@ -139,49 +139,30 @@ __global__ void sum_slots_kernel(const float *__restrict__ y, const float *__res
 
 // Same sum when the partial rows are unscaled and in expert-sorted order: row spos[flat id] of `y`
 // times scale[that row]; likewise for the shared expert's rows, then + residual.  A negative position marks an empty slot.
-// Twelve rows' loads are in flight per element.  A block takes a token and, where the tokens are many (per = 1), all of its columns: the
-// rows' places and scales, which the loads wait for, are read once for them (hidden 3072, ten experts and the shared one, 2048 / 16384 tokens 59 / 444 us
-// with a block for every 256 columns, 55 / 372 so, 6.5 TB/s; 512 tokens 18.5 and 21.5).
-__global__ void __launch_bounds__(256, 3) sum_sorted_kernel(const float *__restrict__ y, const float *__restrict__ scale,
-                                  const int32_t *__restrict__ spos, const float *__restrict__ shared,
-                                  const float *__restrict__ sh_scale, const int32_t *__restrict__ sh_spos,
-                                  const float *__restrict__ residual, int top_k, int n4, int per, float *__restrict__ out) {
-    const int64_t tok = blockIdx.x / (unsigned)per;
-    const int c0 = (int)(blockIdx.x % (unsigned)per) * 256 + threadIdx.x;
-    const int32_t *sp = spos + tok * top_k;
-    const int n = top_k + (shared ? 1 : 0);
-    if (n <= 12 && per == 1) {
-        int row[12];
-        float sc[12];
-#pragma unroll
-        for (int k = 0; k < 12; k++) {
-            const bool sh = k == top_k;
-            row[k] = k >= n ? -1 : (sh ? (sh_spos ? sh_spos[tok] : (int)tok) : sp[k]);
-            const float *sb = sh ? sh_scale : scale;
-            sc[k] = row[k] >= 0 && sb ? sb[row[k]] : 1.0f;
+struct SumRows {
+    const float *y, *scale;
+    const int32_t *spos;
+    const float *shared, *sh_scale;
+    const int32_t *sh_spos;
+    const float *residual;
+    int64_t t;
+    int top_k, n4;
+    float *out;
+    __device__ __forceinline__ void put(int64_t i, float4 s) const {
+        if (residual) {
+            const float4 v = reinterpret_cast<const float4 *>(residual)[i];
+            s.x = __fadd_rn(s.x, v.x); s.y = __fadd_rn(s.y, v.y); s.z = __fadd_rn(s.z, v.z); s.w = __fadd_rn(s.w, v.w);
         }
-        for (int c = c0; c < n4; c += per * 256) {
-            float4 v[12];
-#pragma unroll
-            for (int k = 0; k < 12; k++)
-                v[k] = row[k] >= 0 ? __ldcs(reinterpret_cast<const float4 *>(k == top_k ? shared : y) + (int64_t)row[k] * n4 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int k = 0; k < 12; k++) {
-                if (row[k] >= 0) {
-                    s.x = __fadd_rn(s.x, __fmul_rn(v[k].x, sc[k])); s.y = __fadd_rn(s.y, __fmul_rn(v[k].y, sc[k]));
-                    s.z = __fadd_rn(s.z, __fmul_rn(v[k].z, sc[k])); s.w = __fadd_rn(s.w, __fmul_rn(v[k].w, sc[k]));
-                }
-            }
-            if (residual) {
-                const float4 v = reinterpret_cast<const float4 *>(residual)[tok * n4 + c];
-                s.x = __fadd_rn(s.x, v.x); s.y = __fadd_rn(s.y, v.y); s.z = __fadd_rn(s.z, v.z); s.w = __fadd_rn(s.w, v.w);
-            }
-            reinterpret_cast<float4 *>(out)[tok * n4 + c] = s;
-        }
-        return;
+        reinterpret_cast<float4 *>(out)[i] = s;
     }
-    for (int c = c0; c < n4; c += per * 256) { // few tokens, or more rows: twelve at a time
+    __device__ __forceinline__ static void add(float4 &s, const float4 v, float sc) {
+        s.x = __fadd_rn(s.x, __fmul_rn(v.x, sc)); s.y = __fadd_rn(s.y, __fmul_rn(v.y, sc));
+        s.z = __fadd_rn(s.z, __fmul_rn(v.z, sc)); s.w = __fadd_rn(s.w, __fmul_rn(v.w, sc));
+    }
+    // four columns of a token; twelve rows' loads are in flight
+    __device__ __forceinline__ void columns(int64_t tok, int64_t c) const {
+        const int32_t *sp = spos + tok * top_k;
+        const int n = top_k + (shared ? 1 : 0);
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int k0 = 0; k0 < n; k0 += 12) {
             float4 v[12];
@@ -198,22 +179,61 @@ __global__ void __launch_bounds__(256, 3) sum_sorted_kernel(const float *__restr
                 present |= (uint32_t)(r >= 0) << j;
             }
 #pragma unroll
-            for (int j = 0; j < 12; j++) {
-                if (present & (1u << j)) {
-                    s.x = __fadd_rn(s.x, __fmul_rn(v[j].x, sc[j])); s.y = __fadd_rn(s.y, __fmul_rn(v[j].y, sc[j]));
-                    s.z = __fadd_rn(s.z, __fmul_rn(v[j].z, sc[j])); s.w = __fadd_rn(s.w, __fmul_rn(v[j].w, sc[j]));
-                }
-            }
+            for (int j = 0; j < 12; j++)
+                if (present & (1u << j)) add(s, v[j], sc[j]);
         }
-        if (residual) {
-            const float4 v = reinterpret_cast<const float4 *>(residual)[tok * n4 + c];
-            s.x = __fadd_rn(s.x, v.x); s.y = __fadd_rn(s.y, v.y); s.z = __fadd_rn(s.z, v.z); s.w = __fadd_rn(s.w, v.w);
-        }
-        reinterpret_cast<float4 *>(out)[tok * n4 + c] = s;
+        put(tok * n4 + c, s);
+    }
+};
+__global__ void __launch_bounds__(256) sum_sorted_kernel(const SumRows R) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= R.t * R.n4) return;
+    const int64_t tok = i / R.n4;
+    R.columns(tok, i - tok * R.n4);
+}
+// A block a token: up to twelve rows' places and scales, which the loads wait for, are read once for all of its columns.
+__global__ void __launch_bounds__(256, 3) sum_tokens_kernel(const SumRows R) {
+    const int64_t tok = blockIdx.x;
+    const int n = R.top_k + (R.shared ? 1 : 0);
+    if (n > 12) {
+        for (int c = threadIdx.x; c < R.n4; c += 256) R.columns(tok, c);
+        return;
+    }
+    int row[12];
+    float sc[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+        const bool sh = k == R.top_k;
+        row[k] = k >= n ? -1 : (sh ? (R.sh_spos ? R.sh_spos[tok] : (int)tok) : R.spos[tok * R.top_k + k]);
+        const float *sb = sh ? R.sh_scale : R.scale;
+        sc[k] = row[k] >= 0 && sb ? sb[row[k]] : 1.0f;
+    }
+    for (int c = threadIdx.x; c < R.n4; c += 256) {
+        float4 v[12];
+#pragma unroll
+        for (int k = 0; k < 12; k++)
+            v[k] = row[k] >= 0 ? __ldcs(reinterpret_cast<const float4 *>(k == R.top_k ? R.shared : R.y) + (int64_t)row[k] * R.n4 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 12; k++)
+            if (row[k] >= 0) SumRows::add(s, v[k], sc[k]);
+        R.put(tok * R.n4 + c, s);
     }
 }
-// blocks of a token: one once the tokens fill the device several times over, else one for every 256 columns
-int sum_sorted_per(int64_t t, int64_t n4) { return t >= 1024 ? 1 : (int)((n4 + 255) / 256); }
+// Which of the two, us for (columns over the whole grid) / (a block a token), cold L2, 11 rows a token:
+//   hidden              512          1024         1536         2048         3072         7168
+//   1024 tokens    14.3 / 14.3  18.4 / 16.4  22.5 / 22.5  26.6 / 26.6  34.8 / 34.8  69.6 / 67.6
+//   2048 tokens    18.5 / 20.5  26.6 / 24.6  34.8 / 34.8  45.1 / 41.0  61.4 / 57.3   129 / 119
+//   16384 tokens   77.8 / 94.1   150 / 137    217 / 200    289 / 252    428 / 373
+// Rows of fewer than 2048 columns leave threads without work, or gain with some numbers of rows and lose with others (16384 tokens of 1536, 2 / 5 / 9 / 11 rows
+// 131 / 135, 145 / 152, 178 / 180, 217 / 200; of 1280 111 / 129, 123 / 145, 150 / 168, 182 / 182).  More than twelve rows gain from 2048 tokens on (17 rows of 3072, 1024 /
+// 2048 / 4096 tokens 51.2 / 51.2, 92.2 / 85.9, 172 / 162; 24 rows of 7168, 1024 tokens 131 / 135).
+bool sum_by_token(int64_t t, int64_t n4, int n) { return t >= (n > 12 ? 2048 : 1024) && n4 >= 512 && t * n4 >= 768 * 1024; }
+cudaError_t launch_sum_sorted(const SumRows &R, cudaStream_t s) {
+    if (sum_by_token(R.t, R.n4, R.top_k + (R.shared ? 1 : 0))) sum_tokens_kernel<<<(unsigned)R.t, 256, 0, s>>>(R);
+    else sum_sorted_kernel<<<(unsigned)((R.t * R.n4 + 255) / 256), 256, 0, s>>>(R);
+    return cudaGetLastError();
+}
 
 // Expert-parallel dispatch packing: the routed rows of expert e (list `ids_map[e]`) go to positions
 // [prefix(e), prefix(e) + tpe[e]) of the send buffers, as f16; experts are contiguous per destination rank,
@@ -418,8 +438,7 @@ static lmoe_status experts_prefill(const lmoe_layer *L, const void *x, int x_f16
     }
     const int64_t n = t * (H / 4);
     if (sorted)
-        sum_sorted_kernel<<<(unsigned)(t * sum_sorted_per(t, H / 4)), 256, 0, s>>>(y, rscale, spos, shared ? y : nullptr, rscale, spos + rows, residual,
-                                                                                   (int)top_k, (int)(H / 4), sum_sorted_per(t, H / 4), out);
+        LMOE_CUDA(launch_sum_sorted({y, rscale, spos, shared ? y : nullptr, rscale, spos + rows, residual, t, (int)top_k, (int)(H / 4), out}, s));
     else
         sum_slots_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(y, shared ? ysh : nullptr, residual, t, (int)top_k, (int)(H / 4), out);
     LMOE_LAUNCH_CHECK("sum_slots_kernel");
@@ -788,9 +807,6 @@ extern "C" lmoe_status lmoe_ep_combine(const float *rows, const int32_t *row_pos
     if ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(shared)) & 15u)
         return lmoe_fail(LMOE_ERR_INVALID, "ep_combine: rows, shared and out must be 16-byte aligned");
     if (t == 0) return LMOE_OK;
-    const int per = sum_sorted_per(t, hidden / 4);
-    sum_sorted_kernel<<<(unsigned)(t * per), 256, 0, (cudaStream_t)stream>>>(rows, nullptr, row_pos, shared, nullptr, nullptr, nullptr, (int)top_k,
-                                                                       (int)(hidden / 4), per, out);
-    LMOE_LAUNCH_CHECK("sum_sorted_kernel");
+    LMOE_CUDA(launch_sum_sorted({rows, nullptr, row_pos, shared, nullptr, nullptr, nullptr, t, (int)top_k, (int)(hidden / 4), out}, (cudaStream_t)stream));
     return LMOE_OK;
 }

@@ -660,3 +660,25 @@ def test_ffn_mv_errors(dev):
                 (e, ids, w, (e[0], e[1], mk(14, 1, 256, 256)), x), (e, ids, w.double(), None, x)):
         with pytest.raises(LmoeError):
             ops.ffn_mv(*bad)
+
+
+@pytest.mark.parametrize("t,hidden", [(1023, 2048), (1535, 2048), (1536, 2048), (1024, 3076), (2047, 2052), (2048, 2052), (1100, 2044), (2, 4), (333, 1540)])
+@pytest.mark.parametrize("top_k,shared", [(1, False), (3, True), (11, True), (12, False), (12, True), (25, False)])
+def test_sum_of_sorted_rows(dev, t, hidden, top_k, shared):
+    """The slot sum by token and by columns, on either side of the line between them and of twelve rows: the additions in slot order, empty
+    slots left out, the shared row last.  f32 additions in the same order, so the bits."""
+    from maxuna_b200._native import check, lib
+    from maxuna_b200.gguf import stream_ptr
+
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(t + hidden + top_k)
+    rows = torch.randn(t * top_k, hidden, generator=gen, device=dev)
+    pos = torch.randperm(t * top_k, generator=gen, device=dev).to(torch.int32).view(t, top_k)
+    pos[torch.rand(t, top_k, generator=gen, device=dev) < 0.1] = -1
+    sh = torch.randn(t, hidden, generator=gen, device=dev) if shared else None
+    out = torch.empty(t, hidden, device=dev)
+    check(lib().lmoe_ep_combine(rows.data_ptr(), pos.data_ptr(), sh.data_ptr() if shared else None, t, top_k, hidden, out.data_ptr(), stream_ptr()))
+    want = torch.zeros(t, hidden, device=dev)
+    for k in range(top_k):
+        want = torch.where((pos[:, k] >= 0)[:, None], want + rows[pos[:, k].clamp(min=0).long()], want)
+    assert torch.equal(out, want + sh if shared else want)
