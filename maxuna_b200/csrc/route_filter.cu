@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__res
         flag[1] = 0x2000u + warp;
         flag[2] = blockIdx.x;
     }
-    __syncthreads();
+    if (__syncthreads_or(!ok)) // a wait ran out: no bound is known, and the tokens keep all their experts
+        for (int i = tid; i < nt * n_expert; i += 320) logits[((size_t)blockIdx.y * t + t0) * n_expert + i] = __int_as_float(0x7fffffff);
     if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
 }
 
