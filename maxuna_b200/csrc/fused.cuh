@@ -10,8 +10,8 @@ enum {
     LMOE_FLAG_BAD_INDEX = 0x4,
 };
 // What follows it when a prompt's routing went through the filter (route_filter.cu): [LMOE_CONTROL_LEFT] the experts that
-// the bounds left, over all tokens of the call.
-enum { LMOE_CONTROL_LEFT = 4, LMOE_CONTROL_WORDS = 8 };
+// the bounds left, over all tokens of the call, [LMOE_CONTROL_DENSE] the tokens that got all their logits from route_dense_kernel.
+enum { LMOE_CONTROL_LEFT = 4, LMOE_CONTROL_DENSE = 5, LMOE_CONTROL_WORDS = 8 };
 
 // seam checks shared by the mat-vec and grouped-GEMM entry points (api.cu)
 lmoe_status lmoe_id_shape_check(const lmoe_expert_stack *stack, const void *x, int64_t t, int64_t x_per_row,

@@ -445,12 +445,22 @@ static lmoe_status experts_prefill(const lmoe_layer *L, const void *x, int x_f16
     return LMOE_OK;
 }
 
-// Routing through route_filter.cu once the f32 product is the longer one (a block's forward, cold L2, us without / with: hidden 3072, 256
-// experts, 256 / 384 / 512 / 640 / 2048 / 4096 / 16384 tokens 379 / 386, 421 / 417, 456 / 450, 482 / 466, 806 / 728, 1295 / 1166, 4550 / 3920; hidden 2048,
-// 128 experts, 400 / 800 / 1200 / 2400 tokens 175 / 180, 207 / 204, 248 / 241, 366 / 351; of 64 experts more are left: hidden 4096, 1200 / 2400 tokens
-// 245 / 248, 373 / 370).
+// Routing through route_filter.cu once the f32 product is the longer one.  A block's forward with experts of width 256, cold L2, us without / with:
+//   tokens                    512          768         1024         2048         4096        16384
+//   hidden 3072, 256     223 / 220    257 / 239    288 / 265    422 / 357    677 / 576   2290 / 1867
+//   hidden 4096, 256     238 / 234    283 / 256    314 / 275    488 / 404    772 / 630   2599 / 2066
+//   hidden 1024, 256         -        126 / 118    134 / 124    189 / 163    295 / 241    902 / 709
+//   hidden 4096, 128     177 / 187    214 / 212    239 / 230    377 / 353    625 / 579   2115 / 1977
+//   hidden 2048, 128         -        136 / 134    150 / 145    228 / 216    375 / 341   1197 / 1107
+//   hidden 2048, 96          -            -        142 / 142    214 / 208    351 / 335   1138 / 1099
+//   hidden 4096, 64          -        163 / 171    207 / 215    310 / 314    549 / 535   1880 / 1930
+//   hidden 2304, 64          -            -            -        233 / 189    397 / 308   1374 / 1010
+//   hidden 1280, 256         -        189 / 136    217 / 151    344 / 204    585 / 311   2079 / 961
+// The tiled f32 product is for hidden a multiple of 512; without it the filter pays far sooner, and for 64 experts too.  Where the bounds tell next to nothing
+// apart a call takes up to 4 to 25 % longer than without, see route_filter.cu; at half of the lines up to 60 %.
 static bool prefill_filters(const lmoe_layer *L, int64_t t) {
-    return (double)t * L->n_expert * L->hidden >= (L->n_expert >= 128 ? 3e8 : 6e8) && route_filter_available(L->hidden, L->n_expert, L->top_k);
+    const bool tiled = L->hidden % 512 == 0;
+    return (double)t * L->n_expert * L->hidden >= (tiled ? 6e8 : 3e8) && (!tiled || L->n_expert >= 96) && route_filter_available(L->hidden, L->n_expert, L->top_k);
 }
 
 size_t prefill_workspace_bytes(const lmoe_layer *L, int64_t t) {

@@ -3,19 +3,26 @@
 // Reference: `route_logits` and `route_from_logits`, src/moe.rs:84-119.
 //
 // The specified logits (route_math.cuh) are f32 products in a fixed order: for 16384 tokens, 256 experts and hidden 3072 they and the selection
-// take 730 us at half of the f32 rate, for 2048 tokens 115.  This takes 290 and 57: 5 for the router's f16 image, 42 / 13 for the approximate product
+// take 730 us at half of the f32 rate, for 2048 tokens 115.  This takes 290 and 60: 5 for the router's f16 image, 42 / 13 for the approximate product
 // (16384 tokens: the tokens from memory at 4.8 TB/s), 240 / 38 for the rest (the router rows from the L2 cache).  A product of the operands rounded to f16 differs from it by at most
 //   |x| |w| (2^-10 + 2^-22 + 17/16 hidden 2^-23 + 2^-18) + 2^-25 sqrt(hidden) (|x| + |w|)
 // (2^-11 for the rounding of either operand by Cauchy's inequality; the tensor core adds sixteen products to a sum at a time, each of the seventeen
 // cut, at worst, at the last of 24 bits of the largest of them; 2^-18 for the sum of the parts and for the specified sum, each a chain of at most 39 roundings; the last
 // term for values below the f16 range), so it bounds every score, and an expert whose
-// upper bound is below the top_k-th largest lower bound is out.  13 of 256 experts are left for a token of the benchmark's
-// router.  A token with a bound that is not finite (an operand beyond the f16 range, an infinity, NaN) keeps all its experts.
+// upper bound is below the top_k-th largest lower bound is out.  13 of 256 experts are left for a token of random normal values and weights, 12 with
+// weights ten times as large, 39 where eight of the 3072 channels are a hundred times the others and their weights a hundredth.  A token with a bound that is not
+// finite (an operand beyond the f16 range, an infinity, NaN) keeps all its experts, as do scores that all tie.
+// How many are left hangs on the data, so it is counted: up to a quarter of the experts on the average of a block's tokens, and one token that keeps all, the block
+// computes their logits itself; beyond, the router rows that it reads for every four tokens take longer than the tiled f32 product does, and the tokens that keep
+// too many go to a kernel of that product.
+// A block's forward, hidden 3072, 256 experts of 256, 2048 tokens (3072 tokens), f32 routing alone 409 us (534): 345 (468) at 13 left, 364 (499) at 24, 384 (535) at 39,
+// 466 (635) at 97, 447 (606) at 165 and 426 (591) at all 256; with all computed in the blocks 20 to 35 % more than the f32 routing from 97 left on.
 #include <math.h>
 #include <type_traits>
 
 #include "fused.cuh"
 #include "route_math.cuh"
+#include "route_tile.cuh"
 #include "tc.cuh"
 
 namespace {
@@ -26,12 +33,13 @@ constexpr int RF_SPLITS = 4; // most parts that hidden is cut into
 constexpr int RF_AHEAD = 3; // stages whose words a producing thread has in flight
 
 // The router as f16 in the order of the B operand's stages (64 values of all experts: a 128-byte-swizzled tile), and its rows' norms.
-// A block per expert.  clear: the call's control words.
+// A block per expert.  clear: the call's control words; done: route_dense_kernel's counts.
 __global__ void __launch_bounds__(128) route_prep_kernel(const float *__restrict__ router, int hidden, int n_expert, uint8_t *__restrict__ img,
-                                                         float *__restrict__ wnorm, uint32_t *__restrict__ clear) {
+                                                         float *__restrict__ wnorm, uint32_t *__restrict__ clear, uint32_t *__restrict__ done, int tiles) {
     pdl_begin();
     const int e = blockIdx.x;
     if (e == 0 && threadIdx.x < LMOE_CONTROL_WORDS) clear[threadIdx.x] = 0u;
+    for (int i = e * 128 + threadIdx.x; i < tiles; i += n_expert * 128) done[i] = 0u;
     const float4 *w = reinterpret_cast<const float4 *>(router + (size_t)e * hidden);
     float ss = 0.f;
     for (int ci = threadIdx.x; ci < hidden / 8; ci += 128) {
@@ -226,11 +234,33 @@ __device__ __forceinline__ float route_bound(float v, float side) {
     return p + side * (p * (8e-7f + (1e-6f + 2e-7f * fabsf(a)) * (1.f - p)) + 1e-37f);
 }
 
+// As in route_select_kernel, from a token's logits in shared memory; the experts that are out do not exist.
+template <int PER>
+__device__ __forceinline__ void route_select_token(float *probs, const float *__restrict__ bias, int n_expert, int top_k, float scale, int norm, uint32_t *ids_row,
+                                                   float *w_row, int lane) {
+    uint32_t key[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int e = lane + 32 * j;
+        key[j] = 0u;
+        if (e < n_expert) {
+            const float v = probs[e];
+            if (__float_as_uint(v) != RV_OUT) {
+                const float p = lmoe_sigmoid_fixed(v);
+                probs[e] = p;
+                key[j] = lmoe_score_key(bias ? __fadd_rn(p, __ldg(bias + e)) : p);
+            }
+        }
+    }
+    __syncwarp();
+    lmoe_warp_select_keys<PER>(key, probs, top_k, scale, norm, ids_row, w_row, lane);
+}
+
 template <int TB, int PER>
 __global__ void __launch_bounds__(RV_WARPS * 32, 1)
 route_verify_kernel(const float *__restrict__ router, const float *__restrict__ x, const float *__restrict__ bias, const float *__restrict__ approx,
                     const float *__restrict__ xss, int splits, const float *__restrict__ wnorm, int t, int hidden, int n_expert, int top_k, float scale, int norm,
-                    uint32_t *__restrict__ ids, float *__restrict__ weights, uint32_t *__restrict__ control) {
+                    uint32_t *__restrict__ ids, float *__restrict__ weights, int dense_from, uint32_t *__restrict__ dense, uint32_t *__restrict__ control) {
     extern __shared__ __align__(16) uint8_t rv_raw[];
     float4 *xs = reinterpret_cast<float4 *>(rv_raw);
     float *lg = reinterpret_cast<float *>(rv_raw + (size_t)TB * hidden * 4); // [token][expert]
@@ -247,7 +277,8 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s32(xs + i)), "l"(reinterpret_cast<const float4 *>(x + (size_t)t0 * hidden) + i) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
     __syncthreads();
-    int left = 0; // experts left for the warp's token
+    int left = 0;      // experts left for the warp's token
+    uint32_t mine = 0; // this lane's of them
     if (warp < nt) { // a warp's token: bounds of its scores
         const int tok = t0 + warp;
         float lo[PER], hi[PER], l[PER], W[PER], b[PER];
@@ -293,22 +324,33 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
             }
         }
 #pragma unroll
-        for (int j = 0; j < PER; j++) {
-            const int e = lane + 32 * j;
-            const bool in = e < n_expert && (all || lmoe_score_key(hi[j]) >= kth);
-            const uint32_t who = __ballot_sync(0xffffffffu, in);
-            if (e < n_expert && !in) lg[warp * n_expert + e] = __uint_as_float(RV_OUT);
-            if (in) {
-                const int at = left + __popc(who & ((1u << lane) - 1u));
-                if (at < 32) cand[warp][at] = (uint16_t)e;
-                atomicOr(&mask[e], 1u << warp);
-            }
-            left += __popc(who);
-        }
+        for (int j = 0; j < PER; j++) mine |= (uint32_t)(lane + 32 * j < n_expert && (all || lmoe_score_key(hi[j]) >= kth)) << j;
+        left = (int)__reduce_add_sync(0xffffffffu, (uint32_t)__popc(mine));
         if (lane == 0) atomicAdd(&n_left, left);
     }
     __syncthreads();
     if (tid == 0) atomicAdd(control + LMOE_CONTROL_LEFT, (uint32_t)n_left);
+    // where the bounds hardly tell the experts of a block's tokens apart, the tokens that keep too many go to route_dense_kernel
+    const bool handed = left > dense_from && n_left > TB * dense_from + n_expert / 4;
+    if (handed) {
+        if (lane == 0) dense[atomicAdd(control + LMOE_CONTROL_DENSE, 1u)] = (uint32_t)(t0 + warp);
+    } else if (warp < nt) {
+        int at = 0;
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const int e = lane + 32 * j;
+            const bool in = mine >> j & 1u;
+            const uint32_t who = __ballot_sync(0xffffffffu, in);
+            if (e < n_expert && !in) lg[warp * n_expert + e] = __uint_as_float(RV_OUT);
+            if (in) {
+                const int place = at + __popc(who & ((1u << lane) - 1u));
+                if (place < 32) cand[warp][place] = (uint16_t)e;
+                atomicOr(&mask[e], 1u << warp);
+            }
+            at += __popc(who);
+        }
+    }
+    __syncthreads();
     for (int e = tid; e < n_expert; e += RV_WARPS * 32) {
         uint32_t m = mask[e];
         const int groups = (__popc(m) + RV_TOKENS - 1) / RV_TOKENS;
@@ -379,7 +421,7 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
         while (multiply(wa, wb) && multiply(wb, wa)) {}
     }
     __syncthreads();
-    if (warp >= nt) return;
+    if (warp >= nt || handed) return;
     uint32_t *ids_row = ids + (size_t)(t0 + warp) * top_k;
     float *w_row = weights + (size_t)(t0 + warp) * top_k, *probs = lg + warp * n_expert;
     if (left <= 32) {
@@ -410,25 +452,61 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
         }
         return;
     }
-    // as in route_select_kernel; the experts that are out do not exist
-    uint32_t key[PER];
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-        const int e = lane + 32 * j;
-        key[j] = 0u;
-        if (e < n_expert) {
-            const float v = probs[e];
-            if (__float_as_uint(v) != RV_OUT) {
-                const float p = lmoe_sigmoid_fixed(v);
-                probs[e] = p;
-                key[j] = lmoe_score_key(bias ? __fadd_rn(p, __ldg(bias + e)) : p);
-            }
-        }
-    }
-    __syncwarp();
-    lmoe_warp_select_keys<PER>(key, probs, top_k, scale, norm, ids_row, w_row, lane);
+    route_select_token<PER>(probs, bias, n_expert, top_k, scale, norm, ids_row, w_row, lane);
 }
 
+// The tokens that route_verify_kernel hands over: all their specified logits, as route_logits_tiled_kernel computes them, then the selection, by the block that
+// finishes a tile's last share of the experts.  The number of tokens is known only here, so the tiles and shares are chosen here: by the
+// time of the longest block, in half passes (of 16 tokens x 16 experts or 8 x 32; the staging of a tile is about a pass for 16 tokens).
+template <int T, int PER>
+__device__ __forceinline__ void route_dense(const float *router, const float *x, const float *bias, const uint32_t *list, int n, int passes, int hidden, int n_expert,
+                                            int top_k, float scale, int norm, float *logits, uint32_t *done, uint32_t *ids, float *weights, uint8_t *smem) {
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, share = passes * (256 / T), shares = (n_expert + share - 1) / share;
+    float *probs = reinterpret_cast<float *>(smem + (size_t)T * hidden * 4 + RT_FOLD) + warp * n_expert;
+    for (int i = blockIdx.x; i < (n + T - 1) / T * shares; i += gridDim.x) {
+        const int tile = i / shares, e0 = (i - tile * shares) * share, t0 = tile * T, nt = min(T, n - t0);
+        route_tile<T>(router, [&](int k) { return x + (size_t)list[t0 + k] * hidden; }, nt, hidden, n_expert, e0, min(n_expert, e0 + share), smem,
+                      logits + (size_t)t0 * n_expert);
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            last = atomicAdd(done + tile, 1u) == (uint32_t)shares - 1u;
+            __threadfence();
+        }
+        __syncthreads();
+        if (last)
+            for (int k = warp; k < nt; k += RT_THREADS / 32) {
+                const size_t tok = list[t0 + k];
+                for (int e = lane; e < n_expert; e += 32) probs[e] = __ldcg(logits + (size_t)(t0 + k) * n_expert + e);
+                __syncwarp();
+                route_select_token<PER>(probs, bias, n_expert, top_k, scale, norm, ids + tok * top_k, weights + tok * top_k, lane);
+                __syncwarp();
+            }
+    }
+}
+template <int PER>
+__global__ void __launch_bounds__(RT_THREADS, 1)
+route_dense_kernel(const float *__restrict__ router, const float *__restrict__ x, const float *__restrict__ bias, const uint32_t *__restrict__ list,
+                   const uint32_t *__restrict__ control, int hidden, int n_expert, int top_k, float scale, int norm, float *logits, uint32_t *done,
+                   uint32_t *__restrict__ ids, float *__restrict__ weights, int sixteen) {
+    extern __shared__ __align__(16) uint8_t rd_smem[];
+    pdl_begin();
+    const int n = (int)__ldcg(control + LMOE_CONTROL_DENSE);
+    if (n == 0) return;
+    // a lane a choice: 1 to 16 passes of 16 tokens, 1 to 8 of 8 (n_expert <= 256)
+    const int lane = threadIdx.x & 31, g = (int)gridDim.x;
+    auto cost = [&](int T, int p) {
+        const int passes = (n_expert * T + 255) / 256, blocks = (n + T - 1) / T * ((passes + p - 1) / p);
+        return p > passes || (T == 16 && !sixteen) ? 0xffffffffu : (uint32_t)((blocks + g - 1) / g * (2 * p + T / 8)) << 5;
+    };
+    const uint32_t mine = lane < 16 ? cost(16, 16 - lane) : (lane < 24 ? cost(8, 24 - lane) : 0xffffffffu);
+    const int choice = (int)(__reduce_min_sync(0xffffffffu, mine == 0xffffffffu ? mine : mine | lane) & 31u);
+    if (choice < 16) route_dense<16, PER>(router, x, bias, list, n, 16 - choice, hidden, n_expert, top_k, scale, norm, logits, done, ids, weights, rd_smem);
+    else route_dense<8, PER>(router, x, bias, list, n, 24 - choice, hidden, n_expert, top_k, scale, norm, logits, done, ids, weights, rd_smem);
+}
+
+int rd_smem_bytes(int t, int64_t hidden, int64_t n_expert) { return (int)(t * hidden * 4 + RT_FOLD + RT_THREADS / 32 * n_expert * 4); }
 int rv_smem(int tb, int64_t hidden, int64_t n_expert) { return (int)(tb * hidden * 4 + tb * n_expert * 4 + (tb + RV_TOKENS - 1) / RV_TOKENS * n_expert * 4 + n_expert * 4); }
 
 } // namespace
@@ -438,17 +516,20 @@ bool route_filter_available(int64_t hidden, int64_t n_expert, int64_t top_k) {
     return hidden % 128 == 0 && hidden >= 512 && hidden <= 4096 && n_expert % 32 == 0 && n_expert >= 64 && n_expert <= 256 && top_k <= 32 && top_k * 8 <= n_expert &&
            rv_smem(8, hidden, n_expert) <= 227 * 1024 - 4096;
 }
-// Scratch: the router's f16 image, the norms, and the approximate logits by part of hidden, for at most this many token rows (never fewer for more
+// Scratch: the list of the tokens handed over and a count by tile of them, the router's f16 image, the norms, and the approximate logits by part of hidden, for at most this many token rows (never fewer for more
 // tokens: a workspace for t tokens serves any smaller number).
+static size_t rf_list_bytes(int64_t t) { return lmoe_align_up((size_t)t * 4, 256) + lmoe_align_up((size_t)(t + 7) / 8 * 4, 256); }
 static int64_t rf_rows(int64_t t) { return t > 16384 ? t : (RF_SPLITS * t < 16384 ? RF_SPLITS * t : 16384); }
 size_t route_filter_bytes(int64_t t, int64_t hidden, int64_t n_expert) {
-    return lmoe_align_up((size_t)n_expert * hidden * 2, 256) + lmoe_align_up((size_t)n_expert * 4, 256) + lmoe_align_up((size_t)rf_rows(t) * 4, 256) +
+    return rf_list_bytes(t) + lmoe_align_up((size_t)n_expert * hidden * 2, 256) + lmoe_align_up((size_t)n_expert * 4, 256) + lmoe_align_up((size_t)rf_rows(t) * 4, 256) +
            (size_t)rf_rows(t) * n_expert * 4;
 }
 
 cudaError_t launch_route_filter(const float *router, const float *bias, const float *x, int t, int hidden, int n_expert, int top_k, float scale, int norm,
                                 void *scratch, uint32_t *ids, float *weights, uint32_t *flag, cudaStream_t s) {
-    uint8_t *img = static_cast<uint8_t *>(scratch);
+    uint32_t *list = static_cast<uint32_t *>(scratch);
+    uint32_t *done = list + lmoe_align_up((size_t)t * 4, 256) / 4;
+    uint8_t *img = static_cast<uint8_t *>(scratch) + rf_list_bytes(t);
     float *wnorm = reinterpret_cast<float *>(img + lmoe_align_up((size_t)n_expert * hidden * 2, 256));
     float *xss = wnorm + lmoe_align_up((size_t)n_expert * 4, 256) / 4, *logits = xss + lmoe_align_up((size_t)rf_rows(t) * 4, 256) / 4;
     const int most = 227 * 1024 - 4096;
@@ -462,9 +543,11 @@ cudaError_t launch_route_filter(const float *router, const float *bias, const fl
             if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most - 1024)) != cudaSuccess) return e;
         for (auto f : {route_verify_kernel<16, 4>, route_verify_kernel<16, 8>, route_verify_kernel<8, 4>, route_verify_kernel<8, 8>})
             if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most)) != cudaSuccess) return e;
+        for (auto f : {route_dense_kernel<4>, route_dense_kernel<8>})
+            if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most)) != cudaSuccess) return e;
         c_dev = dev;
     }
-    launch_pdl(route_prep_kernel, n_expert, 128, 0, s, router, hidden, n_expert, img, wnorm, flag);
+    launch_pdl(route_prep_kernel, n_expert, 128, 0, s, router, hidden, n_expert, img, wnorm, flag, done, (t + 7) / 8);
     // 128 tokens a block where that covers two thirds of the device, else 64 and hidden in as many parts as there are SMs for
     const bool large = (t + 127) / 128 * 3 >= 2 * c_sms;
     const int tiles = large ? (t + 127) / 128 : (t + 63) / 64;
@@ -472,11 +555,18 @@ cudaError_t launch_route_filter(const float *router, const float *bias, const fl
     while (!large && splits < RF_SPLITS && tiles * splits * 2 <= c_sms && (int64_t)t * splits * 2 <= rf_rows(t) && hidden / 64 % (2 * splits) == 0) splits *= 2;
     launch_pdl(large ? route_approx_kernel<128> : route_approx_kernel<64>, dim3((unsigned)tiles, (unsigned)splits), 320,
                RF_STAGES * (RF_A_BYTES + n_expert * 128) + 1024, s, x, img, t, hidden, n_expert, logits, xss, flag);
+    const bool dense = hidden % (128 * RT_AHEAD) == 0; // else a block computes what is left whatever it is, in no more time than the untiled product
     // sixteen tokens a block where the rows fit and the blocks are enough for the device
     const int tb = rv_smem(16, hidden, n_expert) <= most && (t + 15) / 16 * 5 >= 4 * c_sms ? 16 : 8;
     auto verify = n_expert <= 128 ? (tb == 16 ? route_verify_kernel<16, 4> : route_verify_kernel<8, 4>)
                                   : (tb == 16 ? route_verify_kernel<16, 8> : route_verify_kernel<8, 8>);
     launch_pdl(verify, (unsigned)((t + tb - 1) / tb), RV_WARPS * 32, rv_smem(tb, hidden, n_expert), s, router, x, bias, logits, xss, splits, wnorm, t, hidden,
-               n_expert, top_k, scale, norm, ids, weights, flag);
+               n_expert, top_k, scale, norm, ids, weights, dense ? n_expert / 4 : n_expert, list, flag);
+    if (dense) {
+        const bool sixteen = rd_smem_bytes(16, hidden, n_expert) <= most;
+        launch_pdl(n_expert <= 128 ? route_dense_kernel<4> : route_dense_kernel<8>, (unsigned)c_sms, RT_THREADS,
+                   rd_smem_bytes(sixteen ? 16 : 8, hidden, n_expert), s, router, x, bias, list, flag, hidden, n_expert, top_k, scale, norm, logits, done, ids,
+                   weights, (int)sixteen);
+    }
     return cudaGetLastError();
 }

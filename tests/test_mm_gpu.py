@@ -208,8 +208,9 @@ def test_prefill_block_tile_heights(orc, dev, hidden, ff, t):
     _check_block(orc, blk, blk.host_layer(orc), np.random.default_rng(t).standard_normal((t, hidden)).astype(np.float32), 2e-3)
 
 
-@pytest.mark.parametrize("hidden,ne,top_k,t,bias", [(3072, 256, 10, 385, False), (3072, 256, 10, 2501, True), (4096, 96, 12, 1531, True),
-                                                    (1024, 256, 32, 1921, False), (512, 64, 8, 18313, True), (768, 128, 1, 5089, False)])
+@pytest.mark.parametrize("hidden,ne,top_k,t,bias", [(3072, 256, 10, 771, False), (3072, 256, 10, 2501, True), (4096, 96, 12, 1531, True),
+                                                    (1024, 256, 32, 2401, False), (512, 96, 8, 18313, True), (768, 128, 1, 5089, False),
+                                                    (1280, 64, 8, 5001, True)])
 def test_prefill_routing_through_the_filter(dev, hidden, ne, top_k, t, bias):
     """Long prompts take the tensor core's bounds first: ids and weights are those of the stand-alone routing, which are the oracle's, to
     the bit.  Both token tiles of either kernel, ragged counts; tokens that keep all experts (an infinity, NaN, values beyond the f16
@@ -237,21 +238,21 @@ def test_prefill_routing_through_the_filter(dev, hidden, ne, top_k, t, bias):
     assert t * top_k <= left <= t * (1.5 * top_k + 3) + 12 * ne
 
 
-def _check_routing(blk, x):
+def _check_routing(blk, x, with_handed=False):
     """Ids and weights of a prompt against the stand-alone routing, to the bit; returns the count of experts that the filter left
-    (0: the filter did not run)."""
+    (0: the filter did not run), and that of the tokens that got all their logits."""
     blk.workspace(x.shape[0])[:32].zero_()
     _, ids, w = blk.forward(x, return_routing=True, path="prefill")
     ids2, w2 = blk.route(x)
     torch.cuda.synchronize()
-    left = int(blk.workspace(x.shape[0])[16:20].view(torch.int32))
+    left, handed = blk.workspace(x.shape[0])[16:24].view(torch.int32).tolist()
     blk.check_device_flag()
     assert torch.equal(ids, ids2) and torch.equal(w.view(torch.int32), w2.view(torch.int32))
-    return left
+    return (left, handed) if with_handed else left
 
 
 @pytest.mark.parametrize("value", [float("-inf"), torch.finfo(torch.float32).min, -1e9, float("inf"), float("nan")])
-@pytest.mark.parametrize("hidden,ne,top_k,t", [(3072, 256, 10, 2048), (4096, 64, 8, 2500)])
+@pytest.mark.parametrize("hidden,ne,top_k,t", [(3072, 256, 10, 2048), (4096, 96, 8, 2500)])
 def test_prefill_routing_filter_with_any_bias(dev, hidden, ne, top_k, t, value):
     """An expert that its bias excludes or fixes, by an infinity, the type's lowest value or NaN, leaves the other experts' bounds as they
     are."""
@@ -278,6 +279,29 @@ def test_prefill_routing_filter_with_small_scores(dev):
     blk.router[:, 0] = -1.4
     left = _check_routing(blk, x)
     assert 2048 * 10 <= left <= 2048 * 30
+
+
+@pytest.mark.parametrize("hidden,ne,top_k,t,hands", [(3072, 256, 10, 2501, True), (3072, 256, 10, 801, True), (1024, 256, 32, 20001, True), (4096, 96, 12, 1531, True),
+                                                     (512, 96, 8, 18313, True), (768, 128, 1, 5089, False)])
+@pytest.mark.parametrize("case", ["all", "runs", "few"])
+def test_prefill_routing_where_bounds_do_not_tell(dev, hidden, ne, top_k, t, hands, case):
+    """Tokens whose scores all tie, or whose bounds are wider than the scores' differences, get all their logits from the tiled product: every token, runs of
+    them between ordinary ones, or one in fifty, which most blocks compute themselves.  Tile heights of 16 and 8, ragged last tiles, more and fewer tiles than SMs; a hidden
+    size that the tiled product does not take."""
+    from maxuna_b200.moe import MoeBlock
+
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(t)
+    blk = MoeBlock.random(hidden, 256, ne, top_k, seed=hidden + ne, device=dev, bias=torch.zeros(ne, device=dev))
+    x = torch.randn(t, hidden, generator=gen, device=dev)
+    blk.router[:, 7] = blk.router[0, 7]  # a channel that no expert prefers: a large value in it widens the bounds only
+    at = torch.arange(t, device=dev)
+    tie = {"all": at >= 0, "runs": at // 37 % 2 == 0, "few": at % 50 == 13}[case]
+    x[tie, 7] = 3e4 * (1 - 2 * (at[tie] % 2).float())
+    left, handed = _check_routing(blk, x, with_handed=True)
+    ties = int(tie.sum())
+    assert left >= ties * ne // 2 + (t - ties) * top_k
+    assert (ties // 2 if hands and case != "few" else 0) <= handed <= (t if hands else 0)
 
 
 def test_prefill_block_wide_ff(orc, dev):
