@@ -11,7 +11,7 @@
 // term for values below the f16 range), so it bounds every score, and an expert whose
 // upper bound is below the top_k-th largest lower bound is out.  13 of 256 experts are left for a token of random normal values and weights, 12 with
 // weights ten times as large, 39 where eight of the 3072 channels are a hundred times the others and their weights a hundredth.  A token with a bound that is not
-// finite (an operand beyond the f16 range, an infinity, NaN) keeps all its experts, as do scores that all tie.
+// finite (an operand beyond the f16 range, an infinity, NaN) keeps all its experts, as do scores that all tie, but for a row of zeros, whose logits are known.
 // How many are left hangs on the data, so it is counted: up to a quarter of the experts on the average of a block's tokens, and one token that keeps all, the block
 // computes their logits itself; beyond, the router rows that it reads for every four tokens take longer than the tiled f32 product does, and the tokens that keep
 // too many go to a kernel of that product.
@@ -279,10 +279,11 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
     __syncthreads();
     int left = 0;      // experts left for the warp's token
     uint32_t mine = 0; // this lane's of them
+    bool flat = false; // a row of zeros, of a padded prompt
     if (warp < nt) { // a warp's token: bounds of its scores
         const int tok = t0 + warp;
         float lo[PER], hi[PER], l[PER], W[PER], b[PER];
-        bool finite = true;
+        bool finite = true, tiny = true;
 #pragma unroll
         for (int j = 0; j < PER; j++) {
             const int e = min(lane + 32 * j, n_expert - 1);
@@ -305,7 +306,11 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
             lo[j] = __fadd_rn(route_bound(l[j] - d, -1.f), b[j]);
             hi[j] = __fadd_rn(route_bound(l[j] + d, 1.f), b[j]);
             finite = finite && isfinite(l[j]) && isfinite(d);
+            tiny = tiny && X * W[j] < 0x1p-27f && W[j] < 1e8f;
         }
+        // Logits below 2^-26 all have the sigmoid 0.5, exactly (1 + r rounds to 1 in its exponential), so none need be computed.  (Values whose squares
+        // underflow are missing from X: 64 of 1.1e-19 times 1e8 are below 2^-27 as well.)
+        flat = __all_sync(0xffffffffu, finite && tiny);
         const bool all = !__all_sync(0xffffffffu, finite);
         uint32_t key[PER], kth = 0u; // the top_k-th largest lower bound
 #pragma unroll
@@ -325,7 +330,7 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
         }
 #pragma unroll
         for (int j = 0; j < PER; j++) mine |= (uint32_t)(lane + 32 * j < n_expert && (all || lmoe_score_key(hi[j]) >= kth)) << j;
-        left = (int)__reduce_add_sync(0xffffffffu, (uint32_t)__popc(mine));
+        left = flat ? 0 : (int)__reduce_add_sync(0xffffffffu, (uint32_t)__popc(mine));
         if (lane == 0) atomicAdd(&n_left, left);
     }
     __syncthreads();
@@ -334,6 +339,8 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
     const bool handed = left > dense_from && n_left > TB * dense_from + n_expert / 4;
     if (handed) {
         if (lane == 0) dense[atomicAdd(control + LMOE_CONTROL_DENSE, 1u)] = (uint32_t)(t0 + warp);
+    } else if (flat) {
+        for (int e = lane; e < n_expert; e += 32) lg[warp * n_expert + e] = 0.f;
     } else if (warp < nt) {
         int at = 0;
 #pragma unroll
@@ -424,7 +431,7 @@ route_verify_kernel(const float *__restrict__ router, const float *__restrict__ 
     if (warp >= nt || handed) return;
     uint32_t *ids_row = ids + (size_t)(t0 + warp) * top_k;
     float *w_row = weights + (size_t)(t0 + warp) * top_k, *probs = lg + warp * n_expert;
-    if (left <= 32) {
+    if (!flat && left <= 32) {
         // a lane an expert: its slot is the number of those before it (a larger score, or the same and a lower index)
         const int e = lane < left ? cand[warp][lane] : 0;
         const float p = lane < left ? lmoe_sigmoid_fixed(probs[e]) : 0.f;

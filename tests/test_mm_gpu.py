@@ -304,6 +304,30 @@ def test_prefill_routing_where_bounds_do_not_tell(dev, hidden, ne, top_k, t, han
     assert (ties // 2 if hands and case != "few" else 0) <= handed <= (t if hands else 0)
 
 
+@pytest.mark.parametrize("hidden,ne,top_k,t", [(3072, 256, 10, 2501), (3072, 256, 10, 801), (4096, 96, 12, 1531), (768, 128, 1, 5089)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_prefill_routing_of_rows_of_zeros(dev, hidden, ne, top_k, t, bias):
+    """A padded prompt: rows of zeros, of values too small for their squares and of values whose logits just reach 2^-27 get their ids without a
+    logit, larger ones not; a router of zeros."""
+    from maxuna_b200.moe import MoeBlock
+
+    gen = torch.Generator(device=dev)
+    gen.manual_seed(t)
+    b = 0.2 * torch.rand(ne, generator=gen, device=dev) - 0.1 if bias else torch.zeros(ne, device=dev)
+    blk = MoeBlock.random(hidden, 256, ne, top_k, seed=hidden + ne, device=dev, bias=b)
+    x = torch.randn(t, hidden, generator=gen, device=dev)
+    at = torch.arange(t, device=dev)
+    small = torch.tensor([0.0, 1e-25, 1e-20, 2.0 ** -40, 2.0 ** -33, 2.0 ** -30, 2.0 ** -24], device=dev)
+    pad = at % 16 >= 9
+    x[pad] *= small[at[pad] % 16 - 9][:, None]
+    left = _check_routing(blk, x)
+    ordinary = int((~pad).sum())
+    # of the seven kinds of small rows the last three may count as others do
+    assert ordinary * top_k <= left <= ordinary * (1.5 * top_k + 3) + 3 * t // 16 * ne
+    blk.router.zero_()
+    assert _check_routing(blk, x) == 0
+
+
 def test_prefill_block_wide_ff(orc, dev):
     # expert_ff = 512: two Q6_K super-blocks per down row (the 256-row down kernel), ragged row tiles
     from maxuna_b200.moe import MoeBlock
