@@ -463,13 +463,17 @@ static bool prefill_filters(const lmoe_layer *L, int64_t t) {
     return (double)t * L->n_expert * L->hidden >= (tiled ? 6e8 : 3e8) && (!tiled || L->n_expert >= 96) && route_filter_available(L->hidden, L->n_expert, L->top_k);
 }
 
+// Scratch of the routing: the f32 logits, or the filter's, which has room for them (a call with unaligned operands takes the f32 routing all the same).
+static size_t prefill_route_bytes(const lmoe_layer *L, int64_t t) {
+    return prefill_filters(L, t) ? route_filter_bytes(t, L->hidden, L->n_expert) : (size_t)t * L->n_expert * 4;
+}
+
 size_t prefill_workspace_bytes(const lmoe_layer *L, int64_t t) {
     if (t < 1) t = 1;
     const int64_t rows = t * L->top_k;
     size_t o = 65536;
-    o += lmoe_align_up((size_t)t * L->n_expert * 4, 256);            // logits
+    o += lmoe_align_up(prefill_route_bytes(L, t), 256);
     o += 2 * lmoe_align_up((size_t)rows * 4, 256);                   // ids, weights
-    if (prefill_filters(L, t)) o += route_filter_bytes(t, L->hidden, L->n_expert);
     o += experts_ws_bytes(L, t, L->top_k);
     return o;
 }
@@ -485,17 +489,17 @@ lmoe_status launch_moe_prefill(const lmoe_layer *L, const float *x, const float 
     const int64_t rows = t * L->top_k, H = L->hidden;
     Carver c{static_cast<uint8_t *>(workspace), 65536};
     uint32_t *flag = reinterpret_cast<uint32_t *>(workspace);
-    float *logits = c.take<float>((size_t)t * L->n_expert);
+    uint8_t *route_ws = c.take<uint8_t>(prefill_route_bytes(L, t));
     uint32_t *ids = c.take<uint32_t>((size_t)rows);
     float *w = c.take<float>((size_t)rows);
-    uint8_t *rf_ws = c.take<uint8_t>(prefill_filters(L, t) ? route_filter_bytes(t, H, L->n_expert) : 0);
     const bool filter = prefill_filters(L, t) && ((reinterpret_cast<uintptr_t>(L->router) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0;
     uint8_t *ex_ws = static_cast<uint8_t *>(workspace) + c.off;
 
     // (both begin with a fresh device flag: the workspace needs no initialisation)
     if (filter) {
-        LMOE_CUDA(launch_route_filter(L->router, L->bias, x, (int)t, (int)H, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, rf_ws, ids, w, flag, s));
+        LMOE_CUDA(launch_route_filter(L->router, L->bias, x, (int)t, (int)H, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, route_ws, ids, w, flag, s));
     } else {
+        float *logits = reinterpret_cast<float *>(route_ws);
         LMOE_CUDA(launch_route_logits(L->router, x, (int)t, (int)H, (int)L->n_expert, logits, s));
         LMOE_CUDA(launch_route_select(logits, L->bias, (int)t, (int)L->n_expert, (int)L->top_k, L->scale, L->norm, ids, w, s, flag));
     }
