@@ -95,13 +95,7 @@ __device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t *r) {
                  : "memory");
 }
 // ---- dequantisation ----------------------------------------------------------------
-// The conversion is bound by instruction issue, so every operation is one instruction by construction ((v & mask) | magic
-// written in C costs two logic operations): asm for the three-input logic operation.
-__device__ __forceinline__ uint32_t and_or(uint32_t v, uint32_t mask, uint32_t magic) {
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(magic));
-    return r;
-}
+// The conversion is bound by instruction issue, so every operation is one instruction by construction.
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t r;
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
@@ -116,17 +110,6 @@ __device__ __forceinline__ uint32_t h2_sub_fma(uint32_t v, uint32_t base, uint32
 __device__ __forceinline__ uint32_t h2_sub_mul(uint32_t v, uint32_t base, uint32_t s) {
     uint32_t r;
     asm("{\n\t.reg .b32 t;\n\tsub.rn.f16x2 t, %1, %2;\n\tmul.rn.f16x2 %0, t, %3;\n\t}" : "=r"(r) : "r"(v), "r"(base), "r"(s));
-    return r;
-}
-
-__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t r;
-    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
     return r;
 }
 
@@ -381,7 +364,8 @@ struct GmCfg {
     static constexpr int EPI_BYTES = NPROJ == 2 ? GM_EPI_BYTES : 2 * GM_BOX_ROWS * 128;
     static constexpr int B_ROWS = NT / CG;
     static constexpr int B_BLK = B_ROWS * MM_K * 2;     // a CTA's half of a 64-k block of the B operand
-    // blocks of a full tile in a ring slot (two in the slots of gate/up's 128-row tiles: 768 / 1024 tokens 500 / 536 -> 497 / 529 us)
+    // blocks of a full tile in a ring slot (two in the slots of gate/up's 128-row tiles, three runs in turn: 64 experts of 1536, hidden 4096,
+    // 176 / 280 / 400 tokens 285.5 / 295.0 / 310.3 -> 283.6 / 291.8 / 306.1 us, 256 experts of 1024 0.5 to 1.5 % where two runs differ by 1)
     static constexpr int B_FULL = (NPROJ == 2 || CG == 1 ? 1 : 2) * (NT == 64 || (NPROJ == 2 && NT == 128) ? 2 : 1);
     static constexpr int B_SLOT = B_FULL * B_BLK;
     static constexpr int NB = 96 * 1024 / B_SLOT < 8 ? 96 * 1024 / B_SLOT : 8;
@@ -692,7 +676,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) grouped_mm_kernel(const __grid_
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + C::O_BAR);
     // a_full[s]: the eight warps of the stage's group, of both CTAs; a_empty[s]: one commit; b_full[i]: the copies' bytes, or both CTAs'
     // loaders; b_empty[i]: one commit;
-    // raw_full[i]: the copies' bytes; raw_empty[i]: all sixteen dequantising warps; acc_*: per accumulator buffer
+    // raw_full[i]: the copies' bytes; raw_empty[i]: the dequantising warps that read it, all sixteen or the eight of a
+    // group (RAW_READERS); acc_*: per accumulator buffer
     uint64_t *a_full = bars, *a_empty = bars + 4, *b_full = bars + 8, *b_empty = bars + 16, *raw_full = bars + 24,
              *raw_empty = bars + 28, *acc_full = bars + 32, *acc_empty = bars + 34;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 36);

@@ -33,32 +33,14 @@ struct MdCfg {
     static constexpr int SMEM = (Q4 ? O_SUMS + MD_SUMS : O_RAW + MD_ROWS * MD_Q6_PITCH * 4) + 1024;
 };
 
-__device__ __forceinline__ uint32_t md_lop(uint32_t v, uint32_t mask, uint32_t magic) { // (v & mask) | magic
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(magic));
-    return r;
-}
 __device__ __forceinline__ uint32_t md_sub(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
-__device__ __forceinline__ uint32_t md_mul(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-__device__ __forceinline__ uint32_t md_fma(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t r;
-    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-    return r;
-}
 __device__ __forceinline__ uint32_t md_twice(float v) { // f16 pair (v, v)
     const uint32_t h = __half_as_ushort(__float2half_rn(v));
     return h | h << 16;
-}
-__device__ __forceinline__ void tc_ld4(uint32_t taddr, uint32_t (&r)[4]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
 }
 __device__ __forceinline__ void md_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a),
@@ -262,12 +244,12 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
 #pragma unroll
                 for (int d = 1; d < 5; d++) {
 #pragma unroll
-                    for (int p = 0; p < 4; p++) h[p] = md_sub(md_lop((d < 3 ? dig[v][4 + p] : dig[v][p]) >> ((d & 1) ? 7 : 0), seven, 0x64006400u), off);
+                    for (int p = 0; p < 4; p++) h[p] = md_sub(and_or((d < 3 ? dig[v][4 + p] : dig[v][p]) >> ((d & 1) ? 7 : 0), seven, 0x64006400u), off);
                     put(d, h);
                 }
 #pragma unroll
                 for (int p = 0; p < 4; p++)
-                    h[p] = md_sub(md_lop(dig[v][p] >> 12, 0x000C000Cu, md_lop(dig[v][4 + p] >> 14, 0x00030003u, 0x64006400u)), 0x64086408u);
+                    h[p] = md_sub(and_or(dig[v][p] >> 12, 0x000C000Cu, and_or(dig[v][4 + p] >> 14, 0x00030003u, 0x64006400u)), 0x64086408u);
                 put(0, h);
             } else {
 #pragma unroll
@@ -302,13 +284,13 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
             const uint32_t v[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const uint32_t s = __byte_perm(pair, 0u, h ? 0x3232u : 0x1010u), c0 = md_mul(s, 0xE400E400u); // - 1024 scales
+                const uint32_t s = __byte_perm(pair, 0u, h ? 0x3232u : 0x1010u), c0 = h2_mul(s, 0xE400E400u); // - 1024 scales
 #pragma unroll
                 for (int c = 0; c < 4; c++) { // (1024 + q) scale - 1024 scale: exact
                     const uint32_t u0 = v[2 * c] >> (4 * h), u1 = v[2 * c + 1] >> (4 * h);
                     *reinterpret_cast<uint4 *>(a + md_at(rr, 4 * h + c)) =
-                        make_uint4(md_fma(md_lop(u0, 0x000F000Fu, 0x64006400u), s, c0), md_fma(md_lop(u0 >> 8, 0x000F000Fu, 0x64006400u), s, c0),
-                                   md_fma(md_lop(u1, 0x000F000Fu, 0x64006400u), s, c0), md_fma(md_lop(u1 >> 8, 0x000F000Fu, 0x64006400u), s, c0));
+                        make_uint4(h2_fma(and_or(u0, 0x000F000Fu, 0x64006400u), s, c0), h2_fma(and_or(u0 >> 8, 0x000F000Fu, 0x64006400u), s, c0),
+                                   h2_fma(and_or(u1, 0x000F000Fu, 0x64006400u), s, c0), h2_fma(and_or(u1 >> 8, 0x000F000Fu, 0x64006400u), s, c0));
                 }
             }
         } else {
@@ -329,12 +311,12 @@ mv_dense_kernel(const uint8_t *__restrict__ w, int n_out, int k, const float *__
                     for (int i = 0; i < 2; i++) {
                         const uint32_t ql = word(16 * (j >> 1) + 8 * h + 2 * c + i) >> (4 * (j & 1));
                         const uint32_t t = (word(32 + 8 * (j >> 1) + 2 * c + i) >> (4 * (j & 1) + 2 * h) & 0x03030303u) << 4;
-                        const uint32_t q6 = md_lop(ql, 0x0F0F0F0Fu, t);
+                        const uint32_t q6 = and_or(ql, 0x0F0F0F0Fu, t);
                         e[2 * i] = md_sub(__byte_perm(q6, 0x64646464u, 0x4240), 0x64206420u);
                         e[2 * i + 1] = md_sub(__byte_perm(q6, 0x64646464u, 0x4341), 0x64206420u);
                     }
-                    *reinterpret_cast<uint4 *>(a + md_at(rr, 4 * h + c)) = make_uint4(md_mul(e[0], hi), md_mul(e[1], hi), md_mul(e[2], hi), md_mul(e[3], hi));
-                    *reinterpret_cast<uint4 *>(a + C::O_LOW + md_at(rr, 4 * h + c)) = make_uint4(md_mul(e[0], lo), md_mul(e[1], lo), md_mul(e[2], lo), md_mul(e[3], lo));
+                    *reinterpret_cast<uint4 *>(a + md_at(rr, 4 * h + c)) = make_uint4(h2_mul(e[0], hi), h2_mul(e[1], hi), h2_mul(e[2], hi), h2_mul(e[3], hi));
+                    *reinterpret_cast<uint4 *>(a + C::O_LOW + md_at(rr, 4 * h + c)) = make_uint4(h2_mul(e[0], lo), h2_mul(e[1], lo), h2_mul(e[2], lo), h2_mul(e[3], lo));
                 }
             }
         }

@@ -928,10 +928,10 @@ cudaError_t launch_mv(const uint8_t *w, int64_t expert_bytes, int n_expert, int 
     int dev, sms;
     cudaError_t e = mv_device(dev, sms);
     if (e != cudaSuccess) return e;
+    if (mv_dense_better(DT, w, n_expert, n_out, k, pairs, sms)) return launch_mv_dense(DT, w, n_out, k, x, pairs, x_per_row, ids, top_k, out, s);
     // One matrix for all pairs: 32 pairs to an unpacked super-block, once such blocks cover every SM.  (Below that two pairs to a
     // block win by parallelism: [1024 x 3072] Q4_K, 64 / 512 pairs 26 / 92 us against 44 / 68, [3072 x 1024] Q6_K, 32 / 128
     // pairs 19 / 44 against 26 / 39.)
-    if (mv_dense_better(DT, w, n_expert, n_out, k, pairs, sms)) return launch_mv_dense(DT, w, n_out, k, x, pairs, x_per_row, ids, top_k, out, s);
     if (mv_multi_better(n_expert, n_out, pairs, sms)) {
         constexpr int smem = MM_COLS * MM_PITCH<DT> + MV_PARTS * MM_COLS * (MM_KC / QK_K * NS + 8) * 2 + (MM_KC / QK_K) * MM_COLS * 4;
         constexpr int CS = 4;

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(320, 1) route_approx_kernel(const float *__res
 
 // The specified logits of the experts that the approximate ones leave, then the selection: a block of TB tokens, whose rows lie in
 // shared memory.  The experts left for any of them are taken in turn by sixteen warps, each router row once for up to
-// four tokens: 146 rows for the 212 logits of sixteen tokens.  The rows from the L2 cache are what bounds it (16384 tokens: 1.8 GB; with each piece
+// four tokens: some 150 rows for some 210 logits of sixteen tokens.  The rows from the L2 cache are what bounds it (16384 tokens: 1.8 GB; with each piece
 // of a row waited for before the next is asked for 424 us; with sixteen exact sigmoids a lane for the bounds and selection by rounds 297; so 240).
 constexpr int RV_WARPS = 16, RV_TOKENS = 4, RV_PIECE = 8;
 constexpr uint32_t RV_OUT = 0xffa5a5a5u; // in place of the logit of an expert that is out: a NaN that no operation results in

@@ -1,5 +1,4 @@
-// mbarriers, bulk copies and the 5th-generation tensor core in PTX: what grouped_mm_kernel (mm_id.cu) and route_approx_kernel
-// (route_filter.cu) share.
+// mbarriers, bulk copies, the 5th-generation tensor core and pairs of halves in PTX: what mm_id.cu, mv_dense.cu and route_filter.cu share.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -59,6 +58,9 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                    "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr));
 }
+__device__ __forceinline__ void tc_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+}
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // One lane of a converged warp, chosen by the hardware: code under this predicate is known to be single-lane.
 __device__ __forceinline__ bool elect_one() {
@@ -74,6 +76,24 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
     const uint64_t lo = (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16);           // LBO (unused) = 16 B
     const uint64_t hi = (uint64_t)(1024 >> 4) | ((uint64_t)1 << 14) | ((uint64_t)2 << 29);   // SBO 1024 B, version 1, SWIZZLE_128B
     return lo | (hi << 32);
+}
+
+// (v & mask) | magic in one instruction, which it is not when written in C
+__device__ __forceinline__ uint32_t and_or(uint32_t v, uint32_t mask, uint32_t magic) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(magic));
+    return r;
+}
+// f16 pairs
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
 }
 
 } // namespace
