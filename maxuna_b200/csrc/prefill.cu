@@ -457,10 +457,11 @@ static lmoe_status experts_prefill(const lmoe_layer *L, const void *x, int x_f16
 //   hidden 2304, 64          -            -            -        233 / 189    397 / 308   1374 / 1010
 //   hidden 1280, 256         -        189 / 136    217 / 151    344 / 204    585 / 311   2079 / 961
 // The tiled f32 product is for hidden a multiple of 512; without it the filter pays far sooner, and for 64 experts too.  Where the bounds tell next to nothing
-// apart a call takes up to 4 to 25 % longer than without, see route_filter.cu; at half of the lines up to 60 %.
+// apart a call takes up to 4 to 25 % longer than without, see route_filter.cu, so the line lies where a plain prompt gains 4 %: 256 experts of 256, hidden 3072, 512 / 640 tokens
+// 224 / 220 and 244 / 232 us, but with eight channels a hundred times the others 223 / 247 and 246 / 258.
 static bool prefill_filters(const lmoe_layer *L, int64_t t) {
-    const bool tiled = L->hidden % 512 == 0;
-    return (double)t * L->n_expert * L->hidden >= (tiled ? 6e8 : 3e8) && (!tiled || L->n_expert >= 96) && route_filter_available(L->hidden, L->n_expert, L->top_k);
+    const bool tiled = L->hidden % 512 == 0, early = !tiled || (L->hidden <= 2048 && L->n_expert >= 128);
+    return (double)t * L->n_expert * L->hidden >= (early ? 3e8 : 5e8) && (!tiled || L->n_expert >= 96) && route_filter_available(L->hidden, L->n_expert, L->top_k);
 }
 
 // Scratch of the routing: the f32 logits, or the filter's, which has room for them (a call with unaligned operands takes the f32 routing all the same).

@@ -208,7 +208,7 @@ def test_prefill_block_tile_heights(orc, dev, hidden, ff, t):
     _check_block(orc, blk, blk.host_layer(orc), np.random.default_rng(t).standard_normal((t, hidden)).astype(np.float32), 2e-3)
 
 
-@pytest.mark.parametrize("hidden,ne,top_k,t,bias", [(3072, 256, 10, 771, False), (3072, 256, 10, 2501, True), (4096, 96, 12, 1531, True),
+@pytest.mark.parametrize("hidden,ne,top_k,t,bias", [(3072, 256, 10, 641, False), (3072, 256, 10, 771, False), (3072, 256, 10, 2501, True), (4096, 96, 12, 1531, True),
                                                     (1024, 256, 32, 2401, False), (512, 96, 8, 18313, True), (768, 128, 1, 5089, False),
                                                     (1280, 64, 8, 5001, True)])
 def test_prefill_routing_through_the_filter(dev, hidden, ne, top_k, t, bias):
